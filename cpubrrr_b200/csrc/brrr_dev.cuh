@@ -115,12 +115,14 @@ __host__ __device__ __forceinline__ size_t q8_bytes(int rows, int cols) { return
 __host__ __device__ __forceinline__ size_t q8_unit_off(int urow, int pair, int np) { return ((size_t)urow * np + pair) * Q8_UNIT; }
 
 // MXFP4 unit (544 B), rows % 16 == 0, blocks % 2 == 0, np = blocks / 2:
-//   bytes [0, 512):   [16 rows][4 lanes][8 B]; the 8 bytes of (row, pair i, lane j) are the lane
+//   bytes [0, 512):   [row / 8][4 lanes][8 rows][8 B]; the 8 bytes of (row, pair i, lane j) are the lane
 //                     word (bytes 4j..4j+3 of the 16 nibble bytes) of block 2i then of block 2i+1
 //   bytes [512, 544): [16 rows][2] e8m0 bytes
-// A warp (8 rows x 4 lanes) reads 256 contiguous bytes per step.
+// A warp (8 rows x 4 lanes) reads 256 contiguous bytes per step; the 64 bytes of 8 rows and one lane are the unit a
+// tensor copy widens into a column of operand A (kernels_tile.cu).
 constexpr int MX_UNIT = 544;
 constexpr int MX_UNIT_EXPS = 512;
+__host__ __device__ __forceinline__ int mx_word_off(int rl, int j) { return (rl >> 3) * 256 + j * 64 + (rl & 7) * 8; }      // row rl of a unit, lane j
 struct MxDev {
     uint8_t *data;
     int rows, blocks;

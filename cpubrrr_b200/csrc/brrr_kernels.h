@@ -11,9 +11,12 @@ void launch_quant_q8(const float *x, int n, int8_t *q, float *s, cudaStream_t st
 // rows > 1: one CTA per row; rows are n apart in x / xn / q and n / 32 apart in s
 cudaError_t launch_rmsnorm_quant(const float *x, const float *w, float eps, int n, float *xn, int8_t *q, float *s, bool pdl, cudaStream_t st,
                                  int rows = 1);
-// ---- token rows (kernels_rows.cu): y[t][r] (+)= row r of m . activation t (+ bias), t < ntok <= 16
-cudaError_t launch_q8_rows(Q8Dev m, const int8_t *xq, const float *xs, int ntok, const float *bias, float *y, int ldy, int epi, bool pdl,
-                           cudaStream_t st, DevState *state = nullptr, int engine = -1);
+// ---- token rows (kernels_rows.cu): y[t][r] (+)= row r of m . activation t (+ bias) on the integer units
+cudaError_t launch_q8_rows(Q8Dev m, const int8_t *xq, const float *xs, int ntok, const float *bias, float *y, int ldy, int epi, bool pdl, cudaStream_t st);
+// residual rows x [rows][d]: part != nullptr: x[t] += sum over k of wts[8 t + k] * part[t * topk + k]; norm_w != nullptr: RMSNorm, Q8 per 32-block (scales s,
+// int8 q nullable) and activation image img (nullable; image = TI_HALF or TI_PLANES, brrr_tile.cuh), normalised floats xn (nullable)
+cudaError_t launch_rows_norm(float *x, int rows, int d, const float *part, const float *wts, int topk, const float *norm_w, float eps, float *xn, int8_t *q,
+                             float *s, uint8_t *img, int image, bool pdl, cudaStream_t st);
 // RoPE of every row's k and the cache append of k and v (row t: position row_pos[t] of sequence row_seq[t])
 cudaError_t launch_kv_append_rows(const float *qkv, int ldq, int nh, int nkv, float *kc, float *vc, size_t seq_stride, const float *rope,
                                   const int *row_pos, const int *row_seq, int rows, bool pdl, cudaStream_t st);
@@ -144,19 +147,25 @@ cudaError_t launch_down_t(MxtDev down, const float *down_b, const int32_t *top, 
                           int d, const uint8_t *himg, const float *hs, float *x, float *part, uint32_t *counter, DevState *state,
                           bool pdl, cudaStream_t st, const EpCtx *ep = nullptr, int layer = 0);
 
-// ---- token-tile matmul on tcgen05 tensor cores (kernels_tile.cu): y[t][r] = row (row0 + r) . activation t,
-// t < ntok <= BRRR_TILE_MAX, every value bit-identical to launch_mx_gemv on token t alone
-cudaError_t launch_mx_tile(MxDev w, int row0, int nrows, const int8_t *xq, const float *xs, int ntok, float *y, int ldy, DevState *state,
-                           cudaStream_t st);
-
-// every expert of one matrix kind against the (token, slot) entries routed to it (cnt[e], list[e][BRRR_TILE_MAX], at most max_entries per expert);
-// entry i reads activation row entry / src_div and writes y[entry * ldy + col0 + row] (+ bias[e][row])
-cudaError_t launch_mx_tile_experts(MxDev w, int ne, int rows_per_expert, const int *cnt, const int *list, int max_entries, int src_div, const int8_t *xq,
-                                   const float *xs, const float *bias, float *y, int ldy, int col0, DevState *state, cudaStream_t st);
-cudaError_t launch_q8_tile(Q8Dev m, const int8_t *xq, const float *xs, int ntok, const float *bias, float *y, int ldy, int epi, DevState *state,
-                           bool pdl, cudaStream_t st);          // Q8 matrix x token rows on kind::i8 (kernels_tile.cu)
-void launch_tile_route(const int32_t *top, int ntok, int topk, int ne, int *cnt, int *list, cudaStream_t st);
-void launch_tile_combine(const float *part, const float *wts, int topk, int d, int ntok, float *x, cudaStream_t st);
+// ---- matrices x token rows on the tensor cores (kernels_tile.cu), t < ntok <= BRRR_TILE_MAX, every value bit-identical to the one-token kernels.
+// Activations come as images (brrr_tile.cuh), image_bytes(rows, cols, kind) each, and block scales [row][cols / 32].
+size_t image_bytes(int rows, int cols, int kind);      // plane images must be zero before their first use
+void launch_image(const int8_t *xq, int rows, int cols, int kind, uint8_t *img, cudaStream_t st);      // kind = TI_HALF or TI_PLANES
+// Q8 matrix re-laid as operand units (the weights as halves in operand order, 2.1 x the Q8 bytes)
+size_t q8_operand_bytes(int rows, int cols);
+void launch_q8_operand_pack(Q8Dev m, uint8_t *out, cudaStream_t st);
+cudaError_t launch_q8_tile(const uint8_t *op, int rows, int cols, const uint8_t *img, const float *xs, int ntok, const float *bias, float *y, int ldy,
+                           int epi, DevState *state, bool pdl, cudaStream_t st);
+// y[t * ldy + i] = row (row0 + i) of w . activation t
+cudaError_t launch_mx_tile(MxDev w, int row0, int nrows, const uint8_t *img, const float *xs, int ntok, float *y, int ldy, DevState *state, cudaStream_t st);
+// per expert the (token, slot) entries routed to it: cnt[ne], list[ne][BRRR_TILE_MAX], entry = token * topk + slot
+cudaError_t launch_tile_route(const int32_t *top, int ntok, int topk, int ne, int *cnt, int *list, bool pdl, cudaStream_t st);
+// gate and up of every expert for its entries, SwiGLU, Q8 of h: plane images himg [entry] and scales hs [entry][d / 32]
+cudaError_t launch_mx_tile_glu(MxDev gate, MxDev up, int ne, int d, const int *cnt, const int *list, int ntok, int topk, const uint8_t *img, const float *xs,
+                               const float *gate_b, const float *up_b, uint8_t *himg, float *hs, DevState *state, bool pdl, cudaStream_t st);
+// part[entry][d] = down row . h of the entry + bias
+cudaError_t launch_mx_tile_down(MxDev down, int ne, int d, const int *cnt, const int *list, int ntok, int topk, const uint8_t *himg, const float *hs,
+                                const float *bias, float *part, DevState *state, bool pdl, cudaStream_t st);
 
 void launch_ep_begin(const EpCtx &c, DevState *state, cudaStream_t st);
 // down-projection of the local experts, exchange of the 16-row slices, fold in slot order
@@ -192,12 +201,13 @@ cudaError_t launch_router_hint(const float *x_in, const float *norm_w, float eps
 // KV cache layout [n_head_kv][BRRR_MAXSEQ][64].  pos is read from state when state != nullptr,
 // else pos_val.  window = 0 means full attention.
 cudaError_t launch_attn_rows(const float *qkv, int ldq, const float *kc, const float *vc, size_t seq_stride, const float *rope, const float *sinks,
-                             int nh, int nkv, int window, const int *row_pos, const int *row_seq, int rows, float *ao, int8_t *aq, float *as,
+                             int nh, int nkv, int window, const int *row_pos, const int *row_seq, int rows, float *ao, int8_t *aq, float *as, uint8_t *aimg,
                              DevState *err_state, bool pdl, cudaStream_t st);       // rows of one sequence share their K / V tiles (prompt tiles)
 cudaError_t launch_attn_decode(const float *qkv, float *kc, float *vc, const float *rope, const float *sinks, int nh, int nkv,
                                const DevState *state, int pos_val, int window, float *ao, int8_t *aq, float *as,
                                DevState *err_state, bool pdl, cudaStream_t st, int pos_off = 0, const int *row_pos = nullptr,
-                               const int *row_seq = nullptr, size_t seq_stride = 0, int ldq = 0, int rows = 1);
+                               const int *row_seq = nullptr, size_t seq_stride = 0, int ldq = 0, int rows = 1, uint8_t *aimg = nullptr);
+// aimg (token rows; nullable): the half images of the quantised outputs (brrr_tile.cuh), nh * 128 bytes per row; aq may then be nullptr
 // row_pos != nullptr: `rows` tokens in one launch (grid.y), see AttnArgs in kernels_attn.cu; the rows' k / v must be in the cache already
 // pos_off is added to the position read from state (ignored with pos_val)
 

@@ -56,7 +56,7 @@ __device__ __forceinline__ float mx_pairs(const unsigned char *unit, int rl, int
 #pragma unroll
     for (int i = 0; i < N; i++) {
         const unsigned char *u = unit + (size_t)i * MX_UNIT;
-        w[i] = *reinterpret_cast<const uint2 *>(u + rl * 32 + j * 8);
+        w[i] = *reinterpret_cast<const uint2 *>(u + mx_word_off(rl, j));
         e2[i] = *reinterpret_cast<const unsigned short *>(u + MX_UNIT_EXPS + rl * 2);
         x0[i] = xpj[(pair + i) * 8]; x1[i] = xpj[(pair + i) * 8 + 4];
         xs0[i] = xsc[2 * (pair + i)]; xs1[i] = xsc[2 * (pair + i) + 1];

@@ -9,6 +9,15 @@
 
 namespace brrr {
 
+// One lane of a converged warp.  Roles that issue tensor-core products run their loop with the whole warp and elect a lane for the
+// instructions only: the loop's values are then uniform, while inside a one-lane branch every operand of a tcgen05 instruction
+// is first moved to a uniform register (about 100 cycles per product).
+__device__ __forceinline__ bool elect_one() {
+    uint32_t p;
+    asm volatile("{\n\t.reg .pred p;\n\telect.sync _|p, 0xffffffff;\n\tselp.u32 %0, 1, 0, p;\n\t}" : "=r"(p));
+    return p != 0;
+}
+
 __device__ __forceinline__ uint32_t smem_u32(const void *p) { return (uint32_t)__cvta_generic_to_shared(p); }
 
 __device__ __forceinline__ void mbar_init(uint64_t *bar, uint32_t count) {

@@ -2,6 +2,7 @@
 // launches the same kernel the forward pass uses for that stage.
 #include "../../include/brrr.h"
 #include "brrr_kernels.h"
+#include "brrr_tile.cuh"
 
 #include <cstdio>
 
@@ -11,7 +12,7 @@ namespace {
 int check_launch() { return cudaGetLastError() == cudaSuccess ? BRRR_OK : BRRR_ERR_CUDA; }
 }  // namespace
 
-struct brrr_q8mat { Q8Dev m; };
+struct brrr_q8mat { Q8Dev m; uint8_t *op; };      // op: operand units of the tensor-core product (token rows)
 struct brrr_mxmat { MxDev m; };
 
 extern "C" int brrr_quant_q8(const float *d_x, int n, int8_t *d_q, float *d_s, void *stream) {
@@ -49,13 +50,16 @@ extern "C" int brrr_rmsnorm_quant(const float *d_x, const float *d_w, float eps,
     return check_launch();
 }
 
+extern "C" void brrr_q8mat_free(brrr_q8mat *m);
 extern "C" int brrr_q8mat_from_bf16(const uint16_t *d_w, int rows, int cols, brrr_q8mat **out, void *stream) {
     if (!d_w || !out || rows <= 0 || cols <= 0 || cols % 64 || cols > 4096) return BRRR_ERR_ARG;
     brrr_q8mat *q = new brrr_q8mat();
     q->m.rows = rows; q->m.cols = cols;
     if (cudaMalloc(&q->m.data, q8_bytes(rows, cols)) != cudaSuccess) { delete q; return BRRR_ERR_NOMEM; }
-    if (cudaMemsetAsync(q->m.data, 0, q8_bytes(rows, cols), (cudaStream_t)stream) != cudaSuccess) { cudaFree(q->m.data); delete q; return BRRR_ERR_CUDA; }
+    if (cudaMalloc(&q->op, q8_operand_bytes(rows, cols)) != cudaSuccess) { cudaFree(q->m.data); delete q; return BRRR_ERR_NOMEM; }
+    if (cudaMemsetAsync(q->m.data, 0, q8_bytes(rows, cols), (cudaStream_t)stream) != cudaSuccess) { brrr_q8mat_free(q); return BRRR_ERR_CUDA; }
     launch_q8_pack(d_w, rows, 0, q->m, (cudaStream_t)stream);
+    launch_q8_operand_pack(q->m, q->op, (cudaStream_t)stream);
     *out = q;
     return check_launch();
 }
@@ -69,6 +73,7 @@ extern "C" int brrr_q8mat_export(const brrr_q8mat *m, int8_t *d_q, float *d_s, v
 extern "C" void brrr_q8mat_free(brrr_q8mat *m) {
     if (!m) return;
     cudaFree(m->m.data);
+    cudaFree(m->op);
     delete m;
 }
 
@@ -81,9 +86,15 @@ extern "C" int brrr_q8_matvec(const brrr_q8mat *w, const int8_t *d_xq, const flo
 extern "C" int brrr_q8_matmul_rows(const brrr_q8mat *w, const int8_t *d_xq, const float *d_xs, int ntok, float *d_y, int ldy, int tensor_cores,
                                    void *stream) {
     if (!w || !d_xq || !d_xs || !d_y || ntok < 1 || ntok > BRRR_TILE_MAX || ldy < w->m.rows) return BRRR_ERR_ARG;
-    if (launch_q8_rows(w->m, d_xq, d_xs, ntok, nullptr, d_y, ldy, Q8_EPI_PLAIN, false, (cudaStream_t)stream, nullptr, tensor_cores ? 1 : 0) != cudaSuccess)
-        return BRRR_ERR_CUDA;
-    return check_launch();
+    cudaStream_t st = (cudaStream_t)stream;
+    if (!tensor_cores)
+        return launch_q8_rows(w->m, d_xq, d_xs, ntok, nullptr, d_y, ldy, Q8_EPI_PLAIN, false, st) == cudaSuccess ? check_launch() : BRRR_ERR_CUDA;
+    uint8_t *img = nullptr;          // activation images: stream-ordered scratch, so calls on different streams do not share it
+    if (cudaMallocAsync(&img, image_bytes(ntok, w->m.cols, TI_HALF), st) != cudaSuccess) return BRRR_ERR_NOMEM;
+    launch_image(d_xq, ntok, w->m.cols, TI_HALF, img, st);
+    const cudaError_t e = launch_q8_tile(w->op, w->m.rows, w->m.cols, img, d_xs, ntok, nullptr, d_y, ldy, Q8_EPI_PLAIN, nullptr, false, st);
+    cudaFreeAsync(img, st);
+    return e == cudaSuccess ? check_launch() : BRRR_ERR_CUDA;
 }
 
 extern "C" int brrr_mxmat_from_gguf(const uint8_t *d_raw, int rows, int blocks, brrr_mxmat **out, void *stream) {
@@ -112,8 +123,14 @@ extern "C" int brrr_mx_matmul_tile(const brrr_mxmat *w, int row0, int nrows, con
                                    void *stream) {
     if (!w || !d_xq || !d_xs || !d_y || row0 < 0 || nrows <= 0 || row0 + nrows > w->m.rows || ntok < 1 || ntok > BRRR_TILE_MAX || ldy < nrows) return BRRR_ERR_ARG;
     if (((uintptr_t)d_xq & 3)) return BRRR_ERR_ARG;
-    if (launch_mx_tile(w->m, row0, nrows, d_xq, d_xs, ntok, d_y, ldy, nullptr, (cudaStream_t)stream) != cudaSuccess) return BRRR_ERR_CUDA;
-    return check_launch();
+    cudaStream_t st = (cudaStream_t)stream;
+    uint8_t *img = nullptr;          // activation images: stream-ordered scratch, so calls on different streams do not share it
+    if (cudaMallocAsync(&img, image_bytes(ntok, w->m.blocks * 32, TI_PLANES), st) != cudaSuccess) return BRRR_ERR_NOMEM;
+    cudaMemsetAsync(img, 0, image_bytes(ntok, w->m.blocks * 32, TI_PLANES), st);
+    launch_image(d_xq, ntok, w->m.blocks * 32, TI_PLANES, img, st);
+    const cudaError_t e = launch_mx_tile(w->m, row0, nrows, img, d_xs, ntok, d_y, ldy, nullptr, st);
+    cudaFreeAsync(img, st);
+    return e == cudaSuccess ? check_launch() : BRRR_ERR_CUDA;
 }
 
 extern "C" int brrr_router_topk(const float *d_w, const float *d_b, const float *d_xn, int ne, int d, int topk,

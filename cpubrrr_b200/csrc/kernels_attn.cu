@@ -15,6 +15,7 @@
 #include "brrr_kernels.h"
 #include "brrr_block.cuh"
 #include "brrr_tma.cuh"
+#include "brrr_tile.cuh"
 
 namespace brrr {
 
@@ -43,7 +44,17 @@ struct AttnArgs {
     const int *row_pos, *row_seq;
     size_t seq_stride;
     int ldq;
+    uint8_t *img;            // token rows, nullable: half images of the outputs (brrr_tile.cuh)
 };
+
+// Q8 of 32-block b of a row's attention output, held one value per lane: int8 values, scale, half image
+__device__ __forceinline__ void attn_quant(float o, int lane, int b, int8_t *aq, float *as, uint8_t *img) {
+    const float sc = __fdiv_rn(fmaxf(warp_max(fabsf(o)), 1e-12f), 127.0f);
+    const int qv = brrr_q8_round(o, sc);
+    if (lane == 0) as[b] = sc;
+    if (aq) aq[b * 32 + lane] = (int8_t)qv;
+    if (img) ti_emit_block<TI_HALF>(qv, lane, b, img);
+}
 
 #ifndef AT_SCORE_UNROLL
 #define AT_SCORE_UNROLL 8
@@ -73,8 +84,9 @@ __global__ void __launch_bounds__(AT_THREADS) attn_decode_kernel(AttnArgs a) {
         a.kc += (size_t)a.row_seq[t] * a.seq_stride;
         a.vc += (size_t)a.row_seq[t] * a.seq_stride;
         a.ao += (size_t)t * a.nh * HD;
-        a.aq += (size_t)t * a.nh * HD;
+        if (a.aq) a.aq += (size_t)t * a.nh * HD;
         a.as += (size_t)t * a.nh * 2;
+        if (a.img) a.img += (size_t)t * a.nh * ti_pair(TI_HALF);
     }
 
     // The position is an input of this step (written before the graph launch or by the previous
@@ -228,7 +240,7 @@ __global__ void __launch_bounds__(AT_THREADS) attn_decode_kernel(AttnArgs a) {
         float o = __fmul_rn(acc, inv);
         a.ao[h * HD + tid] = o;
         // this head owns Q8 blocks 2h and 2h+1 of the attention output
-        warp_quant_block(o, tid & 31, a.aq + h * HD + (tid >> 5) * 32, a.as + h * 2 + (tid >> 5));
+        attn_quant(o, tid & 31, h * 2 + (tid >> 5), a.aq, a.as, a.img);
     }
     BRRR_STAMP(a.err_state, 165);
     BRRR_GT_END(a.err_state, 191);
@@ -262,6 +274,7 @@ struct AttnRowsArgs {
     float *ao;
     int8_t *aq;
     float *as;
+    uint8_t *img;            // nullable: half images of the outputs
     DevState *err_state;
 };
 
@@ -436,7 +449,7 @@ __global__ void __launch_bounds__(AR_THREADS) attn_rows_kernel(AttnRowsArgs a) {
             const float o = __fmul_rn(acc[j], inv);
             const size_t row = (size_t)(r0 + rr);
             a.ao[row * a.nh * HD + h * HD + u] = o;
-            warp_quant_block(o, lane, a.aq + row * a.nh * HD + h * HD + (u >> 5) * 32, a.as + row * a.nh * 2 + h * 2 + (u >> 5));
+            attn_quant(o, lane, h * 2 + (u >> 5), a.aq ? a.aq + row * a.nh * HD : nullptr, a.as + row * a.nh * 2, a.img ? a.img + row * a.nh * ti_pair(TI_HALF) : nullptr);
         }
     }
 }
@@ -446,8 +459,8 @@ static size_t attn_smem(int tile) { return (size_t)tile * HD * sizeof(float) * A
 cudaError_t launch_attn_decode(const float *qkv, float *kc, float *vc, const float *rope, const float *sinks, int nh, int nkv,
                                const DevState *state, int pos_val, int window, float *ao, int8_t *aq, float *as,
                                DevState *err_state, bool pdl, cudaStream_t st, int pos_off, const int *row_pos, const int *row_seq, size_t seq_stride,
-                               int ldq, int rows) {
-    AttnArgs a{qkv, kc, vc, rope, sinks, nh, nkv, state, pos_val, window, pos_off, ao, aq, as, err_state, row_pos, row_seq, seq_stride, ldq};
+                               int ldq, int rows, uint8_t *aimg) {
+    AttnArgs a{qkv, kc, vc, rope, sinks, nh, nkv, state, pos_val, window, pos_off, ao, aq, as, err_state, row_pos, row_seq, seq_stride, ldq, aimg};
     static unsigned long long configured = 0, configured_rows = 0;      // one bit per device
     if (row_pos) {
         cudaError_t e = smem_optin(attn_decode_kernel<AT_TILE_ROWS>, (int)attn_smem(AT_TILE_ROWS), configured_rows);
@@ -462,11 +475,11 @@ cudaError_t launch_attn_decode(const float *qkv, float *kc, float *vc, const flo
 // Attention for token rows of ONE sequence with ascending positions (a prompt tile): rows share the K / V tiles.
 // Needs the rows' keys in the cache already (launch_kv_append_rows) and nh / nkv a power of two <= 32.
 cudaError_t launch_attn_rows(const float *qkv, int ldq, const float *kc, const float *vc, size_t seq_stride, const float *rope, const float *sinks,
-                             int nh, int nkv, int window, const int *row_pos, const int *row_seq, int rows, float *ao, int8_t *aq, float *as,
+                             int nh, int nkv, int window, const int *row_pos, const int *row_seq, int rows, float *ao, int8_t *aq, float *as, uint8_t *aimg,
                              DevState *err_state, bool pdl, cudaStream_t st) {
     const int group = nkv > 0 ? nh / nkv : 0;
     if (group < 1 || group > 32 || (group & (group - 1)) || nh % nkv || rows < 1) return cudaErrorInvalidValue;
-    AttnRowsArgs a{qkv, kc, vc, rope, sinks, nh, nkv, window, rows, ldq, row_pos, row_seq, seq_stride, ao, aq, as, err_state};
+    AttnRowsArgs a{qkv, kc, vc, rope, sinks, nh, nkv, window, rows, ldq, row_pos, row_seq, seq_stride, ao, aq, as, aimg, err_state};
     static unsigned long long configured = 0;      // one bit per device
     cudaError_t e = smem_optin(attn_rows_kernel, (int)AR_SMEM, configured);
     if (e != cudaSuccess) return e;

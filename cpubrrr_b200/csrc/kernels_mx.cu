@@ -28,7 +28,7 @@ __global__ void mx_pack_kernel(const uint8_t *__restrict__ raw, MxDev m) {
     uint32_t w = (uint32_t)src[1 + 4 * j] | ((uint32_t)src[2 + 4 * j] << 8) | ((uint32_t)src[3 + 4 * j] << 16) | ((uint32_t)src[4 + 4 * j] << 24);
     uint8_t *unit = m.data + mx_unit_off(row >> 4, b >> 1, np);
     int rl = row & 15;
-    *reinterpret_cast<uint32_t *>(unit + rl * 32 + j * 8 + (b & 1) * 4) = w;
+    *reinterpret_cast<uint32_t *>(unit + mx_word_off(rl, j) + (b & 1) * 4) = w;
     if (j == 0) unit[MX_UNIT_EXPS + rl * 2 + (b & 1)] = src[0];
 }
 
@@ -42,7 +42,7 @@ void launch_mx_pack(const uint8_t *raw, MxDev m, cudaStream_t st) {
 // Two blocks (one pair) of one lane chain from a unit in shared memory.
 template <bool DBG>
 __device__ __forceinline__ float mx_pair_step(const unsigned char *unit, int rl, int j, const int2 *xpj, const float *xsc, int pair, float acc, int32_t *dbg) {
-    uint2 w = *reinterpret_cast<const uint2 *>(unit + rl * 32 + j * 8);
+    uint2 w = *reinterpret_cast<const uint2 *>(unit + mx_word_off(rl, j));
     uint32_t e2 = *reinterpret_cast<const unsigned short *>(unit + MX_UNIT_EXPS + rl * 2);
     int2 x0 = xpj[pair * 8], x1 = xpj[pair * 8 + 4];
     int t0 = brrr_mx_lane_dot(w.x, x0.x, x0.y);

@@ -89,7 +89,7 @@ __global__ void mxt_pack_kernel(PackArgs p, size_t total_words) {
         const int q = w >> 9, rem = w & 511, m = (rem >> 5) * 8 + ((rem >> 2) & 7), j = rem & 3;
         int rl = 0;
         const uint8_t *u = locate(m, rl);
-        if (u) v = *reinterpret_cast<const uint32_t *>(u + rl * 32 + j * 8 + q * 4);
+        if (u) v = *reinterpret_cast<const uint32_t *>(u + mx_word_off(rl, j) + q * 4);
     } else {
         for (int k = 0; k < 2; k++) {                 // rows m0, m0 + 1: two exponent bytes each
             int rl = 0;

@@ -10,10 +10,10 @@
 //                                    activations into shared memory, then one chain walk per four token rows
 //   kv_append_rows_kernel            RoPE of every row's k and the cache append of k and v, before any row attends
 //   attn_decode_kernel (grid.y = rows, kernels_attn.cu)
-#include <cstdlib>
 #include "brrr_kernels.h"
 #include "brrr_block.cuh"
 #include "brrr_tma.cuh"
+#include "brrr_tile.cuh"
 
 namespace brrr {
 
@@ -150,6 +150,66 @@ cudaError_t q8_rows_launch(const Q8RowsArgs &a, int epi, dim3 grid, size_t smem,
     return cudaErrorInvalidValue;
 }
 
+// ---------------------------------------------------------------- residual rows: combine, norm, activation image
+// One CTA per token row.  COMBINE: x[t] += w[t][k] * part[t * topk + k], k ascending (part already holds the bias): the
+// combine of down_combine_kernel.  With norm weights: RMSNorm of the new row (16-chain order, block_rms_inv), its Q8
+// per 32-block (one warp per block) and the image the next matmul reads (brrr_tile.cuh); optionally the normalised floats
+// (the router's input) and the int8 values in element order (the integer-unit projections of small tiles).
+struct RowsNormArgs {
+    float *x;
+    int d;
+    const float *part, *wts;        // combine: [row * topk + k][d], [row][8]
+    int topk;
+    const float *norm_w;            // nullable: combine only
+    float eps;
+    float *xn;                      // nullable
+    int8_t *q;                      // nullable
+    float *s;
+    uint8_t *img;                   // nullable
+};
+
+constexpr int RN_THREADS = 384;
+
+template <int IMG, bool COMBINE>
+__global__ void __launch_bounds__(RN_THREADS) rows_norm_kernel(RowsNormArgs a) {
+    extern __shared__ __align__(16) float rsm_x[];
+    __shared__ float inv_sh;
+    const int t = blockIdx.x, tid = threadIdx.x, d = a.d, groups = d >> 2;
+    pdl_wait();
+    pdl_trigger();
+    float4 *x4 = reinterpret_cast<float4 *>(a.x + (size_t)t * d);
+    for (int g = tid; g < groups; g += RN_THREADS) {
+        float4 v = x4[g];
+        if (COMBINE) {
+            float4 pv[8];
+#pragma unroll
+            for (int k = 0; k < 8; k++) if (k < a.topk) pv[k] = reinterpret_cast<const float4 *>(a.part + ((size_t)t * a.topk + k) * d)[g];
+#pragma unroll
+            for (int k = 0; k < 8; k++)
+                if (k < a.topk) {
+                    const float w = a.wts[t * 8 + k];
+                    v.x = __fadd_rn(v.x, __fmul_rn(w, pv[k].x)); v.y = __fadd_rn(v.y, __fmul_rn(w, pv[k].y));
+                    v.z = __fadd_rn(v.z, __fmul_rn(w, pv[k].z)); v.w = __fadd_rn(v.w, __fmul_rn(w, pv[k].w));
+                }
+            x4[g] = v;
+        }
+        reinterpret_cast<float4 *>(rsm_x)[g] = v;
+    }
+    if (!a.norm_w) return;
+    __syncthreads();
+    const float inv = block_rms_inv(rsm_x, d, a.eps, &inv_sh);
+    const int lane = tid & 31, nb = d / 32;
+    for (int b = tid >> 5; b < nb; b += RN_THREADS / 32) {
+        const float v = __fmul_rn(__fmul_rn(rsm_x[b * 32 + lane], inv), a.norm_w[b * 32 + lane]);
+        if (a.xn) a.xn[(size_t)t * d + b * 32 + lane] = v;
+        const float sc = __fdiv_rn(fmaxf(warp_max(fabsf(v)), 1e-12f), 127.0f);
+        const int qv = brrr_q8_round(v, sc);
+        if (lane == 0) a.s[(size_t)t * nb + b] = sc;
+        if (a.q) a.q[(size_t)t * d + b * 32 + lane] = (int8_t)qv;
+        if (a.img) ti_emit_block<IMG>(qv, lane, b, a.img + (size_t)t * (nb / 2) * ti_pair(IMG));
+    }
+}
+
 // RoPE of k (NeoX halves, the same operations as attn_decode_kernel) and the cache append of k and v for every row.
 struct KvRowsArgs {
     const float *qkv;        // [rows][ldq]: q | k | v of every row, bias added, not rotated
@@ -199,20 +259,26 @@ __global__ void __launch_bounds__(1024) rows_argmax_kernel(const float *__restri
 
 }  // namespace
 
+cudaError_t launch_rows_norm(float *x, int rows, int d, const float *part, const float *wts, int topk, const float *norm_w, float eps, float *xn, int8_t *q,
+                             float *s, uint8_t *img, int image, bool pdl, cudaStream_t st) {
+    if (topk > 8 || d % 64) return cudaErrorInvalidValue;
+    RowsNormArgs a{x, d, part, wts, topk, norm_w, eps, xn, q, s, img};
+    const size_t smem = (size_t)d * sizeof(float);
+    if (image == TI_HALF)
+        return part ? launch_k(rows_norm_kernel<TI_HALF, true>, dim3(rows), dim3(RN_THREADS), smem, st, pdl, a)
+                    : launch_k(rows_norm_kernel<TI_HALF, false>, dim3(rows), dim3(RN_THREADS), smem, st, pdl, a);
+    return part ? launch_k(rows_norm_kernel<TI_PLANES, true>, dim3(rows), dim3(RN_THREADS), smem, st, pdl, a)
+                : launch_k(rows_norm_kernel<TI_PLANES, false>, dim3(rows), dim3(RN_THREADS), smem, st, pdl, a);
+}
+
 void launch_rows_argmax(const float *logits, int n_vocab, int rows, uint32_t *out, cudaStream_t st) {
     rows_argmax_kernel<<<rows, 1024, 0, st>>>(logits, n_vocab, out);
 }
 
-// y[t][r] (+)= row r of m . activation t (+ bias) for t < ntok <= BRRR_TILE_MAX.  epi: Q8_EPI_PLAIN / BIAS / RESID_BIAS.
-// engine: 0 = integer units (the default: measured faster at every tile size so far), 1 = tensor cores (launch_q8_tile,
-// kernels_tile.cu), -1 = the environment variable BRRR_Q8_TILE=1 selects the tensor cores for tiles of at least 32 rows of
-// the layer projections.  Same bits either way.
-cudaError_t launch_q8_rows(Q8Dev m, const int8_t *xq, const float *xs, int ntok, const float *bias, float *y, int ldy, int epi, bool pdl,
-                           cudaStream_t st, DevState *state, int engine) {
+// y[t][r] (+)= row r of m . activation t (+ bias) for t < ntok <= BRRR_TILE_MAX on the integer units: tiles of a few rows, where the
+// tensor-core kernel (launch_q8_tile, kernels_tile.cu: 128 matrix rows per CTA) leaves most SMs idle.  epi: Q8_EPI_PLAIN / BIAS / RESID_BIAS.
+cudaError_t launch_q8_rows(Q8Dev m, const int8_t *xq, const float *xs, int ntok, const float *bias, float *y, int ldy, int epi, bool pdl, cudaStream_t st) {
     if (ntok < 1 || ntok > BRRR_TILE_MAX || m.cols % 64) return cudaErrorInvalidValue;
-    static const bool env_tile = [] { const char *e = getenv("BRRR_Q8_TILE"); return e && e[0] && e[0] != '0'; }();
-    const bool tile = engine == 1 || (engine < 0 && env_tile && ntok >= 32 && m.rows <= 16384);
-    if (tile) return launch_q8_tile(m, xq, xs, ntok, bias, y, ldy, epi, state, pdl, st);
     Q8RowsArgs a{m, xq, xs, bias, y, ntok, ldy};
     const int np = m.cols / 64, urows = q8_urows(m.rows);
     const size_t smem = (size_t)QR_TPC * np * 72;

@@ -1,66 +1,73 @@
-// Token-tile MXFP4 matmul on the 5th-generation tensor cores (tcgen05.mma kind::i8, accumulators in
-// tensor memory): the batched counterpart of the per-token expert matvec, for prefill tiles and
-// batched decode.  One pass over the weights serves up to 512 tokens, as the reference's tile path
-// does on the CPU for 16 (src/bin/engine_gpt2.rs:1005-1010, TILE = 16), and every output equals the
-// per-token result bit for bit.
+// Matrices x token rows on the 5th-generation tensor cores (tcgen05.mma, accumulators in tensor memory): the
+// MXFP4 experts and the Q8 projections of prompt tiles and batched decode.  One pass over the weights serves up to
+// 512 token rows, as the reference's tile path does on the CPU for 16 (src/bin/engine_gpt2.rs:1005-1010, TILE = 16),
+// and every output equals the per-token result bit for bit.
 //
-// Arithmetic.  A row's value is four lane chains, each fma(float(t_lane(b)), 2^(e_b-128) * xs[b], acc)
-// over the 32-blocks b, with t_lane(b) the exact int32 sum of the lane's 8 products.  The integer
-// sums of 128 rows x NT tokens x 4 lanes of one block are one 128 x 4 NT x 32 int8 matrix product:
-//   A[row][k]           = the row's 32 codes decoded to signed bytes (k = 8*lane + i),
-//   B[token*4+lane][k]  = the token's activation byte k if k belongs to `lane`, else 0,
-// issued twice, once with the positive and once with the negative decode table (their sum is the
-// signed value), accumulating in the same 128 x 4 NT int32 tile of tensor memory.  The four worker
-// warps read their 32 lanes of tensor memory (tcgen05.ld) and run the float chains, one thread per
-// row with 4 NT accumulators.  NT = 4 entries per CTA for tiles of up to 16 tokens, 8 up to 64, 16 beyond.
+// Arithmetic.  A row's value is a set of float chains over the 32-blocks b, one step per block:
+//   MXFP4: four lane chains,              acc_j    = fma(t_j(b), 2^(e_b-128) * xs[b], acc_j)
+//   Q8:    2 block parities x four lanes, acc_{p,j} = fma(t_j(b), ws[b] * xs[b], acc_{p,j}),  p = b & 1
+// with t_j(b) the exact integer dot of the lane's 8 weights with its 8 activation bytes.  The tensor core supplies
+// t_j(b) as exact floats, so no thread converts an integer:
+//   MXFP4  kind::f8f6f4, A = the raw e2m1 codes (4 bits in the low half of 16-byte containers), B = the two e4m3 planes
+//          of the activation (brrr_tile.cuh).  One product per lane chain j and block pair: its K = 32 is the 16 codes of
+//          lane j (8 of either block) twice - the descriptor's K stride is zero, so both 16-byte columns of operand A
+//          are the same bytes - against plane 0 and plane 1.  |t| <= 12192: 14 bits, exact in the f32 accumulator.
+//   Q8     kind::f16, A = the int8 weights as halves (re-laid at load), B = the activation bytes as halves; K = 16 is the
+//          8 weights of lane j in either block.  |t| <= 129032: exact.
+// Column n of product j is (token, block q): row n of B is zero outside block q, so one product gives both blocks' dots
+// of 128 rows x NT tokens.  The worker threads (thread = matrix row and 8 tokens) read them from tensor memory
+// (tcgen05.ld) and run the chains, two tokens per instruction (fma.rn.f32x2: two independent round-to-nearest operations).
 //
-// Operands are written to shared memory by the threads themselves in the canonical K-major
-// no-swizzle layout (8-row x 16-byte core matrices).
-#include <cstdlib>
+// What bounds it: the workers' instruction stream.  The chains - per row, token and block four fused multiply-adds that nothing may
+// reorder - take about 2.8 cycles per packed instruction (three 64-bit operands from the register file), 490 cycles per pair of
+// 128 rows x 32 tokens and scheduler; with reads, scales and barriers a pair takes 900.  Beside it run the products (four of 50 to
+// 60 cycles) and the copies.  Measured on 512 rows of the 20b shape (ncu, one launch): gate | up 671 us and down 313 us (before,
+// with int8 operands decoded by the workers and one conversion per dot: 2 x 835 and 835), q/k/v 160 and o-proj 142 us (integer
+// units: 520 and 480).
+//
+// Roles of a CTA (128 matrix rows x up to NT tokens).  Worker warps: NT / 8 groups of four.  Then two producer
+// warps (asynchronous copies of the pairs' operands into a ring) and two issuing warps (four products per pair, even
+// pairs into the one accumulator buffer, odd pairs into the other).  Barriers (all waits bounded): full[slot] the pair's
+// operands have landed; empty[slot] the products have read them; dfull[buf] the pair's products are complete; dempty[buf]
+// every live worker warp has read them; scbar the rows' scales of all pairs have landed.
+#include <cuda.h>
 #include "brrr_kernels.h"
 #include "brrr_block.cuh"
 #include "brrr_tma.cuh"
 #include "brrr_mx.cuh"
+#include "brrr_tile.cuh"
 
 namespace brrr {
 
 namespace {
 
-constexpr int TL_ROWS = 128;           // rows per CTA = MMA M
-
+constexpr int TL_ROWS = 128;             // rows per CTA = MMA M
 constexpr int TL_MAXTOK = BRRR_TILE_MAX; // entries per expert and launch (one per token of the tile at most)
-constexpr int TL_A_BYTES = TL_ROWS * 32;       // one decoded A tile (128 rows x 32 k bytes)
 
-constexpr int TL_THREADS = 224;        // four worker warps, the producer warp, two issuer warps (q8_tile_kernel)
-// mx_tile_kernel: one or two issuing threads, ring depth and CTAs per SM.  Measured on the 2048-token prefill (tok/s): 2 issuers /
-// depth 5 / 3 CTAs 3956; 1 issuer 3973; depth 3 3969; 1 issuer + depth 3 + 4 CTAs per SM (80 registers, spills) 3648.
-constexpr int MT_ISSUERS = 2;
-constexpr int MT_CTAS = 3;
-constexpr int MT_NT16_FROM = 65;         // tile size from which a CTA takes 16 entries (128 registers, 2 CTAs per SM: one decode of the weights serves
-                                         // twice the entries; 256-row prefill 5864 against 5469 tok/s); BRRR_TILE_NT16_FROM=n moves it
-constexpr int MT_THREADS = 160 + 32 * MT_ISSUERS;   // four worker warps, the producer warp, the issuer warp(s)
-constexpr int TL_DEPTH = 5;            // weight ring: block pairs in flight per CTA
-constexpr int TL_SLOT = 9 * MX_UNIT;   // one pair of a 128-row tile: up to 9 units of 16 rows
-constexpr int TL_CPL = (TL_SLOT / 16 + 31) / 32;   // 16-byte pieces per producer lane and pair
+constexpr int QOP_UNIT = 16384 + 1024;    // bytes of a Q8 operand tile per block pair (launch_q8_operand_pack)
 
-// shared-memory matrix descriptor: K-major, no swizzle; core matrix = 8 rows x 16 bytes, 128 bytes
-// apart along M/N (stride byte offset), `lbo` bytes apart along K (leading byte offset)
-__device__ __forceinline__ uint64_t tl_smem_desc(const void *p, uint32_t lbo) {
+enum { TK_MX = 0, TK_GLU = 1, TK_Q8 = 2 };      // one MXFP4 matrix; gate | up with the SwiGLU and the Q8 of h; a Q8 matrix
+
+// shared-memory matrix descriptor: K-major, no swizzle; core matrix = 8 rows x 16 bytes, `sbo` bytes apart along M/N (stride byte
+// offset), `lbo` bytes apart along K (leading byte offset)
+__device__ __forceinline__ uint64_t tl_smem_desc(const void *p, uint32_t lbo, uint32_t sbo) {
     uint64_t d = 0;
     d |= (uint64_t)((smem_u32(p) >> 4) & 0x3FFF);
     d |= (uint64_t)((lbo >> 4) & 0x3FFF) << 16;
-    d |= (uint64_t)((128u >> 4) & 0x3FFF) << 32;
+    d |= (uint64_t)((sbo >> 4) & 0x3FFF) << 32;
     d |= (uint64_t)1 << 46;                      // descriptor version of this architecture
     return d;
 }
-
-// kind::i8 product; instruction descriptor: D = s32, A = B = signed 8-bit, both K-major, N / 8 at bit 17, M / 16 at bit 24
-__device__ __forceinline__ void tl_mma(uint32_t tmem_d, uint64_t desc_a, uint64_t desc_b, uint32_t accumulate, uint32_t idesc) {
-    asm volatile(
-        "{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %4, 0;\n\t"
-        "tcgen05.mma.cta_group::1.kind::i8 [%0], %1, %2, %3, {%5, %5, %5, %5}, p;\n\t}"
-        ::"r"(tmem_d), "l"(desc_a), "l"(desc_b), "r"(idesc), "r"(accumulate), "r"(0u)
-        : "memory");
+template <int KIND>
+__device__ __forceinline__ void tl_mma(uint32_t tmem_d, uint64_t desc_a, uint64_t desc_b, uint32_t idesc) {
+    if (KIND == TK_Q8)
+        asm volatile("{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %4, 0;\n\t"
+                     "tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, {%4, %4, %4, %4}, p;\n\t}" ::"r"(tmem_d), "l"(desc_a), "l"(desc_b), "r"(idesc), "r"(0u)
+                     : "memory");
+    else
+        asm volatile("{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %4, 0;\n\t"
+                     "tcgen05.mma.cta_group::1.kind::f8f6f4 [%0], %1, %2, %3, {%4, %4, %4, %4}, p;\n\t}" ::"r"(tmem_d), "l"(desc_a), "l"(desc_b), "r"(idesc), "r"(0u)
+                     : "memory");
 }
 __device__ __forceinline__ void tl_commit(uint64_t *bar) {
     asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(smem_u32(bar)) : "memory");
@@ -68,281 +75,459 @@ __device__ __forceinline__ void tl_commit(uint64_t *bar) {
 __device__ __forceinline__ void tl_fence_before() { asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory"); }
 __device__ __forceinline__ void tl_fence_after() { asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory"); }
 
-// 16 consecutive 32-bit columns of this warp's 32 lanes of tensor memory
-__device__ __forceinline__ void tl_ld16(uint32_t taddr, int (&r)[16]) {
-    asm volatile("tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15}, [%16];"
-                 : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]), "=r"(r[8]), "=r"(r[9]),
-                   "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15])
-                 : "r"(taddr)
+// packed pairs of floats
+typedef unsigned long long f32x2;
+// Two runs of consecutive columns (32-bit floats) of this warp's 32 lanes of tensor memory as pairs, one wait.  Loads, wait and
+// packing are one statement, so nothing can use a register before the wait.
+__device__ __forceinline__ void tl_ld16x2(uint32_t ta, uint32_t tb, f32x2 (&v)[8], f32x2 (&w)[8]) {
+    asm volatile("{\n\t.reg .b32 r<16>;\n\t.reg .b32 s<16>;\n\t"
+                 "tcgen05.ld.sync.aligned.32x32b.x16.b32 {r0,r1,r2,r3,r4,r5,r6,r7,r8,r9,r10,r11,r12,r13,r14,r15}, [%16];\n\t"
+                 "tcgen05.ld.sync.aligned.32x32b.x16.b32 {s0,s1,s2,s3,s4,s5,s6,s7,s8,s9,s10,s11,s12,s13,s14,s15}, [%17];\n\t"
+                 "tcgen05.wait::ld.sync.aligned;\n\t"
+                 "mov.b64 %0, {r0,r1};\n\tmov.b64 %1, {r2,r3};\n\tmov.b64 %2, {r4,r5};\n\tmov.b64 %3, {r6,r7};\n\t"
+                 "mov.b64 %4, {r8,r9};\n\tmov.b64 %5, {r10,r11};\n\tmov.b64 %6, {r12,r13};\n\tmov.b64 %7, {r14,r15};\n\t"
+                 "mov.b64 %8, {s0,s1};\n\tmov.b64 %9, {s2,s3};\n\tmov.b64 %10, {s4,s5};\n\tmov.b64 %11, {s6,s7};\n\t"
+                 "mov.b64 %12, {s8,s9};\n\tmov.b64 %13, {s10,s11};\n\tmov.b64 %14, {s12,s13};\n\tmov.b64 %15, {s14,s15};\n\t"
+                 "}"
+                 : "=l"(v[0]), "=l"(v[1]), "=l"(v[2]), "=l"(v[3]), "=l"(v[4]), "=l"(v[5]), "=l"(v[6]), "=l"(v[7]), "=l"(w[0]), "=l"(w[1]), "=l"(w[2]), "=l"(w[3]), "=l"(w[4]), "=l"(w[5]), "=l"(w[6]), "=l"(w[7])
+                 : "r"(ta), "r"(tb)
                  : "memory");
 }
-// packed pairs of floats for fma.rn.f32x2
-__device__ __forceinline__ unsigned long long tl_pack2(float lo, float hi) {
-    unsigned long long r;
-    asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "r"(__float_as_uint(lo)), "r"(__float_as_uint(hi)));
+__device__ __forceinline__ void tl_ld8x2(uint32_t ta, uint32_t tb, f32x2 (&v)[4], f32x2 (&w)[4]) {
+    asm volatile("{\n\t.reg .b32 r<8>;\n\t.reg .b32 s<8>;\n\t"
+                 "tcgen05.ld.sync.aligned.32x32b.x8.b32 {r0,r1,r2,r3,r4,r5,r6,r7}, [%8];\n\t"
+                 "tcgen05.ld.sync.aligned.32x32b.x8.b32 {s0,s1,s2,s3,s4,s5,s6,s7}, [%9];\n\t"
+                 "tcgen05.wait::ld.sync.aligned;\n\t"
+                 "mov.b64 %0, {r0,r1};\n\tmov.b64 %1, {r2,r3};\n\tmov.b64 %2, {r4,r5};\n\tmov.b64 %3, {r6,r7};\n\t"
+                 "mov.b64 %4, {s0,s1};\n\tmov.b64 %5, {s2,s3};\n\tmov.b64 %6, {s4,s5};\n\tmov.b64 %7, {s6,s7};\n\t"
+                 "}"
+                 : "=l"(v[0]), "=l"(v[1]), "=l"(v[2]), "=l"(v[3]), "=l"(w[0]), "=l"(w[1]), "=l"(w[2]), "=l"(w[3])
+                 : "r"(ta), "r"(tb)
+                 : "memory");
+}
+__device__ __forceinline__ f32x2 tl_pack2(uint32_t lo, uint32_t hi) {
+    f32x2 r;
+    asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "r"(lo), "r"(hi));
     return r;
 }
-__device__ __forceinline__ void tl_unpack2(unsigned long long v, float &lo, float &hi) {
+__device__ __forceinline__ void tl_unpack2(f32x2 v, float &lo, float &hi) {
     uint32_t a, b;
     asm("mov.b64 {%0, %1}, %2;" : "=r"(a), "=r"(b) : "l"(v));
     lo = __uint_as_float(a); hi = __uint_as_float(b);
 }
-__device__ __forceinline__ unsigned long long tl_fma2(unsigned long long a, unsigned long long b, unsigned long long c) {
-    unsigned long long r;
+__device__ __forceinline__ f32x2 tl_fma2(f32x2 a, f32x2 b, f32x2 c) {
+    f32x2 r;
     asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c));
     return r;
 }
-__device__ __forceinline__ void tl_wait_ld() { asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory"); }
+__device__ __forceinline__ f32x2 tl_mul2(f32x2 a, f32x2 b) {
+    f32x2 r;
+    asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+    return r;
+}
+// shared-memory loads by 32-bit address, in program order
+__device__ __forceinline__ uint2 lds64(uint32_t addr) {
+    uint2 r;
+    asm volatile("ld.shared.v2.u32 {%0, %1}, [%2];" : "=r"(r.x), "=r"(r.y) : "r"(addr));
+    return r;
+}
+__device__ __forceinline__ void lds_pairs(uint32_t addr, f32x2 &a, f32x2 &b) { asm volatile("ld.shared.v2.u64 {%0, %1}, [%2];" : "=l"(a), "=l"(b) : "r"(addr)); }
+// box of a 4-d tensor map at (0, 0, c2, c3) -> shared memory
+__device__ __forceinline__ void tensor_g2s(uint32_t dst, const CUtensorMap *map, int c2, int c3, uint64_t *bar) {
+    asm volatile("cp.async.bulk.tensor.4d.shared::cluster.global.tile.mbarrier::complete_tx::bytes [%0], [%1, {%2, %2, %3, %4}], [%5];" ::"r"(dst), "l"(map),
+                 "r"(0), "r"(c2), "r"(c3), "r"(smem_u32(bar))
+                 : "memory");
+}
+__device__ __forceinline__ void cp_async16(uint32_t dst, const void *src) { asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(dst), "l"(src) : "memory"); }
+__device__ __forceinline__ void cp_async_arrive(uint64_t *bar) {
+    asm volatile("cp.async.mbarrier.arrive.noinc.shared::cta.b64 [%0];" ::"r"(smem_u32(bar)) : "memory");
+}
 
-// One launch serves blockIdx.y = (expert or the single matrix, chunk of entries).  Each expert has a list of up to 512
-// entries; entry i multiplies the activation row entry / src_div and writes output row entry.
-struct TileArgs {
-    MxDev w;
-    int row0, nrows;         // rows [row0, row0 + nrows) of each expert's matrix
+// Waits of the pipeline loops: a probe that suspends in hardware, a bounded number of times (far above any copy or product, well
+// under a second); when it runs out the error word is set and this thread does not wait again.  No call and no clock: a function
+// call in the loop would force every accumulator through the calling convention's registers (80 moves per pair and warp).
+constexpr int TL_WAIT_TRIES = 1 << 17;
+struct TlWaiter {
+    uint32_t *err;
+    bool dead;
+    __device__ __forceinline__ void operator()(uint64_t *bar, uint32_t parity) {
+        if (dead || mbar_test_wait(bar, parity)) return;
+        for (int i = 0; !mbar_try_wait_hint(bar, parity, 20000u);)
+            if (++i == TL_WAIT_TRIES) {
+                dead = true;
+                if (err) atomicCAS(err, (uint32_t)DEV_ERR_NONE, (uint32_t)DEV_ERR_COPY_TIMEOUT);
+                break;
+            }
+    }
+};
+
+// One launch serves blockIdx.y = task = (expert or the single matrix, chunk of its entries).  Each expert has a list of up
+// to 512 entries; entry i multiplies the activation row i / src_div and writes output row i.
+struct alignas(64) TileArgs {
+    CUtensorMap ma, mb;      // MX, GLU: the 16-row units as tensors (mx_tensor_map; GLU: gate and up)
+    const uint8_t *wa, *wb;  // MX, GLU: the same units (their exponents); Q8: operand tiles (launch_q8_operand_pack)
+    int np;                  // block pairs per row
+    int row0, nrows;         // rows [row0, row0 + nrows) of each expert's matrix (GLU: nrows of gate and of up)
     int rows_per_expert;     // matrix row of (expert e, row r) = e * rows_per_expert + r
-    const int *cnt;          // [experts] entries per expert; nullptr: one matrix, entries 0 .. ntok - 1
-    const int *list;         // [experts][TL_MAXTOK]
-    int src_div;
-    const int8_t *xq;        // [activation rows][blocks * 32]
-    const float *xs;         // [activation rows][blocks]
-    int ntok;
-    int chunks;              // CTAs per expert along blockIdx.y: ceil(most entries an expert can have / entries per CTA)
-    const float *bias;       // nullable: [experts][rows_per_expert], added to every output
-    float *y;                // element [entry][col0 + row - row0], rows ldy apart
-    int ldy, col0;
+    const int *cnt;          // [ne] entries per expert; nullptr: one matrix, entries 0 .. ntok - 1
+    const int *list;         // [ne][TL_MAXTOK]
+    int ne, ntok, src_div;
+    const uint8_t *img;      // activation images [row][np * ti_pair]: planes (MX, GLU) or halves (Q8)
+    const float *xs;         // block scales [row][2 np]
+    const float *bias, *bias_b;  // nullable: [ne][rows_per_expert], added to every output (GLU: of gate and of up, required)
+    float *y;                // MX, Q8: element [entry][row - row0], rows ldy apart
+    int ldy, epi;            // Q8: Q8_EPI_*
+    uint8_t *himg;           // GLU: plane images of h [entry][nrows / 64 * 256] and its scales [entry][nrows / 32]
+    float *hs;
     DevState *state;
 };
 
-// One CTA = 128 rows of one expert against one chunk of up to NT of its entries (NT = 4, 8 or 16, MMA N = 4 NT; an
-// expert with more entries is served by several CTAs, which re-read its rows from L2).
-//
-// Roles.  A tcgen05.mma or a bulk copy costs its issuing thread on the order of a hundred cycles, so the
-// asynchronous work is spread: warp 4 is the producer (every lane copies 16-byte pieces of the pairs' weight
-// units into a ring TL_DEPTH pairs deep),
-// one thread each of warps 5 and 6 issues the two products of one block of every pair as soon as the
-// workers have staged the operands.  Warps 0-3 are the workers, one
-// thread per row: stage(q) decodes the row's 64 codes of pair q from the ring into half (q & 1) of the
-// operand tiles, chains(p) reads the pair's accumulators from tensor memory and runs the float chains.
-// A worker runs stage(p + 1) before chains(p), so the tensor core works on pair p + 1 meanwhile.
-//
-// Barriers (all waits bounded).  full[slot], 32 arrivals: the producer lanes' copies of the pair have landed;
-// empty[slot], 128 arrivals: the workers have read it.  staged[half], 128 arrivals: the
-// half's operands are written and, because a worker stages pair p + 2 only after chains(p), the half's
-// accumulators have been read.  done[half], 2 arrivals: the issuers' tcgen05.commit of the pair; workers wait for it before they read
-// the accumulators and before they overwrite the half's operands two pairs later.
-template <int NT>
-__global__ void __launch_bounds__(MT_THREADS, NT == 16 ? 2 : MT_CTAS) mx_tile_kernel(TileArgs a) {
-    constexpr int N = 4 * NT;                                    // columns per block: NT tokens x 4 chain lanes
-    constexpr uint32_t TMEM_COLS = 4 * N;                        // two halves x two blocks x N columns (64 or 128)
-    constexpr uint32_t IDESC = (2u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(N >> 3) << 17) | ((TL_ROWS >> 4) << 24);
+// A ring slot holds a pair's operands; the rows' scales stay in a region of their own for the whole kernel, so a worker waits for the
+// products only.  Scales per row and pair: 2 e8m0 bytes, Q8: 2 floats.
+template <int KIND> __host__ __device__ constexpr int tl_a_bytes() { return KIND == TK_Q8 ? 16384 : 8192; }       // four operands of 4 or 2 KB
+template <int KIND> __host__ __device__ constexpr int tl_sc_bytes() { return KIND == TK_Q8 ? 1024 : 256; }        // per pair
+template <int KIND, int NT> __host__ __device__ constexpr bool tl_scale_table() { return KIND != TK_Q8 && NT == 32; }      // e8m0 bytes expanded to floats once
+template <int KIND, int NT> __host__ __device__ constexpr int tl_slot_bytes() { return tl_a_bytes<KIND>() + NT * 256; }
+// Even: each issuing warp then has slots of its own.  (With an odd depth both use every slot, and a warp could take the other one's
+// phase of full[] for its own: a parity wait returns as well while the phase before last is the last complete one.)
+template <int KIND, int NT> __host__ __device__ constexpr int tl_depth() { return KIND == TK_Q8 || NT == 8 ? 4 : 6; }
+template <int KIND, int NT>
+size_t tl_smem(int np) {
+    return (size_t)tl_depth<KIND, NT>() * tl_slot_bytes<KIND, NT>() + (size_t)np * tl_sc_bytes<KIND>() + (tl_scale_table<KIND, NT>() ? (size_t)np * 1024 : 0) +
+           (size_t)np * 2 * NT * 4 + (KIND == TK_GLU ? NT * 128 * 4 : 0);
+}
+
+template <int KIND, int NT>
+__global__ void __launch_bounds__(NT * 16 + 128, KIND == TK_Q8 || NT == 32 ? 1 : NT == 16 ? 2 : 3) tile_kernel(const __grid_constant__ TileArgs a) {
+    constexpr int WORKERS = NT * 16, THREADS = WORKERS + 128;
+    constexpr int TL_DEPTH = tl_depth<KIND, NT>(), SLOT = tl_slot_bytes<KIND, NT>(), A_BYTES = tl_a_bytes<KIND>(), B_OFF = A_BYTES, SC = tl_sc_bytes<KIND>();
+    // operand A of product j at j * A_STEP; MX: core matrix (8 rows, chain j) at (row / 8) * 512 + j * 128, both K columns the same
+    constexpr uint32_t A_STEP = KIND == TK_Q8 ? 4096 : 128, A_LBO = KIND == TK_Q8 ? 2048 : 0, A_SBO = KIND == TK_Q8 ? 128 : 512;
+    constexpr int PAIR = ti_pair(KIND == TK_Q8 ? TI_HALF : TI_PLANES);
+    constexpr uint32_t B_LBO = NT * 32, B_STEP = NT * 64;        // operand B of product j at j * B_STEP: [K column][group of eight tokens][block][8 rows x 16 bytes]
+    constexpr uint32_t BUF_COLS = 8 * NT;                                             // accumulator columns of one pair
+    constexpr uint32_t TMEM_COLS = 2 * BUF_COLS;
+    static_assert(TL_DEPTH % 2 == 0, "each issuing warp has slots of its own");
+    constexpr bool TABLE = tl_scale_table<KIND, NT>();
+    constexpr int CH = KIND == TK_Q8 ? 8 : 4;                                         // chains per row and token
     extern __shared__ __align__(128) unsigned char tsm[];
-    const int nb = a.w.blocks, np = nb / 2;
-    unsigned char (*a_tiles)[TL_A_BYTES] = reinterpret_cast<unsigned char (*)[TL_A_BYTES]>(tsm);           // [half][block of the pair][P, N]
-    unsigned char (*b_tiles)[N * 32] = reinterpret_cast<unsigned char (*)[N * 32]>(tsm + 8 * TL_A_BYTES);  // [half][block of the pair]
-    unsigned char *ring = tsm + 8 * TL_A_BYTES + 4 * N * 32;                                               // [TL_DEPTH][8 units]
-    float *xs_sm = reinterpret_cast<float *>(ring + TL_DEPTH * TL_SLOT);                                   // [NT][nb] activation block scales
+    const int np = a.np;
+    unsigned char *ring = tsm;
+    unsigned char *sc_sm = tsm + TL_DEPTH * SLOT;                                     // [pair][SC]
+    float2 *sc2_sm = reinterpret_cast<float2 *>(sc_sm + (size_t)np * SC);             // scale table: [pair][128 rows]
+    float *xs_sm = reinterpret_cast<float *>(sc2_sm + (TABLE ? (size_t)np * 128 : 0)); // [pair][block of the pair][NT]
+    float *glu_sm = xs_sm + (size_t)np * 2 * NT;                                      // GLU: [NT][128 rows]
     __shared__ float tbl[256];
-    __shared__ __align__(8) uint64_t full[TL_DEPTH], empty[TL_DEPTH], staged[2], done[2];
+    __shared__ __align__(8) uint64_t full[TL_DEPTH], empty[TL_DEPTH], dfull[2], dempty[2], scbar;
     __shared__ uint32_t tmem_base_sh;
+    __shared__ int task_sh[3];               // expert, first entry, entries
     __shared__ int ent[NT];
-    const int tid = threadIdx.x, warp = tid >> 5;
-    const int e = blockIdx.y / a.chunks, chunk = blockIdx.y % a.chunks;
-    const int n_ent = min((a.cnt ? a.cnt[e] : a.ntok) - chunk * NT, NT);
-    if (n_ent <= 0) return;                      // nothing routed here (before anything is allocated)
-    if (tid < NT) ent[tid] = tid < n_ent ? (a.list ? a.list[e * TL_MAXTOK + chunk * NT + tid] : chunk * NT + tid) : 0;
-    mx_fill_scale_table(tbl, tid, MT_THREADS);
-    for (int i = tid; i < 4 * N * 32 / 16; i += MT_THREADS) reinterpret_cast<uint4 *>(&b_tiles[0][0])[i] = make_uint4(0, 0, 0, 0);   // rows of absent tokens stay zero
-    if (tid == 0) {
-        for (int i = 0; i < TL_DEPTH; i++) { mbar_init(&full[i], 32); mbar_init(&empty[i], 128); }
-        mbar_init(&staged[0], 128); mbar_init(&staged[1], 128);
-        mbar_init(&done[0], MT_ISSUERS); mbar_init(&done[1], MT_ISSUERS);
+    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+    // ---- what needs nothing from the kernels before
+    if (KIND != TK_Q8) mx_fill_scale_table(tbl, tid, THREADS);
+    else {
+        // zero rows of operand B (a plane image brings its zeros along); rows of absent tokens only reach columns nobody stores
+        constexpr int Z = (SLOT - B_OFF) / 16;
+        for (int i = tid; i < TL_DEPTH * Z; i += THREADS) *reinterpret_cast<uint4 *>(ring + (i / Z) * SLOT + B_OFF + (i % Z) * 16) = make_uint4(0, 0, 0, 0);
+        fence_proxy_async();                 // these stores -> the tensor core's reads
+    }
+    pdl_wait();
+    pdl_trigger();
+    if (warp == 0) {
+        // task -> (expert, chunk): experts in order, ceil(entries / NT) chunks each
+        const int per = a.cnt ? (a.ne + 31) / 32 : 1, e0 = lane * per;
+        int c[8], mine = 0;
+#pragma unroll
+        for (int i = 0; i < 8; i++) {
+            c[i] = 0;
+            if (i < per) c[i] = a.cnt ? (e0 + i < a.ne ? a.cnt[e0 + i] : 0) : (lane == 0 ? a.ntok : 0);
+            mine += (c[i] + NT - 1) / NT;
+        }
+        int incl = mine;
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) { const int v = __shfl_up_sync(0xffffffffu, incl, o); if (lane >= o) incl += v; }
+        if (lane == 0) task_sh[2] = 0;
+        __syncwarp();
+        int t = (int)blockIdx.y - (incl - mine);
+        if (t >= 0 && t < mine) {
+#pragma unroll
+            for (int i = 0; i < 8; i++) {
+                const int n = (c[i] + NT - 1) / NT;
+                if (t >= 0 && t < n) {
+                    const int step = ((c[i] + n - 1) / n + 7) & ~7;         // equal chunks, whole groups of eight
+                    task_sh[0] = e0 + i; task_sh[1] = t * step; task_sh[2] = min(step, c[i] - t * step);
+                    t = -1;
+                } else if (t >= 0) t -= n;
+            }
+        }
+    }
+    __syncthreads();
+    const int e = task_sh[0], first = task_sh[1], n_ent = task_sh[2];
+    if (n_ent <= 0) return;                  // nothing here (before anything is allocated)
+    const int groups = (n_ent + 7) >> 3;     // live groups of eight tokens
+    const int live_warps = 4 * groups;
+    if (tid == WORKERS) {
+        for (int i = 0; i < TL_DEPTH; i++) { mbar_init(&full[i], 65); mbar_init(&empty[i], 1); }
+        mbar_init(&scbar, KIND == TK_Q8 ? 1 : 32);
+        for (int i = 0; i < 2; i++) { mbar_init(&dfull[i], 1); mbar_init(&dempty[i], live_warps); }
         mbar_fence_init();
     }
     if (warp == 0) {
         asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(&tmem_base_sh)), "r"(TMEM_COLS) : "memory");
         asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
     }
+    if (tid < NT) ent[tid] = tid < n_ent ? (a.list ? a.list[e * TL_MAXTOK + first + tid] : first + tid) : 0;
     tl_fence_before();
     __syncthreads();
     tl_fence_after();
     const uint32_t tmem_base = tmem_base_sh;
-    uint32_t *err = a.state ? &a.state->err : nullptr;
-    Waiter waiter(err);
-    // the tile's live rows lie in up to nine units of 16 rows (a row window may start anywhere); only those are copied
-    const int row_base = e * a.rows_per_expert + a.row0 + blockIdx.x * TL_ROWS;
-    const int live_rows = min(TL_ROWS, a.nrows - (int)blockIdx.x * TL_ROWS);
-    const int n_units = ((row_base & 15) + live_rows + 15) >> 4;
+    TlWaiter wait{a.state ? &a.state->err : nullptr, a.state && *reinterpret_cast<volatile uint32_t *>(&a.state->err) != 0u};
+    const int tile = blockIdx.x;
+    // MX, GLU: a tile starts on a 16-row unit; a row window that does not starts in the middle of its first tile
+    const int row0 = e * a.rows_per_expert + a.row0, unit0 = (row0 >> 4) + tile * (KIND == TK_GLU ? 4 : 8);
+    const int shift = KIND == TK_MX ? row0 & 15 : 0;
+    const int n_units = KIND == TK_GLU ? 8 : min(8, (shift + a.nrows - tile * TL_ROWS + 15) >> 4);
 
-    if (warp == 4) {
-        // ---------------- producer: 16-byte asynchronous copies, one arrival per lane on the slot's barrier
-        const int lane = tid & 31;
-        const int n_chunks = n_units * (MX_UNIT / 16);
-        const unsigned char *wbase = a.w.data + mx_unit_off(row_base >> 4, 0, np);
-        uint32_t src_off[TL_CPL], dst_off[TL_CPL];          // this lane's chunks of a pair: unit g, 16-byte piece o
-#pragma unroll
-        for (int i = 0; i < TL_CPL; i++) {
-            const int c = lane + 32 * i, g = c / (MX_UNIT / 16), o = (c - g * (MX_UNIT / 16)) * 16;
-            src_off[i] = (uint32_t)g * (uint32_t)np * MX_UNIT + o;
-            dst_off[i] = (uint32_t)(g * MX_UNIT + o);
+    if (warp < WORKERS / 32 + 2 && warp >= WORKERS / 32) {
+        // ---------------- producers: two warps share the tokens' activations; lane 0 of the first also issues the weights' copies
+        const bool weights = warp == WORKERS / 32;
+        if (weights) {
+            if (KIND == TK_Q8) {
+                if (lane == 0) {
+                    mbar_expect_tx(&scbar, (uint32_t)np * SC);
+                    bulk_g2s(sc_sm, a.wa + (size_t)tile * np * QOP_UNIT + (size_t)np * A_BYTES, (uint32_t)np * SC, &scbar);
+                }
+            } else {
+                for (int i = lane; i < n_units * 2 * np; i += 32) {      // exponents of every pair
+                    const int p = i / (n_units * 2), k = i % (n_units * 2), u = k >> 1;
+                    const uint8_t *unit = KIND == TK_GLU && u >= 4 ? a.wb + mx_unit_off(unit0 + u - 4, p, np) : a.wa + mx_unit_off(unit0 + u, p, np);
+                    cp_async16(smem_u32(sc_sm) + p * SC + k * 16, unit + MX_UNIT_EXPS + (k & 1) * 16);
+                }
+                cp_async_arrive(&scbar);
+            }
         }
-        auto load = [&](int q, int slot) {
-            const unsigned char *src = wbase + (size_t)q * MX_UNIT;
-            unsigned char *dst = ring + slot * TL_SLOT;
+        // activations: lane = (token of a group of eight, quarter of its 16-byte pieces): planes: (chain jj, plane r >> 1, block r & 1);
+        // halves: (chain 2 i + (r >> 1), block r & 1)
+        constexpr int NG = NT / 8, MINE = (NG + 1) / 2;        // groups of eight tokens, at most MINE of them per producer warp
+        const uint8_t *src[MINE];
+        bool live[MINE];
+        const int r = lane & 3;
 #pragma unroll
-            for (int i = 0; i < TL_CPL; i++)
-                if (lane + 32 * i < n_chunks)
-                    asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(smem_u32(dst + dst_off[i])), "l"(src + src_off[i]) : "memory");
-            asm volatile("cp.async.mbarrier.arrive.noinc.shared::cta.b64 [%0];" ::"r"(smem_u32(&full[slot])) : "memory");
-        };
-        const int pre = min(TL_DEPTH, np);
-        for (int q = 0; q < pre; q++) load(q, q);
+        for (int k = 0; k < MINE; k++) {
+            const int g = weights ? k : MINE + k, t = g * 8 + (lane >> 2);
+            live[k] = g < NG && t < n_ent;
+            src[k] = a.img + (size_t)(ent[live[k] ? t : 0] / a.src_div) * np * PAIR + r * 16;
+        }
+        const uint32_t ring0 = smem_u32(ring);
+        const uint32_t dst0 = ring0 + B_OFF + (weights ? 0 : MINE * 256) + (lane >> 2) * 16 + (r & 1) * 128 +
+                              (KIND == TK_Q8 ? (r >> 1) * B_STEP + (r & 1) * B_LBO : (r >> 1) * B_LBO);
+        const uint8_t *wsrc = a.wa + (size_t)tile * np * QOP_UNIT;
         int slot = 0;
-        uint32_t par = 0;
-        for (int p = 0; p + TL_DEPTH < np; p++) {
-            waiter.wait_suspended(&empty[slot], par);                              // every worker has read pair p out of the slot
-            load(p + TL_DEPTH, slot);
+        uint32_t par = 1;
+        for (int p = 0; p < np; p++) {
+            wait(&empty[slot], par);
+            if (weights && lane == 0) {
+                // MX: a tensor copy (GLU: two) widens each 8-byte word of a row and chain into the 16-byte container of a 4-bit operand;
+                // the barrier counts the packed bytes, not the padding
+                mbar_expect_tx(&full[slot], KIND == TK_Q8 ? A_BYTES : A_BYTES / 2);
+                if (KIND == TK_Q8) bulk_g2s(ring + slot * SLOT, wsrc + (size_t)p * A_BYTES, A_BYTES, &full[slot]);
+                else tensor_g2s(ring0 + slot * SLOT, &a.ma, unit0, p, &full[slot]);
+                if (KIND == TK_GLU) tensor_g2s(ring0 + slot * SLOT + A_BYTES / 2, &a.mb, unit0, p, &full[slot]);
+            }
+            __syncwarp();
+            const uint32_t dst = dst0 + slot * SLOT;
+#pragma unroll
+            for (int k = 0; k < MINE; k++) {
+                if (live[k]) {
+                    if (KIND == TK_Q8) {
+#pragma unroll
+                        for (int i = 0; i < 2; i++) cp_async16(dst + k * 256 + i * 2 * B_STEP, src[k] + i * 64);
+                    } else {
+#pragma unroll
+                        for (int jj = 0; jj < 4; jj++) cp_async16(dst + k * 256 + jj * B_STEP, src[k] + jj * 64);
+                    }
+                }
+                src[k] += PAIR;
+            }
+            cp_async_arrive(&full[slot]);
             if (++slot == TL_DEPTH) { slot = 0; par ^= 1u; }
         }
         asm volatile("cp.async.wait_all;" ::: "memory");
-    } else if (tid == 160 || (MT_ISSUERS == 2 && tid == 192)) {
-        // ---------------- issuer(s): with two, block k of every pair each (two threads in two warps issue side by side); with one, both blocks
-        const int k0 = tid == 160 ? 0 : 1, k1 = MT_ISSUERS == 2 ? k0 + 1 : 2;
-        uint64_t da[2][4], db[2][2];
-#pragma unroll
-        for (int h = 0; h < 2; h++) {
-#pragma unroll
-            for (int i = 0; i < 4; i++) da[h][i] = tl_smem_desc(&a_tiles[4 * h + i][0], 2048);
-            db[h][0] = tl_smem_desc(&b_tiles[2 * h][0], N * 16);
-            db[h][1] = tl_smem_desc(&b_tiles[2 * h + 1][0], N * 16);
-        }
-        for (int p = 0; p < np; p++) {
-            const int h = p & 1;
-            waiter.wait_suspended(&staged[h], (uint32_t)(p >> 1) & 1u);
+    } else if (warp >= WORKERS / 32 + 2) {
+        // ---------------- issuers: one for the even pairs (buffer 0), one for the odd (the whole warp walks the loop, one elected lane issues)
+        // D = f32, both K-major; MX: A = e2m1 (5), B = e4m3 (0); Q8: A = B = f16 (0); N = 16 columns per group of eight tokens
+        const uint32_t idesc = (1u << 4) | (KIND == TK_Q8 ? 0u : (5u << 7)) | ((uint32_t)(2 * groups) << 17) | ((TL_ROWS >> 4) << 24);
+        const uint64_t da0 = tl_smem_desc(ring, A_LBO, A_SBO), db0 = tl_smem_desc(ring + B_OFF, B_LBO, 128);
+        const int buf = warp - (WORKERS / 32 + 2);
+        int slot = buf;
+        uint32_t fpar = 0, dpar = 1;
+        for (int p = buf; p < np; p += 2) {
+            wait(&full[slot], fpar);
+            fence_proxy_async();                   // the copies seen through full[] (generic proxy) -> the tensor core's reads
+            wait(&dempty[buf], dpar);
+            dpar ^= 1u;
             tl_fence_after();
+            const uint64_t da = da0 + (uint64_t)(slot * (SLOT / 16)), db = db0 + (uint64_t)(slot * (SLOT / 16));
+            const uint32_t d0 = tmem_base + buf * BUF_COLS;
+            if (elect_one()) {
 #pragma unroll
-            for (int k = 0; k < 2; k++)
-                if (k >= k0 && k < k1) {
-                    const uint32_t dcol = tmem_base + (uint32_t)((2 * h + k) * N);
-                    if (h == 0) { tl_mma(dcol, da[0][2 * k], db[0][k], 0u, IDESC); tl_mma(dcol, da[0][2 * k + 1], db[0][k], 1u, IDESC); }
-                    else        { tl_mma(dcol, da[1][2 * k], db[1][k], 0u, IDESC); tl_mma(dcol, da[1][2 * k + 1], db[1][k], 1u, IDESC); }
-                }
-            tl_commit(&done[h]);
+                for (int j = 0; j < 4; j++) tl_mma<KIND>(d0 + j * 2 * NT, da + j * (A_STEP / 16), db + j * (B_STEP / 16), idesc);
+                tl_commit(&dfull[buf]);
+                if (p + TL_DEPTH < np) tl_commit(&empty[slot]);      // nobody waits for the last ones
+            }
+            __syncwarp();
+            if ((slot += 2) >= TL_DEPTH) { slot -= TL_DEPTH; fpar ^= 1u; }
         }
-    } else if (tid < 128) {
-        // ---------------- workers
-        const uint32_t P_LO = 0x04030200u, P_HI = 0x0D090705u, N_LO = 0xFDFEFF00u, N_HI = 0xF4F8FAFCu;
-        const int row_local = blockIdx.x * TL_ROWS + tid;
-        const bool row_live = tid < live_rows;
-        // this row in a ring slot: its unit, there its 32 code bytes of the pair and its two exponent bytes
-        const int urow = (row_base & 15) + tid;
-        const unsigned char *my_unit = ring + (urow >> 4) * MX_UNIT;
-        const uint32_t w_off = (uint32_t)(urow & 15) * 32, e_off = MX_UNIT_EXPS + (uint32_t)(urow & 15) * 2;
-        // A element (row m, byte k) lives at (k / 16) * 2048 + (m / 8) * 128 + (m % 8) * 16 + k % 16
-        const uint32_t a_off = (uint32_t)((tid >> 3) * 128 + (tid & 7) * 16);
-        // B row n = token * 4 + lane holds the 8 activation bytes of `lane` at k = 8 * lane .. + 7; threads 0 .. N - 1 serve
-        // the first block of the pair, 64 .. 64 + N - 1 the second
-        const int n_row = tid & 63, bt = n_row >> 2, bl = tid & 3, bblk = tid >> 6;
-        const bool b_live = n_row < N && bt < n_ent;
-        const uint32_t b_off = (uint32_t)((bl >> 1) * (N * 16) + (n_row >> 3) * 128 + (n_row & 7) * 16 + (bl & 1) * 8);
-        // its activation words come straight from global memory (L2), one pair ahead
-        const int8_t *my_x = a.xq + (size_t)(ent[b_live ? bt : 0] / a.src_div) * nb * 32 + bblk * 32 + 4 * bl;
-        uint32_t xlo = 0, xhi = 0;
-        if (b_live) { xlo = *reinterpret_cast<const uint32_t *>(my_x); xhi = *reinterpret_cast<const uint32_t *>(my_x + 16); }
-        for (int i = tid; i < n_ent * nb; i += 128) xs_sm[i] = a.xs[(size_t)(ent[i / nb] / a.src_div) * nb + i % nb];
-        asm volatile("bar.sync 1, 128;" ::: "memory");             // the workers' own barrier: xs_sm is complete
-
-        int f_slot = 0;
-        uint32_t f_par = 0;
-        // operands of pair q -> half (q & 1) of the tiles; returns the row's two exponent bytes
-        auto stage = [&](int q) -> uint32_t {
-            const int h = q & 1;
-            waiter.wait_suspended(&full[f_slot], f_par);
-            const unsigned char *u = my_unit + f_slot * TL_SLOT;
-            const int q_slot = f_slot;
-            if (++f_slot == TL_DEPTH) { f_slot = 0; f_par ^= 1u; }
-            const uint4 w0 = *reinterpret_cast<const uint4 *>(u + w_off), w1 = *reinterpret_cast<const uint4 *>(u + w_off + 16);
-            const uint32_t e2 = *reinterpret_cast<const unsigned short *>(u + e_off);
-            mbar_arrive(&empty[q_slot]);
-            const uint32_t wl[4][2] = {{w0.x, w0.y}, {w0.z, w0.w}, {w1.x, w1.y}, {w1.z, w1.w}};
-            // lanes (0, 1) and (2, 3) of a row are neighbours in the tile: one 16-byte store per (K half, block, table); a warp's
-            // stores then cover 512 contiguous bytes (no bank conflict)
+    } else if (warp < live_warps) {
+        // ---------------- workers: thread = matrix row m, tokens 8 wg .. + 7
+        const int wg = warp >> 2, m = tid & 127;
+        const int t_base = wg * 8;
+        {
+            // block scales of this group's tokens, [pair][block][token] so that two neighbours are one operand; every load before the
+            // first store (a store in between would order the loads behind it, each a round trip to L2)
+            const int t = t_base + (m & 7), nb = np * 2;
+            const float *src = a.xs + (size_t)(ent[t < n_ent ? t : 0] / a.src_div) * nb;
+            float v[8];
 #pragma unroll
-            for (int jh = 0; jh < 2; jh++) {
+            for (int k = 0; k < 8; k++) v[k] = (m >> 3) + 16 * k < nb ? src[(m >> 3) + 16 * k] : 0.0f;
 #pragma unroll
-                for (int k = 0; k < 2; k++) {
-                    const uint32_t wa = wl[2 * jh][k], wb = wl[2 * jh + 1][k], wax = wa ^ 0x88888888u, wbx = wb ^ 0x88888888u;
-                    const uint32_t off = (uint32_t)(jh * 2048) + a_off;
-                    *reinterpret_cast<uint4 *>(&a_tiles[4 * h + 2 * k][off]) =
-                        make_uint4(brrr_prmt(P_LO, P_HI, wa), brrr_prmt(P_LO, P_HI, wa >> 16), brrr_prmt(P_LO, P_HI, wb), brrr_prmt(P_LO, P_HI, wb >> 16));
-                    *reinterpret_cast<uint4 *>(&a_tiles[4 * h + 2 * k + 1][off]) =
-                        make_uint4(brrr_prmt(N_LO, N_HI, wax), brrr_prmt(N_LO, N_HI, wax >> 16), brrr_prmt(N_LO, N_HI, wbx), brrr_prmt(N_LO, N_HI, wbx >> 16));
-                }
+            for (int k = 0; k < 8; k++) if ((m >> 3) + 16 * k < nb) xs_sm[((m >> 3) + 16 * k) * NT + t] = v[k];
+            for (int b = (m >> 3) + 128; b < nb; b += 16) xs_sm[b * NT + t] = src[b];
+        }
+        wait(&scbar, 0u);
+        if (TABLE) {
+            // this group's share of the pairs; then every live group has the whole table
+#pragma unroll 4
+            for (int p = wg; p < np; p += groups) {
+                const uint32_t e2 = *reinterpret_cast<const unsigned short *>(sc_sm + p * SC + m * 2);
+                sc2_sm[p * 128 + m] = make_float2(tbl[e2 & 0xFFu], tbl[e2 >> 8]);
             }
-            if (b_live) {
-                const int2 iv = mx_interleave(xlo, xhi);
-                *reinterpret_cast<uint2 *>(&b_tiles[2 * h + bblk][b_off]) = make_uint2((uint32_t)iv.x, (uint32_t)iv.y);
-                if (q + 1 < np) {
-                    xlo = *reinterpret_cast<const uint32_t *>(my_x + (size_t)(q + 1) * 64);
-                    xhi = *reinterpret_cast<const uint32_t *>(my_x + (size_t)(q + 1) * 64 + 16);
-                }
+        }
+        asm volatile("bar.sync 1, %0;" ::"r"(live_warps * 32) : "memory");
+        uint32_t sc_addr = TABLE ? smem_u32(sc2_sm + m) : smem_u32(sc_sm) + m * (KIND == TK_Q8 ? 8 : 2), xs_addr = smem_u32(xs_sm + t_base);
+        const uint32_t lane_addr = tmem_base + ((uint32_t)((warp & 3) * 32) << 16) + (uint32_t)(t_base * 2);
+        f32x2 acc[CH][4];
+#pragma unroll
+        for (int c = 0; c < CH; c++)
+#pragma unroll
+            for (int i = 0; i < 4; i++) acc[c][i] = 0ull;
+        uint32_t par = 0;                              // of dfull of the pair at hand
+        auto pair_step = [&](int buf) {
+            uint2 w;                                   // this row's scales of the pair's blocks
+            if (KIND == TK_Q8 || TABLE) w = lds64(sc_addr);
+            else {
+                uint32_t e2;
+                asm volatile("ld.shared.u16 %0, [%1];" : "=r"(e2) : "r"(sc_addr));
+                w = make_uint2(__float_as_uint(tbl[e2 & 0xFFu]), __float_as_uint(tbl[e2 >> 8]));
             }
-            fence_proxy_async();               // generic-proxy writes above -> visible to the tensor core's reads
-            tl_fence_before();                 // and this thread's reads of the half's accumulators are done
-            mbar_arrive(&staged[h]);
-            return e2;
-        };
-        // the chains of lanes (0, 1) and (2, 3) of an entry share an instruction (fma.rn.f32x2: two independent
-        // round-to-nearest fused multiply-adds)
-        unsigned long long acc2[N / 2];
+            sc_addr += TABLE ? 1024 : SC;
+            const f32x2 ww[2] = {tl_pack2(w.x, w.x), tl_pack2(w.y, w.y)};
+            const uint32_t addr = lane_addr + buf * BUF_COLS;
+            auto scales = [&](int q, f32x2 (&o)[4]) {  // of the eight tokens in block q: row scale x activation scale
+                lds_pairs(xs_addr + q * NT * 4, o[0], o[1]);
+                lds_pairs(xs_addr + q * NT * 4 + 16, o[2], o[3]);
 #pragma unroll
-        for (int i = 0; i < N / 2; i++) acc2[i] = 0ull;
-        const uint32_t lane_addr = tmem_base + ((uint32_t)(warp * 32) << 16);
-        // float chains of pair p: thread = row (tensor-memory lane), N columns per block
-        auto chains = [&](int p, uint32_t e2c) {
-            const int h = p & 1;
-            waiter.wait_suspended(&done[h], (uint32_t)(p >> 1) & 1u);
-            tl_fence_after();
+                for (int i = 0; i < 4; i++) o[i] = tl_mul2(ww[q], o[i]);
+            };
+            auto release = [&]() {                     // every column of the pair has been read
+                tl_fence_before();
+                __syncwarp();
+                if (lane == 0) mbar_arrive(&dempty[buf]);
+            };
+            if (KIND == TK_Q8) {                       // fewer registers beside 64 of chains: one block at a time
 #pragma unroll
-            for (int k = 0; k < 2; k++) {
-                const float esc = tbl[k ? e2c >> 8 : e2c & 0xFFu];
-                constexpr int G = N > 32 ? 32 : N;                // columns per tensor-memory read round (registers)
+                for (int q = 0; q < 2; q++) {
+                    f32x2 s2[4];
+                    scales(q, s2);
+                    if (q == 0) { wait(&dfull[buf], par); tl_fence_after(); }
 #pragma unroll
-                for (int c0 = 0; c0 < N; c0 += G) {
-                    int d[G / 16][16];
+                    for (int j = 0; j < 4; j += 2) {
+                        f32x2 v[4], u[4];
+                        tl_ld8x2(addr + j * 2 * NT + q * 8, addr + (j + 1) * 2 * NT + q * 8, v, u);
+                        if (j == 2 && q == 1) release();
 #pragma unroll
-                    for (int c = 0; c < G / 16; c++) tl_ld16(lane_addr + (uint32_t)((2 * h + k) * N + c0 + 16 * c), d[c]);
-                    tl_wait_ld();
-#pragma unroll
-                    for (int tt = 0; tt < G / 4; tt++) {
-                        const int t = c0 / 4 + tt;
-                        const float sxs = __fmul_rn(esc, xs_sm[t * nb + 2 * p + k]);
-                        const unsigned long long s2 = tl_pack2(sxs, sxs);
-#pragma unroll
-                        for (int l = 0; l < 2; l++)
-                            acc2[2 * t + l] = tl_fma2(tl_pack2((float)d[tt / 4][4 * (tt % 4) + 2 * l], (float)d[tt / 4][4 * (tt % 4) + 2 * l + 1]), s2, acc2[2 * t + l]);
+                        for (int i = 0; i < 4; i++) {
+                            f32x2 &c0 = acc[(q * 4 + j) % CH][i], &c1 = acc[(q * 4 + j + 1) % CH][i];
+                            c0 = tl_fma2(v[i], s2[i], c0);
+                            c1 = tl_fma2(u[i], s2[i], c1);
+                        }
                     }
                 }
-            }
-        };
-        uint32_t e2c = stage(0);
-        for (int p = 0; p < np; p++) {
-            uint32_t e2n = 0;
-            if (p + 1 < np) e2n = stage(p + 1);      // the tensor core runs pair p + 1 ...
-            chains(p, e2c);                          // ... beside the chains of pair p
-            e2c = e2n;
-        }
-        if (row_live) {
-            const float bias = a.bias ? a.bias[(size_t)e * a.rows_per_expert + a.row0 + row_local] : 0.0f;
+            } else {
+                f32x2 s2[2][4];
+                scales(0, s2[0]);
+                scales(1, s2[1]);
+                wait(&dfull[buf], par);
+                tl_fence_after();
 #pragma unroll
-            for (int t = 0; t < NT; t++)
-                if (t < n_ent) {
-                    float a0, a1, a2, a3;
-                    tl_unpack2(acc2[2 * t], a0, a1);
-                    tl_unpack2(acc2[2 * t + 1], a2, a3);
-                    float v = __fadd_rn(__fadd_rn(a0, a1), __fadd_rn(a2, a3));
-                    if (a.bias) v = __fadd_rn(v, bias);
-                    a.y[(size_t)ent[t] * a.ldy + a.col0 + row_local] = v;
+                for (int j = 0; j < 4; j += 2) {
+                    f32x2 v[8], u[8];
+                    tl_ld16x2(addr + j * 2 * NT, addr + (j + 1) * 2 * NT, v, u);
+                    if (j == 2) release();
+#pragma unroll
+                    for (int q = 0; q < 2; q++)
+#pragma unroll
+                        for (int i = 0; i < 4; i++) {
+                            acc[j][i] = tl_fma2(v[q * 4 + i], s2[q][i], acc[j][i]);
+                            acc[j + 1][i] = tl_fma2(u[q * 4 + i], s2[q][i], acc[j + 1][i]);
+                        }
                 }
+            }
+            xs_addr += 2 * NT * 4;
+        };
+#pragma unroll 1
+        for (int p = 0; p < np; p += 2) {
+            pair_step(0);
+            if (p + 1 < np) pair_step(1);
+            par ^= 1u;
+        }
+        // ---------------- outputs
+        const int row_local = KIND == TK_GLU ? tile * 64 + (m & 63) : tile * TL_ROWS + m - shift;
+        const bool row_live = row_local >= 0 && row_local < a.nrows;
+        const float *bp = KIND == TK_GLU && m >= 64 ? a.bias_b : a.bias;
+        const float bias = bp && row_live ? bp[(size_t)e * a.rows_per_expert + a.row0 + row_local] : 0.0f;
+#pragma unroll
+        for (int i = 0; i < 4; i++) {
+            float c[CH][2], v[2];
+#pragma unroll
+            for (int k = 0; k < CH; k++) tl_unpack2(acc[k][i], c[k][0], c[k][1]);
+#pragma unroll
+            for (int u = 0; u < 2; u++) {
+                if (KIND == TK_Q8)               // acc_even + acc_odd per lane, then (l0 + l1) + (l2 + l3)
+                    v[u] = __fadd_rn(__fadd_rn(__fadd_rn(c[0][u], c[4 % CH][u]), __fadd_rn(c[1][u], c[5 % CH][u])),
+                                     __fadd_rn(__fadd_rn(c[2][u], c[6 % CH][u]), __fadd_rn(c[3][u], c[7 % CH][u])));
+                else v[u] = __fadd_rn(__fadd_rn(c[0][u], c[1][u]), __fadd_rn(c[2][u], c[3][u]));
+                const int t = t_base + 2 * i + u;
+                if (KIND == TK_GLU) glu_sm[t * 128 + m] = __fadd_rn(v[u], bias);
+                else if (row_live && t < n_ent) {
+                    float *yp = a.y + (size_t)ent[t] * a.ldy + row_local;
+                    if (KIND == TK_Q8 && a.epi == Q8_EPI_RESID_BIAS) *yp = __fadd_rn(*yp, __fadd_rn(v[u], bias));        // x += dot + bias
+                    else *yp = a.bias ? __fadd_rn(v[u], bias) : v[u];
+                }
+            }
+        }
+        if (KIND == TK_GLU) {
+            // h = SwiGLU(gate, up) of 64 outputs x 8 tokens, its Q8 and plane image: warp = 32-block (warp & 1) of four tokens, side by side
+            asm volatile("bar.sync %0, 128;" ::"r"(2 + wg) : "memory");
+            const int blk = warp & 1, b = tile * 2 + blk, t0 = t_base + ((warp >> 1) & 1) * 4;
+            float hv[4], amax[4];
+#pragma unroll
+            for (int k = 0; k < 4; k++) {
+                hv[k] = swiglu_oai(glu_sm[(t0 + k) * 128 + blk * 32 + lane], glu_sm[(t0 + k) * 128 + 64 + blk * 32 + lane]);
+                amax[k] = fabsf(hv[k]);
+            }
+#pragma unroll
+            for (int o = 16; o > 0; o >>= 1)
+#pragma unroll
+                for (int k = 0; k < 4; k++) amax[k] = fmaxf(amax[k], __shfl_xor_sync(0xffffffffu, amax[k], o));
+#pragma unroll
+            for (int k = 0; k < 4; k++) {
+                if (t0 + k >= n_ent) break;
+                const float sc = __fdiv_rn(fmaxf(amax[k], 1e-12f), 127.0f);
+                const size_t row = (size_t)ent[t0 + k];
+                if (lane == 0) a.hs[row * (a.nrows / 32) + b] = sc;
+                ti_emit_block<TI_PLANES>(brrr_q8_round(hv[k], sc), lane, b, a.himg + row * (size_t)(a.nrows / 64) * PAIR);
+            }
         }
     }
     tl_fence_before();
@@ -350,204 +535,43 @@ __global__ void __launch_bounds__(MT_THREADS, NT == 16 ? 2 : MT_CTAS) mx_tile_ke
     if (warp == 0) asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem_base), "r"(TMEM_COLS) : "memory");
 }
 
-// ---------------------------------------------------------------- Q8 matrix x token rows (dense projections of a tile)
-// The Q8 row dot (dot_q8_i8, src/bin/engine_gpt2.rs:169-191) is 2 block parities x 4 lanes of chains,
-// chain (p, j) accumulating fma(float(t_j(b)), w_scale[b] * xs[b], acc) over the blocks b of parity p, t_j(b) the
-// exact integer dot of the lane's 8 weights with its 8 activation bytes; the row is (e0 + e1) + (e2 + e3) with
-// e_j = acc[0][j] + acc[1][j].  The weights are int8 already, so the producer warp copies the 16-byte pieces of a
-// unit straight to their place in the K-major operand tile and no thread decodes anything: one product per block
-// (128 rows x 16 columns x 32), workers = entry staging + chains.  One CTA = 128 matrix rows x up to 4 token rows.
-constexpr int QT_DEPTH = 4;
-constexpr int QT_STAGE = 2 * TL_A_BYTES + TL_ROWS * 8;      // two operand tiles (the pair's blocks) + [128 rows][2] f32 block scales
-
-struct Q8TileArgs {
-    Q8Dev m;
-    const int8_t *xq;       // [token rows][cols]
-    const float *xs;        // [token rows][cols / 32]
-    const float *bias;
-    float *y;               // [token rows][ldy]
-    int ntok, ldy;
-    DevState *state;
-};
-
-template <int EPI, int NT>
-__global__ void __maxnreg__(96) q8_tile_kernel(Q8TileArgs a) {      // 96 registers: three CTAs of 7 warps (TL_THREADS) per SM
-    constexpr int N = 4 * NT;
-    constexpr uint32_t IDESC = (2u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(N >> 3) << 17) | ((TL_ROWS >> 4) << 24);
-    constexpr uint32_t TMEM_COLS = 4 * N;
-    extern __shared__ __align__(128) unsigned char tsm[];
-    const int np = a.m.cols / 64, nb = np * 2;
-    unsigned char *ring = tsm;                                                                                  // [QT_DEPTH][QT_STAGE]
-    unsigned char (*b_tiles)[N * 32] = reinterpret_cast<unsigned char (*)[N * 32]>(tsm + QT_DEPTH * QT_STAGE);  // [half][block of the pair]
-    float *xs_sm = reinterpret_cast<float *>(tsm + QT_DEPTH * QT_STAGE + 4 * N * 32);                           // [NT][nb]
-    __shared__ __align__(8) uint64_t full[QT_DEPTH], empty[QT_DEPTH], staged[2], done[2];
-    __shared__ uint32_t tmem_base_sh;
-    const int tid = threadIdx.x, warp = tid >> 5;
-    const int t_first = blockIdx.y * NT, n_ent = min(a.ntok - t_first, NT);
-    for (int i = tid; i < 4 * N * 32 / 16; i += TL_THREADS) reinterpret_cast<uint4 *>(&b_tiles[0][0])[i] = make_uint4(0, 0, 0, 0);   // rows of absent tokens stay zero
-    if (tid == 0) {
-        for (int i = 0; i < QT_DEPTH; i++) { mbar_init(&full[i], 32); mbar_init(&empty[i], 130); }
-        mbar_init(&staged[0], 128); mbar_init(&staged[1], 128);
-        mbar_init(&done[0], 2); mbar_init(&done[1], 2);
-        mbar_fence_init();
+// ---------------------------------------------------------------- load-time re-layout of a Q8 matrix into operand units
+// A 128-row tile is [block pair][16384 B] operands, then [block pair][1024 B] scales.  Operands of a pair: [chain j][block q]
+// [row / 8][row % 8][8 halves] = operand A of the four products; scales: [128 rows][2] f32.  Rows past the end are zero.
+__global__ void q8_operand_kernel(Q8Dev m, uint8_t *__restrict__ out, size_t total) {
+    const int np = m.cols / 64;
+    for (size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x; i < total; i += (size_t)gridDim.x * blockDim.x) {
+        // one thread = 16 bytes: of a tile, np x 1024 pieces of operands, then np x 64 of scales
+        const size_t tile = i / ((size_t)np * (QOP_UNIT / 16));
+        const int k = (int)(i % ((size_t)np * (QOP_UNIT / 16))), row0 = (int)tile * TL_ROWS, op = np * 1024;
+        const int pair = k < op ? k >> 10 : (k - op) >> 6, w = k < op ? k & 1023 : 1024 + ((k - op) & 63);
+        uint4 v = make_uint4(0, 0, 0, 0);
+        if (w < 1024) {
+            const int j = w >> 8, q = (w >> 7) & 1, row = row0 + (w & 127);
+            if (row < m.rows) {
+                const int2 s = *reinterpret_cast<const int2 *>(m.data + q8_unit_off(row >> 4, pair, np) + (row & 15) * 64 + q * 32 + j * 8);
+                __half h[8];
+#pragma unroll
+                for (int k = 0; k < 8; k++) h[k] = __int2half_rn((int)(int8_t)((k < 4 ? s.x : s.y) >> (8 * (k & 3))));
+                v = *reinterpret_cast<const uint4 *>(h);
+            }
+        } else {
+            const int row = row0 + (w - 1024) * 2;
+            if (row < m.rows) {
+                const float *s = reinterpret_cast<const float *>(m.data + q8_unit_off(row >> 4, pair, np) + Q8_UNIT_SCALES) + (row & 15) * 2;
+                v = *reinterpret_cast<const uint4 *>(s);                 // rows row, row + 1 (storage is padded to 16 rows)
+            }
+        }
+        *reinterpret_cast<uint4 *>(out + i * 16) = v;
     }
-    if (warp == 0) {
-        asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(&tmem_base_sh)), "r"(TMEM_COLS) : "memory");
-        asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
-    }
-    tl_fence_before();
-    __syncthreads();
-    tl_fence_after();
-    const uint32_t tmem_base = tmem_base_sh;
-    uint32_t *err = a.state ? &a.state->err : nullptr;
-    Waiter waiter(err);
-    const int urow0 = blockIdx.x * (TL_ROWS / 16);
-    const int n_units = min(TL_ROWS / 16, q8_urows(a.m.rows) - urow0);
+}
 
-    if (warp == 4) {
-        // ---------------- producer: the weights are static, so the ring fills before the dependency wait
-        const int lane = tid & 31;
-        const unsigned char *wbase = a.m.data + q8_unit_off(urow0, 0, np);
-        const uint32_t unit_stride = (uint32_t)np * Q8_UNIT;
-        // this lane's pieces of a pair, offsets recomputed per copy (the producer has time; registers are the workers')
-        auto load = [&](int q, int slot) {
-            const unsigned char *src = wbase + (size_t)q * Q8_UNIT;
-            unsigned char *dst = ring + slot * QT_STAGE;
-#pragma unroll 4
-            for (int i = 0; i < 16; i++) {                       // operand pieces: (unit g, row rl, block p, half kh) -> tile p, K half kh, row m
-                const int idx = lane + 32 * i, kh = idx & 1, pp = (idx >> 1) & 1, rl = (idx >> 2) & 15, g = idx >> 6, m = g * 16 + rl;
-                if (g < n_units)
-                    asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(smem_u32(dst + pp * TL_A_BYTES + kh * 2048 + (m >> 3) * 128 + (m & 7) * 16)),
-                                 "l"(src + g * unit_stride + rl * 64 + pp * 32 + kh * 16) : "memory");
-            }
-#pragma unroll
-            for (int i = 0; i < 2; i++) {                        // block scales: 128 bytes per unit
-                const int idx = lane + 32 * i, g = idx >> 3, part = idx & 7;
-                if (g < n_units)
-                    asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(smem_u32(dst + 2 * TL_A_BYTES + g * 128 + part * 16)),
-                                 "l"(src + g * unit_stride + Q8_UNIT_SCALES + part * 16) : "memory");
-            }
-            asm volatile("cp.async.mbarrier.arrive.noinc.shared::cta.b64 [%0];" ::"r"(smem_u32(&full[slot])) : "memory");
-        };
-        const int pre = min(QT_DEPTH, np);
-        for (int q = 0; q < pre; q++) load(q, q);
-        pdl_wait();
-        pdl_trigger();
-        int slot = 0;
-        uint32_t par = 0;
-        for (int p = 0; p + QT_DEPTH < np; p++) {
-            waiter.wait_suspended(&empty[slot], par);                    // the products of pair p are complete and its scales read
-            load(p + QT_DEPTH, slot);
-            if (++slot == QT_DEPTH) { slot = 0; par ^= 1u; }
-        }
-        asm volatile("cp.async.wait_all;" ::: "memory");
-    } else if (tid == 160 || tid == 192) {
-        // ---------------- issuers: block k of every pair
-        pdl_wait();
-        pdl_trigger();
-        const int k = tid == 160 ? 0 : 1;
-        const uint64_t da0 = tl_smem_desc(ring + k * TL_A_BYTES, 2048);
-        const uint64_t db[2] = {tl_smem_desc(&b_tiles[k][0], N * 16), tl_smem_desc(&b_tiles[2 + k][0], N * 16)};
-        int slot = 0;
-        for (int p = 0; p < np; p++) {
-            const int h = p & 1;
-            waiter.wait_suspended(&staged[h], (uint32_t)(p >> 1) & 1u);    // every worker has seen the pair's weights land and staged its entries
-            tl_fence_after();
-            tl_mma(tmem_base + (uint32_t)((2 * h + k) * N), da0 + (uint64_t)(slot * (QT_STAGE / 16)), h ? db[1] : db[0], 0u, IDESC);
-            tl_commit(&done[h]);
-            tl_commit(&empty[slot]);
-            if (++slot == QT_DEPTH) slot = 0;
-        }
-    } else if (tid < 128) {
-        // ---------------- workers: thread = matrix row of the tile
-        pdl_wait();
-        pdl_trigger();
-        const int row = blockIdx.x * TL_ROWS + tid;
-        const bool row_live = row < a.m.rows;
-        const int n_row = tid & 63, bt = n_row >> 2, bl = tid & 3, bblk = tid >> 6;
-        const bool b_live = n_row < N && bt < n_ent;
-        // B row n = token * 4 + lane: the lane's 8 activation bytes (positions 4 lane .. + 3 and 16 + 4 lane .. + 3, the order of the unit) at k = 8 lane .. + 7
-        const uint32_t b_off = (uint32_t)((bl >> 1) * (N * 16) + (n_row >> 3) * 128 + (n_row & 7) * 16 + (bl & 1) * 8);
-        const int8_t *my_x = a.xq + (size_t)(t_first + (b_live ? bt : 0)) * a.m.cols + bblk * 32 + 4 * bl;
-        uint32_t xlo = 0, xhi = 0;
-        if (b_live) { xlo = *reinterpret_cast<const uint32_t *>(my_x); xhi = *reinterpret_cast<const uint32_t *>(my_x + 16); }
-        for (int i = tid; i < n_ent * nb; i += 128) xs_sm[i] = a.xs[(size_t)t_first * nb + i];
-        float bias_pre = 0.0f;
-        if (row_live && (EPI == Q8_EPI_BIAS || EPI == Q8_EPI_RESID_BIAS)) bias_pre = a.bias[row];
-        asm volatile("bar.sync 1, 128;" ::: "memory");             // the workers' own barrier: xs_sm is complete
-        int f_slot = 0;
-        uint32_t f_par = 0;
-        auto stage = [&](int q) -> float2 {
-            const int h = q & 1;
-            waiter.wait_suspended(&full[f_slot], f_par);
-            const float2 sc = *reinterpret_cast<const float2 *>(ring + f_slot * QT_STAGE + 2 * TL_A_BYTES + tid * 8);
-            const int q_slot = f_slot;
-            if (++f_slot == QT_DEPTH) { f_slot = 0; f_par ^= 1u; }
-            if (b_live) {
-                *reinterpret_cast<uint2 *>(&b_tiles[2 * h + bblk][b_off]) = make_uint2(xlo, xhi);
-                if (q + 1 < np) {
-                    xlo = *reinterpret_cast<const uint32_t *>(my_x + (size_t)(q + 1) * 64);
-                    xhi = *reinterpret_cast<const uint32_t *>(my_x + (size_t)(q + 1) * 64 + 16);
-                }
-            }
-            fence_proxy_async();               // generic-proxy writes (these, and the producer's copies seen through full[]) -> the tensor core's reads
-            tl_fence_before();                 // this thread's reads of the half's accumulators are done
-            mbar_arrive(&staged[h]);
-            mbar_arrive(&empty[q_slot]);
-            return sc;
-        };
-        float acc[2][N];
-#pragma unroll
-        for (int i = 0; i < N; i++) { acc[0][i] = 0.0f; acc[1][i] = 0.0f; }
-        const uint32_t lane_addr = tmem_base + ((uint32_t)(warp * 32) << 16);
-        auto chains = [&](int p, float2 sc) {
-            const int h = p & 1;
-            waiter.wait_suspended(&done[h], (uint32_t)(p >> 1) & 1u);
-            tl_fence_after();
-#pragma unroll
-            for (int k = 0; k < 2; k++) {
-                const float ws = k ? sc.y : sc.x;
-#pragma unroll
-                for (int c = 0; c < N / 16; c++) {             // 16 columns = four token rows at a time (registers)
-                    int d[16];
-                    tl_ld16(lane_addr + (uint32_t)((2 * h + k) * N + 16 * c), d);
-                    tl_wait_ld();
-#pragma unroll
-                    for (int t = 0; t < 4; t++) {
-                        const float sxs = __fmul_rn(ws, xs_sm[(4 * c + t) * nb + 2 * p + k]);
-#pragma unroll
-                        for (int l = 0; l < 4; l++) acc[k][16 * c + 4 * t + l] = __fmaf_rn((float)d[4 * t + l], sxs, acc[k][16 * c + 4 * t + l]);
-                    }
-                }
-            }
-        };
-        float2 scc = stage(0);
-        for (int p = 0; p < np; p++) {
-            float2 scn = make_float2(0.0f, 0.0f);
-            if (p + 1 < np) scn = stage(p + 1);
-            chains(p, scc);
-            scc = scn;
-        }
-        if (row_live) {
-#pragma unroll
-            for (int t = 0; t < NT; t++)
-                if (t < n_ent) {
-                    const float e0 = __fadd_rn(acc[0][4 * t], acc[1][4 * t]), e1 = __fadd_rn(acc[0][4 * t + 1], acc[1][4 * t + 1]);
-                    const float e2 = __fadd_rn(acc[0][4 * t + 2], acc[1][4 * t + 2]), e3 = __fadd_rn(acc[0][4 * t + 3], acc[1][4 * t + 3]);
-                    const float r = __fadd_rn(__fadd_rn(e0, e1), __fadd_rn(e2, e3));
-                    float *yp = a.y + (size_t)(t_first + t) * a.ldy + row;
-                    if (EPI == Q8_EPI_PLAIN) *yp = r;
-                    else if (EPI == Q8_EPI_BIAS) *yp = __fadd_rn(r, bias_pre);
-                    else *yp = __fadd_rn(*yp, __fadd_rn(r, bias_pre));                // x += dot + bias
-                }
-        }
-    } else {
-        pdl_wait();
-        pdl_trigger();
-    }
-    tl_fence_before();
-    __syncthreads();
-    if (warp == 0) asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem_base), "r"(TMEM_COLS) : "memory");
+// int8 activations and their scales -> image (callers that hold a Q8 vector only)
+template <int IMG>
+__global__ void image_kernel(const int8_t *__restrict__ xq, int nblocks_row, int nblocks, uint8_t *__restrict__ img) {
+    const int b = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5), lane = threadIdx.x & 31;
+    if (b >= nblocks) return;
+    ti_emit_block<IMG>((int)xq[(size_t)b * 32 + lane], lane, b % nblocks_row, img + (size_t)(b / nblocks_row) * (nblocks_row / 2) * ti_pair(IMG));
 }
 
 // Per expert, the (token, slot) pairs routed to it, in ascending order: entry = token * topk + slot.  One CTA per
@@ -555,6 +579,8 @@ __global__ void __maxnreg__(96) q8_tile_kernel(Q8TileArgs a) {      // 96 regist
 __global__ void __launch_bounds__(TL_MAXTOK) tile_route_kernel(const int32_t *__restrict__ top, int ntok, int topk, int *__restrict__ cnt, int *__restrict__ list) {
     __shared__ int warp_cnt[TL_MAXTOK / 32];
     const int e = blockIdx.x, t = threadIdx.x;
+    pdl_wait();
+    pdl_trigger();
     int slot = -1;
     if (t < ntok)
         for (int s = 0; s < topk; s++)
@@ -568,87 +594,114 @@ __global__ void __launch_bounds__(TL_MAXTOK) tile_route_kernel(const int32_t *__
     if (t == TL_MAXTOK - 1) cnt[e] = before + (slot >= 0 ? 1 : 0);
 }
 
-// x[t] += w[t][k] * part[t * topk + k], k ascending (part already holds the bias): the fold of
-// down_combine_kernel, one thread per (token, row).
-__global__ void tile_combine_kernel(const float *__restrict__ part, const float *__restrict__ wts, int topk, int d, float *__restrict__ x) {
-    const int t = blockIdx.y, r = blockIdx.x * blockDim.x + threadIdx.x;
-    if (r >= d) return;
-    float s = x[(size_t)t * d + r];
-    for (int k = 0; k < topk; k++) s = __fadd_rn(s, __fmul_rn(wts[t * 8 + k], part[((size_t)t * topk + k) * d + r]));
-    x[(size_t)t * d + r] = s;
+// The 16-row units of an MXFP4 matrix as a tensor of 4-bit elements: [pair][unit][8 = (row half, lane chain)][128 = 8 rows x 16 codes], boxes of
+// `units` units of one pair.  In shared memory 16 codes take 16 bytes (the upper 8 unused), the form tcgen05 reads 4-bit operands in.
+cudaError_t mx_tensor_map(MxDev w, int units, CUtensorMap *map) {
+    typedef CUresult (*encode_t)(CUtensorMap *, CUtensorMapDataType, cuuint32_t, void *, const cuuint64_t *, const cuuint64_t *, const cuuint32_t *,
+                                 const cuuint32_t *, CUtensorMapInterleave, CUtensorMapSwizzle, CUtensorMapL2promotion, CUtensorMapFloatOOBfill);
+    static encode_t encode = [] {
+        void *f = nullptr;
+        cudaDriverEntryPointQueryResult r;
+        if (cudaGetDriverEntryPointByVersion("cuTensorMapEncodeTiled", &f, 12000, cudaEnableDefault, &r) != cudaSuccess || r != cudaDriverEntryPointSuccess) f = nullptr;
+        return (encode_t)f;
+    }();
+    if (!encode) return cudaErrorNotSupported;
+    const cuuint64_t np = (cuuint64_t)w.blocks / 2;
+    const cuuint64_t dims[4] = {128, 8, (cuuint64_t)w.rows / 16, np}, strides[3] = {64, np * MX_UNIT, MX_UNIT};
+    const cuuint32_t box[4] = {128, 8, (cuuint32_t)units, 1}, ones[4] = {1, 1, 1, 1};
+    const CUresult r = encode(map, CU_TENSOR_MAP_DATA_TYPE_16U4_ALIGN16B, 4, w.data, dims, strides, box, ones, CU_TENSOR_MAP_INTERLEAVE_NONE,
+                              CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+    return r == CUDA_SUCCESS ? cudaSuccess : cudaErrorInvalidValue;
 }
 
-size_t tl_smem(int nt, int nb) { return 8 * TL_A_BYTES + 4 * (size_t)(4 * nt) * 32 + (size_t)TL_DEPTH * TL_SLOT + (size_t)nt * nb * 4; }
-
-// Block pairs need an even block count.  Entries per CTA: 4 while no expert can have more than 16 entries, 8 up to 64, else 16.
-cudaError_t tl_launch(TileArgs a, int tiles, int experts, int max_entries, cudaStream_t st) {
-    if ((a.w.blocks & 1) || a.w.blocks < 2 || max_entries < 1 || max_entries > TL_MAXTOK) return cudaErrorInvalidValue;
-    static const int wide_from = [] { const char *e = getenv("BRRR_TILE_NT16_FROM"); const int v = e ? atoi(e) : 0; return v >= 1 ? v : MT_NT16_FROM; }();
-    const int nt = max_entries <= 16 ? 4 : max_entries < wide_from ? 8 : 16;
-    const size_t smem = tl_smem(nt, a.w.blocks);
-    if (smem > 200 * 1024) return cudaErrorInvalidValue;
-    static unsigned long long configured4 = 0, configured8 = 0, configured16 = 0;      // one bit per device
-    cudaError_t ce = nt == 4 ? smem_optin(mx_tile_kernel<4>, 200 * 1024, configured4)
-                   : nt == 8 ? smem_optin(mx_tile_kernel<8>, 200 * 1024, configured8) : smem_optin(mx_tile_kernel<16>, 200 * 1024, configured16);
-    if (ce != cudaSuccess) return ce;
-    a.chunks = (max_entries + nt - 1) / nt;
-    const dim3 grid(tiles, experts * a.chunks);
-    if (nt == 4) mx_tile_kernel<4><<<grid, MT_THREADS, smem, st>>>(a);
-    else if (nt == 8) mx_tile_kernel<8><<<grid, MT_THREADS, smem, st>>>(a);
-    else mx_tile_kernel<16><<<grid, MT_THREADS, smem, st>>>(a);
-    return cudaGetLastError();
-}
-
-template <int EPI, int NT>
-cudaError_t q8_tile_launch(const Q8TileArgs &a, bool pdl, cudaStream_t st) {
-    static unsigned long long configured = 0;      // one bit per device
-    cudaError_t e = smem_optin(q8_tile_kernel<EPI, NT>, 100 * 1024, configured);
-    if (e != cudaSuccess) return e;
-    const size_t smem = (size_t)QT_DEPTH * QT_STAGE + 4 * (4 * NT) * 32 + (size_t)NT * (a.m.cols / 32) * 4;
-    if (smem > 100 * 1024) return cudaErrorInvalidValue;
-    const dim3 grid((unsigned)((a.m.rows + TL_ROWS - 1) / TL_ROWS), (unsigned)((a.ntok + NT - 1) / NT));
-    return launch_k(q8_tile_kernel<EPI, NT>, grid, dim3(TL_THREADS), smem, st, pdl, a);
+// Tokens per CTA.  Experts: by the entries an expert has on average - few tokens keep more CTAs and copies in flight (up to 16 rows
+// the launch is a stream of weights), many amortise the products' reads of operand A.  One matrix: the most that leaves a CTA for
+// most of the 148 SMs (64 rows x 2880 outputs: 8 tokens, 184 CTAs of 64 pairs, against 46 of 32 tokens that take twice as long).
+template <int KIND>
+cudaError_t tl_launch(TileArgs a, int tiles, int entries, int experts, bool pdl, cudaStream_t st) {
+    const int avg = (entries + experts - 1) / experts, most = a.cnt ? a.ntok : entries;
+    if (most < 1 || most > TL_MAXTOK) return cudaErrorInvalidValue;
+    int nt = avg > 12 ? 32 : avg > 6 ? 16 : 8;
+    if (!a.cnt) {
+        nt = entries > 16 ? 32 : entries > 8 ? 16 : 8;
+        while (nt > 8 && tiles * ((entries + nt - 1) / nt) < 120) nt /= 2;
+    }
+    static unsigned long long configured[3] = {0, 0, 0};      // one bit per device
+    // at most one partly filled chunk per expert, and never more chunks than entries
+    const int full_chunks = entries / nt, tasks = full_chunks + experts < entries ? full_chunks + experts : entries;
+    const dim3 grid(tiles, tasks);
+    cudaError_t ce;
+        if (nt == 32) {
+        if ((ce = smem_optin(tile_kernel<KIND, 32>, 220 * 1024, configured[0])) != cudaSuccess) return ce;
+        return launch_k(tile_kernel<KIND, 32>, grid, dim3(32 * 16 + 128), tl_smem<KIND, 32>(a.np), st, pdl, a);
+    }
+    if (nt == 16) {
+        if ((ce = smem_optin(tile_kernel<KIND, 16>, 220 * 1024, configured[1])) != cudaSuccess) return ce;
+        return launch_k(tile_kernel<KIND, 16>, grid, dim3(16 * 16 + 128), tl_smem<KIND, 16>(a.np), st, pdl, a);
+    }
+    if ((ce = smem_optin(tile_kernel<KIND, 8>, 220 * 1024, configured[2])) != cudaSuccess) return ce;
+    return launch_k(tile_kernel<KIND, 8>, grid, dim3(256), tl_smem<KIND, 8>(a.np), st, pdl, a);
 }
 
 }  // namespace
 
-// y[t][r] (+)= row r of m . activation t (+ bias) on the tensor cores, t < ntok <= BRRR_TILE_MAX: bit-identical to the
-// integer-unit kernels (kernels_q8.cu, kernels_rows.cu).  Four token rows per CTA up to 4 rows, eight beyond.
-cudaError_t launch_q8_tile(Q8Dev m, const int8_t *xq, const float *xs, int ntok, const float *bias, float *y, int ldy, int epi, DevState *state,
-                           bool pdl, cudaStream_t st) {
-    if (ntok < 1 || ntok > BRRR_TILE_MAX || m.cols % 64 || m.cols < 64) return cudaErrorInvalidValue;
-    Q8TileArgs a{m, xq, xs, bias, y, ntok, ldy, state};
-    const bool wide = ntok > 4;
-    switch (epi) {
-    case Q8_EPI_PLAIN: return wide ? q8_tile_launch<Q8_EPI_PLAIN, 8>(a, pdl, st) : q8_tile_launch<Q8_EPI_PLAIN, 4>(a, pdl, st);
-    case Q8_EPI_BIAS: return wide ? q8_tile_launch<Q8_EPI_BIAS, 8>(a, pdl, st) : q8_tile_launch<Q8_EPI_BIAS, 4>(a, pdl, st);
-    case Q8_EPI_RESID_BIAS: return wide ? q8_tile_launch<Q8_EPI_RESID_BIAS, 8>(a, pdl, st) : q8_tile_launch<Q8_EPI_RESID_BIAS, 4>(a, pdl, st);
-    }
-    return cudaErrorInvalidValue;
+size_t image_bytes(int rows, int cols, int kind) { return (size_t)rows * (cols / 64) * ti_pair(kind); }
+
+void launch_image(const int8_t *xq, int rows, int cols, int kind, uint8_t *img, cudaStream_t st) {
+    const int nb = cols / 32, n = rows * nb;
+    if (n <= 0) return;
+    if (kind == TI_HALF) image_kernel<TI_HALF><<<(n + 7) / 8, 256, 0, st>>>(xq, nb, n, img);
+    else image_kernel<TI_PLANES><<<(n + 7) / 8, 256, 0, st>>>(xq, nb, n, img);
 }
 
-cudaError_t launch_mx_tile(MxDev w, int row0, int nrows, const int8_t *xq, const float *xs, int ntok, float *y, int ldy, DevState *state,
-                           cudaStream_t st) {
+size_t q8_operand_bytes(int rows, int cols) { return (size_t)((rows + TL_ROWS - 1) / TL_ROWS) * (cols / 64) * QOP_UNIT; }
+
+void launch_q8_operand_pack(Q8Dev m, uint8_t *out, cudaStream_t st) {
+    const size_t total = q8_operand_bytes(m.rows, m.cols) / 16;
+    if (total) q8_operand_kernel<<<148 * 8, 256, 0, st>>>(m, out, total);
+}
+
+cudaError_t launch_q8_tile(const uint8_t *op, int rows, int cols, const uint8_t *img, const float *xs, int ntok, const float *bias, float *y, int ldy,
+                           int epi, DevState *state, bool pdl, cudaStream_t st) {
+    if (ntok < 1 || ntok > BRRR_TILE_MAX || cols % 64 || cols < 64) return cudaErrorInvalidValue;
     TileArgs a{};
-    a.w = w; a.row0 = row0; a.nrows = nrows; a.src_div = 1; a.xq = xq; a.xs = xs; a.ntok = ntok; a.y = y; a.ldy = ldy; a.state = state;
-    return tl_launch(a, (nrows + TL_ROWS - 1) / TL_ROWS, 1, ntok, st);
+    a.wa = op; a.np = cols / 64; a.nrows = rows; a.ntok = ntok; a.src_div = 1; a.img = img; a.xs = xs; a.bias = bias; a.y = y; a.ldy = ldy; a.epi = epi;
+    a.state = state;
+    return tl_launch<TK_Q8>(a, (rows + TL_ROWS - 1) / TL_ROWS, ntok, 1, pdl, st);
 }
 
-// All experts of one matrix kind against their routed entries (see TileArgs).
-cudaError_t launch_mx_tile_experts(MxDev w, int ne, int rows_per_expert, const int *cnt, const int *list, int max_entries, int src_div, const int8_t *xq,
-                                   const float *xs, const float *bias, float *y, int ldy, int col0, DevState *state, cudaStream_t st) {
+cudaError_t launch_mx_tile(MxDev w, int row0, int nrows, const uint8_t *img, const float *xs, int ntok, float *y, int ldy, DevState *state, cudaStream_t st) {
+    if ((w.blocks & 1) || w.blocks < 2) return cudaErrorInvalidValue;
     TileArgs a{};
-    a.w = w; a.row0 = 0; a.nrows = rows_per_expert; a.rows_per_expert = rows_per_expert; a.cnt = cnt; a.list = list; a.src_div = src_div;
-    a.xq = xq; a.xs = xs; a.bias = bias; a.y = y; a.ldy = ldy; a.col0 = col0; a.state = state;
-    return tl_launch(a, (rows_per_expert + TL_ROWS - 1) / TL_ROWS, ne, max_entries, st);
+    a.wa = w.data; a.np = w.blocks / 2; a.row0 = row0; a.nrows = nrows; a.ntok = ntok; a.src_div = 1; a.img = img; a.xs = xs; a.y = y; a.ldy = ldy;
+    a.state = state;
+    if (cudaError_t e = mx_tensor_map(w, 8, &a.ma)) return e;
+    return tl_launch<TK_MX>(a, ((row0 & 15) + nrows + TL_ROWS - 1) / TL_ROWS, ntok, 1, false, st);
 }
 
-void launch_tile_route(const int32_t *top, int ntok, int topk, int ne, int *cnt, int *list, cudaStream_t st) {
-    tile_route_kernel<<<ne, TL_MAXTOK, 0, st>>>(top, ntok, topk, cnt, list);
+cudaError_t launch_mx_tile_glu(MxDev gate, MxDev up, int ne, int d, const int *cnt, const int *list, int ntok, int topk, const uint8_t *img, const float *xs,
+                               const float *gate_b, const float *up_b, uint8_t *himg, float *hs, DevState *state, bool pdl, cudaStream_t st) {
+    if ((gate.blocks & 1) || gate.blocks < 2 || d % 64 || ne > 256) return cudaErrorInvalidValue;
+    TileArgs a{};
+    a.wa = gate.data; a.wb = up.data; a.np = gate.blocks / 2; a.nrows = d; a.rows_per_expert = d; a.cnt = cnt; a.list = list; a.ne = ne; a.ntok = ntok;
+    a.src_div = topk; a.img = img; a.xs = xs; a.bias = gate_b; a.bias_b = up_b; a.himg = himg; a.hs = hs; a.state = state;
+    if (cudaError_t e = mx_tensor_map(gate, 4, &a.ma)) return e;
+    if (cudaError_t e = mx_tensor_map(up, 4, &a.mb)) return e;
+    return tl_launch<TK_GLU>(a, d / 64, ntok * topk, ne, pdl, st);
 }
 
-void launch_tile_combine(const float *part, const float *wts, int topk, int d, int ntok, float *x, cudaStream_t st) {
-    tile_combine_kernel<<<dim3((d + 255) / 256, ntok), 256, 0, st>>>(part, wts, topk, d, x);
+cudaError_t launch_mx_tile_down(MxDev down, int ne, int d, const int *cnt, const int *list, int ntok, int topk, const uint8_t *himg, const float *hs,
+                                const float *bias, float *part, DevState *state, bool pdl, cudaStream_t st) {
+    if ((down.blocks & 1) || down.blocks < 2 || ne > 256) return cudaErrorInvalidValue;
+    TileArgs a{};
+    a.wa = down.data; a.np = down.blocks / 2; a.nrows = d; a.rows_per_expert = d; a.cnt = cnt; a.list = list; a.ne = ne; a.ntok = ntok; a.src_div = 1;
+    a.img = himg; a.xs = hs; a.bias = bias; a.y = part; a.ldy = d; a.state = state;
+    if (cudaError_t e = mx_tensor_map(down, 8, &a.ma)) return e;
+    return tl_launch<TK_MX>(a, (d + TL_ROWS - 1) / TL_ROWS, ntok * topk, ne, pdl, st);
+}
+
+cudaError_t launch_tile_route(const int32_t *top, int ntok, int topk, int ne, int *cnt, int *list, bool pdl, cudaStream_t st) {
+    return launch_k(tile_route_kernel, dim3(ne), dim3(TL_MAXTOK), 0, st, pdl, top, ntok, topk, cnt, list);
 }
 
 }  // namespace brrr

@@ -8,6 +8,7 @@
 #include "../../include/brrr.h"
 #include "brrr_kernels.h"
 #include "brrr_synth.h"
+#include "brrr_tile.cuh"
 
 #include <cmath>
 #include <cstdio>
@@ -59,6 +60,7 @@ struct Layer {
     MxDev gate{}, up{}, down{};
     float *gate_b = nullptr, *up_b = nullptr, *down_b = nullptr;
     MxtDev gu_t{}, down_t{};     // tensor-core tile units of gate|up and down (use_mxt)
+    uint8_t *wqkv_op = nullptr, *wo_op = nullptr;      // operand units of the Q8 projections for token rows (use_q8op)
     float *kc = nullptr, *vc = nullptr;
 };
 
@@ -108,6 +110,7 @@ struct brrr_model {
     std::vector<Layer> L;
     float *out_norm = nullptr;
     Q8Dev head{};
+    uint8_t *head_op = nullptr;      // its operand units, made by brrr_batch_open
     uint16_t *tok_embd = nullptr;
     float *rope = nullptr;
     // activations
@@ -146,15 +149,17 @@ struct brrr_model {
     EpCtx epc{};
     void *ep_buf = nullptr;
     std::vector<void *> ep_peers;
-    // scratch of the token-tile MoE step (allocated at first use): BRRR_TILE_MAX tokens x top-k entries
-    int8_t *tl_xq = nullptr, *tl_hq = nullptr;
-    float *tl_xs = nullptr, *tl_hs = nullptr, *tl_logits = nullptr, *tl_wts = nullptr, *tl_gu = nullptr, *tl_part = nullptr;
+    // token rows (prompt tiles, batched decode): up to BRRR_TILE_MAX rows walk the layers together.  Scratch, allocated at first
+    // use: residual, normalised residual, q|k|v and attention output of the rows; Q8 values, block scales and activation images
+    // (brrr_tile.cuh) of the normalised residual (n: dense half, e: experts), the attention output (a) and the experts' h (h)
+    bool use_q8op = false;       // the projections exist as operand units
+    float *tl_x = nullptr, *tl_xn = nullptr, *tl_qkv = nullptr, *tl_ao = nullptr;
+    int8_t *tl_nq = nullptr, *tl_aq = nullptr;
+    float *tl_ns = nullptr, *tl_as = nullptr, *tl_es = nullptr, *tl_hs = nullptr;
+    uint8_t *tl_nimg = nullptr, *tl_aimg = nullptr, *tl_eimg = nullptr, *tl_himg = nullptr;
+    float *tl_logits = nullptr, *tl_wts = nullptr, *tl_part = nullptr;
     int32_t *tl_top = nullptr;
     int *tl_cnt = nullptr, *tl_list = nullptr;
-    // token rows (prompt tiles, batched decode): up to BRRR_TILE_MAX rows walk the layers together
-    float *tl_x = nullptr, *tl_xn = nullptr;     // residual and normalised residual of the rows
-    float *tl_qkv = nullptr, *tl_ao = nullptr, *tl_ns = nullptr, *tl_as = nullptr;
-    int8_t *tl_nq = nullptr, *tl_aq = nullptr;
     uint32_t *tl_toks = nullptr;                 // per row: token id, position, sequence (device; filled from a pinned slot)
     int *tl_pos = nullptr, *tl_seq = nullptr;
     uint32_t *h_tile = nullptr;                  // pinned: one 64-word slot per tile in flight
@@ -479,6 +484,9 @@ int build_model(brrr_model *m, const Source &src) {
         const size_t experts = (size_t)c.n_layer * (m->ep ? m->epc.e_cnt : ne) * 3 * d * nb * 17;      // this rank's share
         const size_t rest = (size_t)c.n_vocab * d * 4 + (size_t)c.n_layer * ((size_t)(qkv_rows + d) * d * 2 + (size_t)BRRR_MAXSEQ * nkv * hd * 8) + (2ull << 30);
         m->use_mxt = d % 64 == 0 && nb % 2 == 0 && topk <= 8 && free_b > experts * 2.2 + rest;
+        // operand units of the Q8 projections for token rows: 2.1 x their Q8 bytes, single GPU, where they fit beside the rest
+        const size_t dense_op = (size_t)c.n_layer * (q8_operand_bytes(qkv_rows, d) + q8_operand_bytes(d, nh * hd));
+        m->use_q8op = !m->ep && free_b > experts * (m->use_mxt ? 2.2 : 1.1) + rest + dense_op;
         if (const char *e = getenv("BRRR_NOMXT")) if (e[0] && e[0] != '0') m->use_mxt = false;
         if (const char *e = getenv("BRRR_NOFUSEDFOLD")) if (e[0] && e[0] != '0') m->fused_fold = false;
         if (const char *e = getenv("BRRR_TILE_PREFILL")) m->tile_prefill = e[0] && e[0] != '0';
@@ -495,6 +503,13 @@ int build_model(brrr_model *m, const Source &src) {
         TRY(load_q8_part(m, src, il, BRRR_T_WV, nkv * hd, (nh + nkv) * hd, ly.wqkv, scratch));
         TRY(alloc_q8(m, d, nh * hd, &ly.wo));
         TRY(load_q8_part(m, src, il, BRRR_T_WO, d, 0, ly.wo, scratch));
+        if (m->use_q8op) {
+            TRY(m->alloc(&ly.wqkv_op, q8_operand_bytes(qkv_rows, d)));
+            TRY(m->alloc(&ly.wo_op, q8_operand_bytes(d, nh * hd)));
+            launch_q8_operand_pack(ly.wqkv, ly.wqkv_op, m->stream);
+            launch_q8_operand_pack(ly.wo, ly.wo_op, m->stream);
+            CU(cudaGetLastError());
+        }
         TRY(m->alloc(&ly.bqkv, (size_t)qkv_rows));
         TRY(fetch(m, src, il, BRRR_T_BQ, 0, nh * hd, ly.bqkv));
         TRY(fetch(m, src, il, BRRR_T_BK, 0, nkv * hd, ly.bqkv + nh * hd));
@@ -857,7 +872,7 @@ extern "C" int brrr_forward(brrr_model *m, uint32_t tok, uint32_t pos, int want,
     return BRRR_OK;
 }
 
-static int moe_tile_enqueue(brrr_model *m, int il, const float *d_xn, float *d_x, int ntok);
+static int moe_tile_enqueue(brrr_model *m, int il, const float *d_xn, int ntok, bool pdl);
 
 // Up to BRRR_TILE_MAX token rows walk the layers together (forward_tile_worker, src/bin/engine_gpt2.rs:1011-1250:
 // every stage gains a token dimension, weight row outer, tokens inner).  A row is (token, position,
@@ -876,21 +891,32 @@ enum { ROWS_PROMPT = 0, ROWS_BATCH = 1, ROWS_BATCH_PROMPT = 2 };
 static int rows_alloc(brrr_model *m) {
     if (m->tl_x) return BRRR_OK;
     const brrr_cfg &c = m->cfg;
-    const int d = c.n_embd, nb = d / 32, qkv_rows = (c.n_head + 2 * c.n_head_kv) * c.head_dim, ao = c.n_head * c.head_dim;
-    const size_t R = BRRR_TILE_MAX;
-    TRY(m->alloc(&m->tl_x, R * d)); TRY(m->alloc(&m->tl_xn, R * d));
-    TRY(m->alloc(&m->tl_qkv, R * qkv_rows)); TRY(m->alloc(&m->tl_ao, R * ao));
-    TRY(m->alloc(&m->tl_nq, R * d)); TRY(m->alloc(&m->tl_ns, R * nb));
-    TRY(m->alloc(&m->tl_aq, R * ao)); TRY(m->alloc(&m->tl_as, R * (ao / 32)));
+    const int d = c.n_embd, nb = d / 32, qkv_rows = (c.n_head + 2 * c.n_head_kv) * c.head_dim, ao = c.n_head * c.head_dim, topk = c.n_expert_used, ne = c.n_expert;
+    const size_t R = BRRR_TILE_MAX, E = R * topk;
+    TRY(m->alloc(&m->tl_xn, R * d)); TRY(m->alloc(&m->tl_qkv, R * qkv_rows)); TRY(m->alloc(&m->tl_ao, R * ao));
+    TRY(m->alloc(&m->tl_nq, R * d)); TRY(m->alloc(&m->tl_ns, R * nb)); TRY(m->alloc(&m->tl_nimg, image_bytes(R, d, TI_HALF)));
+    TRY(m->alloc(&m->tl_aq, R * ao)); TRY(m->alloc(&m->tl_as, R * (ao / 32))); TRY(m->alloc(&m->tl_aimg, image_bytes(R, ao, TI_HALF)));
+    TRY(m->alloc(&m->tl_es, R * nb)); TRY(m->alloc(&m->tl_eimg, image_bytes(R, d, TI_PLANES)));
+    TRY(m->alloc(&m->tl_hs, E * nb)); TRY(m->alloc(&m->tl_himg, image_bytes((int)E, d, TI_PLANES))); TRY(m->alloc(&m->tl_part, E * d));
+    TRY(m->alloc(&m->tl_logits, R * ne)); TRY(m->alloc(&m->tl_top, R * 8)); TRY(m->alloc(&m->tl_wts, R * 8));
+    TRY(m->alloc(&m->tl_counter, R)); TRY(m->alloc(&m->tl_cnt, ne)); TRY(m->alloc(&m->tl_list, (size_t)ne * R));
+    CU(cudaMemsetAsync(m->tl_counter, 0, R * sizeof(unsigned int), m->stream));
+    CU(cudaMemsetAsync(m->tl_eimg, 0, image_bytes(R, d, TI_PLANES), m->stream));      // producers write the non-zero bytes only
+    CU(cudaMemsetAsync(m->tl_himg, 0, image_bytes((int)E, d, TI_PLANES), m->stream));
     TRY(m->alloc(&m->tl_toks, R)); TRY(m->alloc(&m->tl_pos, R)); TRY(m->alloc(&m->tl_seq, R));
     CU(cudaMallocHost(&m->h_tile, (size_t)ROWS_SLOTS * 3 * R * sizeof(uint32_t)));
+    TRY(m->alloc(&m->tl_x, R * d));
     return BRRR_OK;
 }
+
+// Rows from which the Q8 projections of a pass run on the tensor cores.
+constexpr int ROWS_TENSOR_FROM = 9;
 
 static int enqueue_rows(brrr_model *m, int n, int kind, bool pdl) {
     const bool batch = kind != ROWS_PROMPT, one_sequence = kind != ROWS_BATCH;
     const brrr_cfg &c = m->cfg;
-    const int d = c.n_embd, nh = c.n_head, nkv = c.n_head_kv, qkv_rows = (nh + 2 * nkv) * c.head_dim;
+    const int d = c.n_embd, nh = c.n_head, nkv = c.n_head_kv, ao = nh * c.head_dim, qkv_rows = (nh + 2 * nkv) * c.head_dim, topk = c.n_expert_used;
+    const bool tensor = m->use_q8op && n >= ROWS_TENSOR_FROM;
     cudaStream_t s = m->stream;
     launch_embed_tile(m->tok_embd, d, m->tl_toks, n, m->tl_x, s);
     for (int il = 0; il < c.n_layer; il++) {
@@ -899,22 +925,28 @@ static int enqueue_rows(brrr_model *m, int n, int kind, bool pdl) {
         if (window >= BRRR_MAXSEQ) window = 0;
         float *kc = batch ? m->kcb[il] : ly.kc, *vc = batch ? m->vcb[il] : ly.vc;
         const size_t seq_stride = batch ? (size_t)nkv * BRRR_MAXSEQ * c.head_dim : 0;
-        // the first kernel after a plain launch takes the full dependency
-        CUL(launch_rmsnorm_quant(m->tl_x, ly.attn_norm, c.rms_eps, d, nullptr, m->tl_nq, m->tl_ns, false, s, n));
-        CUL(launch_q8_rows(ly.wqkv, m->tl_nq, m->tl_ns, n, ly.bqkv, m->tl_qkv, qkv_rows, Q8_EPI_BIAS, pdl, s, m->st));
+        // the previous layer's expert outputs onto the residual, attention norm (the first kernel after a plain launch takes the full dependency)
+        CUL(launch_rows_norm(m->tl_x, n, d, il ? m->tl_part : nullptr, m->tl_wts, topk, ly.attn_norm, c.rms_eps, nullptr, tensor ? nullptr : m->tl_nq, m->tl_ns,
+                             tensor ? m->tl_nimg : nullptr, TI_HALF, pdl && il, s));
+        if (tensor) CUL(launch_q8_tile(ly.wqkv_op, qkv_rows, d, m->tl_nimg, m->tl_ns, n, ly.bqkv, m->tl_qkv, qkv_rows, Q8_EPI_BIAS, m->st, pdl, s));
+        else CUL(launch_q8_rows(ly.wqkv, m->tl_nq, m->tl_ns, n, ly.bqkv, m->tl_qkv, qkv_rows, Q8_EPI_BIAS, pdl, s));
         CUL(launch_kv_append_rows(m->tl_qkv, qkv_rows, nh, nkv, kc, vc, seq_stride, m->rope, m->tl_pos, m->tl_seq, n, pdl, s));
         // prompt tiles (rows of one sequence, ascending positions) share their K / V tiles; rows of different sequences cannot
         const int group = nh / nkv;
+        int8_t *aq = tensor ? nullptr : m->tl_aq;
+        uint8_t *aimg = tensor ? m->tl_aimg : nullptr;
         if (one_sequence && !m->no_attn_rows && group <= 32 && (group & (group - 1)) == 0)
-            CUL(launch_attn_rows(m->tl_qkv, qkv_rows, kc, vc, seq_stride, m->rope, ly.sinks, nh, nkv, window, m->tl_pos, m->tl_seq, n, m->tl_ao, m->tl_aq,
-                                 m->tl_as, m->st, pdl, s));
+            CUL(launch_attn_rows(m->tl_qkv, qkv_rows, kc, vc, seq_stride, m->rope, ly.sinks, nh, nkv, window, m->tl_pos, m->tl_seq, n, m->tl_ao, aq,
+                                 m->tl_as, aimg, m->st, pdl, s));
         else
-            CUL(launch_attn_decode(m->tl_qkv, kc, vc, m->rope, ly.sinks, nh, nkv, nullptr, 0, window, m->tl_ao, m->tl_aq, m->tl_as, m->st, pdl, s, 0,
-                                   m->tl_pos, m->tl_seq, seq_stride, qkv_rows, n));
-        CUL(launch_q8_rows(ly.wo, m->tl_aq, m->tl_as, n, ly.bo, m->tl_x, d, Q8_EPI_RESID_BIAS, pdl, s, m->st));
-        CUL(launch_rmsnorm_quant(m->tl_x, ly.ffn_norm, c.rms_eps, d, m->tl_xn, m->tl_nq, m->tl_ns, pdl, s, n));
-        TRY(moe_tile_enqueue(m, il, m->tl_xn, m->tl_x, n));
+            CUL(launch_attn_decode(m->tl_qkv, kc, vc, m->rope, ly.sinks, nh, nkv, nullptr, 0, window, m->tl_ao, aq, m->tl_as, m->st, pdl, s, 0,
+                                   m->tl_pos, m->tl_seq, seq_stride, qkv_rows, n, aimg));
+        if (tensor) CUL(launch_q8_tile(ly.wo_op, d, ao, m->tl_aimg, m->tl_as, n, ly.bo, m->tl_x, d, Q8_EPI_RESID_BIAS, m->st, pdl, s));
+        else CUL(launch_q8_rows(ly.wo, m->tl_aq, m->tl_as, n, ly.bo, m->tl_x, d, Q8_EPI_RESID_BIAS, pdl, s));
+        CUL(launch_rows_norm(m->tl_x, n, d, nullptr, nullptr, 0, ly.ffn_norm, c.rms_eps, m->tl_xn, nullptr, m->tl_es, m->tl_eimg, TI_PLANES, pdl, s));
+        TRY(moe_tile_enqueue(m, il, m->tl_xn, n, pdl));
     }
+    CUL(launch_rows_norm(m->tl_x, n, d, m->tl_part, m->tl_wts, topk, nullptr, 0.0f, nullptr, nullptr, nullptr, nullptr, TI_HALF, pdl, s));
     CU(cudaGetLastError());
     return BRRR_OK;
 }
@@ -1007,6 +1039,15 @@ extern "C" int brrr_batch_open(brrr_model *m, int nseq) {
     TRY(m->alloc(&m->bt_logits, (size_t)BRRR_TILE_MAX * c.n_vocab));
     TRY(m->alloc(&m->bt_tok, BRRR_TILE_MAX));
     TRY(rows_alloc(m));
+    if (m->use_q8op) {
+        size_t free_b = 0, total_b = 0;
+        CU(cudaMemGetInfo(&free_b, &total_b));
+        if (free_b > q8_operand_bytes(c.n_vocab, c.n_embd) + (1ull << 30)) {
+            TRY(m->alloc(&m->head_op, q8_operand_bytes(c.n_vocab, c.n_embd)));
+            launch_q8_operand_pack(m->head, m->head_op, m->stream);
+            CU(cudaGetLastError());
+        }
+    }
     m->nseq = nseq;
     return BRRR_OK;
 }
@@ -1019,6 +1060,9 @@ static int batch_check(brrr_model *m, int n, const uint32_t *toks, const uint32_
     return BRRR_OK;
 }
 
+// Rows from which the vocabulary projection of a batch runs on the tensor cores.
+constexpr int HEAD_TENSOR_FROM = 5;
+
 // The layers for n rows on the sequences' caches; with out_toks, the vocabulary projection and argmax of every row.
 static int batch_rows(brrr_model *m, int n, const uint32_t *toks, const uint32_t *pos, const uint32_t *seq, uint32_t *out_toks, float *out_logits,
                       int kind = ROWS_BATCH) {
@@ -1028,11 +1072,11 @@ static int batch_rows(brrr_model *m, int n, const uint32_t *toks, const uint32_t
     cudaStream_t s = m->stream;
     TRY(rows_run(m, n, toks, pos, seq, kind));
     if (out_toks || out_logits) {
-        CUL(launch_rmsnorm_quant(m->tl_x, m->out_norm, c.rms_eps, c.n_embd, nullptr, m->tl_nq, m->tl_ns, false, s, n));
-        // from 8 rows on the vocabulary projection runs on the tensor cores (measured: 3726 against 3564 tok/s at 64 rows, 1790 against
-        // 1754 at 16; BRRR_HEAD_TILE_MIN=n moves the threshold, above BRRR_TILE_MAX = never); same bits either way
-        static const int head_tile_min = [] { const char *e = getenv("BRRR_HEAD_TILE_MIN"); const int v = e ? atoi(e) : 0; return v >= 1 ? v : 8; }();
-        CUL(launch_q8_rows(m->head, m->tl_nq, m->tl_ns, n, nullptr, m->bt_logits, c.n_vocab, Q8_EPI_PLAIN, false, s, m->st, n >= head_tile_min ? 1 : 0));
+        const bool tensor = m->head_op && n >= HEAD_TENSOR_FROM;
+        CUL(launch_rows_norm(m->tl_x, n, c.n_embd, nullptr, nullptr, 0, m->out_norm, c.rms_eps, nullptr, tensor ? nullptr : m->tl_nq, m->tl_ns,
+                             tensor ? m->tl_nimg : nullptr, TI_HALF, false, s));
+        if (tensor) CUL(launch_q8_tile(m->head_op, c.n_vocab, c.n_embd, m->tl_nimg, m->tl_ns, n, nullptr, m->bt_logits, c.n_vocab, Q8_EPI_PLAIN, m->st, m->use_pdl, s));
+        else CUL(launch_q8_rows(m->head, m->tl_nq, m->tl_ns, n, nullptr, m->bt_logits, c.n_vocab, Q8_EPI_PLAIN, false, s));
         launch_rows_argmax(m->bt_logits, c.n_vocab, n, m->bt_tok, s);
         CU(cudaGetLastError());
         CU(cudaMemcpyAsync(m->h_out + 8, m->bt_tok, (size_t)n * 4, cudaMemcpyDeviceToHost, s));
@@ -1200,32 +1244,19 @@ extern "C" int brrr_moe_ffn_step_tc(brrr_model *m, int il, const float *d_xn, fl
 
 extern "C" int brrr_model_uses_tensor_experts(const brrr_model *m) { return m && m->use_mxt ? 1 : 0; }
 
-// MoE FFN of one layer for a tile of up to BRRR_TILE_MAX (64) normalised tokens: per-token router (one launch),
-// routing lists per expert, then three grouped tensor-core matmuls (gate, up, down) that read every
-// needed expert matrix once for all its tokens, SwiGLU + Q8 per (token, slot), and the fold in slot
-// order.  Bit-identical to brrr_moe_ffn_step applied to the tokens one by one.
-// Enqueue only (no synchronisation): the tile's MoE step on m->stream.
-static int moe_tile_enqueue(brrr_model *m, int il, const float *d_xn, float *d_x, int ntok) {
+// MoE FFN of one layer for n normalised rows (floats xn for the router, plane images tl_eimg / tl_es for the experts), enqueue
+// only: per-row router (one launch), routing lists per expert, then gate | up with the SwiGLU and down as two grouped tensor-core
+// launches that read every needed expert matrix once for all its rows.  The outputs stay in tl_part, one row per (token, slot);
+// launch_rows_norm adds them to the residual in slot order.  Bit-identical to brrr_moe_ffn_step applied to the rows one by one.
+static int moe_tile_enqueue(brrr_model *m, int il, const float *d_xn, int ntok, bool pdl) {
     const brrr_cfg &c = m->cfg;
-    const int d = c.n_embd, nb = d / 32, topk = c.n_expert_used, ne = c.n_expert, R = BRRR_TILE_MAX, np_ = R * topk;
-    if (!m->tl_xq) {
-        TRY(m->alloc(&m->tl_xq, (size_t)R * d)); TRY(m->alloc(&m->tl_xs, (size_t)R * nb));
-        TRY(m->alloc(&m->tl_logits, (size_t)R * ne)); TRY(m->alloc(&m->tl_top, R * 8)); TRY(m->alloc(&m->tl_wts, R * 8));
-        TRY(m->alloc(&m->tl_counter, R)); TRY(m->alloc(&m->tl_cnt, ne)); TRY(m->alloc(&m->tl_list, (size_t)ne * R));
-        TRY(m->alloc(&m->tl_gu, (size_t)np_ * 2 * d)); TRY(m->alloc(&m->tl_hq, (size_t)np_ * d)); TRY(m->alloc(&m->tl_hs, (size_t)np_ * nb));
-        TRY(m->alloc(&m->tl_part, (size_t)np_ * d));
-        CU(cudaMemsetAsync(m->tl_counter, 0, R * sizeof(unsigned int), m->stream));
-    }
+    const int d = c.n_embd, topk = c.n_expert_used, ne = c.n_expert;
     Layer &ly = m->L[il];
     cudaStream_t s = m->stream;
-    launch_quant_q8(d_xn, ntok * d, m->tl_xq, m->tl_xs, s);
-    CUL(launch_ffn_in(d_xn, nullptr, c.rms_eps, d, ly.ginp, ly.ginp_b, ne, topk, m->tl_logits, m->tl_top, m->tl_wts, m->tl_counter, m->st, false, s, ntok));
-    launch_tile_route(m->tl_top, ntok, topk, ne, m->tl_cnt, m->tl_list, s);
-    CUL(launch_mx_tile_experts(ly.gate, ne, d, m->tl_cnt, m->tl_list, ntok, topk, m->tl_xq, m->tl_xs, ly.gate_b, m->tl_gu, 2 * d, 0, m->st, s));
-    CUL(launch_mx_tile_experts(ly.up, ne, d, m->tl_cnt, m->tl_list, ntok, topk, m->tl_xq, m->tl_xs, ly.up_b, m->tl_gu, 2 * d, d, m->st, s));
-    launch_swiglu_quant(m->tl_gu, ntok * topk, d, m->tl_hq, m->tl_hs, s);
-    CUL(launch_mx_tile_experts(ly.down, ne, d, m->tl_cnt, m->tl_list, ntok, 1, m->tl_hq, m->tl_hs, ly.down_b, m->tl_part, d, 0, m->st, s));
-    launch_tile_combine(m->tl_part, m->tl_wts, topk, d, ntok, d_x, s);
+    CUL(launch_ffn_in(d_xn, nullptr, c.rms_eps, d, ly.ginp, ly.ginp_b, ne, topk, m->tl_logits, m->tl_top, m->tl_wts, m->tl_counter, m->st, pdl, s, ntok));
+    CUL(launch_tile_route(m->tl_top, ntok, topk, ne, m->tl_cnt, m->tl_list, pdl, s));
+    CUL(launch_mx_tile_glu(ly.gate, ly.up, ne, d, m->tl_cnt, m->tl_list, ntok, topk, m->tl_eimg, m->tl_es, ly.gate_b, ly.up_b, m->tl_himg, m->tl_hs, m->st, pdl, s));
+    CUL(launch_mx_tile_down(ly.down, ne, d, m->tl_cnt, m->tl_list, ntok, topk, m->tl_himg, m->tl_hs, ly.down_b, m->tl_part, m->st, pdl, s));
     CU(cudaGetLastError());
     return BRRR_OK;
 }
@@ -1236,7 +1267,11 @@ extern "C" int brrr_moe_ffn_tile(brrr_model *m, int il, const float *d_xn, float
     CU(cudaSetDevice(m->device));
     const int topk = m->cfg.n_expert_used;
     cudaStream_t s = m->stream;
-    TRY(moe_tile_enqueue(m, il, d_xn, d_x, ntok));
+    TRY(rows_alloc(m));
+    launch_quant_q8(d_xn, ntok * m->cfg.n_embd, m->tl_nq, m->tl_es, s);
+    launch_image(m->tl_nq, ntok, m->cfg.n_embd, TI_PLANES, m->tl_eimg, s);
+    TRY(moe_tile_enqueue(m, il, d_xn, ntok, false));
+    CUL(launch_rows_norm(d_x, ntok, m->cfg.n_embd, m->tl_part, m->tl_wts, topk, nullptr, 0.0f, nullptr, nullptr, nullptr, nullptr, TI_HALF, false, s));
     if (d_top) CU(cudaMemcpy2DAsync(d_top, topk * sizeof(int32_t), m->tl_top, 8 * sizeof(int32_t), topk * sizeof(int32_t), ntok, cudaMemcpyDeviceToDevice, s));
     if (d_wts) CU(cudaMemcpy2DAsync(d_wts, topk * sizeof(float), m->tl_wts, 8 * sizeof(float), topk * sizeof(float), ntok, cudaMemcpyDeviceToDevice, s));
     CU(cudaStreamSynchronize(s));
