@@ -78,6 +78,7 @@ SIGNATURES = {
     "brrr_qwen_cfg_get": (_I, [_P, C.POINTER(QwenCfg)]),
     "brrr_qwen_close": (None, [_P]),
     "brrr_qwen_forward": (_I, [_P, C.c_uint32, C.c_uint32, _I, C.POINTER(C.c_uint32)]),
+    "brrr_qwen_prefill": (_I, [_P, _P, C.c_uint32, C.c_uint32, C.POINTER(C.c_uint32)]),
     "brrr_qwen_decode": (_I, [_P, C.c_uint32, C.c_uint32, C.c_uint32, _P]),
     "brrr_qwen_decode_enqueue": (_I, [_P, C.c_uint32, C.c_uint32, C.c_uint32]),
     "brrr_qwen_decode_wait": (_I, [_P, C.c_uint32, _P]),
@@ -94,6 +95,7 @@ SIGNATURES = {
     "brrr_quant_q8": (_I, [_P, _I, _P, _P, _P]),
     "brrr_quant_q8k": (_I, [_P, _I, _P, _P, _P, _P]),
     "brrr_q4k_matvec": (_I, [_P, _I, _I, _P, _P, _P, _P, _P, _P]),
+    "brrr_kquant_rows": (_I, [_P, _I, _I, _I, _P, _I, _P, _P]),
     "brrr_q6k_matvec": (_I, [_P, _I, _I, _P, _P, _P, _P, _P]),
     "brrr_rmsnorm_quant": (_I, [_P, _P, C.c_float, _I, _P, _P, _P, _P]),
     "brrr_fold_norm": (_I, [_P, _P, _I, _I, _P, _P, _P, _P, C.c_float, _P, _P, _I, _P]),

@@ -64,6 +64,26 @@ cudaError_t launch_qw_head(const KMatDev &head, const int8_t *xq, const float *y
                            bool pdl, cudaStream_t st);
 // Q6_K rows from the GGUF layout (210-byte superblocks) into the aligned planes of KMatDev (planes = 1)
 void launch_q6k_planes(const uint8_t *src, size_t rows, int cols, uint8_t *dst, cudaStream_t st);
+// ---- qwen3moe token rows (kernels_qwrows.cu, kernels_kqt.cu): images and handles are described in brrr_kqt.cuh
+struct KqtMat;
+cudaError_t kqt_matrix(const KMatDev &m, size_t rows_total, KqtMat *out);      // rows_total: rows in memory (experts x rows)
+// y[i][entry][row] (+)= matrix i (nmat of equal width, stacked) . activation row entry / src_div.  cnt / list: per expert the entries routed to it
+// (launch_tile_route), matrices of rows_per_expert rows per expert; cnt == nullptr: entries 0 .. ntok - 1 of one matrix
+cudaError_t launch_kqt(const KqtMat *const *mats, float *const *ys_out, const int *ldy, int nmat, int rows_per_expert, const int *cnt, const int *list, int ne, int ntok,
+                       int topk, int src_div, const uint8_t *img, const float *ys, bool resid, DevState *state, bool pdl, cudaStream_t st);
+cudaError_t launch_qr_embed(const uint8_t *embd, int d, const uint32_t *toks, int rows, float *x, bool pdl, cudaStream_t st);
+// part (nullable): x[t] += sum over k of wts[8 t + k] part[t topk + k]; w (nullable): norm and image (ys: scales per superblock), normalised floats xn (nullable)
+cudaError_t launch_qr_norm(float *x, int rows, int d, const float *part, const float *wts, int topk, const float *w, float eps, float *xn, uint8_t *img, float *ys, bool pdl,
+                           cudaStream_t st);
+cudaError_t launch_qr_qknorm(float *q, const float *k, const float *v, const float *q_norm, const float *k_norm, const float *rope, float eps, int nh, int nkv, int pos0,
+                             int rows, float *kc, float *vc, bool pdl, cudaStream_t st);
+bool qr_attn_fits(int nh, int nkv);       // head groupings the row attention is written for
+cudaError_t launch_qr_attn(const float *q, const float *kc, const float *vc, int nh, int nkv, int pos0, int rows, uint8_t *img, float *ys, bool pdl, cudaStream_t st);
+cudaError_t launch_qr_glu(const float *g, const float *u, int entries, int ff, uint8_t *img, float *ys, bool pdl, cudaStream_t st);
+void launch_qr_image(const float *x, int rows, int cols, uint8_t *img, float *ys, cudaStream_t st);
+// router of normalised token rows: logits [ntok][ne], routing [ntok][8]; counter: one zeroed word per four tokens
+cudaError_t launch_router_rows(const float *xn, int d, const float *Wt, const float *b, int ne, int topk, int ntok, float *logits, int32_t *top, float *wts,
+                               unsigned int *counter, DevState *state, bool pdl, cudaStream_t st);
 char *host_err_buf();   // thread-local text behind brrr_last_cuda_error (512 bytes)
 
 // ---- Q8 matrices (kernels_q8.cu)

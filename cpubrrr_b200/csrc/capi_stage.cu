@@ -2,6 +2,7 @@
 // launches the same kernel the forward pass uses for that stage.
 #include "../../include/brrr.h"
 #include "brrr_kernels.h"
+#include "brrr_kqt.cuh"
 #include "brrr_tile.cuh"
 
 #include <cstdio>
@@ -42,6 +43,27 @@ extern "C" int brrr_q6k_matvec(const uint8_t *d_w, int rows, int cols, const int
     if (((uintptr_t)d_w & 1) || ((uintptr_t)d_xq & 1)) return BRRR_ERR_ARG;
     launch_q6k_matvec(d_w, rows, cols, d_xq, d_ys, d_y, d_sbdots, (cudaStream_t)stream);
     return check_launch();
+}
+
+extern "C" int brrr_kquant_rows(const uint8_t *d_w, int type, int rows, int cols, const float *d_x, int ntok, float *d_y, void *stream) {
+    if (!d_w || !d_x || !d_y || (type != 12 && type != 14) || rows <= 0 || rows % 128 || cols <= 0 || cols % 256 || ntok < 1 || ntok > BRRR_TILE_MAX) return BRRR_ERR_ARG;
+    if (((uintptr_t)d_w & 15) || ((uintptr_t)d_x & 15)) return BRRR_ERR_ARG;
+    cudaStream_t st = (cudaStream_t)stream;
+    KMatDev m{d_w, type, rows, cols, type == 14};
+    const size_t wb = type == 14 ? m.bpr() * rows : 0, nblk = (size_t)ntok * (cols / 256), ib = nblk * KIMG_SB;
+    uint8_t *buf = nullptr;
+    if (cudaMallocAsync(&buf, wb + ib + nblk * 4, st) != cudaSuccess) return BRRR_ERR_NOMEM;
+    uint8_t *img = buf + wb;
+    float *ys = (float *)(img + ib);
+    if (type == 14) { launch_q6k_planes(d_w, rows, cols, buf, st); m.p = buf; }
+    launch_qr_image(d_x, ntok, cols, img, ys, st);
+    KqtMat t;
+    const KqtMat *mats[1] = {&t};
+    float *out[1] = {d_y};
+    cudaError_t e = kqt_matrix(m, rows, &t);
+    if (e == cudaSuccess) e = launch_kqt(mats, out, &rows, 1, 0, nullptr, nullptr, 1, ntok, 1, 1, img, ys, false, nullptr, false, st);
+    cudaFreeAsync(buf, st);
+    return e == cudaSuccess ? check_launch() : BRRR_ERR_CUDA;
 }
 
 extern "C" int brrr_rmsnorm_quant(const float *d_x, const float *d_w, float eps, int n, float *d_xn, int8_t *d_q, float *d_s, void *stream) {

@@ -371,8 +371,7 @@ extern "C" int brrr_qwen_generate(brrr_qwen *m, const brrr_tokenizer *t, const u
     auto t0 = std::chrono::steady_clock::now();
     uint32_t next = 0;
     int st;
-    for (size_t i = 0; i < n_ids; i++)
-        if ((st = brrr_qwen_forward(m, ids[i], (uint32_t)i, i + 1 == n_ids, &next)) != BRRR_OK) return st;
+    if ((st = brrr_qwen_prefill(m, ids, (uint32_t)n_ids, 0, &next)) != BRRR_OK) return st;
     auto t1 = std::chrono::steady_clock::now();
     size_t pos = n_ids;
     uint32_t n = 0;

@@ -267,6 +267,121 @@ __global__ void __launch_bounds__(RT_THREADS) ffn_in_kernel(RouterArgs a) {
     }
 }
 
+// ---------------------------------------------------------------- router of token rows (normalised rows in, routing out)
+// The serial sum of a (token, expert) pair cannot be split, but the pairs are independent: lane = expert of a 32-expert group, TPW
+// tokens per warp, four warps.  Weight and activation tiles (256 elements of d) come through one ring of bulk copies; a lane's 16-byte
+// weight read serves TPW tokens, the activations are broadcast reads.  Shared-memory reads are the bound: (4 + TPW) x 4 wavefronts
+// per four elements.  With several groups the last CTA of a token block runs the top-k of its tokens.
+constexpr int RR_WARPS = 4, RR_STAGES = 3;
+
+template <int TPW>
+__global__ void __launch_bounds__(RR_WARPS * 32) router_rows_kernel(RouterArgs a, int ntok) {
+    constexpr int TT = RR_WARPS * TPW;
+    constexpr size_t STAGE = (size_t)(RT_TILE_FLOATS + TT * RT_TJ) * 4;
+    extern __shared__ __align__(128) unsigned char smraw[];
+    __shared__ __align__(8) uint64_t full[RR_STAGES];
+    __shared__ int last_sh;
+    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, d = a.d;
+    const int e0 = blockIdx.x * 32, t0 = blockIdx.y * TT, nt = min(TT, ntok - t0);
+    const int ntiles = (d + RT_TJ - 1) / RT_TJ;
+    const float *wsrc = a.Wt + (size_t)blockIdx.x * ntiles * RT_TILE_FLOATS;
+    Waiter waiter(a.state ? &a.state->err : nullptr);
+    if (tid == 0) {
+        for (int s = 0; s < RR_STAGES; s++) mbar_init(&full[s], 1);
+        mbar_fence_init();
+    }
+    auto issue = [&](int t, bool weights, bool rows) {            // warp 0; the barrier counts both parts
+        unsigned char *st = smraw + (size_t)(t % RR_STAGES) * STAGE;
+        const uint32_t len = (uint32_t)min(RT_TJ, d - t * RT_TJ) * 4;
+        if (weights && lane == 0) {
+            mbar_expect_tx(&full[t % RR_STAGES], RT_TILE_FLOATS * 4 + nt * len);
+            bulk_g2s(st, wsrc + (size_t)t * RT_TILE_FLOATS, RT_TILE_FLOATS * 4, &full[t % RR_STAGES]);
+        }
+        __syncwarp();
+        if (rows && lane < nt) bulk_g2s(st + (size_t)RT_TILE_FLOATS * 4 + lane * RT_TJ * 4, a.x_in + (size_t)(t0 + lane) * d + t * RT_TJ, len, &full[t % RR_STAGES]);
+    };
+    __syncthreads();
+    if (warp == 0)
+        for (int t = 0; t < min(RR_STAGES, ntiles); t++) issue(t, true, false);        // weights do not depend on the kernel before
+    pdl_wait();
+    pdl_trigger();
+    waiter.poison_if_failed();
+    if (warp == 0)
+        for (int t = 0; t < min(RR_STAGES, ntiles); t++) issue(t, false, true);
+    float acc[TPW];
+#pragma unroll
+    for (int k = 0; k < TPW; k++) acc[k] = (a.b && e0 + lane < a.ne) ? a.b[e0 + lane] : 0.0f;
+    for (int t = 0; t < ntiles; t++) {
+        const unsigned char *st = smraw + (size_t)(t % RR_STAGES) * STAGE;
+        waiter.wait(&full[t % RR_STAGES], (uint32_t)(t / RR_STAGES) & 1u);
+        const float *w = reinterpret_cast<const float *>(st) + lane * RT_STRIDE, *x = reinterpret_cast<const float *>(st) + RT_TILE_FLOATS + warp * TPW * RT_TJ;
+        const int len = min(RT_TJ, d - t * RT_TJ);
+#pragma unroll 4
+        for (int j = 0; j < len; j += 4) {
+            const float4 wv = *reinterpret_cast<const float4 *>(w + j);
+#pragma unroll
+            for (int k = 0; k < TPW; k++) {
+                const float4 xv = *reinterpret_cast<const float4 *>(x + k * RT_TJ + j);
+                acc[k] = __fadd_rn(acc[k], __fmul_rn(wv.x, xv.x));
+                acc[k] = __fadd_rn(acc[k], __fmul_rn(wv.y, xv.y));
+                acc[k] = __fadd_rn(acc[k], __fmul_rn(wv.z, xv.z));
+                acc[k] = __fadd_rn(acc[k], __fmul_rn(wv.w, xv.w));
+            }
+        }
+        __syncthreads();                      // the stage is free
+        if (warp == 0 && t + RR_STAGES < ntiles) { fence_proxy_async(); issue(t + RR_STAGES, true, true); }
+    }
+    float *lg = reinterpret_cast<float *>(smraw) + warp * 256;        // top-k staging, a warp's own
+    const bool one = gridDim.x == 1;
+#pragma unroll
+    for (int k = 0; k < TPW; k++)
+        if (warp * TPW + k < nt && e0 + lane < a.ne) a.logits[(size_t)(t0 + warp * TPW + k) * a.ne + e0 + lane] = acc[k];
+    if (!one) {
+        __threadfence();
+        __syncthreads();
+        if (tid == 0) last_sh = atomicAdd(a.counter + blockIdx.y, 1u) == gridDim.x - 1;
+        __syncthreads();
+        if (!last_sh) return;
+        __threadfence();
+        if (tid == 0) a.counter[blockIdx.y] = 0u;
+    }
+#pragma unroll
+    for (int k = 0; k < TPW; k++) {
+        const int t = warp * TPW + k;
+        if (t >= nt) break;
+        __syncwarp();
+        if (one) { if (lane < a.ne) lg[lane] = acc[k]; }
+        else for (int e = lane; e < a.ne; e += 32) lg[e] = __ldcg(a.logits + (size_t)(t0 + t) * a.ne + e);
+        __syncwarp();
+        RouterArgs b = a;
+        b.top = a.top + (t0 + t) * 8;
+        b.wts = a.wts + (t0 + t) * 8;
+        warp_topk(b, lg, lane);
+    }
+}
+
+template <int TPW>
+static cudaError_t router_rows_launch(const RouterArgs &a, int ntok, bool pdl, cudaStream_t st) {
+    constexpr int TT = RR_WARPS * TPW;
+    constexpr size_t smem = (size_t)RR_STAGES * (RT_TILE_FLOATS + TT * RT_TJ) * 4;
+    static unsigned long long configured = 0;      // one bit per device
+    cudaError_t e = smem_optin(router_rows_kernel<TPW>, (int)smem, configured);
+    if (e != cudaSuccess) return e;
+    return launch_k(router_rows_kernel<TPW>, dim3((a.ne + 31) / 32, (ntok + TT - 1) / TT), dim3(RR_WARPS * 32), smem, st, pdl, a, ntok);
+}
+
+cudaError_t launch_router_rows(const float *xn, int d, const float *Wt, const float *b, int ne, int topk, int ntok, float *logits, int32_t *top, float *wts,
+                               unsigned int *counter, DevState *state, bool pdl, cudaStream_t st) {
+    if (d % 64 || ne > 256 || topk > 8 || ntok < 1) return cudaErrorInvalidValue;
+    RouterArgs a{};
+    a.x_in = xn; a.d = d; a.Wt = Wt; a.b = b; a.ne = ne; a.topk = topk; a.logits = logits; a.top = top; a.wts = wts; a.counter = counter; a.state = state;
+    // few tokens per warp are fast while every CTA finds an SM of its own (a CTA of four warps leaves its SM's schedulers half idle)
+    const int groups = (ne + 31) / 32;
+    if (groups * ((ntok + 3) / 4) <= 148) return router_rows_launch<1>(a, ntok, pdl, st);
+    if (groups * ((ntok + 7) / 8) <= 148) return router_rows_launch<2>(a, ntok, pdl, st);
+    return router_rows_launch<4>(a, ntok, pdl, st);
+}
+
 size_t router_packed_floats(int ne, int d) { return (size_t)((ne + 31) / 32) * ((d + RT_TJ - 1) / RT_TJ) * RT_TILE_FLOATS; }
 
 cudaError_t launch_ffn_in(const float *x_in, const float *norm_w, float eps, int d, const float *Wt, const float *b, int ne, int topk,

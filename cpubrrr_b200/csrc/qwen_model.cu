@@ -8,7 +8,7 @@
 // uses them straight from the mapped blob.
 #include "../../include/brrr.h"
 #include "brrr_kernels.h"
-#include "brrr_kq.cuh"
+#include "brrr_kqt.cuh"
 #include "brrr_synth.h"
 
 #include <cmath>
@@ -41,6 +41,7 @@ namespace {
 struct QLayer {
     float *attn_norm = nullptr, *ffn_norm = nullptr, *q_norm = nullptr, *k_norm = nullptr, *ginp = nullptr;
     KMatDev wq{}, wk{}, wv{}, wo{}, gate{}, up{}, down{};
+    KqtMat tq, tk, tv, to, tgate, tup, tdown;      // the same matrices for token rows (has_rows)
     float *kc = nullptr, *vc = nullptr;      // [kv head][position][head_dim]
 };
 
@@ -88,6 +89,16 @@ struct brrr_qwen {
     cudaGraphExec_t g_head = nullptr, g_nohead = nullptr;
     int launches_head = 0, launches_nohead = 0;
     bool use_pdl = true;
+    // prompt tiles: up to BRRR_TILE_MAX consecutive positions walk the layers together
+    bool has_rows = false;
+    struct {
+        float *x, *xn, *q, *k, *v, *gate, *up, *part, *xs, *as, *hs, *wts, *rlogits;
+        uint8_t *img, *aimg, *himg;
+        int32_t *top;
+        int *cnt, *list;
+        unsigned int *counter;
+        uint32_t *toks;
+    } r{};
     std::vector<void *> allocs;
 
     template <typename T> int alloc(T **p, size_t n) {
@@ -227,6 +238,70 @@ int qenqueue_step(brrr_qwen *m, bool want, float *trace_dev, int *nlaunch) {
     return BRRR_OK;
 }
 
+// Buffers and matrix handles of the prompt tiles; a model whose shape the row kernels do not cover goes without.
+int qrows_alloc(brrr_qwen *m) {
+    const brrr_qwen_cfg &c = m->cfg;
+    const int d = c.n_embd, nh = c.n_head, nkv = c.n_head_kv, hd = c.head_dim, ne = c.n_expert, ff = c.n_ff_exp, topk = c.n_expert_used;
+    if (!qr_attn_fits(nh, nkv)) return BRRR_OK;
+    for (QLayer &ly : m->L) {
+        const struct { const KMatDev *m; size_t rows; KqtMat *t; } all[7] = {
+            {&ly.wq, (size_t)ly.wq.rows, &ly.tq}, {&ly.wk, (size_t)ly.wk.rows, &ly.tk}, {&ly.wv, (size_t)ly.wv.rows, &ly.tv}, {&ly.wo, (size_t)ly.wo.rows, &ly.to},
+            {&ly.gate, (size_t)ne * ff, &ly.tgate}, {&ly.up, (size_t)ne * ff, &ly.tup}, {&ly.down, (size_t)ne * d, &ly.tdown}};
+        for (const auto &t : all) CU(kqt_matrix(*t.m, t.rows, t.t));
+    }
+    auto &r = m->r;
+    const size_t T = BRRR_TILE_MAX, E = T * topk;
+    TRY(m->alloc(&r.x, T * d)); TRY(m->alloc(&r.xn, T * d)); TRY(m->alloc(&r.q, T * nh * hd)); TRY(m->alloc(&r.k, T * nkv * hd)); TRY(m->alloc(&r.v, T * nkv * hd));
+    TRY(m->alloc(&r.gate, E * ff)); TRY(m->alloc(&r.up, E * ff)); TRY(m->alloc(&r.part, E * d));
+    TRY(m->alloc(&r.img, T * (d / 256) * KIMG_SB)); TRY(m->alloc(&r.aimg, T * (nh * hd / 256) * KIMG_SB)); TRY(m->alloc(&r.himg, E * (ff / 256) * KIMG_SB));
+    TRY(m->alloc(&r.xs, T * (d / 256))); TRY(m->alloc(&r.as, T * (nh * hd / 256))); TRY(m->alloc(&r.hs, E * (ff / 256)));
+    TRY(m->alloc(&r.wts, T * 8)); TRY(m->alloc(&r.top, T * 8)); TRY(m->alloc(&r.rlogits, T * ne));
+    TRY(m->alloc(&r.cnt, ne)); TRY(m->alloc(&r.list, (size_t)ne * T)); TRY(m->alloc(&r.counter, T)); TRY(m->alloc(&r.toks, T));
+    CU(cudaMemsetAsync(r.counter, 0, T * sizeof(unsigned int), m->stream));
+    m->has_rows = true;
+    return BRRR_OK;
+}
+
+// Rows 0 .. rows - 1 of m->r.toks at positions pos0 .. through every layer; last: the final row's vocabulary projection as well.
+int qenqueue_rows(brrr_qwen *m, int rows, int pos0, bool last) {
+    const brrr_qwen_cfg &c = m->cfg;
+    const int d = c.n_embd, nh = c.n_head, nkv = c.n_head_kv, hd = c.head_dim, ne = c.n_expert, ff = c.n_ff_exp, topk = c.n_expert_used;
+    auto &r = m->r;
+    cudaStream_t s = m->stream;
+    const bool pdl = m->use_pdl;
+    CU(launch_qr_embed(m->embd.p, d, r.toks, rows, r.x, false, s));
+    const float *part = nullptr;
+    for (int il = 0; il < c.n_layer; il++) {
+        QLayer &ly = m->L[il];
+        CU(launch_qr_norm(r.x, rows, d, part, r.wts, topk, ly.attn_norm, c.rms_eps, nullptr, r.img, r.xs, pdl, s));
+        const KqtMat *qkv[3] = {&ly.tq, &ly.tk, &ly.tv};
+        float *qkv_out[3] = {r.q, r.k, r.v};
+        const int ld3[3] = {nh * hd, nkv * hd, nkv * hd};
+        CU(launch_kqt(qkv, qkv_out, ld3, 3, 0, nullptr, nullptr, 1, rows, 1, 1, r.img, r.xs, false, m->st, pdl, s));
+        CU(launch_qr_qknorm(r.q, r.k, r.v, ly.q_norm, ly.k_norm, m->rope, c.rms_eps, nh, nkv, pos0, rows, ly.kc, ly.vc, pdl, s));
+        CU(launch_qr_attn(r.q, ly.kc, ly.vc, nh, nkv, pos0, rows, r.aimg, r.as, pdl, s));
+        const KqtMat *o[1] = {&ly.to}, *gu[2] = {&ly.tgate, &ly.tup}, *dn[1] = {&ly.tdown};
+        float *xo[1] = {r.x}, *guo[2] = {r.gate, r.up}, *dno[1] = {r.part};
+        const int ldd[1] = {d}, ldf[2] = {ff, ff};
+        CU(launch_kqt(o, xo, ldd, 1, 0, nullptr, nullptr, 1, rows, 1, 1, r.aimg, r.as, true, m->st, pdl, s));
+        CU(launch_qr_norm(r.x, rows, d, nullptr, nullptr, 0, ly.ffn_norm, c.rms_eps, r.xn, r.img, r.xs, pdl, s));
+        CU(launch_router_rows(r.xn, d, ly.ginp, nullptr, ne, topk, rows, r.rlogits, r.top, r.wts, r.counter, m->st, pdl, s));
+        CU(launch_tile_route(r.top, rows, topk, ne, r.cnt, r.list, pdl, s));
+        CU(launch_kqt(gu, guo, ldf, 2, ff, r.cnt, r.list, ne, rows, topk, topk, r.img, r.xs, false, m->st, pdl, s));
+        CU(launch_qr_glu(r.gate, r.up, rows * topk, ff, r.himg, r.hs, pdl, s));
+        CU(launch_kqt(dn, dno, ldd, 1, d, r.cnt, r.list, ne, rows, topk, 1, r.himg, r.hs, false, m->st, pdl, s));
+        part = r.part;
+    }
+    if (!last) return BRRR_OK;            // rows that only fill the cache: nobody reads their residual
+    CU(launch_qr_norm(r.x, rows, d, part, r.wts, topk, nullptr, c.rms_eps, nullptr, nullptr, nullptr, pdl, s));
+    CU(cudaMemcpyAsync(m->x, r.x + (size_t)(rows - 1) * d, (size_t)d * 4, cudaMemcpyDeviceToDevice, s));
+    CU(launch_qw_norm_quant(m->x, m->out_norm, c.rms_eps, d, nullptr, m->xq, m->xs, m->xsum, false, s));
+    CU(launch_qw_head(m->head, m->xq, m->xs, m->xsum, m->logits, m->st, pdl, s));
+    launch_finish_token(m->st, s);
+    CU(cudaGetLastError());
+    return BRRR_OK;
+}
+
 int qcapture(brrr_qwen *m, bool want, cudaGraphExec_t *out, int *nlaunch) {
     cudaGraph_t g = nullptr;
     CU(cudaStreamBeginCapture(m->stream, cudaStreamCaptureModeThreadLocal));
@@ -307,7 +382,8 @@ int qbuild(brrr_qwen *m, const QSource &src) {
     CU(cudaMemsetAsync(m->down_counter, 0, sizeof(unsigned int), m->stream));
     CU(cudaMemsetAsync(m->st, 0, sizeof(DevState), m->stream));
     CU(cudaMemsetAsync(m->x, 0, d * 4, m->stream));
-    CU(cudaMallocHost(&m->h_in, 16));
+    TRY(qrows_alloc(m));
+    CU(cudaMallocHost(&m->h_in, (BRRR_MAXSEQ + 4) * sizeof(uint32_t)));
     CU(cudaMallocHost(&m->h_out, BRRR_MAXSEQ * sizeof(uint32_t)));
     CU(cudaStreamSynchronize(m->stream));
     // one direct (un-captured) step configures kernel attributes and validates the launches
@@ -453,6 +529,34 @@ extern "C" int brrr_qwen_forward(brrr_qwen *m, uint32_t tok, uint32_t pos, int w
     CU(cudaStreamSynchronize(m->stream));
     if (m->h_out[6] != 0) { QERR("device wait timed out (code %u)", m->h_out[6]); return BRRR_ERR_STATE; }
     if (want && out_tok) *out_tok = m->h_out[0];
+    return BRRR_OK;
+}
+
+extern "C" int brrr_qwen_prefill(brrr_qwen *m, const uint32_t *toks, uint32_t n, uint32_t pos0, uint32_t *out_tok) {
+    if (!m || !toks || n == 0) return BRRR_ERR_ARG;
+    if (pos0 >= BRRR_MAXSEQ || n > BRRR_MAXSEQ - pos0) return BRRR_ERR_RANGE;
+    for (uint32_t i = 0; i < n; i++)
+        if (toks[i] >= (uint32_t)m->cfg.n_vocab) return BRRR_ERR_RANGE;
+    if (n == 1 || !m->has_rows) {
+        for (uint32_t i = 0; i < n; i++) TRY(brrr_qwen_forward(m, toks[i], pos0 + i, i + 1 == n, out_tok));
+        return BRRR_OK;
+    }
+    CU(cudaSetDevice(m->device));
+    memcpy(m->h_in + 2, toks, (size_t)n * sizeof(uint32_t));
+    for (uint32_t i = 0; i < n; i += BRRR_TILE_MAX) {
+        const uint32_t rows = n - i < BRRR_TILE_MAX ? n - i : BRRR_TILE_MAX;
+        CU(cudaMemcpyAsync(m->r.toks, m->h_in + 2 + i, rows * sizeof(uint32_t), cudaMemcpyHostToDevice, m->stream));
+        const bool last = i + rows == n;
+        if (last) {
+            m->h_in[0] = toks[n - 1]; m->h_in[1] = pos0 + n - 1;
+            CU(cudaMemcpyAsync(m->st, m->h_in, 8, cudaMemcpyHostToDevice, m->stream));      // DevState.tok, .pos of the last token
+        }
+        TRY(qenqueue_rows(m, (int)rows, (int)(pos0 + i), last));
+    }
+    CU(cudaMemcpyAsync(m->h_out, m->st, 32, cudaMemcpyDeviceToHost, m->stream));
+    CU(cudaStreamSynchronize(m->stream));
+    if (m->h_out[6] != 0) { QERR("device wait timed out (code %u)", m->h_out[6]); return BRRR_ERR_STATE; }
+    if (out_tok) *out_tok = m->h_out[0];
     return BRRR_OK;
 }
 

@@ -60,11 +60,13 @@ class QwenEngine:
         return int(out.value)
 
     def prefill(self, ids, pos0=0):
-        """Feed a prompt token by token (generate(), engine_qwen2.rs:606-609); returns the first generated token."""
-        nxt = 0
-        for i, t in enumerate(ids):
-            nxt = self.run(t, pos0 + i, i == len(ids) - 1)
-        return nxt
+        """Feed a prompt (generate(), engine_qwen2.rs:606-609); returns the first generated token."""
+        ids = np.ascontiguousarray(ids, dtype=np.uint32)
+        if ids.size == 0:
+            return 0
+        out = C.c_uint32(0)
+        check(lib().brrr_qwen_prefill(self._h, ids.ctypes.data, ids.size, int(pos0), C.byref(out)), "brrr_qwen_prefill")
+        return int(out.value)
 
     def decode(self, first_tok, pos, n):
         out = np.empty(n, np.uint32)

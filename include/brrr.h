@@ -243,6 +243,10 @@ void brrr_qwen_close(brrr_qwen *m);
  * the greedy token (first strict maximum).  Replaces run(t, pos) and the worker pool
  * (src/bin/engine_qwen2.rs:302-451, 571-595). */
 int brrr_qwen_forward(brrr_qwen *m, uint32_t tok, uint32_t pos, int want_logits, uint32_t *out_tok);
+/* n tokens of a prompt at positions pos0 ..: fills the cache, *out_tok (nullable) and the logits are the last
+ * token's.  Same results as n calls of brrr_qwen_forward; up to BRRR_TILE_MAX tokens walk the layers together.
+ * Replaces the prompt loop of generate (src/bin/engine_qwen2.rs:606-609). */
+int brrr_qwen_prefill(brrr_qwen *m, const uint32_t *toks, uint32_t n, uint32_t pos0, uint32_t *out_tok);
 /* n greedy steps starting from first_tok at position pos with the token fed back on the device;
  * out_toks[i] is the token produced by step i.  Replaces the decode loop of generate
  * (src/bin/engine_qwen2.rs:613-619) without its stop test. */
@@ -305,6 +309,11 @@ int brrr_q4k_matvec(const uint8_t *d_w, int rows, int cols, const int8_t *d_xq, 
  * aligned.  Replaces q6k_dot (src/bin/engine_qwen2.rs:164-200). */
 int brrr_q6k_matvec(const uint8_t *d_w, int rows, int cols, const int8_t *d_xq, const float *d_ys, float *d_y,
                     int32_t *d_sbdots, void *stream);
+
+/* y[t][r] = row r . token row t for ntok rows of floats (quantised to Q8_K inside), type 12 (Q4_K) or 14 (Q6_K) in the GGUF
+ * byte layout: the tensor-core product of the prompt tiles, same bits as brrr_q4k_matvec / brrr_q6k_matvec per row.
+ * rows % 128 == 0, ntok <= BRRR_TILE_MAX; d_w and d_x 16-byte aligned. */
+int brrr_kquant_rows(const uint8_t *d_w, int type, int rows, int cols, const float *d_x, int ntok, float *d_y, void *stream);
 
 /* RMSNorm then brrr_quant_q8; d_xn (nullable) receives the normalised floats.
  * Replaces ssq + rmsnorm_quant_par (src/bin/engine_gpt2.rs:709-738). */
