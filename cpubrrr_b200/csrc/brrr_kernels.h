@@ -67,10 +67,15 @@ void launch_q6k_planes(const uint8_t *src, size_t rows, int cols, uint8_t *dst, 
 // ---- qwen3moe token rows (kernels_qwrows.cu, kernels_kqt.cu): images and handles are described in brrr_kqt.cuh
 struct KqtMat;
 cudaError_t kqt_matrix(const KMatDev &m, size_t rows_total, KqtMat *out);      // rows_total: rows in memory (experts x rows)
-// y[i][entry][row] (+)= matrix i (nmat of equal width, stacked) . activation row entry / src_div.  cnt / list: per expert the entries routed to it
-// (launch_tile_route), matrices of rows_per_expert rows per expert; cnt == nullptr: entries 0 .. ntok - 1 of one matrix
-cudaError_t launch_kqt(const KqtMat *const *mats, float *const *ys_out, const int *ldy, int nmat, int rows_per_expert, const int *cnt, const int *list, int ne, int ntok,
-                       int topk, int src_div, const uint8_t *img, const float *ys, bool resid, DevState *state, bool pdl, cudaStream_t st);
+struct KqPlan;
+// y[i][..][row] (+)= matrix i (nmat of equal width, stacked) . token row.  plan == nullptr: rows 0 .. ntok - 1 of one matrix; else matrices of
+// rows_per_expert rows per expert against the plan's chunks, outputs at the plan's entries (by_entry) or at positions 32 chunk + i
+cudaError_t launch_kqt(const KqtMat *const *mats, float *const *ys_out, const int *ldy, int nmat, int rows_per_expert, const KqPlan *plan, int ne, int ntok, int topk,
+                       bool by_entry, const uint8_t *img, const float *ys, bool resid, DevState *state, bool pdl, cudaStream_t st);
+int kqt_max_chunks(int entries, int ne);
+cudaError_t launch_qr_plan(const int32_t *top, int ntok, int topk, int ne, KqPlan *plan, bool pdl, cudaStream_t st);
+cudaError_t launch_qr_gather(const KqPlan *plan, const uint8_t *img, const float *ys, int rows, int topk, int ne, int nsb, uint8_t *out, float *out_ys, bool pdl,
+                             cudaStream_t st);
 cudaError_t launch_qr_embed(const uint8_t *embd, int d, const uint32_t *toks, int rows, float *x, bool pdl, cudaStream_t st);
 // part (nullable): x[t] += sum over k of wts[8 t + k] part[t topk + k]; w (nullable): norm and image (ys: scales per superblock), normalised floats xn (nullable)
 cudaError_t launch_qr_norm(float *x, int rows, int d, const float *part, const float *wts, int topk, const float *w, float eps, float *xn, uint8_t *img, float *ys, bool pdl,
@@ -79,7 +84,7 @@ cudaError_t launch_qr_qknorm(float *q, const float *k, const float *v, const flo
                              int rows, float *kc, float *vc, bool pdl, cudaStream_t st);
 bool qr_attn_fits(int nh, int nkv);       // head groupings the row attention is written for
 cudaError_t launch_qr_attn(const float *q, const float *kc, const float *vc, int nh, int nkv, int pos0, int rows, uint8_t *img, float *ys, bool pdl, cudaStream_t st);
-cudaError_t launch_qr_glu(const float *g, const float *u, int entries, int ff, uint8_t *img, float *ys, bool pdl, cudaStream_t st);
+cudaError_t launch_qr_glu(const KqPlan *plan, const float *g, const float *u, int entries, int ne, int ff, uint8_t *img, float *ys, bool pdl, cudaStream_t st);
 void launch_qr_image(const float *x, int rows, int cols, uint8_t *img, float *ys, cudaStream_t st);
 // router of normalised token rows: logits [ntok][ne], routing [ntok][8]; counter: one zeroed word per four tokens
 cudaError_t launch_router_rows(const float *xn, int d, const float *Wt, const float *b, int ne, int topk, int ntok, float *logits, int32_t *top, float *wts,

@@ -1,18 +1,47 @@
 // K-quant matrices against token rows (kernels_kqt.cu): the activation image they read and the matrix handle.
 //
-// Activation image of a row, 544 bytes per superblock: 256 halves, then sixteen for the minima.  Halves: sub-block j (32 values) at
-// 64 j, in groups of eight values in the order 0 2 1 3 4 6 5 7 - the order in which two 32-bit masks pull a word's nibbles apart.
-// Minima: the eight 32-sums bs = 64 h + l with l in [-32, 31] as l[0..7], h[0..7] (both exact halves; a sum has 13 bits).
+// Activation images are written as operand B of the products, so that one bulk copy brings a superblock of up to 32 tokens.  Tokens
+// come in chunks of at most 32 (rows 32 c .. of a prompt tile, or tokens of one expert in the order of a KqPlan); a chunk of n has room
+// for kq_cap(n) tokens.  Block (chunk, superblock), KIMG_BLOCK bytes apart: [34 pieces][kq_cap(n) tokens][16 bytes].  Piece 4 j + i:
+// values 8 i .. 8 i + 7 of sub-block j (32 values) as halves in the order 0 2 1 3 4 6 5 7 - the order in which two 32-bit masks pull a
+// word's nibbles apart.  Pieces 32, 33: the eight 32-sums bs = 64 h + l, l in [-32, 31], as l[0..7] and h[0..7] (halves are exact up to
+// 2048, a sum has 13 bits).  The scales of block (chunk, superblock): 32 floats.
 #pragma once
 #include <cuda.h>
 #include "brrr_kq.cuh"
 
 namespace brrr {
 
-constexpr int KIMG_SB = 544;
+constexpr int KT_NT = 32;                                 // tokens per chunk
+constexpr int KIMG_BLOCK = 34 * KT_NT * 16;
+constexpr int KT_MAXCHUNK = 512;
+__host__ __device__ __forceinline__ int kq_cap(int n) { return n <= 8 ? 8 : n <= 16 ? 16 : KT_NT; }
+__host__ __device__ __forceinline__ size_t kimg_bytes(int chunks, int nsb) { return (size_t)chunks * nsb * KIMG_BLOCK; }
+
+// Tokens of every expert, cut into chunks: chunk c serves expert e[c] with n[c] entries (token * topk + slot) ent[32 c ..].
+struct KqPlan {
+    int nchunk;
+    int e[KT_MAXCHUNK], n[KT_MAXCHUNK];
+    int ent[KT_MAXCHUNK * KT_NT];
+};
+
+// where token `t` of a chunk keeps superblock sb
+struct KimgSlot {
+    uint8_t *p;      // its 16 bytes of piece 0
+    int step;        // bytes from piece to piece
+    float *ys;
+};
+__device__ __forceinline__ KimgSlot kimg_slot(uint8_t *img, float *ys, int chunk, int n, int i, int nsb, int sb) {
+    const size_t b = (size_t)chunk * nsb + sb;
+    return KimgSlot{img + b * KIMG_BLOCK + i * 16, kq_cap(n) * 16, ys + b * KT_NT + i};
+}
+// row t of a tile of `rows` rows
+__device__ __forceinline__ KimgSlot kimg_row(uint8_t *img, float *ys, int t, int rows, int nsb, int sb) {
+    return kimg_slot(img, ys, t / KT_NT, min(KT_NT, rows - t / KT_NT * KT_NT), t % KT_NT, nsb, sb);
+}
 
 // Q8_K quantisation of one superblock by one warp (the arithmetic of warp_quant_q8k), straight into the image.
-__device__ __forceinline__ void warp_quant_q8k_image(const float (&v)[8], int lane, uint8_t *img_sb, float *s) {
+__device__ __forceinline__ void warp_quant_q8k_image(const float (&v)[8], int lane, const KimgSlot &o) {
     float amax = 1e-12f;
 #pragma unroll
     for (int i = 0; i < 8; i++) amax = fmaxf(amax, fabsf(v[i]));
@@ -29,12 +58,12 @@ __device__ __forceinline__ void warp_quant_q8k_image(const float (&v)[8], int la
         const __half2 h = __halves2half2(__int2half_rn(q[order[2 * i]]), __int2half_rn(q[order[2 * i + 1]]));
         w[i] = *reinterpret_cast<const uint32_t *>(&h);
     }
-    *reinterpret_cast<uint4 *>(img_sb + lane * 16) = make_uint4(w[0], w[1], w[2], w[3]);
+    *reinterpret_cast<uint4 *>(o.p + lane * o.step) = make_uint4(w[0], w[1], w[2], w[3]);
     sum += __shfl_xor_sync(0xffffffffu, sum, 1);
     sum += __shfl_xor_sync(0xffffffffu, sum, 2);
     const int h = (sum + 32) >> 6, l = sum - 64 * h;
-    if ((lane & 3) < 2) *reinterpret_cast<__half *>(img_sb + 512 + (lane & 1) * 16 + 2 * (lane >> 2)) = __int2half_rn((lane & 1) ? h : l);
-    if (lane == 0) *s = sc;
+    if ((lane & 3) < 2) *reinterpret_cast<__half *>(o.p + (32 + (lane & 1)) * o.step + 2 * (lane >> 2)) = __int2half_rn((lane & 1) ? h : l);
+    if (lane == 0) *o.ys = sc;
 }
 
 // A matrix of 128-row tiles: its bytes as tensors [row][byte] for the copies (Q4_K: boxes of 128 x 144; Q6_K planes: 128 x 128, 64, 16).

@@ -50,9 +50,9 @@ extern "C" int brrr_kquant_rows(const uint8_t *d_w, int type, int rows, int cols
     if (((uintptr_t)d_w & 15) || ((uintptr_t)d_x & 15)) return BRRR_ERR_ARG;
     cudaStream_t st = (cudaStream_t)stream;
     KMatDev m{d_w, type, rows, cols, type == 14};
-    const size_t wb = type == 14 ? m.bpr() * rows : 0, nblk = (size_t)ntok * (cols / 256), ib = nblk * KIMG_SB;
+    const size_t wb = type == 14 ? m.bpr() * rows : 0, nblk = (size_t)(ntok + KT_NT - 1) / KT_NT * (cols / 256), ib = nblk * KIMG_BLOCK;
     uint8_t *buf = nullptr;
-    if (cudaMallocAsync(&buf, wb + ib + nblk * 4, st) != cudaSuccess) return BRRR_ERR_NOMEM;
+    if (cudaMallocAsync(&buf, wb + ib + nblk * KT_NT * 4, st) != cudaSuccess) return BRRR_ERR_NOMEM;
     uint8_t *img = buf + wb;
     float *ys = (float *)(img + ib);
     if (type == 14) { launch_q6k_planes(d_w, rows, cols, buf, st); m.p = buf; }
@@ -61,7 +61,7 @@ extern "C" int brrr_kquant_rows(const uint8_t *d_w, int type, int rows, int cols
     const KqtMat *mats[1] = {&t};
     float *out[1] = {d_y};
     cudaError_t e = kqt_matrix(m, rows, &t);
-    if (e == cudaSuccess) e = launch_kqt(mats, out, &rows, 1, 0, nullptr, nullptr, 1, ntok, 1, 1, img, ys, false, nullptr, false, st);
+    if (e == cudaSuccess) e = launch_kqt(mats, out, &rows, 1, 0, nullptr, 1, ntok, 1, false, img, ys, false, nullptr, false, st);
     cudaFreeAsync(buf, st);
     return e == cudaSuccess ? check_launch() : BRRR_ERR_CUDA;
 }

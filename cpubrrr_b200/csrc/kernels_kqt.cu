@@ -9,11 +9,12 @@
 //         (<= 8.4 M and 15.6 M), a = fma(16, Dh, Dl).
 // Then, per row and token, sum += (ys d) a - (ys dmin) mint in superblock order, every operation rounded as in q4k_row_dot.
 //
-// A CTA is persistent over (expert, up to 32 of its tokens, 128 rows) tasks.  Warp roles: one lane brings raw superblocks of the 128
-// rows (TMA boxes, 4 deep); eight warps widen them - thread = row and half superblock - into tensor memory, where operand A is read
-// from (128 rows x 256 halves would otherwise cross shared memory twice: 64 KB written and 64 KB read per superblock, the bound of the
-// layout with A in shared memory); two warps gather the tokens' images into operand B; one issues the products; eight warps - thread =
-// row and 16 tokens - read the accumulators and carry the float chain.  Operand A and the accumulators are double-buffered.
+// A CTA is persistent over (chunk of up to 32 tokens, 128 rows) tasks.  Warp roles: one lane brings raw superblocks of the 128 rows (TMA
+// boxes) and the chunk's image (bulk copies: gathered with 16-byte copies per token and piece instead, they filled the load/store
+// pipe and every wait and shared-memory read of the CTA with them: 2650 cycles per superblock); eight warps widen the weights - thread =
+// row and half superblock - into tensor memory, where operand A is read from (128 rows x 256 halves would otherwise cross shared
+// memory twice, 64 KB written and 64 KB read per superblock); one warp issues the products; eight warps - thread = row and 16 tokens -
+// read the accumulators and carry the float chain.  Operand A and the accumulators are double-buffered.
 #include "brrr_kernels.h"
 #include "brrr_kqt.cuh"
 #include "brrr_tc.cuh"
@@ -23,24 +24,23 @@ namespace brrr {
 
 namespace {
 
-constexpr int KT_ROWS = 128, KT_NT = 32;
+constexpr int KT_ROWS = 128;
 constexpr int KT_RAW = 28672, KT_RAW_DEPTH = 4;                // raw superblocks of 128 rows (Q4_K 18432, Q6_K 28672 bytes)
-constexpr int KT_B = 34 * KT_NT * 16, KT_B_DEPTH = 4;          // operand B of a superblock: [16-byte chunk][token] (the last two: minima)
-constexpr int KT_WARPS = 20, KT_THREADS = KT_WARPS * 32;       // 8 epilogue, 8 widening, 1 issuing, 1 raw copies, 2 images
-constexpr int KT_MAXCHUNK = 512;                               // chunks of tokens: entries / 32 + experts at most
+constexpr int KT_B_DEPTH = 4;                                  // operand B blocks
+constexpr int KT_WARPS = 18, KT_THREADS = KT_WARPS * 32;       // 8 epilogue, 8 widening, 1 issuing, 1 copies
 constexpr uint32_t KT_COL_A = 192, KT_COL_MIN = 448;           // tensor memory columns: 2 x 3 x 32 accumulators, 2 halves x 2 x 64, 2 x 8
-constexpr size_t KT_SMEM = (size_t)KT_RAW * KT_RAW_DEPTH + (size_t)KT_B * KT_B_DEPTH + 1024;
+constexpr size_t KT_SMEM = (size_t)KT_RAW * KT_RAW_DEPTH + (size_t)KIMG_BLOCK * KT_B_DEPTH + 1024;
 
 struct alignas(64) KqtArgs {
     KqtMat m[3];             // stacked matrices of equal width
-    float *y[3];             // outputs [entry][ldy] (+ row of the matrix)
+    float *y[3];             // outputs [entry or position][ldy] (+ row of the matrix)
     int ldy[3];
     int tile_end[3];         // running number of 128-row tiles of one expert
-    int nmat, tiles, nsb;
-    const int *cnt, *list;   // entries per expert, [ne][512] entry ids; cnt == nullptr: one matrix, entries 0 .. ntok - 1
-    int ne, ntok, src_div, resid;
-    const uint8_t *img;      // images [entry / src_div][nsb * 544]
-    const float *ys;         // scales [entry / src_div][nsb]
+    int tiles, nsb;
+    const KqPlan *plan;      // nullptr: one matrix, rows 0 .. ntok - 1
+    int ntok, resid, by_entry;      // by_entry: outputs go to the plan's entries, else to positions 32 chunk + i
+    const uint8_t *img;
+    const float *ys;
     DevState *state;
 };
 
@@ -113,84 +113,89 @@ constexpr uint32_t H2_1024 = 0x64006400u, H2_1032 = 0x64086408u, H2_SIXTEENTH = 
 // byte j of w (below 64) as a pair of equal halves 1024 + byte
 __device__ __forceinline__ uint32_t h2_byte(uint32_t w, int j) { return __byte_perm(w, 0x64u, 0x4040u | (uint32_t)j | ((uint32_t)j << 8)); }
 
-// one task: expert, first entry and number of entries of its chunk, 128-row tile of the stack
-struct KtTask { int e, first, n, mi, row; };      // row: of the expert's matrix mi
+// one task: chunk of tokens, 128-row tile of the stack
+struct KtTask { int chunk, e, n, mi, row; };      // row: of the expert's matrix mi
 
 __global__ void __launch_bounds__(KT_THREADS, 1) kqt_kernel(const __grid_constant__ KqtArgs a) {
     extern __shared__ unsigned char ksm_[];
     unsigned char *raw = ksm_ + ((1024u - (smem_u32(ksm_) & 1023u)) & 1023u);          // swizzled copies want 1024-byte alignment
     unsigned char *bsm = raw + KT_RAW * KT_RAW_DEPTH;
-    __shared__ __align__(8) uint64_t rfull[KT_RAW_DEPTH], rempty[KT_RAW_DEPTH], bfull[KT_B_DEPTH], bempty[KT_B_DEPTH], afull[2][2], aempty[2][2], dfull[2], dempty[2];
-    __shared__ float2 drow[4][KT_ROWS];              // d, dmin of the rows, four superblocks deep
+    // rfull / rempty: raw slot; bfull: B slot; afull: a half's operand (two stages); half0[n & 3]: the first half of superblock n has been
+    // read; done[n & 3]: all of it, its block of B, and the accumulators are complete; dempty: they have been read
+    __shared__ __align__(8) uint64_t rfull[KT_RAW_DEPTH], rempty[KT_RAW_DEPTH], bfull[KT_B_DEPTH], afull[2][2], half0[4], done[4], dempty[2];
+    __shared__ float2 drow[4][KT_ROWS];              // d, dmin of the rows; written once the accumulators of four superblocks before have been read
     __shared__ __align__(16) float ysr[8][KT_NT];    // activation scales, eight superblocks deep
-    __shared__ int chunk_e[KT_MAXCHUNK], chunk_fn[KT_MAXCHUNK], nchunk_sh;      // fn: first | entries << 16
+    __shared__ short chunk_e[KT_MAXCHUNK], chunk_n[KT_MAXCHUNK];
     __shared__ uint32_t tmem_sh;
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, nsb = a.nsb;
     if (tid == 0) {
         for (int i = 0; i < KT_RAW_DEPTH; i++) { mbar_init(&rfull[i], 1); mbar_init(&rempty[i], 8); }
-        for (int i = 0; i < KT_B_DEPTH; i++) { mbar_init(&bfull[i], 64); mbar_init(&bempty[i], 1); }
-        for (int i = 0; i < 2; i++) {
-            mbar_init(&afull[0][i], 4); mbar_init(&afull[1][i], 4); mbar_init(&aempty[0][i], 1); mbar_init(&aempty[1][i], 1);
-            mbar_init(&dfull[i], 2); mbar_init(&dempty[i], 8);
-        }
+        for (int i = 0; i < KT_B_DEPTH; i++) mbar_init(&bfull[i], 1);
+        for (int i = 0; i < 4; i++) { mbar_init(&half0[i], 1); mbar_init(&done[i], 2); }
+        for (int i = 0; i < 2; i++) { mbar_init(&afull[0][i], 4); mbar_init(&afull[1][i], 4); mbar_init(&dempty[i], 8); }
         mbar_fence_init();
     }
     if (warp == 1) {
         asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(&tmem_sh)), "r"(512u) : "memory");
         asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
     }
-    if (a.cnt) pdl_wait();       // the chunks depend on the routing; a single matrix's weights do not
-    if (warp == 0) {
-        // chunks: experts in order, ceil(entries / 32) each, of equal size in whole groups of sixteen
-        const int per = a.cnt ? (a.ne + 31) / 32 : 1, e0 = lane * per;
-        int c[8], mine = 0;
-#pragma unroll
-        for (int i = 0; i < 8; i++) {
-            c[i] = 0;
-            if (i < per) c[i] = a.cnt ? (e0 + i < a.ne ? a.cnt[e0 + i] : 0) : (lane == 0 ? a.ntok : 0);
-            mine += (c[i] + KT_NT - 1) / KT_NT;
-        }
-        int incl = mine;
-#pragma unroll
-        for (int o = 1; o < 32; o <<= 1) { const int v = __shfl_up_sync(0xffffffffu, incl, o); if (lane >= o) incl += v; }
-        int at = incl - mine;
-#pragma unroll
-        for (int i = 0; i < 8; i++) {
-            const int n = (c[i] + KT_NT - 1) / KT_NT, step = n ? ((c[i] + n - 1) / n + 15) & ~15 : 0;
-            for (int k = 0; k < n; k++, at++)
-                if (at < KT_MAXCHUNK) { chunk_e[at] = e0 + i; chunk_fn[at] = (k * step) | (max(min(step, c[i] - k * step), 0) << 16); }
-        }
-        if (lane == 31) nchunk_sh = min(incl, KT_MAXCHUNK);
+    int nchunk = (a.ntok + KT_NT - 1) / KT_NT;
+    if (a.plan) {                // the chunks depend on the routing; a single matrix's weights do not
+        pdl_wait();
+        nchunk = min(a.plan->nchunk, KT_MAXCHUNK);
+        for (int i = tid; i < nchunk; i += KT_THREADS) { chunk_e[i] = (short)a.plan->e[i]; chunk_n[i] = (short)a.plan->n[i]; }
     }
     tl_fence_before();
     __syncthreads();
     tl_fence_after();
     pdl_trigger();
     const uint32_t tmem = tmem_sh;
-    const int ntask = nchunk_sh * a.tiles;
+    const int ntask = nchunk * a.tiles;
     TlWaiter wait{a.state ? &a.state->err : nullptr, a.state && *reinterpret_cast<volatile uint32_t *>(&a.state->err) != 0u};
     auto task = [&](int t) {
         KtTask k;
-        const int ch = t / a.tiles, tile = t % a.tiles;
-        k.e = chunk_e[ch]; k.first = chunk_fn[ch] & 0xFFFF; k.n = chunk_fn[ch] >> 16;
+        k.chunk = t / a.tiles;
+        const int tile = t - k.chunk * a.tiles;
+        k.e = a.plan ? chunk_e[k.chunk] : 0;
+        k.n = a.plan ? chunk_n[k.chunk] : min(KT_NT, a.ntok - k.chunk * KT_NT);
         k.mi = 0;
         while (tile >= a.tile_end[k.mi]) k.mi++;
         k.row = (tile - (k.mi ? a.tile_end[k.mi - 1] : 0)) * KT_ROWS;
         return k;
     };
+    // parity with which superblock n - back released its stages
+    auto released = [](int n, int back) { return (uint32_t)((n - back) >> 2) & 1u; };
     const uint32_t raw0 = smem_u32(raw), b0 = smem_u32(bsm);
 
     if (warp == 17) {
-        // ---------------- raw superblocks of the rows
+        // ---------------- copies: raw superblocks of the rows, the chunk's block of operand B, its scales
         if (lane == 0) {
             int n = 0;
+            bool waited = a.plan != nullptr;
             for (int t = blockIdx.x; t < ntask; t += gridDim.x) {
                 const KtTask k = task(t);
                 const KqtMat &m = a.m[k.mi];
                 const int row = k.e * (a.tile_end[k.mi] - (k.mi ? a.tile_end[k.mi - 1] : 0)) * KT_ROWS + k.row;
+                const uint32_t bytes = (m.type == 12 ? 34u : 32u) * kq_cap(k.n) * 16;
+                auto brings_b = [&](int sb, int nn) {
+                    const int slot = nn % KT_B_DEPTH;
+                    if (nn >= KT_B_DEPTH) wait(&done[(nn - KT_B_DEPTH) & 3], released(nn, KT_B_DEPTH));
+                    const size_t blk = (size_t)k.chunk * nsb + sb;
+                    mbar_expect_tx(&bfull[slot], bytes + KT_NT * 4);
+                    bulk_g2s(bsm + slot * KIMG_BLOCK, a.img + blk * KIMG_BLOCK, bytes, &bfull[slot]);
+                    bulk_g2s(&ysr[nn & 7][0], a.ys + blk * KT_NT, KT_NT * 4, &bfull[slot]);
+                };
+                const int first = n;
+                int held = 0;                          // blocks of B not requested yet: the kernel before may still be writing the image
                 for (int sb = 0; sb < nsb; sb++, n++) {
                     const int slot = n % KT_RAW_DEPTH;
-                    wait(&rempty[slot], ((n / KT_RAW_DEPTH) & 1) ^ 1);
+                    if (!waited && n >= min(KT_RAW_DEPTH, nsb)) {
+                        pdl_wait();
+                        waited = true;
+                        for (int h = 0; h < held; h++) brings_b(h, first + h);
+                        held = 0;
+                    }
+                    if (n >= KT_RAW_DEPTH) wait(&rempty[slot], ((n / KT_RAW_DEPTH) & 1) ^ 1);
                     const uint32_t dst = raw0 + slot * KT_RAW;
                     if (m.type == 12) {
                         mbar_expect_tx(&rfull[slot], KT_ROWS * 144);
@@ -202,108 +207,75 @@ __global__ void __launch_bounds__(KT_THREADS, 1) kqt_kernel(const __grid_constan
                         kt_box(dst + 24576, &m.map[2], nsb * 192 + sb * 16, row, &rfull[slot]);
                         kt_box(dst + 26624, &m.map[2], nsb * 208 + (sb & ~7) * 2, row, &rfull[slot]);
                     }
+                    if (waited) brings_b(sb, n);
+                    else held++;
+                }
+                if (!waited) {                         // nsb <= KT_RAW_DEPTH
+                    pdl_wait();
+                    waited = true;
+                    for (int h = 0; h < held; h++) brings_b(h, first + h);
                 }
             }
         }
-    } else if (warp >= 18) {
-        // ---------------- images of the tokens: lane = (token of a group of eight, 16-byte chunk of four); the two warps take alternate groups
-        if (!a.cnt) pdl_wait();
-        const int lw = warp - 18, tok8 = lane >> 2, c4 = lane & 3;
-        int n = 0;
-        for (int t = blockIdx.x; t < ntask; t += gridDim.x) {
-            const KtTask k = task(t);
-            const int quads = a.m[k.mi].type == 12 ? 9 : 8;
-            const uint8_t *src[2];
-            bool live[2];
-#pragma unroll
-            for (int g = 0; g < 2; g++) {
-                const int i = (2 * g + lw) * 8 + tok8;
-                live[g] = i < k.n;
-                const int ent = live[g] ? (a.list ? a.list[k.e * BRRR_TILE_MAX + k.first + i] : k.first + i) : 0;
-                src[g] = a.img + (size_t)(ent / a.src_div) * nsb * KIMG_SB + c4 * 16;
-            }
-            const float *ysrc = a.ys + (size_t)((lane < k.n ? (a.list ? a.list[k.e * BRRR_TILE_MAX + k.first + lane] : k.first + lane) : 0) / a.src_div) * nsb;
-            for (int sb = 0; sb < nsb; sb++, n++) {
-                const int slot = n % KT_B_DEPTH;
-                wait(&bempty[slot], ((n / KT_B_DEPTH) & 1) ^ 1);
-                const uint32_t dst = b0 + slot * KT_B + lw * 128 + tok8 * 16 + c4 * (KT_NT * 16);
-#pragma unroll
-                for (int g = 0; g < 2; g++) {
-                    if (live[g]) {
-#pragma unroll
-                        for (int q = 0; q < 8; q++) cp_async16(dst + g * 256 + q * 4 * (KT_NT * 16), src[g] + q * 64);
-                        if (quads == 9 && c4 < 2) cp_async16(dst + g * 256 + 32 * (KT_NT * 16), src[g] + 512);
-                    }
-                    src[g] += KIMG_SB;
-                }
-                if (lw == 0 && lane < k.n)
-                    asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"(smem_u32(&ysr[n & 7][lane])), "l"(ysrc + sb) : "memory");
-                cp_async_arrive(&bfull[slot]);
-            }
-        }
-        asm volatile("cp.async.wait_all;" ::: "memory");
     } else if (warp == 16) {
         // ---------------- products (the whole warp walks the loop, an elected lane issues)
         int n = 0, ca = 0;
-        const uint64_t db0 = tl_smem_desc(bsm, KT_NT * 16, 128);
         for (int t = blockIdx.x; t < ntask; t += gridDim.x) {
             const KtTask k = task(t);
             const bool q4 = a.m[k.mi].type == 12;
-            const uint32_t idesc = (1u << 4) | ((uint32_t)(2 * ((k.n + 15) >> 4)) << 17) | ((KT_ROWS >> 4) << 24);      // f32 += f16 x f16, N = 16 or 32
+            const int cap = kq_cap(k.n);
+            const uint32_t idesc = (1u << 4) | ((uint32_t)(k.n > 16 ? 4 : 2) << 17) | ((KT_ROWS >> 4) << 24);      // f32 += f16 x f16, N = 16 or 32
+            const uint64_t db0 = tl_smem_desc(bsm, cap * 16, cap == 8 ? 0 : 128);      // room for eight: both groups of eight columns read them
             for (int sb = 0; sb < nsb; sb++, n++) {
                 const int slot = n % KT_B_DEPTH, buf = n & 1;
                 wait(&bfull[slot], (n / KT_B_DEPTH) & 1);
-                fence_proxy_async();                   // the copies seen through bfull[] (generic proxy) -> the tensor core's reads
                 wait(&dempty[buf], ((n >> 1) & 1) ^ 1);
-                const uint64_t db = db0 + (uint64_t)(slot * (KT_B / 16));
+                const uint64_t db = db0 + (uint64_t)(slot * (KIMG_BLOCK / 16));
                 const uint32_t d = tmem + buf * 96;
                 if (q4) {
+                    const int ab = ca & 1;
 #pragma unroll
                     for (int g = 0; g < 2; g++) {
-                        const int ab = ca & 1;
                         wait(&afull[g][ab], (ca >> 1) & 1);
                         tl_fence_after();
                         if (elect_one()) {
 #pragma unroll
-                            for (int s = 0; s < 8; s++)
-                                kt_mma(d + g * 32, tmem + KT_COL_A + (g * 2 + ab) * 64 + s * 8, db + (g * 8 + s) * (2 * KT_NT), idesc, s > 0);
-                            if (g == 1) kt_mma(d + 64, tmem + KT_COL_MIN + ab * 8, db + 16 * (2 * KT_NT), idesc, 0);
-                            tl_commit(&aempty[g][ab]);
+                            for (int s = 0; s < 8; s++) kt_mma(d + g * 32, tmem + KT_COL_A + (g * 2 + ab) * 64 + s * 8, db + (g * 8 + s) * 2 * cap, idesc, s > 0);
+                            if (g == 1) kt_mma(d + 64, tmem + KT_COL_MIN + ab * 8, db + 32 * cap, idesc, 0);
+                            tl_commit(g == 0 ? &half0[n & 3] : &done[n & 3]);
+                            if (g == 1) mbar_arrive(&done[n & 3]);      // orders drow and ysr, seen through afull and bfull, before the readers
                         }
                         __syncwarp();
                     }
                     ca++;
                 } else {
 #pragma unroll
-                    for (int g = 0; g < 2; g++)
+                    for (int g = 0; g < 2; g++) {
 #pragma unroll
-                        for (int dig = 0; dig < 2; dig++) {
-                            const int ab = (ca + dig) & 1;
-                            wait(&afull[g][ab], ((ca + dig) >> 1) & 1);
-                            tl_fence_after();
-                            if (elect_one()) {
+                        for (int dig = 0; dig < 2; dig++) wait(&afull[g][(ca + dig) & 1], ((ca + dig) >> 1) & 1);
+                        tl_fence_after();
+                        if (elect_one()) {
+#pragma unroll
+                            for (int dig = 0; dig < 2; dig++)
 #pragma unroll
                                 for (int s = 0; s < 8; s++)
-                                    kt_mma(d + dig * 32, tmem + KT_COL_A + (g * 2 + ab) * 64 + s * 8, db + (g * 8 + s) * (2 * KT_NT), idesc, g > 0 || s > 0);
-                                tl_commit(&aempty[g][ab]);
-                            }
-                            __syncwarp();
+                                    kt_mma(d + dig * 32, tmem + KT_COL_A + (g * 2 + ((ca + dig) & 1)) * 64 + s * 8, db + (g * 8 + s) * 2 * cap, idesc, g > 0 || s > 0);
+                            tl_commit(g == 0 ? &half0[n & 3] : &done[n & 3]);
+                            if (g == 1) mbar_arrive(&done[n & 3]);
                         }
+                        __syncwarp();
+                    }
                     ca += 2;
                 }
-                if (elect_one()) {
-                    tl_commit(&bempty[slot]);
-                    tl_commit(&dfull[buf]);
-                    mbar_arrive(&dfull[buf]);          // orders drow and ysr, seen through afull and bfull, before the readers
-                }
-                __syncwarp();
             }
         }
     } else if (warp >= 8) {
         // ---------------- widening: thread = row m, half g of the superblock
         const int g = (warp - 8) >> 2, m = (warp & 3) * 32 + lane;
         const uint32_t arow = tmem + ((uint32_t)((warp & 3) * 32) << 16);
+        uint64_t *const rel = g == 0 ? half0 : done;
         int n = 0, ca = 0;
+        bool both = false;                             // the superblock before took both stages of this half (Q6_K)
         for (int t = blockIdx.x; t < ntask; t += gridDim.x) {
             const KtTask k = task(t);
             const bool q4 = a.m[k.mi].type == 12;
@@ -319,12 +291,14 @@ __global__ void __launch_bounds__(KT_THREADS, 1) kqt_kernel(const __grid_constan
                         const uint4 v = lds128(src + m * 144 + 16 + g * 64 + i * 16);
                         w[4 * i] = v.x; w[4 * i + 1] = v.y; w[4 * i + 2] = v.z; w[4 * i + 3] = v.w;
                     }
-                    if (g == 0) drow[n & 3][m] = make_float2(half_bits_to_f32(h.x & 0xffffu), half_bits_to_f32(h.x >> 16));
                     __syncwarp();
                     if (lane == 0) mbar_arrive(&rempty[slot]);
                     const int ab = ca & 1;
-                    wait(&aempty[g][ab], ((ca >> 1) & 1) ^ 1);
+                    const int back = both ? 1 : 2;
+                    if (n >= back) wait(&rel[(n - back) & 3], released(n, back));
+                    both = false;
                     ca++;
+                    if (g == 0) drow[n & 3][m] = make_float2(half_bits_to_f32(h.x & 0xffffu), half_bits_to_f32(h.x >> 16));
                     tl_fence_after();
                     const uint32_t dst = arow + KT_COL_A + (g * 2 + ab) * 64;
                     // 6-bit scales of sub-blocks 4g .. 4g + 3
@@ -371,16 +345,14 @@ __global__ void __launch_bounds__(KT_THREADS, 1) kqt_kernel(const __grid_constan
                         qh[4 * i] = vh.x; qh[4 * i + 1] = vh.y; qh[4 * i + 2] = vh.z; qh[4 * i + 3] = vh.w;
                     }
                     const uint2 scw = lds64(src + 24576 + m * 16 + g * 8);
-                    if (g == 0) {
-                        const uint32_t dw = lds32(src + 26624 + m * 16 + (sb & 6) * 2);
-                        drow[n & 3][m] = make_float2(half_bits_to_f32((sb & 1) ? dw >> 16 : dw & 0xffffu), 0.0f);
-                    }
+                    const uint32_t dw = lds32(src + 26624 + m * 16 + (sb & 6) * 2);
                     __syncwarp();
                     if (lane == 0) mbar_arrive(&rempty[slot]);
                     const int a0 = ca & 1, a1 = a0 ^ 1;
-                    wait(&aempty[g][a0], ((ca >> 1) & 1) ^ 1);
-                    wait(&aempty[g][a1], (((ca + 1) >> 1) & 1) ^ 1);
+                    if (n >= 1) wait(&rel[(n - 1) & 3], released(n, 1));
+                    both = true;
                     ca += 2;
+                    if (g == 0) drow[n & 3][m] = make_float2(half_bits_to_f32((sb & 1) ? dw >> 16 : dw & 0xffffu), 0.0f);
                     tl_fence_after();
                     const uint32_t d0 = arow + KT_COL_A + (g * 2 + a0) * 64, d1 = arow + KT_COL_A + (g * 2 + a1) * 64;
 #pragma unroll
@@ -416,7 +388,7 @@ __global__ void __launch_bounds__(KT_THREADS, 1) kqt_kernel(const __grid_constan
         }
     } else {
         // ---------------- accumulators and the float chain: thread = row m, tokens 16 wg .. + 15
-        if (!a.cnt) pdl_wait();
+        if (!a.plan) pdl_wait();
         const int wg = warp >> 2, m = (warp & 3) * 32 + lane;
         const uint32_t lane_addr = tmem + ((uint32_t)((warp & 3) * 32) << 16) + wg * 16;
         int n = 0;
@@ -424,13 +396,13 @@ __global__ void __launch_bounds__(KT_THREADS, 1) kqt_kernel(const __grid_constan
             const KtTask k = task(t);
             const bool q4 = a.m[k.mi].type == 12, live = wg * 16 < k.n;
             const int ti = wg * 16 + (lane & 15);
-            const int ent = ti < k.n ? (a.list ? a.list[k.e * BRRR_TILE_MAX + k.first + ti] : k.first + ti) : 0;
+            const int ent = ti < k.n ? (a.by_entry ? a.plan->ent[k.chunk * KT_NT + ti] : k.chunk * KT_NT + ti) : 0;
             f32x2 acc[8];
 #pragma unroll
             for (int i = 0; i < 8; i++) acc[i] = 0ull;
             for (int sb = 0; sb < nsb; sb++, n++) {
                 const int buf = n & 1;
-                wait(&dfull[buf], (n >> 1) & 1);
+                wait(&done[n & 3], (n >> 2) & 1);
                 if (!live) {
                     __syncwarp();
                     if (lane == 0) mbar_arrive(&dempty[buf]);
@@ -513,25 +485,27 @@ cudaError_t kqt_matrix(const KMatDev &m, size_t rows_total, KqtMat *out) {
     return cudaSuccess;
 }
 
-cudaError_t launch_kqt(const KqtMat *const *mats, float *const *ys_out, const int *ldy, int nmat, int rows_per_expert, const int *cnt, const int *list, int ne, int ntok,
-                       int topk, int src_div, const uint8_t *img, const float *ys, bool resid, DevState *state, bool pdl, cudaStream_t st) {
-    const int entries = cnt ? ntok * topk : ntok;
-    if (nmat < 1 || nmat > 3 || ntok < 1 || ntok > BRRR_TILE_MAX || entries / KT_NT + (cnt ? ne : 1) > KT_MAXCHUNK || (cnt && ne > 256)) return cudaErrorInvalidValue;
+// Tasks are known on the host up to the number of chunks an expert's tokens fall into: at most one partly filled per expert, and never
+// more than entries.
+int kqt_max_chunks(int entries, int ne) { return entries / KT_NT + ne < entries ? entries / KT_NT + ne : entries; }
+
+cudaError_t launch_kqt(const KqtMat *const *mats, float *const *ys_out, const int *ldy, int nmat, int rows_per_expert, const KqPlan *plan, int ne, int ntok, int topk,
+                       bool by_entry, const uint8_t *img, const float *ys, bool resid, DevState *state, bool pdl, cudaStream_t st) {
+    const int chunks = plan ? kqt_max_chunks(ntok * topk, ne) : (ntok + KT_NT - 1) / KT_NT;
+    if (nmat < 1 || nmat > 3 || ntok < 1 || ntok > BRRR_TILE_MAX || chunks > KT_MAXCHUNK || ne > 256) return cudaErrorInvalidValue;
     KqtArgs a{};
     int tiles = 0;
     for (int i = 0; i < nmat; i++) {
-        const int rows = cnt ? rows_per_expert : mats[i]->rows;
+        const int rows = plan ? rows_per_expert : mats[i]->rows;
         if (mats[i]->cols != mats[0]->cols || rows % KT_ROWS) return cudaErrorInvalidValue;
         a.m[i] = *mats[i]; a.y[i] = ys_out[i]; a.ldy[i] = ldy[i];
         a.tile_end[i] = tiles += rows / KT_ROWS;
     }
-    a.nmat = nmat; a.tiles = tiles; a.nsb = mats[0]->cols / 256; a.cnt = cnt; a.list = list; a.ne = ne; a.ntok = ntok; a.src_div = src_div; a.resid = resid;
+    a.tiles = tiles; a.nsb = mats[0]->cols / 256; a.plan = plan; a.ntok = ntok; a.resid = resid; a.by_entry = plan && by_entry;
     a.img = img; a.ys = ys; a.state = state;
     static unsigned long long configured = 0;      // one bit per device
     cudaError_t e = smem_optin(kqt_kernel, (int)KT_SMEM, configured);
     if (e != cudaSuccess) return e;
-    // chunks of tokens: at most one partly filled per expert, and never more than entries
-    const int chunks = cnt ? (entries / KT_NT + ne < entries ? entries / KT_NT + ne : entries) : (ntok + KT_NT - 1) / KT_NT;
     const int tasks = chunks * tiles;
     return launch_k(kqt_kernel, dim3(tasks < 148 ? tasks : 148), dim3(KT_THREADS), KT_SMEM, st, pdl, a);
 }

@@ -95,7 +95,7 @@ __global__ void __launch_bounds__(256) qr_norm_kernel(QrNormArgs a) {
             dst[0] = make_float4(v[0], v[1], v[2], v[3]);
             dst[1] = make_float4(v[4], v[5], v[6], v[7]);
         }
-        warp_quant_q8k_image(v, lane, a.img + ((size_t)t * nsb + sb) * KIMG_SB, a.ys + (size_t)t * nsb + sb);
+        warp_quant_q8k_image(v, lane, kimg_row(a.img, a.ys, t, gridDim.x, nsb, sb));
     }
 }
 
@@ -305,34 +305,114 @@ __global__ void __launch_bounds__(QA_THREADS) qr_attn_kernel(QaArgs a) {
         if (rr >= nrows) break;
         const float4 v0 = reinterpret_cast<const float4 *>(qs)[u * 64 + lane * 2], v1 = reinterpret_cast<const float4 *>(qs)[u * 64 + lane * 2 + 1];
         const float v[8] = {v0.x, v0.y, v0.z, v0.w, v1.x, v1.y, v1.z, v1.w};
-        const size_t sb = (size_t)(r0 + rr) * (a.nh / 2) + (kvh * group + 2 * u % group) / 2;
-        warp_quant_q8k_image(v, lane, a.img + sb * KIMG_SB, a.ys + sb);
+        warp_quant_q8k_image(v, lane, kimg_row(a.img, a.ys, r0 + rr, a.rows, a.nh / 2, (kvh * group + 2 * u % group) / 2));
+    }
+}
+
+// ---------------------------------------------------------------- tokens of every expert, in chunks
+// One CTA.  Counts, the chunks (experts in order; ceil(entries / 32) each, of equal size in whole groups of eight), then every entry to
+// the next free place of its expert.  Which of an expert's places an entry takes changes no result: entries do not meet before the
+// combine, which goes by token and slot.
+__global__ void __launch_bounds__(1024) qr_plan_kernel(const int32_t *__restrict__ top, int ntok, int topk, int ne, KqPlan *__restrict__ plan) {
+    __shared__ int cnt[256], chunk0[256], step[256], fill[256], wsum[8];
+    const int tid = threadIdx.x, lane = tid & 31;
+    if (tid < 256) { cnt[tid] = 0; fill[tid] = 0; }
+    __syncthreads();
+    pdl_wait();
+    pdl_trigger();
+    int mine[(BRRR_TILE_MAX * 8 + 1023) / 1024];
+#pragma unroll
+    for (int k = 0; k < BRRR_TILE_MAX * 8 / 1024; k++) {
+        const int i = tid + k * 1024, t = i >> 3, s = i & 7;
+        mine[k] = t < ntok && s < topk ? top[i] : -1;
+        if (mine[k] >= 0) atomicAdd(&cnt[mine[k]], 1);
+    }
+    __syncthreads();
+    int c = 0, nc = 0, incl = 0;
+    if (tid < 256) {
+        c = tid < ne ? cnt[tid] : 0;
+        nc = (c + KT_NT - 1) / KT_NT;
+        incl = nc;
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) { const int v = __shfl_up_sync(0xffffffffu, incl, o); if (lane >= o) incl += v; }
+        if (lane == 31) wsum[tid >> 5] = incl;
+    }
+    __syncthreads();
+    if (tid < 256) {
+        for (int w = 0; w < (tid >> 5); w++) incl += wsum[w];
+        const int at = incl - nc, st = nc ? ((c + nc - 1) / nc + 7) & ~7 : 0;
+        chunk0[tid] = at; step[tid] = st;
+        for (int k = 0; k < nc; k++)
+            if (at + k < KT_MAXCHUNK) { plan->e[at + k] = tid; plan->n[at + k] = max(min(st, c - k * st), 0); }
+        if (tid == 255) plan->nchunk = min(incl, KT_MAXCHUNK);
+    }
+    __syncthreads();
+#pragma unroll
+    for (int k = 0; k < BRRR_TILE_MAX * 8 / 1024; k++) {
+        const int i = tid + k * 1024, e = mine[k];
+        if (e < 0) continue;
+        const int p = atomicAdd(&fill[e], 1), ch = chunk0[e] + p / step[e];
+        if (ch < KT_MAXCHUNK) plan->ent[ch * KT_NT + p % step[e]] = (i >> 3) * topk + (i & 7);
+    }
+}
+
+// images of the rows -> images of the chunks: a CTA per (chunk, superblock) at a time
+__global__ void __launch_bounds__(256) qr_gather_kernel(const KqPlan *__restrict__ plan, const uint8_t *__restrict__ img, const float *__restrict__ ys, int rows, int topk,
+                                                        int nsb, uint8_t *__restrict__ out, float *__restrict__ out_ys) {
+    __shared__ int src[KT_NT];
+    const int tid = threadIdx.x;
+    pdl_wait();
+    pdl_trigger();
+    const int total = plan->nchunk * nsb;
+    for (int u = blockIdx.x; u < total; u += gridDim.x) {
+        const int ch = u / nsb, sb = u % nsb, n = plan->n[ch], cap = kq_cap(n), lg = cap == 8 ? 3 : cap == 16 ? 4 : 5;
+        if (tid < n) {
+            const int t = plan->ent[ch * KT_NT + tid] / topk;
+            src[tid] = t;
+            out_ys[(size_t)u * KT_NT + tid] = ys[((size_t)(t / KT_NT) * nsb + sb) * KT_NT + t % KT_NT];
+        }
+        __syncthreads();
+        for (int i = tid; i < 34 << lg; i += 256) {
+            const int piece = i >> lg, k = i & (cap - 1);
+            if (k < n) {
+                const int t = src[k], c0 = t / KT_NT, step = kq_cap(min(KT_NT, rows - c0 * KT_NT)) * 16;
+                *reinterpret_cast<uint4 *>(out + (size_t)u * KIMG_BLOCK + i * 16) =
+                    *reinterpret_cast<const uint4 *>(img + ((size_t)c0 * nsb + sb) * KIMG_BLOCK + piece * step + (t % KT_NT) * 16);
+            }
+        }
+        __syncthreads();
     }
 }
 
 // ---------------------------------------------------------------- SiLU-GLU and Q8_K of h (engine_qwen2.rs:419-431): one warp per superblock
-__global__ void __launch_bounds__(256) qr_glu_kernel(const float *__restrict__ g, const float *__restrict__ u, int nblk, uint8_t *__restrict__ img, float *__restrict__ ys) {
-    const int sb = blockIdx.x * 8 + (threadIdx.x >> 5), lane = threadIdx.x & 31;
+// of a position (32 chunk + i); g, u: [position][ff]
+__global__ void __launch_bounds__(256) qr_glu_kernel(const KqPlan *__restrict__ plan, const float *__restrict__ g, const float *__restrict__ u, int nsb,
+                                                     uint8_t *__restrict__ img, float *__restrict__ ys) {
+    const int lane = threadIdx.x & 31;
     pdl_wait();
     pdl_trigger();
-    if (sb >= nblk) return;
-    const float4 *gp = reinterpret_cast<const float4 *>(g + (size_t)sb * 256 + lane * 8), *up = reinterpret_cast<const float4 *>(u + (size_t)sb * 256 + lane * 8);
-    const float4 g0 = gp[0], g1 = gp[1], u0 = up[0], u1 = up[1];
-    const float gv[8] = {g0.x, g0.y, g0.z, g0.w, g1.x, g1.y, g1.z, g1.w}, uv[8] = {u0.x, u0.y, u0.z, u0.w, u1.x, u1.y, u1.z, u1.w};
-    float h[8];
+    const int total = plan->nchunk * KT_NT * nsb;
+    for (int w = blockIdx.x * 8 + (threadIdx.x >> 5); w < total; w += gridDim.x * 8) {
+        const int pos = w / nsb, sb = w % nsb, ch = pos / KT_NT, i = pos % KT_NT, n = plan->n[ch];
+        if (i >= n) continue;
+        const float4 *gp = reinterpret_cast<const float4 *>(g + (size_t)w * 256 + lane * 8), *up = reinterpret_cast<const float4 *>(u + (size_t)w * 256 + lane * 8);
+        const float4 g0 = gp[0], g1 = gp[1], u0 = up[0], u1 = up[1];
+        const float gv[8] = {g0.x, g0.y, g0.z, g0.w, g1.x, g1.y, g1.z, g1.w}, uv[8] = {u0.x, u0.y, u0.z, u0.w, u1.x, u1.y, u1.z, u1.w};
+        float h[8];
 #pragma unroll
-    for (int i = 0; i < 8; i++) h[i] = __fmul_rn(__fdiv_rn(gv[i], __fadd_rn(1.0f, brrr_expf_dev(-gv[i]))), uv[i]);
-    warp_quant_q8k_image(h, lane, img + (size_t)sb * KIMG_SB, ys + sb);
+        for (int k = 0; k < 8; k++) h[k] = __fmul_rn(__fdiv_rn(gv[k], __fadd_rn(1.0f, brrr_expf_dev(-gv[k]))), uv[k]);
+        warp_quant_q8k_image(h, lane, kimg_slot(img, ys, ch, n, i, nsb, sb));
+    }
 }
 
 // rows of floats -> images
-__global__ void __launch_bounds__(256) qr_image_kernel(const float *__restrict__ x, int nblk, uint8_t *__restrict__ img, float *__restrict__ ys) {
-    const int sb = blockIdx.x * 8 + (threadIdx.x >> 5), lane = threadIdx.x & 31;
-    if (sb >= nblk) return;
-    const float4 *p = reinterpret_cast<const float4 *>(x + (size_t)sb * 256 + lane * 8);
+__global__ void __launch_bounds__(256) qr_image_kernel(const float *__restrict__ x, int rows, int nsb, uint8_t *__restrict__ img, float *__restrict__ ys) {
+    const int w = blockIdx.x * 8 + (threadIdx.x >> 5), lane = threadIdx.x & 31;
+    if (w >= rows * nsb) return;
+    const float4 *p = reinterpret_cast<const float4 *>(x + (size_t)w * 256 + lane * 8);
     const float4 a = p[0], b = p[1];
     const float v[8] = {a.x, a.y, a.z, a.w, b.x, b.y, b.z, b.w};
-    warp_quant_q8k_image(v, lane, img + (size_t)sb * KIMG_SB, ys + sb);
+    warp_quant_q8k_image(v, lane, kimg_row(img, ys, w / nsb, rows, nsb, w % nsb));
 }
 
 template <int R>
@@ -380,14 +460,25 @@ cudaError_t launch_qr_attn(const float *q, const float *kc, const float *vc, int
     return qa_launch<8>(a, pdl, st);
 }
 
-cudaError_t launch_qr_glu(const float *g, const float *u, int entries, int ff, uint8_t *img, float *ys, bool pdl, cudaStream_t st) {
-    const int nblk = entries * (ff / 256);
-    return launch_k(qr_glu_kernel, dim3((nblk + 7) / 8), dim3(256), 0, st, pdl, g, u, nblk, img, ys);
+cudaError_t launch_qr_plan(const int32_t *top, int ntok, int topk, int ne, KqPlan *plan, bool pdl, cudaStream_t st) {
+    if (ne > 256 || topk > 8 || ntok > BRRR_TILE_MAX) return cudaErrorInvalidValue;
+    return launch_k(qr_plan_kernel, dim3(1), dim3(1024), 0, st, pdl, top, ntok, topk, ne, plan);
+}
+
+cudaError_t launch_qr_gather(const KqPlan *plan, const uint8_t *img, const float *ys, int rows, int topk, int ne, int nsb, uint8_t *out, float *out_ys, bool pdl,
+                             cudaStream_t st) {
+    const int blocks = kqt_max_chunks(rows * topk, ne) * nsb;
+    return launch_k(qr_gather_kernel, dim3(blocks < 148 * 8 ? blocks : 148 * 8), dim3(256), 0, st, pdl, plan, img, ys, rows, topk, nsb, out, out_ys);
+}
+
+cudaError_t launch_qr_glu(const KqPlan *plan, const float *g, const float *u, int entries, int ne, int ff, uint8_t *img, float *ys, bool pdl, cudaStream_t st) {
+    const int warps = kqt_max_chunks(entries, ne) * KT_NT * (ff / 256), blocks = (warps + 7) / 8;
+    return launch_k(qr_glu_kernel, dim3(blocks < 148 * 8 ? blocks : 148 * 8), dim3(256), 0, st, pdl, plan, g, u, ff / 256, img, ys);
 }
 
 void launch_qr_image(const float *x, int rows, int cols, uint8_t *img, float *ys, cudaStream_t st) {
     const int nblk = rows * (cols / 256);
-    if (nblk > 0) qr_image_kernel<<<(nblk + 7) / 8, 256, 0, st>>>(x, nblk, img, ys);
+    if (nblk > 0) qr_image_kernel<<<(nblk + 7) / 8, 256, 0, st>>>(x, rows, cols / 256, img, ys);
 }
 
 }  // namespace brrr

@@ -276,7 +276,7 @@ constexpr int RR_WARPS = 4, RR_STAGES = 3;
 
 template <int TPW>
 __global__ void __launch_bounds__(RR_WARPS * 32) router_rows_kernel(RouterArgs a, int ntok) {
-    constexpr int TT = RR_WARPS * TPW;
+    constexpr int TT = RR_WARPS * TPW, STEP = TPW == 4 ? 8 : 16;
     constexpr size_t STAGE = (size_t)(RT_TILE_FLOATS + TT * RT_TJ) * 4;
     extern __shared__ __align__(128) unsigned char smraw[];
     __shared__ __align__(8) uint64_t full[RR_STAGES];
@@ -316,17 +316,35 @@ __global__ void __launch_bounds__(RR_WARPS * 32) router_rows_kernel(RouterArgs a
         waiter.wait(&full[t % RR_STAGES], (uint32_t)(t / RR_STAGES) & 1u);
         const float *w = reinterpret_cast<const float *>(st) + lane * RT_STRIDE, *x = reinterpret_cast<const float *>(st) + RT_TILE_FLOATS + warp * TPW * RT_TJ;
         const int len = min(RT_TJ, d - t * RT_TJ);
-#pragma unroll 4
-        for (int j = 0; j < len; j += 4) {
-            const float4 wv = *reinterpret_cast<const float4 *>(w + j);
+        // STEP elements of the row and of every token are in registers while the STEP before them are added up (len % 64 == 0)
+        float4 wv[STEP / 4], xv[TPW][STEP / 4];
 #pragma unroll
-            for (int k = 0; k < TPW; k++) {
-                const float4 xv = *reinterpret_cast<const float4 *>(x + k * RT_TJ + j);
-                acc[k] = __fadd_rn(acc[k], __fmul_rn(wv.x, xv.x));
-                acc[k] = __fadd_rn(acc[k], __fmul_rn(wv.y, xv.y));
-                acc[k] = __fadd_rn(acc[k], __fmul_rn(wv.z, xv.z));
-                acc[k] = __fadd_rn(acc[k], __fmul_rn(wv.w, xv.w));
+        for (int q = 0; q < STEP / 4; q++) {
+            wv[q] = *reinterpret_cast<const float4 *>(w + 4 * q);
+#pragma unroll
+            for (int k = 0; k < TPW; k++) xv[k][q] = *reinterpret_cast<const float4 *>(x + k * RT_TJ + 4 * q);
+        }
+#pragma unroll 2
+        for (int j = 0; j < len; j += STEP) {
+            float p[TPW][STEP];
+#pragma unroll
+            for (int k = 0; k < TPW; k++)
+#pragma unroll
+                for (int q = 0; q < STEP / 4; q++) {
+                    p[k][4 * q] = __fmul_rn(wv[q].x, xv[k][q].x); p[k][4 * q + 1] = __fmul_rn(wv[q].y, xv[k][q].y);
+                    p[k][4 * q + 2] = __fmul_rn(wv[q].z, xv[k][q].z); p[k][4 * q + 3] = __fmul_rn(wv[q].w, xv[k][q].w);
+                }
+            const int jn = j + STEP < len ? j + STEP : 0;         // past the end: the first step again, unused
+#pragma unroll
+            for (int q = 0; q < STEP / 4; q++) {
+                wv[q] = *reinterpret_cast<const float4 *>(w + jn + 4 * q);
+#pragma unroll
+                for (int k = 0; k < TPW; k++) xv[k][q] = *reinterpret_cast<const float4 *>(x + k * RT_TJ + jn + 4 * q);
             }
+#pragma unroll
+            for (int i = 0; i < STEP; i++)
+#pragma unroll
+                for (int k = 0; k < TPW; k++) acc[k] = __fadd_rn(acc[k], p[k][i]);
         }
         __syncthreads();                      // the stage is free
         if (warp == 0 && t + RR_STAGES < ntiles) { fence_proxy_async(); issue(t + RR_STAGES, true, true); }

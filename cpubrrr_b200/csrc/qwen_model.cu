@@ -92,10 +92,10 @@ struct brrr_qwen {
     // prompt tiles: up to BRRR_TILE_MAX consecutive positions walk the layers together
     bool has_rows = false;
     struct {
-        float *x, *xn, *q, *k, *v, *gate, *up, *part, *xs, *as, *hs, *wts, *rlogits;
-        uint8_t *img, *aimg, *himg;
+        float *x, *xn, *q, *k, *v, *gate, *up, *part, *xs, *as, *es, *hs, *wts, *rlogits;
+        uint8_t *img, *aimg, *eimg, *himg;       // images of the rows, of the attention output, of the experts' tokens and of h
         int32_t *top;
-        int *cnt, *list;
+        KqPlan *plan;
         unsigned int *counter;
         uint32_t *toks;
     } r{};
@@ -250,13 +250,16 @@ int qrows_alloc(brrr_qwen *m) {
         for (const auto &t : all) CU(kqt_matrix(*t.m, t.rows, t.t));
     }
     auto &r = m->r;
-    const size_t T = BRRR_TILE_MAX, E = T * topk;
+    const size_t T = BRRR_TILE_MAX, E = T * topk, C = T / KT_NT;
+    const size_t X = kqt_max_chunks((int)E, ne);
+    if (X > KT_MAXCHUNK) return BRRR_OK;
     TRY(m->alloc(&r.x, T * d)); TRY(m->alloc(&r.xn, T * d)); TRY(m->alloc(&r.q, T * nh * hd)); TRY(m->alloc(&r.k, T * nkv * hd)); TRY(m->alloc(&r.v, T * nkv * hd));
-    TRY(m->alloc(&r.gate, E * ff)); TRY(m->alloc(&r.up, E * ff)); TRY(m->alloc(&r.part, E * d));
-    TRY(m->alloc(&r.img, T * (d / 256) * KIMG_SB)); TRY(m->alloc(&r.aimg, T * (nh * hd / 256) * KIMG_SB)); TRY(m->alloc(&r.himg, E * (ff / 256) * KIMG_SB));
-    TRY(m->alloc(&r.xs, T * (d / 256))); TRY(m->alloc(&r.as, T * (nh * hd / 256))); TRY(m->alloc(&r.hs, E * (ff / 256)));
+    TRY(m->alloc(&r.gate, X * KT_NT * ff)); TRY(m->alloc(&r.up, X * KT_NT * ff)); TRY(m->alloc(&r.part, E * d));
+    TRY(m->alloc(&r.img, kimg_bytes(C, d / 256))); TRY(m->alloc(&r.aimg, kimg_bytes(C, nh * hd / 256)));
+    TRY(m->alloc(&r.eimg, kimg_bytes(X, d / 256))); TRY(m->alloc(&r.himg, kimg_bytes(X, ff / 256)));
+    TRY(m->alloc(&r.xs, T * (d / 256))); TRY(m->alloc(&r.as, T * (nh * hd / 256))); TRY(m->alloc(&r.es, X * KT_NT * (d / 256))); TRY(m->alloc(&r.hs, X * KT_NT * (ff / 256)));
     TRY(m->alloc(&r.wts, T * 8)); TRY(m->alloc(&r.top, T * 8)); TRY(m->alloc(&r.rlogits, T * ne));
-    TRY(m->alloc(&r.cnt, ne)); TRY(m->alloc(&r.list, (size_t)ne * T)); TRY(m->alloc(&r.counter, T)); TRY(m->alloc(&r.toks, T));
+    TRY(m->alloc(&r.plan, 1)); TRY(m->alloc(&r.counter, T)); TRY(m->alloc(&r.toks, T));
     CU(cudaMemsetAsync(r.counter, 0, T * sizeof(unsigned int), m->stream));
     m->has_rows = true;
     return BRRR_OK;
@@ -277,19 +280,20 @@ int qenqueue_rows(brrr_qwen *m, int rows, int pos0, bool last) {
         const KqtMat *qkv[3] = {&ly.tq, &ly.tk, &ly.tv};
         float *qkv_out[3] = {r.q, r.k, r.v};
         const int ld3[3] = {nh * hd, nkv * hd, nkv * hd};
-        CU(launch_kqt(qkv, qkv_out, ld3, 3, 0, nullptr, nullptr, 1, rows, 1, 1, r.img, r.xs, false, m->st, pdl, s));
+        CU(launch_kqt(qkv, qkv_out, ld3, 3, 0, nullptr, 1, rows, 1, false, r.img, r.xs, false, m->st, pdl, s));
         CU(launch_qr_qknorm(r.q, r.k, r.v, ly.q_norm, ly.k_norm, m->rope, c.rms_eps, nh, nkv, pos0, rows, ly.kc, ly.vc, pdl, s));
         CU(launch_qr_attn(r.q, ly.kc, ly.vc, nh, nkv, pos0, rows, r.aimg, r.as, pdl, s));
         const KqtMat *o[1] = {&ly.to}, *gu[2] = {&ly.tgate, &ly.tup}, *dn[1] = {&ly.tdown};
         float *xo[1] = {r.x}, *guo[2] = {r.gate, r.up}, *dno[1] = {r.part};
         const int ldd[1] = {d}, ldf[2] = {ff, ff};
-        CU(launch_kqt(o, xo, ldd, 1, 0, nullptr, nullptr, 1, rows, 1, 1, r.aimg, r.as, true, m->st, pdl, s));
+        CU(launch_kqt(o, xo, ldd, 1, 0, nullptr, 1, rows, 1, false, r.aimg, r.as, true, m->st, pdl, s));
         CU(launch_qr_norm(r.x, rows, d, nullptr, nullptr, 0, ly.ffn_norm, c.rms_eps, r.xn, r.img, r.xs, pdl, s));
         CU(launch_router_rows(r.xn, d, ly.ginp, nullptr, ne, topk, rows, r.rlogits, r.top, r.wts, r.counter, m->st, pdl, s));
-        CU(launch_tile_route(r.top, rows, topk, ne, r.cnt, r.list, pdl, s));
-        CU(launch_kqt(gu, guo, ldf, 2, ff, r.cnt, r.list, ne, rows, topk, topk, r.img, r.xs, false, m->st, pdl, s));
-        CU(launch_qr_glu(r.gate, r.up, rows * topk, ff, r.himg, r.hs, pdl, s));
-        CU(launch_kqt(dn, dno, ldd, 1, d, r.cnt, r.list, ne, rows, topk, 1, r.himg, r.hs, false, m->st, pdl, s));
+        CU(launch_qr_plan(r.top, rows, topk, ne, r.plan, pdl, s));
+        CU(launch_qr_gather(r.plan, r.img, r.xs, rows, topk, ne, d / 256, r.eimg, r.es, pdl, s));
+        CU(launch_kqt(gu, guo, ldf, 2, ff, r.plan, ne, rows, topk, false, r.eimg, r.es, false, m->st, pdl, s));
+        CU(launch_qr_glu(r.plan, r.gate, r.up, rows * topk, ne, ff, r.himg, r.hs, pdl, s));
+        CU(launch_kqt(dn, dno, ldd, 1, d, r.plan, ne, rows, topk, true, r.himg, r.hs, false, m->st, pdl, s));
         part = r.part;
     }
     if (!last) return BRRR_OK;            // rows that only fill the cache: nobody reads their residual
