@@ -163,85 +163,102 @@ __device__ __forceinline__ void qw_slice(int w, int n, int &a, int &b) {
     b = a + base + (w < rem ? 1 : 0);
 }
 
-// ---------------------------------------------------------------- lane-group form (decode kernels)
-// Eight lanes own one superblock (a warp covers four superblocks at a time) and every lane moves 16
-// bytes per load.  A unit = what one lane holds of one superblock.
-//   Q4_K:         a = the 16-byte header (d | dmin, 12 packed scale bytes), b = nibble bytes 16 l8 .. 16 l8 + 15
-//   Q6_K planes:  a = ql bytes 16 l8 .. +15, b = the 16 qh bytes that go with them,
-//                 c = scale of the low nibbles | scale of the high nibbles << 8 | d (f16 bits) << 16
-struct KUnit { uint4 a, b; uint32_t c; };
-
-__device__ __forceinline__ void kq_unit_load(const KMatDev &m, const uint8_t *row, int sb, int l8, KUnit &u) {
-    if (m.type == 12) {
-        const uint4 *p = reinterpret_cast<const uint4 *>(row + (size_t)sb * 144);
-        u.a = __ldg(p);
-        u.b = __ldg(p + 1 + l8);
-        u.c = 0u;
-    } else {
-        const int nsb = m.cols / 256, h = l8 >> 2, q = l8 & 3;
-        u.a = __ldg(reinterpret_cast<const uint4 *>(row + (size_t)sb * 128 + 16 * l8));
-        u.b = __ldg(reinterpret_cast<const uint4 *>(row + (size_t)nsb * 128 + (size_t)sb * 64 + 32 * h + 16 * (q & 1)));
-        const uint8_t *sc = row + (size_t)nsb * 192 + (size_t)sb * 16 + 8 * h + (q >= 2 ? 2 : 0) + (q & 1);
-        const uint32_t dh = __ldg(reinterpret_cast<const unsigned short *>(row + (size_t)nsb * 208 + (size_t)sb * 2));
-        u.c = (uint32_t)__ldg(sc) | ((uint32_t)__ldg(sc + 4) << 8) | (dh << 16);
-    }
+// ---------------------------------------------------------------- rows in shared memory (decode kernels)
+// Q8_K activation of the decode kernels: quants, one scale per 256 values, and the sums of every 16 quants (Q4_K minima need pairs of
+// them, the -32 of Q6_K each).
+__device__ __forceinline__ void warp_quant_q8k16(const float (&v)[8], int lane, int8_t *q, float *s, int32_t *b16) {
+    float amax = 1e-12f;
+#pragma unroll
+    for (int i = 0; i < 8; i++) amax = fmaxf(amax, fabsf(v[i]));
+#pragma unroll
+    for (int o = 16; o; o >>= 1) amax = fmaxf(amax, __shfl_xor_sync(0xffffffffu, amax, o));
+    const float sc = __fdiv_rn(amax, 127.0f);
+    int qi[8], sum = 0;
+#pragma unroll
+    for (int i = 0; i < 8; i++) { qi[i] = brrr_q8_round(v[i], sc); sum += qi[i]; }
+    const uint32_t lo = (qi[0] & 0xff) | ((qi[1] & 0xff) << 8) | ((qi[2] & 0xff) << 16) | ((uint32_t)(qi[3] & 0xff) << 24);
+    const uint32_t hi = (qi[4] & 0xff) | ((qi[5] & 0xff) << 8) | ((qi[6] & 0xff) << 16) | ((uint32_t)(qi[7] & 0xff) << 24);
+    *reinterpret_cast<uint2 *>(q + lane * 8) = make_uint2(lo, hi);
+    sum += __shfl_xor_sync(0xffffffffu, sum, 1);
+    if (!(lane & 1)) b16[lane >> 1] = sum;
+    if (lane == 0) *s = sc;
 }
 
-// The superblock's term of the row sum, valid in all eight lanes of the group: (ys d) acc - (ys dmin) mint
-// for Q4_K, (ys d) acc for Q6_K, every product rounded separately as in q4k_row_dot / q6k_row_dot.
-// xsb: the 256 int8 activations of the superblock (16-byte aligned), bs: its eight 32-sums, gmask: the
-// group's lanes.
-__device__ __forceinline__ float kq_unit_term(int type, const KUnit &u, int l8, const int8_t *xsb, float ys, const int32_t *bs, unsigned gmask) {
+// Eight lanes own one superblock; lane l8 holds the activations that meet its 16 bytes of quants.
+//   Q4_K: nibble bytes 16 l8 ..: x0 / x1 for the low / high nibbles, b0 = the 32-sum of sub-block l8
+//   Q6_K planes: ql bytes 16 l8 ..: x0 / x1 for the low / high nibbles, b0 / b1 = 32 times their sums
+struct KAct { int4 x0, x1; int b0, b1; };
+__device__ __forceinline__ void kact_load(int type, const int8_t *xsb, const int32_t *b16, int l8, KAct &a) {
+    const int at = type == 12 ? 64 * (l8 >> 1) + 16 * (l8 & 1) : 128 * (l8 >> 2) + 16 * (l8 & 3);
+    a.x0 = *reinterpret_cast<const int4 *>(xsb + at);
+    a.x1 = *reinterpret_cast<const int4 *>(xsb + at + (type == 12 ? 32 : 64));
     if (type == 12) {
-        const int jj = l8 >> 1, hh = l8 & 1;
-        const int4 x0 = *reinterpret_cast<const int4 *>(xsb + (2 * jj) * 32 + 16 * hh);
-        const int4 x1 = *reinterpret_cast<const int4 *>(xsb + (2 * jj + 1) * 32 + 16 * hh);
-        int sc0, mn0, sc1, mn1, scj, mnj;
-        k4_scale_min(u.a.y, u.a.z, u.a.w, 2 * jj, sc0, mn0);
-        k4_scale_min(u.a.y, u.a.z, u.a.w, 2 * jj + 1, sc1, mn1);
-        k4_scale_min(u.a.y, u.a.z, u.a.w, l8, scj, mnj);
-        const uint32_t M = 0x0F0F0F0Fu;
-        int lo = __dp4a((int)(u.b.x & M), x0.x, 0);
-        lo = __dp4a((int)(u.b.y & M), x0.y, lo);
-        lo = __dp4a((int)(u.b.z & M), x0.z, lo);
-        lo = __dp4a((int)(u.b.w & M), x0.w, lo);
-        int hi = __dp4a((int)((u.b.x >> 4) & M), x1.x, 0);
-        hi = __dp4a((int)((u.b.y >> 4) & M), x1.y, hi);
-        hi = __dp4a((int)((u.b.z >> 4) & M), x1.z, hi);
-        hi = __dp4a((int)((u.b.w >> 4) & M), x1.w, hi);
-        int a = lo * sc0 + hi * sc1;
-        int mt = mnj * bs[l8];
-        a = __reduce_add_sync(gmask, a);
-        mt = __reduce_add_sync(gmask, mt);
-        const float d = half_bits_to_f32(u.a.x & 0xffffu), dmin = half_bits_to_f32(u.a.x >> 16);
-        return __fsub_rn(__fmul_rn(__fmul_rn(ys, d), (float)a), __fmul_rn(__fmul_rn(ys, dmin), (float)mt));
-    }
-    const int h = l8 >> 2, q = l8 & 3;
-    const int base = 128 * h + (q >= 2 ? 32 : 0) + 16 * (q & 1);
-    const int4 xl = *reinterpret_cast<const int4 *>(xsb + base);
-    const int4 xh = *reinterpret_cast<const int4 *>(xsb + base + 64);
-    const int sl = q >= 2 ? 2 : 0, sh = sl + 4;
-    const uint32_t M4 = 0x0F0F0F0Fu, M2 = 0x03030303u;
-    int accl = 0, acch = 0, sxl = 0, sxh = 0;
-#define BRRR_Q6_WORD(QL, QH, XL, XH)                                                                   \
-    accl = __dp4a((int)(((QL) & M4) | ((((QH) >> sl) & M2) << 4)), (XL), accl);                         \
-    acch = __dp4a((int)((((QL) >> 4) & M4) | ((((QH) >> sh) & M2) << 4)), (XH), acch);                  \
-    sxl = __dp4a(0x01010101, (XL), sxl);                                                                \
-    sxh = __dp4a(0x01010101, (XH), sxh);
-    BRRR_Q6_WORD(u.a.x, u.b.x, xl.x, xh.x)
-    BRRR_Q6_WORD(u.a.y, u.b.y, xl.y, xh.y)
-    BRRR_Q6_WORD(u.a.z, u.b.z, xl.z, xh.z)
-    BRRR_Q6_WORD(u.a.w, u.b.w, xl.w, xh.w)
-#undef BRRR_Q6_WORD
-    const int scl = (int)(signed char)(u.c & 0xffu), sch = (int)(signed char)((u.c >> 8) & 0xffu);
-    int a = (accl - 32 * sxl) * scl + (acch - 32 * sxh) * sch;
-    a = __reduce_add_sync(gmask, a);
-    return __fmul_rn(__fmul_rn(ys, half_bits_to_f32(u.c >> 16)), (float)a);
+        const int2 s = *reinterpret_cast<const int2 *>(b16 + 2 * l8);
+        a.b0 = s.x + s.y; a.b1 = 0;
+    } else { a.b0 = 32 * b16[at >> 4]; a.b1 = 32 * b16[(at >> 4) + 4]; }
 }
 
-__device__ __forceinline__ float kq_row_dot(const KMatDev &m, size_t row, const int8_t *xq, const float *ys, const int32_t *bsum, int lane) {
-    const uint8_t *r = m.p + row * m.bpr();
-    return m.type == 12 ? q4k_row_dot(r, m.cols / 256, xq, ys, bsum, lane) : q6k_row_dot(r, m.cols / 256, xq, ys, lane);
+// This lane's share of a superblock's integers (a: scaled quant sum, mt: minima sum) and the superblock's float scales.
+__device__ __forceinline__ void kq_unit(int type, int nsb, const unsigned char *row, int sb, int l8, const KAct &x, int &a, int &mt, float &d, float &dmin) {
+    const uint32_t M4 = 0x0F0F0F0Fu;
+    int lo = 0, hi = 0;
+    if (type == 12) {
+        const unsigned char *p = row + sb * 144;
+        const uint4 h = *reinterpret_cast<const uint4 *>(p), b = *reinterpret_cast<const uint4 *>(p + 16 + 16 * l8);
+        const bool up = l8 >= 4;                     // sub-blocks 4 .. 7: six bits in two fields
+        const uint32_t sc4 = up ? (h.w & M4) | ((h.y >> 2) & 0x30303030u) : h.y & 0x3F3F3F3Fu;
+        const uint32_t mn4 = up ? ((h.w >> 4) & M4) | ((h.z >> 2) & 0x30303030u) : h.z & 0x3F3F3F3Fu;
+        const uint32_t scp = sc4 >> ((l8 & 2) * 8);
+        lo = __dp4a((int)(b.x & M4), x.x0.x, lo); lo = __dp4a((int)(b.y & M4), x.x0.y, lo);
+        lo = __dp4a((int)(b.z & M4), x.x0.z, lo); lo = __dp4a((int)(b.w & M4), x.x0.w, lo);
+        hi = __dp4a((int)((b.x >> 4) & M4), x.x1.x, hi); hi = __dp4a((int)((b.y >> 4) & M4), x.x1.y, hi);
+        hi = __dp4a((int)((b.z >> 4) & M4), x.x1.z, hi); hi = __dp4a((int)((b.w >> 4) & M4), x.x1.w, hi);
+        a = lo * (int)(scp & 0xFFu) + hi * (int)((scp >> 8) & 0xFFu);
+        mt = (int)((mn4 >> ((l8 & 3) * 8)) & 0xFFu) * x.b0;
+        d = half_bits_to_f32(h.x & 0xffffu); dmin = half_bits_to_f32(h.x >> 16);
+    } else {
+        const int h = l8 >> 2, q = l8 & 3;
+        const uint4 l = *reinterpret_cast<const uint4 *>(row + sb * 128 + 16 * l8);
+        const uint4 u = *reinterpret_cast<const uint4 *>(row + nsb * 128 + sb * 64 + 32 * h + 16 * (q & 1));
+        const signed char *sc = reinterpret_cast<const signed char *>(row) + nsb * 192 + sb * 16 + 8 * h + q;
+        const int sl = q & 2;                        // 2-bit fields: 0 and 4, or 2 and 6
+        const uint32_t M2 = 0x30303030u;
+        const uint32_t ux = u.x >> sl, uy = u.y >> sl, uz = u.z >> sl, uw = u.w >> sl;
+        lo = __dp4a((int)((l.x & M4) | ((ux << 4) & M2)), x.x0.x, lo); lo = __dp4a((int)((l.y & M4) | ((uy << 4) & M2)), x.x0.y, lo);
+        lo = __dp4a((int)((l.z & M4) | ((uz << 4) & M2)), x.x0.z, lo); lo = __dp4a((int)((l.w & M4) | ((uw << 4) & M2)), x.x0.w, lo);
+        hi = __dp4a((int)(((l.x >> 4) & M4) | (ux & M2)), x.x1.x, hi); hi = __dp4a((int)(((l.y >> 4) & M4) | (uy & M2)), x.x1.y, hi);
+        hi = __dp4a((int)(((l.z >> 4) & M4) | (uz & M2)), x.x1.z, hi); hi = __dp4a((int)(((l.w >> 4) & M4) | (uw & M2)), x.x1.w, hi);
+        a = (lo - x.b0) * (int)sc[0] + (hi - x.b1) * (int)sc[4];
+        mt = 0;
+        d = half_bits_to_f32(*reinterpret_cast<const unsigned short *>(row + nsb * 208 + sb * 2)); dmin = 0.0f;
+    }
+}
+
+// Terms of two superblocks per group of eight lanes: (ys d) a - (ys dmin) mt for Q4_K, (ys d) a for Q6_K, every product rounded on its
+// own as in q4k_row_dot / q6k_row_dot.  The four sums meet in five shuffles: lanes 4 .. 7 of a group keep the second superblock, odd pairs
+// the minima.  Lane 0 of the group returns the first term, lane 4 the second.  All 32 lanes must call it.
+__device__ __forceinline__ float kq_pair_term(int type, int nsb, const unsigned char *row0, int sb0, const KAct &x0, float ys0, const unsigned char *row1, int sb1,
+                                              const KAct &x1, float ys1, int l8) {
+    int a0, a1, m0, m1;
+    float d0, d1, n0, n1;
+    kq_unit(type, nsb, row0, sb0, l8, x0, a0, m0, d0, n0);
+    kq_unit(type, nsb, row1, sb1, l8, x1, a1, m1, d1, n1);
+    const bool second = l8 & 4, minima = l8 & 2;
+    const float ys = second ? ys1 : ys0;
+    int a = second ? a1 : a0;
+    a += __shfl_xor_sync(0xffffffffu, second ? a0 : a1, 4);
+    if (type == 12) {
+        int m = second ? m1 : m0;
+        m += __shfl_xor_sync(0xffffffffu, second ? m0 : m1, 4);
+        int r = minima ? m : a;
+        r += __shfl_xor_sync(0xffffffffu, minima ? a : m, 2);
+        r += __shfl_xor_sync(0xffffffffu, r, 1);
+        const float f = __fmul_rn(__fmul_rn(ys, minima ? (second ? n1 : n0) : (second ? d1 : d0)), (float)r);
+        return __fsub_rn(f, __shfl_xor_sync(0xffffffffu, f, 2));
+    }
+    a += __shfl_xor_sync(0xffffffffu, a, 2);
+    a += __shfl_xor_sync(0xffffffffu, a, 1);
+    return __fmul_rn(__fmul_rn(ys, second ? d1 : d0), (float)a);
 }
 
 }  // namespace brrr

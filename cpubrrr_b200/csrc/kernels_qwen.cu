@@ -1,20 +1,19 @@
-// Decode kernels of the qwen3moe engine (src/bin/engine_qwen2.rs:302-451): Q4_K embedding row,
-// RMS norm with the reference's 12 partial sums + Q8_K quantisation, K-quant matrix-vector
-// products with their epilogues, per-head QK norm + RoPE + cache append, full causal GQA
-// attention (head_dim 128), SiLU-GLU experts, weighted down-projection and the vocabulary argmax.
+// Decode kernels of the qwen3moe engine (src/bin/engine_qwen2.rs:302-451): Q4_K embedding row, RMS norm with the reference's 12
+// partial sums + Q8_K quantisation, K-quant matrix-vector products, per-head QK norm + RoPE + cache append, full causal GQA attention
+// (head_dim 128), SiLU-GLU experts, weighted down-projection and the vocabulary argmax.
 //
-// Float order: every sum the reference forms serially is formed serially by one thread here
-// (norm partials, head mean square, softmax denominator, probability-weighted values, the
-// expert combine); integer sums are exact and split across lanes.
+// Float order: every sum the reference forms serially is formed serially by one thread here (norm partials, head mean square, softmax
+// denominator, probability-weighted values, superblock terms, the expert combine); integer sums are exact and split across lanes.
 //
-// One layer is seven launches chained by programmatic dependent launch:
-//   q|k|v matvec -> QK norm + RoPE + cache append -> attention (+ Q8_K of its output) -> o-proj (+ residual)
-//   -> router (FFN norm + Q8_K of the normalised token in its prologue) -> gate/up + SiLU-GLU
-//   -> down (Q8_K of h in its prologue, weighted accumulate, and - by the last CTA to finish - the
-//      next layer's attention norm + Q8_K, or the output norm after the last layer).
-// Matrix rows are read in the lane-group form of brrr_kq.cuh (16 bytes per lane and load); kernels
-// whose matrices are known before their predecessor ends (q|k|v, o-proj, down) fetch every weight
-// byte into registers ahead of the dependency wait.
+// A step is bound by latency: 36 MB of weights per layer are 5.6 us of memory time, the serial chains and hand-overs more.  So
+// every kernel brings its matrix rows into shared memory with bulk copies, before its dependency wait wherever the rows are known by
+// then (q|k|v, o-proj, down, the first rows of the head; K and V of the cached positions), and the layer is the chain
+//   q|k|v (prologue: expert combine of the layer before, norm, Q8_K - every CTA its own: 64 KB from L2 cost less than a kernel)
+//   -> attention (prologue: QK norm, RoPE, cache append) -> o-proj (prologue: Q8_K) -> routing hint (norm, Q8_K, estimate of the router)
+//   -> gate/up + SiLU-GLU of the estimated experts -> down of the same
+// joined by programmatic dependent launch, while the exact router - a chain of d dependent adds, 4.3 us at best at d = 2048 - runs
+// beside the last three on another stream and publishes its choice to the next combine, which takes the weights and the order from
+// it and flags the step if the estimate missed an expert (the host runs that step again without the estimate).
 #include "brrr_kernels.h"
 #include "brrr_kq.cuh"
 #include "brrr_block.cuh"
@@ -25,13 +24,15 @@ namespace brrr {
 namespace {
 
 constexpr int QW_HD = 128;
-constexpr int QW_HEAD_ROWS = 64;   // vocabulary rows per CTA of the head kernel
+constexpr int QG_WARPS = 16, QG_THREADS = QG_WARPS * 32;
+constexpr size_t QG_ROW_BYTES = 100 * 1024;      // shared memory for rows per CTA (two kernels share an SM)
 
 // ---------------------------------------------------------------- embedding (engine_qwen2.rs:310-330)
-__global__ void __launch_bounds__(256) qw_embed_kernel(const uint8_t *__restrict__ embd, int d, const DevState *__restrict__ state,
+__global__ void __launch_bounds__(256) qw_embed_kernel(const uint8_t *__restrict__ embd, int d, DevState *__restrict__ state,
                                                        float *__restrict__ x) {
     pdl_wait();
     pdl_trigger();
+    if (blockIdx.x == 0 && threadIdx.x == 0) state->fold_seq = state->router_seq;      // routings published before this step (no router runs now)
     const size_t tok = state->tok;
     const int sb = blockIdx.x, i = threadIdx.x;
     const uint32_t *b32 = reinterpret_cast<const uint32_t *>(embd + (tok * (size_t)(d / 256) + sb) * 144);
@@ -44,442 +45,703 @@ __global__ void __launch_bounds__(256) qw_embed_kernel(const uint8_t *__restrict
     x[sb * 256 + i] = __fsub_rn(__fmul_rn(__fmul_rn(dv, (float)sc), (float)q), __fmul_rn(dmin, (float)mn));
 }
 
-// ---------------------------------------------------------------- RMS norm + Q8_K (engine_qwen2.rs:453-465, 287-300)
-// One CTA.  12 threads walk the 12 slices serially, the partials are added in worker order.
-__global__ void __launch_bounds__(256) qw_norm_quant_kernel(const float *__restrict__ x, const float *__restrict__ w, float eps, int d,
-                                                            float *__restrict__ xn_out, int8_t *__restrict__ q, float *__restrict__ s,
-                                                            int32_t *__restrict__ bsum) {
-    extern __shared__ __align__(16) float xs_sh[];
-    __shared__ float part[QW_NT];
-    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-    pdl_wait();
-    pdl_trigger();
-    for (int i = tid; i < d / 4; i += 256) reinterpret_cast<float4 *>(xs_sh)[i] = reinterpret_cast<const float4 *>(x)[i];
+// ---------------------------------------------------------------- expert selection
+// sel[r] = expert of rank r of est[0 .. ne) (the larger first, the lower index among equals).  Block-wide; ends synchronised.
+struct alignas(16) SelectScratch { float lg[256]; int rank[256]; };
+__device__ __forceinline__ void qw_select(const float *est, int ne, int topk, const DevState *state, SelectScratch &w, int *sel, int tid, int nthreads) {
+#ifdef BRRR_TEST_HOOKS
+    const bool spoil = state && (state->test_hooks & 1u) && state->pos % 3 == 0;
+#else
+    constexpr bool spoil = false;
+    (void)state;
+#endif
+    for (int e = tid; e < 256; e += nthreads) { w.lg[e] = e < ne ? __ldcg(est + e) : -INFINITY; w.rank[e] = 0; }
+    if (tid < 8) sel[tid] = 0;
     __syncthreads();
+    const int quarter = ((ne + 15) / 16) * 4;
+    for (int i = tid; i < 4 * ne; i += nthreads) {
+        const int p = i / ne, e = i - p * ne, o0 = p * quarter;
+        const float v = w.lg[e];
+        int r = 0;
+        for (int o = o0; o < min(o0 + quarter, 256); o += 4) {
+            const float4 u = *reinterpret_cast<const float4 *>(w.lg + o);
+            r += (u.x > v || (u.x == v && o < e)) + (u.y > v || (u.y == v && o + 1 < e)) + (u.z > v || (u.z == v && o + 2 < e)) + (u.w > v || (u.w == v && o + 3 < e));
+        }
+        if (r) atomicAdd(&w.rank[e], r);
+    }
+    __syncthreads();
+    for (int e = tid; e < ne; e += nthreads)
+        if (w.rank[e] < topk) sel[w.rank[e]] = (spoil && w.rank[e] == topk - 1) ? (e + 1) % ne : e;
+    __syncthreads();
+}
+
+// ---------------------------------------------------------------- expert combine + RMS norm + Q8_K (engine_qwen2.rs:432-465, 287-300)
+// x += w[k] part[slot of k], exact experts in rank order (part == nullptr: nothing to add); then norm and quants.
+struct QFold {
+    const float *x_in, *part;        // residual; [slot][d]
+    float *x_out;                    // the new residual (CTA 0 writes it; never x_in: other CTAs may still read that)
+    const float *est;                // slot s of part belongs to rank s of the estimate; nullptr: of top
+    const int32_t *top;              // exact routing (est == nullptr)
+    const float *wts;
+    int ne, topk, d;
+    uint32_t seq;                    // est: this step's seq-th routing is awaited from the router
+    const float *norm_w;             // nullable: combine only
+    float eps;
+    DevState *state;
+};
+struct QFoldShared {
+    SelectScratch sel_ws;
+    int sel[8], slot_of[8];
+    float wts[8], part[QW_NT];
+};
+
+// Before the dependency wait: the estimate's experts and the exact routing, a bounded wait for the router's words (it does not depend on
+// any kernel that waits here, and this kernel leaves it room on every SM).
+__device__ __forceinline__ void qw_fold_routing(const QFold &a, QFoldShared &w, int tid) {
+    if (!a.part) return;
+    if (a.est) qw_select(a.est, a.ne, a.topk, a.state, w.sel_ws, w.sel, tid, QG_THREADS);
+    if (tid < 32) {
+        uint32_t payload = 0u;
+        if (a.est) {
+            if (tid < 16 && (tid & 7) < a.topk) {
+                const uint32_t want = __ldcg(&a.state->fold_seq) + a.seq;
+                const volatile unsigned long long *p = a.state->route_pub + tid;
+                bool ok = false;
+                const long long t0 = clock64();
+                do {
+                    for (int i = 0; i < 64 && !ok; i++) {
+                        const unsigned long long v = *p;
+                        ok = (uint32_t)(v >> 32) == want;
+                        payload = (uint32_t)v;
+                    }
+                } while (!ok && clock64() - t0 < WAIT_CYCLES && *reinterpret_cast<volatile uint32_t *>(&a.state->err) == 0u);
+                if (!ok) {               // the step is void from here: the host runs it again without the estimate
+                    atomicCAS(&a.state->err, (uint32_t)DEV_ERR_NONE, (uint32_t)DEV_ERR_PEER_TIMEOUT);
+                    atomicMin(&a.state->spec_fail_step, a.state->n_out);
+                }
+            }
+        } else if (tid < 16 && (tid & 7) < a.topk) payload = tid < 8 ? (uint32_t)__ldcg(a.top + tid) : __float_as_uint(__ldcg(a.wts + (tid - 8)));
+        if (tid >= 8 && tid < 8 + a.topk) w.wts[tid - 8] = __uint_as_float(payload);
+        if (tid < a.topk) {
+            int slot = tid;
+            if (a.est) {
+                slot = -1;
+                for (int s = 0; s < a.topk; s++) if (w.sel[s] == (int)payload) slot = s;
+                if (slot < 0) { slot = 0; atomicMin(&a.state->spec_fail_step, a.state->n_out); }      // the estimate missed this expert
+            }
+            w.slot_of[tid] = slot;
+        }
+    }
+    __syncthreads();
+}
+
+// The 12-slice norm of xf (shared memory, synchronised): 1 / sqrt(mean + eps) in every thread.
+__device__ __forceinline__ float qw_norm_inv(const float *xf, int d, float eps, float *part, int tid) {
     if (tid < QW_NT) {
-        int a, b;
-        qw_slice(tid, d, a, b);
+        int lo, hi;
+        qw_slice(tid, d, lo, hi);
         float ps = 0.0f;
 #pragma unroll 8
-        for (int i = a; i < b; i++) { float v = xs_sh[i]; ps = __fadd_rn(ps, __fmul_rn(v, v)); }
+        for (int i = lo; i < hi; i++) { const float v = xf[i]; ps = __fadd_rn(ps, __fmul_rn(v, v)); }
         part[tid] = ps;
     }
     __syncthreads();
     float tot = 0.0f;
 #pragma unroll
     for (int k = 0; k < QW_NT; k++) tot = __fadd_rn(tot, part[k]);
-    const float inv = __fdiv_rn(1.0f, __fsqrt_rn(__fadd_rn(__fdiv_rn(tot, (float)d), eps)));
-    for (int sb = warp; sb < d / 256; sb += 8) {
+    return __fdiv_rn(1.0f, __fsqrt_rn(__fadd_rn(__fdiv_rn(tot, (float)d), eps)));
+}
+
+// After the wait.  xf: d floats of shared memory; q, s, b16: the Q8_K image (shared or global).
+__device__ __forceinline__ void qw_fold_norm(const QFold &a, QFoldShared &w, float *xf, int8_t *q, float *s, int32_t *b16, bool store, int tid) {
+    const int d = a.d, warp = tid >> 5, lane = tid & 31;
+    for (int g = tid; g < d / 4; g += QG_THREADS) {
+        float4 x = reinterpret_cast<const float4 *>(a.x_in)[g];
+        if (a.part) {
+            float4 p[8];
+#pragma unroll
+            for (int k = 0; k < 8; k++) if (k < a.topk) p[k] = __ldcg(reinterpret_cast<const float4 *>(a.part + (size_t)w.slot_of[k] * d) + g);
+#pragma unroll
+            for (int k = 0; k < 8; k++)
+                if (k < a.topk) {
+                    const float t = w.wts[k];
+                    x.x = __fadd_rn(x.x, __fmul_rn(t, p[k].x)); x.y = __fadd_rn(x.y, __fmul_rn(t, p[k].y));
+                    x.z = __fadd_rn(x.z, __fmul_rn(t, p[k].z)); x.w = __fadd_rn(x.w, __fmul_rn(t, p[k].w));
+                }
+        }
+        reinterpret_cast<float4 *>(xf)[g] = x;
+        if (store) reinterpret_cast<float4 *>(a.x_out)[g] = x;
+    }
+    if (!a.norm_w) return;
+    __syncthreads();
+    const float inv = qw_norm_inv(xf, d, a.eps, w.part, tid);
+    for (int sb = warp; sb < d / 256; sb += QG_WARPS) {
         float v[8];
+        const float4 w0 = reinterpret_cast<const float4 *>(a.norm_w + sb * 256)[lane * 2], w1 = reinterpret_cast<const float4 *>(a.norm_w + sb * 256)[lane * 2 + 1];
+        const float nw[8] = {w0.x, w0.y, w0.z, w0.w, w1.x, w1.y, w1.z, w1.w};
 #pragma unroll
-        for (int i = 0; i < 8; i++) {
-            int idx = sb * 256 + lane * 8 + i;
-            v[i] = __fmul_rn(__fmul_rn(xs_sh[idx], inv), w[idx]);
-        }
-        if (xn_out) {
-            float4 *dst = reinterpret_cast<float4 *>(xn_out + sb * 256 + lane * 8);
-            dst[0] = make_float4(v[0], v[1], v[2], v[3]);
-            dst[1] = make_float4(v[4], v[5], v[6], v[7]);
-        }
-        warp_quant_q8k(v, lane, q + sb * 256, s + sb, bsum + sb * 8);
+        for (int i = 0; i < 8; i++) v[i] = __fmul_rn(__fmul_rn(xf[sb * 256 + lane * 8 + i], inv), nw[i]);
+        warp_quant_q8k16(v, lane, q + sb * 256, s + sb, b16 + sb * 16);
     }
 }
 
-
-// ---------------------------------------------------------------- lane-group rows
-// A warp owns a row; lane group g = lane / 8 owns superblocks g, g + 4, ... (UPL per lane).
-template <int UPL>
-__device__ __forceinline__ void qw_row_load(const KMatDev &m, const uint8_t *row, int nsb, int lane, KUnit (&u)[UPL]) {
-    const int g = lane >> 3, l8 = lane & 7;
-#pragma unroll
-    for (int i = 0; i < UPL; i++)
-        if (g + 4 * i < nsb) kq_unit_load(m, row, g + 4 * i, l8, u[i]);
+// the same as a kernel of its own, for the vocabulary head: one CTA, image to global memory
+__global__ void __launch_bounds__(QG_THREADS) qw_fold_kernel(QFold a, int8_t *q, float *s, int32_t *b16) {
+    extern __shared__ __align__(16) unsigned char qsm[];
+    __shared__ QFoldShared w;
+    qw_fold_routing(a, w, threadIdx.x);
+    pdl_wait();
+    pdl_trigger();
+    qw_fold_norm(a, w, reinterpret_cast<float *>(qsm), q, s, b16, true, threadIdx.x);
 }
 
-// Row sum from units in registers and the Q8_K activation in shared memory: superblock terms are
-// added in superblock order, one unfused add each (q4k_dot / q6k_dot of the reference); the result
-// is valid in every lane.
-template <int UPL>
-__device__ __forceinline__ float qw_row_sum(int type, const KUnit (&u)[UPL], int nsb, int lane, const int8_t *xq, const float *ys,
-                                            const int32_t *bsum) {
-    const int g = lane >> 3, l8 = lane & 7;
-    const unsigned gmask = 0xFFu << (8 * g);
-    float sumf = 0.0f;
+// ---------------------------------------------------------------- matrix rows x one activation (q|k|v, o-proj)
+// Lane group g = lane / 8 takes superblocks g, g + 4, ... of every row.  Up to eight superblocks the activation stays in registers from row
+// to row; of wider rows a warp has one or two, and it is read per pair of superblocks (64 registers: two CTAs per SM).
+template <int UPL> struct QLane {
+    KAct x[2];
+    float ys[2];
+    const int8_t *q;
+    const float *s;
+    const int32_t *b16;
+};
+__device__ __forceinline__ void qw_lane_pair(int type, int nsb, const int8_t *q, const float *s, const int32_t *b16, int lane, int i0, KAct (&x)[2], float (&ys)[2]) {
 #pragma unroll
-    for (int i = 0; i < UPL; i++) {
-        const int sb = g + 4 * i;
-        float term = 0.0f;
-        if (sb < nsb) term = kq_unit_term(type, u[i], l8, xq + sb * 256, ys[sb], bsum + sb * 8, gmask);
-#pragma unroll
-        for (int k = 0; k < 4; k++) {
-            const float t = __shfl_sync(0xffffffffu, term, 8 * k);
-            if (4 * i + k < nsb) sumf = __fadd_rn(sumf, t);
-        }
+    for (int i = 0; i < 2; i++) {
+        const int sb = min((lane >> 3) + 4 * (i0 + i), nsb - 1);
+        kact_load(type, q + sb * 256, b16 + sb * 16, lane & 7, x[i]);
+        ys[i] = s[sb];
     }
-    return sumf;
 }
-
-// Q8_K activation (n values) from global memory into shared memory: quants, scales, 32-sums.
-__device__ __forceinline__ void qw_stage_q8k(const int8_t *q, const float *s, const int32_t *bsum, int n, int8_t *sq, float *ss, int32_t *sb,
-                                             int tid, int nthreads) {
-    for (int i = tid; i < n / 16; i += nthreads) reinterpret_cast<int4 *>(sq)[i] = reinterpret_cast<const int4 *>(q)[i];
-    for (int i = tid; i < n / 256; i += nthreads) ss[i] = s[i];
-    for (int i = tid; i < n / 32; i += nthreads) sb[i] = bsum[i];
+template <int UPL>
+__device__ __forceinline__ void qw_lane_load(int type, int nsb, const int8_t *q, const float *s, const int32_t *b16, int lane, QLane<UPL> &a) {
+    if (UPL == 2) qw_lane_pair(type, nsb, q, s, b16, lane, 0, a.x, a.ys);
+    else { a.q = q; a.s = s; a.b16 = b16; }
 }
-
-// ---------------------------------------------------------------- matvec over up to three stacked matrices (q|k|v, o-proj)
+// superblock terms of a row -> terms[0 .. nsb)
+template <int UPL>
+__device__ __forceinline__ void qw_row_terms(int type, int nsb, const unsigned char *row, QLane<UPL> &a, int lane, float *terms) {
+    const int g = lane >> 3, l8 = lane & 7;
+#pragma unroll 1
+    for (int i = 0; i < UPL; i += 2) {
+        const int sb0 = g + 4 * i, sb1 = sb0 + 4;
+        if (UPL > 2) qw_lane_pair(type, nsb, a.q, a.s, a.b16, lane, i, a.x, a.ys);
+        const float t = kq_pair_term(type, nsb, row, min(sb0, nsb - 1), a.x[0], a.ys[0], row, min(sb1, nsb - 1), a.x[1], a.ys[1], l8);
+        const int sb = l8 ? sb1 : sb0;
+        if (!(l8 & 3) && sb < nsb) terms[sb] = t;
+    }
+}
+__device__ __forceinline__ float qw_terms_sum(const float *t, int nsb) {      // superblocks in order, from zero
+    float v = 0.0f;
+    for (int i = 0; i < nsb; i++) v = __fadd_rn(v, t[i]);
+    return v;
+}
+// up to three matrices of equal width, stacked
 struct KStack {
     KMatDev m[3];
     float *y[3];
-    int n;
-    const int8_t *xq;          // Q8_K activation of the previous stage
-    const float *ys;
-    const int32_t *bsum;
-    // optional: K/V cache of the attention kernel that follows ([nkv][MAXSEQ][128] each): positions
-    // 0 .. pos-1 are requested into L2 ahead of time (last touched a whole step ago)
-    const float *pf_k, *pf_v;
-    int pf_nkv;
-    const DevState *state;
+    int n, rows, per_cta, stride;      // rows in all, rows per CTA, bytes per row in shared memory
+    __device__ int find(int row, int &local) const {
+        int i = 0;
+        while (i < n - 1 && row >= m[i].rows) { row -= m[i].rows; i++; }
+        local = row;
+        return i;
+    }
 };
-enum { KEPI_PLAIN = 0, KEPI_RESID = 1 };
 
-__device__ __forceinline__ void qw_l2_prefetch(const void *p, uint32_t n) {
-    asm volatile("cp.async.bulk.prefetch.L2.global [%0], %1;" ::"l"(p), "r"(n) : "memory");
-}
+struct QGemvArgs {
+    KStack k;
+    QFold f;                 // FOLD: the activation is the combined, normalised residual
+    const float *act;        // else: these floats, as they are; outputs are added to y
+    DevState *state;
+};
 
-template <int EPI, int UPL>
-__global__ void __launch_bounds__(256) qw_matvec_kernel(KStack a) {
+// Shared memory: rows | xf (FOLD: d floats) | q | scales | 16-sums | terms.
+// Bound: the hand-over, the prologue (combine, norm: 1.3 us) and one pass over rows that are already on chip (35 rows of 8 superblocks on
+// 16 warps: 0.7 us).
+template <int UPL, bool FOLD>
+__global__ void __launch_bounds__(QG_THREADS, 2) qw_gemv_kernel(const __grid_constant__ QGemvArgs a) {
     extern __shared__ __align__(16) unsigned char qsm[];
-    const int tid = threadIdx.x, lane = tid & 31;
-    int row = (blockIdx.x * 256 + tid) >> 5;
-    int mi = 0;
-    while (mi < a.n && row >= a.m[mi].rows) { row -= a.m[mi].rows; mi++; }
-    const bool live = mi < a.n;
-    const KMatDev &m = a.m[live ? mi : 0];
-    const int K = a.m[0].cols, nsb = K / 256;
-    KUnit u[UPL];
-    if (live) qw_row_load<UPL>(m, m.p + (size_t)row * m.bpr(), nsb, lane, u);          // static weights: before the wait
-    float resid = 0.0f;
-    if (EPI == KEPI_RESID && live && lane == 0) resid = a.y[mi][row];                      // written several kernels back
-    if (a.pf_k && a.state && tid == 0 && blockIdx.x < 2 * a.pf_nkv) {
-        const int pos = (int)a.state->pos;
-        const float *base = ((blockIdx.x & 1) ? a.pf_v : a.pf_k) + (size_t)(blockIdx.x >> 1) * BRRR_MAXSEQ * QW_HD;
-        for (int k = 0; k < pos; k += 64) qw_l2_prefetch(base + (size_t)k * QW_HD, (uint32_t)min(64, pos - k) * QW_HD * 4u);
-    }
-    pdl_wait();
-    pdl_trigger();
-    int8_t *sq = reinterpret_cast<int8_t *>(qsm);
-    float *ss = reinterpret_cast<float *>(qsm + K);
-    int32_t *sbs = reinterpret_cast<int32_t *>(ss + nsb);
-    qw_stage_q8k(a.xq, a.ys, a.bsum, K, sq, ss, sbs, tid, 256);
-    __syncthreads();
-    if (!live) return;
-    const float v = qw_row_sum<UPL>(m.type, u, nsb, lane, sq, ss, sbs);
-    if (lane == 0) a.y[mi][row] = EPI == KEPI_RESID ? __fadd_rn(resid, v) : v;
-}
-
-// ---------------------------------------------------------------- QK norm + RoPE + cache append (engine_qwen2.rs:353-362, 466-482)
-// One CTA of head_dim threads per q or k head.  Cache layout [kv head][position][head_dim].
-__global__ void __launch_bounds__(QW_HD) qw_qknorm_rope_kernel(float *__restrict__ q, const float *__restrict__ k, const float *__restrict__ v,
-                                                               const float *__restrict__ q_norm, const float *__restrict__ k_norm,
-                                                               const float *__restrict__ rope, float eps, int nh, int nkv,
-                                                               const DevState *__restrict__ state, int pos_val, float *__restrict__ kc,
-                                                               float *__restrict__ vc) {
-    __shared__ float raw[QW_HD], nv[QW_HD];
-    const int h = blockIdx.x, tid = threadIdx.x, hd = QW_HD, half = QW_HD / 2;
-    const int pos = state ? (int)state->pos : pos_val;
-    const bool is_q = h < nh;
-    const float *src = is_q ? q + h * hd : k + (h - nh) * hd;
-    const float wv = (is_q ? q_norm : k_norm)[tid];
-    const float co = rope[((size_t)pos * half + (tid % half)) * 2], si = rope[((size_t)pos * half + (tid % half)) * 2 + 1];
-    pdl_wait();
-    pdl_trigger();
-    raw[tid] = src[tid];
-    __syncthreads();
-    float ms = 0.0f;
-#pragma unroll 16
-    for (int i = 0; i < hd; i++) { float t = raw[i]; ms = __fadd_rn(ms, __fmul_rn(t, t)); }
-    const float inv = __fdiv_rn(1.0f, __fsqrt_rn(__fadd_rn(__fdiv_rn(ms, (float)hd), eps)));
-    nv[tid] = __fmul_rn(__fmul_rn(raw[tid], inv), wv);
-    __syncthreads();
-    const float aa = nv[tid % half], bb = nv[half + tid % half];
-    const float out = tid < half ? __fsub_rn(__fmul_rn(aa, co), __fmul_rn(bb, si)) : __fadd_rn(__fmul_rn(bb, co), __fmul_rn(aa, si));
-    if (is_q) q[h * hd + tid] = out;
-    else {
-        const int hh = h - nh;
-        const size_t o = ((size_t)hh * BRRR_MAXSEQ + pos) * hd + tid;
-        kc[o] = out;
-        vc[o] = v[hh * hd + tid];
-    }
-}
-
-// ---------------------------------------------------------------- attention (engine_qwen2.rs:365-389)
-// One CTA per pair of q heads (256 threads each).  score(t): 8 chains (chain c covers dims c, c+8,
-// ..., fused), combined as (c + c+4) per lane then (l0+l1)+(l2+l3), times 1/sqrt(128); softmax with
-// the running maximum taken over all keys; denominator and the 128 output sums serial over t.  The
-// two heads' outputs are one 256-value superblock of the o-proj's activation, quantised here
-// (Q8_K, engine_qwen2.rs:390).
-__global__ void __launch_bounds__(512) qw_attn_kernel(const float *__restrict__ q, const float *__restrict__ kc, const float *__restrict__ vc,
-                                                      int nh, int nkv, const DevState *__restrict__ state, int pos_val,
-                                                      int8_t *__restrict__ aq, float *__restrict__ as, int32_t *__restrict__ asum) {
-    extern __shared__ __align__(16) float asm_[];       // sc[2][MAXSEQ]
-    __shared__ float qs[2][QW_HD];
-    __shared__ float red[2][8];
-    __shared__ float den_sh[2];
-    __shared__ __align__(16) float outv[2 * QW_HD];
-    const int hh = threadIdx.x >> 8, tid = threadIdx.x & 255;
-    const int h = 2 * blockIdx.x + hh, kvh = h / (nh / nkv);
-    const int pos = state ? (int)state->pos : pos_val;
-    const int n = pos + 1;
-    float *sc = asm_ + hh * BRRR_MAXSEQ;
-    const float *kbase = kc + (size_t)kvh * BRRR_MAXSEQ * QW_HD, *vbase = vc + (size_t)kvh * BRRR_MAXSEQ * QW_HD;
-    auto bar_half = [&]() { asm volatile("bar.sync %0, 256;" ::"r"(1 + hh) : "memory"); };
-    pdl_wait();
-    pdl_trigger();
-    if (tid < QW_HD) qs[hh][tid] = q[h * QW_HD + tid];
-    bar_half();
-    {
-        const int g = tid >> 3, c = tid & 7;
-        float qr[16];
-#pragma unroll
-        for (int i = 0; i < 16; i++) qr[i] = qs[hh][8 * i + c];
-        const float scale = __fdiv_rn(1.0f, __fsqrt_rn((float)QW_HD));
-        for (int t0 = 0; t0 < n; t0 += 32) {
-            const int t = t0 + g;
-            const bool live = t < n;
-            float s = 0.0f;
-            if (live) {
-                const float *kp = kbase + (size_t)t * QW_HD + c;
-#pragma unroll
-                for (int i = 0; i < 16; i++) s = __fmaf_rn(kp[8 * i], qr[i], s);
+    __shared__ QFoldShared w;
+    __shared__ __align__(8) uint64_t bar;
+    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+    const int K = a.k.m[0].cols, nsb = K / 256, row0 = blockIdx.x * a.k.per_cta, n = min(a.k.per_cta, a.k.rows - row0);
+    unsigned char *rows = qsm;
+    float *xf = reinterpret_cast<float *>(qsm + (size_t)a.k.per_cta * a.k.stride);
+    int8_t *q = reinterpret_cast<int8_t *>(xf + (FOLD ? K : 0));
+    float *s = reinterpret_cast<float *>(q + K);
+    int32_t *b16 = reinterpret_cast<int32_t *>(s + ((nsb + 3) & ~3));
+    float *terms = reinterpret_cast<float *>(b16 + nsb * 16);
+    Waiter waiter(a.state ? &a.state->err : nullptr);
+    if (warp == 0) {
+        if (lane == 0) {
+            mbar_init(&bar, 1);
+            mbar_fence_init();
+            uint32_t bytes = 0;
+            for (int i = 0, r = row0, l; i < n;) {           // whole runs of a matrix
+                const int mi = a.k.find(r, l), run = min(n - i, a.k.m[mi].rows - l);
+                bytes += (uint32_t)run * (uint32_t)a.k.m[mi].bpr();
+                i += run; r += run;
             }
-            s = __fadd_rn(s, __shfl_xor_sync(0xffffffffu, s, 4));
-            s = __fadd_rn(s, __shfl_xor_sync(0xffffffffu, s, 1));
-            s = __fadd_rn(s, __shfl_xor_sync(0xffffffffu, s, 2));
-            if (live && c == 0) sc[t] = __fmul_rn(s, scale);
+            mbar_expect_tx(&bar, bytes);
+        }
+        __syncwarp();
+        for (int i = lane; i < n; i += 32) {
+            int l;
+            const KMatDev &m = a.k.m[a.k.find(row0 + i, l)];
+            bulk_g2s(rows + (size_t)i * a.k.stride, m.p + (size_t)l * m.bpr(), (uint32_t)m.bpr(), &bar);
         }
     }
-    bar_half();
+    float resid = 0.0f;
+    int my_l = 0;
+    const int my_m = tid < n ? a.k.find(row0 + tid, my_l) : 0;
+    if (!FOLD && tid < n) resid = a.k.y[my_m][my_l];         // written two kernels back
+    if (FOLD) qw_fold_routing(a.f, w, tid);
+    pdl_wait();
+    pdl_trigger();
+    if (FOLD) qw_fold_norm(a.f, w, xf, q, s, b16, blockIdx.x == 0, tid);
+    else
+        for (int sb = warp; sb < nsb; sb += QG_WARPS) {
+            const float4 *src = reinterpret_cast<const float4 *>(a.act + sb * 256 + lane * 8);
+            const float4 p0 = src[0], p1 = src[1];
+            const float v[8] = {p0.x, p0.y, p0.z, p0.w, p1.x, p1.y, p1.z, p1.w};
+            warp_quant_q8k16(v, lane, q + sb * 256, s + sb, b16 + sb * 16);
+        }
+    __syncthreads();
+    waiter.wait(&bar, 0u);
+    QLane<UPL> x;
+    int type = 0;
+    for (int i = warp; i < n; i += QG_WARPS) {
+        int l;
+        const int t = a.k.m[a.k.find(row0 + i, l)].type;
+        if (t != type) { type = t; qw_lane_load<UPL>(type, nsb, q, s, b16, lane, x); }
+        qw_row_terms<UPL>(type, nsb, rows + (size_t)i * a.k.stride, x, lane, terms + i * nsb);
+    }
+    __syncthreads();
+    if (tid < n) {
+        const float v = qw_terms_sum(terms + tid * nsb, nsb);
+        a.k.y[my_m][my_l] = FOLD ? v : __fadd_rn(resid, v);
+    }
+}
+
+// ---------------------------------------------------------------- attention (engine_qwen2.rs:353-389, 466-482)
+// One CTA per query head.  Prologue: QK norm (serial mean square) and RoPE of q and of the position's own k; the first head of a KV group
+// appends k and v to the cache.  score(t): 8 chains (chain c covers dims c, c+8, ..., fused), (c + c+4) per lane, (l0+l1)+(l2+l3), times
+// 1/sqrt(128); maximum over all keys; denominator and the 128 output sums serial over t.
+// K, then V of the cached positions run through one ring of 64-position tiles, a copy per position (rows 136 floats apart: the score
+// threads - (key, half of the chains) - read 16 bytes each from different banks).  The ring starts before the dependency wait.
+// Bound: the chains over the keys (4 cycles each) and 5 cycles of shared-memory reads per key; at 100 positions the prologue.
+constexpr int QA_TILE = 64, QA_STRIDE = 136, QA_SLOTS = 5, QA_THREADS = 288;
+constexpr size_t QA_SMEM = (size_t)QA_SLOTS * QA_TILE * QA_STRIDE * 4 + (size_t)BRRR_MAXSEQ * 4;
+
+struct QAttnArgs {
+    const float *q, *k, *v, *q_norm, *k_norm, *rope;
+    float eps;
+    float *kc, *vc;              // [nkv][MAXSEQ][128]
+    int nh, nkv;
+    DevState *state;
+    float *out;                  // [nh][128]
+};
+
+__device__ __forceinline__ float qa_half_score(const float *kp, const float *qp) {       // four chains of a key, then (c + c+4) with the other half's
+    float s0 = 0.0f, s1 = 0.0f, s2 = 0.0f, s3 = 0.0f;
+#pragma unroll
+    for (int i = 0; i < 16; i++) {
+        const float4 k = *reinterpret_cast<const float4 *>(kp + 8 * i), q = *reinterpret_cast<const float4 *>(qp + 8 * i);
+        s0 = __fmaf_rn(k.x, q.x, s0); s1 = __fmaf_rn(k.y, q.y, s1); s2 = __fmaf_rn(k.z, q.z, s2); s3 = __fmaf_rn(k.w, q.w, s3);
+    }
+    s0 = __fadd_rn(s0, __shfl_xor_sync(0xffffffffu, s0, 1)); s1 = __fadd_rn(s1, __shfl_xor_sync(0xffffffffu, s1, 1));
+    s2 = __fadd_rn(s2, __shfl_xor_sync(0xffffffffu, s2, 1)); s3 = __fadd_rn(s3, __shfl_xor_sync(0xffffffffu, s3, 1));
+    return __fadd_rn(__fadd_rn(s0, s1), __fadd_rn(s2, s3));
+}
+
+__global__ void __launch_bounds__(QA_THREADS) qw_attn_kernel(QAttnArgs a) {
+    extern __shared__ __align__(16) float asm_[];
+    float *ring = asm_, *sc = asm_ + QA_SLOTS * QA_TILE * QA_STRIDE;
+    __shared__ __align__(8) uint64_t full[QA_SLOTS], empty[QA_SLOTS];
+    __shared__ __align__(16) float raw[2][QW_HD], nv[2][QW_HD], qs[QW_HD], ks[QW_HD], vs[QW_HD];
+    __shared__ float red[8], inv_sh[2], den_sh;
+    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+    const int h = blockIdx.x, group = a.nh / a.nkv, kvh = h / group;
+    const int pos = (int)a.state->pos, n = pos + 1, nt = (pos + QA_TILE - 1) / QA_TILE;        // the position is an input of the step
+    float *kbase = a.kc + (size_t)kvh * BRRR_MAXSEQ * QW_HD, *vbase = a.vc + (size_t)kvh * BRRR_MAXSEQ * QW_HD;
+    Waiter waiter(&a.state->err);
+    if (tid == 256) {
+        for (int i = 0; i < QA_SLOTS; i++) { mbar_init(&full[i], 1); mbar_init(&empty[i], 4); }
+        mbar_fence_init();
+    }
+    float wv = 0.0f, co = 0.0f, si = 0.0f;
+    if (tid < 256) {
+        wv = (tid < QW_HD ? a.q_norm : a.k_norm)[tid & (QW_HD - 1)];
+        const float2 cs = reinterpret_cast<const float2 *>(a.rope)[(size_t)pos * (QW_HD / 2) + (tid & 63)];
+        co = cs.x; si = cs.y;
+    }
+    __syncthreads();
+    if (warp == 8) {
+        // ---- copies: K tiles, then V tiles
+        bool waited = false;
+        for (int t = 0; t < 2 * nt; t++) {
+            const int slot = t % QA_SLOTS, k0 = (t < nt ? t : t - nt) * QA_TILE, cnt = min(QA_TILE, pos - k0);
+            if (t >= QA_SLOTS) {
+                if (!waited) { pdl_wait(); pdl_trigger(); waiter.poison_if_failed(); waited = true; }      // with the others: the next kernel may start
+                waiter.wait(&empty[slot], (uint32_t)(t / QA_SLOTS - 1) & 1u);
+            }
+            if (lane == 0) mbar_expect_tx(&full[slot], (uint32_t)cnt * QW_HD * 4);
+            __syncwarp();
+            const float *src = (t < nt ? kbase : vbase) + (size_t)k0 * QW_HD;
+            for (int i = lane; i < cnt; i += 32) bulk_g2s(ring + (size_t)(slot * QA_TILE + i) * QA_STRIDE, src + (size_t)i * QW_HD, QW_HD * 4, &full[slot]);
+        }
+        if (!waited) { pdl_wait(); pdl_trigger(); }
+        return;
+    }
+    pdl_wait();
+    pdl_trigger();
+    waiter.poison_if_failed();
+    auto bar = [&]() { asm volatile("bar.sync 1, 256;" ::: "memory"); };
+    {
+        const int u = tid & (QW_HD - 1);
+        raw[tid >> 7][u] = tid < QW_HD ? a.q[h * QW_HD + u] : a.k[kvh * QW_HD + u];
+        if (tid < QW_HD) vs[u] = a.v[kvh * QW_HD + u];
+    }
+    bar();
+    if (tid == 0 || tid == 32) {
+        const float4 *r = reinterpret_cast<const float4 *>(raw[tid >> 5]);
+        float ms = 0.0f;
+#pragma unroll 8
+        for (int i = 0; i < QW_HD / 4; i++) {
+            const float4 t = r[i];
+            ms = __fadd_rn(ms, __fmul_rn(t.x, t.x)); ms = __fadd_rn(ms, __fmul_rn(t.y, t.y));
+            ms = __fadd_rn(ms, __fmul_rn(t.z, t.z)); ms = __fadd_rn(ms, __fmul_rn(t.w, t.w));
+        }
+        inv_sh[tid >> 5] = __fdiv_rn(1.0f, __fsqrt_rn(__fadd_rn(__fdiv_rn(ms, (float)QW_HD), a.eps)));
+    }
+    bar();
+    nv[tid >> 7][tid & (QW_HD - 1)] = __fmul_rn(__fmul_rn(raw[tid >> 7][tid & (QW_HD - 1)], inv_sh[tid >> 7]), wv);
+    bar();
+    {
+        const int u = tid & (QW_HD - 1), c = u & 63;
+        const float aa = nv[tid >> 7][c], bb = nv[tid >> 7][64 + c];
+        const float o = u < 64 ? __fsub_rn(__fmul_rn(aa, co), __fmul_rn(bb, si)) : __fadd_rn(__fmul_rn(bb, co), __fmul_rn(aa, si));
+        (tid < QW_HD ? qs : ks)[u] = o;
+        if (h % group == 0) {
+            if (tid >= QW_HD) kbase[(size_t)pos * QW_HD + u] = o;
+            else vbase[(size_t)pos * QW_HD + u] = vs[u];
+        }
+    }
+    bar();
+    // ---- scores: a group of four warps per tile, thread = (key, half of the chains)
+    const float scale = __fdiv_rn(1.0f, __fsqrt_rn((float)QW_HD));
+    const int hf = lane & 1, key = (warp & 3) * 16 + (lane >> 1);
+    for (int t = warp >> 2; t < nt; t += 2) {
+        const int slot = t % QA_SLOTS;
+        waiter.wait(&full[slot], (uint32_t)(t / QA_SLOTS) & 1u);
+        const float s = qa_half_score(ring + (size_t)(slot * QA_TILE + key) * QA_STRIDE + 4 * hf, qs + 4 * hf);
+        if (hf == 0 && t * QA_TILE + key < pos) sc[t * QA_TILE + key] = __fmul_rn(s, scale);
+        __syncwarp();
+        if (lane == 0) mbar_arrive(&empty[slot]);
+    }
+    if (warp == 7) {                 // the position itself
+        const float s = qa_half_score(ks + 4 * hf, qs + 4 * hf);
+        if (lane == 0) sc[pos] = __fmul_rn(s, scale);
+    }
+    bar();
     float mx = -3.402823466e+38f;
     for (int t = tid; t < n; t += 256) mx = fmaxf(mx, sc[t]);
     mx = warp_max(mx);
-    if ((tid & 31) == 0) red[hh][tid >> 5] = mx;
-    bar_half();
-    mx = red[hh][0];
+    if (lane == 0) red[warp] = mx;
+    bar();
+    mx = red[0];
 #pragma unroll
-    for (int w = 1; w < 8; w++) mx = fmaxf(mx, red[hh][w]);
-    for (int t = tid; t < n; t += 256) sc[t] = brrr_expf_dev(__fsub_rn(sc[t], mx));
-    bar_half();
+    for (int w = 1; w < 8; w++) mx = fmaxf(mx, red[w]);
+    for (int t = tid; t < ((n + 3) & ~3); t += 256) sc[t] = t < n ? brrr_expf_dev(__fsub_rn(sc[t], mx)) : 0.0f;      // +0 past the end changes no sum
+    bar();
     float acc = 0.0f;
-    if (tid == QW_HD) {
+    if (warp < 4) {
+        for (int t = 0; t < nt; t++) {
+            const int u = nt + t, slot = u % QA_SLOTS, cnt = min(QA_TILE, pos - t * QA_TILE);
+            waiter.wait(&full[slot], (uint32_t)(u / QA_SLOTS) & 1u);
+            const float *vt = ring + (size_t)slot * QA_TILE * QA_STRIDE + tid, *pt = sc + t * QA_TILE;
+            int k = 0;
+#pragma unroll 4
+            for (; k + 4 <= cnt; k += 4) {
+                const float4 p = *reinterpret_cast<const float4 *>(pt + k);
+                acc = __fmaf_rn(vt[k * QA_STRIDE], p.x, acc); acc = __fmaf_rn(vt[(k + 1) * QA_STRIDE], p.y, acc);
+                acc = __fmaf_rn(vt[(k + 2) * QA_STRIDE], p.z, acc); acc = __fmaf_rn(vt[(k + 3) * QA_STRIDE], p.w, acc);
+            }
+            for (; k < cnt; k++) acc = __fmaf_rn(vt[k * QA_STRIDE], pt[k], acc);
+            __syncwarp();
+            if (lane == 0) mbar_arrive(&empty[slot]);
+        }
+        acc = __fmaf_rn(vs[tid], sc[pos], acc);
+    } else if (tid == 128) {
         float den = 0.0f;
-#pragma unroll 8
-        for (int t = 0; t < n; t++) den = __fadd_rn(den, sc[t]);
-        den_sh[hh] = den;
-    } else if (tid < QW_HD) {
-        const float *vp = vbase + tid;
-#pragma unroll 8
-        for (int t = 0; t < n; t++) acc = __fmaf_rn(vp[(size_t)t * QW_HD], sc[t], acc);
+#pragma unroll 4
+        for (int t = 0; t < n; t += 4) {
+            const float4 p = *reinterpret_cast<const float4 *>(sc + t);
+            den = __fadd_rn(den, p.x); den = __fadd_rn(den, p.y); den = __fadd_rn(den, p.z); den = __fadd_rn(den, p.w);
+        }
+        den_sh = den;
     }
-    bar_half();
-    if (tid < QW_HD) outv[hh * QW_HD + tid] = __fmul_rn(acc, __fdiv_rn(1.0f, den_sh[hh]));
-    __syncthreads();
-    if (threadIdx.x < 32) {
-        const int lane = threadIdx.x;
-        const float4 a0 = reinterpret_cast<const float4 *>(outv)[lane * 2], a1 = reinterpret_cast<const float4 *>(outv)[lane * 2 + 1];
-        const float v[8] = {a0.x, a0.y, a0.z, a0.w, a1.x, a1.y, a1.z, a1.w};
-        warp_quant_q8k(v, lane, aq + (size_t)blockIdx.x * 256, as + blockIdx.x, asum + blockIdx.x * 8);
-    }
+    bar();
+    if (tid < QW_HD) a.out[h * QW_HD + tid] = __fmul_rn(acc, __fdiv_rn(1.0f, den_sh));
 }
 
-// ---------------------------------------------------------------- experts
-// gate/up rows of the selected experts and SiLU-GLU (engine_qwen2.rs:419-426): one warp per (slot, row).
-template <int UPL>
-__global__ void __launch_bounds__(256) qw_gate_up_kernel(KMatDev gate, KMatDev up, const int32_t *__restrict__ top, int topk, int ff,
-                                                         const int8_t *__restrict__ xq, const float *__restrict__ ys,
-                                                         const int32_t *__restrict__ bsum, float *__restrict__ hbuf) {
-    extern __shared__ __align__(16) unsigned char qsm[];
-    const int tid = threadIdx.x, lane = tid & 31;
-    const int it = (blockIdx.x * 256 + tid) >> 5;
-    const int K = gate.cols, nsb = K / 256;
-    const bool live = it < topk * ff;
-    pdl_wait();          // the routing comes from the kernel before this one
-    pdl_trigger();
-    KUnit ug[UPL], uu[UPL];
-    int ei = 0, r = 0;
-    if (live) {
-        ei = it / ff; r = it % ff;
-        const size_t gr = (size_t)top[ei] * ff + r;
-        qw_row_load<UPL>(gate, gate.p + gr * gate.bpr(), nsb, lane, ug);
-        qw_row_load<UPL>(up, up.p + gr * up.bpr(), nsb, lane, uu);
-    }
-    int8_t *sq = reinterpret_cast<int8_t *>(qsm);
-    float *ss = reinterpret_cast<float *>(qsm + K);
-    int32_t *sbs = reinterpret_cast<int32_t *>(ss + nsb);
-    qw_stage_q8k(xq, ys, bsum, K, sq, ss, sbs, tid, 256);
-    __syncthreads();
-    if (!live) return;
-    const float g = qw_row_sum<UPL>(gate.type, ug, nsb, lane, sq, ss, sbs), u = qw_row_sum<UPL>(up.type, uu, nsb, lane, sq, ss, sbs);
-    if (lane == 0) hbuf[it] = __fmul_rn(__fdiv_rn(g, __fadd_rn(1.0f, brrr_expf_dev(-g))), u);
-}
-
-// down-projection and weighted accumulate in slot order (engine_qwen2.rs:432-441): one warp per
-// output row, all (slot, superblock) units of the row in registers before the dependency wait (the
-// routing is two kernels old by then).  Prologue: Q8_K of h (every CTA quantises all of it: 24 KB
-// from L2).  Epilogue: the last CTA to finish normalises and quantises the finished residual for
-// the next consumer (next layer's q|k|v, or the vocabulary head).
-struct QDownArgs {
-    KMatDev down;
-    const int32_t *top;
-    const float *wts;
-    int topk, d, ff;
-    const float *hbuf;
-    float *x;
-    unsigned int *counter;           // arrival counter, zero between launches
-    const float *next_norm_w;        // nullable: no norm epilogue
+// ---------------------------------------------------------------- routing hint
+// One CTA per expert: an order-free estimate of its router logit (a few ulps from the serial chain), which only decides whose weights start
+// moving (see qw_fold_routing), and a share of the normalised token's Q8_K.  The router row and the norm weights are in registers before
+// the dependency wait.
+constexpr int QH_THREADS = 128, QH_MAXG = 8;
+struct QHintArgs {
+    const float *x, *norm_w;
     float eps;
-    int8_t *nq; float *ns; int32_t *nsum;
+    int d, ne;
+    const float *Wt;             // tiled router matrix
+    float *est;
+    int8_t *q;
+    float *s;
+    int32_t *b16;
 };
 
-template <int NSBF>
-__global__ void __launch_bounds__(256) qw_down_kernel(QDownArgs a) {
-    extern __shared__ __align__(16) unsigned char qsm[];
-    constexpr int UPL = 2 * NSBF;                    // units per lane: up to 8 slots x NSBF superblocks over 4 lane groups
-    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, g = lane >> 3, l8 = lane & 7;
-    const int r = blockIdx.x * 8 + warp;
-    const int nun = a.topk * NSBF, hn = a.topk * a.ff;
-    __shared__ int last_sh;
-    __shared__ float part[QW_NT];
-    KUnit u[UPL];
-    float w[8];
-    if (r < a.d) {
+__global__ void __launch_bounds__(QH_THREADS) qw_hint_kernel(QHintArgs a) {
+    extern __shared__ __align__(16) float xf[];
+    __shared__ float part[QW_NT], red[QH_THREADS / 32];
+    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, e = blockIdx.x, d = a.d, groups = d >> 2;
+    const int ntiles = (d + RT_TJ - 1) / RT_TJ;
+    const float *wrow = a.Wt + ((size_t)(e >> 5) * ntiles * 32 + (e & 31)) * RT_STRIDE;
+    float4 w[QH_MAXG];           // router weight x norm weight
 #pragma unroll
-        for (int i = 0; i < UPL; i++) {
-            const int ui = g + 4 * i;
-            if (ui < nun) {
-                const int ei = ui / NSBF, sb = ui % NSBF;
-                kq_unit_load(a.down, a.down.p + ((size_t)a.top[ei] * a.d + r) * a.down.bpr(), sb, l8, u[i]);
-            }
+    for (int p = 0; p < QH_MAXG; p++) {
+        const int g = tid + p * QH_THREADS;
+        w[p] = make_float4(0.f, 0.f, 0.f, 0.f);
+        if (g < groups) {
+            const int j = g * 4, t = j / RT_TJ, jj = j % RT_TJ;
+            const float4 r = *reinterpret_cast<const float4 *>(wrow + (size_t)t * RT_TILE_FLOATS + jj), n = reinterpret_cast<const float4 *>(a.norm_w)[g];
+            w[p] = make_float4(r.x * n.x, r.y * n.y, r.z * n.z, r.w * n.w);
+        }
+    }
+    pdl_wait();
+    pdl_trigger();
+    stage_vec4(a.x, xf, d, tid, QH_THREADS);
+    __syncthreads();
+    float dot = 0.0f;
+#pragma unroll
+    for (int p = 0; p < QH_MAXG; p++) {
+        const int g = tid + p * QH_THREADS;
+        if (g < groups) {
+            const float4 x = reinterpret_cast<const float4 *>(xf)[g];
+            dot += w[p].x * x.x + w[p].y * x.y + w[p].z * x.z + w[p].w * x.w;
         }
     }
 #pragma unroll
-    for (int k = 0; k < 8; k++) w[k] = k < a.topk ? a.wts[k] : 0.0f;
-    float acc = r < a.d ? a.x[r] : 0.0f;
+    for (int o = 16; o > 0; o >>= 1) dot += __shfl_xor_sync(0xffffffffu, dot, o);
+    if (lane == 0) red[warp] = dot;
+    const float inv = qw_norm_inv(xf, d, a.eps, part, tid);
+    if (tid == 0) a.est[e] = inv * (red[0] + red[1] + red[2] + red[3]);
+    for (int sb = e + warp * gridDim.x; sb < d / 256; sb += gridDim.x * (QH_THREADS / 32)) {
+        float v[8];
+#pragma unroll
+        for (int i = 0; i < 8; i++) v[i] = __fmul_rn(__fmul_rn(xf[sb * 256 + lane * 8 + i], inv), a.norm_w[sb * 256 + lane * 8 + i]);
+        warp_quant_q8k16(v, lane, a.q + sb * 256, a.s + sb, a.b16 + sb * 16);
+    }
+}
+
+// ---------------------------------------------------------------- experts: gate/up + SiLU-GLU (engine_qwen2.rs:419-426)
+// The (slot, row) pairs of gate and up rows are dealt out in runs, so that every SM streams the same bytes (42 pairs, 97 KB); the rows land
+// in groups of sixteen, a row of each matrix per warp.  Nothing is known before the wait: est picks the experts here.
+struct QGateUpArgs {
+    KMatDev gate, up;
+    const float *est;            // nullptr: top
+    const int32_t *top;
+    int ne, topk, ff, per_cta, stride_g, stride_u;
+    const int8_t *q;
+    const float *s;
+    const int32_t *b16;
+    float *hbuf;                 // [slot][ff]
+    DevState *state;
+};
+
+template <int UPL>
+__global__ void __launch_bounds__(QG_THREADS, 2) qw_gate_up_kernel(const __grid_constant__ QGateUpArgs a) {
+    extern __shared__ __align__(16) unsigned char qsm[];
+    __shared__ SelectScratch ws;
+    __shared__ int sel[8];
+    __shared__ __align__(8) uint64_t bar[16];
+    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, K = a.gate.cols, nsb = K / 256;
+    const int i0 = blockIdx.x * a.per_cta, n = min(a.per_cta, a.topk * a.ff - i0), groups = (n + QG_WARPS - 1) / QG_WARPS;
+    unsigned char *rg = qsm, *ru = qsm + (size_t)a.per_cta * a.stride_g;
+    int8_t *q = reinterpret_cast<int8_t *>(ru + (size_t)a.per_cta * a.stride_u);
+    float *s = reinterpret_cast<float *>(q + K);
+    int32_t *b16 = reinterpret_cast<int32_t *>(s + ((nsb + 3) & ~3));
+    float *terms = reinterpret_cast<float *>(b16 + nsb * 16);      // [row][gate, up][nsb]
+    Waiter waiter(a.state ? &a.state->err : nullptr);
+    if (tid == 0) {
+        for (int i = 0; i < groups; i++) mbar_init(&bar[i], 1);
+        mbar_fence_init();
+    }
+    pdl_wait();
+    pdl_trigger();
+    waiter.poison_if_failed();
+    for (int i = tid; i < K / 16; i += QG_THREADS) reinterpret_cast<int4 *>(q)[i] = reinterpret_cast<const int4 *>(a.q)[i];
+    for (int i = tid; i < nsb; i += QG_THREADS) s[i] = a.s[i];
+    for (int i = tid; i < nsb * 16; i += QG_THREADS) b16[i] = a.b16[i];
+    if (a.est) qw_select(a.est, a.ne, a.topk, a.state, ws, sel, tid, QG_THREADS);
+    else { if (tid < a.topk) sel[tid] = a.top[tid]; __syncthreads(); }
+    if (tid < groups) mbar_expect_tx(&bar[tid], (uint32_t)min(QG_WARPS, n - tid * QG_WARPS) * (uint32_t)(a.stride_g + a.stride_u));
+    for (int i = tid; i < 2 * n; i += QG_THREADS) {
+        const int r = i >> 1, it = i0 + r, ei = it / a.ff;
+        const size_t row = (size_t)sel[ei] * a.ff + (it - ei * a.ff);
+        if (i & 1) bulk_g2s(ru + (size_t)r * a.stride_u, a.up.p + row * a.stride_u, (uint32_t)a.stride_u, &bar[r / QG_WARPS]);
+        else bulk_g2s(rg + (size_t)r * a.stride_g, a.gate.p + row * a.stride_g, (uint32_t)a.stride_g, &bar[r / QG_WARPS]);
+    }
+    QLane<UPL> x;
+    qw_lane_load<UPL>(a.gate.type, nsb, q, s, b16, lane, x);
+    for (int k = 0; k < groups; k++) {
+        const int i = k * QG_WARPS + warp;
+        if (i >= n) break;
+        waiter.wait(&bar[k], 0u);
+        qw_row_terms<UPL>(a.gate.type, nsb, rg + (size_t)i * a.stride_g, x, lane, terms + (size_t)i * 2 * nsb);
+        if (a.up.type != a.gate.type) qw_lane_load<UPL>(a.up.type, nsb, q, s, b16, lane, x);
+        qw_row_terms<UPL>(a.up.type, nsb, ru + (size_t)i * a.stride_u, x, lane, terms + (size_t)i * 2 * nsb + nsb);
+        if (a.up.type != a.gate.type) qw_lane_load<UPL>(a.gate.type, nsb, q, s, b16, lane, x);
+    }
+    __syncthreads();
+    if (tid < n) {
+        const float g = qw_terms_sum(terms + (size_t)tid * 2 * nsb, nsb), u = qw_terms_sum(terms + (size_t)tid * 2 * nsb + nsb, nsb);
+        a.hbuf[i0 + tid] = __fmul_rn(__fdiv_rn(g, __fadd_rn(1.0f, brrr_expf_dev(-g))), u);
+    }
+}
+
+// ---------------------------------------------------------------- down projection of every slot (engine_qwen2.rs:432-441)
+// A CTA owns per_cta rows of each of the slots' matrices: contiguous in memory, fetched before the wait (the routing is two kernels
+// old).  Prologue: Q8_K of h (every CTA all of it: 24 KB from L2).  part[slot][row] = dot; the weights and the order of the combine come
+// later (QFold).
+struct QDownArgs {
+    KMatDev down;
+    const float *est;
+    const int32_t *top;
+    int ne, topk, d, ff, per_cta;
+    const float *hbuf;
+    float *part;
+    DevState *state;
+};
+
+__global__ void __launch_bounds__(QG_THREADS, 2) qw_down_kernel(const __grid_constant__ QDownArgs a) {
+    extern __shared__ __align__(16) unsigned char qsm[];
+    __shared__ SelectScratch ws;
+    __shared__ int sel[8];
+    __shared__ __align__(8) uint64_t bar;
+    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, g = lane >> 3, l8 = lane & 7;
+    const int nsb = a.ff / 256, nun = a.topk * nsb, rb = (int)a.down.bpr(), r0 = blockIdx.x * a.per_cta, n = min(a.per_cta, a.d - r0);
+    unsigned char *rows = qsm;                                         // [slot][row]
+    int8_t *q = reinterpret_cast<int8_t *>(rows + (size_t)a.topk * a.per_cta * rb);
+    float *s = reinterpret_cast<float *>(q + nun * 256);
+    int32_t *b16 = reinterpret_cast<int32_t *>(s + ((nun + 3) & ~3));
+    float *terms = reinterpret_cast<float *>(b16 + nun * 16);          // [row][slot][nsb]
+    Waiter waiter(a.state ? &a.state->err : nullptr);
+    if (tid == 0) { mbar_init(&bar, 1); mbar_fence_init(); }
+    if (a.est) qw_select(a.est, a.ne, a.topk, a.state, ws, sel, tid, QG_THREADS);
+    else { if (tid < a.topk) sel[tid] = a.top[tid]; __syncthreads(); }
+    if (tid == 0) mbar_expect_tx(&bar, (uint32_t)a.topk * n * rb);
+    if (tid < a.topk) bulk_g2s(rows + (size_t)tid * a.per_cta * rb, a.down.p + ((size_t)sel[tid] * a.d + r0) * rb, (uint32_t)n * rb, &bar);
     pdl_wait();          // h is complete
     pdl_trigger();
-    int8_t *sq = reinterpret_cast<int8_t *>(qsm);
-    float *ss = reinterpret_cast<float *>(qsm + hn);
-    int32_t *sbs = reinterpret_cast<int32_t *>(ss + hn / 256);
-    for (int sb = warp; sb < hn / 256; sb += 8) {
+    waiter.poison_if_failed();
+    for (int sb = warp; sb < nun; sb += QG_WARPS) {
         const float4 *src = reinterpret_cast<const float4 *>(a.hbuf + (size_t)sb * 256 + lane * 8);
         const float4 p0 = src[0], p1 = src[1];
         const float v[8] = {p0.x, p0.y, p0.z, p0.w, p1.x, p1.y, p1.z, p1.w};
-        warp_quant_q8k(v, lane, sq + sb * 256, ss + sb, sbs + sb * 8);
+        warp_quant_q8k16(v, lane, q + sb * 256, s + sb, b16 + sb * 16);
     }
     __syncthreads();
-    if (r < a.d) {
-        const unsigned gmask = 0xFFu << (8 * g);
-        float tv[UPL];
-#pragma unroll
-        for (int i = 0; i < UPL; i++) {
-            const int ui = g + 4 * i;
-            tv[i] = 0.0f;
-            if (ui < nun) {
-                const int ei = ui / NSBF, sb = ui % NSBF, hsb = ei * NSBF + sb;
-                tv[i] = kq_unit_term(a.down.type, u[i], l8, sq + hsb * 256, ss[hsb], sbs + hsb * 8, gmask);
-            }
-        }
-        // slot ei: dot = ((0 + t0) + t1) + ...; x += w[ei] * dot, slots in order
-        float dot = 0.0f;
-#pragma unroll
-        for (int ui = 0; ui < 4 * UPL; ui++) {
-            const float t = __shfl_sync(0xffffffffu, tv[ui / 4], 8 * (ui % 4));
-            if (ui < nun) {
-                dot = __fadd_rn(dot, t);
-                if (ui % NSBF == NSBF - 1) { acc = __fadd_rn(acc, __fmul_rn(w[ui / NSBF], dot)); dot = 0.0f; }
-            }
-        }
-        if (lane == 0) a.x[r] = acc;
-    }
-    if (!a.next_norm_w) return;
-    // ---- the last CTA to finish: RMS norm (12 slices, engine_qwen2.rs:453-465) + Q8_K of the whole residual
-    __threadfence();
-    __syncthreads();
-    if (tid == 0) last_sh = atomicAdd(a.counter, 1u) == gridDim.x - 1;
-    __syncthreads();
-    if (!last_sh) return;
-    __threadfence();
-    float *xs_sh = reinterpret_cast<float *>(qsm);          // d floats (the Q8_K image of h is no longer needed)
-    for (int i = tid; i < a.d / 4; i += 256) reinterpret_cast<float4 *>(xs_sh)[i] = __ldcg(reinterpret_cast<const float4 *>(a.x) + i);
-    __syncthreads();
-    if (tid < QW_NT) {
-        int lo, hi;
-        qw_slice(tid, a.d, lo, hi);
-        float ps = 0.0f;
-#pragma unroll 8
-        for (int i = lo; i < hi; i++) { const float v = xs_sh[i]; ps = __fadd_rn(ps, __fmul_rn(v, v)); }
-        part[tid] = ps;
+    waiter.wait(&bar, 0u);
+    // (row, eight units) at a time: unit = slot * nsb + superblock
+    const int per_row = (nun + 7) / 8, type = a.down.type;
+    for (int it = warp; it < n * per_row; it += QG_WARPS) {
+        const int r = it / per_row, u0 = (it - r * per_row) * 8 + g, u1 = u0 + 4, c0 = min(u0, nun - 1), c1 = min(u1, nun - 1);
+        KAct x0, x1;
+        kact_load(type, q + c0 * 256, b16 + c0 * 16, l8, x0);
+        kact_load(type, q + c1 * 256, b16 + c1 * 16, l8, x1);
+        const int e0 = c0 / nsb, e1 = c1 / nsb;
+        const float t = kq_pair_term(type, nsb, rows + ((size_t)e0 * a.per_cta + r) * rb, c0 - e0 * nsb, x0, s[c0], rows + ((size_t)e1 * a.per_cta + r) * rb, c1 - e1 * nsb, x1,
+                                     s[c1], l8);
+        const int u = l8 ? u1 : u0;
+        if (!(l8 & 3) && u < nun) terms[r * nun + u] = t;
     }
     __syncthreads();
-    float tot = 0.0f;
-#pragma unroll
-    for (int k = 0; k < QW_NT; k++) tot = __fadd_rn(tot, part[k]);
-    const float inv = __fdiv_rn(1.0f, __fsqrt_rn(__fadd_rn(__fdiv_rn(tot, (float)a.d), a.eps)));
-    for (int sb = warp; sb < a.d / 256; sb += 8) {
-        float v[8];
-#pragma unroll
-        for (int i = 0; i < 8; i++) {
-            const int idx = sb * 256 + lane * 8 + i;
-            v[i] = __fmul_rn(__fmul_rn(xs_sh[idx], inv), a.next_norm_w[idx]);
-        }
-        warp_quant_q8k(v, lane, a.nq + sb * 256, a.ns + sb, a.nsum + sb * 8);
+    for (int i = tid; i < n * a.topk; i += QG_THREADS) {
+        const int slot = i / n, r = i - slot * n;
+        a.part[(size_t)slot * a.d + r0 + r] = qw_terms_sum(terms + r * nun + slot * nsb, nsb);
     }
-    if (tid == 0) *a.counter = 0u;
 }
 
 // ---------------------------------------------------------------- vocabulary projection + argmax (engine_qwen2.rs:436-448)
+// Persistent: a CTA streams its run of rows through a ring of 16-row stages, a row per warp; the ring fills before the dependency wait.
+// Bound: HBM (255 MB at 151936 x 2048).
+struct QHeadArgs {
+    KMatDev m;
+    const int8_t *q;
+    const float *s;
+    const int32_t *b16;
+    float *logits;
+    DevState *state;
+    int per_cta, depth;
+};
+
 template <int UPL>
-__global__ void __launch_bounds__(256) qw_head_kernel(KMatDev head, const int8_t *__restrict__ xq, const float *__restrict__ ys,
-                                                      const int32_t *__restrict__ bsum, float *__restrict__ logits, DevState *state) {
+__global__ void __launch_bounds__(QG_THREADS + 32) qw_head_kernel(const __grid_constant__ QHeadArgs a) {
     extern __shared__ __align__(16) unsigned char qsm[];
-    __shared__ unsigned long long wbest[8];
-    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-    const int K = head.cols, nsb = K / 256;
-    int8_t *sq = reinterpret_cast<int8_t *>(qsm);
-    float *ss = reinterpret_cast<float *>(qsm + K);
-    int32_t *sbs = reinterpret_cast<int32_t *>(ss + nsb);
-    // a CTA walks QW_HEAD_ROWS rows, eight at a time, the next eight rows' units in flight while the current ones are summed
-    const int row0 = blockIdx.x * QW_HEAD_ROWS;
-    KUnit u[UPL], un[UPL];
-    int row = row0 + warp;
-    if (row < head.rows) qw_row_load<UPL>(head, head.p + (size_t)row * head.bpr(), nsb, lane, u);
+    __shared__ __align__(8) uint64_t full[8], empty[8];
+    __shared__ unsigned long long wbest[QG_WARPS];
+    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, nsb = a.m.cols / 256, rb = (int)a.m.bpr(), depth = a.depth;
+    const int row0 = blockIdx.x * a.per_cta, n = min(a.per_cta, a.m.rows - row0), stages = (n + QG_WARPS - 1) / QG_WARPS;
+    Waiter waiter(&a.state->err);
+    if (tid == 0) {
+        for (int i = 0; i < depth; i++) { mbar_init(&full[i], 1); mbar_init(&empty[i], QG_WARPS); }
+        mbar_fence_init();
+    }
+    __syncthreads();
+    if (warp == QG_WARPS) {
+        if (lane == 0) {
+            pdl_trigger();
+            for (int t = 0; t < stages; t++) {
+                const int slot = t % depth;
+                if (t >= depth) waiter.wait(&empty[slot], (uint32_t)(t / depth - 1) & 1u);
+                const uint32_t bytes = (uint32_t)min(QG_WARPS, n - t * QG_WARPS) * rb;
+                mbar_expect_tx(&full[slot], bytes);
+                bulk_g2s(qsm + (size_t)slot * QG_WARPS * rb, a.m.p + (size_t)(row0 + t * QG_WARPS) * rb, bytes, &full[slot]);
+            }
+        }
+        return;
+    }
     pdl_wait();
     pdl_trigger();
-    qw_stage_q8k(xq, ys, bsum, K, sq, ss, sbs, tid, 256);
-    __syncthreads();
+    waiter.poison_if_failed();
+    QLane<UPL> x;
+    qw_lane_load<UPL>(a.m.type, nsb, a.q, a.s, a.b16, lane, x);
+    float *terms = reinterpret_cast<float *>(qsm + (size_t)depth * QG_WARPS * rb) + warp * 2 * nsb;      // the warp's own, two rows
     unsigned long long best = 0ull;
-    for (int i = 0; i < QW_HEAD_ROWS; i += 8) {
-        const int nrow = row + 8;
-        const bool more = i + 8 < QW_HEAD_ROWS && nrow < head.rows;
-        if (more) qw_row_load<UPL>(head, head.p + (size_t)nrow * head.bpr(), nsb, lane, un);
-        if (row < head.rows) {
-            const float v = qw_row_sum<UPL>(head.type, u, nsb, lane, sq, ss, sbs);
-            if (lane == 0) logits[row] = v;
-            const unsigned long long key = ((unsigned long long)float_orderable(v) << 32) | (0xFFFFFFFFu - (uint32_t)row);
-            best = key > best ? key : best;
+    for (int t = 0; t < stages; t++) {
+        const int slot = t % depth, i = t * QG_WARPS + warp;
+        waiter.wait(&full[slot], (uint32_t)(t / depth) & 1u);
+        float *tr = terms + (t & 1) * nsb;
+        if (i < n) qw_row_terms<UPL>(a.m.type, nsb, qsm + (size_t)(slot * QG_WARPS + warp) * rb, x, lane, tr);
+        __syncwarp();
+        if (lane == 0) {
+            mbar_arrive(&empty[slot]);
+            if (i < n) {
+                const float v = qw_terms_sum(tr, nsb);
+                a.logits[row0 + i] = v;
+                const unsigned long long key = ((unsigned long long)float_orderable(v) << 32) | (0xFFFFFFFFu - (uint32_t)(row0 + i));
+                best = key > best ? key : best;
+            }
         }
-        if (more) {
-#pragma unroll
-            for (int k = 0; k < UPL; k++) u[k] = un[k];
-        }
-        row = nrow;
     }
     if (lane == 0) wbest[warp] = best;
-    __syncthreads();
+    asm volatile("bar.sync 1, %0;" ::"r"(QG_THREADS) : "memory");
     if (tid == 0) {
 #pragma unroll
-        for (int w = 1; w < 8; w++) best = wbest[w] > best ? wbest[w] : best;
-        if (best) atomicMax(&state->best, best);
+        for (int w = 1; w < QG_WARPS; w++) best = wbest[w] > best ? wbest[w] : best;
+        if (best) atomicMax(&a.state->best, best);
     }
 }
 
@@ -499,105 +761,131 @@ __global__ void q6k_planes_kernel(const uint8_t *__restrict__ src, size_t rows, 
     }
 }
 
+// units per lane for rows of nsb superblocks: 2 or 4 (nsb <= 16)
+int qw_upl(int nsb) { return nsb <= 8 ? 2 : nsb <= 16 ? 4 : 0; }
+size_t qw_act_bytes(int nsb) { return (size_t)nsb * 256 + (size_t)((nsb + 3) & ~3) * 4 + (size_t)nsb * 64; }
+bool qw_type_ok(const KMatDev &m) { return m.type == 12 || (m.type == 14 && m.planes); }
+int qw_rows_per_cta(int rows, size_t bytes_per_row) {      // an even share of 148 SMs, unless that takes more shared memory than two kernels can share
+    const int share = (rows + 147) / 148, fit = (int)(QG_ROW_BYTES / bytes_per_row);
+    return share < fit ? share : fit;
+}
+constexpr int QG_SMEM_MAX = 200 * 1024;
+
+template <int UPL, bool FOLD>
+cudaError_t qw_gemv_launch(const QGemvArgs &a, size_t smem, bool pdl, cudaStream_t st) {
+    static unsigned long long configured = 0;      // one bit per device
+    cudaError_t e = smem_optin(qw_gemv_kernel<UPL, FOLD>, QG_SMEM_MAX, configured);
+    if (e != cudaSuccess) return e;
+    return launch_k(qw_gemv_kernel<UPL, FOLD>, dim3((a.k.rows + a.k.per_cta - 1) / a.k.per_cta), dim3(QG_THREADS), smem, st, pdl, a);
+}
+
+cudaError_t qw_gemv(const KMatDev *mats, float *const *ys_out, int n, const QFold *f, const float *act, DevState *state, bool pdl, cudaStream_t st) {
+    QGemvArgs a{};
+    a.k.n = n;
+    size_t stride = 0;
+    for (int i = 0; i < n; i++) {
+        a.k.m[i] = mats[i]; a.k.y[i] = ys_out[i]; a.k.rows += mats[i].rows;
+        if (mats[i].bpr() > stride) stride = mats[i].bpr();
+        if (mats[i].cols != mats[0].cols || !qw_type_ok(mats[i])) return cudaErrorInvalidValue;
+    }
+    const int K = mats[0].cols, nsb = K / 256, upl = qw_upl(nsb);
+    if (!upl || (f && (f->d != K || f->topk > 8 || f->ne > 256))) return cudaErrorInvalidValue;
+    a.k.stride = (int)stride;
+    a.k.per_cta = qw_rows_per_cta(a.k.rows, stride + nsb * 4);
+    if (f) a.f = *f;
+    a.act = act; a.state = state;
+    const size_t smem = (size_t)a.k.per_cta * (stride + nsb * 4) + qw_act_bytes(nsb) + (f ? (size_t)K * 4 : 0);
+    if (f) return upl == 2 ? qw_gemv_launch<2, true>(a, smem, pdl, st) : qw_gemv_launch<4, true>(a, smem, pdl, st);
+    return upl == 2 ? qw_gemv_launch<2, false>(a, smem, pdl, st) : qw_gemv_launch<4, false>(a, smem, pdl, st);
+}
+
+template <int UPL>
+cudaError_t qw_gate_up_launch(const QGateUpArgs &a, size_t smem, bool pdl, cudaStream_t st) {
+    static unsigned long long configured = 0;      // one bit per device
+    cudaError_t e = smem_optin(qw_gate_up_kernel<UPL>, QG_SMEM_MAX, configured);
+    if (e != cudaSuccess) return e;
+    return launch_k(qw_gate_up_kernel<UPL>, dim3((a.topk * a.ff + a.per_cta - 1) / a.per_cta), dim3(QG_THREADS), smem, st, pdl, a);
+}
+template <int UPL>
+cudaError_t qw_head_launch(const QHeadArgs &a, size_t smem, bool pdl, cudaStream_t st) {
+    static unsigned long long configured = 0;      // one bit per device
+    cudaError_t e = smem_optin(qw_head_kernel<UPL>, 224 * 1024, configured);
+    if (e != cudaSuccess) return e;
+    return launch_k(qw_head_kernel<UPL>, dim3((a.m.rows + a.per_cta - 1) / a.per_cta), dim3(QG_THREADS + 32), smem, st, pdl, a);
+}
+QFold qw_fold_args(const QwCombine &c) { return QFold{c.x_in, c.part, c.x_out, c.est, c.top, c.wts, c.ne, c.topk, c.d, c.seq, c.norm_w, c.eps, c.state}; }
+
 }  // namespace
 
 // ---------------------------------------------------------------- launchers
-cudaError_t launch_qw_embed(const uint8_t *embd, int d, const DevState *state, float *x, bool pdl, cudaStream_t st) {
+cudaError_t launch_qw_embed(const uint8_t *embd, int d, DevState *state, float *x, bool pdl, cudaStream_t st) {
     return launch_k(qw_embed_kernel, dim3(d / 256), dim3(256), 0, st, pdl, embd, d, state, x);
 }
 
-cudaError_t launch_qw_norm_quant(const float *x, const float *w, float eps, int d, float *xn, int8_t *q, float *s, int32_t *bsum,
-                                 bool pdl, cudaStream_t st) {
-    return launch_k(qw_norm_quant_kernel, dim3(1), dim3(256), (size_t)d * 4, st, pdl, x, w, eps, d, xn, q, s, bsum);
+cudaError_t launch_qw_fold(const QwCombine &c, int8_t *q, float *s, int32_t *b16, bool pdl, cudaStream_t st) {
+    if (c.topk > 8 || c.ne > 256 || c.d > 8192) return cudaErrorInvalidValue;
+    return launch_k(qw_fold_kernel, dim3(1), dim3(QG_THREADS), (size_t)c.d * 4, st, pdl, qw_fold_args(c), q, s, b16);
 }
 
-// units per lane for rows of nsb superblocks: 1, 2 or 4 (nsb <= 16)
-static int qw_upl(int nsb) { return nsb <= 4 ? 1 : nsb <= 8 ? 2 : nsb <= 16 ? 4 : 0; }
-static size_t qw_act_smem(int K) { return (size_t)K + (size_t)(K / 256) * 4 + (size_t)(K / 32) * 4; }
-
-template <int EPI>
-static cudaError_t qw_matvec_launch(const KStack &a, int upl, dim3 grid, size_t smem, bool pdl, cudaStream_t st) {
-    switch (upl) {
-    case 1: return launch_k(qw_matvec_kernel<EPI, 1>, grid, dim3(256), smem, st, pdl, a);
-    case 2: return launch_k(qw_matvec_kernel<EPI, 2>, grid, dim3(256), smem, st, pdl, a);
-    case 4: return launch_k(qw_matvec_kernel<EPI, 4>, grid, dim3(256), smem, st, pdl, a);
-    }
-    return cudaErrorInvalidValue;
+cudaError_t launch_qw_qkv(const KMatDev *mats, float *const *ys_out, const QwCombine &c, bool pdl, cudaStream_t st) {
+    const QFold f = qw_fold_args(c);
+    return qw_gemv(mats, ys_out, 3, &f, nullptr, c.state, pdl, st);
 }
 
-cudaError_t launch_qw_matvec(const KMatDev *mats, float *const *ys_out, int n, bool resid, const int8_t *xq, const float *ys,
-                             const int32_t *bsum, bool pdl, cudaStream_t st, const float *pf_k, const float *pf_v, int pf_nkv,
-                             const DevState *state) {
-    KStack a{};
-    int rows = 0;
-    a.n = n;
-    for (int i = 0; i < n; i++) {
-        a.m[i] = mats[i]; a.y[i] = ys_out[i]; rows += mats[i].rows;
-        if (mats[i].cols != mats[0].cols || (mats[i].type == 14 && !mats[i].planes)) return cudaErrorInvalidValue;
-    }
-    a.xq = xq; a.ys = ys; a.bsum = bsum; a.pf_k = pf_k; a.pf_v = pf_v; a.pf_nkv = pf_nkv; a.state = state;
-    const int K = mats[0].cols, upl = qw_upl(K / 256);
-    dim3 grid((rows + 7) / 8);
-    return resid ? qw_matvec_launch<KEPI_RESID>(a, upl, grid, qw_act_smem(K), pdl, st) : qw_matvec_launch<KEPI_PLAIN>(a, upl, grid, qw_act_smem(K), pdl, st);
+cudaError_t launch_qw_oproj(const KMatDev &wo, const float *act, float *x, DevState *state, bool pdl, cudaStream_t st) {
+    return qw_gemv(&wo, &x, 1, nullptr, act, state, pdl, st);
 }
 
-cudaError_t launch_qw_qknorm_rope(float *q, const float *k, const float *v, const float *q_norm, const float *k_norm, const float *rope,
-                                  float eps, int nh, int nkv, const DevState *state, int pos_val, float *kc, float *vc, bool pdl,
-                                  cudaStream_t st) {
-    return launch_k(qw_qknorm_rope_kernel, dim3(nh + nkv), dim3(QW_HD), 0, st, pdl, q, k, v, q_norm, k_norm, rope, eps, nh, nkv, state,
-                    pos_val, kc, vc);
-}
-
-cudaError_t launch_qw_attn(const float *q, const float *kc, const float *vc, int nh, int nkv, const DevState *state, int pos_val, int8_t *aq,
-                           float *as, int32_t *asum, bool pdl, cudaStream_t st) {
-    if (nh % 2) return cudaErrorInvalidValue;
+cudaError_t launch_qw_attn(const float *q, const float *k, const float *v, const float *q_norm, const float *k_norm, const float *rope, float eps, float *kc, float *vc,
+                           int nh, int nkv, DevState *state, float *out, bool pdl, cudaStream_t st) {
     static unsigned long long configured = 0;      // one bit per device
-    const size_t smem = (size_t)2 * BRRR_MAXSEQ * sizeof(float);
-    cudaError_t e = smem_optin(qw_attn_kernel, (int)smem, configured);
+    cudaError_t e = smem_optin(qw_attn_kernel, (int)QA_SMEM, configured);
     if (e != cudaSuccess) return e;
-    return launch_k(qw_attn_kernel, dim3(nh / 2), dim3(512), smem, st, pdl, q, kc, vc, nh, nkv, state, pos_val, aq, as, asum);
+    QAttnArgs a{q, k, v, q_norm, k_norm, rope, eps, kc, vc, nh, nkv, state, out};
+    return launch_k(qw_attn_kernel, dim3(nh), dim3(QA_THREADS), QA_SMEM, st, pdl, a);
 }
 
-cudaError_t launch_qw_gate_up(const KMatDev &gate, const KMatDev &up, const int32_t *top, int topk, int ff, const int8_t *xq, const float *ys,
-                              const int32_t *bsum, float *hbuf, bool pdl, cudaStream_t st) {
-    if (gate.cols != up.cols || (gate.type == 14 && !gate.planes) || (up.type == 14 && !up.planes)) return cudaErrorInvalidValue;
-    const int K = gate.cols;
-    dim3 grid((topk * ff + 7) / 8);
-    switch (qw_upl(K / 256)) {
-    case 1: return launch_k(qw_gate_up_kernel<1>, grid, dim3(256), qw_act_smem(K), st, pdl, gate, up, top, topk, ff, xq, ys, bsum, hbuf);
-    case 2: return launch_k(qw_gate_up_kernel<2>, grid, dim3(256), qw_act_smem(K), st, pdl, gate, up, top, topk, ff, xq, ys, bsum, hbuf);
-    case 4: return launch_k(qw_gate_up_kernel<4>, grid, dim3(256), qw_act_smem(K), st, pdl, gate, up, top, topk, ff, xq, ys, bsum, hbuf);
-    }
-    return cudaErrorInvalidValue;
-}
-
-cudaError_t launch_qw_down(const KMatDev &down, const int32_t *top, const float *wts, int topk, int d, int ff, const float *hbuf, float *x,
-                           unsigned int *counter, const float *next_norm_w, float eps, int8_t *nq, float *ns, int32_t *nsum, bool pdl,
+cudaError_t launch_qw_hint(const float *x, const float *norm_w, float eps, int d, const float *Wt, int ne, float *est, int8_t *q, float *s, int32_t *b16, bool pdl,
                            cudaStream_t st) {
-    if ((down.type == 14 && !down.planes) || ff % 256 || ff > 1024 || topk > 8) return cudaErrorInvalidValue;
-    QDownArgs a{down, top, wts, topk, d, ff, hbuf, x, counter, next_norm_w, eps, nq, ns, nsum};
-    const size_t act = qw_act_smem(topk * ff), smem = act > (size_t)d * 4 ? act : (size_t)d * 4;
-    dim3 grid((d + 7) / 8);
-    switch (ff / 256) {
-    case 1: return launch_k(qw_down_kernel<1>, grid, dim3(256), smem, st, pdl, a);
-    case 2: return launch_k(qw_down_kernel<2>, grid, dim3(256), smem, st, pdl, a);
-    case 3: return launch_k(qw_down_kernel<3>, grid, dim3(256), smem, st, pdl, a);
-    case 4: return launch_k(qw_down_kernel<4>, grid, dim3(256), smem, st, pdl, a);
-    }
-    return cudaErrorInvalidValue;
+    if (d > QH_MAXG * QH_THREADS * 4) return cudaErrorInvalidValue;
+    QHintArgs a{x, norm_w, eps, d, ne, Wt, est, q, s, b16};
+    return launch_k(qw_hint_kernel, dim3(ne), dim3(QH_THREADS), (size_t)d * 4, st, pdl, a);
 }
 
-cudaError_t launch_qw_head(const KMatDev &head, const int8_t *xq, const float *ys, const int32_t *bsum, float *logits, DevState *state, bool pdl,
-                           cudaStream_t st) {
-    if (head.type == 14 && !head.planes) return cudaErrorInvalidValue;
-    const int K = head.cols;
-    dim3 grid((head.rows + QW_HEAD_ROWS - 1) / QW_HEAD_ROWS);
-    switch (qw_upl(K / 256)) {
-    case 1: return launch_k(qw_head_kernel<1>, grid, dim3(256), qw_act_smem(K), st, pdl, head, xq, ys, bsum, logits, state);
-    case 2: return launch_k(qw_head_kernel<2>, grid, dim3(256), qw_act_smem(K), st, pdl, head, xq, ys, bsum, logits, state);
-    case 4: return launch_k(qw_head_kernel<4>, grid, dim3(256), qw_act_smem(K), st, pdl, head, xq, ys, bsum, logits, state);
-    }
-    return cudaErrorInvalidValue;
+cudaError_t launch_qw_gate_up(const KMatDev &gate, const KMatDev &up, const float *est, const int32_t *top, int ne, int topk, int ff, const int8_t *q, const float *s,
+                              const int32_t *b16, float *hbuf, DevState *state, bool pdl, cudaStream_t st) {
+    const int nsb = gate.cols / 256, upl = qw_upl(nsb);
+    if (gate.cols != up.cols || !qw_type_ok(gate) || !qw_type_ok(up) || !upl || ne > 256 || topk > 8) return cudaErrorInvalidValue;
+    QGateUpArgs a{gate, up, est, top, ne, topk, ff, 0, (int)gate.bpr(), (int)up.bpr(), q, s, b16, hbuf, state};
+    const size_t row = (size_t)a.stride_g + a.stride_u + nsb * 8;
+    a.per_cta = qw_rows_per_cta(topk * ff, row);
+    if (a.per_cta > 256) return cudaErrorInvalidValue;
+    const size_t smem = a.per_cta * row + qw_act_bytes(nsb);
+    return upl == 2 ? qw_gate_up_launch<2>(a, smem, pdl, st) : qw_gate_up_launch<4>(a, smem, pdl, st);
+}
+
+cudaError_t launch_qw_down(const KMatDev &down, const float *est, const int32_t *top, int ne, int topk, int d, int ff, const float *hbuf, float *part, DevState *state,
+                           bool pdl, cudaStream_t st) {
+    if (!qw_type_ok(down) || ff % 256 || ff > 1024 || topk > 8 || ne > 256) return cudaErrorInvalidValue;
+    QDownArgs a{down, est, top, ne, topk, d, ff, 0, hbuf, part, state};
+    const int nun = topk * (ff / 256);
+    const size_t row = (size_t)topk * down.bpr() + nun * 4;
+    a.per_cta = qw_rows_per_cta(d, row);
+    static unsigned long long configured = 0;      // one bit per device
+    cudaError_t e = smem_optin(qw_down_kernel, QG_SMEM_MAX, configured);
+    if (e != cudaSuccess) return e;
+    return launch_k(qw_down_kernel, dim3((d + a.per_cta - 1) / a.per_cta), dim3(QG_THREADS), a.per_cta * row + qw_act_bytes(nun), st, pdl, a);
+}
+
+cudaError_t launch_qw_head(const KMatDev &head, const int8_t *q, const float *s, const int32_t *b16, float *logits, DevState *state, bool pdl, cudaStream_t st) {
+    const int nsb = head.cols / 256, upl = qw_upl(nsb);
+    if (!qw_type_ok(head) || !upl) return cudaErrorInvalidValue;
+    const size_t stage = QG_WARPS * head.bpr(), terms = (size_t)QG_WARPS * 2 * nsb * 4;
+    const int depth = (int)((220 * 1024 - terms) / stage);
+    QHeadArgs a{head, q, s, b16, logits, state, (head.rows + 147) / 148, depth < 8 ? depth : 8};
+    a.per_cta = (a.per_cta + QG_WARPS - 1) / QG_WARPS * QG_WARPS;
+    const size_t smem = a.depth * stage + terms;
+    return upl == 2 ? qw_head_launch<2>(a, smem, pdl, st) : qw_head_launch<4>(a, smem, pdl, st);
 }
 
 void launch_q6k_planes(const uint8_t *src, size_t rows, int cols, uint8_t *dst, cudaStream_t st) {

@@ -75,11 +75,12 @@ struct RouterArgs {
     uint32_t *signal;        // nullable: sequence number of the published routing (see publish_route)
     unsigned long long *pub;
     // qwen3moe: the norm is the 12-slice one, and the first CTA also leaves the Q8_K image of the
-    // normalised token (quants, scales per 256, sums per 32) for the gate/up kernel
+    // normalised token (quants, scales per 256, sums per 16) for the gate/up kernel
     int qwen_norm;
     int8_t *q8k_q;
     float *q8k_s;
-    int32_t *q8k_bsum;
+    int32_t *q8k_b16;
+    int stages;              // tiles in flight: 5, or 3 where several CTAs share the experts (an SM then holds a decode kernel beside one)
 };
 
 // k rounds of warp arg-max over the logits (lane l holds experts l, l+32, ...): the largest value
@@ -141,12 +142,13 @@ __global__ void __launch_bounds__(RT_THREADS) ffn_in_kernel(RouterArgs a) {
     a.wts += blockIdx.y * 8;
     a.counter += blockIdx.y;
     extern __shared__ __align__(128) unsigned char smraw[];
-    float *tiles = reinterpret_cast<float *>(smraw);                                        // [RT_STAGES][32][RT_STRIDE]
-    float *xn = reinterpret_cast<float *>(smraw + (size_t)RT_TILE_FLOATS * 4 * RT_STAGES);   // d floats
+    const int stages = a.stages;
+    float *tiles = reinterpret_cast<float *>(smraw);                                        // [stages][32][RT_STRIDE]
+    float *xn = reinterpret_cast<float *>(smraw + (size_t)RT_TILE_FLOATS * 4 * stages);   // d floats
     float *lg = xn + a.d;                                                                   // ne floats (top-k staging)
     float *wn = lg + ((a.ne + 3) & ~3);                                        // d floats: norm weights (16-byte aligned: float4 stores)
-    uint64_t *bars = reinterpret_cast<uint64_t *>(wn + a.d);                   // [RT_STAGES] tile landed
-    uint64_t *empty = bars + RT_STAGES;                                        // [RT_STAGES] tile consumed
+    uint64_t *bars = reinterpret_cast<uint64_t *>(wn + a.d);                   // [stages] tile landed
+    uint64_t *empty = bars + stages;                                        // [stages] tile consumed
     __shared__ float inv_sh;
     __shared__ int last_sh;
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, d = a.d;
@@ -158,17 +160,17 @@ __global__ void __launch_bounds__(RT_THREADS) ffn_in_kernel(RouterArgs a) {
     const float *wsrc = a.Wt + (size_t)blockIdx.x * ntiles * RT_TILE_FLOATS;
 
     auto issue = [&](int t) {                                       // one thread
-        int slot = t % RT_STAGES;
+        int slot = t % stages;
         mbar_expect_tx(&bars[slot], (uint32_t)RT_TILE_FLOATS * 4);
         bulk_g2s(tiles + (size_t)slot * RT_TILE_FLOATS, wsrc + (size_t)t * RT_TILE_FLOATS, (uint32_t)RT_TILE_FLOATS * 4, &bars[slot]);
     };
     BRRR_STAMP(a.state, 0);
     if (tid == 0) {
-        for (int s = 0; s < RT_STAGES; s++) { mbar_init(&bars[s], 1); mbar_init(&empty[s], 1); }
+        for (int s = 0; s < stages; s++) { mbar_init(&bars[s], 1); mbar_init(&empty[s], 1); }
         mbar_fence_init();
     }
     __syncwarp();
-    if (tid < min(RT_STAGES, ntiles)) issue(tid);        // one lane per stage: the copies' address translations overlap
+    if (tid < min(stages, ntiles)) issue(tid);        // one lane per stage: the copies' address translations overlap
     if (a.norm_w) stage_vec4(a.norm_w, wn, d, tid, RT_THREADS);             // static: fetched before the wait
     const float bias_pre = (warp == 0 && lane < nloc && a.b) ? a.b[e0 + lane] : 0.0f;
     BRRR_STAMP(a.state, 1);
@@ -206,15 +208,15 @@ __global__ void __launch_bounds__(RT_THREADS) ffn_in_kernel(RouterArgs a) {
             float v[8];
 #pragma unroll
             for (int i = 0; i < 8; i++) v[i] = xn[sb * 256 + lane * 8 + i];
-            warp_quant_q8k(v, lane, a.q8k_q + sb * 256, a.q8k_s + sb, a.q8k_bsum + sb * 8);
+            warp_quant_q8k16(v, lane, a.q8k_q + sb * 256, a.q8k_s + sb, a.q8k_b16 + sb * 16);
         }
     }
 
     BRRR_STAMP(a.state, 3);
     if (warp == 1 && lane == 0) {
-        // refill thread: as soon as the chain warp releases a slot, the tile RT_STAGES ahead goes in
-        for (int t = RT_STAGES; t < ntiles; t++) {
-            waiter.wait(&empty[t % RT_STAGES], (uint32_t)(t / RT_STAGES - 1) & 1u);
+        // refill thread: as soon as the chain warp releases a slot, the tile stages ahead goes in
+        for (int t = stages; t < ntiles; t++) {
+            waiter.wait(&empty[t % stages], (uint32_t)(t / stages - 1) & 1u);
             fence_proxy_async();
             issue(t);
         }
@@ -223,15 +225,15 @@ __global__ void __launch_bounds__(RT_THREADS) ffn_in_kernel(RouterArgs a) {
         float acc = bias_pre;
         for (int t = 0; t < ntiles; t++) {
             if (t < 12) BRRR_STAMP(a.state, 8 + t);
-            const int slot = t % RT_STAGES, j0 = t * RT_TJ, len = min(RT_TJ, d - j0);
-            waiter.wait(&bars[slot], (uint32_t)(t / RT_STAGES) & 1u);
+            const int slot = t % stages, j0 = t * RT_TJ, len = min(RT_TJ, d - j0);
+            waiter.wait(&bars[slot], (uint32_t)(t / stages) & 1u);
             const float *row = tiles + (size_t)slot * RT_TILE_FLOATS + lane * RT_STRIDE;
             const float *xr = xn + j0;
             if (len == RT_TJ) acc = chain_span<RT_TJ>(row, xr, acc);
             else
                 for (int jj = 0; jj < len; jj += 32) acc = chain_span<32>(row + jj, xr + jj, acc);   // d % 64 == 0
             __syncwarp();                      // all lanes are done reading this slot
-            if (lane == 0 && t + RT_STAGES < ntiles) mbar_arrive(&empty[slot]);
+            if (lane == 0 && t + stages < ntiles) mbar_arrive(&empty[slot]);
         }
         if (lane < nloc) {
             if (gridDim.x == 1) lg[lane] = acc;
@@ -404,11 +406,11 @@ size_t router_packed_floats(int ne, int d) { return (size_t)((ne + 31) / 32) * (
 
 cudaError_t launch_ffn_in(const float *x_in, const float *norm_w, float eps, int d, const float *Wt, const float *b, int ne, int topk,
                           float *logits, int32_t *top, float *wts, unsigned int *counter, DevState *state, bool pdl, cudaStream_t st, int ntok,
-                          uint32_t *signal, int qwen_norm, int8_t *q8k_q, float *q8k_s, int32_t *q8k_bsum) {
+                          uint32_t *signal, int qwen_norm, int8_t *q8k_q, float *q8k_s, int32_t *q8k_b16) {
     RouterArgs a{x_in, norm_w, eps, d, Wt, b, ne, topk, logits, top, wts, counter, state, signal, (signal && state) ? state->route_pub : nullptr,
-                 qwen_norm, q8k_q, q8k_s, q8k_bsum};
+                 qwen_norm, q8k_q, q8k_s, q8k_b16, ne > 32 ? 3 : RT_STAGES};
     if (signal && !state) return cudaErrorInvalidValue;
-    size_t smem = (size_t)RT_TILE_FLOATS * 4 * RT_STAGES + (size_t)d * 8 + (size_t)((ne + 3) & ~3) * 4 + RT_STAGES * 16;
+    size_t smem = (size_t)RT_TILE_FLOATS * 4 * a.stages + (size_t)d * 8 + (size_t)((ne + 3) & ~3) * 4 + a.stages * 16;
     static unsigned long long configured = 0;      // one bit per device
     {
         cudaError_t e = smem_optin(ffn_in_kernel, 200 * 1024, configured);

@@ -79,14 +79,22 @@ struct brrr_qwen {
     std::vector<QLayer> L;
     float *out_norm = nullptr, *rope = nullptr;
     KMatDev head{}, embd{};
-    float *x = nullptr, *xn = nullptr, *q = nullptr, *k = nullptr, *v = nullptr, *ao = nullptr, *hbuf = nullptr, *rlogits = nullptr,
-          *logits = nullptr, *xs = nullptr, *as = nullptr, *hs = nullptr, *wts = nullptr;
-    int8_t *xq = nullptr, *aq = nullptr, *hq = nullptr;
-    int32_t *xsum = nullptr, *asum = nullptr, *hsum = nullptr, *top = nullptr;
-    unsigned int *down_counter = nullptr;      // arrival counter of the down kernel's CTAs (self-resetting)
+    float *x = nullptr, *xb[2] = {nullptr, nullptr};      // residual: of the finished step; of the running one, alternating from layer to layer
+    float *q = nullptr, *k = nullptr, *v = nullptr, *ao = nullptr, *hbuf = nullptr, *part = nullptr, *est = nullptr, *rlogits = nullptr, *logits = nullptr, *xs = nullptr,
+          *wts = nullptr;
+    int8_t *xq = nullptr;
+    int32_t *xsum = nullptr, *top = nullptr;
     DevState *st = nullptr;
     uint32_t *h_in = nullptr, *h_out = nullptr;
-    cudaGraphExec_t g_head = nullptr, g_nohead = nullptr;
+    cudaStream_t side = nullptr;                                     // the exact router of the speculative step
+    cudaEvent_t ev_fork = nullptr, ev_join = nullptr;
+    cudaGraphExec_t g_head = nullptr, g_nohead = nullptr;            // speculative routing (null: switched off)
+    cudaGraphExec_t g_head_safe = nullptr, g_nohead_safe = nullptr;  // routing in the chain; redoes a missed speculation
+    bool use_spec = true;
+    bool spec_off = false;               // a bounded device wait of the speculative step ran out once
+    uint64_t spec_redos = 0;
+    uint32_t run_tok = 0, run_pos = 0;   // of the decode run in flight
+    uint32_t test_hooks = 0;
     int launches_head = 0, launches_nohead = 0;
     bool use_pdl = true;
     // prompt tiles: up to BRRR_TILE_MAX consecutive positions walk the layers together
@@ -200,39 +208,49 @@ int qcheck_cfg(const brrr_qwen_cfg &c) {
     return BRRR_OK;
 }
 
-// The decode step (forward_worker, engine_qwen2.rs:302-451), kernel by kernel.
-int qenqueue_step(brrr_qwen *m, bool want, float *trace_dev, int *nlaunch) {
+// The decode step (forward_worker, engine_qwen2.rs:302-451), kernel by kernel.  spec: the experts are those of the routing hint, the
+// exact router runs on the side stream and reaches the next combine through published words (kernels_qwen.cu); else the router is a
+// link of the chain and everything follows its choice.
+int qenqueue_step(brrr_qwen *m, bool want, float *trace_dev, int *nlaunch, bool spec) {
     const brrr_qwen_cfg &c = m->cfg;
-    const int d = c.n_embd, nh = c.n_head, nkv = c.n_head_kv, hd = c.head_dim, ff = c.n_ff_exp, topk = c.n_expert_used;
+    const int d = c.n_embd, nh = c.n_head, nkv = c.n_head_kv, ff = c.n_ff_exp, topk = c.n_expert_used, ne = c.n_expert;
     cudaStream_t s = m->stream;
     const bool pdl = m->use_pdl && !trace_dev;
-    int n = 0;
-    CU(launch_qw_embed(m->embd.p, d, m->st, m->x, false, s)); n++;
-    if (trace_dev) CU(cudaMemcpyAsync(trace_dev, m->x, d * sizeof(float), cudaMemcpyDeviceToDevice, s));
-    // layer 0 has no down kernel before it: its attention norm + Q8_K is a launch of its own
-    CU(launch_qw_norm_quant(m->x, m->L[0].attn_norm, c.rms_eps, d, nullptr, m->xq, m->xs, m->xsum, pdl, s)); n++;
+    int n = 0, cur = 0;
+    CU(launch_qw_embed(m->embd.p, d, m->st, m->xb[0], false, s)); n++;
+    const float *est = spec ? m->est : nullptr;
+    auto combine = [&](int layers, float *x_out, const float *norm_w) {      // of the last of `layers` layers run so far
+        return QwCombine{m->xb[cur], layers ? m->part : nullptr, x_out, est, m->top, m->wts, ne, topk, d, (uint32_t)layers, norm_w, c.rms_eps, m->st};
+    };
+    if (trace_dev) CU(cudaMemcpyAsync(trace_dev, m->xb[0], d * sizeof(float), cudaMemcpyDeviceToDevice, s));
     for (int il = 0; il < c.n_layer; il++) {
         QLayer &ly = m->L[il];
         KMatDev qkv[3] = {ly.wq, ly.wk, ly.wv};
-        float *qkv_out[3] = {m->q, m->k, m->v};
-        CU(launch_qw_matvec(qkv, qkv_out, 3, false, m->xq, m->xs, m->xsum, pdl, s, ly.kc, ly.vc, nkv, m->st)); n++;
-        CU(launch_qw_qknorm_rope(m->q, m->k, m->v, ly.q_norm, ly.k_norm, m->rope, c.rms_eps, nh, nkv, m->st, 0, ly.kc, ly.vc, pdl, s)); n++;
-        CU(launch_qw_attn(m->q, ly.kc, ly.vc, nh, nkv, m->st, 0, m->aq, m->as, m->asum, pdl, s)); n++;
-        float *xo[1] = {m->x};
-        CU(launch_qw_matvec(&ly.wo, xo, 1, true, m->aq, m->as, m->asum, pdl, s)); n++;
-        // router: FFN norm (12 slices) and the Q8_K image of the normalised token in its prologue
-        CU(launch_ffn_in(m->x, ly.ffn_norm, c.rms_eps, d, ly.ginp, nullptr, c.n_expert, topk, m->rlogits, m->top, m->wts, &m->st->router_done, m->st,
-                         pdl, s, 1, nullptr, 1, m->xq, m->xs, m->xsum)); n++;
-        CU(launch_qw_gate_up(ly.gate, ly.up, m->top, topk, ff, m->xq, m->xs, m->xsum, m->hbuf, pdl, s)); n++;
-        const bool last = il == c.n_layer - 1;
-        const float *nw = last ? (want ? m->out_norm : nullptr) : m->L[il + 1].attn_norm;
-        CU(launch_qw_down(ly.down, m->top, m->wts, topk, d, ff, m->hbuf, m->x, m->down_counter, nw, c.rms_eps, m->xq, m->xs, m->xsum, pdl, s)); n++;
-        if (trace_dev) CU(cudaMemcpyAsync(trace_dev + (size_t)(il + 1) * d, m->x, d * sizeof(float), cudaMemcpyDeviceToDevice, s));
+        float *qkv_out[3] = {m->q, m->k, m->v}, *x = m->xb[cur ^ 1];
+        CU(launch_qw_qkv(qkv, qkv_out, combine(il, x, ly.attn_norm), pdl, s)); n++;
+        cur ^= 1;
+        if (trace_dev && il) CU(cudaMemcpyAsync(trace_dev + (size_t)il * d, x, d * sizeof(float), cudaMemcpyDeviceToDevice, s));
+        CU(launch_qw_attn(m->q, m->k, m->v, ly.q_norm, ly.k_norm, m->rope, c.rms_eps, ly.kc, ly.vc, nh, nkv, m->st, m->ao, pdl, s)); n++;
+        CU(launch_qw_oproj(ly.wo, m->ao, x, m->st, pdl, s)); n++;
+        if (spec) {
+            CU(cudaEventRecord(m->ev_fork, s));
+            CU(cudaStreamWaitEvent(m->side, m->ev_fork, 0));
+            CU(launch_ffn_in(x, ly.ffn_norm, c.rms_eps, d, ly.ginp, nullptr, ne, topk, m->rlogits, m->top, m->wts, &m->st->router_done, m->st, false, m->side, 1,
+                             &m->st->router_seq, 1)); n++;
+            CU(cudaEventRecord(m->ev_join, m->side));
+            CU(launch_qw_hint(x, ly.ffn_norm, c.rms_eps, d, ly.ginp, ne, m->est, m->xq, m->xs, m->xsum, pdl, s)); n++;
+        } else {
+            CU(launch_ffn_in(x, ly.ffn_norm, c.rms_eps, d, ly.ginp, nullptr, ne, topk, m->rlogits, m->top, m->wts, &m->st->router_done, m->st, pdl, s, 1, nullptr, 1,
+                             m->xq, m->xs, m->xsum)); n++;
+        }
+        CU(launch_qw_gate_up(ly.gate, ly.up, est, m->top, ne, topk, ff, m->xq, m->xs, m->xsum, m->hbuf, m->st, pdl, s)); n++;
+        CU(launch_qw_down(ly.down, est, m->top, ne, topk, d, ff, m->hbuf, m->part, m->st, pdl, s)); n++;
     }
-    if (want) {
-        CU(launch_qw_head(m->head, m->xq, m->xs, m->xsum, m->logits, m->st, pdl, s)); n++;
-        launch_finish_token(m->st, s); n++;
-    }
+    CU(launch_qw_fold(combine(c.n_layer, m->x, want ? m->out_norm : nullptr), m->xq, m->xs, m->xsum, pdl, s)); n++;
+    if (trace_dev) CU(cudaMemcpyAsync(trace_dev + (size_t)c.n_layer * d, m->x, d * sizeof(float), cudaMemcpyDeviceToDevice, s));
+    if (want) { CU(launch_qw_head(m->head, m->xq, m->xs, m->xsum, m->logits, m->st, pdl, s)); n++; }
+    if (spec) CU(cudaStreamWaitEvent(s, m->ev_join, 0));
+    if (want) { launch_finish_token(m->st, s); n++; }
     CU(cudaGetLastError());
     if (nlaunch) *nlaunch = n;
     return BRRR_OK;
@@ -298,18 +316,18 @@ int qenqueue_rows(brrr_qwen *m, int rows, int pos0, bool last) {
     }
     if (!last) return BRRR_OK;            // rows that only fill the cache: nobody reads their residual
     CU(launch_qr_norm(r.x, rows, d, part, r.wts, topk, nullptr, c.rms_eps, nullptr, nullptr, nullptr, pdl, s));
-    CU(cudaMemcpyAsync(m->x, r.x + (size_t)(rows - 1) * d, (size_t)d * 4, cudaMemcpyDeviceToDevice, s));
-    CU(launch_qw_norm_quant(m->x, m->out_norm, c.rms_eps, d, nullptr, m->xq, m->xs, m->xsum, false, s));
+    CU(launch_qw_fold(QwCombine{r.x + (size_t)(rows - 1) * d, nullptr, m->x, nullptr, nullptr, nullptr, ne, topk, d, 0, m->out_norm, c.rms_eps, m->st}, m->xq, m->xs, m->xsum,
+                      pdl, s));
     CU(launch_qw_head(m->head, m->xq, m->xs, m->xsum, m->logits, m->st, pdl, s));
     launch_finish_token(m->st, s);
     CU(cudaGetLastError());
     return BRRR_OK;
 }
 
-int qcapture(brrr_qwen *m, bool want, cudaGraphExec_t *out, int *nlaunch) {
+int qcapture(brrr_qwen *m, bool want, cudaGraphExec_t *out, int *nlaunch, bool spec) {
     cudaGraph_t g = nullptr;
     CU(cudaStreamBeginCapture(m->stream, cudaStreamCaptureModeThreadLocal));
-    int s = qenqueue_step(m, want, nullptr, nlaunch);
+    int s = qenqueue_step(m, want, nullptr, nlaunch, spec);
     cudaError_t e = cudaStreamEndCapture(m->stream, &g);
     if (s != BRRR_OK) { if (g) cudaGraphDestroy(g); return s; }
     CU(e);
@@ -318,12 +336,29 @@ int qcapture(brrr_qwen *m, bool want, cudaGraphExec_t *out, int *nlaunch) {
     return BRRR_OK;
 }
 
+int qreset_state(brrr_qwen *m) {      // as a fresh model has it
+    CU(cudaMemsetAsync(m->st, 0, sizeof(DevState), m->stream));
+    CU(cudaMemsetAsync(&m->st->spec_fail_step, 0xFF, 4, m->stream));
+#ifdef BRRR_TEST_HOOKS
+    if (m->test_hooks) CU(cudaMemcpyAsync(&m->st->test_hooks, &m->test_hooks, 4, cudaMemcpyHostToDevice, m->stream));
+#endif
+    return BRRR_OK;
+}
+
 int qbuild(brrr_qwen *m, const QSource &src) {
     const brrr_qwen_cfg &c = m->cfg;
     const int d = c.n_embd, nh = c.n_head, nkv = c.n_head_kv, hd = c.head_dim, ne = c.n_expert, ff = c.n_ff_exp, topk = c.n_expert_used;
     CU(cudaSetDevice(m->device));
     CU(cudaStreamCreateWithFlags(&m->stream, cudaStreamNonBlocking));
+    CU(cudaStreamCreateWithFlags(&m->side, cudaStreamNonBlocking));
+    CU(cudaEventCreateWithFlags(&m->ev_fork, cudaEventDisableTiming));
+    CU(cudaEventCreateWithFlags(&m->ev_join, cudaEventDisableTiming));
     if (const char *e = getenv("BRRR_NOPDL")) m->use_pdl = !(e[0] && e[0] != '0');
+    if (const char *e = getenv("BRRR_NOSPEC")) m->use_spec = !(e[0] && e[0] != '0');
+#ifdef BRRR_TEST_HOOKS
+    if (const char *e = getenv("BRRR_SPEC_SABOTAGE")) if (e[0] && e[0] != '0') m->test_hooks |= 1u;
+    if (const char *e = getenv("BRRR_ROUTER_MUTE")) if (e[0] && e[0] != '0') m->test_hooks |= 2u;
+#endif
     float *scratch = nullptr;
     if (cudaMalloc(&scratch, (size_t)ne * d * 4) != cudaSuccess) return BRRR_ERR_NOMEM;
     struct Guard { void *p; ~Guard() { cudaFree(p); } } guard{scratch};
@@ -376,26 +411,27 @@ int qbuild(brrr_qwen *m, const QSource &src) {
     TRY(m->alloc(&m->rope, tab.size()));
     CU(cudaMemcpyAsync(m->rope, tab.data(), tab.size() * 4, cudaMemcpyHostToDevice, m->stream));
 
-    TRY(m->alloc(&m->x, d)); TRY(m->alloc(&m->xn, d)); TRY(m->alloc(&m->q, nh * hd)); TRY(m->alloc(&m->k, nkv * hd)); TRY(m->alloc(&m->v, nkv * hd));
-    TRY(m->alloc(&m->ao, nh * hd)); TRY(m->alloc(&m->hbuf, (size_t)topk * ff)); TRY(m->alloc(&m->rlogits, ne)); TRY(m->alloc(&m->logits, c.n_vocab));
-    TRY(m->alloc(&m->xs, d / 256)); TRY(m->alloc(&m->as, nh * hd / 256)); TRY(m->alloc(&m->hs, (size_t)topk * ff / 256)); TRY(m->alloc(&m->wts, 8));
-    TRY(m->alloc(&m->xq, d)); TRY(m->alloc(&m->aq, nh * hd)); TRY(m->alloc(&m->hq, (size_t)topk * ff));
-    TRY(m->alloc(&m->xsum, d / 32)); TRY(m->alloc(&m->asum, nh * hd / 32)); TRY(m->alloc(&m->hsum, (size_t)topk * ff / 32));
+    TRY(m->alloc(&m->x, d)); TRY(m->alloc(&m->xb[0], d)); TRY(m->alloc(&m->xb[1], d)); TRY(m->alloc(&m->q, nh * hd)); TRY(m->alloc(&m->k, nkv * hd));
+    TRY(m->alloc(&m->v, nkv * hd)); TRY(m->alloc(&m->ao, nh * hd)); TRY(m->alloc(&m->hbuf, (size_t)topk * ff)); TRY(m->alloc(&m->part, (size_t)topk * d));
+    TRY(m->alloc(&m->est, ne)); TRY(m->alloc(&m->rlogits, ne)); TRY(m->alloc(&m->logits, c.n_vocab));
+    TRY(m->alloc(&m->xs, d / 256)); TRY(m->alloc(&m->wts, 8)); TRY(m->alloc(&m->xq, d)); TRY(m->alloc(&m->xsum, d / 16));
     TRY(m->alloc(&m->top, 8)); TRY(m->alloc(&m->st, 1));
-    TRY(m->alloc(&m->down_counter, 1));
-    CU(cudaMemsetAsync(m->down_counter, 0, sizeof(unsigned int), m->stream));
-    CU(cudaMemsetAsync(m->st, 0, sizeof(DevState), m->stream));
+    TRY(qreset_state(m));
     CU(cudaMemsetAsync(m->x, 0, d * 4, m->stream));
     TRY(qrows_alloc(m));
     CU(cudaMallocHost(&m->h_in, (BRRR_MAXSEQ + 4) * sizeof(uint32_t)));
     CU(cudaMallocHost(&m->h_out, BRRR_MAXSEQ * sizeof(uint32_t)));
     CU(cudaStreamSynchronize(m->stream));
-    // one direct (un-captured) step configures kernel attributes and validates the launches
-    TRY(qenqueue_step(m, true, nullptr, nullptr));
+    // direct (un-captured) steps configure kernel attributes and validate the launches
+    TRY(qenqueue_step(m, true, nullptr, nullptr, false));
     CU(cudaStreamSynchronize(m->stream));
-    CU(cudaMemsetAsync(m->st, 0, sizeof(DevState), m->stream));
-    TRY(qcapture(m, true, &m->g_head, &m->launches_head));
-    TRY(qcapture(m, false, &m->g_nohead, &m->launches_nohead));
+    TRY(qreset_state(m));
+    TRY(qcapture(m, true, &m->g_head_safe, &m->launches_head, false));
+    TRY(qcapture(m, false, &m->g_nohead_safe, &m->launches_nohead, false));
+    if (m->use_spec) {
+        TRY(qcapture(m, true, &m->g_head, &m->launches_head, true));
+        TRY(qcapture(m, false, &m->g_nohead, &m->launches_nohead, true));
+    }
     CU(cudaStreamSynchronize(m->stream));
     return BRRR_OK;
 }
@@ -440,9 +476,14 @@ extern "C" void brrr_qwen_close(brrr_qwen *m) {
     if (m->stream) cudaStreamSynchronize(m->stream);
     if (m->g_head) cudaGraphExecDestroy(m->g_head);
     if (m->g_nohead) cudaGraphExecDestroy(m->g_nohead);
+    if (m->g_head_safe) cudaGraphExecDestroy(m->g_head_safe);
+    if (m->g_nohead_safe) cudaGraphExecDestroy(m->g_nohead_safe);
+    if (m->ev_fork) cudaEventDestroy(m->ev_fork);
+    if (m->ev_join) cudaEventDestroy(m->ev_join);
     for (void *p : m->allocs) cudaFree(p);
     if (m->h_in) cudaFreeHost(m->h_in);
     if (m->h_out) cudaFreeHost(m->h_out);
+    if (m->side) cudaStreamDestroy(m->side);
     if (m->stream) cudaStreamDestroy(m->stream);
     delete m;
 }
@@ -517,21 +558,36 @@ extern "C" uint64_t brrr_qwen_bytes_per_step(const brrr_qwen *m, uint32_t pos) {
     return total;
 }
 
-static int qrun_graph(brrr_qwen *m, bool want) {
-    CU(cudaGraphLaunch(want ? m->g_head : m->g_nohead, m->stream));
+static int qrun_graph(brrr_qwen *m, bool want, bool safe = false) {
+    safe = safe || m->spec_off || !m->g_head;
+    CU(cudaGraphLaunch(safe ? (want ? m->g_head_safe : m->g_nohead_safe) : (want ? m->g_head : m->g_nohead), m->stream));
     return BRRR_OK;
+}
+
+// A combine that gave up waiting for the router's words has flagged its step like a missed speculation: clear the error and do without
+// speculation from here on.  False: another error.
+static bool qrecover(brrr_qwen *m, uint32_t err) {
+    if (err != (uint32_t)DEV_ERR_PEER_TIMEOUT || !m->g_head || m->spec_off) return false;
+    if (cudaMemsetAsync(&m->st->err, 0, 4, m->stream) != cudaSuccess) return false;
+    m->spec_off = true;
+    return true;
 }
 
 extern "C" int brrr_qwen_forward(brrr_qwen *m, uint32_t tok, uint32_t pos, int want, uint32_t *out_tok) {
     if (!m) return BRRR_ERR_ARG;
     if (tok >= (uint32_t)m->cfg.n_vocab || pos >= BRRR_MAXSEQ) return BRRR_ERR_RANGE;
     CU(cudaSetDevice(m->device));
-    m->h_in[0] = tok; m->h_in[1] = pos;
-    CU(cudaMemcpyAsync(m->st, m->h_in, 8, cudaMemcpyHostToDevice, m->stream));   // DevState.tok, .pos
-    TRY(qrun_graph(m, want != 0));
-    CU(cudaMemcpyAsync(m->h_out, m->st, 32, cudaMemcpyDeviceToHost, m->stream));
-    CU(cudaStreamSynchronize(m->stream));
-    if (m->h_out[6] != 0) { QERR("device wait timed out (code %u)", m->h_out[6]); return BRRR_ERR_STATE; }
+    for (int pass = 0; pass < 2; pass++) {
+        m->h_in[0] = tok; m->h_in[1] = pos;
+        CU(cudaMemcpyAsync(m->st, m->h_in, 8, cudaMemcpyHostToDevice, m->stream));   // DevState.tok, .pos
+        TRY(qrun_graph(m, want != 0, pass != 0));
+        CU(cudaMemcpyAsync(m->h_out, m->st, 32, cudaMemcpyDeviceToHost, m->stream));   // tok .. spec_fail_step
+        CU(cudaStreamSynchronize(m->stream));
+        if (m->h_out[6] != 0 && !qrecover(m, m->h_out[6])) { QERR("device wait timed out (code %u)", m->h_out[6]); return BRRR_ERR_STATE; }
+        if (m->h_out[7] == 0xFFFFFFFFu) break;
+        m->spec_redos++;                 // the estimate missed an expert: the same step with the routing in the chain
+        CU(cudaMemsetAsync(&m->st->spec_fail_step, 0xFF, 4, m->stream));
+    }
     if (want && out_tok) *out_tok = m->h_out[0];
     return BRRR_OK;
 }
@@ -569,6 +625,7 @@ extern "C" int brrr_qwen_decode_enqueue(brrr_qwen *m, uint32_t first_tok, uint32
     if (first_tok >= (uint32_t)m->cfg.n_vocab || n == 0 || n > BRRR_MAXSEQ || pos + n > BRRR_MAXSEQ) return BRRR_ERR_RANGE;
     CU(cudaSetDevice(m->device));
     m->h_in[0] = first_tok; m->h_in[1] = pos; m->h_in[2] = 0;
+    m->run_tok = first_tok; m->run_pos = pos;
     CU(cudaMemcpyAsync(m->st, m->h_in, 12, cudaMemcpyHostToDevice, m->stream));  // tok, pos, n_out = 0
     for (uint32_t i = 0; i < n; i++) TRY(qrun_graph(m, true));
     return BRRR_OK;
@@ -577,10 +634,22 @@ extern "C" int brrr_qwen_decode_enqueue(brrr_qwen *m, uint32_t first_tok, uint32
 extern "C" int brrr_qwen_decode_wait(brrr_qwen *m, uint32_t n, uint32_t *out_toks) {
     if (!m || !out_toks || n == 0 || n > BRRR_MAXSEQ) return BRRR_ERR_ARG;
     CU(cudaSetDevice(m->device));
-    CU(cudaMemcpyAsync(m->h_out, m->st->out, n * sizeof(uint32_t), cudaMemcpyDeviceToHost, m->stream));
-    CU(cudaMemcpyAsync(m->h_in, &m->st->err, 4, cudaMemcpyDeviceToHost, m->stream));
-    CU(cudaStreamSynchronize(m->stream));
-    if (m->h_in[0] != 0) { QERR("device wait timed out (code %u)", m->h_in[0]); return BRRR_ERR_STATE; }
+    for (uint32_t pass = 0; pass <= n; pass++) {
+        CU(cudaMemcpyAsync(m->h_out, m->st->out, n * sizeof(uint32_t), cudaMemcpyDeviceToHost, m->stream));
+        CU(cudaMemcpyAsync(m->h_in, &m->st->err, 8, cudaMemcpyDeviceToHost, m->stream));       // err, spec_fail_step
+        CU(cudaStreamSynchronize(m->stream));
+        if (m->h_in[0] != 0 && !qrecover(m, m->h_in[0])) { QERR("device wait timed out (code %u)", m->h_in[0]); return BRRR_ERR_STATE; }
+        const uint32_t f = m->h_in[1];
+        if (f >= n) break;
+        // step f ran with experts the router did not confirm: it and what followed are void.  Resume there (the cache entries of the
+        // voided steps are overwritten).
+        m->spec_redos++;
+        CU(cudaMemsetAsync(&m->st->spec_fail_step, 0xFF, 4, m->stream));
+        m->h_in[0] = f ? m->h_out[f - 1] : m->run_tok; m->h_in[1] = m->run_pos + f; m->h_in[2] = f;
+        CU(cudaMemcpyAsync(m->st, m->h_in, 12, cudaMemcpyHostToDevice, m->stream));
+        TRY(qrun_graph(m, true, true));
+        for (uint32_t i = f + 1; i < n; i++) TRY(qrun_graph(m, true));
+    }
     memcpy(out_toks, m->h_out, n * sizeof(uint32_t));
     return BRRR_OK;
 }
@@ -617,7 +686,7 @@ extern "C" int brrr_qwen_forward_trace(brrr_qwen *m, uint32_t tok, uint32_t pos,
     CU(cudaMalloc(&dev, n * 4));
     m->h_in[0] = tok; m->h_in[1] = pos;
     cudaMemcpyAsync(m->st, m->h_in, 8, cudaMemcpyHostToDevice, m->stream);
-    int s = qenqueue_step(m, true, dev, nullptr);
+    int s = qenqueue_step(m, true, dev, nullptr, false);
     if (s == BRRR_OK && cudaMemcpyAsync(trace, dev, n * 4, cudaMemcpyDeviceToHost, m->stream) != cudaSuccess) s = BRRR_ERR_CUDA;
     if (cudaStreamSynchronize(m->stream) != cudaSuccess) s = BRRR_ERR_CUDA;
     cudaFree(dev);
