@@ -51,7 +51,6 @@ __device__ __forceinline__ int brrr_q8_round(float v, float sc) {
     r = fminf(fmaxf(r, -127.0f), 127.0f);
     return (int)r;
 }
-
 __device__ __forceinline__ float brrr_bf16_to_f32(uint16_t v) { return __int_as_float((uint32_t)v << 16); }
 
 __device__ __forceinline__ uint32_t brrr_prmt(uint32_t a, uint32_t b, uint32_t c) {

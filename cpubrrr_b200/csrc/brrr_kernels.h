@@ -39,34 +39,22 @@ void launch_q6k_matvec(const uint8_t *w, int rows, int cols, const int8_t *xq, c
 
 // ---- qwen3moe decode kernels (kernels_qwen.cu); KMatDev is declared in brrr_kq.cuh
 struct KMatDev;
-// Combine of the experts' row sums into the residual and the next norm: x_out = x_in + sum over k of w[k] part[slot of k].  est: the slots are the
-// estimate's ranks and the exact routing is the step's seq-th publication of the router; else slots, weights and order are top's.
-struct QwCombine {
-    const float *x_in, *part;        // part nullable: nothing to add
-    float *x_out;
-    const float *est;
-    const int32_t *top;
-    const float *wts;
-    int ne, topk, d;
-    uint32_t seq;
-    const float *norm_w;             // nullable: combine only
-    float eps;
-    DevState *state;
-};
 // Q8_K images of one token: quants, scales per 256, sums per 16.  kernels fetch rows known before their dependency wait ahead of it.
 cudaError_t launch_qw_embed(const uint8_t *embd_q4k, int d, DevState *state, float *x, bool pdl, cudaStream_t st);
-cudaError_t launch_qw_fold(const QwCombine &c, int8_t *q, float *s, int32_t *b16, bool pdl, cudaStream_t st);      // combine, norm, image in global memory
-cudaError_t launch_qw_qkv(const KMatDev *mats, float *const *ys_out, const QwCombine &c, bool pdl, cudaStream_t st);
+// norm and image of x in global memory; x_copy (nullable): x as well
+cudaError_t launch_qw_norm(const float *x, const float *norm_w, float eps, int d, int8_t *q, float *s, int32_t *b16, float *x_copy, bool pdl, cudaStream_t st);
+cudaError_t launch_qw_qkv(const KMatDev *mats, float *const *ys_out, const float *x, const float *norm_w, float eps, DevState *state, bool pdl, cudaStream_t st);
 cudaError_t launch_qw_oproj(const KMatDev &wo, const float *act, float *x, DevState *state, bool pdl, cudaStream_t st);      // x += wo . Q8_K(act)
 cudaError_t launch_qw_attn(const float *q, const float *k, const float *v, const float *q_norm, const float *k_norm, const float *rope, float eps, float *kc, float *vc,
                            int nh, int nkv, DevState *state, float *out, bool pdl, cudaStream_t st);
 cudaError_t launch_qw_hint(const float *x, const float *norm_w, float eps, int d, const float *Wt, int ne, float *est, int8_t *q, float *s, int32_t *b16, bool pdl,
                            cudaStream_t st);
-// experts: est's topk largest, or top when est is null; hbuf, part: [slot][ff], [slot][d]
+// experts: est's topk largest, or top when est is null; hbuf: [slot][ff].  down: x += sum over k of w[k] dot of expert k, with the routing that the
+// router publishes as the step's seq-th (est), or top and wts
 cudaError_t launch_qw_gate_up(const KMatDev &gate, const KMatDev &up, const float *est, const int32_t *top, int ne, int topk, int ff, const int8_t *q, const float *s,
                               const int32_t *b16, float *hbuf, DevState *state, bool pdl, cudaStream_t st);
-cudaError_t launch_qw_down(const KMatDev &down, const float *est, const int32_t *top, int ne, int topk, int d, int ff, const float *hbuf, float *part, DevState *state,
-                           bool pdl, cudaStream_t st);
+cudaError_t launch_qw_down(const KMatDev &down, const float *est, const int32_t *top, const float *wts, uint32_t seq, int ne, int topk, int d, int ff, const float *hbuf,
+                           float *x, DevState *state, bool pdl, cudaStream_t st);
 cudaError_t launch_qw_head(const KMatDev &head, const int8_t *q, const float *s, const int32_t *b16, float *logits, DevState *state, bool pdl, cudaStream_t st);
 // Q6_K rows from the GGUF layout (210-byte superblocks) into the aligned planes of KMatDev (planes = 1)
 void launch_q6k_planes(const uint8_t *src, size_t rows, int cols, uint8_t *dst, cudaStream_t st);

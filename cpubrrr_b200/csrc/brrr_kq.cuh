@@ -164,101 +164,171 @@ __device__ __forceinline__ void qw_slice(int w, int n, int &a, int &b) {
 }
 
 // ---------------------------------------------------------------- rows in shared memory (decode kernels)
+// Eight values per lane of a superblock, one warp -> quants packed four to a word, their sum, the scale (the arithmetic of warp_quant_q8k).
+// The quotient v / scale is formed as v (127 / amax) with an approximate reciprocal, which is within 1e-4 of it; rounding by adding
+// 1.5 x 2^23 then gives the same integer unless the value lies that close to a half, where (and for scales out of range) the lane divides.
+// Every lane returns the same scale.  350 cycles with eight warps at work; dividing each value: 1220.
+__device__ __forceinline__ float warp_q8k(const float (&v)[8], uint32_t (&w)[2], int &sum) {
+    float m = 1e-12f;
+#pragma unroll
+    for (int i = 0; i < 8; i++) m = fmaxf(m, fabsf(v[i]));
+    const float amax = __uint_as_float(__reduce_max_sync(0xffffffffu, __float_as_uint(m)));      // not negative: ordered as integers
+    const float sc = __fdiv_rn(amax, 127.0f), inv = __fdividef(127.0f, amax);
+    uint32_t b[8];
+    bool sure = amax < 1e30f;
+#pragma unroll
+    for (int i = 0; i < 8; i++) {
+        const float t = __fmul_rn(v[i], inv), r = __fadd_rn(t, 12582912.0f);
+        b[i] = __float_as_uint(r);
+        sure = sure && fabsf(__fsub_rn(t, __fsub_rn(r, 12582912.0f))) < 0.4995f;
+    }
+    if (!sure) {
+#pragma unroll
+        for (int i = 0; i < 8; i++) b[i] = (uint32_t)brrr_q8_round(v[i], sc);
+    }
+#pragma unroll
+    for (int i = 0; i < 2; i++) w[i] = __byte_perm(__byte_perm(b[4 * i], b[4 * i + 1], 0x0040), __byte_perm(b[4 * i + 2], b[4 * i + 3], 0x0040), 0x5410);
+    sum = __dp4a((int)w[0], 0x01010101, __dp4a((int)w[1], 0x01010101, 0));
+    return sc;
+}
 // Q8_K activation of the decode kernels: quants, one scale per 256 values, and the sums of every 16 quants (Q4_K minima need pairs of
-// them, the -32 of Q6_K each).
-__device__ __forceinline__ void warp_quant_q8k16(const float (&v)[8], int lane, int8_t *q, float *s, int32_t *b16) {
-    float amax = 1e-12f;
-#pragma unroll
-    for (int i = 0; i < 8; i++) amax = fmaxf(amax, fabsf(v[i]));
-#pragma unroll
-    for (int o = 16; o; o >>= 1) amax = fmaxf(amax, __shfl_xor_sync(0xffffffffu, amax, o));
-    const float sc = __fdiv_rn(amax, 127.0f);
-    int qi[8], sum = 0;
-#pragma unroll
-    for (int i = 0; i < 8; i++) { qi[i] = brrr_q8_round(v[i], sc); sum += qi[i]; }
-    const uint32_t lo = (qi[0] & 0xff) | ((qi[1] & 0xff) << 8) | ((qi[2] & 0xff) << 16) | ((uint32_t)(qi[3] & 0xff) << 24);
-    const uint32_t hi = (qi[4] & 0xff) | ((qi[5] & 0xff) << 8) | ((qi[6] & 0xff) << 16) | ((uint32_t)(qi[7] & 0xff) << 24);
-    *reinterpret_cast<uint2 *>(q + lane * 8) = make_uint2(lo, hi);
+// them, the -32 of Q6_K each).  CHUNK: bytes from one run of 64 quants to the next - 64 in global memory, 80 in shared memory, where four
+// lanes per superblock then read theirs from different banks.
+constexpr int KQ_SM_CHUNK = 80;
+template <int CHUNK>
+__device__ __forceinline__ void warp_quant_q8k16(const float (&v)[8], int lane, int sb, int8_t *q, float *s, int32_t *b16) {
+    uint32_t w[2];
+    int sum;
+    const float sc = warp_q8k(v, w, sum);
+    *reinterpret_cast<uint2 *>(q + (4 * sb + (lane >> 3)) * CHUNK + (lane & 7) * 8) = make_uint2(w[0], w[1]);
     sum += __shfl_xor_sync(0xffffffffu, sum, 1);
-    if (!(lane & 1)) b16[lane >> 1] = sum;
-    if (lane == 0) *s = sc;
+    if (!(lane & 1)) b16[sb * 16 + (lane >> 1)] = sum;
+    if (lane == 0) s[sb] = sc;
 }
 
-// Eight lanes own one superblock; lane l8 holds the activations that meet its 16 bytes of quants.
-//   Q4_K: nibble bytes 16 l8 ..: x0 / x1 for the low / high nibbles, b0 = the 32-sum of sub-block l8
-//   Q6_K planes: ql bytes 16 l8 ..: x0 / x1 for the low / high nibbles, b0 / b1 = 32 times their sums
-struct KAct { int4 x0, x1; int b0, b1; };
-__device__ __forceinline__ void kact_load(int type, const int8_t *xsb, const int32_t *b16, int l8, KAct &a) {
-    const int at = type == 12 ? 64 * (l8 >> 1) + 16 * (l8 & 1) : 128 * (l8 >> 2) + 16 * (l8 & 3);
-    a.x0 = *reinterpret_cast<const int4 *>(xsb + at);
-    a.x1 = *reinterpret_cast<const int4 *>(xsb + at + (type == 12 ? 32 : 64));
-    if (type == 12) {
-        const int2 s = *reinterpret_cast<const int2 *>(b16 + 2 * l8);
-        a.b0 = s.x + s.y; a.b1 = 0;
-    } else { a.b0 = 32 * b16[at >> 4]; a.b1 = 32 * b16[(at >> 4) + 4]; }
-}
-
-// This lane's share of a superblock's integers (a: scaled quant sum, mt: minima sum) and the superblock's float scales.
-__device__ __forceinline__ void kq_unit(int type, int nsb, const unsigned char *row, int sb, int l8, const KAct &x, int &a, int &mt, float &d, float &dmin) {
-    const uint32_t M4 = 0x0F0F0F0Fu;
-    int lo = 0, hi = 0;
-    if (type == 12) {
-        const unsigned char *p = row + sb * 144;
-        const uint4 h = *reinterpret_cast<const uint4 *>(p), b = *reinterpret_cast<const uint4 *>(p + 16 + 16 * l8);
-        const bool up = l8 >= 4;                     // sub-blocks 4 .. 7: six bits in two fields
-        const uint32_t sc4 = up ? (h.w & M4) | ((h.y >> 2) & 0x30303030u) : h.y & 0x3F3F3F3Fu;
-        const uint32_t mn4 = up ? ((h.w >> 4) & M4) | ((h.z >> 2) & 0x30303030u) : h.z & 0x3F3F3F3Fu;
-        const uint32_t scp = sc4 >> ((l8 & 2) * 8);
-        lo = __dp4a((int)(b.x & M4), x.x0.x, lo); lo = __dp4a((int)(b.y & M4), x.x0.y, lo);
-        lo = __dp4a((int)(b.z & M4), x.x0.z, lo); lo = __dp4a((int)(b.w & M4), x.x0.w, lo);
-        hi = __dp4a((int)((b.x >> 4) & M4), x.x1.x, hi); hi = __dp4a((int)((b.y >> 4) & M4), x.x1.y, hi);
-        hi = __dp4a((int)((b.z >> 4) & M4), x.x1.z, hi); hi = __dp4a((int)((b.w >> 4) & M4), x.x1.w, hi);
-        a = lo * (int)(scp & 0xFFu) + hi * (int)((scp >> 8) & 0xFFu);
-        mt = (int)((mn4 >> ((l8 & 3) * 8)) & 0xFFu) * x.b0;
-        d = half_bits_to_f32(h.x & 0xffffu); dmin = half_bits_to_f32(h.x >> 16);
+// Four lanes own one superblock (a warp covers eight at a time); lane l4 holds the 64 activations that meet its 32 bytes of quants.
+//   Q4_K: nibble bytes 32 l4 ..: x[0..1] for the low nibbles (sub-block 2 l4), x[2..3] for the high (2 l4 + 1); b[0], b[1] their sums
+//   Q6_K planes: ql bytes 32 l4 ..: x[0..1] / x[2..3] for the low / high nibbles; b: 32 times the sums of the four sixteens.  Lanes with
+//   sw = 1 (every other superblock) hold and read the two sixteens of each in the other order, so that neighbours do not meet in a bank.
+struct KAct { int4 x[4]; int b[4]; };
+template <int TYPE, int CHUNK>
+__device__ __forceinline__ void kact_load(const int8_t *q, const int32_t *b16, int sb, int l4, int sw, KAct &a) {
+    b16 += sb * 16;
+    if (TYPE == 12) {
+        const int4 *p = reinterpret_cast<const int4 *>(q + (4 * sb + l4) * CHUNK);
+        a.x[0] = p[0]; a.x[1] = p[1]; a.x[2] = p[2]; a.x[3] = p[3];
+        const int4 s = *reinterpret_cast<const int4 *>(b16 + 4 * l4);
+        a.b[0] = s.x + s.y; a.b[1] = s.z + s.w; a.b[2] = a.b[3] = 0;
     } else {
-        const int h = l8 >> 2, q = l8 & 3;
-        const uint4 l = *reinterpret_cast<const uint4 *>(row + sb * 128 + 16 * l8);
-        const uint4 u = *reinterpret_cast<const uint4 *>(row + nsb * 128 + sb * 64 + 32 * h + 16 * (q & 1));
-        const signed char *sc = reinterpret_cast<const signed char *>(row) + nsb * 192 + sb * 16 + 8 * h + q;
-        const int sl = q & 2;                        // 2-bit fields: 0 and 4, or 2 and 6
-        const uint32_t M2 = 0x30303030u;
-        const uint32_t ux = u.x >> sl, uy = u.y >> sl, uz = u.z >> sl, uw = u.w >> sl;
-        lo = __dp4a((int)((l.x & M4) | ((ux << 4) & M2)), x.x0.x, lo); lo = __dp4a((int)((l.y & M4) | ((uy << 4) & M2)), x.x0.y, lo);
-        lo = __dp4a((int)((l.z & M4) | ((uz << 4) & M2)), x.x0.z, lo); lo = __dp4a((int)((l.w & M4) | ((uw << 4) & M2)), x.x0.w, lo);
-        hi = __dp4a((int)(((l.x >> 4) & M4) | (ux & M2)), x.x1.x, hi); hi = __dp4a((int)(((l.y >> 4) & M4) | (uy & M2)), x.x1.y, hi);
-        hi = __dp4a((int)(((l.z >> 4) & M4) | (uz & M2)), x.x1.z, hi); hi = __dp4a((int)(((l.w >> 4) & M4) | (uw & M2)), x.x1.w, hi);
-        a = (lo - x.b0) * (int)sc[0] + (hi - x.b1) * (int)sc[4];
-        mt = 0;
-        d = half_bits_to_f32(*reinterpret_cast<const unsigned short *>(row + nsb * 208 + sb * 2)); dmin = 0.0f;
+        const int h = l4 >> 1, b = l4 & 1;
+        const int4 *p = reinterpret_cast<const int4 *>(q + (4 * sb + 2 * h) * CHUNK + 32 * b), *r = reinterpret_cast<const int4 *>(q + (4 * sb + 2 * h + 1) * CHUNK + 32 * b);
+        a.x[0] = p[sw]; a.x[1] = p[sw ^ 1]; a.x[2] = r[sw]; a.x[3] = r[sw ^ 1];
+        const int2 s = *reinterpret_cast<const int2 *>(b16 + 8 * h + 2 * b), t = *reinterpret_cast<const int2 *>(b16 + 8 * h + 4 + 2 * b);
+        a.b[0] = 32 * (sw ? s.y : s.x); a.b[1] = 32 * (sw ? s.x : s.y); a.b[2] = 32 * (sw ? t.y : t.x); a.b[3] = 32 * (sw ? t.x : t.y);
     }
 }
+__device__ __forceinline__ int dp4a_us(uint32_t u, int s, int c) {      // unsigned bytes x signed bytes
+    int r;
+    asm("dp4a.u32.s32 %0, %1, %2, %3;" : "=r"(r) : "r"(u), "r"(s), "r"(c));
+    return r;
+}
 
-// Terms of two superblocks per group of eight lanes: (ys d) a - (ys dmin) mt for Q4_K, (ys d) a for Q6_K, every product rounded on its
-// own as in q4k_row_dot / q6k_row_dot.  The four sums meet in five shuffles: lanes 4 .. 7 of a group keep the second superblock, odd pairs
-// the minima.  Lane 0 of the group returns the first term, lane 4 the second.  All 32 lanes must call it.
-__device__ __forceinline__ float kq_pair_term(int type, int nsb, const unsigned char *row0, int sb0, const KAct &x0, float ys0, const unsigned char *row1, int sb1,
-                                              const KAct &x1, float ys1, int l8) {
-    int a0, a1, m0, m1;
-    float d0, d1, n0, n1;
-    kq_unit(type, nsb, row0, sb0, l8, x0, a0, m0, d0, n0);
-    kq_unit(type, nsb, row1, sb1, l8, x1, a1, m1, d1, n1);
-    const bool second = l8 & 4, minima = l8 & 2;
-    const float ys = second ? ys1 : ys0;
-    int a = second ? a1 : a0;
-    a += __shfl_xor_sync(0xffffffffu, second ? a0 : a1, 4);
-    if (type == 12) {
-        int m = second ? m1 : m0;
-        m += __shfl_xor_sync(0xffffffffu, second ? m0 : m1, 4);
-        int r = minima ? m : a;
-        r += __shfl_xor_sync(0xffffffffu, minima ? a : m, 2);
-        r += __shfl_xor_sync(0xffffffffu, r, 1);
-        const float f = __fmul_rn(__fmul_rn(ys, minima ? (second ? n1 : n0) : (second ? d1 : d0)), (float)r);
-        return __fsub_rn(f, __shfl_xor_sync(0xffffffffu, f, 2));
+__device__ __forceinline__ uint4 kq_lds128(uint32_t a) {
+    uint4 r;
+    asm volatile("ld.shared.v4.u32 {%0, %1, %2, %3}, [%4];" : "=r"(r.x), "=r"(r.y), "=r"(r.z), "=r"(r.w) : "r"(a));
+    return r;
+}
+__device__ __forceinline__ uint2 kq_lds64(uint32_t a) {
+    uint2 r;
+    asm volatile("ld.shared.v2.u32 {%0, %1}, [%2];" : "=r"(r.x), "=r"(r.y) : "r"(a));
+    return r;
+}
+__device__ __forceinline__ uint32_t kq_lds16(uint32_t a) {
+    unsigned short r;
+    asm volatile("ld.shared.u16 %0, [%1];" : "=h"(r) : "r"(a));
+    return r;
+}
+
+// Term of a superblock in the row sum: (ys d) a - (ys dmin) mt for Q4_K, (ys d) a for Q6_K, every product rounded on its own as in
+// q4k_row_dot / q6k_row_dot; valid in the first of its four lanes.  row: address of the matrix row in shared memory.  All 32 lanes must
+// call it.  About 100 instructions; 120 cycles per warp and scheduler.
+template <int TYPE>
+__device__ __forceinline__ float kq_term(int nsb, uint32_t row, int sb, const KAct &x, float ys, int l4, int sw) {
+    const uint32_t M4 = 0x0F0F0F0Fu;
+    const int lo4[8] = {x.x[0].x, x.x[0].y, x.x[0].z, x.x[0].w, x.x[1].x, x.x[1].y, x.x[1].z, x.x[1].w};
+    const int hi4[8] = {x.x[2].x, x.x[2].y, x.x[2].z, x.x[2].w, x.x[3].x, x.x[3].y, x.x[3].z, x.x[3].w};
+    if (TYPE == 12) {
+        const uint32_t p = row + sb * 144;
+        const uint4 h = kq_lds128(p), u = kq_lds128(p + 16 + 32 * l4), v = kq_lds128(p + 32 + 32 * l4);
+        const bool upper = l4 >= 2;                  // sub-blocks 4 .. 7: six bits in two fields
+        const uint32_t sc = (upper ? (h.w & M4) | ((h.y >> 2) & 0x30303030u) : h.y & 0x3F3F3F3Fu) >> ((l4 & 1) * 16);
+        const uint32_t mn = (upper ? ((h.w >> 4) & M4) | ((h.z >> 2) & 0x30303030u) : h.z & 0x3F3F3F3Fu) >> ((l4 & 1) * 16);
+        const uint32_t w[8] = {u.x, u.y, u.z, u.w, v.x, v.y, v.z, v.w};
+        int lo[2] = {0, 0}, hi[2] = {0, 0};
+#pragma unroll
+        for (int i = 0; i < 8; i++) { lo[i & 1] = dp4a_us(w[i] & M4, lo4[i], lo[i & 1]); hi[i & 1] = dp4a_us(w[i] & 0xF0F0F0F0u, hi4[i], hi[i & 1]); }      // hi: sixteen times its sum
+        const int a = (lo[0] + lo[1]) * (int)(sc & 0xFFu) + ((hi[0] + hi[1]) >> 4) * (int)((sc >> 8) & 0xFFu);
+        const int m = (int)(mn & 0xFFu) * x.b[0] + (int)((mn >> 8) & 0xFFu) * x.b[1];
+        // two shuffles for both sums: even lanes keep a, odd lanes the minima
+        const bool odd = l4 & 1;
+        int r = odd ? m : a;
+        r += __shfl_xor_sync(0xffffffffu, odd ? a : m, 1);
+        r += __shfl_xor_sync(0xffffffffu, r, 2);
+        const float f = __fmul_rn(__fmul_rn(ys, half_bits_to_f32(odd ? h.x >> 16 : h.x & 0xffffu)), (float)r);
+        return __fsub_rn(f, __shfl_xor_sync(0xffffffffu, f, 1));
     }
-    a += __shfl_xor_sync(0xffffffffu, a, 2);
+    const int h = l4 >> 1, b = l4 & 1;
+    const uint32_t lp = row + sb * 128 + 32 * l4, up = row + nsb * 128 + sb * 64 + 32 * h;
+    const int o = sw * 16;
+    const uint4 l0 = kq_lds128(lp + o), l1 = kq_lds128(lp + 16 - o), u0 = kq_lds128(up + o), u1 = kq_lds128(up + 16 - o);
+    const uint2 s8 = kq_lds64(row + nsb * 192 + sb * 16 + 8 * h);
+    const float d = half_bits_to_f32(kq_lds16(row + nsb * 208 + sb * 2));
+    const uint32_t order = (b ? 0x32u : 0x10u), pick = sw ? (order >> 4) | ((order & 15u) << 4) : order;
+    const uint32_t slo = __byte_perm(s8.x, 0, pick), shi = __byte_perm(s8.y, 0, pick), M2 = 0x30303030u;
+    const uint32_t l[8] = {l0.x, l0.y, l0.z, l0.w, l1.x, l1.y, l1.z, l1.w}, u[8] = {u0.x, u0.y, u0.z, u0.w, u1.x, u1.y, u1.z, u1.w};
+    int a = 0;
+#pragma unroll
+    for (int g = 0; g < 2; g++) {                    // sixteen values share a scale
+        int lo = 0, hi = 0;
+#pragma unroll
+        for (int i = 4 * g; i < 4 * g + 4; i++) {
+            const uint32_t t = u[i] >> (2 * b);      // 2-bit fields: 0 and 4, or 2 and 6
+            lo = dp4a_us((l[i] & M4) | ((t << 4) & M2), lo4[i], lo);
+            hi = dp4a_us(((l[i] >> 4) & M4) | (t & M2), hi4[i], hi);
+        }
+        a += (lo - x.b[g]) * (int)(signed char)(slo >> (8 * g)) + (hi - x.b[2 + g]) * (int)(signed char)(shi >> (8 * g));
+    }
     a += __shfl_xor_sync(0xffffffffu, a, 1);
-    return __fmul_rn(__fmul_rn(ys, second ? d1 : d0), (float)a);
+    a += __shfl_xor_sync(0xffffffffu, a, 2);
+    return __fmul_rn(__fmul_rn(ys, d), (float)a);
+}
+
+// Sum of squares of v[0 .. n) in order by one thread: the next sixteen values are read while sixteen squares are added (7 cycles a value;
+// with a bounds check per value 11, without reading ahead 16).  v must be readable for 16 floats.
+__device__ __forceinline__ float chain_squares(const float *v, int n) {
+    float ps = 0.0f, b[16];
+    const int m = n & ~15;
+#pragma unroll
+    for (int k = 0; k < 16; k++) b[k] = v[k];
+#pragma unroll 1
+    for (int i = 16; i <= m; i += 16) {
+        float p[16];
+#pragma unroll
+        for (int k = 0; k < 16; k++) p[k] = __fmul_rn(b[k], b[k]);
+        const float *w = v + (i + 16 <= n ? i : n > 16 ? n - 16 : 0);        // the last ones: the end, of which the tail picks its part
+#pragma unroll
+        for (int k = 0; k < 16; k++) b[k] = w[k];
+#pragma unroll
+        for (int k = 0; k < 16; k++) ps = __fadd_rn(ps, p[k]);
+    }
+    // tail: the last n - m values; in b from index 16 - (n - m) on (n < 16: from 0 on)
+    const int from = m ? 16 - (n - m) : 0;
+#pragma unroll
+    for (int k = 0; k < 16; k++) {
+        const float t = __fmul_rn(b[k], b[k]);
+        if (m ? k >= from : k < n) ps = __fadd_rn(ps, t);
+    }
+    return ps;
 }
 
 }  // namespace brrr

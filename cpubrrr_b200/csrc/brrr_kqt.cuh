@@ -42,15 +42,11 @@ __device__ __forceinline__ KimgSlot kimg_row(uint8_t *img, float *ys, int t, int
 
 // Q8_K quantisation of one superblock by one warp (the arithmetic of warp_quant_q8k), straight into the image.
 __device__ __forceinline__ void warp_quant_q8k_image(const float (&v)[8], int lane, const KimgSlot &o) {
-    float amax = 1e-12f;
+    uint32_t b[2];
+    int sum, q[8];
+    const float sc = warp_q8k(v, b, sum);
 #pragma unroll
-    for (int i = 0; i < 8; i++) amax = fmaxf(amax, fabsf(v[i]));
-#pragma unroll
-    for (int o = 16; o; o >>= 1) amax = fmaxf(amax, __shfl_xor_sync(0xffffffffu, amax, o));
-    const float sc = __fdiv_rn(amax, 127.0f);
-    int q[8], sum = 0;
-#pragma unroll
-    for (int i = 0; i < 8; i++) { q[i] = brrr_q8_round(v[i], sc); sum += q[i]; }
+    for (int i = 0; i < 8; i++) q[i] = (int)(int8_t)(b[i >> 2] >> (8 * (i & 3)));
     const int order[8] = {0, 2, 1, 3, 4, 6, 5, 7};
     uint32_t w[4];
 #pragma unroll

@@ -8,12 +8,11 @@
 // A step is bound by latency: 36 MB of weights per layer are 5.6 us of memory time, the serial chains and hand-overs more.  So
 // every kernel brings its matrix rows into shared memory with bulk copies, before its dependency wait wherever the rows are known by
 // then (q|k|v, o-proj, down, the first rows of the head; K and V of the cached positions), and the layer is the chain
-//   q|k|v (prologue: expert combine of the layer before, norm, Q8_K - every CTA its own: 64 KB from L2 cost less than a kernel)
-//   -> attention (prologue: QK norm, RoPE, cache append) -> o-proj (prologue: Q8_K) -> routing hint (norm, Q8_K, estimate of the router)
-//   -> gate/up + SiLU-GLU of the estimated experts -> down of the same
+//   q|k|v (prologue: norm, Q8_K) -> attention (prologue: QK norm, RoPE, cache append) -> o-proj (prologue: Q8_K) -> routing hint (norm,
+//   Q8_K, estimate of the router) -> gate/up + SiLU-GLU of the estimated experts -> down of the same (prologue: Q8_K of h) + combine
 // joined by programmatic dependent launch, while the exact router - a chain of d dependent adds, 4.3 us at best at d = 2048 - runs
-// beside the last three on another stream and publishes its choice to the next combine, which takes the weights and the order from
-// it and flags the step if the estimate missed an expert (the host runs that step again without the estimate).
+// beside the last three on another stream and publishes its choice to the combine, which takes the weights and the order from it and
+// flags the step if the estimate missed an expert (the host runs that step again without the estimate).
 #include "brrr_kernels.h"
 #include "brrr_kq.cuh"
 #include "brrr_block.cuh"
@@ -46,104 +45,83 @@ __global__ void __launch_bounds__(256) qw_embed_kernel(const uint8_t *__restrict
 }
 
 // ---------------------------------------------------------------- expert selection
-// sel[r] = expert of rank r of est[0 .. ne) (the larger first, the lower index among equals).  Block-wide; ends synchronised.
-struct alignas(16) SelectScratch { float lg[256]; int rank[256]; };
-__device__ __forceinline__ void qw_select(const float *est, int ne, int topk, const DevState *state, SelectScratch &w, int *sel, int tid, int nthreads) {
+// sel[r] = expert of rank r of est[0 .. ne) (the larger first, the lower index among equals).  Block-wide over QG_THREADS (four threads count
+// the rank of an expert, a quarter of the others each); ends synchronised.  All in one warp - eight rounds of a maximum - it took 2.2 us.
+struct alignas(16) QSelect { uint32_t key[256]; };
+__device__ __forceinline__ void qw_select(const float *est, int ne, int topk, const DevState *state, QSelect &w, int *sel, int tid) {
 #ifdef BRRR_TEST_HOOKS
     const bool spoil = state && (state->test_hooks & 1u) && state->pos % 3 == 0;
 #else
     constexpr bool spoil = false;
     (void)state;
 #endif
-    for (int e = tid; e < 256; e += nthreads) { w.lg[e] = e < ne ? __ldcg(est + e) : -INFINITY; w.rank[e] = 0; }
-    if (tid < 8) sel[tid] = 0;
+    if (tid < 256) w.key[tid] = tid < ne ? max(float_orderable(__ldcg(est + tid)), 1u) : 0u;
+    if (tid >= 256 && tid < 264) sel[tid - 256] = 0;
     __syncthreads();
-    const int quarter = ((ne + 15) / 16) * 4;
-    for (int i = tid; i < 4 * ne; i += nthreads) {
-        const int p = i / ne, e = i - p * ne, o0 = p * quarter;
-        const float v = w.lg[e];
+    const int per = (ne + 15) / 16;              // groups of four others per quarter
+#pragma unroll 1
+    for (int e0 = 0; e0 < ne; e0 += QG_THREADS / 4) {
+        const int e = e0 + (tid >> 2), ec = min(e, ne - 1);
+        const uint32_t key = w.key[ec];
         int r = 0;
-        for (int o = o0; o < min(o0 + quarter, 256); o += 4) {
-            const float4 u = *reinterpret_cast<const float4 *>(w.lg + o);
-            r += (u.x > v || (u.x == v && o < e)) + (u.y > v || (u.y == v && o + 1 < e)) + (u.z > v || (u.z == v && o + 2 < e)) + (u.w > v || (u.w == v && o + 3 < e));
+        const int o0 = (tid & 3) * per;
+#pragma unroll 4
+        for (int o = o0; o < o0 + per; o++) {    // among equals the lower index comes first; those of its own group: below
+            const uint4 u = reinterpret_cast<const uint4 *>(w.key)[o];
+            const uint32_t t = o < (ec >> 2) ? key - 1 : key;
+            r += (u.x > t) + (u.y > t) + (u.z > t) + (u.w > t);
         }
-        if (r) atomicAdd(&w.rank[e], r);
+        if ((tid & 3) < (ec & 3)) r += w.key[(ec & ~3) + (tid & 3)] == key;
+        r += __shfl_xor_sync(0xffffffffu, r, 1);
+        r += __shfl_xor_sync(0xffffffffu, r, 2);
+        if (!(tid & 3) && e < ne && tid < QG_THREADS && r < topk) sel[r] = (spoil && r == topk - 1) ? (e + 1) % ne : e;
     }
-    __syncthreads();
-    for (int e = tid; e < ne; e += nthreads)
-        if (w.rank[e] < topk) sel[w.rank[e]] = (spoil && w.rank[e] == topk - 1) ? (e + 1) % ne : e;
     __syncthreads();
 }
 
-// ---------------------------------------------------------------- expert combine + RMS norm + Q8_K (engine_qwen2.rs:432-465, 287-300)
-// x += w[k] part[slot of k], exact experts in rank order (part == nullptr: nothing to add); then norm and quants.
-struct QFold {
-    const float *x_in, *part;        // residual; [slot][d]
-    float *x_out;                    // the new residual (CTA 0 writes it; never x_in: other CTAs may still read that)
-    const float *est;                // slot s of part belongs to rank s of the estimate; nullptr: of top
-    const int32_t *top;              // exact routing (est == nullptr)
-    const float *wts;
-    int ne, topk, d;
-    uint32_t seq;                    // est: this step's seq-th routing is awaited from the router
-    const float *norm_w;             // nullable: combine only
-    float eps;
-    DevState *state;
-};
-struct QFoldShared {
-    SelectScratch sel_ws;
-    int sel[8], slot_of[8];
-    float wts[8], part[QW_NT];
-};
-
-// Before the dependency wait: the estimate's experts and the exact routing, a bounded wait for the router's words (it does not depend on
-// any kernel that waits here, and this kernel leaves it room on every SM).
-__device__ __forceinline__ void qw_fold_routing(const QFold &a, QFoldShared &w, int tid) {
-    if (!a.part) return;
-    if (a.est) qw_select(a.est, a.ne, a.topk, a.state, w.sel_ws, w.sel, tid, QG_THREADS);
-    if (tid < 32) {
-        uint32_t payload = 0u;
-        if (a.est) {
-            if (tid < 16 && (tid & 7) < a.topk) {
-                const uint32_t want = __ldcg(&a.state->fold_seq) + a.seq;
-                const volatile unsigned long long *p = a.state->route_pub + tid;
-                bool ok = false;
-                const long long t0 = clock64();
-                do {
-                    for (int i = 0; i < 64 && !ok; i++) {
-                        const unsigned long long v = *p;
-                        ok = (uint32_t)(v >> 32) == want;
-                        payload = (uint32_t)v;
-                    }
-                } while (!ok && clock64() - t0 < WAIT_CYCLES && *reinterpret_cast<volatile uint32_t *>(&a.state->err) == 0u);
-                if (!ok) {               // the step is void from here: the host runs it again without the estimate
-                    atomicCAS(&a.state->err, (uint32_t)DEV_ERR_NONE, (uint32_t)DEV_ERR_PEER_TIMEOUT);
-                    atomicMin(&a.state->spec_fail_step, a.state->n_out);
+// The exact routing a step's combine uses, by one warp: slot_of[k] = slot (rank of the estimate) of the expert of rank k, wts[k] its weight.
+// est: the words of the step's seq-th publication by the router, awaited with a bound (the router does not depend on any kernel that waits
+// here, and the waiting kernels leave it room on an SM); sel: the estimate's experts.  Else top and weights as they are.
+__device__ __forceinline__ void qw_routing(bool est, const int *sel, const int32_t *top, const float *weights, int topk, uint32_t seq, DevState *state, int *slot_of, float *wts,
+                                           int lane) {
+    uint32_t payload = 0u;
+    if (lane < 16 && (lane & 7) < topk) {
+        if (est) {
+            const uint32_t want = __ldcg(&state->fold_seq) + seq;
+            const volatile unsigned long long *p = state->route_pub + lane;
+            bool ok = false;
+            const long long t0 = clock64();
+            do {
+                for (int i = 0; i < 64 && !ok; i++) {
+                    const unsigned long long v = *p;
+                    ok = (uint32_t)(v >> 32) == want;
+                    payload = (uint32_t)v;
                 }
+            } while (!ok && clock64() - t0 < WAIT_CYCLES && *reinterpret_cast<volatile uint32_t *>(&state->err) == 0u);
+            if (!ok) {               // the step is void from here: the host runs it again without the estimate
+                atomicCAS(&state->err, (uint32_t)DEV_ERR_NONE, (uint32_t)DEV_ERR_PEER_TIMEOUT);
+                atomicMin(&state->spec_fail_step, state->n_out);
             }
-        } else if (tid < 16 && (tid & 7) < a.topk) payload = tid < 8 ? (uint32_t)__ldcg(a.top + tid) : __float_as_uint(__ldcg(a.wts + (tid - 8)));
-        if (tid >= 8 && tid < 8 + a.topk) w.wts[tid - 8] = __uint_as_float(payload);
-        if (tid < a.topk) {
-            int slot = tid;
-            if (a.est) {
-                slot = -1;
-                for (int s = 0; s < a.topk; s++) if (w.sel[s] == (int)payload) slot = s;
-                if (slot < 0) { slot = 0; atomicMin(&a.state->spec_fail_step, a.state->n_out); }      // the estimate missed this expert
-            }
-            w.slot_of[tid] = slot;
-        }
+        } else payload = lane < 8 ? (uint32_t)__ldcg(top + lane) : __float_as_uint(__ldcg(weights + (lane - 8)));
     }
-    __syncthreads();
+    if (lane >= 8 && lane < 8 + topk) wts[lane - 8] = __uint_as_float(payload);
+    if (lane < topk) {
+        int slot = lane;
+        if (est) {
+            slot = -1;
+            for (int s = 0; s < topk; s++) if (sel[s] == (int)payload) slot = s;
+            if (slot < 0) { slot = 0; atomicMin(&state->spec_fail_step, state->n_out); }      // the estimate missed this expert
+        }
+        slot_of[lane] = slot;
+    }
 }
 
-// The 12-slice norm of xf (shared memory, synchronised): 1 / sqrt(mean + eps) in every thread.
+// The 12-slice norm (engine_qwen2.rs:453-465) of xf (shared memory, synchronised): 1 / sqrt(mean + eps) in every thread.
 __device__ __forceinline__ float qw_norm_inv(const float *xf, int d, float eps, float *part, int tid) {
     if (tid < QW_NT) {
         int lo, hi;
         qw_slice(tid, d, lo, hi);
-        float ps = 0.0f;
-#pragma unroll 8
-        for (int i = lo; i < hi; i++) { const float v = xf[i]; ps = __fadd_rn(ps, __fmul_rn(v, v)); }
-        part[tid] = ps;
+        part[tid] = chain_squares(xf + lo, hi - lo);
     }
     __syncthreads();
     float tot = 0.0f;
@@ -151,89 +129,94 @@ __device__ __forceinline__ float qw_norm_inv(const float *xf, int d, float eps, 
     for (int k = 0; k < QW_NT; k++) tot = __fadd_rn(tot, part[k]);
     return __fdiv_rn(1.0f, __fsqrt_rn(__fadd_rn(__fdiv_rn(tot, (float)d), eps)));
 }
-
-// After the wait.  xf: d floats of shared memory; q, s, b16: the Q8_K image (shared or global).
-__device__ __forceinline__ void qw_fold_norm(const QFold &a, QFoldShared &w, float *xf, int8_t *q, float *s, int32_t *b16, bool store, int tid) {
-    const int d = a.d, warp = tid >> 5, lane = tid & 31;
-    for (int g = tid; g < d / 4; g += QG_THREADS) {
-        float4 x = reinterpret_cast<const float4 *>(a.x_in)[g];
-        if (a.part) {
-            float4 p[8];
-#pragma unroll
-            for (int k = 0; k < 8; k++) if (k < a.topk) p[k] = __ldcg(reinterpret_cast<const float4 *>(a.part + (size_t)w.slot_of[k] * d) + g);
-#pragma unroll
-            for (int k = 0; k < 8; k++)
-                if (k < a.topk) {
-                    const float t = w.wts[k];
-                    x.x = __fadd_rn(x.x, __fmul_rn(t, p[k].x)); x.y = __fadd_rn(x.y, __fmul_rn(t, p[k].y));
-                    x.z = __fadd_rn(x.z, __fmul_rn(t, p[k].z)); x.w = __fadd_rn(x.w, __fmul_rn(t, p[k].w));
-                }
-        }
-        reinterpret_cast<float4 *>(xf)[g] = x;
-        if (store) reinterpret_cast<float4 *>(a.x_out)[g] = x;
-    }
-    if (!a.norm_w) return;
+__device__ __forceinline__ void qw_load8(const float *p, float (&v)[8]) {
+    const float4 a = reinterpret_cast<const float4 *>(p)[0], b = reinterpret_cast<const float4 *>(p)[1];
+    v[0] = a.x; v[1] = a.y; v[2] = a.z; v[3] = a.w; v[4] = b.x; v[5] = b.y; v[6] = b.z; v[7] = b.w;
+}
+// Norm and Q8_K of x (global) by a CTA of QG_THREADS, d <= 4096: warp w owns superblock w, whose norm weights it holds in nw.
+template <int CHUNK>
+__device__ __forceinline__ void qw_norm_image(const float *x, const float (&nw)[8], int d, float eps, float *xf, float *part, int8_t *q, float *s, int32_t *b16, int tid) {
+    const int warp = tid >> 5, lane = tid & 31;
+    for (int g = tid; g < d / 4; g += QG_THREADS) reinterpret_cast<float4 *>(xf)[g] = reinterpret_cast<const float4 *>(x)[g];
     __syncthreads();
-    const float inv = qw_norm_inv(xf, d, a.eps, w.part, tid);
-    for (int sb = warp; sb < d / 256; sb += QG_WARPS) {
+    const float inv = qw_norm_inv(xf, d, eps, part, tid);
+    if (warp < d / 256) {
         float v[8];
-        const float4 w0 = reinterpret_cast<const float4 *>(a.norm_w + sb * 256)[lane * 2], w1 = reinterpret_cast<const float4 *>(a.norm_w + sb * 256)[lane * 2 + 1];
-        const float nw[8] = {w0.x, w0.y, w0.z, w0.w, w1.x, w1.y, w1.z, w1.w};
+        qw_load8(xf + warp * 256 + lane * 8, v);
 #pragma unroll
-        for (int i = 0; i < 8; i++) v[i] = __fmul_rn(__fmul_rn(xf[sb * 256 + lane * 8 + i], inv), nw[i]);
-        warp_quant_q8k16(v, lane, q + sb * 256, s + sb, b16 + sb * 16);
+        for (int i = 0; i < 8; i++) v[i] = __fmul_rn(__fmul_rn(v[i], inv), nw[i]);
+        warp_quant_q8k16<CHUNK>(v, lane, warp, q, s, b16);
     }
 }
 
-// the same as a kernel of its own, for the vocabulary head: one CTA, image to global memory
-__global__ void __launch_bounds__(QG_THREADS) qw_fold_kernel(QFold a, int8_t *q, float *s, int32_t *b16) {
-    extern __shared__ __align__(16) unsigned char qsm[];
-    __shared__ QFoldShared w;
-    qw_fold_routing(a, w, threadIdx.x);
-    pdl_wait();
+// the same as a kernel of its own, one CTA, image to global memory (the vocabulary head); x_copy (nullable): x as well
+__global__ void __launch_bounds__(QG_THREADS) qw_norm_kernel(const float *__restrict__ x, const float *__restrict__ w, float eps, int d, int8_t *q, float *s, int32_t *b16,
+                                                             float *x_copy) {
+    extern __shared__ __align__(16) float xf[];
+    __shared__ float part[QW_NT];
+    const int tid = threadIdx.x;
+    float nw[8] = {0, 0, 0, 0, 0, 0, 0, 0};
+    if ((tid >> 5) < d / 256) qw_load8(w + tid * 8, nw);
+    pdl_wait_cta();
     pdl_trigger();
-    qw_fold_norm(a, w, reinterpret_cast<float *>(qsm), q, s, b16, true, threadIdx.x);
+    qw_norm_image<64>(x, nw, d, eps, xf, part, q, s, b16, tid);
+    if (x_copy)
+        for (int i = tid; i < d; i += QG_THREADS) x_copy[i] = xf[i];
 }
 
 // ---------------------------------------------------------------- matrix rows x one activation (q|k|v, o-proj)
-// Lane group g = lane / 8 takes superblocks g, g + 4, ... of every row.  Up to eight superblocks the activation stays in registers from row
-// to row; of wider rows a warp has one or two, and it is read per pair of superblocks (64 registers: two CTAs per SM).
-template <int UPL> struct QLane {
-    KAct x[2];
-    float ys[2];
+// Lane group g = lane / 4 takes superblocks g, g + 8 of every row.  Up to eight superblocks the activation stays in registers from row to row;
+// of wider rows a warp has one or two, and it is read per eight superblocks (64 registers: two CTAs per SM).
+template <int PASSES> struct QLane {
+    KAct x;
+    float ys;
     const int8_t *q;
     const float *s;
     const int32_t *b16;
 };
-__device__ __forceinline__ void qw_lane_pair(int type, int nsb, const int8_t *q, const float *s, const int32_t *b16, int lane, int i0, KAct (&x)[2], float (&ys)[2]) {
-#pragma unroll
-    for (int i = 0; i < 2; i++) {
-        const int sb = min((lane >> 3) + 4 * (i0 + i), nsb - 1);
-        kact_load(type, q + sb * 256, b16 + sb * 16, lane & 7, x[i]);
-        ys[i] = s[sb];
-    }
+template <int TYPE, int CHUNK, int PASSES>
+__device__ __forceinline__ void qw_lane_load(int nsb, const int8_t *q, const float *s, const int32_t *b16, int lane, QLane<PASSES> &a) {
+    if (PASSES == 1) {
+        const int sb = min(lane >> 2, nsb - 1);
+        kact_load<TYPE, CHUNK>(q, b16, sb, lane & 3, sb & 1, a.x);
+        a.ys = s[sb];
+    } else { a.q = q; a.s = s; a.b16 = b16; }
 }
-template <int UPL>
-__device__ __forceinline__ void qw_lane_load(int type, int nsb, const int8_t *q, const float *s, const int32_t *b16, int lane, QLane<UPL> &a) {
-    if (UPL == 2) qw_lane_pair(type, nsb, q, s, b16, lane, 0, a.x, a.ys);
-    else { a.q = q; a.s = s; a.b16 = b16; }
-}
-// superblock terms of a row -> terms[0 .. nsb)
-template <int UPL>
-__device__ __forceinline__ void qw_row_terms(int type, int nsb, const unsigned char *row, QLane<UPL> &a, int lane, float *terms) {
-    const int g = lane >> 3, l8 = lane & 7;
+// superblock terms of a row (address in shared memory) -> terms[0 .. nsb)
+template <int TYPE, int CHUNK, int PASSES>
+__device__ __forceinline__ void qw_row_terms(int nsb, uint32_t row, QLane<PASSES> &a, int lane, float *terms) {
 #pragma unroll 1
-    for (int i = 0; i < UPL; i += 2) {
-        const int sb0 = g + 4 * i, sb1 = sb0 + 4;
-        if (UPL > 2) qw_lane_pair(type, nsb, a.q, a.s, a.b16, lane, i, a.x, a.ys);
-        const float t = kq_pair_term(type, nsb, row, min(sb0, nsb - 1), a.x[0], a.ys[0], row, min(sb1, nsb - 1), a.x[1], a.ys[1], l8);
-        const int sb = l8 ? sb1 : sb0;
-        if (!(l8 & 3) && sb < nsb) terms[sb] = t;
+    for (int i = 0; i < PASSES; i++) {
+        const int sb = (lane >> 2) + 8 * i, c = min(sb, nsb - 1);
+        if (PASSES > 1) {
+            kact_load<TYPE, CHUNK>(a.q, a.b16, c, lane & 3, c & 1, a.x);
+            a.ys = a.s[c];
+        }
+        const float t = kq_term<TYPE>(nsb, row, c, a.x, a.ys, lane & 3, c & 1);
+        if (!(lane & 3) && sb < nsb) terms[sb] = t;
     }
+}
+// rows [i0, i1) of a matrix, in shared memory from address rows on, a warp each
+template <int TYPE, int PASSES>
+__device__ __forceinline__ void qw_rows(int nsb, uint32_t rows, int stride, int i0, int i1, int8_t *q, const float *s, const int32_t *b16, float *terms, int warp, int lane) {
+    QLane<PASSES> x;
+    qw_lane_load<TYPE, KQ_SM_CHUNK>(nsb, q, s, b16, lane, x);
+#pragma unroll 1
+    for (int i = i0 + warp; i < i1; i += QG_WARPS) qw_row_terms<TYPE, KQ_SM_CHUNK>(nsb, rows + i * stride, x, lane, terms + i * nsb);
 }
 __device__ __forceinline__ float qw_terms_sum(const float *t, int nsb) {      // superblocks in order, from zero
     float v = 0.0f;
-    for (int i = 0; i < nsb; i++) v = __fadd_rn(v, t[i]);
+    int i = 0;
+#pragma unroll 1
+    for (; i + 8 <= nsb; i += 8) {
+        float b[8];
+#pragma unroll
+        for (int k = 0; k < 8; k++) b[k] = t[i + k];
+#pragma unroll
+        for (int k = 0; k < 8; k++) v = __fadd_rn(v, b[k]);
+    }
+#pragma unroll 1
+    for (; i < nsb; i++) v = __fadd_rn(v, t[i]);
     return v;
 }
 // up to three matrices of equal width, stacked
@@ -251,76 +234,73 @@ struct KStack {
 
 struct QGemvArgs {
     KStack k;
-    QFold f;                 // FOLD: the activation is the combined, normalised residual
-    const float *act;        // else: these floats, as they are; outputs are added to y
+    const float *x, *norm_w;     // NORM: the activation is the normalised residual x
+    float eps;
+    // else: x as it is; outputs are added to y
     DevState *state;
 };
 
-// Shared memory: rows | xf (FOLD: d floats) | q | scales | 16-sums | terms.
-// Bound: the hand-over, the prologue (combine, norm: 1.3 us) and one pass over rows that are already on chip (35 rows of 8 superblocks on
-// 16 warps: 0.7 us).
-template <int UPL, bool FOLD>
+// Shared memory: rows | xf (NORM: K floats) | q | scales | 16-sums | terms.
+// Bound: the hand-over, the prologue (norm: a chain of K / 12 adds) and one pass over rows that are already on chip.
+template <int PASSES, bool NORM>
 __global__ void __launch_bounds__(QG_THREADS, 2) qw_gemv_kernel(const __grid_constant__ QGemvArgs a) {
     extern __shared__ __align__(16) unsigned char qsm[];
-    __shared__ QFoldShared w;
+    __shared__ float part[QW_NT];
     __shared__ __align__(8) uint64_t bar;
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     const int K = a.k.m[0].cols, nsb = K / 256, row0 = blockIdx.x * a.k.per_cta, n = min(a.k.per_cta, a.k.rows - row0);
     unsigned char *rows = qsm;
     float *xf = reinterpret_cast<float *>(qsm + (size_t)a.k.per_cta * a.k.stride);
-    int8_t *q = reinterpret_cast<int8_t *>(xf + (FOLD ? K : 0));
-    float *s = reinterpret_cast<float *>(q + K);
+    int8_t *q = reinterpret_cast<int8_t *>(xf + (NORM ? K : 0));
+    float *s = reinterpret_cast<float *>(q + nsb * 4 * KQ_SM_CHUNK);
     int32_t *b16 = reinterpret_cast<int32_t *>(s + ((nsb + 3) & ~3));
     float *terms = reinterpret_cast<float *>(b16 + nsb * 16);
     Waiter waiter(a.state ? &a.state->err : nullptr);
-    if (warp == 0) {
-        if (lane == 0) {
-            mbar_init(&bar, 1);
-            mbar_fence_init();
-            uint32_t bytes = 0;
-            for (int i = 0, r = row0, l; i < n;) {           // whole runs of a matrix
-                const int mi = a.k.find(r, l), run = min(n - i, a.k.m[mi].rows - l);
-                bytes += (uint32_t)run * (uint32_t)a.k.m[mi].bpr();
-                i += run; r += run;
+    if (tid == 0) {
+        // whole runs of a matrix's rows; rows narrower than the stride (a stack of both types) one by one
+        mbar_init(&bar, 1);
+        mbar_fence_init();
+        uint32_t bytes = 0;
+        for (int pass = 0; pass < 2; pass++) {
+            for (int i = 0, l; i < n;) {
+                const KMatDev &m = a.k.m[a.k.find(row0 + i, l)];
+                const int run = min(n - i, m.rows - l), rb = (int)m.bpr();
+                if (pass == 0) bytes += (uint32_t)run * rb;
+                else if (rb == a.k.stride) bulk_g2s(rows + (size_t)i * rb, m.p + (size_t)l * rb, (uint32_t)run * rb, &bar);
+                else
+                    for (int r = 0; r < run; r++) bulk_g2s(rows + (size_t)(i + r) * a.k.stride, m.p + (size_t)(l + r) * rb, (uint32_t)rb, &bar);
+                i += run;
             }
-            mbar_expect_tx(&bar, bytes);
-        }
-        __syncwarp();
-        for (int i = lane; i < n; i += 32) {
-            int l;
-            const KMatDev &m = a.k.m[a.k.find(row0 + i, l)];
-            bulk_g2s(rows + (size_t)i * a.k.stride, m.p + (size_t)l * m.bpr(), (uint32_t)m.bpr(), &bar);
+            if (pass == 0) mbar_expect_tx(&bar, bytes);
         }
     }
-    float resid = 0.0f;
+    float resid = 0.0f, nw[8] = {0, 0, 0, 0, 0, 0, 0, 0};
     int my_l = 0;
     const int my_m = tid < n ? a.k.find(row0 + tid, my_l) : 0;
-    if (!FOLD && tid < n) resid = a.k.y[my_m][my_l];         // written two kernels back
-    if (FOLD) qw_fold_routing(a.f, w, tid);
-    pdl_wait();
+    if (!NORM && tid < n) resid = a.k.y[my_m][my_l];         // written several kernels back
+    if (NORM && warp < nsb) qw_load8(a.norm_w + tid * 8, nw);
+    pdl_wait_cta();
     pdl_trigger();
-    if (FOLD) qw_fold_norm(a.f, w, xf, q, s, b16, blockIdx.x == 0, tid);
-    else
-        for (int sb = warp; sb < nsb; sb += QG_WARPS) {
-            const float4 *src = reinterpret_cast<const float4 *>(a.act + sb * 256 + lane * 8);
-            const float4 p0 = src[0], p1 = src[1];
-            const float v[8] = {p0.x, p0.y, p0.z, p0.w, p1.x, p1.y, p1.z, p1.w};
-            warp_quant_q8k16(v, lane, q + sb * 256, s + sb, b16 + sb * 16);
-        }
+    if (NORM) qw_norm_image<KQ_SM_CHUNK>(a.x, nw, K, a.eps, xf, part, q, s, b16, tid);
+    else if (warp < nsb) {
+        float v[8];
+        qw_load8(a.x + tid * 8, v);
+        warp_quant_q8k16<KQ_SM_CHUNK>(v, lane, warp, q, s, b16);
+    }
     __syncthreads();
     waiter.wait(&bar, 0u);
-    QLane<UPL> x;
-    int type = 0;
-    for (int i = warp; i < n; i += QG_WARPS) {
-        int l;
-        const int t = a.k.m[a.k.find(row0 + i, l)].type;
-        if (t != type) { type = t; qw_lane_load<UPL>(type, nsb, q, s, b16, lane, x); }
-        qw_row_terms<UPL>(type, nsb, rows + (size_t)i * a.k.stride, x, lane, terms + i * nsb);
+    const uint32_t rows0 = smem_u32(rows);
+#pragma unroll 1
+    for (int i = 0, l; i < n;) {                 // one matrix of the stack after the other
+        const int mi = a.k.find(row0 + i, l), end = i + min(n - i, a.k.m[mi].rows - l);
+        if (a.k.m[mi].type == 12) qw_rows<12, PASSES>(nsb, rows0, a.k.stride, i, end, q, s, b16, terms, warp, lane);
+        else qw_rows<14, PASSES>(nsb, rows0, a.k.stride, i, end, q, s, b16, terms, warp, lane);
+        i = end;
     }
     __syncthreads();
     if (tid < n) {
         const float v = qw_terms_sum(terms + tid * nsb, nsb);
-        a.k.y[my_m][my_l] = FOLD ? v : __fadd_rn(resid, v);
+        a.k.y[my_m][my_l] = NORM ? v : __fadd_rn(resid, v);
     }
 }
 
@@ -328,10 +308,11 @@ __global__ void __launch_bounds__(QG_THREADS, 2) qw_gemv_kernel(const __grid_con
 // One CTA per query head.  Prologue: QK norm (serial mean square) and RoPE of q and of the position's own k; the first head of a KV group
 // appends k and v to the cache.  score(t): 8 chains (chain c covers dims c, c+8, ..., fused), (c + c+4) per lane, (l0+l1)+(l2+l3), times
 // 1/sqrt(128); maximum over all keys; denominator and the 128 output sums serial over t.
-// K, then V of the cached positions run through one ring of 64-position tiles, a copy per position (rows 136 floats apart: the score
-// threads - (key, half of the chains) - read 16 bytes each from different banks).  The ring starts before the dependency wait.
-// Bound: the chains over the keys (4 cycles each) and 5 cycles of shared-memory reads per key; at 100 positions the prologue.
-constexpr int QA_TILE = 64, QA_STRIDE = 136, QA_SLOTS = 5, QA_THREADS = 288;
+// K, then V of the cached positions run through one ring of 64-position tiles, filled by 16-byte copies that start before the dependency
+// wait (rows 136 floats apart: the score threads - (key, two chains) - read 8 bytes each from different banks; a bulk copy per position
+// costs 53 cycles each, 3400 a tile).
+// Bound: at 100 positions the prologue's and softmax's latencies; then the chains over the keys (4 cycles each).
+constexpr int QA_TILE = 64, QA_STRIDE = 136, QA_SLOTS = 5, QA_THREADS = 256;
 constexpr size_t QA_SMEM = (size_t)QA_SLOTS * QA_TILE * QA_STRIDE * 4 + (size_t)BRRR_MAXSEQ * 4;
 
 struct QAttnArgs {
@@ -343,153 +324,160 @@ struct QAttnArgs {
     float *out;                  // [nh][128]
 };
 
-__device__ __forceinline__ float qa_half_score(const float *kp, const float *qp) {       // four chains of a key, then (c + c+4) with the other half's
-    float s0 = 0.0f, s1 = 0.0f, s2 = 0.0f, s3 = 0.0f;
+__device__ __forceinline__ void qa_cp16(uint32_t dst, const void *src) { asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(dst), "l"(src) : "memory"); }
+
+// two chains of a key, then the others' in the four threads of a key: (c + c+4), (l0 + l1) + (l2 + l3)
+__device__ __forceinline__ float qa_score(const float *kp, const float2 (&q)[16]) {
+    float s0 = 0.0f, s1 = 0.0f;
 #pragma unroll
     for (int i = 0; i < 16; i++) {
-        const float4 k = *reinterpret_cast<const float4 *>(kp + 8 * i), q = *reinterpret_cast<const float4 *>(qp + 8 * i);
-        s0 = __fmaf_rn(k.x, q.x, s0); s1 = __fmaf_rn(k.y, q.y, s1); s2 = __fmaf_rn(k.z, q.z, s2); s3 = __fmaf_rn(k.w, q.w, s3);
+        const float2 k = *reinterpret_cast<const float2 *>(kp + 8 * i);
+        s0 = __fmaf_rn(k.x, q[i].x, s0); s1 = __fmaf_rn(k.y, q[i].y, s1);
     }
-    s0 = __fadd_rn(s0, __shfl_xor_sync(0xffffffffu, s0, 1)); s1 = __fadd_rn(s1, __shfl_xor_sync(0xffffffffu, s1, 1));
-    s2 = __fadd_rn(s2, __shfl_xor_sync(0xffffffffu, s2, 1)); s3 = __fadd_rn(s3, __shfl_xor_sync(0xffffffffu, s3, 1));
-    return __fadd_rn(__fadd_rn(s0, s1), __fadd_rn(s2, s3));
+    s0 = __fadd_rn(s0, __shfl_xor_sync(0xffffffffu, s0, 2));
+    s1 = __fadd_rn(s1, __shfl_xor_sync(0xffffffffu, s1, 2));
+    const float l = __fadd_rn(s0, s1);
+    return __fadd_rn(l, __shfl_xor_sync(0xffffffffu, l, 1));
 }
 
 __global__ void __launch_bounds__(QA_THREADS) qw_attn_kernel(QAttnArgs a) {
     extern __shared__ __align__(16) float asm_[];
     float *ring = asm_, *sc = asm_ + QA_SLOTS * QA_TILE * QA_STRIDE;
-    __shared__ __align__(8) uint64_t full[QA_SLOTS], empty[QA_SLOTS];
     __shared__ __align__(16) float raw[2][QW_HD], nv[2][QW_HD], qs[QW_HD], ks[QW_HD], vs[QW_HD];
     __shared__ float red[8], inv_sh[2], den_sh;
-    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, u = tid & (QW_HD - 1), qk = tid >> 7;
     const int h = blockIdx.x, group = a.nh / a.nkv, kvh = h / group;
     const int pos = (int)a.state->pos, n = pos + 1, nt = (pos + QA_TILE - 1) / QA_TILE;        // the position is an input of the step
     float *kbase = a.kc + (size_t)kvh * BRRR_MAXSEQ * QW_HD, *vbase = a.vc + (size_t)kvh * BRRR_MAXSEQ * QW_HD;
-    Waiter waiter(&a.state->err);
-    if (tid == 256) {
-        for (int i = 0; i < QA_SLOTS; i++) { mbar_init(&full[i], 1); mbar_init(&empty[i], 4); }
-        mbar_fence_init();
-    }
-    float wv = 0.0f, co = 0.0f, si = 0.0f;
-    if (tid < 256) {
-        wv = (tid < QW_HD ? a.q_norm : a.k_norm)[tid & (QW_HD - 1)];
-        const float2 cs = reinterpret_cast<const float2 *>(a.rope)[(size_t)pos * (QW_HD / 2) + (tid & 63)];
-        co = cs.x; si = cs.y;
-    }
-    __syncthreads();
-    if (warp == 8) {
-        // ---- copies: K tiles, then V tiles
-        bool waited = false;
-        for (int t = 0; t < 2 * nt; t++) {
-            const int slot = t % QA_SLOTS, k0 = (t < nt ? t : t - nt) * QA_TILE, cnt = min(QA_TILE, pos - k0);
-            if (t >= QA_SLOTS) {
-                if (!waited) { pdl_wait(); pdl_trigger(); waiter.poison_if_failed(); waited = true; }      // with the others: the next kernel may start
-                waiter.wait(&empty[slot], (uint32_t)(t / QA_SLOTS - 1) & 1u);
-            }
-            if (lane == 0) mbar_expect_tx(&full[slot], (uint32_t)cnt * QW_HD * 4);
-            __syncwarp();
+    const uint32_t ring0 = smem_u32(ring);
+    auto issue = [&](int t) {            // tile t of 2 nt: K, then V; one group of copies, empty past the end
+        if (t < 2 * nt) {
+            const int k0 = (t < nt ? t : t - nt) * QA_TILE, cnt = min(QA_TILE, pos - k0);
             const float *src = (t < nt ? kbase : vbase) + (size_t)k0 * QW_HD;
-            for (int i = lane; i < cnt; i += 32) bulk_g2s(ring + (size_t)(slot * QA_TILE + i) * QA_STRIDE, src + (size_t)i * QW_HD, QW_HD * 4, &full[slot]);
+            const uint32_t dst = ring0 + (t % QA_SLOTS) * QA_TILE * QA_STRIDE * 4;
+#pragma unroll
+            for (int i = 0; i < QA_TILE * 32 / QA_THREADS; i++) {
+                const int k = (tid >> 5) + i * 8;
+                if (k < cnt) qa_cp16(dst + (k * QA_STRIDE + lane * 4) * 4, src + (size_t)k * QW_HD + lane * 4);
+            }
         }
-        if (!waited) { pdl_wait(); pdl_trigger(); }
-        return;
-    }
-    pdl_wait();
+        asm volatile("cp.async.commit_group;" ::: "memory");
+    };
+    auto bar = [&]() { __syncthreads(); };
+    auto landed = [&]() { asm volatile("cp.async.wait_group %0;" ::"n"(QA_SLOTS - 1) : "memory"); };
+#pragma unroll 1
+    for (int t = 0; t < QA_SLOTS; t++) issue(t);      // positions before this one: written in earlier steps
+    const float wv = (qk ? a.k_norm : a.q_norm)[u];
+    const float2 cs = reinterpret_cast<const float2 *>(a.rope)[(size_t)pos * (QW_HD / 2) + (tid & 63)];
+    pdl_wait_cta();
     pdl_trigger();
-    waiter.poison_if_failed();
-    auto bar = [&]() { asm volatile("bar.sync 1, 256;" ::: "memory"); };
-    {
-        const int u = tid & (QW_HD - 1);
-        raw[tid >> 7][u] = tid < QW_HD ? a.q[h * QW_HD + u] : a.k[kvh * QW_HD + u];
-        if (tid < QW_HD) vs[u] = a.v[kvh * QW_HD + u];
-    }
+    raw[qk][u] = qk ? a.k[kvh * QW_HD + u] : a.q[h * QW_HD + u];
+    if (!qk) vs[u] = a.v[kvh * QW_HD + u];
     bar();
-    if (tid == 0 || tid == 32) {
-        const float4 *r = reinterpret_cast<const float4 *>(raw[tid >> 5]);
-        float ms = 0.0f;
-#pragma unroll 8
-        for (int i = 0; i < QW_HD / 4; i++) {
-            const float4 t = r[i];
-            ms = __fadd_rn(ms, __fmul_rn(t.x, t.x)); ms = __fadd_rn(ms, __fmul_rn(t.y, t.y));
-            ms = __fadd_rn(ms, __fmul_rn(t.z, t.z)); ms = __fadd_rn(ms, __fmul_rn(t.w, t.w));
-        }
-        inv_sh[tid >> 5] = __fdiv_rn(1.0f, __fsqrt_rn(__fadd_rn(__fdiv_rn(ms, (float)QW_HD), a.eps)));
-    }
+    if (u == 0) inv_sh[qk] = __fdiv_rn(1.0f, __fsqrt_rn(__fadd_rn(__fdiv_rn(chain_squares(raw[qk], QW_HD), (float)QW_HD), a.eps)));
     bar();
-    nv[tid >> 7][tid & (QW_HD - 1)] = __fmul_rn(__fmul_rn(raw[tid >> 7][tid & (QW_HD - 1)], inv_sh[tid >> 7]), wv);
+    nv[qk][u] = __fmul_rn(__fmul_rn(raw[qk][u], inv_sh[qk]), wv);
     bar();
     {
-        const int u = tid & (QW_HD - 1), c = u & 63;
-        const float aa = nv[tid >> 7][c], bb = nv[tid >> 7][64 + c];
-        const float o = u < 64 ? __fsub_rn(__fmul_rn(aa, co), __fmul_rn(bb, si)) : __fadd_rn(__fmul_rn(bb, co), __fmul_rn(aa, si));
-        (tid < QW_HD ? qs : ks)[u] = o;
+        const int c = u & 63;
+        const float aa = nv[qk][c], bb = nv[qk][64 + c];
+        const float o = u < 64 ? __fsub_rn(__fmul_rn(aa, cs.x), __fmul_rn(bb, cs.y)) : __fadd_rn(__fmul_rn(bb, cs.x), __fmul_rn(aa, cs.y));
+        (qk ? ks : qs)[u] = o;
         if (h % group == 0) {
-            if (tid >= QW_HD) kbase[(size_t)pos * QW_HD + u] = o;
+            if (qk) kbase[(size_t)pos * QW_HD + u] = o;
             else vbase[(size_t)pos * QW_HD + u] = vs[u];
         }
     }
     bar();
-    // ---- scores: a group of four warps per tile, thread = (key, half of the chains)
+    // ---- scores: thread = (key, two chains)
     const float scale = __fdiv_rn(1.0f, __fsqrt_rn((float)QW_HD));
-    const int hf = lane & 1, key = (warp & 3) * 16 + (lane >> 1);
-    for (int t = warp >> 2; t < nt; t += 2) {
-        const int slot = t % QA_SLOTS;
-        waiter.wait(&full[slot], (uint32_t)(t / QA_SLOTS) & 1u);
-        const float s = qa_half_score(ring + (size_t)(slot * QA_TILE + key) * QA_STRIDE + 4 * hf, qs + 4 * hf);
-        if (hf == 0 && t * QA_TILE + key < pos) sc[t * QA_TILE + key] = __fmul_rn(s, scale);
-        __syncwarp();
-        if (lane == 0) mbar_arrive(&empty[slot]);
+    const int c2 = (lane & 3) * 2, key = tid >> 2;
+    float2 qr[16];
+#pragma unroll
+    for (int i = 0; i < 16; i++) qr[i] = *reinterpret_cast<const float2 *>(qs + 8 * i + c2);
+    float mx = __fmul_rn(qa_score(ks + c2, qr), scale);                       // the position's own score, in every thread
+    if (tid == 0) sc[pos] = mx;
+#pragma unroll 1
+    for (int t = 0; t < nt; t++) {
+        landed();
+        bar();
+        const float s = __fmul_rn(qa_score(ring + ((t % QA_SLOTS) * QA_TILE + key) * QA_STRIDE + c2, qr), scale);
+        if (t * QA_TILE + key < pos) {
+            mx = fmaxf(mx, s);
+            if (!(lane & 3)) sc[t * QA_TILE + key] = s;
+        }
+        bar();
+        issue(t + QA_SLOTS);
     }
-    if (warp == 7) {                 // the position itself
-        const float s = qa_half_score(ks + 4 * hf, qs + 4 * hf);
-        if (lane == 0) sc[pos] = __fmul_rn(s, scale);
-    }
-    bar();
-    float mx = -3.402823466e+38f;
-    for (int t = tid; t < n; t += 256) mx = fmaxf(mx, sc[t]);
     mx = warp_max(mx);
     if (lane == 0) red[warp] = mx;
     bar();
     mx = red[0];
 #pragma unroll
     for (int w = 1; w < 8; w++) mx = fmaxf(mx, red[w]);
-    for (int t = tid; t < ((n + 3) & ~3); t += 256) sc[t] = t < n ? brrr_expf_dev(__fsub_rn(sc[t], mx)) : 0.0f;      // +0 past the end changes no sum
+#pragma unroll 1
+    for (int t = tid; t < ((n + 3) & ~3); t += QA_THREADS) sc[t] = t < n ? brrr_expf_dev(__fsub_rn(sc[t], mx)) : 0.0f;      // +0 past the end changes no sum
     bar();
     float acc = 0.0f;
-    if (warp < 4) {
-        for (int t = 0; t < nt; t++) {
-            const int u = nt + t, slot = u % QA_SLOTS, cnt = min(QA_TILE, pos - t * QA_TILE);
-            waiter.wait(&full[slot], (uint32_t)(u / QA_SLOTS) & 1u);
-            const float *vt = ring + (size_t)slot * QA_TILE * QA_STRIDE + tid, *pt = sc + t * QA_TILE;
-            int k = 0;
-#pragma unroll 4
-            for (; k + 4 <= cnt; k += 4) {
-                const float4 p = *reinterpret_cast<const float4 *>(pt + k);
-                acc = __fmaf_rn(vt[k * QA_STRIDE], p.x, acc); acc = __fmaf_rn(vt[(k + 1) * QA_STRIDE], p.y, acc);
-                acc = __fmaf_rn(vt[(k + 2) * QA_STRIDE], p.z, acc); acc = __fmaf_rn(vt[(k + 3) * QA_STRIDE], p.w, acc);
-            }
-            for (; k < cnt; k++) acc = __fmaf_rn(vt[k * QA_STRIDE], pt[k], acc);
-            __syncwarp();
-            if (lane == 0) mbar_arrive(&empty[slot]);
-        }
-        acc = __fmaf_rn(vs[tid], sc[pos], acc);
-    } else if (tid == 128) {
+    if (tid == 128) {
         float den = 0.0f;
-#pragma unroll 4
-        for (int t = 0; t < n; t += 4) {
-            const float4 p = *reinterpret_cast<const float4 *>(sc + t);
-            den = __fadd_rn(den, p.x); den = __fadd_rn(den, p.y); den = __fadd_rn(den, p.z); den = __fadd_rn(den, p.w);
+        float4 p = *reinterpret_cast<const float4 *>(sc);
+#pragma unroll 2
+        for (int t = 4; t < n + 4; t += 4) {
+            const float4 c = p;
+            p = *reinterpret_cast<const float4 *>(sc + (t < n ? t : 0));
+            den = __fadd_rn(den, c.x); den = __fadd_rn(den, c.y); den = __fadd_rn(den, c.z); den = __fadd_rn(den, c.w);
         }
         den_sh = den;
     }
+#pragma unroll 1
+    for (int t = 0; t < nt; t++) {
+        landed();
+        bar();
+        if (tid < QW_HD) {
+            // whole sixteens, the next one's values on the way while this one's are added up; then the rest
+            const int cnt = min(QA_TILE, pos - t * QA_TILE);
+            const float *vt = ring + ((nt + t) % QA_SLOTS) * QA_TILE * QA_STRIDE + tid, *pt = sc + t * QA_TILE;
+            float v[16];
+            float4 p[4];
+#pragma unroll
+            for (int i = 0; i < 16; i++) v[i] = vt[i * QA_STRIDE];
+#pragma unroll
+            for (int i = 0; i < 4; i++) p[i] = *reinterpret_cast<const float4 *>(pt + 4 * i);
+            int k = 0;
+#pragma unroll 1
+            for (; k + 16 <= cnt; k += 16) {
+                const float *w = vt + ((k + 16) & (QA_TILE - 1)) * QA_STRIDE;
+                const float *o = pt + ((k + 16) & (QA_TILE - 1));
+#pragma unroll
+                for (int i = 0; i < 4; i++) {
+                    acc = __fmaf_rn(v[4 * i], p[i].x, acc); v[4 * i] = w[4 * i * QA_STRIDE];
+                    acc = __fmaf_rn(v[4 * i + 1], p[i].y, acc); v[4 * i + 1] = w[(4 * i + 1) * QA_STRIDE];
+                    acc = __fmaf_rn(v[4 * i + 2], p[i].z, acc); v[4 * i + 2] = w[(4 * i + 2) * QA_STRIDE];
+                    acc = __fmaf_rn(v[4 * i + 3], p[i].w, acc); v[4 * i + 3] = w[(4 * i + 3) * QA_STRIDE];
+                    p[i] = *reinterpret_cast<const float4 *>(o + 4 * i);
+                }
+            }
+#pragma unroll
+            for (int i = 0; i < 4; i++) {
+                if (k + 4 * i < cnt) acc = __fmaf_rn(v[4 * i], p[i].x, acc);
+                if (k + 4 * i + 1 < cnt) acc = __fmaf_rn(v[4 * i + 1], p[i].y, acc);
+                if (k + 4 * i + 2 < cnt) acc = __fmaf_rn(v[4 * i + 2], p[i].z, acc);
+                if (k + 4 * i + 3 < cnt) acc = __fmaf_rn(v[4 * i + 3], p[i].w, acc);
+            }
+        }
+        bar();
+        issue(nt + t + QA_SLOTS);
+    }
+    asm volatile("cp.async.wait_all;" ::: "memory");
     bar();
-    if (tid < QW_HD) a.out[h * QW_HD + tid] = __fmul_rn(acc, __fdiv_rn(1.0f, den_sh));
+    if (tid < QW_HD) a.out[h * QW_HD + tid] = __fmul_rn(__fmaf_rn(vs[tid], sc[pos], acc), __fdiv_rn(1.0f, den_sh));
 }
 
 // ---------------------------------------------------------------- routing hint
 // One CTA per expert: an order-free estimate of its router logit (a few ulps from the serial chain), which only decides whose weights start
-// moving (see qw_fold_routing), and a share of the normalised token's Q8_K.  The router row and the norm weights are in registers before
-// the dependency wait.
+// moving (see qw_routing), and a share of the normalised token's Q8_K.  The router row and the norm weights are in registers before
+// the dependency wait; the dot runs beside the norm's chains.
 constexpr int QH_THREADS = 128, QH_MAXG = 8;
 struct QHintArgs {
     const float *x, *norm_w;
@@ -508,7 +496,9 @@ __global__ void __launch_bounds__(QH_THREADS) qw_hint_kernel(QHintArgs a) {
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, e = blockIdx.x, d = a.d, groups = d >> 2;
     const int ntiles = (d + RT_TJ - 1) / RT_TJ;
     const float *wrow = a.Wt + ((size_t)(e >> 5) * ntiles * 32 + (e & 31)) * RT_STRIDE;
+    const int sb = e + warp * gridDim.x;         // this warp's superblock, if any (further ones: at the end)
     float4 w[QH_MAXG];           // router weight x norm weight
+    float nw[8] = {0, 0, 0, 0, 0, 0, 0, 0};
 #pragma unroll
     for (int p = 0; p < QH_MAXG; p++) {
         const int g = tid + p * QH_THREADS;
@@ -519,35 +509,39 @@ __global__ void __launch_bounds__(QH_THREADS) qw_hint_kernel(QHintArgs a) {
             w[p] = make_float4(r.x * n.x, r.y * n.y, r.z * n.z, r.w * n.w);
         }
     }
-    pdl_wait();
+    if (sb < d / 256) qw_load8(a.norm_w + sb * 256 + lane * 8, nw);
+    pdl_wait_cta();
     pdl_trigger();
-    stage_vec4(a.x, xf, d, tid, QH_THREADS);
-    __syncthreads();
     float dot = 0.0f;
 #pragma unroll
     for (int p = 0; p < QH_MAXG; p++) {
         const int g = tid + p * QH_THREADS;
         if (g < groups) {
-            const float4 x = reinterpret_cast<const float4 *>(xf)[g];
+            const float4 x = reinterpret_cast<const float4 *>(a.x)[g];
+            reinterpret_cast<float4 *>(xf)[g] = x;
             dot += w[p].x * x.x + w[p].y * x.y + w[p].z * x.z + w[p].w * x.w;
         }
     }
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) dot += __shfl_xor_sync(0xffffffffu, dot, o);
     if (lane == 0) red[warp] = dot;
+    __syncthreads();
     const float inv = qw_norm_inv(xf, d, a.eps, part, tid);
     if (tid == 0) a.est[e] = inv * (red[0] + red[1] + red[2] + red[3]);
-    for (int sb = e + warp * gridDim.x; sb < d / 256; sb += gridDim.x * (QH_THREADS / 32)) {
+    for (int b = sb; b < d / 256; b += gridDim.x * (QH_THREADS / 32)) {
         float v[8];
+        if (b != sb) qw_load8(a.norm_w + b * 256 + lane * 8, nw);
+        qw_load8(xf + b * 256 + lane * 8, v);
 #pragma unroll
-        for (int i = 0; i < 8; i++) v[i] = __fmul_rn(__fmul_rn(xf[sb * 256 + lane * 8 + i], inv), a.norm_w[sb * 256 + lane * 8 + i]);
-        warp_quant_q8k16(v, lane, a.q + sb * 256, a.s + sb, a.b16 + sb * 16);
+        for (int i = 0; i < 8; i++) v[i] = __fmul_rn(__fmul_rn(v[i], inv), nw[i]);
+        warp_quant_q8k16<64>(v, lane, b, a.q, a.s, a.b16);
     }
 }
 
 // ---------------------------------------------------------------- experts: gate/up + SiLU-GLU (engine_qwen2.rs:419-426)
-// The (slot, row) pairs of gate and up rows are dealt out in runs, so that every SM streams the same bytes (42 pairs, 97 KB); the rows land
-// in groups of sixteen, a row of each matrix per warp.  Nothing is known before the wait: est picks the experts here.
+// The (slot, row) pairs of gate and up rows are dealt out in runs, so that every SM streams the same bytes (42 pairs, 97 KB); they land in
+// groups of sixteen, a row of each matrix per warp.  Nothing is known before the wait: the experts are picked here, then the copies start,
+// one per run of rows (a bulk copy costs its SM about 50 cycles).
 struct QGateUpArgs {
     KMatDev gate, up;
     const float *est;            // nullptr: top
@@ -560,50 +554,65 @@ struct QGateUpArgs {
     DevState *state;
 };
 
-template <int UPL>
+template <int G, int U> struct KPair { static constexpr int gate = G, up = U; };
+
+template <int PASSES>
 __global__ void __launch_bounds__(QG_THREADS, 2) qw_gate_up_kernel(const __grid_constant__ QGateUpArgs a) {
     extern __shared__ __align__(16) unsigned char qsm[];
-    __shared__ SelectScratch ws;
+    __shared__ QSelect ws;
     __shared__ int sel[8];
     __shared__ __align__(8) uint64_t bar[16];
-    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, K = a.gate.cols, nsb = K / 256;
+    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, nsb = a.gate.cols / 256;
     const int i0 = blockIdx.x * a.per_cta, n = min(a.per_cta, a.topk * a.ff - i0), groups = (n + QG_WARPS - 1) / QG_WARPS;
     unsigned char *rg = qsm, *ru = qsm + (size_t)a.per_cta * a.stride_g;
-    int8_t *q = reinterpret_cast<int8_t *>(ru + (size_t)a.per_cta * a.stride_u);
-    float *s = reinterpret_cast<float *>(q + K);
-    int32_t *b16 = reinterpret_cast<int32_t *>(s + ((nsb + 3) & ~3));
-    float *terms = reinterpret_cast<float *>(b16 + nsb * 16);      // [row][gate, up][nsb]
+    float *terms = reinterpret_cast<float *>(ru + (size_t)a.per_cta * a.stride_u);      // [row][gate, up][nsb]
     Waiter waiter(a.state ? &a.state->err : nullptr);
-    if (tid == 0) {
-        for (int i = 0; i < groups; i++) mbar_init(&bar[i], 1);
+    if (tid < 4 * groups && !(tid & 3)) {
+        mbar_init(&bar[tid >> 2], 1);
         mbar_fence_init();
     }
-    pdl_wait();
+    // thread = (group, matrix, first or second run: a group of sixteen pairs touches two slots at most)
+    int run = 0, slot = 0, grp = tid >> 2;
+    uint32_t bytes = 0, expert_bytes = 0;
+    const uint8_t *src = nullptr;
+    unsigned char *dst = nullptr;
+    if (tid < 4 * groups) {
+        const int up = (tid >> 1) & 1, r0 = grp * QG_WARPS, cnt = min(QG_WARPS, n - r0), stride = up ? a.stride_u : a.stride_g;
+        int it = i0 + r0, r = r0;
+        slot = it / a.ff;
+        run = min(cnt, (slot + 1) * a.ff - it);
+        if (tid & 1) { r += run; it += run; run = cnt - run; slot++; }
+        dst = (up ? ru : rg) + (size_t)r * stride;
+        src = (up ? a.up.p : a.gate.p) + (size_t)(it - slot * a.ff) * stride;
+        bytes = (uint32_t)run * stride;
+        expert_bytes = (uint32_t)a.ff * stride;
+        if ((tid & 3) == 0) mbar_expect_tx(&bar[grp], (uint32_t)cnt * (uint32_t)(a.stride_g + a.stride_u));
+    }
+    pdl_wait_cta();
     pdl_trigger();
-    waiter.poison_if_failed();
-    for (int i = tid; i < K / 16; i += QG_THREADS) reinterpret_cast<int4 *>(q)[i] = reinterpret_cast<const int4 *>(a.q)[i];
-    for (int i = tid; i < nsb; i += QG_THREADS) s[i] = a.s[i];
-    for (int i = tid; i < nsb * 16; i += QG_THREADS) b16[i] = a.b16[i];
-    if (a.est) qw_select(a.est, a.ne, a.topk, a.state, ws, sel, tid, QG_THREADS);
+    if (a.est) qw_select(a.est, a.ne, a.topk, a.state, ws, sel, tid);
     else { if (tid < a.topk) sel[tid] = a.top[tid]; __syncthreads(); }
-    if (tid < groups) mbar_expect_tx(&bar[tid], (uint32_t)min(QG_WARPS, n - tid * QG_WARPS) * (uint32_t)(a.stride_g + a.stride_u));
-    for (int i = tid; i < 2 * n; i += QG_THREADS) {
-        const int r = i >> 1, it = i0 + r, ei = it / a.ff;
-        const size_t row = (size_t)sel[ei] * a.ff + (it - ei * a.ff);
-        if (i & 1) bulk_g2s(ru + (size_t)r * a.stride_u, a.up.p + row * a.stride_u, (uint32_t)a.stride_u, &bar[r / QG_WARPS]);
-        else bulk_g2s(rg + (size_t)r * a.stride_g, a.gate.p + row * a.stride_g, (uint32_t)a.stride_g, &bar[r / QG_WARPS]);
-    }
-    QLane<UPL> x;
-    qw_lane_load<UPL>(a.gate.type, nsb, q, s, b16, lane, x);
-    for (int k = 0; k < groups; k++) {
-        const int i = k * QG_WARPS + warp;
-        if (i >= n) break;
-        waiter.wait(&bar[k], 0u);
-        qw_row_terms<UPL>(a.gate.type, nsb, rg + (size_t)i * a.stride_g, x, lane, terms + (size_t)i * 2 * nsb);
-        if (a.up.type != a.gate.type) qw_lane_load<UPL>(a.up.type, nsb, q, s, b16, lane, x);
-        qw_row_terms<UPL>(a.up.type, nsb, ru + (size_t)i * a.stride_u, x, lane, terms + (size_t)i * 2 * nsb + nsb);
-        if (a.up.type != a.gate.type) qw_lane_load<UPL>(a.gate.type, nsb, q, s, b16, lane, x);
-    }
+    if (tid < 4 * groups && run > 0) bulk_g2s(dst, src + (size_t)sel[slot] * expert_bytes, bytes, &bar[grp]);
+    waiter.poison_if_failed();
+    // the activation from global memory (L1 after the first warp)
+    const uint32_t rg0 = smem_u32(rg), ru0 = smem_u32(ru);
+    auto walk = [&](auto types) {
+        constexpr int TG = decltype(types)::gate, TU = decltype(types)::up;
+        QLane<PASSES> x;
+        qw_lane_load<TG, 64>(nsb, a.q, a.s, a.b16, lane, x);
+#pragma unroll 1
+        for (int k = 0; k < groups; k++) {
+            const int i = k * QG_WARPS + warp;
+            if (i >= n) break;
+            waiter.wait(&bar[k], 0u);
+            qw_row_terms<TG, 64>(nsb, rg0 + i * a.stride_g, x, lane, terms + (size_t)i * 2 * nsb);
+            if (TG != TU) qw_lane_load<TU, 64>(nsb, a.q, a.s, a.b16, lane, x);
+            qw_row_terms<TU, 64>(nsb, ru0 + i * a.stride_u, x, lane, terms + ((size_t)i * 2 + 1) * nsb);
+            if (TG != TU) qw_lane_load<TG, 64>(nsb, a.q, a.s, a.b16, lane, x);
+        }
+    };
+    if (a.gate.type == 12) { if (a.up.type == 12) walk(KPair<12, 12>()); else walk(KPair<12, 14>()); }
+    else { if (a.up.type == 12) walk(KPair<14, 12>()); else walk(KPair<14, 14>()); }
     __syncthreads();
     if (tid < n) {
         const float g = qw_terms_sum(terms + (size_t)tid * 2 * nsb, nsb), u = qw_terms_sum(terms + (size_t)tid * 2 * nsb + nsb, nsb);
@@ -611,66 +620,95 @@ __global__ void __launch_bounds__(QG_THREADS, 2) qw_gate_up_kernel(const __grid_
     }
 }
 
-// ---------------------------------------------------------------- down projection of every slot (engine_qwen2.rs:432-441)
-// A CTA owns per_cta rows of each of the slots' matrices: contiguous in memory, fetched before the wait (the routing is two kernels
-// old).  Prologue: Q8_K of h (every CTA all of it: 24 KB from L2).  part[slot][row] = dot; the weights and the order of the combine come
-// later (QFold).
+// ---------------------------------------------------------------- down projection and combine (engine_qwen2.rs:432-441)
+// A CTA owns per_cta outputs: their rows of every slot's matrix are contiguous, fetched before the wait (the routing is two kernels
+// old).  Prologue: Q8_K of h (every CTA all of it: 24 KB from L2).  Then x += w[k] dot[slot of k], the exact experts in rank order.
 struct QDownArgs {
     KMatDev down;
     const float *est;
     const int32_t *top;
+    const float *wts;
+    uint32_t seq;
     int ne, topk, d, ff, per_cta;
     const float *hbuf;
-    float *part;
+    float *x;
     DevState *state;
 };
 
-__global__ void __launch_bounds__(QG_THREADS, 2) qw_down_kernel(const __grid_constant__ QDownArgs a) {
+constexpr int QD_THREADS = QG_THREADS + 32;        // the last warp fetches the routing beside the others
+
+template <int TYPE>
+__device__ __forceinline__ void qw_down_rows(const QDownArgs &a, uint32_t rows, int rb, int nsb, int nun, int n, const int8_t *q, const float *s, const int32_t *b16, float *terms,
+                                             int warp, int lane) {
+    // unit = slot * nsb + superblock; a warp keeps eight units' activations and takes every (16 / passes)-th row
+    const int passes = (nun + 7) / 8, step = QG_WARPS / passes, pass = warp % passes;
+    if (warp >= passes * step) return;
+    const int un = pass * 8 + (lane >> 2), c = min(un, nun - 1), slot = c / nsb;
+    KAct x;
+    kact_load<TYPE, KQ_SM_CHUNK>(q, b16, c, lane & 3, c & 1, x);
+    const float ys = s[c];
+    const uint32_t base = rows + slot * a.per_cta * rb;
+#pragma unroll 1
+    for (int r = warp / passes; r < n; r += step) {
+        const float t = kq_term<TYPE>(nsb, base + r * rb, c - slot * nsb, x, ys, lane & 3, c & 1);
+        if (!(lane & 3) && un < nun) terms[r * nun + un] = t;
+    }
+}
+
+__global__ void __launch_bounds__(QD_THREADS, 2) qw_down_kernel(const __grid_constant__ QDownArgs a) {
     extern __shared__ __align__(16) unsigned char qsm[];
-    __shared__ SelectScratch ws;
-    __shared__ int sel[8];
+    __shared__ QSelect ws;
+    __shared__ int sel[8], slot_of[8];
+    __shared__ float wts[8];
     __shared__ __align__(8) uint64_t bar;
-    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, g = lane >> 3, l8 = lane & 7;
+    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     const int nsb = a.ff / 256, nun = a.topk * nsb, rb = (int)a.down.bpr(), r0 = blockIdx.x * a.per_cta, n = min(a.per_cta, a.d - r0);
     unsigned char *rows = qsm;                                         // [slot][row]
     int8_t *q = reinterpret_cast<int8_t *>(rows + (size_t)a.topk * a.per_cta * rb);
-    float *s = reinterpret_cast<float *>(q + nun * 256);
+    float *s = reinterpret_cast<float *>(q + nun * 4 * KQ_SM_CHUNK);
     int32_t *b16 = reinterpret_cast<int32_t *>(s + ((nun + 3) & ~3));
     float *terms = reinterpret_cast<float *>(b16 + nun * 16);          // [row][slot][nsb]
+    float *dots = terms + (size_t)a.per_cta * nun;                     // [slot][row]
     Waiter waiter(a.state ? &a.state->err : nullptr);
-    if (tid == 0) { mbar_init(&bar, 1); mbar_fence_init(); }
-    if (a.est) qw_select(a.est, a.ne, a.topk, a.state, ws, sel, tid, QG_THREADS);
+    if (a.est) qw_select(a.est, a.ne, a.topk, a.state, ws, sel, tid);
     else { if (tid < a.topk) sel[tid] = a.top[tid]; __syncthreads(); }
-    if (tid == 0) mbar_expect_tx(&bar, (uint32_t)a.topk * n * rb);
-    if (tid < a.topk) bulk_g2s(rows + (size_t)tid * a.per_cta * rb, a.down.p + ((size_t)sel[tid] * a.d + r0) * rb, (uint32_t)n * rb, &bar);
-    pdl_wait();          // h is complete
+    if (warp == 0) {
+        if (lane == 0) {
+            mbar_init(&bar, 1);
+            mbar_fence_init();
+            mbar_expect_tx(&bar, (uint32_t)a.topk * n * rb);
+        }
+        __syncwarp();
+        if (lane < a.topk) bulk_g2s(rows + (size_t)lane * a.per_cta * rb, a.down.p + ((size_t)sel[lane] * a.d + r0) * rb, (uint32_t)n * rb, &bar);
+    }
+    float xr = tid < n ? a.x[r0 + tid] : 0.0f;                         // written several kernels back
+    pdl_wait_cta();      // h is complete
     pdl_trigger();
-    waiter.poison_if_failed();
-    for (int sb = warp; sb < nun; sb += QG_WARPS) {
-        const float4 *src = reinterpret_cast<const float4 *>(a.hbuf + (size_t)sb * 256 + lane * 8);
-        const float4 p0 = src[0], p1 = src[1];
-        const float v[8] = {p0.x, p0.y, p0.z, p0.w, p1.x, p1.y, p1.z, p1.w};
-        warp_quant_q8k16(v, lane, q + sb * 256, s + sb, b16 + sb * 16);
+    if (warp == QG_WARPS) qw_routing(a.est != nullptr, sel, a.top, a.wts, a.topk, a.seq, a.state, slot_of, wts, lane);
+    else {
+        for (int sb = warp; sb < nun; sb += QG_WARPS) {
+            float v[8];
+            qw_load8(a.hbuf + (size_t)sb * 256 + lane * 8, v);
+            warp_quant_q8k16<KQ_SM_CHUNK>(v, lane, sb, q, s, b16);
+        }
+        asm volatile("bar.sync 1, %0;" ::"r"(QG_THREADS) : "memory");
+        waiter.wait(&bar, 0u);
+        if (a.down.type == 12) qw_down_rows<12>(a, smem_u32(rows), rb, nsb, nun, n, q, s, b16, terms, warp, lane);
+        else qw_down_rows<14>(a, smem_u32(rows), rb, nsb, nun, n, q, s, b16, terms, warp, lane);
+        asm volatile("bar.sync 1, %0;" ::"r"(QG_THREADS) : "memory");
+        for (int i = tid; i < n * a.topk; i += QG_THREADS) {
+            const int slot = i / n, r = i - slot * n;
+            dots[slot * n + r] = qw_terms_sum(terms + r * nun + slot * nsb, nsb);
+        }
     }
     __syncthreads();
-    waiter.wait(&bar, 0u);
-    // (row, eight units) at a time: unit = slot * nsb + superblock
-    const int per_row = (nun + 7) / 8, type = a.down.type;
-    for (int it = warp; it < n * per_row; it += QG_WARPS) {
-        const int r = it / per_row, u0 = (it - r * per_row) * 8 + g, u1 = u0 + 4, c0 = min(u0, nun - 1), c1 = min(u1, nun - 1);
-        KAct x0, x1;
-        kact_load(type, q + c0 * 256, b16 + c0 * 16, l8, x0);
-        kact_load(type, q + c1 * 256, b16 + c1 * 16, l8, x1);
-        const int e0 = c0 / nsb, e1 = c1 / nsb;
-        const float t = kq_pair_term(type, nsb, rows + ((size_t)e0 * a.per_cta + r) * rb, c0 - e0 * nsb, x0, s[c0], rows + ((size_t)e1 * a.per_cta + r) * rb, c1 - e1 * nsb, x1,
-                                     s[c1], l8);
-        const int u = l8 ? u1 : u0;
-        if (!(l8 & 3) && u < nun) terms[r * nun + u] = t;
-    }
-    __syncthreads();
-    for (int i = tid; i < n * a.topk; i += QG_THREADS) {
-        const int slot = i / n, r = i - slot * n;
-        a.part[(size_t)slot * a.d + r0 + r] = qw_terms_sum(terms + r * nun + slot * nsb, nsb);
+    if (tid < n) {
+        float p[8];
+#pragma unroll
+        for (int k = 0; k < 8; k++) p[k] = k < a.topk ? __fmul_rn(wts[k], dots[slot_of[k] * n + tid]) : 0.0f;
+#pragma unroll
+        for (int k = 0; k < 8; k++) if (k < a.topk) xr = __fadd_rn(xr, p[k]);
+        a.x[r0 + tid] = xr;
     }
 }
 
@@ -687,7 +725,7 @@ struct QHeadArgs {
     int per_cta, depth;
 };
 
-template <int UPL>
+template <int PASSES>
 __global__ void __launch_bounds__(QG_THREADS + 32) qw_head_kernel(const __grid_constant__ QHeadArgs a) {
     extern __shared__ __align__(16) unsigned char qsm[];
     __shared__ __align__(8) uint64_t full[8], empty[8];
@@ -716,26 +754,33 @@ __global__ void __launch_bounds__(QG_THREADS + 32) qw_head_kernel(const __grid_c
     pdl_wait();
     pdl_trigger();
     waiter.poison_if_failed();
-    QLane<UPL> x;
-    qw_lane_load<UPL>(a.m.type, nsb, a.q, a.s, a.b16, lane, x);
     float *terms = reinterpret_cast<float *>(qsm + (size_t)depth * QG_WARPS * rb) + warp * 2 * nsb;      // the warp's own, two rows
     unsigned long long best = 0ull;
-    for (int t = 0; t < stages; t++) {
-        const int slot = t % depth, i = t * QG_WARPS + warp;
-        waiter.wait(&full[slot], (uint32_t)(t / depth) & 1u);
-        float *tr = terms + (t & 1) * nsb;
-        if (i < n) qw_row_terms<UPL>(a.m.type, nsb, qsm + (size_t)(slot * QG_WARPS + warp) * rb, x, lane, tr);
-        __syncwarp();
-        if (lane == 0) {
-            mbar_arrive(&empty[slot]);
-            if (i < n) {
-                const float v = qw_terms_sum(tr, nsb);
-                a.logits[row0 + i] = v;
-                const unsigned long long key = ((unsigned long long)float_orderable(v) << 32) | (0xFFFFFFFFu - (uint32_t)(row0 + i));
-                best = key > best ? key : best;
+    auto walk = [&](auto types) {
+        constexpr int T = decltype(types)::gate;
+        QLane<PASSES> x;
+        qw_lane_load<T, 64>(nsb, a.q, a.s, a.b16, lane, x);
+        const uint32_t mine = smem_u32(qsm) + warp * rb;
+#pragma unroll 1
+        for (int t = 0; t < stages; t++) {
+            const int slot = t % depth, i = t * QG_WARPS + warp;
+            waiter.wait(&full[slot], (uint32_t)(t / depth) & 1u);
+            float *tr = terms + (t & 1) * nsb;
+            if (i < n) qw_row_terms<T, 64>(nsb, mine + slot * QG_WARPS * rb, x, lane, tr);
+            __syncwarp();
+            if (lane == 0) {
+                mbar_arrive(&empty[slot]);
+                if (i < n) {
+                    const float v = qw_terms_sum(tr, nsb);
+                    a.logits[row0 + i] = v;
+                    const unsigned long long key = ((unsigned long long)float_orderable(v) << 32) | (0xFFFFFFFFu - (uint32_t)(row0 + i));
+                    best = key > best ? key : best;
+                }
             }
         }
-    }
+    };
+    if (a.m.type == 12) walk(KPair<12, 12>());
+    else walk(KPair<14, 14>());
     if (lane == 0) wbest[warp] = best;
     asm volatile("bar.sync 1, %0;" ::"r"(QG_THREADS) : "memory");
     if (tid == 0) {
@@ -761,25 +806,27 @@ __global__ void q6k_planes_kernel(const uint8_t *__restrict__ src, size_t rows, 
     }
 }
 
-// units per lane for rows of nsb superblocks: 2 or 4 (nsb <= 16)
-int qw_upl(int nsb) { return nsb <= 8 ? 2 : nsb <= 16 ? 4 : 0; }
-size_t qw_act_bytes(int nsb) { return (size_t)nsb * 256 + (size_t)((nsb + 3) & ~3) * 4 + (size_t)nsb * 64; }
+// passes of eight superblocks per row (16 at most)
+int qw_passes(int nsb) { return nsb <= 8 ? 1 : nsb <= 16 ? 2 : 0; }
+size_t qw_act_bytes(int nsb) { return (size_t)nsb * 4 * KQ_SM_CHUNK + (size_t)((nsb + 3) & ~3) * 4 + (size_t)nsb * 64; }
 bool qw_type_ok(const KMatDev &m) { return m.type == 12 || (m.type == 14 && m.planes); }
-int qw_rows_per_cta(int rows, size_t bytes_per_row) {      // an even share of 148 SMs, unless that takes more shared memory than two kernels can share
-    const int share = (rows + 147) / 148, fit = (int)(QG_ROW_BYTES / bytes_per_row);
+// An even share of 140 SMs, unless that takes more shared memory than two kernels can share.  Two such kernels, one of them waiting for
+// the router's words, then never fill the 148 SMs' registers and shared memory: the router's CTAs always find room.
+int qw_rows_per_cta(int rows, size_t bytes_per_row) {
+    const int share = (rows + 139) / 140, fit = (int)(QG_ROW_BYTES / bytes_per_row);
     return share < fit ? share : fit;
 }
 constexpr int QG_SMEM_MAX = 200 * 1024;
 
-template <int UPL, bool FOLD>
+template <int PASSES, bool NORM>
 cudaError_t qw_gemv_launch(const QGemvArgs &a, size_t smem, bool pdl, cudaStream_t st) {
     static unsigned long long configured = 0;      // one bit per device
-    cudaError_t e = smem_optin(qw_gemv_kernel<UPL, FOLD>, QG_SMEM_MAX, configured);
+    cudaError_t e = smem_optin(qw_gemv_kernel<PASSES, NORM>, QG_SMEM_MAX, configured);
     if (e != cudaSuccess) return e;
-    return launch_k(qw_gemv_kernel<UPL, FOLD>, dim3((a.k.rows + a.k.per_cta - 1) / a.k.per_cta), dim3(QG_THREADS), smem, st, pdl, a);
+    return launch_k(qw_gemv_kernel<PASSES, NORM>, dim3((a.k.rows + a.k.per_cta - 1) / a.k.per_cta), dim3(QG_THREADS), smem, st, pdl, a);
 }
 
-cudaError_t qw_gemv(const KMatDev *mats, float *const *ys_out, int n, const QFold *f, const float *act, DevState *state, bool pdl, cudaStream_t st) {
+cudaError_t qw_gemv(const KMatDev *mats, float *const *ys_out, int n, const float *x, const float *norm_w, float eps, DevState *state, bool pdl, cudaStream_t st) {
     QGemvArgs a{};
     a.k.n = n;
     size_t stride = 0;
@@ -788,32 +835,30 @@ cudaError_t qw_gemv(const KMatDev *mats, float *const *ys_out, int n, const QFol
         if (mats[i].bpr() > stride) stride = mats[i].bpr();
         if (mats[i].cols != mats[0].cols || !qw_type_ok(mats[i])) return cudaErrorInvalidValue;
     }
-    const int K = mats[0].cols, nsb = K / 256, upl = qw_upl(nsb);
-    if (!upl || (f && (f->d != K || f->topk > 8 || f->ne > 256))) return cudaErrorInvalidValue;
+    const int K = mats[0].cols, nsb = K / 256, passes = qw_passes(nsb);
+    if (!passes) return cudaErrorInvalidValue;
     a.k.stride = (int)stride;
     a.k.per_cta = qw_rows_per_cta(a.k.rows, stride + nsb * 4);
-    if (f) a.f = *f;
-    a.act = act; a.state = state;
-    const size_t smem = (size_t)a.k.per_cta * (stride + nsb * 4) + qw_act_bytes(nsb) + (f ? (size_t)K * 4 : 0);
-    if (f) return upl == 2 ? qw_gemv_launch<2, true>(a, smem, pdl, st) : qw_gemv_launch<4, true>(a, smem, pdl, st);
-    return upl == 2 ? qw_gemv_launch<2, false>(a, smem, pdl, st) : qw_gemv_launch<4, false>(a, smem, pdl, st);
+    a.x = x; a.norm_w = norm_w; a.eps = eps; a.state = state;
+    const size_t smem = (size_t)a.k.per_cta * (stride + nsb * 4) + qw_act_bytes(nsb) + (norm_w ? (size_t)K * 4 : 0);
+    if (norm_w) return passes == 1 ? qw_gemv_launch<1, true>(a, smem, pdl, st) : qw_gemv_launch<2, true>(a, smem, pdl, st);
+    return passes == 1 ? qw_gemv_launch<1, false>(a, smem, pdl, st) : qw_gemv_launch<2, false>(a, smem, pdl, st);
 }
 
-template <int UPL>
+template <int PASSES>
 cudaError_t qw_gate_up_launch(const QGateUpArgs &a, size_t smem, bool pdl, cudaStream_t st) {
     static unsigned long long configured = 0;      // one bit per device
-    cudaError_t e = smem_optin(qw_gate_up_kernel<UPL>, QG_SMEM_MAX, configured);
+    cudaError_t e = smem_optin(qw_gate_up_kernel<PASSES>, QG_SMEM_MAX, configured);
     if (e != cudaSuccess) return e;
-    return launch_k(qw_gate_up_kernel<UPL>, dim3((a.topk * a.ff + a.per_cta - 1) / a.per_cta), dim3(QG_THREADS), smem, st, pdl, a);
+    return launch_k(qw_gate_up_kernel<PASSES>, dim3((a.topk * a.ff + a.per_cta - 1) / a.per_cta), dim3(QG_THREADS), smem, st, pdl, a);
 }
-template <int UPL>
+template <int PASSES>
 cudaError_t qw_head_launch(const QHeadArgs &a, size_t smem, bool pdl, cudaStream_t st) {
     static unsigned long long configured = 0;      // one bit per device
-    cudaError_t e = smem_optin(qw_head_kernel<UPL>, 224 * 1024, configured);
+    cudaError_t e = smem_optin(qw_head_kernel<PASSES>, 224 * 1024, configured);
     if (e != cudaSuccess) return e;
-    return launch_k(qw_head_kernel<UPL>, dim3((a.m.rows + a.per_cta - 1) / a.per_cta), dim3(QG_THREADS + 32), smem, st, pdl, a);
+    return launch_k(qw_head_kernel<PASSES>, dim3((a.m.rows + a.per_cta - 1) / a.per_cta), dim3(QG_THREADS + 32), smem, st, pdl, a);
 }
-QFold qw_fold_args(const QwCombine &c) { return QFold{c.x_in, c.part, c.x_out, c.est, c.top, c.wts, c.ne, c.topk, c.d, c.seq, c.norm_w, c.eps, c.state}; }
 
 }  // namespace
 
@@ -822,18 +867,17 @@ cudaError_t launch_qw_embed(const uint8_t *embd, int d, DevState *state, float *
     return launch_k(qw_embed_kernel, dim3(d / 256), dim3(256), 0, st, pdl, embd, d, state, x);
 }
 
-cudaError_t launch_qw_fold(const QwCombine &c, int8_t *q, float *s, int32_t *b16, bool pdl, cudaStream_t st) {
-    if (c.topk > 8 || c.ne > 256 || c.d > 8192) return cudaErrorInvalidValue;
-    return launch_k(qw_fold_kernel, dim3(1), dim3(QG_THREADS), (size_t)c.d * 4, st, pdl, qw_fold_args(c), q, s, b16);
+cudaError_t launch_qw_norm(const float *x, const float *norm_w, float eps, int d, int8_t *q, float *s, int32_t *b16, float *x_copy, bool pdl, cudaStream_t st) {
+    if (d > 256 * QG_WARPS) return cudaErrorInvalidValue;
+    return launch_k(qw_norm_kernel, dim3(1), dim3(QG_THREADS), (size_t)d * 4, st, pdl, x, norm_w, eps, d, q, s, b16, x_copy);
 }
 
-cudaError_t launch_qw_qkv(const KMatDev *mats, float *const *ys_out, const QwCombine &c, bool pdl, cudaStream_t st) {
-    const QFold f = qw_fold_args(c);
-    return qw_gemv(mats, ys_out, 3, &f, nullptr, c.state, pdl, st);
+cudaError_t launch_qw_qkv(const KMatDev *mats, float *const *ys_out, const float *x, const float *norm_w, float eps, DevState *state, bool pdl, cudaStream_t st) {
+    return qw_gemv(mats, ys_out, 3, x, norm_w, eps, state, pdl, st);
 }
 
 cudaError_t launch_qw_oproj(const KMatDev &wo, const float *act, float *x, DevState *state, bool pdl, cudaStream_t st) {
-    return qw_gemv(&wo, &x, 1, nullptr, act, state, pdl, st);
+    return qw_gemv(&wo, &x, 1, act, nullptr, 0.0f, state, pdl, st);
 }
 
 cudaError_t launch_qw_attn(const float *q, const float *k, const float *v, const float *q_norm, const float *k_norm, const float *rope, float eps, float *kc, float *vc,
@@ -854,38 +898,38 @@ cudaError_t launch_qw_hint(const float *x, const float *norm_w, float eps, int d
 
 cudaError_t launch_qw_gate_up(const KMatDev &gate, const KMatDev &up, const float *est, const int32_t *top, int ne, int topk, int ff, const int8_t *q, const float *s,
                               const int32_t *b16, float *hbuf, DevState *state, bool pdl, cudaStream_t st) {
-    const int nsb = gate.cols / 256, upl = qw_upl(nsb);
-    if (gate.cols != up.cols || !qw_type_ok(gate) || !qw_type_ok(up) || !upl || ne > 256 || topk > 8) return cudaErrorInvalidValue;
+    const int nsb = gate.cols / 256, passes = qw_passes(nsb);
+    if (gate.cols != up.cols || !qw_type_ok(gate) || !qw_type_ok(up) || !passes || ne > 256 || topk > 8) return cudaErrorInvalidValue;
     QGateUpArgs a{gate, up, est, top, ne, topk, ff, 0, (int)gate.bpr(), (int)up.bpr(), q, s, b16, hbuf, state};
     const size_t row = (size_t)a.stride_g + a.stride_u + nsb * 8;
     a.per_cta = qw_rows_per_cta(topk * ff, row);
     if (a.per_cta > 256) return cudaErrorInvalidValue;
-    const size_t smem = a.per_cta * row + qw_act_bytes(nsb);
-    return upl == 2 ? qw_gate_up_launch<2>(a, smem, pdl, st) : qw_gate_up_launch<4>(a, smem, pdl, st);
+    const size_t smem = a.per_cta * row;
+    return passes == 1 ? qw_gate_up_launch<1>(a, smem, pdl, st) : qw_gate_up_launch<2>(a, smem, pdl, st);
 }
 
-cudaError_t launch_qw_down(const KMatDev &down, const float *est, const int32_t *top, int ne, int topk, int d, int ff, const float *hbuf, float *part, DevState *state,
-                           bool pdl, cudaStream_t st) {
+cudaError_t launch_qw_down(const KMatDev &down, const float *est, const int32_t *top, const float *wts, uint32_t seq, int ne, int topk, int d, int ff, const float *hbuf,
+                           float *x, DevState *state, bool pdl, cudaStream_t st) {
     if (!qw_type_ok(down) || ff % 256 || ff > 1024 || topk > 8 || ne > 256) return cudaErrorInvalidValue;
-    QDownArgs a{down, est, top, ne, topk, d, ff, 0, hbuf, part, state};
+    QDownArgs a{down, est, top, wts, seq, ne, topk, d, ff, 0, hbuf, x, state};
     const int nun = topk * (ff / 256);
-    const size_t row = (size_t)topk * down.bpr() + nun * 4;
+    const size_t row = (size_t)topk * down.bpr() + nun * 4 + topk * 4;
     a.per_cta = qw_rows_per_cta(d, row);
     static unsigned long long configured = 0;      // one bit per device
     cudaError_t e = smem_optin(qw_down_kernel, QG_SMEM_MAX, configured);
     if (e != cudaSuccess) return e;
-    return launch_k(qw_down_kernel, dim3((d + a.per_cta - 1) / a.per_cta), dim3(QG_THREADS), a.per_cta * row + qw_act_bytes(nun), st, pdl, a);
+    return launch_k(qw_down_kernel, dim3((d + a.per_cta - 1) / a.per_cta), dim3(QD_THREADS), a.per_cta * row + qw_act_bytes(nun), st, pdl, a);
 }
 
 cudaError_t launch_qw_head(const KMatDev &head, const int8_t *q, const float *s, const int32_t *b16, float *logits, DevState *state, bool pdl, cudaStream_t st) {
-    const int nsb = head.cols / 256, upl = qw_upl(nsb);
-    if (!qw_type_ok(head) || !upl) return cudaErrorInvalidValue;
+    const int nsb = head.cols / 256, passes = qw_passes(nsb);
+    if (!qw_type_ok(head) || !passes) return cudaErrorInvalidValue;
     const size_t stage = QG_WARPS * head.bpr(), terms = (size_t)QG_WARPS * 2 * nsb * 4;
     const int depth = (int)((220 * 1024 - terms) / stage);
     QHeadArgs a{head, q, s, b16, logits, state, (head.rows + 147) / 148, depth < 8 ? depth : 8};
     a.per_cta = (a.per_cta + QG_WARPS - 1) / QG_WARPS * QG_WARPS;
     const size_t smem = a.depth * stage + terms;
-    return upl == 2 ? qw_head_launch<2>(a, smem, pdl, st) : qw_head_launch<4>(a, smem, pdl, st);
+    return passes == 1 ? qw_head_launch<1>(a, smem, pdl, st) : qw_head_launch<2>(a, smem, pdl, st);
 }
 
 void launch_q6k_planes(const uint8_t *src, size_t rows, int cols, uint8_t *dst, cudaStream_t st) {

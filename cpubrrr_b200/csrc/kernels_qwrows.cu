@@ -72,10 +72,7 @@ __global__ void __launch_bounds__(256) qr_norm_kernel(QrNormArgs a) {
     if (tid < QW_NT) {
         int lo, hi;
         qw_slice(tid, d, lo, hi);
-        float ps = 0.0f;
-#pragma unroll 8
-        for (int i = lo; i < hi; i++) { const float v = xs_sh[i]; ps = __fadd_rn(ps, __fmul_rn(v, v)); }
-        part[tid] = ps;
+        part[tid] = chain_squares(xs_sh + lo, hi - lo);
     }
     __syncthreads();
     float tot = 0.0f;

@@ -38,23 +38,25 @@ void launch_router_pack(const float *W, int ne, int d, float *out, cudaStream_t 
     router_pack_kernel<<<148, 256, 0, st>>>(W, ne, d, out);
 }
 
-// acc += w[j] * x[j] for j = 0..LEN-1, strictly in order, product and sum rounded separately.
-// Products are formed 32 at a time from 128-bit shared-memory reads so that only the adds sit
-// on the dependent chain.
-template <int LEN>
-__device__ __forceinline__ float chain_span(const float *__restrict__ w, const float *__restrict__ x, float acc) {
+// acc += w[j] * x[j] for j = 0..len-1 (len % 64 == 0), strictly in order, product and sum rounded separately.  The operands of the next
+// sixteen products are read while sixteen sums are formed, so that only the adds sit on the dependent path (4 cycles each).
+__device__ __forceinline__ float chain_span(const float *__restrict__ w, const float *__restrict__ x, int len, float acc) {
+    float4 a[4], b[4];
 #pragma unroll
-    for (int j0 = 0; j0 < LEN; j0 += 32) {
-        float p[32];
+    for (int k = 0; k < 4; k++) { a[k] = *reinterpret_cast<const float4 *>(w + 4 * k); b[k] = *reinterpret_cast<const float4 *>(x + 4 * k); }
+#pragma unroll 4
+    for (int j = 0; j < len; j += 16) {
+        float p[16];
 #pragma unroll
-        for (int k = 0; k < 8; k++) {
-            float4 a = *reinterpret_cast<const float4 *>(w + j0 + 4 * k);
-            float4 b = *reinterpret_cast<const float4 *>(x + j0 + 4 * k);
-            p[4 * k] = __fmul_rn(a.x, b.x); p[4 * k + 1] = __fmul_rn(a.y, b.y);
-            p[4 * k + 2] = __fmul_rn(a.z, b.z); p[4 * k + 3] = __fmul_rn(a.w, b.w);
+        for (int k = 0; k < 4; k++) {
+            p[4 * k] = __fmul_rn(a[k].x, b[k].x); p[4 * k + 1] = __fmul_rn(a[k].y, b[k].y);
+            p[4 * k + 2] = __fmul_rn(a[k].z, b[k].z); p[4 * k + 3] = __fmul_rn(a[k].w, b[k].w);
         }
+        const int n = j + 16 < len ? j + 16 : 0;         // past the end: the first ones again, unused
 #pragma unroll
-        for (int k = 0; k < 32; k++) acc = __fadd_rn(acc, p[k]);
+        for (int k = 0; k < 4; k++) { a[k] = *reinterpret_cast<const float4 *>(w + n + 4 * k); b[k] = *reinterpret_cast<const float4 *>(x + n + 4 * k); }
+#pragma unroll
+        for (int k = 0; k < 16; k++) acc = __fadd_rn(acc, p[k]);
     }
     return acc;
 }
@@ -80,43 +82,40 @@ struct RouterArgs {
     int8_t *q8k_q;
     float *q8k_s;
     int32_t *q8k_b16;
-    int stages;              // tiles in flight: 5, or 3 where several CTAs share the experts (an SM then holds a decode kernel beside one)
+    int epc, stages;         // experts per CTA, tiles in flight: 32 and 5; many experts: 8 and all (a lane per expert, nothing to refill, the
+                             // start of every row at once, and room beside the decode kernels of an SM)
 };
 
-// k rounds of warp arg-max over the logits (lane l holds experts l, l+32, ...): the largest value
-// wins, the lower index among equals, which is the order the reference's strict-'>' insertion
-// produces.  Then the softmax over the selected k in rank order.  Warp 0 only.
+// k rounds of warp arg-max over the logits: the largest value wins, the lower index among equals, which is the order the reference's
+// strict-'>' insertion produces.  Lane l holds experts l * per ..., so among equal keys the lowest lane has the lowest index.  Then the
+// softmax over the selected k in rank order, the exponentials side by side.  Warp 0 only.
 __device__ __forceinline__ void warp_topk(const RouterArgs &a, const float *lg, int lane) {
-    float v[8];                                  // up to 256 experts
-    const int per = (a.ne + 31) / 32;
-    for (int i = 0; i < 8; i++) v[i] = (i < per && lane + 32 * i < a.ne) ? lg[lane + 32 * i] : 0.0f;
-    unsigned taken = 0;
-    float tv[8];
-    int tp[8];
-    for (int r = 0; r < a.topk; r++) {
-        unsigned long long best = 0ull;
-        for (int i = 0; i < per; i++) {
-            int e = lane + 32 * i;
-            if (e < a.ne && !(taken & (1u << i))) {
-                unsigned long long key = ((unsigned long long)float_orderable(v[i]) << 32) | (0xFFFFFFFFu - (uint32_t)e);
-                best = key > best ? key : best;
-            }
-        }
+    const int per = (a.ne + 31) / 32;            // up to 256 experts
+    uint32_t key[8];
 #pragma unroll
-        for (int o = 16; o > 0; o >>= 1) {
-            unsigned long long other = __shfl_xor_sync(0xffffffffu, best, o);
-            best = other > best ? other : best;
+    for (int i = 0; i < 8; i++) key[i] = i < per && lane * per + i < a.ne ? max(float_orderable(lg[lane * per + i]), 1u) : 0u;
+    float mine = 0.0f;                           // lane r: logit and expert of rank r
+    int mine_e = 0;
+#pragma unroll 1
+    for (int r = 0; r < a.topk; r++) {
+        uint32_t best = key[0];
+        int at = 0;
+#pragma unroll
+        for (int i = 1; i < 8; i++) if (key[i] > best) { best = key[i]; at = i; }
+        const uint32_t top = __reduce_max_sync(0xffffffffu, best);
+        const int owner = __ffs(__ballot_sync(0xffffffffu, best == top)) - 1, e = min(__shfl_sync(0xffffffffu, lane * per + at, owner), a.ne - 1);
+        if (lane == owner) {
+#pragma unroll
+            for (int i = 0; i < 8; i++) if (i == at) key[i] = 0u;
         }
-        int e = (int)(0xFFFFFFFFu - (uint32_t)(best & 0xFFFFFFFFull));
-        if ((e & 31) == lane) taken |= 1u << (e >> 5);
-        tp[r] = e;
-        tv[r] = lg[e];
+        if (lane == r) { mine = lg[e]; mine_e = e; }
     }
-    if (lane == 0) {
-        float ex[8], wsum = 0.0f;
-        for (int i = 0; i < a.topk; i++) { ex[i] = brrr_expf_dev(__fsub_rn(tv[i], tv[0])); wsum = __fadd_rn(wsum, ex[i]); }
-        for (int i = 0; i < a.topk; i++) { a.wts[i] = __fdiv_rn(ex[i], wsum); a.top[i] = tp[i]; }
-    }
+    const float first = __shfl_sync(0xffffffffu, mine, 0);
+    const float ex = lane < a.topk ? brrr_expf_dev(__fsub_rn(mine, first)) : 0.0f;
+    float wsum = 0.0f;
+    for (int i = 0; i < a.topk; i++) wsum = __fadd_rn(wsum, __shfl_sync(0xffffffffu, ex, i));
+    if (lane < a.topk) { a.wts[lane] = __fdiv_rn(ex, wsum); a.top[lane] = mine_e; }
+    __syncwarp();
 }
 
 // Publication for a consumer that does not wait for this kernel to end (the fused fold of the
@@ -142,9 +141,9 @@ __global__ void __launch_bounds__(RT_THREADS) ffn_in_kernel(RouterArgs a) {
     a.wts += blockIdx.y * 8;
     a.counter += blockIdx.y;
     extern __shared__ __align__(128) unsigned char smraw[];
-    const int stages = a.stages;
+    const int stages = a.stages, epc = a.epc, tile_floats = epc * RT_STRIDE;
     float *tiles = reinterpret_cast<float *>(smraw);                                        // [stages][32][RT_STRIDE]
-    float *xn = reinterpret_cast<float *>(smraw + (size_t)RT_TILE_FLOATS * 4 * stages);   // d floats
+    float *xn = reinterpret_cast<float *>(smraw + (size_t)tile_floats * 4 * stages);   // d floats
     float *lg = xn + a.d;                                                                   // ne floats (top-k staging)
     float *wn = lg + ((a.ne + 3) & ~3);                                        // d floats: norm weights (16-byte aligned: float4 stores)
     uint64_t *bars = reinterpret_cast<uint64_t *>(wn + a.d);                   // [stages] tile landed
@@ -154,15 +153,15 @@ __global__ void __launch_bounds__(RT_THREADS) ffn_in_kernel(RouterArgs a) {
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, d = a.d;
     uint32_t *err = a.state ? &a.state->err : nullptr;
     Waiter waiter(err);
-    const int e0 = blockIdx.x * 32;
-    const int nloc = min(32, a.ne - e0);
+    const int e0 = blockIdx.x * epc;
+    const int nloc = min(epc, a.ne - e0);
     const int ntiles = (d + RT_TJ - 1) / RT_TJ;
-    const float *wsrc = a.Wt + (size_t)blockIdx.x * ntiles * RT_TILE_FLOATS;
+    const float *wsrc = a.Wt + (size_t)(e0 >> 5) * ntiles * RT_TILE_FLOATS + (e0 & 31) * RT_STRIDE;
 
     auto issue = [&](int t) {                                       // one thread
         int slot = t % stages;
-        mbar_expect_tx(&bars[slot], (uint32_t)RT_TILE_FLOATS * 4);
-        bulk_g2s(tiles + (size_t)slot * RT_TILE_FLOATS, wsrc + (size_t)t * RT_TILE_FLOATS, (uint32_t)RT_TILE_FLOATS * 4, &bars[slot]);
+        mbar_expect_tx(&bars[slot], (uint32_t)tile_floats * 4);
+        bulk_g2s(tiles + (size_t)slot * tile_floats, wsrc + (size_t)t * RT_TILE_FLOATS, (uint32_t)tile_floats * 4, &bars[slot]);
     };
     BRRR_STAMP(a.state, 0);
     if (tid == 0) {
@@ -174,7 +173,7 @@ __global__ void __launch_bounds__(RT_THREADS) ffn_in_kernel(RouterArgs a) {
     if (a.norm_w) stage_vec4(a.norm_w, wn, d, tid, RT_THREADS);             // static: fetched before the wait
     const float bias_pre = (warp == 0 && lane < nloc && a.b) ? a.b[e0 + lane] : 0.0f;
     BRRR_STAMP(a.state, 1);
-    pdl_wait();          // residual stream complete
+    pdl_wait_cta();      // residual stream complete
     BRRR_STAMP(a.state, 2);
     BRRR_GT_GO(a.state, 30);
     pdl_trigger();
@@ -188,10 +187,7 @@ __global__ void __launch_bounds__(RT_THREADS) ffn_in_kernel(RouterArgs a) {
             if (tid < QW_NT) {
                 int lo, hi;
                 qw_slice(tid, d, lo, hi);
-                float ps = 0.0f;
-#pragma unroll 8
-                for (int i = lo; i < hi; i++) { const float v = xn[i]; ps = __fadd_rn(ps, __fmul_rn(v, v)); }
-                part[tid] = ps;
+                part[tid] = chain_squares(xn + lo, hi - lo);
             }
             __syncthreads();
             float tot = 0.0f;
@@ -208,7 +204,7 @@ __global__ void __launch_bounds__(RT_THREADS) ffn_in_kernel(RouterArgs a) {
             float v[8];
 #pragma unroll
             for (int i = 0; i < 8; i++) v[i] = xn[sb * 256 + lane * 8 + i];
-            warp_quant_q8k16(v, lane, a.q8k_q + sb * 256, a.q8k_s + sb, a.q8k_b16 + sb * 16);
+            warp_quant_q8k16<64>(v, lane, sb, a.q8k_q, a.q8k_s, a.q8k_b16);
         }
     }
 
@@ -227,11 +223,9 @@ __global__ void __launch_bounds__(RT_THREADS) ffn_in_kernel(RouterArgs a) {
             if (t < 12) BRRR_STAMP(a.state, 8 + t);
             const int slot = t % stages, j0 = t * RT_TJ, len = min(RT_TJ, d - j0);
             waiter.wait(&bars[slot], (uint32_t)(t / stages) & 1u);
-            const float *row = tiles + (size_t)slot * RT_TILE_FLOATS + lane * RT_STRIDE;
+            const float *row = tiles + (size_t)slot * tile_floats + min(lane, epc - 1) * RT_STRIDE;
             const float *xr = xn + j0;
-            if (len == RT_TJ) acc = chain_span<RT_TJ>(row, xr, acc);
-            else
-                for (int jj = 0; jj < len; jj += 32) acc = chain_span<32>(row + jj, xr + jj, acc);   // d % 64 == 0
+            acc = chain_span(row, xr, len, acc);
             __syncwarp();                      // all lanes are done reading this slot
             if (lane == 0 && t + stages < ntiles) mbar_arrive(&empty[slot]);
         }
@@ -408,15 +402,15 @@ cudaError_t launch_ffn_in(const float *x_in, const float *norm_w, float eps, int
                           float *logits, int32_t *top, float *wts, unsigned int *counter, DevState *state, bool pdl, cudaStream_t st, int ntok,
                           uint32_t *signal, int qwen_norm, int8_t *q8k_q, float *q8k_s, int32_t *q8k_b16) {
     RouterArgs a{x_in, norm_w, eps, d, Wt, b, ne, topk, logits, top, wts, counter, state, signal, (signal && state) ? state->route_pub : nullptr,
-                 qwen_norm, q8k_q, q8k_s, q8k_b16, ne > 32 ? 3 : RT_STAGES};
+                 qwen_norm, q8k_q, q8k_s, q8k_b16, ne > 32 ? 8 : 32, ne > 32 ? (d + RT_TJ - 1) / RT_TJ : RT_STAGES};
     if (signal && !state) return cudaErrorInvalidValue;
-    size_t smem = (size_t)RT_TILE_FLOATS * 4 * a.stages + (size_t)d * 8 + (size_t)((ne + 3) & ~3) * 4 + a.stages * 16;
+    size_t smem = (size_t)a.epc * RT_STRIDE * 4 * a.stages + (size_t)d * 8 + (size_t)((ne + 3) & ~3) * 4 + a.stages * 16;
     static unsigned long long configured = 0;      // one bit per device
     {
         cudaError_t e = smem_optin(ffn_in_kernel, 200 * 1024, configured);
         if (e != cudaSuccess) return e;
     }
-    return launch_k(ffn_in_kernel, dim3((ne + 31) / 32, ntok), dim3(RT_THREADS), smem, st, pdl, a);
+    return launch_k(ffn_in_kernel, dim3((ne + a.epc - 1) / a.epc, ntok), dim3(RT_THREADS), smem, st, pdl, a);
 }
 
 // ---------------------------------------------------------------- routing hint (speculation)

@@ -79,8 +79,7 @@ struct brrr_qwen {
     std::vector<QLayer> L;
     float *out_norm = nullptr, *rope = nullptr;
     KMatDev head{}, embd{};
-    float *x = nullptr, *xb[2] = {nullptr, nullptr};      // residual: of the finished step; of the running one, alternating from layer to layer
-    float *q = nullptr, *k = nullptr, *v = nullptr, *ao = nullptr, *hbuf = nullptr, *part = nullptr, *est = nullptr, *rlogits = nullptr, *logits = nullptr, *xs = nullptr,
+    float *x = nullptr, *q = nullptr, *k = nullptr, *v = nullptr, *ao = nullptr, *hbuf = nullptr, *est = nullptr, *rlogits = nullptr, *logits = nullptr, *xs = nullptr,
           *wts = nullptr;
     int8_t *xq = nullptr;
     int32_t *xsum = nullptr, *top = nullptr;
@@ -216,39 +215,36 @@ int qenqueue_step(brrr_qwen *m, bool want, float *trace_dev, int *nlaunch, bool 
     const int d = c.n_embd, nh = c.n_head, nkv = c.n_head_kv, ff = c.n_ff_exp, topk = c.n_expert_used, ne = c.n_expert;
     cudaStream_t s = m->stream;
     const bool pdl = m->use_pdl && !trace_dev;
-    int n = 0, cur = 0;
-    CU(launch_qw_embed(m->embd.p, d, m->st, m->xb[0], false, s)); n++;
+    int n = 0;
+    CU(launch_qw_embed(m->embd.p, d, m->st, m->x, false, s)); n++;
+    if (trace_dev) CU(cudaMemcpyAsync(trace_dev, m->x, d * sizeof(float), cudaMemcpyDeviceToDevice, s));
     const float *est = spec ? m->est : nullptr;
-    auto combine = [&](int layers, float *x_out, const float *norm_w) {      // of the last of `layers` layers run so far
-        return QwCombine{m->xb[cur], layers ? m->part : nullptr, x_out, est, m->top, m->wts, ne, topk, d, (uint32_t)layers, norm_w, c.rms_eps, m->st};
-    };
-    if (trace_dev) CU(cudaMemcpyAsync(trace_dev, m->xb[0], d * sizeof(float), cudaMemcpyDeviceToDevice, s));
     for (int il = 0; il < c.n_layer; il++) {
         QLayer &ly = m->L[il];
         KMatDev qkv[3] = {ly.wq, ly.wk, ly.wv};
-        float *qkv_out[3] = {m->q, m->k, m->v}, *x = m->xb[cur ^ 1];
-        CU(launch_qw_qkv(qkv, qkv_out, combine(il, x, ly.attn_norm), pdl, s)); n++;
-        cur ^= 1;
-        if (trace_dev && il) CU(cudaMemcpyAsync(trace_dev + (size_t)il * d, x, d * sizeof(float), cudaMemcpyDeviceToDevice, s));
+        float *qkv_out[3] = {m->q, m->k, m->v};
+        CU(launch_qw_qkv(qkv, qkv_out, m->x, ly.attn_norm, c.rms_eps, m->st, pdl, s)); n++;
         CU(launch_qw_attn(m->q, m->k, m->v, ly.q_norm, ly.k_norm, m->rope, c.rms_eps, ly.kc, ly.vc, nh, nkv, m->st, m->ao, pdl, s)); n++;
-        CU(launch_qw_oproj(ly.wo, m->ao, x, m->st, pdl, s)); n++;
+        CU(launch_qw_oproj(ly.wo, m->ao, m->x, m->st, pdl, s)); n++;
         if (spec) {
             CU(cudaEventRecord(m->ev_fork, s));
             CU(cudaStreamWaitEvent(m->side, m->ev_fork, 0));
-            CU(launch_ffn_in(x, ly.ffn_norm, c.rms_eps, d, ly.ginp, nullptr, ne, topk, m->rlogits, m->top, m->wts, &m->st->router_done, m->st, false, m->side, 1,
+            CU(launch_ffn_in(m->x, ly.ffn_norm, c.rms_eps, d, ly.ginp, nullptr, ne, topk, m->rlogits, m->top, m->wts, &m->st->router_done, m->st, false, m->side, 1,
                              &m->st->router_seq, 1)); n++;
             CU(cudaEventRecord(m->ev_join, m->side));
-            CU(launch_qw_hint(x, ly.ffn_norm, c.rms_eps, d, ly.ginp, ne, m->est, m->xq, m->xs, m->xsum, pdl, s)); n++;
+            CU(launch_qw_hint(m->x, ly.ffn_norm, c.rms_eps, d, ly.ginp, ne, m->est, m->xq, m->xs, m->xsum, pdl, s)); n++;
         } else {
-            CU(launch_ffn_in(x, ly.ffn_norm, c.rms_eps, d, ly.ginp, nullptr, ne, topk, m->rlogits, m->top, m->wts, &m->st->router_done, m->st, pdl, s, 1, nullptr, 1,
+            CU(launch_ffn_in(m->x, ly.ffn_norm, c.rms_eps, d, ly.ginp, nullptr, ne, topk, m->rlogits, m->top, m->wts, &m->st->router_done, m->st, pdl, s, 1, nullptr, 1,
                              m->xq, m->xs, m->xsum)); n++;
         }
         CU(launch_qw_gate_up(ly.gate, ly.up, est, m->top, ne, topk, ff, m->xq, m->xs, m->xsum, m->hbuf, m->st, pdl, s)); n++;
-        CU(launch_qw_down(ly.down, est, m->top, ne, topk, d, ff, m->hbuf, m->part, m->st, pdl, s)); n++;
+        CU(launch_qw_down(ly.down, est, m->top, m->wts, (uint32_t)il + 1, ne, topk, d, ff, m->hbuf, m->x, m->st, pdl, s)); n++;
+        if (trace_dev) CU(cudaMemcpyAsync(trace_dev + (size_t)(il + 1) * d, m->x, d * sizeof(float), cudaMemcpyDeviceToDevice, s));
     }
-    CU(launch_qw_fold(combine(c.n_layer, m->x, want ? m->out_norm : nullptr), m->xq, m->xs, m->xsum, pdl, s)); n++;
-    if (trace_dev) CU(cudaMemcpyAsync(trace_dev + (size_t)c.n_layer * d, m->x, d * sizeof(float), cudaMemcpyDeviceToDevice, s));
-    if (want) { CU(launch_qw_head(m->head, m->xq, m->xs, m->xsum, m->logits, m->st, pdl, s)); n++; }
+    if (want) {
+        CU(launch_qw_norm(m->x, m->out_norm, c.rms_eps, d, m->xq, m->xs, m->xsum, nullptr, pdl, s)); n++;
+        CU(launch_qw_head(m->head, m->xq, m->xs, m->xsum, m->logits, m->st, pdl, s)); n++;
+    }
     if (spec) CU(cudaStreamWaitEvent(s, m->ev_join, 0));
     if (want) { launch_finish_token(m->st, s); n++; }
     CU(cudaGetLastError());
@@ -316,8 +312,7 @@ int qenqueue_rows(brrr_qwen *m, int rows, int pos0, bool last) {
     }
     if (!last) return BRRR_OK;            // rows that only fill the cache: nobody reads their residual
     CU(launch_qr_norm(r.x, rows, d, part, r.wts, topk, nullptr, c.rms_eps, nullptr, nullptr, nullptr, pdl, s));
-    CU(launch_qw_fold(QwCombine{r.x + (size_t)(rows - 1) * d, nullptr, m->x, nullptr, nullptr, nullptr, ne, topk, d, 0, m->out_norm, c.rms_eps, m->st}, m->xq, m->xs, m->xsum,
-                      pdl, s));
+    CU(launch_qw_norm(r.x + (size_t)(rows - 1) * d, m->out_norm, c.rms_eps, d, m->xq, m->xs, m->xsum, m->x, pdl, s));
     CU(launch_qw_head(m->head, m->xq, m->xs, m->xsum, m->logits, m->st, pdl, s));
     launch_finish_token(m->st, s);
     CU(cudaGetLastError());
@@ -411,8 +406,8 @@ int qbuild(brrr_qwen *m, const QSource &src) {
     TRY(m->alloc(&m->rope, tab.size()));
     CU(cudaMemcpyAsync(m->rope, tab.data(), tab.size() * 4, cudaMemcpyHostToDevice, m->stream));
 
-    TRY(m->alloc(&m->x, d)); TRY(m->alloc(&m->xb[0], d)); TRY(m->alloc(&m->xb[1], d)); TRY(m->alloc(&m->q, nh * hd)); TRY(m->alloc(&m->k, nkv * hd));
-    TRY(m->alloc(&m->v, nkv * hd)); TRY(m->alloc(&m->ao, nh * hd)); TRY(m->alloc(&m->hbuf, (size_t)topk * ff)); TRY(m->alloc(&m->part, (size_t)topk * d));
+    TRY(m->alloc(&m->x, d)); TRY(m->alloc(&m->q, nh * hd)); TRY(m->alloc(&m->k, nkv * hd));
+    TRY(m->alloc(&m->v, nkv * hd)); TRY(m->alloc(&m->ao, nh * hd)); TRY(m->alloc(&m->hbuf, (size_t)topk * ff));
     TRY(m->alloc(&m->est, ne)); TRY(m->alloc(&m->rlogits, ne)); TRY(m->alloc(&m->logits, c.n_vocab));
     TRY(m->alloc(&m->xs, d / 256)); TRY(m->alloc(&m->wts, 8)); TRY(m->alloc(&m->xq, d)); TRY(m->alloc(&m->xsum, d / 16));
     TRY(m->alloc(&m->top, 8)); TRY(m->alloc(&m->st, 1));
