@@ -45,8 +45,10 @@ cudaError_t launch_qw_embed(const uint8_t *embd_q4k, int d, DevState *state, flo
 cudaError_t launch_qw_norm(const float *x, const float *norm_w, float eps, int d, int8_t *q, float *s, int32_t *b16, float *x_copy, bool pdl, cudaStream_t st);
 cudaError_t launch_qw_qkv(const KMatDev *mats, float *const *ys_out, const float *x, const float *norm_w, float eps, DevState *state, bool pdl, cudaStream_t st);
 cudaError_t launch_qw_oproj(const KMatDev &wo, const float *act, float *x, DevState *state, bool pdl, cudaStream_t st);      // x += wo . Q8_K(act)
-cudaError_t launch_qw_attn(const float *q, const float *k, const float *v, const float *q_norm, const float *k_norm, const float *rope, float eps, float *kc, float *vc,
-                           int nh, int nkv, DevState *state, float *out, bool pdl, cudaStream_t st);
+struct QwCache;
+cudaError_t qw_cache(float *kc, float *vc, int nkv, QwCache *out);
+cudaError_t launch_qw_attn(const QwCache &c, const float *q, const float *k, const float *v, const float *q_norm, const float *k_norm, const float *rope, float eps, int nh,
+                           int nkv, DevState *state, float *out, bool pdl, cudaStream_t st);
 cudaError_t launch_qw_hint(const float *x, const float *norm_w, float eps, int d, const float *Wt, int ne, float *est, int8_t *q, float *s, int32_t *b16, bool pdl,
                            cudaStream_t st);
 // experts: est's topk largest, or top when est is null; hbuf: [slot][ff].  down: x += sum over k of w[k] dot of expert k, with the routing that the

@@ -174,17 +174,17 @@ __device__ __forceinline__ float warp_q8k(const float (&v)[8], uint32_t (&w)[2],
     for (int i = 0; i < 8; i++) m = fmaxf(m, fabsf(v[i]));
     const float amax = __uint_as_float(__reduce_max_sync(0xffffffffu, __float_as_uint(m)));      // not negative: ordered as integers
     const float sc = __fdiv_rn(amax, 127.0f), inv = __fdividef(127.0f, amax);
-    uint32_t b[8];
-    bool sure = amax < 1e30f;
+    uint32_t b[8], unsure = 0;
 #pragma unroll
     for (int i = 0; i < 8; i++) {
         const float t = __fmul_rn(v[i], inv), r = __fadd_rn(t, 12582912.0f);
         b[i] = __float_as_uint(r);
-        sure = sure && fabsf(__fsub_rn(t, __fsub_rn(r, 12582912.0f))) < 0.4995f;
+        unsure |= (uint32_t)!(fabsf(__fsub_rn(t, __fsub_rn(r, 12582912.0f))) < 0.4999f) << i;
     }
-    if (!sure) {
+    if (!(amax < 1e30f)) unsure = 0xFFu;
+    if (unsure) {
 #pragma unroll
-        for (int i = 0; i < 8; i++) b[i] = (uint32_t)brrr_q8_round(v[i], sc);
+        for (int i = 0; i < 8; i++) if (unsure & (1u << i)) b[i] = (uint32_t)brrr_q8_round(v[i], sc);
     }
 #pragma unroll
     for (int i = 0; i < 2; i++) w[i] = __byte_perm(__byte_perm(b[4 * i], b[4 * i + 1], 0x0040), __byte_perm(b[4 * i + 2], b[4 * i + 3], 0x0040), 0x5410);
@@ -303,25 +303,25 @@ __device__ __forceinline__ float kq_term(int nsb, uint32_t row, int sb, const KA
     return __fmul_rn(__fmul_rn(ys, d), (float)a);
 }
 
-// Sum of squares of v[0 .. n) in order by one thread: the next sixteen values are read while sixteen squares are added (7 cycles a value;
-// with a bounds check per value 11, without reading ahead 16).  v must be readable for 16 floats.
+// Sum of squares of v[0 .. n) in order by one thread: the next sixteen values are read while sixteen squares are added.  v must be readable
+// for 16 floats.
 __device__ __forceinline__ float chain_squares(const float *v, int n) {
     float ps = 0.0f, b[16];
-    const int m = n & ~15;
+    const int m = n & ~15, last = n > 16 ? n - 16 : 0;
 #pragma unroll
     for (int k = 0; k < 16; k++) b[k] = v[k];
-#pragma unroll 1
+#pragma unroll 2
     for (int i = 16; i <= m; i += 16) {
         float p[16];
 #pragma unroll
         for (int k = 0; k < 16; k++) p[k] = __fmul_rn(b[k], b[k]);
-        const float *w = v + (i + 16 <= n ? i : n > 16 ? n - 16 : 0);        // the last ones: the end, of which the tail picks its part
+        const float *w = v + min(i, last);                   // after the last whole sixteen: the end, of which the tail picks its part
 #pragma unroll
         for (int k = 0; k < 16; k++) b[k] = w[k];
 #pragma unroll
         for (int k = 0; k < 16; k++) ps = __fadd_rn(ps, p[k]);
     }
-    // tail: the last n - m values; in b from index 16 - (n - m) on (n < 16: from 0 on)
+    // tail: the last n - m values, in b from index 16 - (n - m) on (n < 16: from 0 on)
     const int from = m ? 16 - (n - m) : 0;
 #pragma unroll
     for (int k = 0; k < 16; k++) {
@@ -329,6 +329,12 @@ __device__ __forceinline__ float chain_squares(const float *v, int n) {
         if (m ? k >= from : k < n) ps = __fadd_rn(ps, t);
     }
     return ps;
+}
+
+// 1 / sqrt(sum / n + eps); a power of two divides exactly as its reciprocal multiplies
+__device__ __forceinline__ float rms_inv(float sum, int n, float eps) {
+    const float mean = (n & (n - 1)) ? __fdiv_rn(sum, (float)n) : __fmul_rn(sum, __int_as_float((127 - (31 - __clz(n))) << 23));
+    return __fdiv_rn(1.0f, __fsqrt_rn(__fadd_rn(mean, eps)));
 }
 
 }  // namespace brrr

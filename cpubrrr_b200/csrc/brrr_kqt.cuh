@@ -62,6 +62,12 @@ __device__ __forceinline__ void warp_quant_q8k_image(const float (&v)[8], int la
     if (lane == 0) *o.ys = sc;
 }
 
+// K and V of a layer, [kv head][position][128], and as tensors for the decode attention's copies
+struct alignas(64) QwCache {
+    CUtensorMap km, vm;
+    float *k, *v;
+};
+
 // A matrix of 128-row tiles: its bytes as tensors [row][byte] for the copies (Q4_K: boxes of 128 x 144; Q6_K planes: 128 x 128, 64, 16).
 struct alignas(64) KqtMat {
     CUtensorMap map[3];

@@ -460,15 +460,35 @@ __global__ void __launch_bounds__(KT_THREADS, 1) kqt_kernel(const __grid_constan
 
 }  // namespace
 
-cudaError_t kqt_matrix(const KMatDev &m, size_t rows_total, KqtMat *out) {
-    typedef CUresult (*encode_t)(CUtensorMap *, CUtensorMapDataType, cuuint32_t, void *, const cuuint64_t *, const cuuint64_t *, const cuuint32_t *,
-                                 const cuuint32_t *, CUtensorMapInterleave, CUtensorMapSwizzle, CUtensorMapL2promotion, CUtensorMapFloatOOBfill);
+namespace {
+typedef CUresult (*encode_t)(CUtensorMap *, CUtensorMapDataType, cuuint32_t, void *, const cuuint64_t *, const cuuint64_t *, const cuuint32_t *, const cuuint32_t *,
+                             CUtensorMapInterleave, CUtensorMapSwizzle, CUtensorMapL2promotion, CUtensorMapFloatOOBfill);
+encode_t tensor_encode() {
     static encode_t encode = [] {
         void *f = nullptr;
         cudaDriverEntryPointQueryResult r;
         if (cudaGetDriverEntryPointByVersion("cuTensorMapEncodeTiled", &f, 12000, cudaEnableDefault, &r) != cudaSuccess || r != cudaDriverEntryPointSuccess) f = nullptr;
         return (encode_t)f;
     }();
+    return encode;
+}
+}  // namespace
+
+cudaError_t qw_cache(float *kc, float *vc, int nkv, QwCache *out) {
+    const encode_t encode = tensor_encode();
+    if (!encode) return cudaErrorNotSupported;
+    const cuuint64_t dims[2] = {128, (cuuint64_t)nkv * BRRR_MAXSEQ}, strides[1] = {512};
+    const cuuint32_t box[2] = {32, 64}, ones[2] = {1, 1};
+    for (int i = 0; i < 2; i++)
+        if (encode(i ? &out->vm : &out->km, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 2, i ? vc : kc, dims, strides, box, ones, CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B,
+                   CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) != CUDA_SUCCESS)
+            return cudaErrorInvalidValue;
+    out->k = kc; out->v = vc;
+    return cudaSuccess;
+}
+
+cudaError_t kqt_matrix(const KMatDev &m, size_t rows_total, KqtMat *out) {
+    const encode_t encode = tensor_encode();
     if (!encode) return cudaErrorNotSupported;
     if (m.rows % KT_ROWS || m.cols % 256 || (m.type != 12 && !(m.type == 14 && m.planes)) || rows_total % KT_ROWS) return cudaErrorInvalidValue;
     const cuuint64_t dims[2] = {(cuuint64_t)m.bpr(), (cuuint64_t)rows_total}, strides[1] = {(cuuint64_t)m.bpr()};

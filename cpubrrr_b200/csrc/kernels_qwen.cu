@@ -14,7 +14,7 @@
 // beside the last three on another stream and publishes its choice to the combine, which takes the weights and the order from it and
 // flags the step if the estimate missed an expert (the host runs that step again without the estimate).
 #include "brrr_kernels.h"
-#include "brrr_kq.cuh"
+#include "brrr_kqt.cuh"
 #include "brrr_block.cuh"
 #include "brrr_tma.cuh"
 
@@ -47,7 +47,7 @@ __global__ void __launch_bounds__(256) qw_embed_kernel(const uint8_t *__restrict
 // ---------------------------------------------------------------- expert selection
 // sel[r] = expert of rank r of est[0 .. ne) (the larger first, the lower index among equals).  Block-wide over QG_THREADS (four threads count
 // the rank of an expert, a quarter of the others each); ends synchronised.  All in one warp - eight rounds of a maximum - it took 2.2 us.
-struct alignas(16) QSelect { uint32_t key[256]; };
+struct alignas(16) QSelect { uint32_t key[4 * 68]; };        // a quarter of the experts every per * 4 + 4 words: the four read different banks
 __device__ __forceinline__ void qw_select(const float *est, int ne, int topk, const DevState *state, QSelect &w, int *sel, int tid) {
 #ifdef BRRR_TEST_HOOKS
     const bool spoil = state && (state->test_hooks & 1u) && state->pos % 3 == 0;
@@ -55,23 +55,24 @@ __device__ __forceinline__ void qw_select(const float *est, int ne, int topk, co
     constexpr bool spoil = false;
     (void)state;
 #endif
-    if (tid < 256) w.key[tid] = tid < ne ? max(float_orderable(__ldcg(est + tid)), 1u) : 0u;
+    const int per = (ne + 15) / 16, stride = per * 4 + 4;        // groups of four experts per quarter
+    if (tid < 4 * per * 4) w.key[tid / (per * 4) * 4 + tid] = tid < ne ? max(float_orderable(__ldcg(est + tid)), 1u) : 0u;
     if (tid >= 256 && tid < 264) sel[tid - 256] = 0;
     __syncthreads();
-    const int per = (ne + 15) / 16;              // groups of four others per quarter
 #pragma unroll 1
     for (int e0 = 0; e0 < ne; e0 += QG_THREADS / 4) {
         const int e = e0 + (tid >> 2), ec = min(e, ne - 1);
-        const uint32_t key = w.key[ec];
+        const int at = ec / (per * 4) * 4 + ec, quarter = tid & 3;
+        const uint32_t key = w.key[at];
+        const uint4 *others = reinterpret_cast<const uint4 *>(w.key + quarter * stride);
         int r = 0;
-        const int o0 = (tid & 3) * per;
 #pragma unroll 4
-        for (int o = o0; o < o0 + per; o++) {    // among equals the lower index comes first; those of its own group: below
-            const uint4 u = reinterpret_cast<const uint4 *>(w.key)[o];
-            const uint32_t t = o < (ec >> 2) ? key - 1 : key;
+        for (int o = 0; o < per; o++) {          // among equals the lower index comes first; those of its own group: below
+            const uint4 u = others[o];
+            const uint32_t t = quarter * per + o < (ec >> 2) ? key - 1 : key;
             r += (u.x > t) + (u.y > t) + (u.z > t) + (u.w > t);
         }
-        if ((tid & 3) < (ec & 3)) r += w.key[(ec & ~3) + (tid & 3)] == key;
+        if (quarter < (ec & 3)) r += w.key[at - (ec & 3) + quarter] == key;
         r += __shfl_xor_sync(0xffffffffu, r, 1);
         r += __shfl_xor_sync(0xffffffffu, r, 2);
         if (!(tid & 3) && e < ne && tid < QG_THREADS && r < topk) sel[r] = (spoil && r == topk - 1) ? (e + 1) % ne : e;
@@ -124,10 +125,12 @@ __device__ __forceinline__ float qw_norm_inv(const float *xf, int d, float eps, 
         part[tid] = chain_squares(xf + lo, hi - lo);
     }
     __syncthreads();
+    const float4 p0 = reinterpret_cast<const float4 *>(part)[0], p1 = reinterpret_cast<const float4 *>(part)[1], p2 = reinterpret_cast<const float4 *>(part)[2];
+    const float p[QW_NT] = {p0.x, p0.y, p0.z, p0.w, p1.x, p1.y, p1.z, p1.w, p2.x, p2.y, p2.z, p2.w};
     float tot = 0.0f;
 #pragma unroll
-    for (int k = 0; k < QW_NT; k++) tot = __fadd_rn(tot, part[k]);
-    return __fdiv_rn(1.0f, __fsqrt_rn(__fadd_rn(__fdiv_rn(tot, (float)d), eps)));
+    for (int k = 0; k < QW_NT; k++) tot = __fadd_rn(tot, p[k]);
+    return rms_inv(tot, d, eps);
 }
 __device__ __forceinline__ void qw_load8(const float *p, float (&v)[8]) {
     const float4 a = reinterpret_cast<const float4 *>(p)[0], b = reinterpret_cast<const float4 *>(p)[1];
@@ -153,7 +156,7 @@ __device__ __forceinline__ void qw_norm_image(const float *x, const float (&nw)[
 __global__ void __launch_bounds__(QG_THREADS) qw_norm_kernel(const float *__restrict__ x, const float *__restrict__ w, float eps, int d, int8_t *q, float *s, int32_t *b16,
                                                              float *x_copy) {
     extern __shared__ __align__(16) float xf[];
-    __shared__ float part[QW_NT];
+    __shared__ __align__(16) float part[QW_NT];
     const int tid = threadIdx.x;
     float nw[8] = {0, 0, 0, 0, 0, 0, 0, 0};
     if ((tid >> 5) < d / 256) qw_load8(w + tid * 8, nw);
@@ -245,7 +248,7 @@ struct QGemvArgs {
 template <int PASSES, bool NORM>
 __global__ void __launch_bounds__(QG_THREADS, 2) qw_gemv_kernel(const __grid_constant__ QGemvArgs a) {
     extern __shared__ __align__(16) unsigned char qsm[];
-    __shared__ float part[QW_NT];
+    __shared__ __align__(16) float part[QW_NT];
     __shared__ __align__(8) uint64_t bar;
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     const int K = a.k.m[0].cols, nsb = K / 256, row0 = blockIdx.x * a.k.per_cta, n = min(a.k.per_cta, a.k.rows - row0);
@@ -308,14 +311,17 @@ __global__ void __launch_bounds__(QG_THREADS, 2) qw_gemv_kernel(const __grid_con
 // One CTA per query head.  Prologue: QK norm (serial mean square) and RoPE of q and of the position's own k; the first head of a KV group
 // appends k and v to the cache.  score(t): 8 chains (chain c covers dims c, c+8, ..., fused), (c + c+4) per lane, (l0+l1)+(l2+l3), times
 // 1/sqrt(128); maximum over all keys; denominator and the 128 output sums serial over t.
-// K, then V of the cached positions run through one ring of 64-position tiles, filled by 16-byte copies that start before the dependency
-// wait (rows 136 floats apart: the score threads - (key, two chains) - read 8 bytes each from different banks; a bulk copy per position
-// costs 53 cycles each, 3400 a tile).
+// K, then V of the cached positions run through one ring of 64-position tiles that starts before the dependency wait: four tensor copies
+// per tile, 32 dims each, their 16-byte chunks swizzled over the banks (chunk ^ position & 7) - 16-byte copies by the threads took 1000
+// cycles of the load/store pipe per tile, a bulk copy per position 3400.
+// Score threads are (key, two chains), keys of a phase two apart; p.V threads are the dims.
 // Bound: at 100 positions the prologue's and softmax's latencies; then the chains over the keys (4 cycles each).
-constexpr int QA_TILE = 64, QA_STRIDE = 136, QA_SLOTS = 5, QA_THREADS = 256;
-constexpr size_t QA_SMEM = (size_t)QA_SLOTS * QA_TILE * QA_STRIDE * 4 + (size_t)BRRR_MAXSEQ * 4;
+constexpr int QA_TILE = 64, QA_SLOTS = 5, QA_THREADS = 256;
+constexpr uint32_t QA_BOX = QA_TILE * 128, QA_TILE_BYTES = 4 * QA_BOX;
+constexpr size_t QA_SMEM = (size_t)QA_SLOTS * QA_TILE_BYTES + (size_t)BRRR_MAXSEQ * 4 + 1024;
 
-struct QAttnArgs {
+struct alignas(64) QAttnArgs {
+    CUtensorMap km, vm;          // the caches as [nkv * MAXSEQ][128], boxes of 64 positions x 32 dims
     const float *q, *k, *v, *q_norm, *k_norm, *rope;
     float eps;
     float *kc, *vc;              // [nkv][MAXSEQ][128]
@@ -324,105 +330,129 @@ struct QAttnArgs {
     float *out;                  // [nh][128]
 };
 
-__device__ __forceinline__ void qa_cp16(uint32_t dst, const void *src) { asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(dst), "l"(src) : "memory"); }
-
+__device__ __forceinline__ void qa_box(uint32_t dst, const CUtensorMap *map, int x, int row, uint64_t *bar) {
+    asm volatile("cp.async.bulk.tensor.2d.shared::cluster.global.tile.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3}], [%4];" ::"r"(dst), "l"(map), "r"(x), "r"(row),
+                 "r"(smem_u32(bar))
+                 : "memory");
+}
+__device__ __forceinline__ float2 qa_lds2(uint32_t a) {
+    float2 r;
+    asm volatile("ld.shared.v2.f32 {%0, %1}, [%2];" : "=f"(r.x), "=f"(r.y) : "r"(a));
+    return r;
+}
+__device__ __forceinline__ float qa_lds(uint32_t a) {
+    float r;
+    asm volatile("ld.shared.f32 %0, [%1];" : "=f"(r) : "r"(a));
+    return r;
+}
 // two chains of a key, then the others' in the four threads of a key: (c + c+4), (l0 + l1) + (l2 + l3)
-__device__ __forceinline__ float qa_score(const float *kp, const float2 (&q)[16]) {
-    float s0 = 0.0f, s1 = 0.0f;
-#pragma unroll
-    for (int i = 0; i < 16; i++) {
-        const float2 k = *reinterpret_cast<const float2 *>(kp + 8 * i);
-        s0 = __fmaf_rn(k.x, q[i].x, s0); s1 = __fmaf_rn(k.y, q[i].y, s1);
-    }
+__device__ __forceinline__ float qa_combine(float s0, float s1) {
     s0 = __fadd_rn(s0, __shfl_xor_sync(0xffffffffu, s0, 2));
     s1 = __fadd_rn(s1, __shfl_xor_sync(0xffffffffu, s1, 2));
     const float l = __fadd_rn(s0, s1);
     return __fadd_rn(l, __shfl_xor_sync(0xffffffffu, l, 1));
 }
 
-__global__ void __launch_bounds__(QA_THREADS) qw_attn_kernel(QAttnArgs a) {
-    extern __shared__ __align__(16) float asm_[];
-    float *ring = asm_, *sc = asm_ + QA_SLOTS * QA_TILE * QA_STRIDE;
+__global__ void __launch_bounds__(QA_THREADS) qw_attn_kernel(const __grid_constant__ QAttnArgs a) {
+    extern __shared__ __align__(16) unsigned char asm_[];
+    unsigned char *ring = asm_ + ((1024u - (smem_u32(asm_) & 1023u)) & 1023u);          // swizzled copies want 1024-byte alignment
+    float *sc = reinterpret_cast<float *>(ring + QA_SLOTS * QA_TILE_BYTES);
     __shared__ __align__(16) float raw[2][QW_HD], nv[2][QW_HD], qs[QW_HD], ks[QW_HD], vs[QW_HD];
     __shared__ float red[8], inv_sh[2], den_sh;
+    __shared__ __align__(8) uint64_t full[QA_SLOTS];
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, u = tid & (QW_HD - 1), qk = tid >> 7;
     const int h = blockIdx.x, group = a.nh / a.nkv, kvh = h / group;
     const int pos = (int)a.state->pos, n = pos + 1, nt = (pos + QA_TILE - 1) / QA_TILE;        // the position is an input of the step
-    float *kbase = a.kc + (size_t)kvh * BRRR_MAXSEQ * QW_HD, *vbase = a.vc + (size_t)kvh * BRRR_MAXSEQ * QW_HD;
     const uint32_t ring0 = smem_u32(ring);
-    auto issue = [&](int t) {            // tile t of 2 nt: K, then V; one group of copies, empty past the end
-        if (t < 2 * nt) {
-            const int k0 = (t < nt ? t : t - nt) * QA_TILE, cnt = min(QA_TILE, pos - k0);
-            const float *src = (t < nt ? kbase : vbase) + (size_t)k0 * QW_HD;
-            const uint32_t dst = ring0 + (t % QA_SLOTS) * QA_TILE * QA_STRIDE * 4;
+    Waiter waiter(&a.state->err);
+    auto issue = [&](int t) {            // one thread: tile t of 2 nt, K then V (positions past the last cached one come along unused)
+        const int slot = t % QA_SLOTS, row = kvh * BRRR_MAXSEQ + (t < nt ? t : t - nt) * QA_TILE;
+        mbar_expect_tx(&full[slot], QA_TILE_BYTES);
 #pragma unroll
-            for (int i = 0; i < QA_TILE * 32 / QA_THREADS; i++) {
-                const int k = (tid >> 5) + i * 8;
-                if (k < cnt) qa_cp16(dst + (k * QA_STRIDE + lane * 4) * 4, src + (size_t)k * QW_HD + lane * 4);
-            }
-        }
-        asm volatile("cp.async.commit_group;" ::: "memory");
+        for (int b = 0; b < 4; b++) qa_box(ring0 + slot * QA_TILE_BYTES + b * QA_BOX, t < nt ? &a.km : &a.vm, b * 32, row, &full[slot]);
     };
-    auto bar = [&]() { __syncthreads(); };
-    auto landed = [&]() { asm volatile("cp.async.wait_group %0;" ::"n"(QA_SLOTS - 1) : "memory"); };
-#pragma unroll 1
-    for (int t = 0; t < QA_SLOTS; t++) issue(t);      // positions before this one: written in earlier steps
+    if (tid == 0) {
+        for (int i = 0; i < QA_SLOTS; i++) mbar_init(&full[i], 1);
+        mbar_fence_init();
+        for (int t = 0; t < min(QA_SLOTS, 2 * nt); t++) issue(t);      // written in earlier steps
+    }
     const float wv = (qk ? a.k_norm : a.q_norm)[u];
     const float2 cs = reinterpret_cast<const float2 *>(a.rope)[(size_t)pos * (QW_HD / 2) + (tid & 63)];
     pdl_wait_cta();
     pdl_trigger();
     raw[qk][u] = qk ? a.k[kvh * QW_HD + u] : a.q[h * QW_HD + u];
     if (!qk) vs[u] = a.v[kvh * QW_HD + u];
-    bar();
-    if (u == 0) inv_sh[qk] = __fdiv_rn(1.0f, __fsqrt_rn(__fadd_rn(__fdiv_rn(chain_squares(raw[qk], QW_HD), (float)QW_HD), a.eps)));
-    bar();
+    waiter.poison_if_failed();
+    __syncthreads();
+    if (u == 0) inv_sh[qk] = rms_inv(chain_squares(raw[qk], QW_HD), QW_HD, a.eps);
+    __syncthreads();
     nv[qk][u] = __fmul_rn(__fmul_rn(raw[qk][u], inv_sh[qk]), wv);
-    bar();
+    __syncthreads();
     {
         const int c = u & 63;
         const float aa = nv[qk][c], bb = nv[qk][64 + c];
         const float o = u < 64 ? __fsub_rn(__fmul_rn(aa, cs.x), __fmul_rn(bb, cs.y)) : __fadd_rn(__fmul_rn(bb, cs.x), __fmul_rn(aa, cs.y));
         (qk ? ks : qs)[u] = o;
         if (h % group == 0) {
-            if (qk) kbase[(size_t)pos * QW_HD + u] = o;
-            else vbase[(size_t)pos * QW_HD + u] = vs[u];
+            const size_t at = ((size_t)kvh * BRRR_MAXSEQ + pos) * QW_HD + u;
+            if (qk) a.kc[at] = o;
+            else a.vc[at] = vs[u];
         }
     }
-    bar();
+    __syncthreads();
     // ---- scores: thread = (key, two chains)
     const float scale = __fdiv_rn(1.0f, __fsqrt_rn((float)QW_HD));
-    const int c2 = (lane & 3) * 2, key = tid >> 2;
+    const int c2 = (lane & 3) * 2, k8 = lane >> 2, key = warp * 8 + ((k8 & 3) * 2 | k8 >> 2);        // keys 0 2 4 6 1 3 5 7 of eight
     float2 qr[16];
 #pragma unroll
     for (int i = 0; i < 16; i++) qr[i] = *reinterpret_cast<const float2 *>(qs + 8 * i + c2);
-    float mx = __fmul_rn(qa_score(ks + c2, qr), scale);                       // the position's own score, in every thread
+    float s0 = 0.0f, s1 = 0.0f;
+#pragma unroll
+    for (int i = 0; i < 16; i++) {
+        const float2 k = *reinterpret_cast<const float2 *>(ks + 8 * i + c2);
+        s0 = __fmaf_rn(k.x, qr[i].x, s0); s1 = __fmaf_rn(k.y, qr[i].y, s1);
+    }
+    float mx = __fmul_rn(qa_combine(s0, s1), scale);  // the position's own score, in every thread
     if (tid == 0) sc[pos] = mx;
+    // chunk 2 (i & 3) + (c2 >> 2) of the key's row in box i >> 2
+    uint32_t off[4];
+#pragma unroll
+    for (int i = 0; i < 4; i++) off[i] = (uint32_t)(key * 128 + (((2 * i + (c2 >> 2)) ^ (key & 7)) << 4) + (c2 & 2) * 4);
 #pragma unroll 1
     for (int t = 0; t < nt; t++) {
-        landed();
-        bar();
-        const float s = __fmul_rn(qa_score(ring + ((t % QA_SLOTS) * QA_TILE + key) * QA_STRIDE + c2, qr), scale);
+        const int slot = t % QA_SLOTS;
+        const uint32_t base = ring0 + slot * QA_TILE_BYTES;
+        waiter.wait(&full[slot], (uint32_t)(t / QA_SLOTS) & 1u);
+        s0 = s1 = 0.0f;
+#pragma unroll
+        for (int i = 0; i < 16; i++) {
+            const float2 k = qa_lds2(base + (i >> 2) * QA_BOX + off[i & 3]);
+            s0 = __fmaf_rn(k.x, qr[i].x, s0); s1 = __fmaf_rn(k.y, qr[i].y, s1);
+        }
+        const float s = __fmul_rn(qa_combine(s0, s1), scale);
         if (t * QA_TILE + key < pos) {
             mx = fmaxf(mx, s);
             if (!(lane & 3)) sc[t * QA_TILE + key] = s;
         }
-        bar();
-        issue(t + QA_SLOTS);
+        if (t + QA_SLOTS < 2 * nt) {
+            __syncthreads();
+            if (tid == 0) { fence_proxy_async(); issue(t + QA_SLOTS); }
+        }
     }
     mx = warp_max(mx);
     if (lane == 0) red[warp] = mx;
-    bar();
+    __syncthreads();
     mx = red[0];
 #pragma unroll
     for (int w = 1; w < 8; w++) mx = fmaxf(mx, red[w]);
 #pragma unroll 1
     for (int t = tid; t < ((n + 3) & ~3); t += QA_THREADS) sc[t] = t < n ? brrr_expf_dev(__fsub_rn(sc[t], mx)) : 0.0f;      // +0 past the end changes no sum
-    bar();
+    __syncthreads();
     float acc = 0.0f;
     if (tid == 128) {
         float den = 0.0f;
         float4 p = *reinterpret_cast<const float4 *>(sc);
-#pragma unroll 2
+#pragma unroll 4
         for (int t = 4; t < n + 4; t += 4) {
             const float4 c = p;
             p = *reinterpret_cast<const float4 *>(sc + (t < n ? t : 0));
@@ -430,31 +460,37 @@ __global__ void __launch_bounds__(QA_THREADS) qw_attn_kernel(QAttnArgs a) {
         }
         den_sh = den;
     }
+    // chunk lane / 4 of the position's row in box `warp`
+    uint32_t voff[8];
+#pragma unroll
+    for (int i = 0; i < 8; i++) voff[i] = (uint32_t)((warp & 3) * QA_BOX + i * 128 + (((lane >> 2) ^ i) << 4) + (lane & 3) * 4);
 #pragma unroll 1
     for (int t = 0; t < nt; t++) {
-        landed();
-        bar();
+        const int slot = (nt + t) % QA_SLOTS;
         if (tid < QW_HD) {
+            waiter.wait(&full[slot], (uint32_t)((nt + t) / QA_SLOTS) & 1u);
             // whole sixteens, the next one's values on the way while this one's are added up; then the rest
             const int cnt = min(QA_TILE, pos - t * QA_TILE);
-            const float *vt = ring + ((nt + t) % QA_SLOTS) * QA_TILE * QA_STRIDE + tid, *pt = sc + t * QA_TILE;
+            const uint32_t vt = ring0 + slot * QA_TILE_BYTES;
+            const float *pt = sc + t * QA_TILE;
             float v[16];
             float4 p[4];
 #pragma unroll
-            for (int i = 0; i < 16; i++) v[i] = vt[i * QA_STRIDE];
+            for (int i = 0; i < 16; i++) v[i] = qa_lds(vt + voff[i & 7] + (i >> 3) * 1024);
 #pragma unroll
             for (int i = 0; i < 4; i++) p[i] = *reinterpret_cast<const float4 *>(pt + 4 * i);
             int k = 0;
 #pragma unroll 1
             for (; k + 16 <= cnt; k += 16) {
-                const float *w = vt + ((k + 16) & (QA_TILE - 1)) * QA_STRIDE;
-                const float *o = pt + ((k + 16) & (QA_TILE - 1));
+                const int kn = (k + 16) & (QA_TILE - 1);
+                const uint32_t w = vt + kn * 128;
+                const float *o = pt + kn;
 #pragma unroll
                 for (int i = 0; i < 4; i++) {
-                    acc = __fmaf_rn(v[4 * i], p[i].x, acc); v[4 * i] = w[4 * i * QA_STRIDE];
-                    acc = __fmaf_rn(v[4 * i + 1], p[i].y, acc); v[4 * i + 1] = w[(4 * i + 1) * QA_STRIDE];
-                    acc = __fmaf_rn(v[4 * i + 2], p[i].z, acc); v[4 * i + 2] = w[(4 * i + 2) * QA_STRIDE];
-                    acc = __fmaf_rn(v[4 * i + 3], p[i].w, acc); v[4 * i + 3] = w[(4 * i + 3) * QA_STRIDE];
+                    acc = __fmaf_rn(v[4 * i], p[i].x, acc); v[4 * i] = qa_lds(w + voff[(4 * i) & 7] + (i >> 1) * 1024);
+                    acc = __fmaf_rn(v[4 * i + 1], p[i].y, acc); v[4 * i + 1] = qa_lds(w + voff[(4 * i + 1) & 7] + (i >> 1) * 1024);
+                    acc = __fmaf_rn(v[4 * i + 2], p[i].z, acc); v[4 * i + 2] = qa_lds(w + voff[(4 * i + 2) & 7] + (i >> 1) * 1024);
+                    acc = __fmaf_rn(v[4 * i + 3], p[i].w, acc); v[4 * i + 3] = qa_lds(w + voff[(4 * i + 3) & 7] + (i >> 1) * 1024);
                     p[i] = *reinterpret_cast<const float4 *>(o + 4 * i);
                 }
             }
@@ -466,11 +502,12 @@ __global__ void __launch_bounds__(QA_THREADS) qw_attn_kernel(QAttnArgs a) {
                 if (k + 4 * i + 3 < cnt) acc = __fmaf_rn(v[4 * i + 3], p[i].w, acc);
             }
         }
-        bar();
-        issue(nt + t + QA_SLOTS);
+        if (nt + t + QA_SLOTS < 2 * nt) {
+            __syncthreads();
+            if (tid == 0) { fence_proxy_async(); issue(nt + t + QA_SLOTS); }
+        }
     }
-    asm volatile("cp.async.wait_all;" ::: "memory");
-    bar();
+    __syncthreads();
     if (tid < QW_HD) a.out[h * QW_HD + tid] = __fmul_rn(__fmaf_rn(vs[tid], sc[pos], acc), __fdiv_rn(1.0f, den_sh));
 }
 
@@ -492,7 +529,7 @@ struct QHintArgs {
 
 __global__ void __launch_bounds__(QH_THREADS) qw_hint_kernel(QHintArgs a) {
     extern __shared__ __align__(16) float xf[];
-    __shared__ float part[QW_NT], red[QH_THREADS / 32];
+    __shared__ __align__(16) float part[QW_NT], red[QH_THREADS / 32];
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, e = blockIdx.x, d = a.d, groups = d >> 2;
     const int ntiles = (d + RT_TJ - 1) / RT_TJ;
     const float *wrow = a.Wt + ((size_t)(e >> 5) * ntiles * 32 + (e & 31)) * RT_STRIDE;
@@ -880,12 +917,12 @@ cudaError_t launch_qw_oproj(const KMatDev &wo, const float *act, float *x, DevSt
     return qw_gemv(&wo, &x, 1, act, nullptr, 0.0f, state, pdl, st);
 }
 
-cudaError_t launch_qw_attn(const float *q, const float *k, const float *v, const float *q_norm, const float *k_norm, const float *rope, float eps, float *kc, float *vc,
-                           int nh, int nkv, DevState *state, float *out, bool pdl, cudaStream_t st) {
+cudaError_t launch_qw_attn(const QwCache &c, const float *q, const float *k, const float *v, const float *q_norm, const float *k_norm, const float *rope, float eps, int nh,
+                           int nkv, DevState *state, float *out, bool pdl, cudaStream_t st) {
     static unsigned long long configured = 0;      // one bit per device
     cudaError_t e = smem_optin(qw_attn_kernel, (int)QA_SMEM, configured);
     if (e != cudaSuccess) return e;
-    QAttnArgs a{q, k, v, q_norm, k_norm, rope, eps, kc, vc, nh, nkv, state, out};
+    QAttnArgs a{c.km, c.vm, q, k, v, q_norm, k_norm, rope, eps, c.k, c.v, nh, nkv, state, out};
     return launch_k(qw_attn_kernel, dim3(nh), dim3(QA_THREADS), QA_SMEM, st, pdl, a);
 }
 

@@ -74,7 +74,7 @@ struct RouterArgs {
     float *wts;
     unsigned int *counter;
     DevState *state;
-    uint32_t *signal;        // nullable: sequence number of the published routing (see publish_route)
+    uint32_t *signal;        // nullable: sequence number of the published routing
     unsigned long long *pub;
     // qwen3moe: the norm is the 12-slice one, and the first CTA also leaves the Q8_K image of the
     // normalised token (quants, scales per 256, sums per 16) for the gate/up kernel
@@ -86,51 +86,60 @@ struct RouterArgs {
                              // start of every row at once, and room beside the decode kernels of an SM)
 };
 
-// k rounds of warp arg-max over the logits: the largest value wins, the lower index among equals, which is the order the reference's
-// strict-'>' insertion produces.  Lane l holds experts l * per ..., so among equal keys the lowest lane has the lowest index.  Then the
-// softmax over the selected k in rank order, the exponentials side by side.  Warp 0 only.
-__device__ __forceinline__ void warp_topk(const RouterArgs &a, const float *lg, int lane) {
-    const int per = (a.ne + 31) / 32;            // up to 256 experts
-    uint32_t key[8];
+// The k largest logits, the lower index first among equals, which is the order the reference's strict-'>' insertion produces; then the
+// softmax over them in rank order.  One warp: rounds of a maximum over order-preserving keys (lane l holds experts l * per ..., so among
+// equals the lowest lane has the lowest index).  Lane r ends with the expert and weight of rank r, and publishes them if asked to: words
+// tagged with the sequence number `seq`, each valid by itself, for a consumer that does not wait for this kernel to end (the
+// combine of the speculative step).  Launches that publish are serialised on one stream, so the sequence word has a single writer.
+template <int PER>
+__device__ __forceinline__ void warp_topk_n(const RouterArgs &a, const float *lg, int lane, uint32_t seq) {
+    uint32_t key[PER];
 #pragma unroll
-    for (int i = 0; i < 8; i++) key[i] = i < per && lane * per + i < a.ne ? max(float_orderable(lg[lane * per + i]), 1u) : 0u;
+    for (int i = 0; i < PER; i++) key[i] = lane * PER + i < a.ne ? max(float_orderable(lg[lane * PER + i]), 1u) : 0u;
     float mine = 0.0f;                           // lane r: logit and expert of rank r
     int mine_e = 0;
 #pragma unroll 1
     for (int r = 0; r < a.topk; r++) {
         uint32_t best = key[0];
+#pragma unroll
+        for (int i = 1; i < PER; i++) best = max(best, key[i]);
+        const uint32_t top = __reduce_max_sync(0xffffffffu, best);
+        const int owner = __ffs(__ballot_sync(0xffffffffu, best == top)) - 1;
         int at = 0;
 #pragma unroll
-        for (int i = 1; i < 8; i++) if (key[i] > best) { best = key[i]; at = i; }
-        const uint32_t top = __reduce_max_sync(0xffffffffu, best);
-        const int owner = __ffs(__ballot_sync(0xffffffffu, best == top)) - 1, e = min(__shfl_sync(0xffffffffu, lane * per + at, owner), a.ne - 1);
+        for (int i = PER - 1; i >= 0; i--) if (key[i] == top) at = i;
+        const int e = min(__shfl_sync(0xffffffffu, lane * PER + at, owner), a.ne - 1);
         if (lane == owner) {
 #pragma unroll
-            for (int i = 0; i < 8; i++) if (i == at) key[i] = 0u;
+            for (int i = 0; i < PER; i++) if (i == at) key[i] = 0u;
         }
         if (lane == r) { mine = lg[e]; mine_e = e; }
     }
     const float first = __shfl_sync(0xffffffffu, mine, 0);
     const float ex = lane < a.topk ? brrr_expf_dev(__fsub_rn(mine, first)) : 0.0f;
     float wsum = 0.0f;
+#pragma unroll 4
     for (int i = 0; i < a.topk; i++) wsum = __fadd_rn(wsum, __shfl_sync(0xffffffffu, ex, i));
-    if (lane < a.topk) { a.wts[lane] = __fdiv_rn(ex, wsum); a.top[lane] = mine_e; }
-    __syncwarp();
-}
-
-// Publication for a consumer that does not wait for this kernel to end (the fused fold of the
-// speculative step): sequence-tagged 64-bit copies of the routing this thread has just written.
-// Launches that publish are serialised on one stream, so the sequence word has a single writer.
-__device__ __forceinline__ void publish_route(const RouterArgs &a) {
+    const float w = __fdiv_rn(ex, wsum);
+    if (lane < a.topk) {
 #ifdef BRRR_TEST_HOOKS
-    if (a.state && (a.state->test_hooks & 2u)) return;      // test hook: stay silent, the consumer's bounded wait runs out
+        const bool silent = a.state && (a.state->test_hooks & 2u);      // test hook: the consumer's bounded wait runs out
+#else
+        constexpr bool silent = false;
 #endif
-    const uint32_t seq = __ldcg(a.signal) + 1u;
-    for (int i = 0; i < a.topk; i++) {
-        __stcg(&a.pub[i], ((unsigned long long)seq << 32) | (uint32_t)a.top[i]);
-        __stcg(&a.pub[8 + i], ((unsigned long long)seq << 32) | __float_as_uint(a.wts[i]));
+        if (a.signal && !silent) {
+            __stcg(&a.pub[lane], ((unsigned long long)seq << 32) | (uint32_t)mine_e);
+            __stcg(&a.pub[8 + lane], ((unsigned long long)seq << 32) | __float_as_uint(w));
+        }
+        a.wts[lane] = w;
+        a.top[lane] = mine_e;
+        if (a.signal && !silent && lane == 0) __stcg(a.signal, seq);
     }
-    __stcg(a.signal, seq);
+}
+__device__ __forceinline__ void warp_topk(const RouterArgs &a, const float *lg, int lane, uint32_t seq) {
+    if (a.ne <= 32) warp_topk_n<1>(a, lg, lane, seq);
+    else if (a.ne <= 128) warp_topk_n<4>(a, lg, lane, seq);
+    else warp_topk_n<8>(a, lg, lane, seq);
 }
 
 __global__ void __launch_bounds__(RT_THREADS) ffn_in_kernel(RouterArgs a) {
@@ -171,6 +180,7 @@ __global__ void __launch_bounds__(RT_THREADS) ffn_in_kernel(RouterArgs a) {
     __syncwarp();
     if (tid < min(stages, ntiles)) issue(tid);        // one lane per stage: the copies' address translations overlap
     if (a.norm_w) stage_vec4(a.norm_w, wn, d, tid, RT_THREADS);             // static: fetched before the wait
+    const uint32_t seq = a.signal ? __ldcg(a.signal) + 1u : 0u;             // the launch before on this stream has ended
     const float bias_pre = (warp == 0 && lane < nloc && a.b) ? a.b[e0 + lane] : 0.0f;
     BRRR_STAMP(a.state, 1);
     pdl_wait_cta();      // residual stream complete
@@ -193,7 +203,7 @@ __global__ void __launch_bounds__(RT_THREADS) ffn_in_kernel(RouterArgs a) {
             float tot = 0.0f;
 #pragma unroll
             for (int k = 0; k < QW_NT; k++) tot = __fadd_rn(tot, part[k]);
-            inv = __fdiv_rn(1.0f, __fsqrt_rn(__fadd_rn(__fdiv_rn(tot, (float)d), a.eps)));
+            inv = rms_inv(tot, d, a.eps);
         } else inv = block_rms_inv(xn, d, a.eps, &inv_sh);
         for (int i = tid; i < d; i += RT_THREADS) xn[i] = __fmul_rn(__fmul_rn(xn[i], inv), wn[i]);
         __syncthreads();
@@ -236,11 +246,10 @@ __global__ void __launch_bounds__(RT_THREADS) ffn_in_kernel(RouterArgs a) {
         BRRR_STAMP(a.state, 4);
         if (gridDim.x == 1) {                  // single CTA: top-k straight from shared memory
             __syncwarp();
-            warp_topk(a, lg, lane);
+            warp_topk(a, lg, lane, seq);
         }
         BRRR_STAMP(a.state, 5);
         BRRR_GT_END(a.state, 31);
-        if (gridDim.x == 1 && lane == 0 && a.signal) publish_route(a);      // routing written by this lane
     }
     if (gridDim.x == 1) return;
 
@@ -256,11 +265,8 @@ __global__ void __launch_bounds__(RT_THREADS) ffn_in_kernel(RouterArgs a) {
     __threadfence();
     for (int e = tid; e < a.ne; e += RT_THREADS) lg[e] = __ldcg(a.logits + e);
     __syncthreads();
-    if (warp == 0) warp_topk(a, lg, lane);
-    if (tid == 0) {
-        *a.counter = 0u;
-        if (a.signal) publish_route(a);
-    }
+    if (warp == 0) warp_topk(a, lg, lane, seq);
+    if (tid == 0) *a.counter = 0u;
 }
 
 // ---------------------------------------------------------------- router of token rows (normalised rows in, routing out)
@@ -370,7 +376,7 @@ __global__ void __launch_bounds__(RR_WARPS * 32) router_rows_kernel(RouterArgs a
         RouterArgs b = a;
         b.top = a.top + (t0 + t) * 8;
         b.wts = a.wts + (t0 + t) * 8;
-        warp_topk(b, lg, lane);
+        warp_topk(b, lg, lane, 0u);
     }
 }
 

@@ -43,6 +43,7 @@ struct QLayer {
     KMatDev wq{}, wk{}, wv{}, wo{}, gate{}, up{}, down{};
     KqtMat tq, tk, tv, to, tgate, tup, tdown;      // the same matrices for token rows (has_rows)
     float *kc = nullptr, *vc = nullptr;      // [kv head][position][head_dim]
+    QwCache cache;
 };
 
 struct QSource {
@@ -224,7 +225,7 @@ int qenqueue_step(brrr_qwen *m, bool want, float *trace_dev, int *nlaunch, bool 
         KMatDev qkv[3] = {ly.wq, ly.wk, ly.wv};
         float *qkv_out[3] = {m->q, m->k, m->v};
         CU(launch_qw_qkv(qkv, qkv_out, m->x, ly.attn_norm, c.rms_eps, m->st, pdl, s)); n++;
-        CU(launch_qw_attn(m->q, m->k, m->v, ly.q_norm, ly.k_norm, m->rope, c.rms_eps, ly.kc, ly.vc, nh, nkv, m->st, m->ao, pdl, s)); n++;
+        CU(launch_qw_attn(ly.cache, m->q, m->k, m->v, ly.q_norm, ly.k_norm, m->rope, c.rms_eps, nh, nkv, m->st, m->ao, pdl, s)); n++;
         CU(launch_qw_oproj(ly.wo, m->ao, m->x, m->st, pdl, s)); n++;
         if (spec) {
             CU(cudaEventRecord(m->ev_fork, s));
@@ -393,6 +394,7 @@ int qbuild(brrr_qwen *m, const QSource &src) {
         TRY(qload_k(m, src, il, BRRR_T_DOWN, ne * d, ff, &ly.down));
         TRY(m->alloc(&ly.kc, (size_t)BRRR_MAXSEQ * nkv * hd));
         TRY(m->alloc(&ly.vc, (size_t)BRRR_MAXSEQ * nkv * hd));
+        CU(qw_cache(ly.kc, ly.vc, nkv, &ly.cache));
         CU(cudaMemsetAsync(ly.kc, 0, (size_t)BRRR_MAXSEQ * nkv * hd * 4, m->stream));
         CU(cudaMemsetAsync(ly.vc, 0, (size_t)BRRR_MAXSEQ * nkv * hd * 4, m->stream));
     }
