@@ -303,30 +303,39 @@ __device__ __forceinline__ float kq_term(int nsb, uint32_t row, int sb, const KA
     return __fmul_rn(__fmul_rn(ys, d), (float)a);
 }
 
-// Sum of squares of v[0 .. n) in order by one thread: the next sixteen values are read while sixteen squares are added.  v must be readable
-// for 16 floats.
-__device__ __forceinline__ float chain_squares(const float *v, int n) {
-    float ps = 0.0f, b[16];
-    const int m = n & ~15, last = n > 16 ? n - 16 : 0;
+// Sum of squares of x[lo .. hi) in order by one thread, x 16-byte aligned: whole float4s, what lies outside the range counted as +0 (which
+// changes no sum), the next sixteen values read while sixteen squares are added (5 cycles a value; scalar reads 8).
+__device__ __forceinline__ float chain_squares(const float *x, int lo, int hi) {
+    const float4 *p = reinterpret_cast<const float4 *>(x) + (lo >> 2);
+    const int head = lo & 3, n = hi - (lo & ~3), n4 = (n + 3) >> 2;      // values from the aligned start, float4s
+    float4 b[4];
+    float ps = 0.0f;
 #pragma unroll
-    for (int k = 0; k < 16; k++) b[k] = v[k];
+    for (int k = 0; k < 4; k++) b[k] = p[min(k, n4 - 1)];
+    if (head > 0) b[0].x = 0.0f;
+    if (head > 1) b[0].y = 0.0f;
+    if (head > 2) b[0].z = 0.0f;
+    int i = 0;                               // float4s that b starts at
 #pragma unroll 2
-    for (int i = 16; i <= m; i += 16) {
-        float p[16];
+    for (; i + 4 < n4; i += 4) {
+        float s[16];
 #pragma unroll
-        for (int k = 0; k < 16; k++) p[k] = __fmul_rn(b[k], b[k]);
-        const float *w = v + min(i, last);                   // after the last whole sixteen: the end, of which the tail picks its part
+        for (int k = 0; k < 4; k++) {
+            s[4 * k] = __fmul_rn(b[k].x, b[k].x); s[4 * k + 1] = __fmul_rn(b[k].y, b[k].y);
+            s[4 * k + 2] = __fmul_rn(b[k].z, b[k].z); s[4 * k + 3] = __fmul_rn(b[k].w, b[k].w);
+        }
 #pragma unroll
-        for (int k = 0; k < 16; k++) b[k] = w[k];
+        for (int k = 0; k < 4; k++) b[k] = p[min(i + 4 + k, n4 - 1)];
 #pragma unroll
-        for (int k = 0; k < 16; k++) ps = __fadd_rn(ps, p[k]);
+        for (int k = 0; k < 16; k++) ps = __fadd_rn(ps, s[k]);
     }
-    // tail: the last n - m values, in b from index 16 - (n - m) on (n < 16: from 0 on)
-    const int from = m ? 16 - (n - m) : 0;
 #pragma unroll
-    for (int k = 0; k < 16; k++) {
-        const float t = __fmul_rn(b[k], b[k]);
-        if (m ? k >= from : k < n) ps = __fadd_rn(ps, t);
+    for (int k = 0; k < 4; k++) {
+        const int at = (i + k) * 4;
+        if (at < n) ps = __fadd_rn(ps, __fmul_rn(b[k].x, b[k].x));
+        if (at + 1 < n) ps = __fadd_rn(ps, __fmul_rn(b[k].y, b[k].y));
+        if (at + 2 < n) ps = __fadd_rn(ps, __fmul_rn(b[k].z, b[k].z));
+        if (at + 3 < n) ps = __fadd_rn(ps, __fmul_rn(b[k].w, b[k].w));
     }
     return ps;
 }

@@ -122,7 +122,7 @@ __device__ __forceinline__ float qw_norm_inv(const float *xf, int d, float eps, 
     if (tid < QW_NT) {
         int lo, hi;
         qw_slice(tid, d, lo, hi);
-        part[tid] = chain_squares(xf + lo, hi - lo);
+        part[tid] = chain_squares(xf, lo, hi);
     }
     __syncthreads();
     const float4 p0 = reinterpret_cast<const float4 *>(part)[0], p1 = reinterpret_cast<const float4 *>(part)[1], p2 = reinterpret_cast<const float4 *>(part)[2];
@@ -384,7 +384,7 @@ __global__ void __launch_bounds__(QA_THREADS) qw_attn_kernel(const __grid_consta
     if (!qk) vs[u] = a.v[kvh * QW_HD + u];
     waiter.poison_if_failed();
     __syncthreads();
-    if (u == 0) inv_sh[qk] = rms_inv(chain_squares(raw[qk], QW_HD), QW_HD, a.eps);
+    if (u == 0) inv_sh[qk] = rms_inv(chain_squares(raw[qk], 0, QW_HD), QW_HD, a.eps);
     __syncthreads();
     nv[qk][u] = __fmul_rn(__fmul_rn(raw[qk][u], inv_sh[qk]), wv);
     __syncthreads();
@@ -941,7 +941,8 @@ cudaError_t launch_qw_gate_up(const KMatDev &gate, const KMatDev &up, const floa
     const size_t row = (size_t)a.stride_g + a.stride_u + nsb * 8;
     a.per_cta = qw_rows_per_cta(topk * ff, row);
     if (a.per_cta > 256) return cudaErrorInvalidValue;
-    const size_t smem = a.per_cta * row;
+    // at least 112 KB: no room beside it for the router's CTAs (117 KB), whose chains then have an SM of their own - 5.4 us instead of 8.8
+    const size_t smem = a.per_cta * row > 112 * 1024 ? a.per_cta * row : 112 * 1024;
     return passes == 1 ? qw_gate_up_launch<1>(a, smem, pdl, st) : qw_gate_up_launch<2>(a, smem, pdl, st);
 }
 

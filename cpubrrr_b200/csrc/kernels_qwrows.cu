@@ -72,7 +72,7 @@ __global__ void __launch_bounds__(256) qr_norm_kernel(QrNormArgs a) {
     if (tid < QW_NT) {
         int lo, hi;
         qw_slice(tid, d, lo, hi);
-        part[tid] = chain_squares(xs_sh + lo, hi - lo);
+        part[tid] = chain_squares(xs_sh, lo, hi);
     }
     __syncthreads();
     float tot = 0.0f;

@@ -40,7 +40,10 @@ void launch_router_pack(const float *W, int ne, int d, float *out, cudaStream_t 
 
 // acc += w[j] * x[j] for j = 0..len-1 (len % 64 == 0), strictly in order, product and sum rounded separately.  The operands of the next
 // sixteen products are read while sixteen sums are formed, so that only the adds sit on the dependent path (4 cycles each).
+// LEN: known at compile time, or 0 (len); known, the loop takes 5 cycles per element, else 7.
+template <int LEN>
 __device__ __forceinline__ float chain_span(const float *__restrict__ w, const float *__restrict__ x, int len, float acc) {
+    if (LEN) len = LEN;
     float4 a[4], b[4];
 #pragma unroll
     for (int k = 0; k < 4; k++) { a[k] = *reinterpret_cast<const float4 *>(w + 4 * k); b[k] = *reinterpret_cast<const float4 *>(x + 4 * k); }
@@ -82,8 +85,8 @@ struct RouterArgs {
     int8_t *q8k_q;
     float *q8k_s;
     int32_t *q8k_b16;
-    int epc, stages;         // experts per CTA, tiles in flight: 32 and 5; many experts: 8 and all (a lane per expert, nothing to refill, the
-                             // start of every row at once, and room beside the decode kernels of an SM)
+    int epc, stages;         // experts per CTA, tiles in flight: 32 and 5; many experts: 16 and 6, a CTA that fits
+                             // beside one waiting decode kernel of an SM but not beside gate/up (whose sixteen warps would slow the chain)
 };
 
 // The k largest logits, the lower index first among equals, which is the order the reference's strict-'>' insertion produces; then the
@@ -197,7 +200,7 @@ __global__ void __launch_bounds__(RT_THREADS) ffn_in_kernel(RouterArgs a) {
             if (tid < QW_NT) {
                 int lo, hi;
                 qw_slice(tid, d, lo, hi);
-                part[tid] = chain_squares(xn + lo, hi - lo);
+                part[tid] = chain_squares(xn, lo, hi);
             }
             __syncthreads();
             float tot = 0.0f;
@@ -229,15 +232,18 @@ __global__ void __launch_bounds__(RT_THREADS) ffn_in_kernel(RouterArgs a) {
     }
     if (warp == 0) {
         float acc = bias_pre;
+        int slot = 0;
+        uint32_t parity = 0;
         for (int t = 0; t < ntiles; t++) {
             if (t < 12) BRRR_STAMP(a.state, 8 + t);
-            const int slot = t % stages, j0 = t * RT_TJ, len = min(RT_TJ, d - j0);
-            waiter.wait(&bars[slot], (uint32_t)(t / stages) & 1u);
+            const int j0 = t * RT_TJ, len = min(RT_TJ, d - j0);
+            waiter.wait(&bars[slot], parity);
             const float *row = tiles + (size_t)slot * tile_floats + min(lane, epc - 1) * RT_STRIDE;
             const float *xr = xn + j0;
-            acc = chain_span(row, xr, len, acc);
+            acc = len == RT_TJ ? chain_span<RT_TJ>(row, xr, len, acc) : chain_span<0>(row, xr, len, acc);
             __syncwarp();                      // all lanes are done reading this slot
             if (lane == 0 && t + stages < ntiles) mbar_arrive(&empty[slot]);
+            if (++slot == stages) { slot = 0; parity ^= 1u; }
         }
         if (lane < nloc) {
             if (gridDim.x == 1) lg[lane] = acc;
@@ -276,9 +282,46 @@ __global__ void __launch_bounds__(RT_THREADS) ffn_in_kernel(RouterArgs a) {
 // per four elements.  With several groups the last CTA of a token block runs the top-k of its tokens.
 constexpr int RR_WARPS = 4, RR_STAGES = 3;
 
+// acc[k] += w[j] * x[k][j] for j = 0 .. len - 1 in order (len % 64 == 0; LEN: known at compile time, or 0)
+template <int TPW, int LEN>
+__device__ __forceinline__ void rows_span(const float *w, const float *x, int len, float (&acc)[TPW]) {
+    constexpr int STEP = TPW == 4 ? 8 : 16;
+    if (LEN) len = LEN;
+    // STEP elements of the row and of every token are in registers while the STEP before them are added up (len % 64 == 0)
+    float4 wv[STEP / 4], xv[TPW][STEP / 4];
+#pragma unroll
+    for (int q = 0; q < STEP / 4; q++) {
+        wv[q] = *reinterpret_cast<const float4 *>(w + 4 * q);
+#pragma unroll
+        for (int k = 0; k < TPW; k++) xv[k][q] = *reinterpret_cast<const float4 *>(x + k * RT_TJ + 4 * q);
+    }
+#pragma unroll 2
+    for (int j = 0; j < len; j += STEP) {
+        float p[TPW][STEP];
+#pragma unroll
+        for (int k = 0; k < TPW; k++)
+#pragma unroll
+            for (int q = 0; q < STEP / 4; q++) {
+                p[k][4 * q] = __fmul_rn(wv[q].x, xv[k][q].x); p[k][4 * q + 1] = __fmul_rn(wv[q].y, xv[k][q].y);
+                p[k][4 * q + 2] = __fmul_rn(wv[q].z, xv[k][q].z); p[k][4 * q + 3] = __fmul_rn(wv[q].w, xv[k][q].w);
+            }
+        const int jn = j + STEP < len ? j + STEP : 0;         // past the end: the first step again, unused
+#pragma unroll
+        for (int q = 0; q < STEP / 4; q++) {
+            wv[q] = *reinterpret_cast<const float4 *>(w + jn + 4 * q);
+#pragma unroll
+            for (int k = 0; k < TPW; k++) xv[k][q] = *reinterpret_cast<const float4 *>(x + k * RT_TJ + jn + 4 * q);
+        }
+#pragma unroll
+        for (int i = 0; i < STEP; i++)
+#pragma unroll
+            for (int k = 0; k < TPW; k++) acc[k] = __fadd_rn(acc[k], p[k][i]);
+    }
+}
+
 template <int TPW>
 __global__ void __launch_bounds__(RR_WARPS * 32) router_rows_kernel(RouterArgs a, int ntok) {
-    constexpr int TT = RR_WARPS * TPW, STEP = TPW == 4 ? 8 : 16;
+    constexpr int TT = RR_WARPS * TPW;
     constexpr size_t STAGE = (size_t)(RT_TILE_FLOATS + TT * RT_TJ) * 4;
     extern __shared__ __align__(128) unsigned char smraw[];
     __shared__ __align__(8) uint64_t full[RR_STAGES];
@@ -313,41 +356,16 @@ __global__ void __launch_bounds__(RR_WARPS * 32) router_rows_kernel(RouterArgs a
     float acc[TPW];
 #pragma unroll
     for (int k = 0; k < TPW; k++) acc[k] = (a.b && e0 + lane < a.ne) ? a.b[e0 + lane] : 0.0f;
+    int slot = 0;
+    uint32_t parity = 0;
     for (int t = 0; t < ntiles; t++) {
-        const unsigned char *st = smraw + (size_t)(t % RR_STAGES) * STAGE;
-        waiter.wait(&full[t % RR_STAGES], (uint32_t)(t / RR_STAGES) & 1u);
+        const unsigned char *st = smraw + (size_t)slot * STAGE;
+        waiter.wait(&full[slot], parity);
+        if (++slot == RR_STAGES) { slot = 0; parity ^= 1u; }
         const float *w = reinterpret_cast<const float *>(st) + lane * RT_STRIDE, *x = reinterpret_cast<const float *>(st) + RT_TILE_FLOATS + warp * TPW * RT_TJ;
         const int len = min(RT_TJ, d - t * RT_TJ);
-        // STEP elements of the row and of every token are in registers while the STEP before them are added up (len % 64 == 0)
-        float4 wv[STEP / 4], xv[TPW][STEP / 4];
-#pragma unroll
-        for (int q = 0; q < STEP / 4; q++) {
-            wv[q] = *reinterpret_cast<const float4 *>(w + 4 * q);
-#pragma unroll
-            for (int k = 0; k < TPW; k++) xv[k][q] = *reinterpret_cast<const float4 *>(x + k * RT_TJ + 4 * q);
-        }
-#pragma unroll 2
-        for (int j = 0; j < len; j += STEP) {
-            float p[TPW][STEP];
-#pragma unroll
-            for (int k = 0; k < TPW; k++)
-#pragma unroll
-                for (int q = 0; q < STEP / 4; q++) {
-                    p[k][4 * q] = __fmul_rn(wv[q].x, xv[k][q].x); p[k][4 * q + 1] = __fmul_rn(wv[q].y, xv[k][q].y);
-                    p[k][4 * q + 2] = __fmul_rn(wv[q].z, xv[k][q].z); p[k][4 * q + 3] = __fmul_rn(wv[q].w, xv[k][q].w);
-                }
-            const int jn = j + STEP < len ? j + STEP : 0;         // past the end: the first step again, unused
-#pragma unroll
-            for (int q = 0; q < STEP / 4; q++) {
-                wv[q] = *reinterpret_cast<const float4 *>(w + jn + 4 * q);
-#pragma unroll
-                for (int k = 0; k < TPW; k++) xv[k][q] = *reinterpret_cast<const float4 *>(x + k * RT_TJ + jn + 4 * q);
-            }
-#pragma unroll
-            for (int i = 0; i < STEP; i++)
-#pragma unroll
-                for (int k = 0; k < TPW; k++) acc[k] = __fadd_rn(acc[k], p[k][i]);
-        }
+        if (len == RT_TJ) rows_span<TPW, RT_TJ>(w, x, len, acc);
+        else rows_span<TPW, 0>(w, x, len, acc);
         __syncthreads();                      // the stage is free
         if (warp == 0 && t + RR_STAGES < ntiles) { fence_proxy_async(); issue(t + RR_STAGES, true, true); }
     }
@@ -390,25 +408,13 @@ static cudaError_t router_rows_launch(const RouterArgs &a, int ntok, bool pdl, c
     return launch_k(router_rows_kernel<TPW>, dim3((a.ne + 31) / 32, (ntok + TT - 1) / TT), dim3(RR_WARPS * 32), smem, st, pdl, a, ntok);
 }
 
-cudaError_t launch_router_rows(const float *xn, int d, const float *Wt, const float *b, int ne, int topk, int ntok, float *logits, int32_t *top, float *wts,
-                               unsigned int *counter, DevState *state, bool pdl, cudaStream_t st) {
-    if (d % 64 || ne > 256 || topk > 8 || ntok < 1) return cudaErrorInvalidValue;
-    RouterArgs a{};
-    a.x_in = xn; a.d = d; a.Wt = Wt; a.b = b; a.ne = ne; a.topk = topk; a.logits = logits; a.top = top; a.wts = wts; a.counter = counter; a.state = state;
-    // few tokens per warp are fast while every CTA finds an SM of its own (a CTA of four warps leaves its SM's schedulers half idle)
-    const int groups = (ne + 31) / 32;
-    if (groups * ((ntok + 3) / 4) <= 148) return router_rows_launch<1>(a, ntok, pdl, st);
-    if (groups * ((ntok + 7) / 8) <= 148) return router_rows_launch<2>(a, ntok, pdl, st);
-    return router_rows_launch<4>(a, ntok, pdl, st);
-}
-
 size_t router_packed_floats(int ne, int d) { return (size_t)((ne + 31) / 32) * ((d + RT_TJ - 1) / RT_TJ) * RT_TILE_FLOATS; }
 
 cudaError_t launch_ffn_in(const float *x_in, const float *norm_w, float eps, int d, const float *Wt, const float *b, int ne, int topk,
                           float *logits, int32_t *top, float *wts, unsigned int *counter, DevState *state, bool pdl, cudaStream_t st, int ntok,
                           uint32_t *signal, int qwen_norm, int8_t *q8k_q, float *q8k_s, int32_t *q8k_b16) {
     RouterArgs a{x_in, norm_w, eps, d, Wt, b, ne, topk, logits, top, wts, counter, state, signal, (signal && state) ? state->route_pub : nullptr,
-                 qwen_norm, q8k_q, q8k_s, q8k_b16, ne > 32 ? 8 : 32, ne > 32 ? (d + RT_TJ - 1) / RT_TJ : RT_STAGES};
+                 qwen_norm, q8k_q, q8k_s, q8k_b16, ne > 32 ? 16 : 32, ne > 32 ? 6 : RT_STAGES};
     if (signal && !state) return cudaErrorInvalidValue;
     size_t smem = (size_t)a.epc * RT_STRIDE * 4 * a.stages + (size_t)d * 8 + (size_t)((ne + 3) & ~3) * 4 + a.stages * 16;
     static unsigned long long configured = 0;      // one bit per device
@@ -417,6 +423,20 @@ cudaError_t launch_ffn_in(const float *x_in, const float *norm_w, float eps, int
         if (e != cudaSuccess) return e;
     }
     return launch_k(ffn_in_kernel, dim3((ne + a.epc - 1) / a.epc, ntok), dim3(RT_THREADS), smem, st, pdl, a);
+}
+
+cudaError_t launch_router_rows(const float *xn, int d, const float *Wt, const float *b, int ne, int topk, int ntok, float *logits, int32_t *top, float *wts,
+                               unsigned int *counter, DevState *state, bool pdl, cudaStream_t st) {
+    if (d % 64 || ne > 256 || topk > 8 || ntok < 1) return cudaErrorInvalidValue;
+    RouterArgs a{};
+    a.x_in = xn; a.d = d; a.Wt = Wt; a.b = b; a.ne = ne; a.topk = topk; a.logits = logits; a.top = top; a.wts = wts; a.counter = counter; a.state = state;
+    // a CTA per token (and sixteen experts) while each finds an SM of its own: its chain is alone there (16 against 18.5 us at 9 rows of 2880)
+    if (ntok * ((ne + (ne > 32 ? 15 : 31)) / (ne > 32 ? 16 : 32)) <= 148) return launch_ffn_in(xn, nullptr, 0.0f, d, Wt, b, ne, topk, logits, top, wts, counter, state, pdl, st, ntok);
+    // few tokens per warp are fast while every CTA finds an SM of its own (a CTA of four warps leaves its SM's schedulers half idle)
+    const int groups = (ne + 31) / 32;
+    if (groups * ((ntok + 3) / 4) <= 148) return router_rows_launch<1>(a, ntok, pdl, st);
+    if (groups * ((ntok + 7) / 8) <= 148) return router_rows_launch<2>(a, ntok, pdl, st);
+    return router_rows_launch<4>(a, ntok, pdl, st);
 }
 
 // ---------------------------------------------------------------- routing hint (speculation)

@@ -1253,7 +1253,7 @@ static int moe_tile_enqueue(brrr_model *m, int il, const float *d_xn, int ntok, 
     const int d = c.n_embd, topk = c.n_expert_used, ne = c.n_expert;
     Layer &ly = m->L[il];
     cudaStream_t s = m->stream;
-    CUL(launch_ffn_in(d_xn, nullptr, c.rms_eps, d, ly.ginp, ly.ginp_b, ne, topk, m->tl_logits, m->tl_top, m->tl_wts, m->tl_counter, m->st, pdl, s, ntok));
+    CUL(launch_router_rows(d_xn, d, ly.ginp, ly.ginp_b, ne, topk, ntok, m->tl_logits, m->tl_top, m->tl_wts, m->tl_counter, m->st, pdl, s));
     CUL(launch_tile_route(m->tl_top, ntok, topk, ne, m->tl_cnt, m->tl_list, pdl, s));
     CUL(launch_mx_tile_glu(ly.gate, ly.up, ne, d, m->tl_cnt, m->tl_list, ntok, topk, m->tl_eimg, m->tl_es, ly.gate_b, ly.up_b, m->tl_himg, m->tl_hs, m->st, pdl, s));
     CUL(launch_mx_tile_down(ly.down, ne, d, m->tl_cnt, m->tl_list, ntok, topk, m->tl_himg, m->tl_hs, ly.down_b, m->tl_part, m->st, pdl, s));
