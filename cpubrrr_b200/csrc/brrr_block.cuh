@@ -22,7 +22,7 @@ __device__ __forceinline__ void warp_quant_block(float v, int lane, int8_t *q, f
     float amax = fmaxf(warp_max(fabsf(v)), 1e-12f);
     float sc = __fdiv_rn(amax, 127.0f);
     if (lane == 0) *s = sc;
-    q[lane] = (int8_t)brrr_q8_round(v, sc);
+    q[lane] = (int8_t)brrr_q8_round_inv(v, sc, brrr_q8_inv(amax));
 }
 
 // Sum of squares in the 16-chain order: chain c (0..15) accumulates x[c], x[c+16], ... with fused
@@ -35,17 +35,24 @@ __device__ __forceinline__ float block_rms_inv(const float *x, int n, float eps,
         float acc = 0.0f;
         int n16 = n & ~15;
         if (c < 16) {
-            // chain c: x[c], x[c+16], ... in order; values are fetched 12 at a time so that only
+            // chain c: x[c], x[c+16], ... in order; the next 12 values are on their way while 12 are added up, so that only
             // the fused multiply-adds sit on the dependent path
             int i = c;
+            float v[12];
+#pragma unroll
+            for (int k = 0; k < 12; k++) v[k] = i + 16 * k < n16 ? x[i + 16 * k] : 0.0f;
+#pragma unroll 2
             for (; i + 16 * 11 < n16; i += 16 * 12) {
-                float v[12];
+                const float *w = x + min(i + 16 * 12, max(n16 - 16 * 12, 0) + c);      // past the last whole twelve: the end, read again below
+                float u[12];
 #pragma unroll
-                for (int k = 0; k < 12; k++) v[k] = x[i + 16 * k];
+                for (int k = 0; k < 12; k++) u[k] = v[k];
 #pragma unroll
-                for (int k = 0; k < 12; k++) acc = __fmaf_rn(v[k], v[k], acc);
+                for (int k = 0; k < 12; k++) v[k] = w[16 * k];
+#pragma unroll
+                for (int k = 0; k < 12; k++) acc = __fmaf_rn(u[k], u[k], acc);
             }
-            for (; i < n16; i += 16) { float v = x[i]; acc = __fmaf_rn(v, v, acc); }
+            for (; i < n16; i += 16) { float t = x[i]; acc = __fmaf_rn(t, t, acc); }
         }
         acc = __fadd_rn(acc, __shfl_xor_sync(0xffffffffu, acc, 4));
         acc = __fadd_rn(acc, __shfl_xor_sync(0xffffffffu, acc, 8));
@@ -136,9 +143,10 @@ __device__ __forceinline__ void block_norm_quant_staged(const float *norm_w, con
         amax = fmaxf(amax, __shfl_xor_sync(0xffffffffu, amax, 1));
         amax = fmaxf(amax, __shfl_xor_sync(0xffffffffu, amax, 2));
         amax = fmaxf(amax, __shfl_xor_sync(0xffffffffu, amax, 4));
-        const float sc = __fdiv_rn(fmaxf(amax, 1e-12f), 127.0f);
-        uint32_t word = (uint32_t)(brrr_q8_round(v.x, sc) & 0xFF) | ((uint32_t)(brrr_q8_round(v.y, sc) & 0xFF) << 8) |
-                        ((uint32_t)(brrr_q8_round(v.z, sc) & 0xFF) << 16) | ((uint32_t)(brrr_q8_round(v.w, sc) & 0xFF) << 24);
+        amax = fmaxf(amax, 1e-12f);
+        const float sc = __fdiv_rn(amax, 127.0f), qi = brrr_q8_inv(amax);
+        uint32_t word = (uint32_t)(brrr_q8_round_inv(v.x, sc, qi) & 0xFF) | ((uint32_t)(brrr_q8_round_inv(v.y, sc, qi) & 0xFF) << 8) |
+                        ((uint32_t)(brrr_q8_round_inv(v.z, sc, qi) & 0xFF) << 16) | ((uint32_t)(brrr_q8_round_inv(v.w, sc, qi) & 0xFF) << 24);
         const int t = g & 7, b = g >> 3;
         if (LAYOUT == NQ_MX) {
             uint32_t other = __shfl_xor_sync(0xffffffffu, word, 4);

@@ -51,6 +51,15 @@ __device__ __forceinline__ int brrr_q8_round(float v, float sc) {
     r = fminf(fmaxf(r, -127.0f), 127.0f);
     return (int)r;
 }
+// The same with an approximate reciprocal of the scale at hand (brrr_q8_inv): the product is within 1e-4 of the quotient, so only a value that
+// lies that close to a half needs the division (170 cycles).
+__device__ __forceinline__ float brrr_q8_inv(float amax) { return amax < 1e30f ? __fdividef(127.0f, amax) : __int_as_float(0x7FC00000); }
+__device__ __forceinline__ int brrr_q8_round_inv(float v, float sc, float inv) {
+    const float t = __fmul_rn(v, inv), r = __fadd_rn(t, 12582912.0f);       // 1.5 x 2^23: rounds to an integer, which the low bits then hold
+    if (!(fabsf(__fsub_rn(t, __fsub_rn(r, 12582912.0f))) < 0.4999f)) return brrr_q8_round(v, sc);
+    return (int)(int8_t)__float_as_uint(r);
+}
+
 __device__ __forceinline__ float brrr_bf16_to_f32(uint16_t v) { return __int_as_float((uint32_t)v << 16); }
 
 __device__ __forceinline__ uint32_t brrr_prmt(uint32_t a, uint32_t b, uint32_t c) {

@@ -49,8 +49,8 @@ struct AttnArgs {
 
 // Q8 of 32-block b of a row's attention output, held one value per lane: int8 values, scale, half image
 __device__ __forceinline__ void attn_quant(float o, int lane, int b, int8_t *aq, float *as, uint8_t *img) {
-    const float sc = __fdiv_rn(fmaxf(warp_max(fabsf(o)), 1e-12f), 127.0f);
-    const int qv = brrr_q8_round(o, sc);
+    const float amax = fmaxf(warp_max(fabsf(o)), 1e-12f), sc = __fdiv_rn(amax, 127.0f);
+    const int qv = brrr_q8_round_inv(o, sc, brrr_q8_inv(amax));
     if (lane == 0) as[b] = sc;
     if (aq) aq[b * 32 + lane] = (int8_t)qv;
     if (img) ti_emit_block<TI_HALF>(qv, lane, b, img);
@@ -121,7 +121,7 @@ __global__ void __launch_bounds__(AT_THREADS) attn_decode_kernel(AttnArgs a) {
     float rc = 0.0f, rs = 0.0f;
     if (tid < 64) { rc = a.rope[((size_t)pos * 32 + (tid & 31)) * 2]; rs = a.rope[((size_t)pos * 32 + (tid & 31)) * 2 + 1]; }
     BRRR_STAMP(a.err_state, 161);
-    pdl_wait();          // qkv projection done
+    pdl_wait_cta();      // qkv projection done
     BRRR_STAMP(a.err_state, 162);
     BRRR_GT_GO(a.err_state, 190);
     pdl_trigger();

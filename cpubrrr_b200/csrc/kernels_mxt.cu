@@ -158,6 +158,22 @@ __device__ __forceinline__ void xt_wait(uint64_t *bar, uint32_t parity, uint32_t
     if (!mbar_test_wait(bar, parity)) xt_wait_slow(bar, parity, err, sleep);
 }
 
+// The issuing warp's waits: suspended in hardware between probes (it waits most of the time, beside busy warps, and its wake-up is on the
+// critical path), a bounded number of times - far above any copy or product; then the error word is set and it waits no more.
+struct XtIssueWait {
+    uint32_t *err;
+    bool dead;
+    __device__ __forceinline__ void operator()(uint64_t *bar, uint32_t parity) {
+        if (dead || mbar_test_wait(bar, parity)) return;
+        for (int i = 0; !mbar_try_wait_hint(bar, parity, 20000u);)
+            if (++i == 1 << 17) {
+                dead = true;
+                if (err) atomicCAS(err, (uint32_t)DEV_ERR_NONE, (uint32_t)DEV_ERR_COPY_TIMEOUT);
+                break;
+            }
+    }
+};
+
 // Operand image of an activation that some other kernel quantised (stage-level entry points).
 __global__ void xt_bimg_kernel(const int8_t *__restrict__ xq, int nb, uint8_t *bimg) {
     const int b = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5), lane = threadIdx.x & 31;
@@ -290,7 +306,8 @@ __global__ void __launch_bounds__(XT_THREADS) xt_expert_kernel(XtArgs a) {
     const unsigned char *src = nullptr;
     const uint32_t ep_epoch = EP ? *a.ep.epoch : 0u;          // the step in flight (written by the step's first kernel)
     auto route_and_start = [&]() {
-        if (a.est) {
+        if (a.est && a.ne <= 32) e = warp_spec_expert(a.est, a.ne, a.topk, a.state, ei, lane);      // every warp by itself: no barrier, a tenth of the time
+        else if (a.est) {
             block_spec_select(a.est, a.ne, a.topk, a.state, lg, sel, tid, XT_THREADS);
             __syncthreads();
             e = sel[ei];
@@ -309,7 +326,7 @@ __global__ void __launch_bounds__(XT_THREADS) xt_expert_kernel(XtArgs a) {
     constexpr bool early = DOWN;
     if (early) route_and_start();
     BRRR_STAMP(a.state, SB + 1);
-    pdl_wait();
+    pdl_wait_cta();
     BRRR_STAMP(a.state, SB + 2);
     BRRR_GT_GO(a.state, SB + 30);
     pdl_trigger();
@@ -346,27 +363,32 @@ __global__ void __launch_bounds__(XT_THREADS) xt_expert_kernel(XtArgs a) {
             }
         }
     } else if (warp == 5) {
-        // ---- MMA issue: one instruction per block pair, four per round into one accumulator region
-        if (lane == 0) {
+        // ---- MMA issue: one instruction per block pair, four per round into one accumulator region (the whole warp walks the loop, an
+        // elected lane issues: in a one-lane branch every product costs 100 cycles of operand moves, 35 here)
+        {
+            XtIssueWait wait{err, err && *reinterpret_cast<volatile uint32_t *>(err) != 0u};
             const uint32_t sfa = tmem_base + XT_SF_COL, sfb = tmem_base + XT_SF_COL + 32;
             const uint64_t dhi = ((uint64_t)((128u >> 4) & 0x3FFF) << 32) | ((uint64_t)1 << 46);     // descriptor bits common to A and B
             const uint64_t alo = dhi | ((uint64_t)((2048u >> 4) & 0x3FFF) << 16), blo = dhi | ((uint64_t)(((uint32_t)XT_B_PAIR / 2 >> 4) & 0x3FFF) << 16);
             uint32_t baddr = smem_u32(sh.bimg) >> 4;              // descriptor start-address fields (16-byte units)
             const uint32_t r0 = smem_u32(sh.ring) >> 4, stage16 = (uint32_t)(stage_bytes >> 4);
-            xt_wait(sh.bfull, 0u, err, true);
+            wait(sh.bfull, 0u);
             int s = 0, reg = 0, left = np;
             uint32_t fpar = 0, epar = 1;             // full-stage parity; region-free parity (first pass: free)
 #pragma unroll 1
             for (int r = 0; r < nchunks; r++) {
-                xt_wait(&sh.full[s], fpar, err, true);
-                xt_wait(&sh.dempty[reg], epar, err, true);
+                wait(&sh.full[s], fpar);
+                wait(&sh.dempty[reg], epar);
                 xt_fence_after();
                 const uint32_t aaddr = r0 + s * stage16, d0 = tmem_base + reg * XT_REGION_COLS;
                 const int cnt = left < XT_CH ? left : XT_CH;
+                if (elect_one()) {
 #pragma unroll
-                for (int k = 0; k < XT_CH; k++)
-                    if (k < cnt) xt_mma(d0 + k * XT_N, alo | (aaddr + k * (MXT_UNIT / 16)), blo | (baddr + k * (XT_B_PAIR / 16)), sfa, sfb);
-                xt_commit(&sh.dfull[reg]);
+                    for (int k = 0; k < XT_CH; k++)
+                        if (k < cnt) xt_mma(d0 + k * XT_N, alo | (aaddr + k * (MXT_UNIT / 16)), blo | (baddr + k * (XT_B_PAIR / 16)), sfa, sfb);
+                    xt_commit(&sh.dfull[reg]);
+                }
+                __syncwarp();
                 baddr += XT_CH * XT_B_PAIR / 16;
                 left -= XT_CH;
                 if (++s == a.stages) { s = 0; fpar ^= 1u; }
@@ -440,7 +462,7 @@ __global__ void __launch_bounds__(XT_THREADS) xt_expert_kernel(XtArgs a) {
                 const float h = swiglu_oai(gu_s[0][warp * 32 + lane], gu_s[1][warp * 32 + lane]);
                 const float amax = fmaxf(warp_max(fabsf(h)), 1e-12f);
                 const float sc = __fdiv_rn(amax, 127.0f);
-                const int qv = brrr_q8_round(h, sc), b = t * 2 + warp;
+                const int qv = brrr_q8_round_inv(h, sc, brrr_q8_inv(amax)), b = t * 2 + warp;
                 if (lane == 0) a.hs[ei * nb + b] = sc;
                 a.hq[(size_t)ei * a.d + b * 32 + lane] = (int8_t)qv;
                 xt_emit_block(qv, lane, b, a.himg + (size_t)ei * np * XT_B_PAIR);
@@ -589,7 +611,7 @@ __global__ void __launch_bounds__(FN_THREADS) xt_fold_norm_kernel(FoldNormArgs a
 #ifdef BRRR_FOLD_EARLY_TRIGGER
     pdl_trigger();       // the next projection may become resident and stream its weights while down still runs
 #endif
-    pdl_wait();          // down's partial sums are complete
+    pdl_wait_cta();      // down's partial sums are complete
     BRRR_GT_GO(a.f.state, 239);
     BRRR_STAMP(a.f.state, 241);
 #ifndef BRRR_FOLD_EARLY_TRIGGER

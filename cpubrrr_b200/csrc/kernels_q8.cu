@@ -184,7 +184,7 @@ __global__ void __launch_bounds__(Q8_THREADS) q8_stream_kernel(Q8Args a) {
         if (EPI == Q8_EPI_RESID_BIAS) resid_pre = a.y[u0 * 16 + rl];
     }
     BRRR_STAMP(a.state, sb + 1);
-    pdl_wait();          // predecessor's outputs (activation, residual) are now visible
+    pdl_wait_cta();      // predecessor's outputs (activation, residual) are now visible
     BRRR_STAMP(a.state, sb + 2);
     BRRR_GT_GO(a.state, sb + 30);
     pdl_trigger();
@@ -286,7 +286,7 @@ __global__ void __launch_bounds__(256) q8_direct_kernel(Q8Dev m, const int8_t *_
     int2 *xp = reinterpret_cast<int2 *>(smraw);
     float *xsc = reinterpret_cast<float *>(smraw + (size_t)nb * 4 * sizeof(int2));
     __shared__ unsigned long long wbest[8];
-    pdl_wait();
+    pdl_wait_cta();
     pdl_trigger();
     for (int idx = threadIdx.x; idx < nb * 4; idx += 256) {
         int b = idx >> 2, j = idx & 3;
@@ -376,7 +376,7 @@ __global__ void __launch_bounds__(Q8_THREADS) q8_reg_kernel(Q8Args a) {
     }
 #endif
     BRRR_GT_START(a.state, EPI == Q8_EPI_BIAS ? 232 : 234);
-    pdl_wait();          // the activation is now visible
+    pdl_wait_cta();      // the activation is now visible
     BRRR_GT_GO(a.state, (EPI == Q8_EPI_BIAS ? 32 : 64) + 30);
     pdl_trigger();
     {
@@ -475,7 +475,7 @@ __global__ void __launch_bounds__(QH_THREADS) q8_head_ring_kernel(QHeadArgs a) {
     // the weights do not depend on the step: the first ring goes out before the dependency wait
     const bool producer = warp == 4;
     if (producer && lane < min(a.stages, nchunks)) issue(lane);
-    pdl_wait();
+    pdl_wait_cta();
     pdl_trigger();
     waiter.poison_if_failed();
     if (producer) {

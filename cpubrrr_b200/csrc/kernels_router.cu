@@ -482,7 +482,7 @@ __global__ void __launch_bounds__(HINT_THREADS) router_hint_kernel(HintArgs a) {
     }
     const float bias = a.b ? a.b[e] : 0.0f;
     BRRR_GT_START(a.state, 235);
-    pdl_wait();
+    pdl_wait_cta();
     BRRR_GT_GO(a.state, 224);
     pdl_trigger();
     stage_vec4(a.x_in, xf, d, tid, HINT_THREADS);
@@ -516,7 +516,7 @@ __global__ void __launch_bounds__(HINT_THREADS) router_hint_kernel(HintArgs a) {
             if (a.norm_w) v = __fmul_rn(__fmul_rn(v, inv), a.norm_w[blk * 32 + lane]);
             const float amax = fmaxf(warp_max(fabsf(v)), 1e-12f);
             const float sc = __fdiv_rn(amax, 127.0f);
-            const int qv = brrr_q8_round(v, sc);
+            const int qv = brrr_q8_round_inv(v, sc, brrr_q8_inv(amax));
             if (lane == 0) a.xs_out[blk] = sc;
             a.xq_out[blk * 32 + lane] = (int8_t)qv;
             if (a.bimg_out) xt_emit_block(qv, lane, blk, a.bimg_out);

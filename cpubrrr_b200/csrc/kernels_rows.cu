@@ -175,7 +175,7 @@ __global__ void __launch_bounds__(RN_THREADS) rows_norm_kernel(RowsNormArgs a) {
     extern __shared__ __align__(16) float rsm_x[];
     __shared__ float inv_sh;
     const int t = blockIdx.x, tid = threadIdx.x, d = a.d, groups = d >> 2;
-    pdl_wait();
+    pdl_wait_cta();
     pdl_trigger();
     float4 *x4 = reinterpret_cast<float4 *>(a.x + (size_t)t * d);
     for (int g = tid; g < groups; g += RN_THREADS) {
@@ -202,8 +202,8 @@ __global__ void __launch_bounds__(RN_THREADS) rows_norm_kernel(RowsNormArgs a) {
     for (int b = tid >> 5; b < nb; b += RN_THREADS / 32) {
         const float v = __fmul_rn(__fmul_rn(rsm_x[b * 32 + lane], inv), a.norm_w[b * 32 + lane]);
         if (a.xn) a.xn[(size_t)t * d + b * 32 + lane] = v;
-        const float sc = __fdiv_rn(fmaxf(warp_max(fabsf(v)), 1e-12f), 127.0f);
-        const int qv = brrr_q8_round(v, sc);
+        const float amax = fmaxf(warp_max(fabsf(v)), 1e-12f), sc = __fdiv_rn(amax, 127.0f);
+        const int qv = brrr_q8_round_inv(v, sc, brrr_q8_inv(amax));
         if (lane == 0) a.s[(size_t)t * nb + b] = sc;
         if (a.q) a.q[(size_t)t * d + b * 32 + lane] = (int8_t)qv;
         if (a.img) ti_emit_block<IMG>(qv, lane, b, a.img + (size_t)t * (nb / 2) * ti_pair(IMG));

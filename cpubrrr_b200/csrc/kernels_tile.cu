@@ -428,10 +428,10 @@ __global__ void __launch_bounds__(NT * 16 + 128, KIND == TK_Q8 || NT == 32 ? 1 :
 #pragma unroll
             for (int k = 0; k < 4; k++) {
                 if (t0 + k >= n_ent) break;
-                const float sc = __fdiv_rn(fmaxf(amax[k], 1e-12f), 127.0f);
+                const float am = fmaxf(amax[k], 1e-12f), sc = __fdiv_rn(am, 127.0f);
                 const size_t row = (size_t)ent[t0 + k];
                 if (lane == 0) a.hs[row * (a.nrows / 32) + b] = sc;
-                ti_emit_block<TI_PLANES>(brrr_q8_round(hv[k], sc), lane, b, a.himg + row * (size_t)(a.nrows / 64) * PAIR);
+                ti_emit_block<TI_PLANES>(brrr_q8_round_inv(hv[k], sc, brrr_q8_inv(am)), lane, b, a.himg + row * (size_t)(a.nrows / 64) * PAIR);
             }
         }
     }
