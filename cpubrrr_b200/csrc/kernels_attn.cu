@@ -9,9 +9,10 @@
 // The serial sums are one thread each (64 output dims + 1 denominator).
 //
 // The cache is laid out [kv head][position][64] so the window of one head is one contiguous
-// range; it is brought into shared memory in tiles of 128 positions (32 for token rows) by bulk asynchronous copies
+// range; K, then V run through one ring of tiles of 64 positions (32 for token rows) by bulk asynchronous copies, the first of them
 // issued before the kernel waits on its predecessor (the cached positions are older than this
-// token).  The current position's k and v never come from the cache: every head recomputes them.
+// token).  Long contexts are bound by the copies' latency and the chains over the keys: with two 128-position tiles in flight per tensor
+// and no reading ahead in the sums a key cost 21 ns, AT_KEY_NS now.  The current position's k and v never come from the cache: every head recomputes them.
 #include "brrr_kernels.h"
 #include "brrr_block.cuh"
 #include "brrr_tma.cuh"
@@ -21,9 +22,9 @@ namespace brrr {
 
 constexpr int HD = 64;
 constexpr int AT_THREADS = 256;
-constexpr int AT_TILE_ONE = 128;                   // positions per tile: one token per launch (one CTA per SM streams its head's window)
+constexpr int AT_TILE_ONE = 64;                    // positions per tile: one token per launch (one CTA per SM streams its head's window)
 constexpr int AT_TILE_ROWS = 32;                   // token rows: many (head, row) CTAs share an SM, so each holds less
-constexpr int AT_SLOTS = 2;                        // ring depth per tensor
+__host__ __device__ constexpr int at_slots(int tile) { return tile == AT_TILE_ONE ? 8 : 4; }      // tiles in flight
 
 struct AttnArgs {
     const float *qkv;
@@ -64,12 +65,11 @@ constexpr int kScoreUnroll = AT_SCORE_UNROLL;      // keys of the score loop in 
 template <int AT_TILE>
 __global__ void __launch_bounds__(AT_THREADS) attn_decode_kernel(AttnArgs a) {
     constexpr size_t AT_TILE_BYTES = (size_t)AT_TILE * HD * sizeof(float);
+    constexpr int SLOTS = at_slots(AT_TILE);
     extern __shared__ __align__(128) unsigned char smraw[];
-    float *ktiles = reinterpret_cast<float *>(smraw);                                   // [AT_SLOTS][128][64]
-    float *vtiles = reinterpret_cast<float *>(smraw + AT_TILE_BYTES * AT_SLOTS);
-    float *sc = reinterpret_cast<float *>(smraw + AT_TILE_BYTES * AT_SLOTS * 2);         // [MAXSEQ]
-    uint64_t *kbar = reinterpret_cast<uint64_t *>(sc + BRRR_MAXSEQ);
-    uint64_t *vbar = kbar + AT_SLOTS;
+    float *tiles = reinterpret_cast<float *>(smraw);                                    // [SLOTS][AT_TILE][64]
+    float *sc = reinterpret_cast<float *>(smraw + AT_TILE_BYTES * SLOTS);                // [MAXSEQ]
+    __shared__ __align__(8) uint64_t full[SLOTS];
     __shared__ float q[HD], kcur[HD], vcur[HD];
     __shared__ float red[AT_THREADS / 32];
     __shared__ float den_sh;
@@ -99,23 +99,20 @@ __global__ void __launch_bounds__(AT_THREADS) attn_decode_kernel(AttnArgs a) {
     const float *kbase = a.kc + ((size_t)kvh * BRRR_MAXSEQ + start) * HD;
     const float *vbase = a.vc + ((size_t)kvh * BRRR_MAXSEQ + start) * HD;
 
-    auto issue = [&](const float *base, float *tiles, uint64_t *bars, int t) {     // thread 0 only
-        int slot = t % AT_SLOTS, cnt = min(AT_TILE, ncached - t * AT_TILE);
-        mbar_expect_tx(&bars[slot], (uint32_t)cnt * HD * 4);
-        bulk_g2s(tiles + (size_t)slot * AT_TILE * HD, base + (size_t)t * AT_TILE * HD, (uint32_t)cnt * HD * 4, &bars[slot]);
+    auto issue = [&](int u) {                       // one thread: tile u of 2 ntiles, K then V
+        const int slot = u % SLOTS, t = u < ntiles ? u : u - ntiles, cnt = min(AT_TILE, ncached - t * AT_TILE);
+        mbar_expect_tx(&full[slot], (uint32_t)cnt * HD * 4);
+        bulk_g2s(tiles + (size_t)slot * AT_TILE * HD, (u < ntiles ? kbase : vbase) + (size_t)t * AT_TILE * HD, (uint32_t)cnt * HD * 4, &full[slot]);
     };
     BRRR_STAMP(a.err_state, 160);
     BRRR_GT_START(a.err_state, 233);
     if (tid == 0) {
-        for (int s = 0; s < AT_SLOTS; s++) { mbar_init(&kbar[s], 1); mbar_init(&vbar[s], 1); }
+        for (int s = 0; s < SLOTS; s++) mbar_init(&full[s], 1);
         mbar_fence_init();
     }
     __syncwarp();
-    // one lane per copy (K and V of the first tiles): their address translations overlap
-    if (!rows && tid < 2 * min(AT_SLOTS, ntiles)) {
-        if (tid & 1) issue(vbase, vtiles, vbar, tid >> 1);
-        else issue(kbase, ktiles, kbar, tid >> 1);
-    }
+    // one lane per copy: their address translations overlap
+    if (!rows && tid < min(SLOTS, 2 * ntiles)) issue(tid);
     // static / step-constant operands: the sink and this position's rotation
     const float sink = a.sinks[h];
     float rc = 0.0f, rs = 0.0f;
@@ -126,10 +123,7 @@ __global__ void __launch_bounds__(AT_THREADS) attn_decode_kernel(AttnArgs a) {
     BRRR_GT_GO(a.err_state, 190);
     pdl_trigger();
     waiter.poison_if_failed();
-    if (rows && tid < 2 * min(AT_SLOTS, ntiles)) {
-        if (tid & 1) issue(vbase, vtiles, vbar, tid >> 1);
-        else issue(kbase, ktiles, kbar, tid >> 1);
-    }
+    if (rows && tid < min(SLOTS, 2 * ntiles)) issue(tid);
 
     // ---- RoPE (NeoX halves, table holds cos*mscale / sin*mscale) on q and k; v passes through
     if (tid < 64) {
@@ -155,9 +149,9 @@ __global__ void __launch_bounds__(AT_THREADS) attn_decode_kernel(AttnArgs a) {
         const int g = tid >> 4, c = tid & 15;
         const float q0 = q[c], q1 = q[16 + c], q2 = q[32 + c], q3 = q[48 + c];
         for (int t = 0; t < ntiles; t++) {
-            const int slot = t % AT_SLOTS, cnt = min(AT_TILE, ncached - t * AT_TILE);
-            waiter.wait(&kbar[slot], (uint32_t)(t / AT_SLOTS) & 1u);
-            const float *kt = ktiles + (size_t)slot * AT_TILE * HD;
+            const int slot = t % SLOTS, cnt = min(AT_TILE, ncached - t * AT_TILE);
+            waiter.wait(&full[slot], (uint32_t)(t / SLOTS) & 1u);
+            const float *kt = tiles + (size_t)slot * AT_TILE * HD;
 #pragma unroll kScoreUnroll
             for (int k0 = 0; k0 < cnt; k0 += AT_THREADS / 16) {
                 int kk = k0 + g;
@@ -176,9 +170,9 @@ __global__ void __launch_bounds__(AT_THREADS) attn_decode_kernel(AttnArgs a) {
                 s = __fadd_rn(s, __shfl_xor_sync(0xffffffffu, s, 2));
                 if (live && c == 0) sc[t * AT_TILE + kk] = __fmul_rn(s, 0.125f);
             }
-            if (t + AT_SLOTS < ntiles) {
+            if (t + SLOTS < 2 * ntiles) {
                 __syncthreads();
-                if (tid == 0) { fence_proxy_async(); issue(kbase, ktiles, kbar, t + AT_SLOTS); }
+                if (tid == 0) { fence_proxy_async(); issue(t + SLOTS); }
             }
         }
         // the current position, from this CTA's own rotated k
@@ -207,7 +201,7 @@ __global__ void __launch_bounds__(AT_THREADS) attn_decode_kernel(AttnArgs a) {
     mx = red[0];
 #pragma unroll
     for (int w = 1; w < AT_THREADS / 32; w++) mx = fmaxf(mx, red[w]);
-    for (int t = tid; t < n; t += AT_THREADS) sc[t] = brrr_expf_dev(__fsub_rn(sc[t], mx));
+    for (int t = tid; t < ((n + 3) & ~3); t += AT_THREADS) sc[t] = t < n ? brrr_expf_dev(__fsub_rn(sc[t], mx)) : 0.0f;      // +0 past the end changes no sum
     __syncthreads();
 
     BRRR_STAMP(a.err_state, 164);
@@ -215,22 +209,58 @@ __global__ void __launch_bounds__(AT_THREADS) attn_decode_kernel(AttnArgs a) {
     float acc = 0.0f;
     if (tid == 64) {
         float den = brrr_expf_dev(__fsub_rn(sink, mx));
-#pragma unroll 8
-        for (int t = 0; t < n; t++) den = __fadd_rn(den, sc[t]);
+        float4 p = *reinterpret_cast<const float4 *>(sc);
+#pragma unroll 4
+        for (int t = 4; t < n + 4; t += 4) {
+            const float4 c = p;
+            p = *reinterpret_cast<const float4 *>(sc + (t < n ? t : 0));
+            den = __fadd_rn(den, c.x); den = __fadd_rn(den, c.y); den = __fadd_rn(den, c.z); den = __fadd_rn(den, c.w);
+        }
         den_sh = den;
     }
     for (int t = 0; t < ntiles; t++) {
-        const int slot = t % AT_SLOTS, cnt = min(AT_TILE, ncached - t * AT_TILE);
+        const int u = ntiles + t, slot = u % SLOTS, cnt = min(AT_TILE, ncached - t * AT_TILE);
         if (tid < 64) {
-            waiter.wait(&vbar[slot], (uint32_t)(t / AT_SLOTS) & 1u);
-            const float *vt = vtiles + (size_t)slot * AT_TILE * HD + tid;
-            const float *pt = sc + t * AT_TILE;
-#pragma unroll 8
-            for (int kk = 0; kk < cnt; kk++) acc = __fmaf_rn(vt[kk * HD], pt[kk], acc);
+            waiter.wait(&full[slot], (uint32_t)(u / SLOTS) & 1u);
+            // sixteen keys at a time, the next sixteen's values on the way (two sets of registers: reloading one set in place exposed every load's
+            // latency, 19 cycles per key instead of 7); then the rest
+            const float *vt = tiles + (size_t)slot * AT_TILE * HD + tid, *pt = sc + t * AT_TILE;
+            float v0[16], v1[16];
+            float4 p0[4], p1[4];
+            auto load = [&](float (&v)[16], float4 (&p)[4], int k) {
+                const float *w = vt + (k & (AT_TILE - 1)) * HD, *o = pt + (k & (AT_TILE - 1));
+#pragma unroll
+                for (int i = 0; i < 16; i++) v[i] = w[i * HD];
+#pragma unroll
+                for (int i = 0; i < 4; i++) p[i] = *reinterpret_cast<const float4 *>(o + 4 * i);
+            };
+            auto add = [&](const float (&v)[16], const float4 (&p)[4], int left) {
+#pragma unroll
+                for (int i = 0; i < 4; i++) {
+                    if (4 * i < left) acc = __fmaf_rn(v[4 * i], p[i].x, acc);
+                    if (4 * i + 1 < left) acc = __fmaf_rn(v[4 * i + 1], p[i].y, acc);
+                    if (4 * i + 2 < left) acc = __fmaf_rn(v[4 * i + 2], p[i].z, acc);
+                    if (4 * i + 3 < left) acc = __fmaf_rn(v[4 * i + 3], p[i].w, acc);
+                }
+            };
+            load(v0, p0, 0);
+            int k = 0;
+#pragma unroll 1
+            for (; k + 32 <= cnt; k += 32) {
+                load(v1, p1, k + 16);
+                add(v0, p0, 16);
+                load(v0, p0, k + 32);
+                add(v1, p1, 16);
+            }
+            if (k < cnt) {
+                load(v1, p1, k + 16);
+                add(v0, p0, cnt - k);
+                add(v1, p1, cnt - k - 16);
+            }
         }
-        if (t + AT_SLOTS < ntiles) {
+        if (u + SLOTS < 2 * ntiles) {
             __syncthreads();
-            if (tid == 0) { fence_proxy_async(); issue(vbase, vtiles, vbar, t + AT_SLOTS); }
+            if (tid == 0) { fence_proxy_async(); issue(u + SLOTS); }
         }
     }
     if (tid < 64) acc = __fmaf_rn(vcur[tid], sc[ncached], acc);          // t = pos: this token's own v
@@ -454,7 +484,7 @@ __global__ void __launch_bounds__(AR_THREADS) attn_rows_kernel(AttnRowsArgs a) {
     }
 }
 
-static size_t attn_smem(int tile) { return (size_t)tile * HD * sizeof(float) * AT_SLOTS * 2 + (size_t)BRRR_MAXSEQ * 4 + AT_SLOTS * 2 * 8; }
+static size_t attn_smem(int tile) { return (size_t)tile * HD * sizeof(float) * at_slots(tile) + (size_t)BRRR_MAXSEQ * 4; }
 
 cudaError_t launch_attn_decode(const float *qkv, float *kc, float *vc, const float *rope, const float *sinks, int nh, int nkv,
                                const DevState *state, int pos_val, int window, float *ao, int8_t *aq, float *as,

@@ -469,37 +469,43 @@ __global__ void __launch_bounds__(QA_THREADS) qw_attn_kernel(const __grid_consta
         const int slot = (nt + t) % QA_SLOTS;
         if (tid < QW_HD) {
             waiter.wait(&full[slot], (uint32_t)((nt + t) / QA_SLOTS) & 1u);
-            // whole sixteens, the next one's values on the way while this one's are added up; then the rest
+            // sixteen positions at a time, the next sixteen's values on the way (two sets of registers: reloading one set in place exposed
+            // every load's latency); then the rest
             const int cnt = min(QA_TILE, pos - t * QA_TILE);
             const uint32_t vt = ring0 + slot * QA_TILE_BYTES;
             const float *pt = sc + t * QA_TILE;
-            float v[16];
-            float4 p[4];
+            float v0[16], v1[16];
+            float4 p0[4], p1[4];
+            auto load = [&](float (&v)[16], float4 (&p)[4], int k) {
+                const uint32_t w = vt + (k & (QA_TILE - 1)) * 128;
+                const float *o = pt + (k & (QA_TILE - 1));
 #pragma unroll
-            for (int i = 0; i < 16; i++) v[i] = qa_lds(vt + voff[i & 7] + (i >> 3) * 1024);
+                for (int i = 0; i < 16; i++) v[i] = qa_lds(w + voff[i & 7] + (i >> 3) * 1024);
 #pragma unroll
-            for (int i = 0; i < 4; i++) p[i] = *reinterpret_cast<const float4 *>(pt + 4 * i);
-            int k = 0;
-#pragma unroll 1
-            for (; k + 16 <= cnt; k += 16) {
-                const int kn = (k + 16) & (QA_TILE - 1);
-                const uint32_t w = vt + kn * 128;
-                const float *o = pt + kn;
+                for (int i = 0; i < 4; i++) p[i] = *reinterpret_cast<const float4 *>(o + 4 * i);
+            };
+            auto add = [&](const float (&v)[16], const float4 (&p)[4], int left) {
 #pragma unroll
                 for (int i = 0; i < 4; i++) {
-                    acc = __fmaf_rn(v[4 * i], p[i].x, acc); v[4 * i] = qa_lds(w + voff[(4 * i) & 7] + (i >> 1) * 1024);
-                    acc = __fmaf_rn(v[4 * i + 1], p[i].y, acc); v[4 * i + 1] = qa_lds(w + voff[(4 * i + 1) & 7] + (i >> 1) * 1024);
-                    acc = __fmaf_rn(v[4 * i + 2], p[i].z, acc); v[4 * i + 2] = qa_lds(w + voff[(4 * i + 2) & 7] + (i >> 1) * 1024);
-                    acc = __fmaf_rn(v[4 * i + 3], p[i].w, acc); v[4 * i + 3] = qa_lds(w + voff[(4 * i + 3) & 7] + (i >> 1) * 1024);
-                    p[i] = *reinterpret_cast<const float4 *>(o + 4 * i);
+                    if (4 * i < left) acc = __fmaf_rn(v[4 * i], p[i].x, acc);
+                    if (4 * i + 1 < left) acc = __fmaf_rn(v[4 * i + 1], p[i].y, acc);
+                    if (4 * i + 2 < left) acc = __fmaf_rn(v[4 * i + 2], p[i].z, acc);
+                    if (4 * i + 3 < left) acc = __fmaf_rn(v[4 * i + 3], p[i].w, acc);
                 }
+            };
+            load(v0, p0, 0);
+            int k = 0;
+#pragma unroll 1
+            for (; k + 32 <= cnt; k += 32) {
+                load(v1, p1, k + 16);
+                add(v0, p0, 16);
+                load(v0, p0, k + 32);
+                add(v1, p1, 16);
             }
-#pragma unroll
-            for (int i = 0; i < 4; i++) {
-                if (k + 4 * i < cnt) acc = __fmaf_rn(v[4 * i], p[i].x, acc);
-                if (k + 4 * i + 1 < cnt) acc = __fmaf_rn(v[4 * i + 1], p[i].y, acc);
-                if (k + 4 * i + 2 < cnt) acc = __fmaf_rn(v[4 * i + 2], p[i].z, acc);
-                if (k + 4 * i + 3 < cnt) acc = __fmaf_rn(v[4 * i + 3], p[i].w, acc);
+            if (k < cnt) {
+                load(v1, p1, k + 16);
+                add(v0, p0, cnt - k);
+                add(v1, p1, cnt - k - 16);
             }
         }
         if (nt + t + QA_SLOTS < 2 * nt) {
