@@ -22,6 +22,7 @@ namespace brrr {
 
 constexpr int HD = 64;
 constexpr int AT_THREADS = 256;
+constexpr int AT_ISSUER = 224;                     // refills the ring: a thread of the last warp, which carries no serial sum (an issue takes 220 cycles)
 constexpr int AT_TILE_ONE = 64;                    // positions per tile: one token per launch (one CTA per SM streams its head's window)
 constexpr int AT_TILE_ROWS = 32;                   // token rows: many (head, row) CTAs share an SM, so each holds less
 __host__ __device__ constexpr int at_slots(int tile) { return tile == AT_TILE_ONE ? 8 : 4; }      // tiles in flight
@@ -58,7 +59,7 @@ __device__ __forceinline__ void attn_quant(float o, int lane, int b, int8_t *aq,
 }
 
 #ifndef AT_SCORE_UNROLL
-#define AT_SCORE_UNROLL 8
+#define AT_SCORE_UNROLL 4
 #endif
 constexpr int kScoreUnroll = AT_SCORE_UNROLL;      // keys of the score loop in flight per thread group (their shuffle chains overlap)
 
@@ -172,7 +173,7 @@ __global__ void __launch_bounds__(AT_THREADS) attn_decode_kernel(AttnArgs a) {
             }
             if (t + SLOTS < 2 * ntiles) {
                 __syncthreads();
-                if (tid == 0) { fence_proxy_async(); issue(t + SLOTS); }
+                if (tid == AT_ISSUER) { fence_proxy_async(); issue(t + SLOTS); }
             }
         }
         // the current position, from this CTA's own rotated k
@@ -207,17 +208,16 @@ __global__ void __launch_bounds__(AT_THREADS) attn_decode_kernel(AttnArgs a) {
     BRRR_STAMP(a.err_state, 164);
     // ---- serial sums: thread u < 64 owns output dim u, thread 64 the denominator
     float acc = 0.0f;
-    if (tid == 64) {
-        float den = brrr_expf_dev(__fsub_rn(sink, mx));
-        float4 p = *reinterpret_cast<const float4 *>(sc);
+    float den = tid == 64 ? brrr_expf_dev(__fsub_rn(sink, mx)) : 0.0f;      // tile by tile: its warp takes part in the ring's barriers
+    auto add_den = [&](int t0, int t1) {                                   // probabilities t0 .. t1 - 1, t0 a multiple of 4, the last four padded with +0
+        float4 p = *reinterpret_cast<const float4 *>(sc + t0);
 #pragma unroll 4
-        for (int t = 4; t < n + 4; t += 4) {
+        for (int t = t0 + 4; t < t1 + 4; t += 4) {
             const float4 c = p;
-            p = *reinterpret_cast<const float4 *>(sc + (t < n ? t : 0));
+            p = *reinterpret_cast<const float4 *>(sc + (t < t1 ? t : t0));
             den = __fadd_rn(den, c.x); den = __fadd_rn(den, c.y); den = __fadd_rn(den, c.z); den = __fadd_rn(den, c.w);
         }
-        den_sh = den;
-    }
+    };
     for (int t = 0; t < ntiles; t++) {
         const int u = ntiles + t, slot = u % SLOTS, cnt = min(AT_TILE, ncached - t * AT_TILE);
         if (tid < 64) {
@@ -258,10 +258,15 @@ __global__ void __launch_bounds__(AT_THREADS) attn_decode_kernel(AttnArgs a) {
                 add(v1, p1, cnt - k - 16);
             }
         }
+        if (tid == 64) add_den(t * AT_TILE, t + 1 < ntiles ? (t + 1) * AT_TILE : n);
         if (u + SLOTS < 2 * ntiles) {
             __syncthreads();
-            if (tid == 0) { fence_proxy_async(); issue(u + SLOTS); }
+            if (tid == AT_ISSUER) { fence_proxy_async(); issue(u + SLOTS); }
         }
+    }
+    if (tid == 64) {
+        if (ntiles == 0) add_den(0, n);
+        den_sh = den;
     }
     if (tid < 64) acc = __fmaf_rn(vcur[tid], sc[ncached], acc);          // t = pos: this token's own v
     __syncthreads();

@@ -316,7 +316,7 @@ __global__ void __launch_bounds__(QG_THREADS, 2) qw_gemv_kernel(const __grid_con
 // cycles of the load/store pipe per tile, a bulk copy per position 3400.
 // Score threads are (key, two chains), keys of a phase two apart; p.V threads are the dims.
 // Bound: at 100 positions the prologue's and softmax's latencies; then the chains over the keys (4 cycles each).
-constexpr int QA_TILE = 64, QA_SLOTS = 5, QA_THREADS = 256;
+constexpr int QA_TILE = 64, QA_SLOTS = 5, QA_THREADS = 256, QA_ISSUER = 224;      // the issuer refills the ring: of the last warp, which carries no serial sum
 constexpr uint32_t QA_BOX = QA_TILE * 128, QA_TILE_BYTES = 4 * QA_BOX;
 constexpr size_t QA_SMEM = (size_t)QA_SLOTS * QA_TILE_BYTES + (size_t)BRRR_MAXSEQ * 4 + 1024;
 
@@ -436,7 +436,7 @@ __global__ void __launch_bounds__(QA_THREADS) qw_attn_kernel(const __grid_consta
         }
         if (t + QA_SLOTS < 2 * nt) {
             __syncthreads();
-            if (tid == 0) { fence_proxy_async(); issue(t + QA_SLOTS); }
+            if (tid == QA_ISSUER) { fence_proxy_async(); issue(t + QA_SLOTS); }
         }
     }
     mx = warp_max(mx);
@@ -449,17 +449,16 @@ __global__ void __launch_bounds__(QA_THREADS) qw_attn_kernel(const __grid_consta
     for (int t = tid; t < ((n + 3) & ~3); t += QA_THREADS) sc[t] = t < n ? brrr_expf_dev(__fsub_rn(sc[t], mx)) : 0.0f;      // +0 past the end changes no sum
     __syncthreads();
     float acc = 0.0f;
-    if (tid == 128) {
-        float den = 0.0f;
-        float4 p = *reinterpret_cast<const float4 *>(sc);
+    float den = 0.0f;
+    auto add_den = [&](int t0, int t1) {      // probabilities t0 .. t1 - 1, t0 a multiple of 4, the last four padded with +0 (tile by tile: this warp takes part in the barriers)
+        float4 p = *reinterpret_cast<const float4 *>(sc + t0);
 #pragma unroll 4
-        for (int t = 4; t < n + 4; t += 4) {
+        for (int t = t0 + 4; t < t1 + 4; t += 4) {
             const float4 c = p;
-            p = *reinterpret_cast<const float4 *>(sc + (t < n ? t : 0));
+            p = *reinterpret_cast<const float4 *>(sc + (t < t1 ? t : t0));
             den = __fadd_rn(den, c.x); den = __fadd_rn(den, c.y); den = __fadd_rn(den, c.z); den = __fadd_rn(den, c.w);
         }
-        den_sh = den;
-    }
+    };
     // chunk lane / 4 of the position's row in box `warp`
     uint32_t voff[8];
 #pragma unroll
@@ -508,10 +507,15 @@ __global__ void __launch_bounds__(QA_THREADS) qw_attn_kernel(const __grid_consta
                 add(v1, p1, cnt - k - 16);
             }
         }
+        if (tid == 128) add_den(t * QA_TILE, t + 1 < nt ? (t + 1) * QA_TILE : n);
         if (nt + t + QA_SLOTS < 2 * nt) {
             __syncthreads();
-            if (tid == 0) { fence_proxy_async(); issue(nt + t + QA_SLOTS); }
+            if (tid == QA_ISSUER) { fence_proxy_async(); issue(nt + t + QA_SLOTS); }
         }
+    }
+    if (tid == 128) {
+        if (nt == 0) add_den(0, n);
+        den_sh = den;
     }
     __syncthreads();
     if (tid < QW_HD) a.out[h * QW_HD + tid] = __fmul_rn(__fmaf_rn(vs[tid], sc[pos], acc), __fdiv_rn(1.0f, den_sh));
