@@ -58,10 +58,6 @@ __device__ __forceinline__ void attn_quant(float o, int lane, int b, int8_t *aq,
     if (img) ti_emit_block<TI_HALF>(qv, lane, b, img);
 }
 
-#ifndef AT_SCORE_UNROLL
-#define AT_SCORE_UNROLL 4
-#endif
-constexpr int kScoreUnroll = AT_SCORE_UNROLL;      // keys of the score loop in flight per thread group (their shuffle chains overlap)
 
 template <int AT_TILE>
 __global__ void __launch_bounds__(AT_THREADS) attn_decode_kernel(AttnArgs a) {
@@ -153,23 +149,27 @@ __global__ void __launch_bounds__(AT_THREADS) attn_decode_kernel(AttnArgs a) {
             const int slot = t % SLOTS, cnt = min(AT_TILE, ncached - t * AT_TILE);
             waiter.wait(&full[slot], (uint32_t)(t / SLOTS) & 1u);
             const float *kt = tiles + (size_t)slot * AT_TILE * HD;
-#pragma unroll kScoreUnroll
-            for (int k0 = 0; k0 < cnt; k0 += AT_THREADS / 16) {
-                int kk = k0 + g;
-                bool live = kk < cnt;
-                float s = 0.0f;
-                if (live) {
-                    const float *kp = kt + kk * HD;
-                    s = __fmaf_rn(kp[c], q0, s);
-                    s = __fmaf_rn(kp[16 + c], q1, s);
-                    s = __fmaf_rn(kp[32 + c], q2, s);
-                    s = __fmaf_rn(kp[48 + c], q3, s);
-                }
-                s = __fadd_rn(s, __shfl_xor_sync(0xffffffffu, s, 4));
-                s = __fadd_rn(s, __shfl_xor_sync(0xffffffffu, s, 8));
-                s = __fadd_rn(s, __shfl_xor_sync(0xffffffffu, s, 1));
-                s = __fadd_rn(s, __shfl_xor_sync(0xffffffffu, s, 2));
-                if (live && c == 0) sc[t * AT_TILE + kk] = __fmul_rn(s, 0.125f);
+            // the tile's keys of this group side by side, so that their shuffles overlap (a key at a time: 265 cycles per sixteen keys); past the
+            // last key the sums are of no account
+            float s[AT_TILE / 16];
+#pragma unroll
+            for (int i = 0; i < AT_TILE / 16; i++) {
+                const float *kp = kt + (i * 16 + g) * HD;
+                s[i] = __fmaf_rn(kp[c], q0, 0.0f);
+                s[i] = __fmaf_rn(kp[16 + c], q1, s[i]);
+                s[i] = __fmaf_rn(kp[32 + c], q2, s[i]);
+                s[i] = __fmaf_rn(kp[48 + c], q3, s[i]);
+            }
+#pragma unroll
+            for (int o = 0; o < 4; o++) {
+                const int x = o == 0 ? 4 : o == 1 ? 8 : o == 2 ? 1 : 2;
+#pragma unroll
+                for (int i = 0; i < AT_TILE / 16; i++) s[i] = __fadd_rn(s[i], __shfl_xor_sync(0xffffffffu, s[i], x));
+            }
+            if (c == 0) {
+#pragma unroll
+                for (int i = 0; i < AT_TILE / 16; i++)
+                    if (i * 16 + g < cnt) sc[t * AT_TILE + i * 16 + g] = __fmul_rn(s[i], 0.125f);
             }
             if (t + SLOTS < 2 * ntiles) {
                 __syncthreads();
