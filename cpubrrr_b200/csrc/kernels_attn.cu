@@ -12,7 +12,7 @@
 // range; K, then V run through one ring of tiles of 64 positions (32 for token rows) by bulk asynchronous copies, the first of them
 // issued before the kernel waits on its predecessor (the cached positions are older than this
 // token).  Long contexts are bound by the copies' latency and the chains over the keys: with two 128-position tiles in flight per tensor
-// and no reading ahead in the sums a key cost 21 ns, AT_KEY_NS now.  The current position's k and v never come from the cache: every head recomputes them.
+// and no reading ahead in the sums a key cost 23 ns, now 15.  The current position's k and v never come from the cache: every head recomputes them.
 #include "brrr_kernels.h"
 #include "brrr_block.cuh"
 #include "brrr_tma.cuh"
@@ -288,11 +288,12 @@ __global__ void __launch_bounds__(AT_THREADS) attn_decode_kernel(AttnArgs a) {
 // memory.  Same operations in the same order per pair as attn_decode_kernel (the row's own key comes from the cache,
 // where kv_append_rows_kernel wrote the same bits):
 //   score(t)  one thread: the 16 four-term chains, then the pairwise combine of the shuffle butterfly (xor 4, 8, 1, 2)
-//   pass 1    scores of every key -> the pair's maximum;  pass 2  scores again -> p = exp(s - mx) into shared memory,
+//   pass 1    scores of every key -> workspace, the pair's maximum;  pass 2  p = exp(s - mx) into shared memory,
 //             then, tile by tile in ascending key order, the serial denominator (one thread per pair) and the serial
 //             p.V sums (one thread per (dim, 8 pairs)).  Keys outside a pair's range carry p = +0: x + 0 = x exactly
 //             (no accumulator is ever -0: the sums start at +0 and round to nearest), so they need no branch.
-// Scores are computed twice instead of being kept: 32 pairs x 4096 keys would not fit shared memory.
+// 32 pairs x 4096 keys of scores do not fit shared memory: they wait in a workspace (written and read by the same thread, 128 bytes per key and
+// warp; mostly L2).  Formed twice instead, a 512-row tile at positions 1024 .. 1535 took 895 us, now 742.
 constexpr int AR_THREADS = 256;
 constexpr int AR_TILE = 128;
 constexpr int AR_PAIRS = 32;
@@ -310,6 +311,7 @@ struct AttnRowsArgs {
     int8_t *aq;
     float *as;
     uint8_t *img;            // nullable: half images of the outputs
+    float *scores;           // workspace: [row block][kv head][MAXSEQ][32]
     DevState *err_state;
 };
 
@@ -402,6 +404,7 @@ __global__ void __launch_bounds__(AR_THREADS) attn_rows_kernel(AttnRowsArgs a) {
         bulk_g2s(vtile + (size_t)buf * AR_TILE * HD, vbase + (size_t)t * AR_TILE * HD, (uint32_t)cnt * HD * 4, &vbar[buf]);
     };
 
+    float *my_scores = a.scores + ((size_t)blockIdx.y * a.nkv + kvh) * BRRR_MAXSEQ * AR_PAIRS + lane;
     // ---- pass 1: the maximum of every pair's scores
     float mx = -3.4028234663852886e38f;
     if (tid == 0) issue_k(0);
@@ -416,6 +419,7 @@ __global__ void __launch_bounds__(AR_THREADS) attn_rows_kernel(AttnRowsArgs a) {
         for (int kk = warp; kk < cnt; kk += AR_THREADS / 32) {
             const float sc = ar_score(q, kt + kk * HD);
             const int key = tb + kk;
+            my_scores[(size_t)(t * AR_TILE + kk) * AR_PAIRS] = sc;
             if (pr_live && key >= my_start && key <= my_pos) mx = fmaxf(mx, sc);
         }
         __syncthreads();              // everyone is done with this buffer
@@ -439,20 +443,20 @@ __global__ void __launch_bounds__(AR_THREADS) attn_rows_kernel(AttnRowsArgs a) {
 #pragma unroll
     for (int j = 0; j < 8; j++) acc[j] = 0.0f;
     float den = tid < AR_PAIRS ? den_sm[tid] : 0.0f;
-    if (tid == 0) { issue_k(0); issue_v(0); }
-    k_issued++; v_issued++;
+    if (tid == 0) issue_v(0);
+    v_issued++;
     for (int t = 0; t < ntiles; t++) {
-        if (t + 1 < ntiles) { if (tid == 0) { issue_k(t + 1); issue_v(t + 1); } k_issued++; v_issued++; }
-        const int kb = k_used & 1, vb = v_used & 1;
-        waiter.wait(&kbar[kb], (uint32_t)(k_used >> 1) & 1u);
-        k_used++;
-        const float *kt = ktile + (size_t)kb * AR_TILE * HD;
+        if (t + 1 < ntiles) { if (tid == 0) issue_v(t + 1); v_issued++; }
+        const int vb = v_used & 1;
         const int cnt = min(AR_TILE, nkeys - t * AR_TILE), tb = t_lo + t * AR_TILE;
-        for (int kk = warp; kk < cnt; kk += AR_THREADS / 32) {
-            const float sc = ar_score(q, kt + kk * HD);
-            const int key = tb + kk;
-            const bool valid = pr_live && key >= my_start && key <= my_pos;
-            psm[kk * AR_PAIRS + pr] = valid ? brrr_expf_dev(__fsub_rn(sc, mx)) : 0.0f;
+        float sv[AR_TILE / 8];                // this thread's keys warp, warp + 8, ... of the tile
+#pragma unroll
+        for (int i = 0; i < AR_TILE / 8; i++) sv[i] = warp + 8 * i < cnt ? my_scores[(size_t)(t * AR_TILE + warp + 8 * i) * AR_PAIRS] : 0.0f;
+#pragma unroll
+        for (int i = 0; i < AR_TILE / 8; i++) {
+            const int kk = warp + 8 * i, key = tb + kk;
+            const bool valid = kk < cnt && pr_live && key >= my_start && key <= my_pos;
+            if (kk < cnt) psm[kk * AR_PAIRS + pr] = valid ? brrr_expf_dev(__fsub_rn(sv[i], mx)) : 0.0f;
         }
         __syncthreads();
         if (tid < AR_PAIRS) {
@@ -511,10 +515,10 @@ cudaError_t launch_attn_decode(const float *qkv, float *kc, float *vc, const flo
 // Needs the rows' keys in the cache already (launch_kv_append_rows) and nh / nkv a power of two <= 32.
 cudaError_t launch_attn_rows(const float *qkv, int ldq, const float *kc, const float *vc, size_t seq_stride, const float *rope, const float *sinks,
                              int nh, int nkv, int window, const int *row_pos, const int *row_seq, int rows, float *ao, int8_t *aq, float *as, uint8_t *aimg,
-                             DevState *err_state, bool pdl, cudaStream_t st) {
+                             float *scores, DevState *err_state, bool pdl, cudaStream_t st) {
     const int group = nkv > 0 ? nh / nkv : 0;
     if (group < 1 || group > 32 || (group & (group - 1)) || nh % nkv || rows < 1) return cudaErrorInvalidValue;
-    AttnRowsArgs a{qkv, kc, vc, rope, sinks, nh, nkv, window, rows, ldq, row_pos, row_seq, seq_stride, ao, aq, as, aimg, err_state};
+    AttnRowsArgs a{qkv, kc, vc, rope, sinks, nh, nkv, window, rows, ldq, row_pos, row_seq, seq_stride, ao, aq, as, aimg, scores, err_state};
     static unsigned long long configured = 0;      // one bit per device
     cudaError_t e = smem_optin(attn_rows_kernel, (int)AR_SMEM, configured);
     if (e != cudaSuccess) return e;

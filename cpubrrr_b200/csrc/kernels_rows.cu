@@ -168,7 +168,7 @@ struct RowsNormArgs {
     uint8_t *img;                   // nullable
 };
 
-constexpr int RN_THREADS = 384;
+constexpr int RN_THREADS = 960;      // 90 blocks of a 2880-wide row in three turns of 30 warps (a turn is 400 cycles of latency)
 
 template <int IMG, bool COMBINE>
 __global__ void __launch_bounds__(RN_THREADS) rows_norm_kernel(RowsNormArgs a) {
@@ -202,7 +202,7 @@ __global__ void __launch_bounds__(RN_THREADS) rows_norm_kernel(RowsNormArgs a) {
     for (int b = tid >> 5; b < nb; b += RN_THREADS / 32) {
         const float v = __fmul_rn(__fmul_rn(rsm_x[b * 32 + lane], inv), a.norm_w[b * 32 + lane]);
         if (a.xn) a.xn[(size_t)t * d + b * 32 + lane] = v;
-        const float amax = fmaxf(warp_max(fabsf(v)), 1e-12f), sc = __fdiv_rn(amax, 127.0f);
+        const float amax = fmaxf(__uint_as_float(__reduce_max_sync(0xffffffffu, __float_as_uint(fabsf(v)))), 1e-12f), sc = __fdiv_rn(amax, 127.0f);      // not negative: ordered as integers
         const int qv = brrr_q8_round_inv(v, sc, brrr_q8_inv(amax));
         if (lane == 0) a.s[(size_t)t * nb + b] = sc;
         if (a.q) a.q[(size_t)t * d + b * 32 + lane] = (int8_t)qv;

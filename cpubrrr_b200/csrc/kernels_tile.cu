@@ -520,16 +520,19 @@ cudaError_t mx_tensor_map(MxDev w, int units, CUtensorMap *map) {
 }
 
 // Tokens per CTA.  Experts: by the entries an expert has on average - few tokens keep more CTAs and copies in flight (up to 16 rows
-// the launch is a stream of weights), many amortise the products' reads of operand A.  One matrix: the most that leaves a CTA for
-// most of the 148 SMs (64 rows x 2880 outputs: 8 tokens, 184 CTAs of 64 pairs, against 46 of 32 tokens that take twice as long).
+// the launch is a stream of weights), many amortise the products' reads of operand A.  One matrix: a CTA per SM, so the fewest
+// rounds of 148 CTAs, a round of 8, 16 or 32 tokens taking 30, 33 and 47 us at 64 pairs (64 rows x 2880 outputs: 92 CTAs of 16 tokens, 33 us;
+// 184 of 8 tokens are two rounds, 65 us).
 template <int KIND>
 cudaError_t tl_launch(TileArgs a, int tiles, int entries, int experts, bool pdl, cudaStream_t st) {
     const int avg = (entries + experts - 1) / experts, most = a.cnt ? a.ntok : entries;
     if (most < 1 || most > TL_MAXTOK) return cudaErrorInvalidValue;
     int nt = avg > 12 ? 32 : avg > 6 ? 16 : 8;
     if (!a.cnt) {
-        nt = entries > 16 ? 32 : entries > 8 ? 16 : 8;
-        while (nt > 8 && tiles * ((entries + nt - 1) / nt) < 120) nt /= 2;
+        auto cost = [&](int n, int round) { return ((tiles * ((entries + n - 1) / n) + 147) / 148) * round; };
+        nt = 8;
+        if (entries > 8 && cost(16, 33) < cost(nt, 30)) nt = 16;
+        if (entries > 16 && cost(32, 47) < cost(nt, nt == 8 ? 30 : 33)) nt = 32;
     }
     static unsigned long long configured[3] = {0, 0, 0};      // one bit per device
     // at most one partly filled chunk per expert, and never more chunks than entries

@@ -157,7 +157,7 @@ struct brrr_model {
     int8_t *tl_nq = nullptr, *tl_aq = nullptr;
     float *tl_ns = nullptr, *tl_as = nullptr, *tl_es = nullptr, *tl_hs = nullptr;
     uint8_t *tl_nimg = nullptr, *tl_aimg = nullptr, *tl_eimg = nullptr, *tl_himg = nullptr;
-    float *tl_logits = nullptr, *tl_wts = nullptr, *tl_part = nullptr;
+    float *tl_logits = nullptr, *tl_wts = nullptr, *tl_part = nullptr, *tl_scores = nullptr;
     int32_t *tl_top = nullptr;
     int *tl_cnt = nullptr, *tl_list = nullptr;
     uint32_t *tl_toks = nullptr;                 // per row: token id, position, sequence (device; filled from a pinned slot)
@@ -898,6 +898,7 @@ static int rows_alloc(brrr_model *m) {
     TRY(m->alloc(&m->tl_aq, R * ao)); TRY(m->alloc(&m->tl_as, R * (ao / 32))); TRY(m->alloc(&m->tl_aimg, image_bytes(R, ao, TI_HALF)));
     TRY(m->alloc(&m->tl_es, R * nb)); TRY(m->alloc(&m->tl_eimg, image_bytes(R, d, TI_PLANES)));
     TRY(m->alloc(&m->tl_hs, E * nb)); TRY(m->alloc(&m->tl_himg, image_bytes((int)E, d, TI_PLANES))); TRY(m->alloc(&m->tl_part, E * d));
+    TRY(m->alloc(&m->tl_scores, R * c.n_head * BRRR_MAXSEQ));      // attention of prompt tiles: every pair's scores
     TRY(m->alloc(&m->tl_logits, R * ne)); TRY(m->alloc(&m->tl_top, R * 8)); TRY(m->alloc(&m->tl_wts, R * 8));
     TRY(m->alloc(&m->tl_counter, R)); TRY(m->alloc(&m->tl_cnt, ne)); TRY(m->alloc(&m->tl_list, (size_t)ne * R));
     CU(cudaMemsetAsync(m->tl_counter, 0, R * sizeof(unsigned int), m->stream));
@@ -937,7 +938,7 @@ static int enqueue_rows(brrr_model *m, int n, int kind, bool pdl) {
         uint8_t *aimg = tensor ? m->tl_aimg : nullptr;
         if (one_sequence && !m->no_attn_rows && group <= 32 && (group & (group - 1)) == 0)
             CUL(launch_attn_rows(m->tl_qkv, qkv_rows, kc, vc, seq_stride, m->rope, ly.sinks, nh, nkv, window, m->tl_pos, m->tl_seq, n, m->tl_ao, aq,
-                                 m->tl_as, aimg, m->st, pdl, s));
+                                 m->tl_as, aimg, m->tl_scores, m->st, pdl, s));
         else
             CUL(launch_attn_decode(m->tl_qkv, kc, vc, m->rope, ly.sinks, nh, nkv, nullptr, 0, window, m->tl_ao, aq, m->tl_as, m->st, pdl, s, 0,
                                    m->tl_pos, m->tl_seq, seq_stride, qkv_rows, n, aimg));
