@@ -117,13 +117,16 @@ __device__ __forceinline__ void qw_routing(bool est, const int *sel, const int32
     }
 }
 
-// The 12-slice norm (engine_qwen2.rs:453-465) of xf (shared memory, synchronised): 1 / sqrt(mean + eps) in every thread.
-__device__ __forceinline__ float qw_norm_inv(const float *xf, int d, float eps, float *part, int tid) {
+// The 12-slice norm (engine_qwen2.rs:453-465) of xf (shared memory, synchronised): 1 / sqrt(mean + eps) in every thread.  beside(): run by every warp
+// before the slices meet.
+template <typename F>
+__device__ __forceinline__ float qw_norm_inv(const float *xf, int d, float eps, float *part, int tid, F beside) {
     if (tid < QW_NT) {
         int lo, hi;
         qw_slice(tid, d, lo, hi);
         part[tid] = chain_squares(xf, lo, hi);
     }
+    beside();
     __syncthreads();
     const float4 p0 = reinterpret_cast<const float4 *>(part)[0], p1 = reinterpret_cast<const float4 *>(part)[1], p2 = reinterpret_cast<const float4 *>(part)[2];
     const float p[QW_NT] = {p0.x, p0.y, p0.z, p0.w, p1.x, p1.y, p1.z, p1.w, p2.x, p2.y, p2.z, p2.w};
@@ -142,7 +145,7 @@ __device__ __forceinline__ void qw_norm_image(const float *x, const float (&nw)[
     const int warp = tid >> 5, lane = tid & 31;
     for (int g = tid; g < d / 4; g += QG_THREADS) reinterpret_cast<float4 *>(xf)[g] = reinterpret_cast<const float4 *>(x)[g];
     __syncthreads();
-    const float inv = qw_norm_inv(xf, d, eps, part, tid);
+    const float inv = qw_norm_inv(xf, d, eps, part, tid, []() {});
     if (warp < d / 256) {
         float v[8];
         qw_load8(xf + warp * 256 + lane * 8, v);
@@ -559,21 +562,23 @@ __global__ void __launch_bounds__(QH_THREADS) qw_hint_kernel(QHintArgs a) {
     if (sb < d / 256) qw_load8(a.norm_w + sb * 256 + lane * 8, nw);
     pdl_wait_cta();
     pdl_trigger();
-    float dot = 0.0f;
+    float4 x[QH_MAXG];
 #pragma unroll
     for (int p = 0; p < QH_MAXG; p++) {
         const int g = tid + p * QH_THREADS;
-        if (g < groups) {
-            const float4 x = reinterpret_cast<const float4 *>(a.x)[g];
-            reinterpret_cast<float4 *>(xf)[g] = x;
-            dot += w[p].x * x.x + w[p].y * x.y + w[p].z * x.z + w[p].w * x.w;
-        }
+        x[p] = g < groups ? reinterpret_cast<const float4 *>(a.x)[g] : make_float4(0.f, 0.f, 0.f, 0.f);
     }
 #pragma unroll
-    for (int o = 16; o > 0; o >>= 1) dot += __shfl_xor_sync(0xffffffffu, dot, o);
-    if (lane == 0) red[warp] = dot;
+    for (int p = 0; p < QH_MAXG; p++) if (tid + p * QH_THREADS < groups) reinterpret_cast<float4 *>(xf)[tid + p * QH_THREADS] = x[p];
     __syncthreads();
-    const float inv = qw_norm_inv(xf, d, a.eps, part, tid);
+    float dot = 0.0f;            // beside the norm's chains, which the twelve threads of warp 0 begin with
+    const float inv = qw_norm_inv(xf, d, a.eps, part, tid, [&]() {
+#pragma unroll
+        for (int p = 0; p < QH_MAXG; p++) dot += w[p].x * x[p].x + w[p].y * x[p].y + w[p].z * x[p].z + w[p].w * x[p].w;
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) dot += __shfl_xor_sync(0xffffffffu, dot, o);
+        if (lane == 0) red[warp] = dot;
+    });
     if (tid == 0) a.est[e] = inv * (red[0] + red[1] + red[2] + red[3]);
     for (int b = sb; b < d / 256; b += gridDim.x * (QH_THREADS / 32)) {
         float v[8];
@@ -636,10 +641,10 @@ __global__ void __launch_bounds__(QG_THREADS, 2) qw_gate_up_kernel(const __grid_
         if ((tid & 3) == 0) mbar_expect_tx(&bar[grp], (uint32_t)cnt * (uint32_t)(a.stride_g + a.stride_u));
     }
     pdl_wait_cta();
-    pdl_trigger();
     if (a.est) qw_select(a.est, a.ne, a.topk, a.state, ws, sel, tid);
     else { if (tid < a.topk) sel[tid] = a.top[tid]; __syncthreads(); }
     if (tid < 4 * groups && run > 0) bulk_g2s(dst, src + (size_t)sel[slot] * expert_bytes, bytes, &bar[grp]);
+    pdl_trigger();           // only now: the down projection fetches its rows at once, and these come first
     waiter.poison_if_failed();
     // the activation from global memory (L1 after the first warp)
     const uint32_t rg0 = smem_u32(rg), ru0 = smem_u32(ru);
