@@ -14,6 +14,9 @@
 #include <string>
 #include <unordered_map>
 #include <vector>
+#ifdef __SSE2__
+#include <emmintrin.h>
+#endif
 
 namespace {
 
@@ -149,7 +152,7 @@ extern "C" uint32_t brrr_sample_logits(const float *logits, uint32_t n, uint32_t
     size_t k = top_k < 1 ? 1 : (top_k > 64 ? 64 : top_k);
     std::vector<std::pair<float, uint32_t>> top;
     top.reserve(k + 1);
-    for (uint32_t i = 0; i < n; i++) {
+    auto take = [&](uint32_t i) {
         float l = logits[i];
         if (top.size() < k || l > top.back().first) {
             size_t pos = 0;                                 // partition_point(|v| v > l)
@@ -157,7 +160,20 @@ extern "C" uint32_t brrr_sample_logits(const float *logits, uint32_t n, uint32_t
             top.insert(top.begin() + pos, std::make_pair(l, i));
             if (top.size() > k) top.pop_back();
         }
+    };
+    uint32_t i = 0;
+    for (; i < n && top.size() < k; i++) take(i);
+#ifdef __SSE2__
+    // sixteen at a time: nearly all of them hold nothing above the smallest kept logit, which only rises
+    for (; i + 16 <= n; i += 16) {
+        const __m128 least = _mm_set1_ps(top.back().first);
+        const __m128 a = _mm_or_ps(_mm_cmpgt_ps(_mm_loadu_ps(logits + i), least), _mm_cmpgt_ps(_mm_loadu_ps(logits + i + 4), least));
+        const __m128 b = _mm_or_ps(_mm_cmpgt_ps(_mm_loadu_ps(logits + i + 8), least), _mm_cmpgt_ps(_mm_loadu_ps(logits + i + 12), least));
+        if (_mm_movemask_ps(_mm_or_ps(a, b)))
+            for (uint32_t j = i; j < i + 16; j++) take(j);
     }
+#endif
+    for (; i < n; i++) take(i);
     const float mx = top[0].first;
     std::vector<float> probs(top.size());
     float sum = 0.0f;

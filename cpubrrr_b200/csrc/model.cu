@@ -103,6 +103,8 @@ size_t type_bytes(uint32_t type, size_t nel) {
 
 }  // namespace
 
+constexpr size_t LOGIT_CHUNK = 1 << 16, LOGIT_SLOTS = 16;      // floats per chunk, chunks of the pinned ring
+
 struct brrr_model {
     brrr_cfg cfg{};
     int device = 0;
@@ -121,6 +123,8 @@ struct brrr_model {
     DevState *st = nullptr;
     // host staging (pinned)
     uint32_t *h_in = nullptr, *h_out = nullptr;
+    float *h_logits = nullptr;                     // pinned ring through which logits leave (fetch_logits)
+    cudaEvent_t ev_logits[LOGIT_SLOTS] = {};
     cudaGraphExec_t g_head = nullptr, g_nohead = nullptr;            // speculative-routing step (or plain when disabled)
     cudaGraphExec_t g_head_safe = nullptr, g_nohead_safe = nullptr;  // plain step, used to redo a missed speculation
     cudaStream_t side = nullptr;                                     // the exact router runs here, beside gate/up
@@ -570,6 +574,8 @@ int build_model(brrr_model *m, const Source &src) {
     CU(cudaMemsetAsync(m->st, 0, sizeof(DevState), m->stream));
     CU(cudaMemsetAsync(m->x, 0, d * 4, m->stream));
     CU(cudaMallocHost(&m->h_in, 16));
+    CU(cudaMallocHost(&m->h_logits, LOGIT_SLOTS * LOGIT_CHUNK * sizeof(float)));
+    for (cudaEvent_t &e : m->ev_logits) CU(cudaEventCreateWithFlags(&e, cudaEventDisableTiming));
     CU(cudaMallocHost(&m->h_out, BRRR_MAXSEQ * sizeof(uint32_t)));
     CU(cudaStreamSynchronize(m->stream));
     if (m->ep) {
@@ -781,6 +787,8 @@ extern "C" void brrr_model_close(brrr_model *m) {
     if (m->ep_buf) cudaFree(m->ep_buf);
     for (void *p : m->allocs) cudaFree(p);
     if (m->h_in) cudaFreeHost(m->h_in);
+    if (m->h_logits) cudaFreeHost(m->h_logits);
+    for (cudaEvent_t e : m->ev_logits) if (e) cudaEventDestroy(e);
     if (m->h_tile) cudaFreeHost(m->h_tile);
     for (auto &gs : m->g_rows) for (cudaGraphExec_t g : gs) if (g) cudaGraphExecDestroy(g);
     if (m->h_out) cudaFreeHost(m->h_out);
@@ -1064,6 +1072,25 @@ static int batch_check(brrr_model *m, int n, const uint32_t *toks, const uint32_
 // Rows from which the vocabulary projection of a batch runs on the tensor cores.
 constexpr int HEAD_TENSOR_FROM = 5;
 
+// n floats from the device to the caller's memory, in chunks through a pinned ring: the copy of a chunk to pageable memory by this thread runs
+// beside the next chunks' transfers (a transfer straight to pageable memory is staged by the driver, one piece after the other).
+static int fetch_logits(brrr_model *m, float *out, const float *dev, size_t n) {
+    const size_t chunks = (n + LOGIT_CHUNK - 1) / LOGIT_CHUNK;
+    for (size_t i = 0; i < chunks + LOGIT_SLOTS; i++) {
+        if (i >= LOGIT_SLOTS && i - LOGIT_SLOTS < chunks) {
+            const size_t k = i - LOGIT_SLOTS, at = k * LOGIT_CHUNK;
+            CU(cudaEventSynchronize(m->ev_logits[k % LOGIT_SLOTS]));
+            memcpy(out + at, m->h_logits + (k % LOGIT_SLOTS) * LOGIT_CHUNK, std::min(LOGIT_CHUNK, n - at) * sizeof(float));
+        }
+        if (i < chunks) {
+            const size_t at = i * LOGIT_CHUNK;
+            CU(cudaMemcpyAsync(m->h_logits + (i % LOGIT_SLOTS) * LOGIT_CHUNK, dev + at, std::min(LOGIT_CHUNK, n - at) * sizeof(float), cudaMemcpyDeviceToHost, m->stream));
+            CU(cudaEventRecord(m->ev_logits[i % LOGIT_SLOTS], m->stream));
+        }
+    }
+    return BRRR_OK;
+}
+
 // The layers for n rows on the sequences' caches; with out_toks, the vocabulary projection and argmax of every row.
 static int batch_rows(brrr_model *m, int n, const uint32_t *toks, const uint32_t *pos, const uint32_t *seq, uint32_t *out_toks, float *out_logits,
                       int kind = ROWS_BATCH) {
@@ -1081,9 +1108,9 @@ static int batch_rows(brrr_model *m, int n, const uint32_t *toks, const uint32_t
         launch_rows_argmax(m->bt_logits, c.n_vocab, n, m->bt_tok, s);
         CU(cudaGetLastError());
         CU(cudaMemcpyAsync(m->h_out + 8, m->bt_tok, (size_t)n * 4, cudaMemcpyDeviceToHost, s));
-        if (out_logits) CU(cudaMemcpyAsync(out_logits, m->bt_logits, (size_t)n * c.n_vocab * sizeof(float), cudaMemcpyDeviceToHost, s));
     }
     CU(cudaMemcpyAsync(m->h_out, m->st, 32, cudaMemcpyDeviceToHost, s));
+    if (out_logits) TRY(fetch_logits(m, out_logits, m->bt_logits, (size_t)n * c.n_vocab));
     CU(cudaStreamSynchronize(s));
     if (m->h_out[6] != 0) { snprintf(g_cuda_err, sizeof g_cuda_err, "device wait timed out (code %u)", m->h_out[6]); return BRRR_ERR_STATE; }
     if (out_toks) for (int t = 0; t < n; t++) out_toks[t] = m->h_out[8 + t];
@@ -1168,9 +1195,7 @@ extern "C" int brrr_decode(brrr_model *m, uint32_t first_tok, uint32_t pos, uint
 extern "C" int brrr_logits(brrr_model *m, float *out) {
     if (!m || !out) return BRRR_ERR_ARG;
     CU(cudaSetDevice(m->device));
-    CU(cudaMemcpyAsync(out, m->logits, (size_t)m->cfg.n_vocab * 4, cudaMemcpyDeviceToHost, m->stream));
-    CU(cudaStreamSynchronize(m->stream));
-    return BRRR_OK;
+    return fetch_logits(m, out, m->logits, (size_t)m->cfg.n_vocab);
 }
 
 extern "C" int brrr_hidden(brrr_model *m, float *out) {
