@@ -97,6 +97,23 @@ def test_batch_ragged_and_mixed_rows(brrr):
     eng.close()
 
 
+@pytest.mark.parametrize("n", [1, 3, 30])
+def test_batch_logits_longer_than_the_pinned_ring(brrr, n):
+    """Logits leave in 65536-float chunks through a ring of sixteen: less than one chunk, a few, and more than the ring holds."""
+    cfg = brrr.make_cfg(128, 1, 4, 2, 8, 4, 48000, sliding_window=8)
+    eng = brrr.Engine.synth(cfg, 33)
+    toks = [1 + 1571 * i for i in range(n)]
+    want = []
+    for t in toks:
+        tok = eng.run(t, 0, True)
+        want.append((tok, eng.logits().copy()))
+    eng.batch_open(n)
+    out, lg = eng.batch_step(toks, [0] * n, list(range(n)), logits=True)
+    for i in range(n):
+        assert int(out[i]) == want[i][0] and np.array_equal(bits(lg[i]), bits(want[i][1])), f"row {i}"
+    eng.close()
+
+
 def test_batch_bad_args(brrr):
     cfg = brrr.make_cfg(64, 1, 2, 1, 4, 2, 256)
     eng = brrr.Engine.synth(cfg, 23)

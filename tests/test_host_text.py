@@ -108,6 +108,20 @@ def test_sampler_matches_reference(L, orc):
         assert L.brrr_sample_logits(few.ctypes.data_as(C.c_void_p), 3, 1000, 40, C.byref(st)) == want
 
 
+@pytest.mark.parametrize("n", [39, 40, 41, 55, 56, 57, 72, 1000, 1003])
+def test_sampler_group_edges(L, orc, n):
+    """Sizes around the first k logits and the groups of sixteen after them; rising, falling and random logits with ties."""
+    from oracle import oracle_host as H
+    rng = np.random.default_rng(n)
+    rnd = np.round(rng.standard_normal(n) * 4).astype(np.float32) / 2
+    for logits in (rnd, np.sort(rnd), np.sort(rnd)[::-1].copy()):
+        st_o = H.rng_seed(n)
+        st = C.c_uint64(st_o)
+        for _ in range(12):
+            want, st_o = H.sample_logits(logits, 1500, 40, st_o)
+            assert L.brrr_sample_logits(logits.ctypes.data_as(C.c_void_p), n, 1500, 40, C.byref(st)) == want and st.value == st_o
+
+
 def test_serve_line_parser(L, orc):
     from oracle import oracle_host as H
     buf = C.create_string_buffer(4096)
