@@ -539,7 +539,7 @@ cudaError_t tl_launch(TileArgs a, int tiles, int entries, int experts, bool pdl,
     const int full_chunks = entries / nt, tasks = full_chunks + experts < entries ? full_chunks + experts : entries;
     const dim3 grid(tiles, tasks);
     cudaError_t ce;
-        if (nt == 32) {
+    if (nt == 32) {
         if ((ce = smem_optin(tile_kernel<KIND, 32>, 220 * 1024, configured[0])) != cudaSuccess) return ce;
         return launch_k(tile_kernel<KIND, 32>, grid, dim3(32 * 16 + 128), tl_smem<KIND, 32>(a.np), st, pdl, a);
     }
