@@ -92,7 +92,7 @@ struct brrr_qwen {
     cudaGraphExec_t g_head_safe = nullptr, g_nohead_safe = nullptr;  // routing in the chain; redoes a missed speculation
     bool use_spec = true;
     bool spec_off = false;               // a bounded device wait of the speculative step ran out once
-    uint64_t spec_redos = 0;
+    uint64_t spec_redos = 0, wait_fallbacks = 0;
     uint32_t run_tok = 0, run_pos = 0;   // of the decode run in flight
     uint32_t test_hooks = 0;
     int launches_head = 0, launches_nohead = 0;
@@ -535,6 +535,9 @@ extern "C" int brrr_qwen_cfg_get(const brrr_qwen *m, brrr_qwen_cfg *out) {
     return BRRR_OK;
 }
 
+extern "C" uint64_t brrr_qwen_spec_redos(const brrr_qwen *m) { return m ? m->spec_redos : 0; }
+extern "C" uint64_t brrr_qwen_wait_fallbacks(const brrr_qwen *m) { return m ? m->wait_fallbacks : 0; }
+
 extern "C" int brrr_qwen_launches_per_step(const brrr_qwen *m, int want) { return m ? (want ? m->launches_head : m->launches_nohead) : 0; }
 
 // Algorithmic bytes one decode step at position pos must read: the K-quant rows it touches, the
@@ -567,6 +570,7 @@ static bool qrecover(brrr_qwen *m, uint32_t err) {
     if (err != (uint32_t)DEV_ERR_PEER_TIMEOUT || !m->g_head || m->spec_off) return false;
     if (cudaMemsetAsync(&m->st->err, 0, 4, m->stream) != cudaSuccess) return false;
     m->spec_off = true;
+    m->wait_fallbacks++;
     return true;
 }
 

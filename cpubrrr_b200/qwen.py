@@ -103,5 +103,13 @@ class QwenEngine:
     def launches_per_step(self, want=True):
         return lib().brrr_qwen_launches_per_step(self._h, int(bool(want)))
 
+    def spec_redos(self):
+        """Steps run again because the routing estimate missed an expert or a wait ran out (performance counter)."""
+        return int(lib().brrr_qwen_spec_redos(self._h))
+
+    def wait_fallbacks(self):
+        """Times the bounded wait for the exact routing ran out and the model gave up speculation (0 or 1)."""
+        return int(lib().brrr_qwen_wait_fallbacks(self._h))
+
     def bytes_per_step(self, pos):
         return int(lib().brrr_qwen_bytes_per_step(self._h, int(pos)))

@@ -262,6 +262,10 @@ int brrr_qwen_hidden(brrr_qwen *m, float *out);               /* [n_embd], resid
 int brrr_qwen_forward_trace(brrr_qwen *m, uint32_t tok, uint32_t pos, float *trace);
 void *brrr_qwen_stream(brrr_qwen *m);
 int brrr_qwen_launches_per_step(const brrr_qwen *m, int want_logits);
+/* Steps that were run again because the routing estimate missed an expert or a wait ran out, and waits that ran out
+ * (0 or 1; the model then decodes without speculation): as brrr_model_spec_redos and brrr_model_wait_fallbacks. */
+uint64_t brrr_qwen_spec_redos(const brrr_qwen *m);
+uint64_t brrr_qwen_wait_fallbacks(const brrr_qwen *m);
 uint64_t brrr_qwen_bytes_per_step(const brrr_qwen *m, uint32_t pos);
 
 /* ChatML prompt ids of the qwen3moe engine: im_start "system\nYou are a helpful assistant." im_end im_start

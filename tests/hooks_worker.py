@@ -3,7 +3,7 @@
 default build, which contains no hook.  No GPU fault is provoked: a missed speculation is a
 flagged step, a silent router is a bounded wait that runs out and is reported.
 
-    python tests/hooks_worker.py sabotage | mute
+    python tests/hooks_worker.py sabotage | mute | qwen_sabotage | qwen_mute
 """
 import os
 import sys
@@ -27,8 +27,72 @@ def greedy(run, prompt, n):
     return out
 
 
+def qwen(mode):
+    """The same two failures in the qwen3moe engine: a missed expert and a silent router, through host-driven steps
+    (brrr_qwen_forward) and through the device-chained run (brrr_qwen_decode_wait)."""
+    import cpubrrr_b200 as B
+    from cpubrrr_b200 import synth as S
+    from oracle import oracle as O
+    bits = lambda a: np.ascontiguousarray(a, dtype=np.float32).view(np.uint32)
+    shape = dict(n_embd=512, n_layer=3, n_head=8, n_head_kv=2, n_expert=40, n_expert_used=8, n_ff_exp=768, n_vocab=515)
+    cfg = B.make_qwen_cfg(**shape)
+    om = O.QwenModel.synth(O.make_qcfg(d=512, nh=8, nkv=2, hd=128, nl=3, ne=40, topk=8, ff=768, nvocab=515), 17)
+    prompt = S.synth_prompt(17, 9, cfg.n_vocab)
+    want = greedy(om.run, prompt, 40)          # positions 0 .. 48
+
+    def check(eng):
+        assert np.array_equal(bits(eng.logits()), bits(om.logits())) and np.array_equal(bits(eng.hidden()), bits(om.hidden()))
+
+    def hooked(var):
+        os.environ[var] = "1"
+        eng = B.QwenEngine.synth(cfg, 17)
+        del os.environ[var]
+        return eng
+
+    def chained(eng):
+        first = eng.prefill(prompt)            # token rows: no speculation in it
+        toks = eng.decode(first, len(prompt), 40)
+        assert [first] + [int(t) for t in toks[:-1]] == want
+        check(eng)
+
+    if mode == "qwen_sabotage":
+        # the estimate is spoiled where the position is a multiple of three: exactly those steps run twice
+        eng = hooked("BRRR_SPEC_SABOTAGE")
+        assert greedy(eng.run, prompt, 40) == want
+        check(eng)
+        assert (eng.spec_redos(), eng.wait_fallbacks()) == (17, 0)         # 0, 3 .. 48
+        chained(eng)
+        assert (eng.spec_redos(), eng.wait_fallbacks()) == (17 + 14, 0)    # 9, 12 .. 48
+        clean = B.QwenEngine.synth(cfg, 17)
+        assert greedy(clean.run, prompt, 40) == want
+        check(clean)
+        chained(clean)
+        assert (clean.spec_redos(), clean.wait_fallbacks()) == (0, 0)
+        clean.close()
+    else:
+        # the router never publishes: the first combine's wait (about a second) runs out, the step runs again with the routing
+        # in the chain, and the model does without speculation from there on
+        eng = hooked("BRRR_ROUTER_MUTE")
+        assert greedy(eng.run, prompt, 40) == want
+        check(eng)
+        chained(eng)
+        assert (eng.spec_redos(), eng.wait_fallbacks()) == (1, 1)
+        eng.close()
+        eng = hooked("BRRR_ROUTER_MUTE")       # the same, met inside a device-chained run first
+        chained(eng)
+        assert (eng.spec_redos(), eng.wait_fallbacks()) == (1, 1)
+        assert greedy(eng.run, prompt, 40) == want
+        assert (eng.spec_redos(), eng.wait_fallbacks()) == (1, 1)
+    eng.close()
+    om.close()
+
+
 def main(mode):
     assert os.environ.get("BRRR_LIBRARY", "").endswith("libbrrr_hooks.so")
+    if mode.startswith("qwen"):
+        qwen(mode)
+        print("hooks_worker ok:", mode)
+        return
     import cpubrrr_b200 as B
     from cpubrrr_b200 import synth as S
     from oracle import oracle as O

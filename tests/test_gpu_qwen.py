@@ -142,6 +142,19 @@ def test_qwen_mixed_kquant_types_per_tensor(brrr, orc, tmp_path):
     eng.close(); plain.close(); om.close()
 
 
+@pytest.mark.parametrize("mode", ["qwen_sabotage", "qwen_mute"])
+def test_qwen_speculation_recovers(brrr, mode):
+    """A step whose estimate missed an expert, and one whose exact router stays silent, run again without the estimate: results
+    are the oracle's and the counters name the steps (test-hook build of the library, tests/hooks_worker.py)."""
+    import subprocess
+    import sys
+    from cpubrrr_b200 import build
+    env = dict(os.environ, BRRR_LIBRARY=build.build_hooks())
+    worker = os.path.join(os.path.dirname(GOLD), "hooks_worker.py")
+    r = subprocess.run([sys.executable, worker, mode], env=env, capture_output=True, text=True, timeout=600)
+    assert r.returncode == 0 and "hooks_worker ok" in r.stdout, r.stdout[-2000:] + r.stderr[-4000:]
+
+
 def test_qwen_open_errors(brrr, tmp_path):
     import ctypes as C
     L = brrr.lib()
