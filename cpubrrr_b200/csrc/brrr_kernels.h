@@ -57,6 +57,14 @@ cudaError_t launch_qw_gate_up(const KMatDev &gate, const KMatDev &up, const floa
                               const int32_t *b16, float *hbuf, DevState *state, bool pdl, cudaStream_t st);
 cudaError_t launch_qw_down(const KMatDev &down, const float *est, const int32_t *top, const float *wts, uint32_t seq, int ne, int topk, int d, int ff, const float *hbuf,
                            float *x, DevState *state, bool pdl, cudaStream_t st);
+// Whether the exact router of a layer always finds room beside the CTAs that wait for its words: this layer's down projection and the next layer's
+// q|k|v (next_qkv: three matrices; null behind the last layer).  Not ok: down has to be enqueued behind the router's end.
+struct QwRoom {
+    int down_ctas, next_ctas;
+    size_t down_smem, next_smem, router_smem;
+    bool ok;
+};
+QwRoom qw_router_room(const KMatDev &down, const KMatDev *next_qkv, int ne, int topk, int d, int ff);
 cudaError_t launch_qw_head(const KMatDev &head, const int8_t *q, const float *s, const int32_t *b16, float *logits, DevState *state, bool pdl, cudaStream_t st);
 // Q6_K rows from the GGUF layout (210-byte superblocks) into the aligned planes of KMatDev (planes = 1)
 void launch_q6k_planes(const uint8_t *src, size_t rows, int cols, uint8_t *dst, cudaStream_t st);
@@ -206,6 +214,8 @@ cudaError_t launch_ffn_in(const float *x_in, const float *norm_w, float eps, int
                           float *logits, int32_t *top, float *wts, unsigned int *counter, DevState *state, bool pdl, cudaStream_t st,
                           int ntok = 1, uint32_t *signal = nullptr, int qwen_norm = 0, int8_t *q8k_q = nullptr, float *q8k_s = nullptr,
                           int32_t *q8k_b16 = nullptr);
+size_t ffn_in_smem(int ne, int d);        // dynamic shared memory of one of its CTAs
+bool ffn_in_takes_half_an_sm();           // its registers, as built: no more than that
 // ntok > 1: a tile of tokens in one launch (token t reads x_in + t * d, writes logits + t * ne, top + 8 t, wts + 8 t, uses counter + t)
 // signal (nullable, ntok == 1): a device word the kernel increments after its routing is written, for a
 // consumer that runs beside it instead of after it (launch_fold_norm)

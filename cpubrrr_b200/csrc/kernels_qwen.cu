@@ -862,13 +862,30 @@ __global__ void q6k_planes_kernel(const uint8_t *__restrict__ src, size_t rows, 
 int qw_passes(int nsb) { return nsb <= 8 ? 1 : nsb <= 16 ? 2 : 0; }
 size_t qw_act_bytes(int nsb) { return (size_t)nsb * 4 * KQ_SM_CHUNK + (size_t)((nsb + 3) & ~3) * 4 + (size_t)nsb * 64; }
 bool qw_type_ok(const KMatDev &m) { return m.type == 12 || (m.type == 14 && m.planes); }
-// An even share of 140 SMs, unless that takes more shared memory than two kernels can share.  Two such kernels, one of them waiting for
-// the router's words, then never fill the 148 SMs' registers and shared memory: the router's CTAs always find room.
+// An even share of 140 SMs, unless that takes more shared memory than two kernels can share.
 int qw_rows_per_cta(int rows, size_t bytes_per_row) {
     const int share = (rows + 139) / 140, fit = (int)(QG_ROW_BYTES / bytes_per_row);
     return share < fit ? share : fit;
 }
 constexpr int QG_SMEM_MAX = 200 * 1024;
+
+struct QwPlan { int per_cta, ctas; size_t smem; };
+// a stack of `rows` rows, `stride` bytes apart in shared memory, against one activation of nsb superblocks
+QwPlan qw_gemv_plan(int rows, size_t stride, int nsb, bool norm) {
+    const int per = qw_rows_per_cta(rows, stride + nsb * 4);
+    return {per, (rows + per - 1) / per, (size_t)per * (stride + nsb * 4) + qw_act_bytes(nsb) + (norm ? (size_t)nsb * 1024 : 0)};
+}
+QwPlan qw_down_plan(const KMatDev &down, int topk, int d, int ff) {
+    const int nun = topk * (ff / 256);
+    const size_t row = (size_t)topk * down.bpr() + nun * 4 + topk * 4;
+    const int per = qw_rows_per_cta(d, row);
+    return {per, (d + per - 1) / per, per * row + qw_act_bytes(nun)};
+}
+size_t qw_stack_stride(const KMatDev *mats, int n) {
+    size_t stride = 0;
+    for (int i = 0; i < n; i++) if (mats[i].bpr() > stride) stride = mats[i].bpr();
+    return stride;
+}
 
 template <int PASSES, bool NORM>
 cudaError_t qw_gemv_launch(const QGemvArgs &a, size_t smem, bool pdl, cudaStream_t st) {
@@ -881,20 +898,18 @@ cudaError_t qw_gemv_launch(const QGemvArgs &a, size_t smem, bool pdl, cudaStream
 cudaError_t qw_gemv(const KMatDev *mats, float *const *ys_out, int n, const float *x, const float *norm_w, float eps, DevState *state, bool pdl, cudaStream_t st) {
     QGemvArgs a{};
     a.k.n = n;
-    size_t stride = 0;
     for (int i = 0; i < n; i++) {
         a.k.m[i] = mats[i]; a.k.y[i] = ys_out[i]; a.k.rows += mats[i].rows;
-        if (mats[i].bpr() > stride) stride = mats[i].bpr();
         if (mats[i].cols != mats[0].cols || !qw_type_ok(mats[i])) return cudaErrorInvalidValue;
     }
-    const int K = mats[0].cols, nsb = K / 256, passes = qw_passes(nsb);
+    const int nsb = mats[0].cols / 256, passes = qw_passes(nsb);
     if (!passes) return cudaErrorInvalidValue;
-    a.k.stride = (int)stride;
-    a.k.per_cta = qw_rows_per_cta(a.k.rows, stride + nsb * 4);
+    a.k.stride = (int)qw_stack_stride(mats, n);
+    const QwPlan p = qw_gemv_plan(a.k.rows, a.k.stride, nsb, norm_w != nullptr);
+    a.k.per_cta = p.per_cta;
     a.x = x; a.norm_w = norm_w; a.eps = eps; a.state = state;
-    const size_t smem = (size_t)a.k.per_cta * (stride + nsb * 4) + qw_act_bytes(nsb) + (norm_w ? (size_t)K * 4 : 0);
-    if (norm_w) return passes == 1 ? qw_gemv_launch<1, true>(a, smem, pdl, st) : qw_gemv_launch<2, true>(a, smem, pdl, st);
-    return passes == 1 ? qw_gemv_launch<1, false>(a, smem, pdl, st) : qw_gemv_launch<2, false>(a, smem, pdl, st);
+    if (norm_w) return passes == 1 ? qw_gemv_launch<1, true>(a, p.smem, pdl, st) : qw_gemv_launch<2, true>(a, p.smem, pdl, st);
+    return passes == 1 ? qw_gemv_launch<1, false>(a, p.smem, pdl, st) : qw_gemv_launch<2, false>(a, p.smem, pdl, st);
 }
 
 template <int PASSES>
@@ -964,14 +979,32 @@ cudaError_t launch_qw_gate_up(const KMatDev &gate, const KMatDev &up, const floa
 cudaError_t launch_qw_down(const KMatDev &down, const float *est, const int32_t *top, const float *wts, uint32_t seq, int ne, int topk, int d, int ff, const float *hbuf,
                            float *x, DevState *state, bool pdl, cudaStream_t st) {
     if (!qw_type_ok(down) || ff % 256 || ff > 1024 || topk > 8 || ne > 256) return cudaErrorInvalidValue;
-    QDownArgs a{down, est, top, wts, seq, ne, topk, d, ff, 0, hbuf, x, state};
-    const int nun = topk * (ff / 256);
-    const size_t row = (size_t)topk * down.bpr() + nun * 4 + topk * 4;
-    a.per_cta = qw_rows_per_cta(d, row);
+    const QwPlan p = qw_down_plan(down, topk, d, ff);
+    QDownArgs a{down, est, top, wts, seq, ne, topk, d, ff, p.per_cta, hbuf, x, state};
     static unsigned long long configured = 0;      // one bit per device
     cudaError_t e = smem_optin(qw_down_kernel, QG_SMEM_MAX, configured);
     if (e != cudaSuccess) return e;
-    return launch_k(qw_down_kernel, dim3((d + a.per_cta - 1) / a.per_cta), dim3(QD_THREADS), a.per_cta * row + qw_act_bytes(nun), st, pdl, a);
+    return launch_k(qw_down_kernel, dim3(p.ctas), dim3(QD_THREADS), p.smem, st, pdl, a);
+}
+
+// The kernels that can be on the SMs while the exact router has not published are the down projection, whose CTAs poll for its words, and the
+// q|k|v projection behind it, whose CTAs wait for down's (what comes after q|k|v is launched only once down has ended, and gate/up and the
+// hint end by themselves).  If an SM with one of their CTAs still takes a router CTA, an SM that refuses one holds two; with fewer
+// than two per SM in all, some SM always has room and the router ends.  Registers and threads allow it (half an SM at most for
+// either: launch bounds, ffn_in_takes_half_an_sm); shared memory decides.  Where this does not hold - rows of 4096 values, say, where the router alone takes 133 KB - the down
+// projection must not start before the router has ended (a graph edge instead of the poll's bounded second).  One decoding
+// engine per device is assumed; the kernels of others can only run the bounded wait out.
+QwRoom qw_router_room(const KMatDev &down, const KMatDev *next_qkv, int ne, int topk, int d, int ff) {
+    constexpr size_t SM_SMEM = 228 * 1024, CTA_EXTRA = 3 * 1024;       // CTA_EXTRA: the system's 1 KB and the kernels' static variables
+    constexpr int SMS = 148;
+    const QwPlan dn = qw_down_plan(down, topk, d, ff);
+    // behind the last layer: the one CTA of the output norm
+    const QwPlan nx = next_qkv ? qw_gemv_plan(next_qkv[0].rows + next_qkv[1].rows + next_qkv[2].rows, qw_stack_stride(next_qkv, 3), d / 256, true) : QwPlan{1, 1, (size_t)d * 4};
+    QwRoom r{dn.ctas, nx.ctas, dn.smem, nx.smem, ffn_in_smem(ne, d), false};
+    const size_t waiting = dn.smem > nx.smem ? dn.smem : nx.smem;
+    const int per_sm = waiting + r.router_smem + 2 * CTA_EXTRA <= SM_SMEM ? 2 : 1;
+    r.ok = dn.ctas + nx.ctas < per_sm * SMS;
+    return r;
 }
 
 cudaError_t launch_qw_head(const KMatDev &head, const int8_t *q, const float *s, const int32_t *b16, float *logits, DevState *state, bool pdl, cudaStream_t st) {

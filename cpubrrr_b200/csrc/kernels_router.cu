@@ -408,15 +408,24 @@ static cudaError_t router_rows_launch(const RouterArgs &a, int ntok, bool pdl, c
     return launch_k(router_rows_kernel<TPW>, dim3((a.ne + 31) / 32, (ntok + TT - 1) / TT), dim3(RR_WARPS * 32), smem, st, pdl, a, ntok);
 }
 
+// (A check and no launch bound: a bound changes the code the compiler makes of the chain, and every router launch runs it.)
+bool ffn_in_takes_half_an_sm() {
+    cudaFuncAttributes at;
+    return cudaFuncGetAttributes(&at, ffn_in_kernel) == cudaSuccess && at.numRegs * RT_THREADS <= 32768;
+}
+static int ffn_in_epc(int ne) { return ne > 32 ? 16 : 32; }
+static int ffn_in_stages(int ne) { return ne > 32 ? 6 : RT_STAGES; }
+size_t ffn_in_smem(int ne, int d) { return (size_t)ffn_in_epc(ne) * RT_STRIDE * 4 * ffn_in_stages(ne) + (size_t)d * 8 + (size_t)((ne + 3) & ~3) * 4 + ffn_in_stages(ne) * 16; }
+
 size_t router_packed_floats(int ne, int d) { return (size_t)((ne + 31) / 32) * ((d + RT_TJ - 1) / RT_TJ) * RT_TILE_FLOATS; }
 
 cudaError_t launch_ffn_in(const float *x_in, const float *norm_w, float eps, int d, const float *Wt, const float *b, int ne, int topk,
                           float *logits, int32_t *top, float *wts, unsigned int *counter, DevState *state, bool pdl, cudaStream_t st, int ntok,
                           uint32_t *signal, int qwen_norm, int8_t *q8k_q, float *q8k_s, int32_t *q8k_b16) {
     RouterArgs a{x_in, norm_w, eps, d, Wt, b, ne, topk, logits, top, wts, counter, state, signal, (signal && state) ? state->route_pub : nullptr,
-                 qwen_norm, q8k_q, q8k_s, q8k_b16, ne > 32 ? 16 : 32, ne > 32 ? 6 : RT_STAGES};
+                 qwen_norm, q8k_q, q8k_s, q8k_b16, ffn_in_epc(ne), ffn_in_stages(ne)};
     if (signal && !state) return cudaErrorInvalidValue;
-    size_t smem = (size_t)a.epc * RT_STRIDE * 4 * a.stages + (size_t)d * 8 + (size_t)((ne + 3) & ~3) * 4 + a.stages * 16;
+    const size_t smem = ffn_in_smem(ne, d);
     static unsigned long long configured = 0;      // one bit per device
     {
         cudaError_t e = smem_optin(ffn_in_kernel, 200 * 1024, configured);

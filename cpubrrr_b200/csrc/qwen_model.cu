@@ -239,7 +239,14 @@ int qenqueue_step(brrr_qwen *m, bool want, float *trace_dev, int *nlaunch, bool 
                              m->xq, m->xs, m->xsum)); n++;
         }
         CU(launch_qw_gate_up(ly.gate, ly.up, est, m->top, ne, topk, ff, m->xq, m->xs, m->xsum, m->hbuf, m->st, pdl, s)); n++;
-        CU(launch_qw_down(ly.down, est, m->top, m->wts, (uint32_t)il + 1, ne, topk, d, ff, m->hbuf, m->x, m->st, pdl, s)); n++;
+        bool poll = true;        // down meets the router by its published words; where the router may find no room beside it, behind its end
+        if (spec) {
+            const QLayer *nx = il + 1 < c.n_layer ? &m->L[il + 1] : nullptr;
+            const KMatDev nqkv[3] = {nx ? nx->wq : KMatDev{}, nx ? nx->wk : KMatDev{}, nx ? nx->wv : KMatDev{}};
+            poll = qw_router_room(ly.down, nx ? nqkv : nullptr, ne, topk, d, ff).ok && ffn_in_takes_half_an_sm();
+            if (!poll) CU(cudaStreamWaitEvent(s, m->ev_join, 0));
+        }
+        CU(launch_qw_down(ly.down, est, m->top, m->wts, (uint32_t)il + 1, ne, topk, d, ff, m->hbuf, m->x, m->st, pdl && poll, s)); n++;
         if (trace_dev) CU(cudaMemcpyAsync(trace_dev + (size_t)(il + 1) * d, m->x, d * sizeof(float), cudaMemcpyDeviceToDevice, s));
     }
     if (want) {
@@ -695,3 +702,18 @@ extern "C" int brrr_qwen_forward_trace(brrr_qwen *m, uint32_t tok, uint32_t pos,
 }
 
 extern "C" void *brrr_qwen_stream(brrr_qwen *m) { return m ? (void *)m->stream : nullptr; }
+
+#ifdef BRRR_TEST_HOOKS
+// Test-hook builds only: the room rule of a layer of shape *cfg with q, k, v of type_qkv and down of type_down (host arithmetic only).
+// out: CTAs of down and of the next q|k|v, shared memory of a CTA of down, of q|k|v and of the router, 1 if down may poll.
+extern "C" int brrr_debug_qwen_room(const brrr_qwen_cfg *cfg, int type_qkv, int type_down, uint64_t *out) {
+    if (!cfg || !out || qcheck_cfg(*cfg) != BRRR_OK) return BRRR_ERR_ARG;
+    const int d = cfg->n_embd, hd = cfg->head_dim;
+    const KMatDev down{nullptr, type_down, cfg->n_expert * d, cfg->n_ff_exp, type_down == 14};
+    const KMatDev qkv[3] = {{nullptr, type_qkv, cfg->n_head * hd, d, type_qkv == 14}, {nullptr, type_qkv, cfg->n_head_kv * hd, d, type_qkv == 14},
+                            {nullptr, type_qkv, cfg->n_head_kv * hd, d, type_qkv == 14}};
+    const QwRoom r = qw_router_room(down, qkv, cfg->n_expert, cfg->n_expert_used, d, cfg->n_ff_exp);
+    out[0] = r.down_ctas; out[1] = r.next_ctas; out[2] = r.down_smem; out[3] = r.next_smem; out[4] = r.router_smem; out[5] = r.ok;
+    return BRRR_OK;
+}
+#endif

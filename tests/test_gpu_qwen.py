@@ -69,6 +69,26 @@ def test_qwen_tokens_logits_hidden_bit_exact(brrr, orc, shape):
     eng.close()
 
 
+@pytest.mark.parametrize("shape", [
+    dict(n_embd=2304, n_layer=2, n_head=4, n_head_kv=2, n_expert=33, n_expert_used=4, n_ff_exp=512, n_vocab=1003),      # nine superblocks: a second pass of one
+    dict(n_embd=4096, n_layer=3, n_head=8, n_head_kv=2, n_expert=40, n_expert_used=8, n_ff_exp=1024, n_vocab=700),      # down behind the router's end
+])
+def test_qwen_rows_wider_than_eight_superblocks(brrr, orc, shape):
+    """n_embd above 2048: the two-pass rows of q|k|v, gate/up and the head; no step is run again."""
+    cfg = brrr.make_qwen_cfg(**shape)
+    eng = brrr.QwenEngine.synth(cfg, 29)
+    om = orc.QwenModel.synth(ocfg_of(orc, cfg), 29)
+    prompt = S.synth_prompt(29, 5, cfg.n_vocab)
+    want = greedy(om.run, prompt, 12)
+    assert greedy(eng.run, prompt, 12) == want
+    assert np.array_equal(bits(eng.logits()), bits(om.logits())) and np.array_equal(bits(eng.hidden()), bits(om.hidden()))
+    first = eng.prefill(prompt)
+    assert [first] + [int(t) for t in eng.decode(first, len(prompt), 12)[:-1]] == want
+    assert np.array_equal(bits(eng.logits()), bits(om.logits())) and np.array_equal(bits(eng.hidden()), bits(om.hidden()))
+    assert (eng.spec_redos(), eng.wait_fallbacks()) == (0, 0)
+    eng.close(); om.close()
+
+
 def test_qwen_layer_trace_bit_exact(brrr, orc):
     cfg = brrr.make_qwen_cfg(512, 4, 4, 2, 16, 4, 256, 772)
     eng = brrr.QwenEngine.synth(cfg, 5)
