@@ -6,6 +6,7 @@
 #include "brrr_tile.cuh"
 
 #include <cstdio>
+#include <mutex>
 
 using namespace brrr;
 
@@ -13,7 +14,11 @@ namespace {
 int check_launch() { return cudaGetLastError() == cudaSuccess ? BRRR_OK : BRRR_ERR_CUDA; }
 }  // namespace
 
-struct brrr_q8mat { Q8Dev m; uint8_t *op; };      // op: operand units of the tensor-core product (token rows)
+struct brrr_q8mat {
+    Q8Dev m{};
+    mutable std::mutex lock;         // of op
+    mutable uint8_t *op = nullptr;   // operand units of the tensor-core product, made by the first call that wants them
+};
 struct brrr_mxmat { MxDev m; };
 
 extern "C" int brrr_quant_q8(const float *d_x, int n, int8_t *d_q, float *d_s, void *stream) {
@@ -78,10 +83,8 @@ extern "C" int brrr_q8mat_from_bf16(const uint16_t *d_w, int rows, int cols, brr
     brrr_q8mat *q = new brrr_q8mat();
     q->m.rows = rows; q->m.cols = cols;
     if (cudaMalloc(&q->m.data, q8_bytes(rows, cols)) != cudaSuccess) { delete q; return BRRR_ERR_NOMEM; }
-    if (cudaMalloc(&q->op, q8_operand_bytes(rows, cols)) != cudaSuccess) { cudaFree(q->m.data); delete q; return BRRR_ERR_NOMEM; }
     if (cudaMemsetAsync(q->m.data, 0, q8_bytes(rows, cols), (cudaStream_t)stream) != cudaSuccess) { brrr_q8mat_free(q); return BRRR_ERR_CUDA; }
     launch_q8_pack(d_w, rows, 0, q->m, (cudaStream_t)stream);
-    launch_q8_operand_pack(q->m, q->op, (cudaStream_t)stream);
     *out = q;
     return check_launch();
 }
@@ -105,6 +108,25 @@ extern "C" int brrr_q8_matvec(const brrr_q8mat *w, const int8_t *d_xq, const flo
     return check_launch();
 }
 
+// The matrix's operand units for a product on st: kept with the matrix once they exist (complete for every stream: the call that makes them
+// waits for its stream), else, inside a capture or where they do not fit, in stream-ordered scratch that the caller frees.
+static const uint8_t *q8mat_operand(const brrr_q8mat *w, cudaStream_t st, uint8_t **scratch) {
+    const size_t bytes = q8_operand_bytes(w->m.rows, w->m.cols);
+    std::lock_guard<std::mutex> g(w->lock);
+    if (w->op) return w->op;
+    cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
+    uint8_t *op = nullptr;
+    if (cudaStreamIsCapturing(st, &cap) == cudaSuccess && cap == cudaStreamCaptureStatusNone && cudaMalloc(&op, bytes) == cudaSuccess) {
+        launch_q8_operand_pack(w->m, op, st);
+        if (cudaStreamSynchronize(st) != cudaSuccess) { cudaFree(op); return nullptr; }
+        return w->op = op;
+    }
+    (void)cudaGetLastError();
+    if (cudaMallocAsync(scratch, bytes, st) != cudaSuccess) { *scratch = nullptr; return nullptr; }
+    launch_q8_operand_pack(w->m, *scratch, st);
+    return *scratch;
+}
+
 extern "C" int brrr_q8_matmul_rows(const brrr_q8mat *w, const int8_t *d_xq, const float *d_xs, int ntok, float *d_y, int ldy, int tensor_cores,
                                    void *stream) {
     if (!w || !d_xq || !d_xs || !d_y || ntok < 1 || ntok > BRRR_TILE_MAX || ldy < w->m.rows) return BRRR_ERR_ARG;
@@ -112,10 +134,17 @@ extern "C" int brrr_q8_matmul_rows(const brrr_q8mat *w, const int8_t *d_xq, cons
     if (!tensor_cores)
         return launch_q8_rows(w->m, d_xq, d_xs, ntok, nullptr, d_y, ldy, Q8_EPI_PLAIN, false, st) == cudaSuccess ? check_launch() : BRRR_ERR_CUDA;
     uint8_t *img = nullptr;          // activation images: stream-ordered scratch, so calls on different streams do not share it
-    if (cudaMallocAsync(&img, image_bytes(ntok, w->m.cols, TI_HALF), st) != cudaSuccess) return BRRR_ERR_NOMEM;
+    uint8_t *scratch = nullptr;
+    const uint8_t *op = q8mat_operand(w, st, &scratch);
+    if (!op || cudaMallocAsync(&img, image_bytes(ntok, w->m.cols, TI_HALF), st) != cudaSuccess) {
+        if (scratch) cudaFreeAsync(scratch, st);
+        (void)cudaGetLastError();
+        return BRRR_ERR_NOMEM;
+    }
     launch_image(d_xq, ntok, w->m.cols, TI_HALF, img, st);
-    const cudaError_t e = launch_q8_tile(w->op, w->m.rows, w->m.cols, img, d_xs, ntok, nullptr, d_y, ldy, Q8_EPI_PLAIN, nullptr, false, st);
+    const cudaError_t e = launch_q8_tile(op, w->m.rows, w->m.cols, img, d_xs, ntok, nullptr, d_y, ldy, Q8_EPI_PLAIN, nullptr, false, st);
     cudaFreeAsync(img, st);
+    if (scratch) cudaFreeAsync(scratch, st);
     return e == cudaSuccess ? check_launch() : BRRR_ERR_CUDA;
 }
 

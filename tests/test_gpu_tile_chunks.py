@@ -38,6 +38,43 @@ def test_q8_rows_tensor_cores_equal_integer_units(brrr, dev, rows, cols, ntok):
     L.brrr_q8mat_free(h)
 
 
+def test_q8_operand_units_are_made_when_wanted(brrr, dev):
+    """A matrix that is only multiplied by vectors takes its Q8 bytes; the tensor-core product adds its copy once, and none of its
+    own where the stream is being captured."""
+    import torch
+    L = brrr.lib()
+    rows, cols, ntok = 24576, 4096, 9
+    q8 = rows * cols * 9 // 8
+    w = torch.empty(rows * cols, dtype=torch.int16, device=dev)
+    assert L.brrr_synth_tensor(7, 1, S.T["WQ"], 30, rows * cols, P(w), None) == 0
+    x = torch.randn((ntok, cols), device=dev)
+    q = torch.empty((ntok, cols), dtype=torch.int8, device=dev); s = torch.empty((ntok, cols // 32), device=dev)
+    assert L.brrr_quant_q8(P(x), x.numel(), P(q), P(s), None) == 0
+    ys = [torch.zeros((ntok, rows), device=dev) for _ in range(4)]
+
+    def taken():
+        torch.cuda.synchronize()
+        return before - torch.cuda.mem_get_info()[0]
+
+    torch.cuda.synchronize()
+    before = torch.cuda.mem_get_info()[0]
+    h = C.c_void_p()
+    assert L.brrr_q8mat_from_bf16(P(w), rows, cols, C.byref(h), None) == 0
+    assert L.brrr_q8_matmul_rows(h, P(q), P(s), ntok, P(ys[0]), rows, 0, None) == 0
+    assert taken() < q8 + (8 << 20)
+    graph, side = torch.cuda.CUDAGraph(), torch.cuda.Stream()
+    with torch.cuda.graph(graph, stream=side):
+        assert L.brrr_q8_matmul_rows(h, P(q), P(s), ntok, P(ys[1]), rows, 1, C.c_void_p(side.cuda_stream)) == 0
+    graph.replay()
+    for y in ys[2:]:
+        assert L.brrr_q8_matmul_rows(h, P(q), P(s), ntok, P(y), rows, 1, None) == 0
+    torch.cuda.synchronize()
+    for y in ys[1:]:
+        assert torch.equal(y, ys[0])
+    del graph
+    L.brrr_q8mat_free(h)
+
+
 @pytest.mark.parametrize("rows,blocks,ntok", [(2880, 90, 9), (2880, 90, 30), (2880, 90, 333), (272, 128, 33), (4096, 4, 8)])
 def test_mx_tile_equals_one_token_kernel(brrr, dev, rows, blocks, ntok):
     import torch
