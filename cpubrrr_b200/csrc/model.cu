@@ -179,17 +179,45 @@ struct brrr_model {
     int tile_rows = BRRR_TILE_MAX;               // tokens per prompt tile (BRRR_TILE_ROWS=n, 2..BRRR_TILE_MAX): any size gives the same bits
     bool tile_prefill = true;                    // run_tile on token tiles (brrr_model_set_tile_prefill / BRRR_TILE_PREFILL=0 switch to token-serial; same bits)
     unsigned int *tl_counter = nullptr;
-    std::vector<void *> allocs;
+    struct Alloc { void *p; size_t bytes; };
+    std::vector<Alloc> allocs;
+    size_t taken = 0;                            // bytes in allocs
 
+    // free device memory (test-hook builds: BRRR_TEST_MEM_BYTES bounds what a model may take)
+    size_t free_bytes() const {
+        size_t free_b = 0, total_b = 0;
+        if (cudaMemGetInfo(&free_b, &total_b) != cudaSuccess) return 0;
+#ifdef BRRR_TEST_HOOKS
+        if (const char *e = getenv("BRRR_TEST_MEM_BYTES")) {
+            const size_t most = strtoull(e, nullptr, 10);
+            free_b = std::min(free_b, most > taken ? most - taken : 0);
+        }
+#endif
+        return free_b;
+    }
     template <typename T> int alloc(T **p, size_t n) {
         void *v = nullptr;
-        if (cudaMalloc(&v, n ? n * sizeof(T) : 16) != cudaSuccess) {
-            snprintf(g_cuda_err, sizeof g_cuda_err, "cudaMalloc of %zu bytes failed", n * sizeof(T));
+        const size_t bytes = n ? n * sizeof(T) : 16;
+#ifdef BRRR_TEST_HOOKS
+        const bool none = getenv("BRRR_TEST_MEM_BYTES") && bytes > free_bytes();
+#else
+        constexpr bool none = false;
+#endif
+        if (none || cudaMalloc(&v, bytes) != cudaSuccess) {
+            (void)cudaGetLastError();            // a caller may go on without
+            snprintf(g_cuda_err, sizeof g_cuda_err, "cudaMalloc of %zu bytes failed", bytes);
             return BRRR_ERR_NOMEM;
         }
-        allocs.push_back(v);
+        allocs.push_back({v, bytes});
+        taken += bytes;
         *p = (T *)v;
         return BRRR_OK;
+    }
+    // give one allocation back (null: nothing); its kernels have ended
+    template <typename T> void release(T **p) {
+        for (size_t i = 0; *p && i < allocs.size(); i++)
+            if (allocs[i].p == *p) { cudaFree(*p); taken -= allocs[i].bytes; allocs.erase(allocs.begin() + i); break; }
+        *p = nullptr;
     }
 };
 
@@ -273,6 +301,12 @@ void rope_table_host(const brrr_cfg &c, float *tab) {
             tab[((size_t)pos * half + i) * 2] = cosf(theta) * mscale;
             tab[((size_t)pos * half + i) * 2 + 1] = sinf(theta) * mscale;
         }
+}
+
+// operand units of the q|k|v and output projections of all layers
+size_t proj_operand_bytes(const brrr_cfg &c) {
+    const int ao = c.n_head * c.head_dim, qkv = ao + 2 * c.n_head_kv * c.head_dim;
+    return (size_t)c.n_layer * (q8_operand_bytes(qkv, c.n_embd) + q8_operand_bytes(c.n_embd, ao));
 }
 
 int check_cfg(const brrr_cfg &c) {
@@ -483,14 +517,13 @@ int build_model(brrr_model *m, const Source &src) {
     {
         // tensor-core expert path: single GPU, speculative step, shapes the tiles cover, and room
         // for the second copy of the expert matrices (about 1.08 x their size)
-        size_t free_b = 0, total_b = 0;
-        CU(cudaMemGetInfo(&free_b, &total_b));
+        const size_t free_b = m->free_bytes();
         const size_t experts = (size_t)c.n_layer * (m->ep ? m->epc.e_cnt : ne) * 3 * d * nb * 17;      // this rank's share
         const size_t rest = (size_t)c.n_vocab * d * 4 + (size_t)c.n_layer * ((size_t)(qkv_rows + d) * d * 2 + (size_t)BRRR_MAXSEQ * nkv * hd * 8) + (2ull << 30);
         m->use_mxt = d % 64 == 0 && nb % 2 == 0 && topk <= 8 && free_b > experts * 2.2 + rest;
-        // operand units of the Q8 projections for token rows: 2.1 x their Q8 bytes, single GPU, where they fit beside the rest
-        const size_t dense_op = (size_t)c.n_layer * (q8_operand_bytes(qkv_rows, d) + q8_operand_bytes(d, nh * hd));
-        m->use_q8op = !m->ep && free_b > experts * (m->use_mxt ? 2.2 : 1.1) + rest + dense_op;
+        // operand units of the Q8 projections for token rows: 1.9 x their Q8 bytes, single GPU, where they fit beside the rest (else rows run
+        // on the integer units, and brrr_model_row_paths says so)
+        m->use_q8op = !m->ep && free_b > experts * (m->use_mxt ? 2.2 : 1.1) + rest + proj_operand_bytes(c);
         if (const char *e = getenv("BRRR_NOMXT")) if (e[0] && e[0] != '0') m->use_mxt = false;
         if (const char *e = getenv("BRRR_NOFUSEDFOLD")) if (e[0] && e[0] != '0') m->fused_fold = false;
         if (const char *e = getenv("BRRR_TILE_PREFILL")) m->tile_prefill = e[0] && e[0] != '0';
@@ -785,7 +818,7 @@ extern "C" void brrr_model_close(brrr_model *m) {
     if (m->side) cudaStreamDestroy(m->side);
     for (void *p : m->ep_peers) if (p) cudaIpcCloseMemHandle(p);
     if (m->ep_buf) cudaFree(m->ep_buf);
-    for (void *p : m->allocs) cudaFree(p);
+    for (const auto &a : m->allocs) cudaFree(a.p);
     if (m->h_in) cudaFreeHost(m->h_in);
     if (m->h_logits) cudaFreeHost(m->h_logits);
     for (cudaEvent_t e : m->ev_logits) if (e) cudaEventDestroy(e);
@@ -906,7 +939,6 @@ static int rows_alloc(brrr_model *m) {
     TRY(m->alloc(&m->tl_aq, R * ao)); TRY(m->alloc(&m->tl_as, R * (ao / 32))); TRY(m->alloc(&m->tl_aimg, image_bytes(R, ao, TI_HALF)));
     TRY(m->alloc(&m->tl_es, R * nb)); TRY(m->alloc(&m->tl_eimg, image_bytes(R, d, TI_PLANES)));
     TRY(m->alloc(&m->tl_hs, E * nb)); TRY(m->alloc(&m->tl_himg, image_bytes((int)E, d, TI_PLANES))); TRY(m->alloc(&m->tl_part, E * d));
-    TRY(m->alloc(&m->tl_scores, R * c.n_head * BRRR_MAXSEQ));      // attention of prompt tiles: every pair's scores
     TRY(m->alloc(&m->tl_logits, R * ne)); TRY(m->alloc(&m->tl_top, R * 8)); TRY(m->alloc(&m->tl_wts, R * 8));
     TRY(m->alloc(&m->tl_counter, R)); TRY(m->alloc(&m->tl_cnt, ne)); TRY(m->alloc(&m->tl_list, (size_t)ne * R));
     CU(cudaMemsetAsync(m->tl_counter, 0, R * sizeof(unsigned int), m->stream));
@@ -916,6 +948,18 @@ static int rows_alloc(brrr_model *m) {
     CU(cudaMallocHost(&m->h_tile, (size_t)ROWS_SLOTS * 3 * R * sizeof(uint32_t)));
     TRY(m->alloc(&m->tl_x, R * d));
     return BRRR_OK;
+}
+
+// Whether rows of one sequence share their K / V tiles in attention (attn_rows_kernel: head groupings it is written for).
+static bool rows_share_keys(const brrr_model *m) {
+    const int group = m->cfg.n_head / m->cfg.n_head_kv;
+    return !m->no_attn_rows && group <= 32 && (group & (group - 1)) == 0;
+}
+// Its workspace, every (head, row) pair's scores: 0.54 GB at the 20b shape, taken by the first pass of prompt rows.  Where it does not fit, the
+// kernel per (head, row) serves them (same bits).
+static void rows_scores_alloc(brrr_model *m) {
+    if (m->tl_scores || !rows_share_keys(m)) return;
+    if (m->alloc(&m->tl_scores, (size_t)BRRR_TILE_MAX * m->cfg.n_head * BRRR_MAXSEQ) != BRRR_OK) m->no_attn_rows = true;
 }
 
 // Rows from which the Q8 projections of a pass run on the tensor cores.
@@ -941,10 +985,9 @@ static int enqueue_rows(brrr_model *m, int n, int kind, bool pdl) {
         else CUL(launch_q8_rows(ly.wqkv, m->tl_nq, m->tl_ns, n, ly.bqkv, m->tl_qkv, qkv_rows, Q8_EPI_BIAS, pdl, s));
         CUL(launch_kv_append_rows(m->tl_qkv, qkv_rows, nh, nkv, kc, vc, seq_stride, m->rope, m->tl_pos, m->tl_seq, n, pdl, s));
         // prompt tiles (rows of one sequence, ascending positions) share their K / V tiles; rows of different sequences cannot
-        const int group = nh / nkv;
         int8_t *aq = tensor ? nullptr : m->tl_aq;
         uint8_t *aimg = tensor ? m->tl_aimg : nullptr;
-        if (one_sequence && !m->no_attn_rows && group <= 32 && (group & (group - 1)) == 0)
+        if (one_sequence && rows_share_keys(m))
             CUL(launch_attn_rows(m->tl_qkv, qkv_rows, kc, vc, seq_stride, m->rope, ly.sinks, nh, nkv, window, m->tl_pos, m->tl_seq, n, m->tl_ao, aq,
                                  m->tl_as, aimg, m->tl_scores, m->st, pdl, s));
         else
@@ -965,6 +1008,7 @@ static int enqueue_rows(brrr_model *m, int n, int kind, bool pdl) {
 // first use of each row count; a direct run comes first so that every kernel has its attributes set).
 static int rows_run(brrr_model *m, int n, const uint32_t *toks, const uint32_t *pos, const uint32_t *seq, int kind) {
     TRY(rows_alloc(m));
+    if (kind != ROWS_BATCH) rows_scores_alloc(m);
     const int R = BRRR_TILE_MAX;
     uint32_t *h = m->h_tile + (size_t)(m->h_tile_next++ % ROWS_SLOTS) * 3 * R;
     if (m->h_tile_next % ROWS_SLOTS == 0) CU(cudaStreamSynchronize(m->stream));        // the ring of pinned slots wraps: nothing may still be reading them
@@ -1037,25 +1081,55 @@ extern "C" int brrr_forward_tile(brrr_model *m, const uint32_t *toks, uint32_t n
 }
 
 // ---- batched decode over independent sequences: one KV cache per sequence, rows = (token, position, sequence)
+// The caches of nseq sequences and the rows' logits; all or nothing.
+static int batch_alloc(brrr_model *m, int nseq) {
+    const brrr_cfg &c = m->cfg;
+    const size_t per_seq = (size_t)c.n_head_kv * BRRR_MAXSEQ * c.head_dim;
+    m->kcb.assign(c.n_layer, nullptr); m->vcb.assign(c.n_layer, nullptr);
+    int s = BRRR_OK;
+    for (int il = 0; il < c.n_layer && s == BRRR_OK; il++) {
+        s = m->alloc(&m->kcb[il], per_seq * nseq);
+        if (s == BRRR_OK) s = m->alloc(&m->vcb[il], per_seq * nseq);
+    }
+    if (s == BRRR_OK) s = m->alloc(&m->bt_logits, (size_t)BRRR_TILE_MAX * c.n_vocab);
+    if (s == BRRR_OK) s = m->alloc(&m->bt_tok, BRRR_TILE_MAX);
+    if (s == BRRR_OK) return s;
+    for (int il = 0; il < c.n_layer; il++) { m->release(&m->kcb[il]); m->release(&m->vcb[il]); }
+    m->release(&m->bt_logits);
+    m->release(&m->bt_tok);
+    return s;
+}
+
+// The projections' operand units make room: rows run on the integer units from here on (same bits).  The captured passes of rows name them.
+static int drop_proj_operands(brrr_model *m) {
+    CU(cudaStreamSynchronize(m->stream));
+    for (auto &gs : m->g_rows)
+        for (cudaGraphExec_t &g : gs)
+            if (g) { cudaGraphExecDestroy(g); g = nullptr; }
+    for (Layer &ly : m->L) { m->release(&ly.wqkv_op); m->release(&ly.wo_op); }
+    m->use_q8op = false;
+    return BRRR_OK;
+}
+
 extern "C" int brrr_batch_open(brrr_model *m, int nseq) {
     if (!m || nseq < 1 || nseq > BRRR_BATCH_MAX) return BRRR_ERR_ARG;
     if (m->ep || m->nseq) return BRRR_ERR_STATE;
     CU(cudaSetDevice(m->device));
     const brrr_cfg &c = m->cfg;
-    const size_t per_seq = (size_t)c.n_head_kv * BRRR_MAXSEQ * c.head_dim;
-    m->kcb.assign(c.n_layer, nullptr); m->vcb.assign(c.n_layer, nullptr);
-    for (int il = 0; il < c.n_layer; il++) { TRY(m->alloc(&m->kcb[il], per_seq * nseq)); TRY(m->alloc(&m->vcb[il], per_seq * nseq)); }
-    TRY(m->alloc(&m->bt_logits, (size_t)BRRR_TILE_MAX * c.n_vocab));
-    TRY(m->alloc(&m->bt_tok, BRRR_TILE_MAX));
     TRY(rows_alloc(m));
-    if (m->use_q8op) {
-        size_t free_b = 0, total_b = 0;
-        CU(cudaMemGetInfo(&free_b, &total_b));
-        if (free_b > q8_operand_bytes(c.n_vocab, c.n_embd) + (1ull << 30)) {
-            TRY(m->alloc(&m->head_op, q8_operand_bytes(c.n_vocab, c.n_embd)));
-            launch_q8_operand_pack(m->head, m->head_op, m->stream);
-            CU(cudaGetLastError());
+    int s = batch_alloc(m, nseq);
+    if (s == BRRR_ERR_NOMEM && m->use_q8op) {        // sequences go before speed, where the copies are what they lack
+        const size_t need = (size_t)c.n_layer * 2 * c.n_head_kv * BRRR_MAXSEQ * c.head_dim * nseq * sizeof(float) + (size_t)BRRR_TILE_MAX * (c.n_vocab + 1) * 4;
+        if (need <= m->free_bytes() + proj_operand_bytes(c)) {
+            TRY(drop_proj_operands(m));
+            s = batch_alloc(m, nseq);
         }
+    }
+    TRY(s);
+    const size_t head_bytes = q8_operand_bytes(c.n_vocab, c.n_embd);
+    if (m->use_q8op && m->free_bytes() > head_bytes + (1ull << 30) && m->alloc(&m->head_op, head_bytes) == BRRR_OK) {
+        launch_q8_operand_pack(m->head, m->head_op, m->stream);
+        CU(cudaGetLastError());
     }
     m->nseq = nseq;
     return BRRR_OK;
@@ -1269,6 +1343,10 @@ extern "C" int brrr_moe_ffn_step_tc(brrr_model *m, int il, const float *d_xn, fl
 }
 
 extern "C" int brrr_model_uses_tensor_experts(const brrr_model *m) { return m && m->use_mxt ? 1 : 0; }
+extern "C" int brrr_model_row_paths(const brrr_model *m) {
+    if (!m) return 0;
+    return (m->use_q8op ? BRRR_ROWS_TENSOR_PROJ : 0) | (m->head_op ? BRRR_ROWS_TENSOR_HEAD : 0) | (rows_share_keys(m) ? BRRR_ROWS_SHARED_KEYS : 0);
+}
 
 // MoE FFN of one layer for n normalised rows (floats xn for the router, plane images tl_eimg / tl_es for the experts), enqueue
 // only: per-row router (one launch), routing lists per expert, then gate | up with the SwiGLU and down as two grouped tensor-core
@@ -1370,7 +1448,10 @@ extern "C" int brrr_stage_time(brrr_model *m, int stage, uint32_t pos, int reps,
 }
 
 #ifdef BRRR_TEST_HOOKS
-// Test-hook builds only (not part of the public interface): the in-kernel clock stamps of the last step.
+// Test-hook builds only (not part of the public interface): device bytes the model holds (what BRRR_TEST_MEM_BYTES bounds).
+extern "C" uint64_t brrr_debug_taken(const brrr_model *m) { return m ? m->taken : 0; }
+
+// the in-kernel clock stamps of the last step.
 extern "C" int brrr_debug_stamps(brrr_model *m, long long *out256) {
     if (!m || !out256) return BRRR_ERR_ARG;
     CU(cudaSetDevice(m->device));

@@ -140,6 +140,11 @@ class Engine:
         return bool(lib().brrr_model_uses_tensor_experts(self._h))
 
     @property
+    def row_paths(self):
+        """BRRR_ROWS_* bits: 1 projections and 2 vocabulary head of token rows on the tensor cores, 4 prompt rows share K / V tiles."""
+        return int(lib().brrr_model_row_paths(self._h))
+
+    @property
     def stream(self):
         return lib().brrr_model_stream(self._h)
 

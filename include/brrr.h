@@ -95,7 +95,10 @@ int brrr_model_set_tile_prefill(brrr_model *m, int on);
  * the vocabulary projection read their weights once per 8 rows, each selected expert is read once
  * for all the rows routed to it.  Every row's result is bit-identical to brrr_forward on that
  * sequence alone.
- *   brrr_batch_open     allocates nseq (1..BRRR_BATCH_MAX) caches; once per model, not with expert-parallel ranks
+ *   brrr_batch_open     allocates nseq (1..BRRR_BATCH_MAX) caches (0.4 GB each at the 20b shape) and the rows' logits (0.4 GB); once per
+ *                       model, not with expert-parallel ranks.  Where the caches only fit without the projections' operand copies,
+ *                       those are given up; where memory is left, the vocabulary matrix is copied in operand order (brrr_model_row_paths).
+ *                       After BRRR_ERR_NOMEM the model works as before, and fewer sequences may be asked for
  *   brrr_batch_prefill  feeds n prompt tokens of one sequence from position pos0 (tiles, no logits)
  *   brrr_batch_step     n rows (1..BRRR_TILE_MAX) in one pass; out_toks[i] = greedy next token of row i.
  *                       A row attends over its sequence's cache up to pos[i] - 1 plus itself; rows of one
@@ -416,6 +419,15 @@ int brrr_moe_ffn_step(brrr_model *m, int il, const float *d_xn, float *d_x, int3
 int brrr_moe_ffn_step_tc(brrr_model *m, int il, const float *d_xn, float *d_x, int32_t *d_top, float *d_wts);
 /* 1 when the decode step of this model runs its expert matvecs on the tensor cores. */
 int brrr_model_uses_tensor_experts(const brrr_model *m);
+
+/* How passes of several token rows (prompts, batched decode) run on this model now.  The bits of the results are the same in every
+ * case; a path that is missing lacked device memory (or, for the shared keys, a head grouping its kernel is written for). */
+enum {
+    BRRR_ROWS_TENSOR_PROJ = 1,   /* q|k|v and output projection on the tensor cores: copies in operand order exist (1.4 GB at the 20b shape) */
+    BRRR_ROWS_TENSOR_HEAD = 2,   /* vocabulary projection likewise: a copy that brrr_batch_open makes (1.2 GB) */
+    BRRR_ROWS_SHARED_KEYS = 4    /* prompt rows share K and V tiles: a workspace of 0.54 GB, taken by the first prompt */
+};
+int brrr_model_row_paths(const brrr_model *m);
 
 /* The same MoE FFN for a tile of 1..BRRR_TILE_MAX normalised tokens (d_xn [ntok][n_embd], d_x [ntok][n_embd]
  * residuals, d_top / d_wts nullable [ntok][n_expert_used]): per-token router, then gate / up /

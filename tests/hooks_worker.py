@@ -3,7 +3,7 @@
 default build, which contains no hook.  No GPU fault is provoked: a missed speculation is a
 flagged step, a silent router is a bounded wait that runs out and is reported.
 
-    python tests/hooks_worker.py sabotage | mute | qwen_sabotage | qwen_mute
+    python tests/hooks_worker.py sabotage | mute | memory | qwen_sabotage | qwen_mute
 """
 import os
 import sys
@@ -87,6 +87,68 @@ def qwen(mode):
     om.close()
 
 
+def memory(cfg, prompt):
+    """Copies and workspaces that do not fit: what goes without them, and that nothing changes but the path."""
+    import ctypes as C
+    import cpubrrr_b200 as B
+    from cpubrrr_b200 import synth as S
+    bits = lambda a: np.ascontiguousarray(a, dtype=np.float32).view(np.uint32)
+    taken = B.lib().brrr_debug_taken
+    taken.restype, taken.argtypes = C.c_uint64, [C.c_void_p]
+    limit = lambda n: os.environ.__setitem__("BRRR_TEST_MEM_BYTES", str(n))
+    free = lambda: os.environ.pop("BRRR_TEST_MEM_BYTES", None)
+    PROJ, HEAD, KEYS = 1, 2, 4
+    long = S.synth_prompt(5, 70, 500)
+
+    def use(eng, nseq):
+        """A prompt, a batch whose sequences have prompts of their own, a step of as many rows."""
+        out = [eng.prefill(long), bits(eng.logits())]
+        for s in range(nseq):
+            eng.batch_prefill(s, long[:20 + s])
+        toks, lg = eng.batch_step(list(long[:nseq]), [20 + s for s in range(nseq)], list(range(nseq)), logits=True)
+        return out + [toks, bits(lg)]
+
+    def same(a, b):
+        return all(np.array_equal(x, y) for x, y in zip(a, b))
+
+    n = 12                                                  # rows enough for the tensor-core projections and head
+    eng = B.Engine.synth(cfg, 17)
+    eng.batch_open(n)
+    want = use(eng, n)
+    assert eng.row_paths == PROJ | HEAD | KEYS and eng.uses_tensor_experts
+    eng.close()
+    # neither copy fits beside the rest (2 GB are kept free): integer units throughout
+    limit(1 << 30)
+    eng = B.Engine.synth(cfg, 17)
+    eng.batch_open(n)
+    assert eng.row_paths == KEYS and not eng.uses_tensor_experts
+    assert same(use(eng, n), want) and eng.row_paths == KEYS
+    eng.close()
+    # the workspace of the prompt rows does not fit: the other attention kernel
+    free()
+    eng = B.Engine.synth(cfg, 17)
+    eng.batch_open(n)
+    limit(taken(eng._h) + 4096)
+    assert same(use(eng, n), want) and eng.row_paths == PROJ | HEAD
+    eng.close()
+    # the caches fit only where the projections' copies were, after a prompt has run on those
+    free()
+    eng = B.Engine.synth(cfg, 17)
+    eng.prefill(long)
+    at = taken(eng._h)
+    limit(at + (64 << 20))
+    assert B.lib().brrr_batch_open(eng._h, 256) == 4        # 256 caches fit neither way: BRRR_ERR_NOMEM, and the model as it was
+    assert taken(eng._h) == at and eng.row_paths == PROJ | KEYS
+    assert eng.prefill(long) == want[0] and np.array_equal(bits(eng.logits()), want[1])
+    need = 2 * cfg.n_layer * cfg.n_head_kv * 4096 * 64 * 4 * n + 512 * (cfg.n_vocab + 1) * 4
+    limit(at + need - 4096)
+    eng.batch_open(n)
+    assert eng.row_paths == KEYS and taken(eng._h) < at + need
+    assert same(use(eng, n), want)
+    eng.close()
+    free()
+
+
 def main(mode):
     assert os.environ.get("BRRR_LIBRARY", "").endswith("libbrrr_hooks.so")
     if mode.startswith("qwen"):
@@ -142,6 +204,8 @@ def main(mode):
         assert [first] + [int(t) for t in toks[:-1]] == want[:12]
         assert eng.wait_fallbacks() == 1
         eng.close()
+    elif mode == "memory":
+        memory(cfg, prompt)
     else:
         raise SystemExit("mode?")
     print("hooks_worker ok:", mode)

@@ -278,6 +278,12 @@ def test_router_wait_runs_out_and_the_model_falls_back(brrr):
     _run_with_hooks(brrr, "mute")
 
 
+def test_rows_without_memory_for_their_copies(brrr):
+    """Where the operand copies or the score workspace do not fit, rows take the paths without them: same bits, and
+    brrr_model_row_paths says which; caches that only fit without the copies get their room."""
+    _run_with_hooks(brrr, "memory")
+
+
 def test_speculation_can_be_disabled(brrr, orc, monkeypatch):
     cfg = brrr.make_cfg(128, 2, 4, 2, 8, 4, 512)
     monkeypatch.setenv("BRRR_NOSPEC", "1")
