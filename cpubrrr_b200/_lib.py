@@ -87,6 +87,7 @@ SIGNATURES = {
     "brrr_qwen_forward_trace": (_I, [_P, C.c_uint32, C.c_uint32, _P]),
     "brrr_qwen_stream": (_P, [_P]),
     "brrr_qwen_launches_per_step": (_I, [_P, _I]),
+    "brrr_qwen_uses_rows": (_I, [_P]),
     "brrr_qwen_spec_redos": (C.c_uint64, [_P]),
     "brrr_qwen_wait_fallbacks": (C.c_uint64, [_P]),
     "brrr_qwen_bytes_per_step": (C.c_uint64, [_P, C.c_uint32]),

@@ -108,10 +108,23 @@ struct brrr_qwen {
         uint32_t *toks;
     } r{};
     std::vector<void *> allocs;
+#ifdef BRRR_TEST_HOOKS
+    size_t taken = 0;                 // bytes asked for so far; BRRR_TEST_MEM_BYTES bounds it
+#endif
 
     template <typename T> int alloc(T **p, size_t n) {
         void *vp = nullptr;
-        if (cudaMalloc(&vp, n ? n * sizeof(T) : 16) != cudaSuccess) { QERR("cudaMalloc of %zu bytes failed", n * sizeof(T)); return BRRR_ERR_NOMEM; }
+        const size_t bytes = n ? n * sizeof(T) : 16;
+        bool none = false;
+#ifdef BRRR_TEST_HOOKS
+        if (const char *e = getenv("BRRR_TEST_MEM_BYTES")) none = taken + bytes > strtoull(e, nullptr, 10);
+        if (!none) taken += bytes;
+#endif
+        if (none || cudaMalloc(&vp, bytes) != cudaSuccess) {
+            (void)cudaGetLastError();            // a caller may go on without
+            QERR("cudaMalloc of %zu bytes failed", bytes);
+            return BRRR_ERR_NOMEM;
+        }
         allocs.push_back(vp);
         *p = (T *)vp;
         return BRRR_OK;
@@ -422,7 +435,11 @@ int qbuild(brrr_qwen *m, const QSource &src) {
     TRY(m->alloc(&m->top, 8)); TRY(m->alloc(&m->st, 1));
     TRY(qreset_state(m));
     CU(cudaMemsetAsync(m->x, 0, d * 4, m->stream));
-    TRY(qrows_alloc(m));
+    const size_t kept = m->allocs.size();
+    const int rows = qrows_alloc(m);
+    if (rows == BRRR_ERR_NOMEM)              // prompts go token by token instead (same bits; brrr_qwen_uses_rows)
+        while (m->allocs.size() > kept) { cudaFree(m->allocs.back()); m->allocs.pop_back(); }
+    else TRY(rows);
     CU(cudaMallocHost(&m->h_in, (BRRR_MAXSEQ + 4) * sizeof(uint32_t)));
     CU(cudaMallocHost(&m->h_out, BRRR_MAXSEQ * sizeof(uint32_t)));
     CU(cudaStreamSynchronize(m->stream));
@@ -542,6 +559,7 @@ extern "C" int brrr_qwen_cfg_get(const brrr_qwen *m, brrr_qwen_cfg *out) {
     return BRRR_OK;
 }
 
+extern "C" int brrr_qwen_uses_rows(const brrr_qwen *m) { return m && m->has_rows ? 1 : 0; }
 extern "C" uint64_t brrr_qwen_spec_redos(const brrr_qwen *m) { return m ? m->spec_redos : 0; }
 extern "C" uint64_t brrr_qwen_wait_fallbacks(const brrr_qwen *m) { return m ? m->wait_fallbacks : 0; }
 
@@ -704,7 +722,10 @@ extern "C" int brrr_qwen_forward_trace(brrr_qwen *m, uint32_t tok, uint32_t pos,
 extern "C" void *brrr_qwen_stream(brrr_qwen *m) { return m ? (void *)m->stream : nullptr; }
 
 #ifdef BRRR_TEST_HOOKS
-// Test-hook builds only: the room rule of a layer of shape *cfg with q, k, v of type_qkv and down of type_down (host arithmetic only).
+// Test-hook builds only: device bytes the model has asked for (what BRRR_TEST_MEM_BYTES bounds).
+extern "C" uint64_t brrr_debug_qwen_taken(const brrr_qwen *m) { return m ? m->taken : 0; }
+
+// The room rule of a layer of shape *cfg with q, k, v of type_qkv and down of type_down (host arithmetic only).
 // out: CTAs of down and of the next q|k|v, shared memory of a CTA of down, of q|k|v and of the router, 1 if down may poll.
 extern "C" int brrr_debug_qwen_room(const brrr_qwen_cfg *cfg, int type_qkv, int type_down, uint64_t *out) {
     if (!cfg || !out || qcheck_cfg(*cfg) != BRRR_OK) return BRRR_ERR_ARG;

@@ -103,6 +103,11 @@ class QwenEngine:
     def launches_per_step(self, want=True):
         return lib().brrr_qwen_launches_per_step(self._h, int(bool(want)))
 
+    @property
+    def uses_rows(self):
+        """Whether prompts walk the layers as token rows (else token by token; same bits)."""
+        return bool(lib().brrr_qwen_uses_rows(self._h))
+
     def spec_redos(self):
         """Steps run again because the routing estimate missed an expert or a wait ran out (performance counter)."""
         return int(lib().brrr_qwen_spec_redos(self._h))

@@ -265,6 +265,9 @@ int brrr_qwen_hidden(brrr_qwen *m, float *out);               /* [n_embd], resid
 int brrr_qwen_forward_trace(brrr_qwen *m, uint32_t tok, uint32_t pos, float *trace);
 void *brrr_qwen_stream(brrr_qwen *m);
 int brrr_qwen_launches_per_step(const brrr_qwen *m, int want_logits);
+/* 1: prompts walk the layers as token rows (scratch of about 0.16 GB at the Qwen3-30B-A3B shape); 0: token by token, where that
+ * does not fit or the row attention is not written for the head grouping.  Same bits. */
+int brrr_qwen_uses_rows(const brrr_qwen *m);
 /* Steps that were run again because the routing estimate missed an expert or a wait ran out, and waits that ran out
  * (0 or 1; the model then decodes without speculation): as brrr_model_spec_redos and brrr_model_wait_fallbacks. */
 uint64_t brrr_qwen_spec_redos(const brrr_qwen *m);

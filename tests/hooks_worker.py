@@ -3,7 +3,7 @@
 default build, which contains no hook.  No GPU fault is provoked: a missed speculation is a
 flagged step, a silent router is a bounded wait that runs out and is reported.
 
-    python tests/hooks_worker.py sabotage | mute | memory | qwen_sabotage | qwen_mute
+    python tests/hooks_worker.py sabotage | mute | memory | qwen_sabotage | qwen_mute | qwen_memory
 """
 import os
 import sys
@@ -43,8 +43,8 @@ def qwen(mode):
     def check(eng):
         assert np.array_equal(bits(eng.logits()), bits(om.logits())) and np.array_equal(bits(eng.hidden()), bits(om.hidden()))
 
-    def hooked(var):
-        os.environ[var] = "1"
+    def hooked(var, value="1"):
+        os.environ[var] = value
         eng = B.QwenEngine.synth(cfg, 17)
         del os.environ[var]
         return eng
@@ -55,7 +55,20 @@ def qwen(mode):
         assert [first] + [int(t) for t in toks[:-1]] == want
         check(eng)
 
-    if mode == "qwen_sabotage":
+    if mode == "qwen_memory":
+        # the rows' scratch does not fit: prompts go token by token
+        import ctypes as C
+        taken = B.lib().brrr_debug_qwen_taken
+        taken.restype, taken.argtypes = C.c_uint64, [C.c_void_p]
+        eng = B.QwenEngine.synth(cfg, 17)
+        assert eng.uses_rows
+        chained(eng)
+        most = taken(eng._h)
+        eng.close()
+        eng = hooked("BRRR_TEST_MEM_BYTES", str(most - 1))
+        assert not eng.uses_rows
+        chained(eng)
+    elif mode == "qwen_sabotage":
         # the estimate is spoiled where the position is a multiple of three: exactly those steps run twice
         eng = hooked("BRRR_SPEC_SABOTAGE")
         assert greedy(eng.run, prompt, 40) == want

@@ -162,10 +162,11 @@ def test_qwen_mixed_kquant_types_per_tensor(brrr, orc, tmp_path):
     eng.close(); plain.close(); om.close()
 
 
-@pytest.mark.parametrize("mode", ["qwen_sabotage", "qwen_mute"])
-def test_qwen_speculation_recovers(brrr, mode):
-    """A step whose estimate missed an expert, and one whose exact router stays silent, run again without the estimate: results
-    are the oracle's and the counters name the steps (test-hook build of the library, tests/hooks_worker.py)."""
+@pytest.mark.parametrize("mode", ["qwen_sabotage", "qwen_mute", "qwen_memory"])
+def test_qwen_failures_are_recovered(brrr, mode):
+    """A step whose estimate missed an expert, and one whose exact router stays silent, run again without the estimate; a model without
+    memory for the rows' scratch feeds prompts token by token: results are the oracle's and the counters name the steps (test-hook
+    build of the library, tests/hooks_worker.py)."""
     import subprocess
     import sys
     from cpubrrr_b200 import build
