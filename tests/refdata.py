@@ -121,3 +121,19 @@ def case_data_dir(out_dir, case, seed):
     arch, cfg, ktypes = case_cfg(case)
     d, blob = make_data_dir(out_dir, cfg, seed, case, arch=arch, ktypes=ktypes)
     return cfg, d, blob
+
+
+def retype_qwen(data_dir, blob, cfg, seed, ktypes):
+    """The blob of a made data directory written again with other K-quant types, and the manifest's types and offsets with it (names, order,
+    element counts and data_start stay: only the type field of a tensor info changes in the header)."""
+    S.write_gguf(blob, cfg, seed, arch="qwen3moe", ktypes=ktypes)
+    path = os.path.join(data_dir, "manifest.txt")
+    head, *rows = open(path).read().split("\n")
+    out, off = [head], 0
+    for (name, ty, _, raw), row in zip(S.qwen_model_tensors(cfg, seed, ktypes), rows):
+        assert row.split()[0] == name
+        out.append(f"{name} {ty} {off} {row.split()[3]}")
+        off = (off + len(raw) + 31) // 32 * 32
+    assert int(head.split()[1]) + off == os.path.getsize(blob)
+    with open(path, "w") as w:
+        w.write("\n".join(out) + "\n")

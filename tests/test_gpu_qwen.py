@@ -162,6 +162,32 @@ def test_qwen_mixed_kquant_types_per_tensor(brrr, orc, tmp_path):
     eng.close(); plain.close(); om.close()
 
 
+@pytest.mark.parametrize("ktypes", [
+    {"blk.0.ffn_gate_exps.weight": 14, "blk.1.ffn_up_exps.weight": 14},                                     # gate 6 / up 4 bits, then 4 / 6
+    {"blk.0.ffn_gate_exps.weight": 14, "blk.0.ffn_up_exps.weight": 14, "blk.1.attn_output.weight": 14,      # both 6
+     "blk.1.attn_q.weight": 14, "blk.1.attn_k.weight": 14, "output.weight": 12},
+])
+def test_qwen_kquant_types_of_gate_up_and_head(brrr, orc, tmp_path, ktypes):
+    """Every pair of types the gate/up kernel takes, Q6_K projections, a Q4_K head: steps, device-chained steps and token rows."""
+    import refdata
+    cfg, d, blob = refdata.case_data_dir(str(tmp_path / "qt"), "qwen_mixed", 12)
+    refdata.retype_qwen(d, blob, cfg, 12, ktypes)
+    eng = brrr.QwenEngine.open(d, blob)
+    om = orc.QwenModel.open(d, blob)
+    prompt = S.synth_prompt(12, 40, cfg.n_vocab)
+    want = greedy(om.run, prompt, 20)
+    for prefill in (False, True):
+        if prefill:
+            first = eng.prefill(prompt)
+            got = [first] + [int(t) for t in eng.decode(first, len(prompt), 20)[:-1]]
+        else:
+            got = greedy(eng.run, prompt, 20)
+        assert got == want
+        assert np.array_equal(bits(eng.logits()), bits(om.logits())) and np.array_equal(bits(eng.hidden()), bits(om.hidden()))
+    assert (eng.spec_redos(), eng.wait_fallbacks()) == (0, 0)
+    eng.close(); om.close()
+
+
 @pytest.mark.parametrize("mode", ["qwen_sabotage", "qwen_mute", "qwen_memory"])
 def test_qwen_failures_are_recovered(brrr, mode):
     """A step whose estimate missed an expert, and one whose exact router stays silent, run again without the estimate; a model without
