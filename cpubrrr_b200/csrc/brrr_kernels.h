@@ -8,9 +8,7 @@ namespace brrr {
 
 // ---- elementwise / small stages (kernels_small.cu)
 void launch_quant_q8(const float *x, int n, int8_t *q, float *s, cudaStream_t st);
-// rows > 1: one CTA per row; rows are n apart in x / xn / q and n / 32 apart in s
-cudaError_t launch_rmsnorm_quant(const float *x, const float *w, float eps, int n, float *xn, int8_t *q, float *s, bool pdl, cudaStream_t st,
-                                 int rows = 1);
+cudaError_t launch_rmsnorm_quant(const float *x, const float *w, float eps, int n, float *xn, int8_t *q, float *s, bool pdl, cudaStream_t st);
 // ---- token rows (kernels_rows.cu): y[t][r] (+)= row r of m . activation t (+ bias) on the integer units
 cudaError_t launch_q8_rows(Q8Dev m, const int8_t *xq, const float *xs, int ntok, const float *bias, float *y, int ldy, int epi, bool pdl, cudaStream_t st);
 // residual rows x [rows][d]: part != nullptr: x[t] += sum over k of wts[8 t + k] * part[t * topk + k]; norm_w != nullptr: RMSNorm, Q8 per 32-block (scales s,
@@ -21,9 +19,8 @@ cudaError_t launch_rows_norm(float *x, int rows, int d, const float *part, const
 cudaError_t launch_kv_append_rows(const float *qkv, int ldq, int nh, int nkv, float *kc, float *vc, size_t seq_stride, const float *rope,
                                   const int *row_pos, const int *row_seq, int rows, bool pdl, cudaStream_t st);
 void launch_embed(const uint16_t *embd, int d, const DevState *state, float *x, cudaStream_t st);
-void launch_embed_tok(const uint16_t *embd, int d, uint32_t tok, float *x, cudaStream_t st);
-// ntok rows from token ids in device memory: x[t] = embedding of toks[t]
 void launch_rows_argmax(const float *logits, int n_vocab, int rows, uint32_t *out, cudaStream_t st);   // out[t] = first index of the largest logit of row t
+// ntok rows from token ids in device memory: x[t] = embedding of toks[t]
 void launch_embed_tile(const uint16_t *embd, int d, const uint32_t *toks_dev, int ntok, float *x, cudaStream_t st);
 void launch_swiglu_quant(const float *gu, int topk, int d, int8_t *hq, float *hs, cudaStream_t st);
 void launch_finish_token(DevState *state, cudaStream_t st);

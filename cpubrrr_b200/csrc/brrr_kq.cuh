@@ -9,6 +9,7 @@
 // integer reduction and every lane carries the same float chain.
 #pragma once
 #include "brrr_dev.cuh"
+#include "brrr_tma.cuh"
 
 #include <cuda_fp16.h>
 
@@ -233,16 +234,6 @@ __device__ __forceinline__ int dp4a_us(uint32_t u, int s, int c) {      // unsig
     return r;
 }
 
-__device__ __forceinline__ uint4 kq_lds128(uint32_t a) {
-    uint4 r;
-    asm volatile("ld.shared.v4.u32 {%0, %1, %2, %3}, [%4];" : "=r"(r.x), "=r"(r.y), "=r"(r.z), "=r"(r.w) : "r"(a));
-    return r;
-}
-__device__ __forceinline__ uint2 kq_lds64(uint32_t a) {
-    uint2 r;
-    asm volatile("ld.shared.v2.u32 {%0, %1}, [%2];" : "=r"(r.x), "=r"(r.y) : "r"(a));
-    return r;
-}
 __device__ __forceinline__ uint32_t kq_lds16(uint32_t a) {
     unsigned short r;
     asm volatile("ld.shared.u16 %0, [%1];" : "=h"(r) : "r"(a));
@@ -259,7 +250,7 @@ __device__ __forceinline__ float kq_term(int nsb, uint32_t row, int sb, const KA
     const int hi4[8] = {x.x[2].x, x.x[2].y, x.x[2].z, x.x[2].w, x.x[3].x, x.x[3].y, x.x[3].z, x.x[3].w};
     if (TYPE == 12) {
         const uint32_t p = row + sb * 144;
-        const uint4 h = kq_lds128(p), u = kq_lds128(p + 16 + 32 * l4), v = kq_lds128(p + 32 + 32 * l4);
+        const uint4 h = lds128(p), u = lds128(p + 16 + 32 * l4), v = lds128(p + 32 + 32 * l4);
         const bool upper = l4 >= 2;                  // sub-blocks 4 .. 7: six bits in two fields
         const uint32_t sc = (upper ? (h.w & M4) | ((h.y >> 2) & 0x30303030u) : h.y & 0x3F3F3F3Fu) >> ((l4 & 1) * 16);
         const uint32_t mn = (upper ? ((h.w >> 4) & M4) | ((h.z >> 2) & 0x30303030u) : h.z & 0x3F3F3F3Fu) >> ((l4 & 1) * 16);
@@ -280,8 +271,8 @@ __device__ __forceinline__ float kq_term(int nsb, uint32_t row, int sb, const KA
     const int h = l4 >> 1, b = l4 & 1;
     const uint32_t lp = row + sb * 128 + 32 * l4, up = row + nsb * 128 + sb * 64 + 32 * h;
     const int o = sw * 16;
-    const uint4 l0 = kq_lds128(lp + o), l1 = kq_lds128(lp + 16 - o), u0 = kq_lds128(up + o), u1 = kq_lds128(up + 16 - o);
-    const uint2 s8 = kq_lds64(row + nsb * 192 + sb * 16 + 8 * h);
+    const uint4 l0 = lds128(lp + o), l1 = lds128(lp + 16 - o), u0 = lds128(up + o), u1 = lds128(up + 16 - o);
+    const uint2 s8 = lds64(row + nsb * 192 + sb * 16 + 8 * h);
     const float d = half_bits_to_f32(kq_lds16(row + nsb * 208 + sb * 2));
     const uint32_t order = (b ? 0x32u : 0x10u), pick = sw ? (order >> 4) | ((order & 15u) << 4) : order;
     const uint32_t slo = __byte_perm(s8.x, 0, pick), shi = __byte_perm(s8.y, 0, pick), M2 = 0x30303030u;

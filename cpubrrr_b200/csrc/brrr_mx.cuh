@@ -24,20 +24,6 @@ __device__ __forceinline__ void mx_stage_x(const int8_t *__restrict__ xq, const 
     for (int b = tid; b < nb; b += nthreads) xsc[b] = xs[b];
 }
 
-// Quantise one 32-block held one value per lane straight into the staged layout.
-__device__ __forceinline__ void mx_quant_stage_block(float v, int lane, int b, int2 *xp, float *xsc) {
-    float amax = fmaxf(warp_max(fabsf(v)), 1e-12f);
-    float sc = __fdiv_rn(amax, 127.0f);
-    uint32_t q = (uint32_t)(brrr_q8_round(v, sc) & 0xFF);
-    uint32_t word = q << (8 * (lane & 3));
-    word |= __shfl_xor_sync(0xffffffffu, word, 1);
-    word |= __shfl_xor_sync(0xffffffffu, word, 2);           // lanes 4j..4j+3 hold lo word j, lanes 16+4j.. hi word j
-    uint32_t other = __shfl_xor_sync(0xffffffffu, word, 16);
-    if (lane < 16 && (lane & 3) == 0) xp[b * 4 + (lane >> 2)] = mx_interleave(word, other);
-    if (lane == 0) xsc[b] = sc;
-}
-
-
 // N consecutive block pairs of one lane chain from units resident in shared memory: operands
 // first, then the 2N exact lane dots and scales (independent work), then the 2N fused
 // multiply-adds in block order.

@@ -20,6 +20,18 @@ __device__ __forceinline__ bool elect_one() {
 
 __device__ __forceinline__ uint32_t smem_u32(const void *p) { return (uint32_t)__cvta_generic_to_shared(p); }
 
+// shared-memory loads by 32-bit address, in program order
+__device__ __forceinline__ uint2 lds64(uint32_t addr) {
+    uint2 r;
+    asm volatile("ld.shared.v2.u32 {%0, %1}, [%2];" : "=r"(r.x), "=r"(r.y) : "r"(addr));
+    return r;
+}
+__device__ __forceinline__ uint4 lds128(uint32_t addr) {
+    uint4 r;
+    asm volatile("ld.shared.v4.u32 {%0, %1, %2, %3}, [%4];" : "=r"(r.x), "=r"(r.y), "=r"(r.z), "=r"(r.w) : "r"(addr));
+    return r;
+}
+
 __device__ __forceinline__ void mbar_init(uint64_t *bar, uint32_t count) {
     asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(smem_u32(bar)), "r"(count) : "memory");
 }
@@ -93,20 +105,6 @@ struct Waiter {
         do {
             for (int i = 0; i < 128; i++)
                 if (mbar_try_wait(bar, parity)) return true;
-        } while (clock64() - t0 < WAIT_CYCLES);
-        dead = true;
-        if (err) atomicCAS(err, (uint32_t)DEV_ERR_NONE, (uint32_t)DEV_ERR_COPY_TIMEOUT);
-        return false;
-    }
-    // The same bounded wait with hardware suspension between probes (see mbar_try_wait_hint): for roles that
-    // spend most of their time waiting beside busy warps (producers, issuing threads) and must still wake at once.
-    __device__ __forceinline__ bool wait_suspended(uint64_t *bar, uint32_t parity) {
-        if (dead) return false;
-        if (mbar_test_wait(bar, parity)) return true;
-        const long long t0 = clock64();
-        do {
-            for (int i = 0; i < 16; i++)
-                if (mbar_try_wait_hint(bar, parity, 4000u)) return true;
         } while (clock64() - t0 < WAIT_CYCLES);
         dead = true;
         if (err) atomicCAS(err, (uint32_t)DEV_ERR_NONE, (uint32_t)DEV_ERR_COPY_TIMEOUT);

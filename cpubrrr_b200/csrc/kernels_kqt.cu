@@ -19,6 +19,7 @@
 #include "brrr_kqt.cuh"
 #include "brrr_tc.cuh"
 #include "brrr_tile.cuh"
+#include "brrr_tmap.h"
 
 namespace brrr {
 
@@ -80,11 +81,6 @@ __device__ __forceinline__ f32x2 kt_mul2_apart(f32x2 a, f32x2 b) {
 __device__ __forceinline__ f32x2 kt_sub2(f32x2 a, f32x2 b) {
     f32x2 r;
     asm("sub.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
-    return r;
-}
-__device__ __forceinline__ uint4 lds128(uint32_t addr) {
-    uint4 r;
-    asm volatile("ld.shared.v4.u32 {%0, %1, %2, %3}, [%4];" : "=r"(r.x), "=r"(r.y), "=r"(r.z), "=r"(r.w) : "r"(addr));
     return r;
 }
 __device__ __forceinline__ uint32_t lds32(uint32_t addr) {
@@ -460,22 +456,8 @@ __global__ void __launch_bounds__(KT_THREADS, 1) kqt_kernel(const __grid_constan
 
 }  // namespace
 
-namespace {
-typedef CUresult (*encode_t)(CUtensorMap *, CUtensorMapDataType, cuuint32_t, void *, const cuuint64_t *, const cuuint64_t *, const cuuint32_t *, const cuuint32_t *,
-                             CUtensorMapInterleave, CUtensorMapSwizzle, CUtensorMapL2promotion, CUtensorMapFloatOOBfill);
-encode_t tensor_encode() {
-    static encode_t encode = [] {
-        void *f = nullptr;
-        cudaDriverEntryPointQueryResult r;
-        if (cudaGetDriverEntryPointByVersion("cuTensorMapEncodeTiled", &f, 12000, cudaEnableDefault, &r) != cudaSuccess || r != cudaDriverEntryPointSuccess) f = nullptr;
-        return (encode_t)f;
-    }();
-    return encode;
-}
-}  // namespace
-
 cudaError_t qw_cache(float *kc, float *vc, int nkv, QwCache *out) {
-    const encode_t encode = tensor_encode();
+    const tmap_encode_t encode = tmap_encode();
     if (!encode) return cudaErrorNotSupported;
     const cuuint64_t dims[2] = {128, (cuuint64_t)nkv * BRRR_MAXSEQ}, strides[1] = {512};
     const cuuint32_t box[2] = {32, 64}, ones[2] = {1, 1};
@@ -488,7 +470,7 @@ cudaError_t qw_cache(float *kc, float *vc, int nkv, QwCache *out) {
 }
 
 cudaError_t kqt_matrix(const KMatDev &m, size_t rows_total, KqtMat *out) {
-    const encode_t encode = tensor_encode();
+    const tmap_encode_t encode = tmap_encode();
     if (!encode) return cudaErrorNotSupported;
     if (m.rows % KT_ROWS || m.cols % 256 || (m.type != 12 && !(m.type == 14 && m.planes)) || rows_total % KT_ROWS) return cudaErrorInvalidValue;
     const cuuint64_t dims[2] = {(cuuint64_t)m.bpr(), (cuuint64_t)rows_total}, strides[1] = {(cuuint64_t)m.bpr()};

@@ -34,6 +34,7 @@
 #include "brrr_kernels.h"
 #include "brrr_block.cuh"
 #include "brrr_tma.cuh"
+#include "brrr_tc.cuh"
 #include "brrr_mx.cuh"
 #include "brrr_mxt.cuh"
 
@@ -216,32 +217,22 @@ struct XtShared {
 // One block pair of one row: the 8 exact lane dots from the three digit planes, then the two
 // blocks' fused multiply-adds of the four chains, in block order.  Two chains share an instruction
 // (fma.rn.f32x2: two independent round-to-nearest fused multiply-adds).
-struct XtAcc { unsigned long long a01, a23; };       // chains (0, 1) and (2, 3), packed f32x2
-__device__ __forceinline__ unsigned long long xt_pack(uint32_t lo, uint32_t hi) {
-    unsigned long long r;
-    asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "r"(lo), "r"(hi));
-    return r;
-}
-__device__ __forceinline__ unsigned long long xt_fma2(unsigned long long a, unsigned long long b, unsigned long long c) {
-    unsigned long long r;
-    asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c));
-    return r;
-}
+struct XtAcc { f32x2 a01, a23; };       // chains (0, 1) and (2, 3), packed f32x2
 __device__ __forceinline__ void xt_pair(const uint32_t *v, float s0, float s1, XtAcc &acc) {
-    const unsigned long long k49 = xt_pack(0x42440000u, 0x42440000u), k7 = xt_pack(0x40E00000u, 0x40E00000u);
-    unsigned long long tq[4];
+    const f32x2 k49 = tl_pack2(0x42440000u, 0x42440000u), k7 = tl_pack2(0x40E00000u, 0x40E00000u);
+    f32x2 tq[4];
 #pragma unroll
     for (int i = 0; i < 4; i++)
-        tq[i] = xt_fma2(xt_pack(v[2 * i], v[2 * i + 1]), k49, xt_fma2(xt_pack(v[8 + 2 * i], v[9 + 2 * i]), k7, xt_pack(v[16 + 2 * i], v[17 + 2 * i])));
-    const unsigned long long p0 = xt_pack(__float_as_uint(s0), __float_as_uint(s0)), p1 = xt_pack(__float_as_uint(s1), __float_as_uint(s1));
-    acc.a01 = xt_fma2(tq[0], p0, acc.a01); acc.a23 = xt_fma2(tq[1], p0, acc.a23);
-    acc.a01 = xt_fma2(tq[2], p1, acc.a01); acc.a23 = xt_fma2(tq[3], p1, acc.a23);
+        tq[i] = tl_fma2(tl_pack2(v[2 * i], v[2 * i + 1]), k49, tl_fma2(tl_pack2(v[8 + 2 * i], v[9 + 2 * i]), k7, tl_pack2(v[16 + 2 * i], v[17 + 2 * i])));
+    const f32x2 p0 = tl_pack2(__float_as_uint(s0), __float_as_uint(s0)), p1 = tl_pack2(__float_as_uint(s1), __float_as_uint(s1));
+    acc.a01 = tl_fma2(tq[0], p0, acc.a01); acc.a23 = tl_fma2(tq[1], p0, acc.a23);
+    acc.a01 = tl_fma2(tq[2], p1, acc.a01); acc.a23 = tl_fma2(tq[3], p1, acc.a23);
 }
 __device__ __forceinline__ float xt_row_sum(const XtAcc &acc) {       // (a0 + a1) + (a2 + a3)
-    uint32_t a0, a1, a2, a3;
-    asm("mov.b64 {%0, %1}, %2;" : "=r"(a0), "=r"(a1) : "l"(acc.a01));
-    asm("mov.b64 {%0, %1}, %2;" : "=r"(a2), "=r"(a3) : "l"(acc.a23));
-    return __fadd_rn(__fadd_rn(__uint_as_float(a0), __uint_as_float(a1)), __fadd_rn(__uint_as_float(a2), __uint_as_float(a3)));
+    float a0, a1, a2, a3;
+    tl_unpack2(acc.a01, a0, a1);
+    tl_unpack2(acc.a23, a2, a3);
+    return __fadd_rn(__fadd_rn(a0, a1), __fadd_rn(a2, a3));
 }
 
 template <bool DOWN, bool EP>

@@ -4,8 +4,8 @@
 // computed by the same operation sequence as in the one-token kernels, so results are bit-identical
 // to the token-serial schedule.
 //
-//   rmsnorm_quant (grid = rows)      one CTA per row, the one-token kernel with row offsets (kernels_small.cu)
-//   q8_rows_kernel                   Q8 matrix x the Q8 activations of the rows: a CTA = 16 matrix rows x 8 token rows;
+//   rows_norm_kernel                 one CTA per row: the previous experts' outputs onto the residual, norm, Q8, activation image
+//   q8_rows_kernel                   Q8 matrix x the Q8 activations of few rows: a CTA = 16 matrix rows x 8 token rows;
 //                                    its weights go into registers once (before the dependency wait), the rows'
 //                                    activations into shared memory, then one chain walk per four token rows
 //   kv_append_rows_kernel            RoPE of every row's k and the cache append of k and v, before any row attends
@@ -13,6 +13,7 @@
 #include "brrr_kernels.h"
 #include "brrr_block.cuh"
 #include "brrr_tma.cuh"
+#include "brrr_tc.cuh"
 #include "brrr_tile.cuh"
 
 namespace brrr {
@@ -21,28 +22,6 @@ namespace {
 
 constexpr int QR_THREADS = 128;
 constexpr int QR_TPC = 8;               // token rows per CTA (blockIdx.y walks the groups)
-
-// packed pairs of floats (mul / fma .rn.f32x2)
-__device__ __forceinline__ unsigned long long qr_pack2(float lo, float hi) {
-    unsigned long long r;
-    asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "r"(__float_as_uint(lo)), "r"(__float_as_uint(hi)));
-    return r;
-}
-__device__ __forceinline__ void qr_unpack2(unsigned long long v, float &lo, float &hi) {
-    uint32_t a, b;
-    asm("mov.b64 {%0, %1}, %2;" : "=r"(a), "=r"(b) : "l"(v));
-    lo = __uint_as_float(a); hi = __uint_as_float(b);
-}
-__device__ __forceinline__ unsigned long long qr_mul2(unsigned long long a, unsigned long long b) {
-    unsigned long long r;
-    asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
-    return r;
-}
-__device__ __forceinline__ unsigned long long qr_fma2(unsigned long long a, unsigned long long b, unsigned long long c) {
-    unsigned long long r;
-    asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c));
-    return r;
-}
 
 struct Q8RowsArgs {
     Q8Dev m;
@@ -95,18 +74,18 @@ __global__ void __launch_bounds__(QR_THREADS) q8_rows_kernel(Q8RowsArgs a) {
     // rows (0, 1) and (2, 3) share the float instructions (mul / fma .f32x2: two independent round-to-nearest operations)
     for (int t0 = 0; t0 < ntok; t0 += 4) {
         const int2 *xpt[4];
-        unsigned long long acc2[2] = {0ull, 0ull};
+        f32x2 acc2[2] = {0ull, 0ull};
 #pragma unroll
         for (int g = 0; g < 4; g++) xpt[g] = xp + (size_t)min(t0 + g, ntok - 1) * nidx + c8;      // rows past the end repeat the last one (never stored)
         const float *xst = xsc + (size_t)p * QR_TPC + t0;          // scales of rows t0 .. t0 + 3 for block 2 i + p at + 2 i * QR_TPC (rows past the end: stale, never stored)
         auto step = [&](int2 wv, float sv, int i) {
-            const unsigned long long s2 = qr_pack2(sv, sv);
+            const f32x2 s2 = tl_pack2(__float_as_uint(sv), __float_as_uint(sv));
 #pragma unroll
             for (int h = 0; h < 2; h++) {
                 const int2 xa = xpt[2 * h][i * 8], xb = xpt[2 * h + 1][i * 8];
                 const int da = __dp4a(wv.y, xa.y, __dp4a(wv.x, xa.x, 0)), db = __dp4a(wv.y, xb.y, __dp4a(wv.x, xb.x, 0));
-                const unsigned long long sx2 = qr_mul2(s2, *reinterpret_cast<const unsigned long long *>(xst + (size_t)2 * i * QR_TPC + 2 * h));
-                acc2[h] = qr_fma2(qr_pack2((float)da, (float)db), sx2, acc2[h]);
+                const f32x2 sx2 = tl_mul2(s2, *reinterpret_cast<const f32x2 *>(xst + (size_t)2 * i * QR_TPC + 2 * h));
+                acc2[h] = tl_fma2(tl_pack2(__float_as_uint((float)da), __float_as_uint((float)db)), sx2, acc2[h]);
             }
         };
         if (NP > 0) {
@@ -116,8 +95,8 @@ __global__ void __launch_bounds__(QR_THREADS) q8_rows_kernel(Q8RowsArgs a) {
             for (int i = 0; i < np; i++) step(__ldg(wp + (size_t)i * (Q8_UNIT / 8)), __ldg(sp + (size_t)i * (Q8_UNIT / 4)), i);
         }
         float acc[4];
-        qr_unpack2(acc2[0], acc[0], acc[1]);
-        qr_unpack2(acc2[1], acc[2], acc[3]);
+        tl_unpack2(acc2[0], acc[0], acc[1]);
+        tl_unpack2(acc2[1], acc[2], acc[3]);
 #pragma unroll
         for (int g = 0; g < 4; g++) {
             float r = __fadd_rn(acc[g], __shfl_xor_sync(0xffffffffu, acc[g], 4));      // acc_even + acc_odd per lane, then (l0+l1)+(l2+l3)

@@ -37,6 +37,7 @@
 #include "brrr_tc.cuh"
 #include "brrr_mx.cuh"
 #include "brrr_tile.cuh"
+#include "brrr_tmap.h"
 
 namespace brrr {
 
@@ -502,14 +503,7 @@ __global__ void __launch_bounds__(TL_MAXTOK) tile_route_kernel(const int32_t *__
 // The 16-row units of an MXFP4 matrix as a tensor of 4-bit elements: [pair][unit][8 = (row half, lane chain)][128 = 8 rows x 16 codes], boxes of
 // `units` units of one pair.  In shared memory 16 codes take 16 bytes (the upper 8 unused), the form tcgen05 reads 4-bit operands in.
 cudaError_t mx_tensor_map(MxDev w, int units, CUtensorMap *map) {
-    typedef CUresult (*encode_t)(CUtensorMap *, CUtensorMapDataType, cuuint32_t, void *, const cuuint64_t *, const cuuint64_t *, const cuuint32_t *,
-                                 const cuuint32_t *, CUtensorMapInterleave, CUtensorMapSwizzle, CUtensorMapL2promotion, CUtensorMapFloatOOBfill);
-    static encode_t encode = [] {
-        void *f = nullptr;
-        cudaDriverEntryPointQueryResult r;
-        if (cudaGetDriverEntryPointByVersion("cuTensorMapEncodeTiled", &f, 12000, cudaEnableDefault, &r) != cudaSuccess || r != cudaDriverEntryPointSuccess) f = nullptr;
-        return (encode_t)f;
-    }();
+    const tmap_encode_t encode = tmap_encode();
     if (!encode) return cudaErrorNotSupported;
     const cuuint64_t np = (cuuint64_t)w.blocks / 2;
     const cuuint64_t dims[4] = {128, 8, (cuuint64_t)w.rows / 16, np}, strides[3] = {64, np * MX_UNIT, MX_UNIT};
