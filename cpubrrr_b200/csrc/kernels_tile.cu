@@ -514,14 +514,19 @@ cudaError_t mx_tensor_map(MxDev w, int units, CUtensorMap *map) {
 }
 
 // Tokens per CTA.  Experts: by the entries an expert has on average - few tokens keep more CTAs and copies in flight (up to 16 rows
-// the launch is a stream of weights), many amortise the products' reads of operand A.  One matrix: a CTA per SM, so the fewest
-// rounds of 148 CTAs, a round of 8, 16 or 32 tokens taking 30, 33 and 47 us at 64 pairs (64 rows x 2880 outputs: 92 CTAs of 16 tokens, 33 us;
-// 184 of 8 tokens are two rounds, 65 us).
+// the launch is a stream of weights), many amortise the products' reads of operand A.  The lines lie where whole prompts of the 20b shape (4 of 32
+// experts: an eighth of the rows each) cross, ms with 8 / 16 / 32 tokens per CTA: 64 rows 7.97 / 8.20 / 10.53, 72 rows 8.30 / 8.35 / 10.53,
+// 80 rows 9.06 / 8.95 / 10.96, 128 rows 12.82 / 12.43 / 12.72, 136 rows 13.25 / 12.82 / 12.86, 144 rows 13.70 / 13.26 / 13.01.
+// One matrix: a CTA per SM, so the fewest rounds of 148 CTAs, a round of 8, 16 or 32 tokens weighing 30, 33 and 47.  Its time follows the rows in it:
+// 19, 21 and 23 to 35 us at 45 pairs, 24, 27 and 30 to 45 us at 64 pairs, 20, 21 and 25 to 32 us of the vocabulary's 11 rounds.  Over 8 to 512 rows
+// of the 20b shape's three matrices the weights pick the fastest (12, 64 rows x 2880 outputs: 24 / 26 / 29 and 47 / 29 / 44 us; 33 rows x the
+// vocabulary 526 us with 32 tokens, 664 with 16), or at most 8 % more where full rounds of 32 meet three of 16 (128 rows x 5120 outputs 64 against
+// 59 us, 256 x 2880 87 against 80); weights of 18, 20 and 32, which these two would ask for, lose 26 % at 33 rows x the vocabulary.
 template <int KIND>
 cudaError_t tl_launch(TileArgs a, int tiles, int entries, int experts, bool pdl, cudaStream_t st) {
     const int avg = (entries + experts - 1) / experts, most = a.cnt ? a.ntok : entries;
     if (most < 1 || most > TL_MAXTOK) return cudaErrorInvalidValue;
-    int nt = avg > 12 ? 32 : avg > 6 ? 16 : 8;
+    int nt = avg > 17 ? 32 : avg > 9 ? 16 : 8;
     if (!a.cnt) {
         auto cost = [&](int n, int round) { return ((tiles * ((entries + n - 1) / n) + 147) / 148) * round; };
         nt = 8;

@@ -962,8 +962,10 @@ static void rows_scores_alloc(brrr_model *m) {
     if (m->alloc(&m->tl_scores, (size_t)BRRR_TILE_MAX * m->cfg.n_head * BRRR_MAXSEQ) != BRRR_OK) m->no_attn_rows = true;
 }
 
-// Rows from which the Q8 projections of a pass run on the tensor cores.
-constexpr int ROWS_TENSOR_FROM = 9;
+// Rows from which the Q8 projections of a pass run on the tensor cores.  There 128 matrix rows share a CTA, so few rows leave most SMs idle: q|k|v
+// takes 20 us and the output projection 25 whatever the rows are, the integer units 20 and 15 us at 12 rows, 25 and 23 at 16, 36 and 27 at 24.
+// A batched step on the integer units / the tensor cores: 12 rows 5.09 / 5.38 ms, 14 rows 5.55 / 5.57, 16 rows 5.66 / 5.64, 24 rows 6.40 / 6.11.
+constexpr int ROWS_TENSOR_FROM = 16;
 
 static int enqueue_rows(brrr_model *m, int n, int kind, bool pdl) {
     const bool batch = kind != ROWS_PROMPT, one_sequence = kind != ROWS_BATCH;
@@ -1143,7 +1145,8 @@ static int batch_check(brrr_model *m, int n, const uint32_t *toks, const uint32_
     return BRRR_OK;
 }
 
-// Rows from which the vocabulary projection of a batch runs on the tensor cores.
+// Rows from which the vocabulary projection of a batch runs on the tensor cores: 225 us for 4 rows, 226 for 5, 230 for 8; the integer units walk the
+// matrix per four rows, 194 us for 4, 292 for 5, 319 for 8.
 constexpr int HEAD_TENSOR_FROM = 5;
 
 // n floats from the device to the caller's memory, in chunks through a pinned ring: the copy of a chunk to pageable memory by this thread runs

@@ -124,7 +124,7 @@ def memory(cfg, prompt):
     def same(a, b):
         return all(np.array_equal(x, y) for x, y in zip(a, b))
 
-    n = 12                                                  # rows enough for the tensor-core projections and head
+    n = 16                                                  # rows enough for the tensor-core projections and head
     eng = B.Engine.synth(cfg, 17)
     eng.batch_open(n)
     want = use(eng, n)

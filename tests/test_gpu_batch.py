@@ -97,6 +97,24 @@ def test_batch_ragged_and_mixed_rows(brrr):
     eng.close()
 
 
+@pytest.mark.parametrize("n", [4, 5, 9, 15, 16, 18, 19, 34, 35])
+def test_rows_where_their_kernels_change(brrr, n):
+    """Row counts on both sides of the lines of the dispatch: head (5) and projections (16) on the tensor cores, and - half of the rows reach an
+    expert here - 8, 16 and 32 tokens per CTA of the experts (9 | 10 and 17 | 18 entries)."""
+    cfg = brrr.make_cfg(256, 2, 8, 2, 8, 4, 1024, sliding_window=8)
+    eng = brrr.Engine.synth(cfg, 31)
+    prompt = [int(t) for t in S.synth_prompt(31, n, 1000)]
+    want = []
+    for i, t in enumerate(prompt):
+        want.append((eng.run(t, i, True), bits(eng.logits())))
+    assert eng.prefill(prompt) == want[-1][0] and np.array_equal(bits(eng.logits()), want[-1][1])
+    eng.batch_open(2)
+    out, lg = eng.batch_step(prompt, list(range(n)), [1] * n, logits=True)
+    for i in range(n):
+        assert int(out[i]) == want[i][0] and np.array_equal(bits(lg[i]), want[i][1]), f"row {i}"
+    eng.close()
+
+
 @pytest.mark.parametrize("n", [1, 3, 30])
 def test_batch_logits_longer_than_the_pinned_ring(brrr, n):
     """Logits leave in 65536-float chunks through a ring of sixteen: less than one chunk, a few, and more than the ring holds."""
