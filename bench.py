@@ -286,7 +286,7 @@ def run_moe_tile(args):
     best = rows[-1]["tile_tcgen05"]
     print(json.dumps({"metric": "MoE FFN stage token-layers/s (gpt-oss-20b layers, token tiles on tcgen05)", "value": best["token_layers_per_s"],
                       "unit": "token-layers/s", "n_gpus": 1, "steps": args.steps, "warmup": args.warmup, "ms_per_step": best["ms_per_pass"],
-                      "higher_is_better": True, "scaling": "weak", "vs_baseline": None, "dtype": "int8xfp4->int32 (tcgen05 kind::i8),f32",
+                      "higher_is_better": True, "scaling": "weak", "vs_baseline": None, "dtype": "int8xfp4 and int8 products exact in f32 (tcgen05 kind::f8f6f4, kind::f16),f32",
                       "data": "synthetic", "config": {"workload": "gpt-oss-20b MoE FFN stage on tiles of 1/4/16 tokens, all layers, host-synchronous calls",
                                                       "l2": "inputs larger than L2 (every pass streams the selected experts of all layers)"},
                       "tiles": rows}), flush=True)
@@ -352,7 +352,7 @@ def run_batched(args):
     best = max(rows, key=lambda r: r["tok_s"])
     print(json.dumps({"metric": "batched decode tok/s (gpt-oss-20b shape, independent sequences)", "value": best["tok_s"], "unit": "tok/s", "n_gpus": 1,
                       "steps": steps, "warmup": max(args.warmup, 3), "ms_per_step": best["ms_per_pass"], "higher_is_better": True, "scaling": "weak",
-                      "vs_baseline": None, "dtype": "int8xfp4->int32 (tcgen05 kind::i8), int8 dp4a, f32", "data": "synthetic",
+                      "vs_baseline": None, "dtype": "int8xfp4 and int8 products exact in f32 (tcgen05 kind::f8f6f4, kind::f16) or int32 (dp4a), f32", "data": "synthetic",
                       "config": {"workload": "gpt-oss-20b batched greedy decode, 32-token prompts, b = 1/4/16/64/256 sequences (one 403 MB KV cache each), wall clock through Engine.batch_step",
                                  "l2": "inputs larger than L2 (every pass streams the dense layers, the routed experts and the vocabulary projection)"},
                       "batches": rows, "one_sequence_decode_tok_s": serial_tok_s,
@@ -416,7 +416,7 @@ def run_prefill(args):
     dt_tile = time.perf_counter() - t0
     print(json.dumps({"metric": "prefill tok/s (gpt-oss-20b shape, one 2048-token prompt)", "value": n / dt_tile, "unit": "tok/s", "n_gpus": 1,
                       "steps": n, "warmup": 16, "ms_per_step": 1000 * dt_tile / n, "higher_is_better": True, "scaling": "weak", "vs_baseline": None,
-                      "dtype": "int8xfp4->int32 (tcgen05 kind::i8),f32", "data": "synthetic",
+                      "dtype": "int8xfp4 and int8 products exact in f32 (tcgen05 kind::f8f6f4, kind::f16),f32", "data": "synthetic",
                       "config": {"workload": f"gpt-oss-20b prefill, 2048-token prompt, tiles of {tile_rows} tokens, wall clock through Engine.run_tile",
                                  "l2": "inputs larger than L2 (every tile streams the dense layers per token and the routed experts per tile)"},
                       "serial": {"tok_s": sample / dt_serial, "sample_tokens": sample}, "tiles_on_sample": {"tok_s": sample / dt_tile_sample, "sample_tokens": sample},
