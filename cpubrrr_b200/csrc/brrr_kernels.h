@@ -177,7 +177,7 @@ cudaError_t launch_down_t(MxtDev down, const float *down_b, const int32_t *top, 
 // Activations come as images (brrr_tile.cuh), image_bytes(rows, cols, kind) each, and block scales [row][cols / 32].
 size_t image_bytes(int rows, int cols, int kind);      // plane images must be zero before their first use
 void launch_image(const int8_t *xq, int rows, int cols, int kind, uint8_t *img, cudaStream_t st);      // kind = TI_HALF or TI_PLANES
-// Q8 matrix re-laid as operand units (the weights as halves in operand order, 2.1 x the Q8 bytes)
+// Q8 matrix re-laid as operand units (the weights as halves in operand order, 1.9 x the Q8 bytes)
 size_t q8_operand_bytes(int rows, int cols);
 void launch_q8_operand_pack(Q8Dev m, uint8_t *out, cudaStream_t st);
 cudaError_t launch_q8_tile(const uint8_t *op, int rows, int cols, const uint8_t *img, const float *xs, int ntok, const float *bias, float *y, int ldy,

@@ -5,7 +5,7 @@
 // changing bits, so one lane owns one expert and walks the whole row: 4 cycles of dependent
 // FADD latency per element is the floor of this stage.  The lane is kept fed from a ring of
 // shared-memory tiles; each tile is ONE bulk asynchronous copy, because the router matrix is
-// re-laid at load time as [32-expert group][tile][32 experts][128 + 4 floats] (the 4-float row
+// re-laid at load time as [32-expert group][tile][32 experts][256 + 4 floats] (the 4-float row
 // padding makes a 128-bit read per lane bank-conflict free).  Experts are split 32 per CTA; with
 // several CTAs the last one to finish runs the top-k.
 #include "brrr_kernels.h"

@@ -82,7 +82,7 @@ int brrr_forward_tile(brrr_model *m, const uint32_t *toks, uint32_t n, uint32_t 
 
 /* Schedule of brrr_forward_tile.  on != 0 (default): tiles of up to BRRR_TILE_MAX tokens walk the layers
  * together as in forward_tile_worker (src/bin/engine_gpt2.rs:1011-1250, where TILE = 16): q/k/v and the
- * output projection once per 16 rows, attention for all rows in one launch, the MoE block once per layer
+ * output projection from one pass over the weights, attention for all rows in one launch, the MoE block once per layer
  * and tile on the tensor-core tile kernels.  on = 0: one graph launch per token.  Same bits either way;
  * the environment variables BRRR_TILE_PREFILL=0/1 and BRRR_TILE_ROWS=n (2..BRRR_TILE_MAX) set the initial
  * values.  Ignored by expert-parallel ranks (always token-serial). */
@@ -91,9 +91,8 @@ int brrr_model_set_tile_prefill(brrr_model *m, int on);
 /* Batched decode over independent sequences.  The reference decodes one sequence; its tile path
  * (forward_tile_worker, src/bin/engine_gpt2.rs:1011-1250) already walks several token rows through a
  * layer together and groups them by routed expert (the `subs` / `active` lists, :1160-1172).  Here a
- * row is (token, position, sequence): every sequence has its own KV cache, the dense projections and
- * the vocabulary projection read their weights once per 8 rows, each selected expert is read once
- * for all the rows routed to it.  Every row's result is bit-identical to brrr_forward on that
+ * row is (token, position, sequence): every sequence has its own KV cache, the dense projections, the
+ * vocabulary projection and every selected expert read their weights once for the rows of a pass (few rows: once per 8).  Every row's result is bit-identical to brrr_forward on that
  * sequence alone.
  *   brrr_batch_open     allocates nseq (1..BRRR_BATCH_MAX) caches (0.4 GB each at the 20b shape) and the rows' logits (0.4 GB); once per
  *                       model, not with expert-parallel ranks.  Where the caches only fit without the projections' operand copies,
@@ -369,7 +368,7 @@ void brrr_mxmat_free(brrr_mxmat *m);
 int brrr_mx_matvec(const brrr_mxmat *w, int row0, int nrows, const int8_t *d_xq, const float *d_xs, float *d_y, int32_t *d_blockdots, void *stream);
 
 /* The same product for a tile of up to BRRR_TILE_MAX tokens in one pass over the weights, on the tcgen05
- * tensor cores (int8 MMA into tensor memory, float chains in the epilogue): d_y[t * ldy + i] = row
+ * tensor cores (exact products in tensor memory, float chains in the epilogue): d_y[t * ldy + i] = row
  * (row0 + i) . activation t, each value bit-identical to brrr_mx_matvec on token t alone.
  * d_xq [ntok][blocks * 32] int8, d_xs [ntok][blocks].  Replaces the expert products of the tile
  * path (forward_tile_worker, src/bin/engine_gpt2.rs:1011-1250, TILE = 16). */

@@ -89,7 +89,7 @@ def test_q8_pack_and_matvec(L, orc, dev, rows, cols):
 @pytest.mark.parametrize("rows,cols,ntok", [(64, 64, 1), (96, 2880, 5), (36, 4096, 16), (1028, 128, 9), (5120, 2880, 64), (2880, 4096, 33)])
 def test_q8_matmul_rows_equal_oracle_on_both_engines(L, orc, dev, rows, cols, ntok):
     """Q8 matrix x token rows (the q/k/v and o-proj products of a tile) on the integer units and on the tcgen05
-    kind::i8 tensor-core kernel: every output equals the oracle's one-row dot bit for bit; nothing is written
+    tensor-core kernel: every output equals the oracle's one-row dot bit for bit; nothing is written
     beyond the matrix rows (ldy > rows), ragged row tiles and chunks included."""
     import torch
     wb = S.synth_bf16(rows + ntok, 1, S.T["WQ"], rows * cols)
