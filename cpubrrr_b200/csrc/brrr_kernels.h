@@ -136,9 +136,10 @@ struct EpCtx {
     unsigned long long *pairs[EP_MAX_WORLD];
 };
 // ---- single-token expert matvecs on the tensor cores in native fp4 (kernels_mxt.cu)
-// Tile units: [expert][tile of 128 rows][block pair][4096 B operand image | 128 x 2 e8m0 bytes].
-constexpr int MXT_UNIT = 4352;
-constexpr int MXT_UNIT_EXPS = 4096;
+// Tile units: [expert][tile of 128 rows][two block pairs][4096 B operand image per pair | 128 x 4 e8m0 bytes].
+constexpr int MXT_PAIR = 4096, MXT_SCALES = 512;
+// block exponents whose products with any activation scale are exact (kernels_mxt.cu)
+constexpr int XT_EXP_MIN = 49, XT_EXP_MAX = 190;
 struct MxtDev {
     uint8_t *data;
     int tiles_per_expert, np;
@@ -147,13 +148,14 @@ size_t mxt_bytes(int experts, int tiles_per_expert, int np);
 // b.data == nullptr: tiles of 128 rows of a (rows past the end are zero); else rows 0-63 of a tile
 // come from a and rows 64-127 from b (same 64 row indices)
 void launch_mxt_pack(MxDev a, MxDev b, int experts, int rows_per_expert, MxtDev out, cudaStream_t st);
-// The activation enters as its digit-plane operand image (brrr_mxt.cuh; [blocks / 2][768] bytes, zero
-// except for the words its producer writes) and its block scales.
-void launch_xt_bimg(const int8_t *xq, int nb, uint8_t *bimg, cudaStream_t st);
+// *bad |= 1 when `blocks` GGUF blocks hold an exponent outside XT_EXP_MIN .. XT_EXP_MAX (zero blocks may lie below)
+void launch_mx_exp_scan(const uint8_t *raw, size_t blocks, uint32_t *bad, cudaStream_t st);
+// The activation enters as its digits (brrr_mxt.cuh; [blocks][48] bytes) and its block scales.
+void launch_xt_digits(const int8_t *xq, int nb, uint8_t *dig, cudaStream_t st);
 // same results, bit for bit, as launch_gate_up / launch_down_combine on the same Q8 activation;
-// himg: [topk][blocks / 2][768] operand images of h for launch_down_t
+// hdig: [topk][blocks][48] digits of h for launch_down_t
 cudaError_t launch_gate_up_t(MxtDev gu, const float *gate_b, const float *up_b, const int32_t *top, const float *est, int ne, int topk,
-                             int d, const uint8_t *ximg, const float *xs, int8_t *hq, float *hs, uint8_t *himg, DevState *state,
+                             int d, const uint8_t *xdig, const float *xs, int8_t *hq, float *hs, uint8_t *hdig, DevState *state,
                              bool pdl, cudaStream_t st, const EpCtx *ep = nullptr, int layer = 0);
 // part: [topk][tiles_per_expert * 128] floats of scratch; counter: [tiles_per_expert] words, zero before the first launch.
 // wts != nullptr (exact routing in top/wts, est == nullptr): the last CTA of a row tile folds it onto x.
@@ -170,7 +172,7 @@ cudaError_t launch_fold_norm(const int32_t *top, const float *wts, const float *
                              uint32_t *router_seq, uint32_t *fold_seq, DevState *state, bool pdl, cudaStream_t st,
                              const EpCtx *ep = nullptr, int layer = 0);
 cudaError_t launch_down_t(MxtDev down, const float *down_b, const int32_t *top, const float *wts, const float *est, int ne, int topk,
-                          int d, const uint8_t *himg, const float *hs, float *x, float *part, uint32_t *counter, DevState *state,
+                          int d, const uint8_t *hdig, const float *hs, float *x, float *part, uint32_t *counter, DevState *state,
                           bool pdl, cudaStream_t st, const EpCtx *ep = nullptr, int layer = 0);
 
 // ---- matrices x token rows on the tensor cores (kernels_tile.cu), t < ntok <= BRRR_TILE_MAX, every value bit-identical to the one-token kernels.
@@ -222,8 +224,8 @@ bool ffn_in_takes_half_an_sm();           // its registers, as built: no more th
 // normalised vector (each CTA writes a share).
 cudaError_t launch_router_hint(const float *x_in, const float *norm_w, float eps, int d, const float *Wt, const float *b, int ne, int topk,
                                float *est, int8_t *xq_out, float *xs_out, DevState *state, bool pdl, cudaStream_t st,
-                               uint8_t *bimg_out = nullptr);
-// bimg_out (nullable): also the operand image of the quantised vector for the tensor-core expert kernels
+                               uint8_t *dig_out = nullptr);
+// dig_out (nullable): also the digits of the quantised vector for the tensor-core expert kernels
 
 // ---- attention (kernels_attn.cu)
 // KV cache layout [n_head_kv][BRRR_MAXSEQ][64].  pos is read from state when state != nullptr,

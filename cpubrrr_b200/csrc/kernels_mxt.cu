@@ -6,34 +6,41 @@
 // Arithmetic (bit-identical to the integer-unit kernels of kernels_mx.cu).  A row's value is four
 // lane chains, chain j accumulating fma(float(t_j(b)), 2^(e_b-128) * xs[b], acc) over the 32-blocks
 // b, where t_j(b) is the exact integer dot of the lane's 8 doubled e2m1 values with the lane's 8
-// activation bytes.  The tensor core supplies t_j(b):
-//   * an activation byte x in [-127, 127] is written as 49 a + 7 b + c with digits in [-3, 3];
-//     twice a digit (0, +-2, +-4, +-6) is an e2m1 value, and (true e2m1 value) x (twice the digit)
-//     = (doubled e2m1 value) x digit, so the three digit planes give three exact partial sums;
+// activation bytes.  The tensor core supplies t_j(b) 2^(e_b-128):
+//   * an activation byte x in [-127, 127] is written as 64 a + 8 b + c with digits in [-4, 4], and half a
+//     digit is an e2m1 value whose code is the digit itself: three digit planes give three exact partial sums;
 //   * one MMA covers a block pair (K = 64): operand A = 128 weight rows x 64 codes, operand B = 24
 //     columns (digit plane t, block of the pair q, lane j), each holding the plane's codes of the 8
-//     positions of lane j in block q and zero elsewhere; all block scales are 1 (ue8m0 0x7F);
-//   * every product and partial sum is a small dyadic number (|sum| <= 8 * 12 * 3), exact in the
-//     f32 accumulator, and t_j(b) = fma(D_a, 49, fma(D_b, 7, D_c)) is exact as well.
-// The four epilogue warps read the 24 accumulator columns of their rows from tensor memory
-// (tcgen05.ld) and run the float chains, one thread per row.
+//     positions of lane j in block q and zero elsewhere;
+//   * the row's block scale is the block's own e8m0 byte (2^(e-127), true e2m1 values), the column's is 128, 16 or 2 for its plane
+//     (ue8m0 134, 131, 128) in its own block and 2^-127 in the other, whose products are all zero: column t holds
+//     64, 8 or 1 times its plane's partial sum, times 2^(e_b-128);
+//   * every sum is an integer of at most 14 bits times 2^(e_b-128), exact in the f32 accumulator, and so are the two additions that
+//     join the planes.  The product of that sum with xs[b] is the exact t_j 2^(e_b-128) xs[b] of the chain's definition whenever
+//     2^(e_b-128) xs[b] neither underflows nor overflows: xs >= 1e-12 / 127, so exponents XT_EXP_MIN .. XT_EXP_MAX qualify
+//     (launch_mx_exp_scan; a model with others keeps the integer-unit kernels).
+// The eight epilogue warps read the accumulator columns of their rows from tensor memory
+// (tcgen05.ld) and run the float chains, a thread for two chains of a row.
 //
-// Layout ("tile units").  A tile is 128 matrix rows; its unit for block pair p is the 4096-byte
-// shared-memory image of operand A in the canonical K-major no-swizzle layout (16-byte chunk of
-// (row m, block q) at q * 2048 + (m / 8) * 128 + (m % 8) * 16, the chunk being the 16 nibble bytes
-// of the GGUF block) followed by 128 x 2 e8m0 bytes.  The units of a tile are contiguous, so any run
-// of them is one bulk copy.  Gate and up share tiles (rows 0-63 gate, 64-127 up, same 64 outputs),
+// Layout ("tile units").  A tile is 128 matrix rows; per two block pairs: the 4096-byte shared-memory image of operand A of either pair
+// in the canonical K-major no-swizzle layout (16-byte chunk of (row m, block q) at q * 2048 + (m / 8) * 128 + (m % 8) * 16, the chunk
+// being the 16 nibble bytes of the GGUF block), then the 512 bytes of the rows' e8m0 bytes of the four blocks in the order tensor
+// memory wants block scales in (row m at (m % 32) * 16 + (m / 32) * 4 + block), so that one tcgen05.cp moves them there.  A tile is
+// contiguous, so any run of these groups is one bulk copy.  Gate and up share tiles (rows 0-63 gate, 64-127 up, same 64 outputs),
 // so the SwiGLU and the Q8 quantiser of h run in the same CTA.
 //
-// Operand B (brrr_mxt.cuh) is written once per activation by the kernel that quantises it (the
-// routing-estimate kernel for the token, the gate/up epilogue for h) and bulk-copied by every CTA.
+// Operand B: the digits of an activation (brrr_mxt.cuh) are written once by the kernel that quantises it (the routing-estimate kernel
+// for the token, the gate/up epilogue for h); every CTA spreads them over a zeroed image in its shared memory.
 //
-// Pipeline per CTA, in rounds of four block pairs: warp 4 issues the bulk copies into a ring of stages, an elected lane of warp 5
-// the MMAs into one of two accumulator regions (96 columns), warps 0-3 read a region at once and carry the chains.  Every wait is bounded.
+// Pipeline per CTA, in rounds of four block pairs: warp 8 issues the bulk copies into a ring of stages, an elected lane of warp 9
+// the scale copies and the MMAs into one of two accumulator regions (96 columns), warps 0-3 and 4-7 read half a region each at once and carry two chains each.
+// Every wait is bounded.
 //
-// What bounds it: the epilogue's rounds.  Clock stamps of gate/up, cycles of a round (975, twelve per row): joining the digit planes and the chains 401 - the
-// chains' own dependence is 8 multiply-adds, 35 cycles -, the rows' block scales 206, waiting for the products 184 and for the copies 125, reading tensor
-// memory 59.  13 us for gate/up and 10.2 for down at the 20b shape, 42 and 27 % of the copy bandwidth; eight epilogue warps took 1107 instead of 1088 us a step.
+// What bounds it: hand-overs and first instructions more than anything.  20b shape, position 100, gate/up from its dependency wait to its end 11.3 us
+// (14.3 with the planes joined by multiply-adds and the scales multiplied in by the epilogue) for 35 MB, down 6.9 us (8.2) for 18 MB: 1.7 us until
+// the experts are picked, 2 us until the first round is through, then 600-700 cycles a round (975), 220 of them arithmetic.
+// What did not help: announcing down's tiles to L2 from gate/up's last rounds (no change), the issuing loop unrolled by ring stage (1300 cycles
+// for each of the first four rounds: instructions met for the first time), running indices in a one-lane branch (1091 against 1050 us a step).
 #include "brrr_kernels.h"
 #include "brrr_block.cuh"
 #include "brrr_tma.cuh"
@@ -48,9 +55,15 @@ namespace {
 constexpr int XT_CH = 4;                 // block pairs per ring stage = per round of the pipeline
 constexpr int XT_REGION_COLS = XT_CH * XT_N;   // accumulator region = one round = 96 tensor-memory columns
 constexpr int XT_REGIONS = 2;
-constexpr uint32_t XT_TMEM_COLS = 256;   // 2 regions + 64 columns of unit scale factors
-constexpr int XT_SF_COL = XT_REGIONS * XT_REGION_COLS;
-constexpr int XT_THREADS = 192;
+constexpr int XT_STAGES = 4;               // two CTAs per SM at the 20b shape
+constexpr uint32_t XT_TMEM_COLS = 256;   // 2 regions, their rows' scales, the columns' scales
+constexpr int XT_SFA_COL = XT_REGIONS * XT_REGION_COLS;          // rows' block scales: four columns per two block pairs, a set per region
+constexpr int XT_SFB_COL = XT_SFA_COL + XT_REGIONS * XT_CH * 2;  // columns' scales: constant
+constexpr int XT_GROUP = 2 * MXT_PAIR + MXT_SCALES;              // bytes of two block pairs and their scales
+constexpr int XT_STAGE = XT_CH / 2 * XT_GROUP;
+__host__ __device__ constexpr uint32_t xt_run_bytes(int pairs) { return (uint32_t)(pairs * MXT_PAIR + (pairs + 1) / 2 * MXT_SCALES); }      // of a run that starts on a group
+constexpr int XT_THREADS = 320;        // eight epilogue warps, producer, issuer
+constexpr int XT_PRODUCER = 8, XT_ISSUER = 9;
 #ifdef BRRR_TEST_HOOKS
 #define XT_T0() long long xt_t0_ = clock64()
 #define XT_ACC(v) do { long long xt_t1_ = clock64(); (v) += xt_t1_ - xt_t0_; xt_t0_ = xt_t1_; } while (0)
@@ -72,15 +85,13 @@ struct PackArgs {
 __global__ void mxt_pack_kernel(PackArgs p, size_t total_words) {
     size_t idx = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
     if (idx >= total_words) return;
-    // word index within the destination: [tile][pair][1024 words of operand A | 64 words of exponents]
-    const int np = p.out.np;
-    const size_t unit = idx / (MXT_UNIT / 4);
-    const int w = (int)(idx % (MXT_UNIT / 4));
-    const int pair = (int)(unit % np);
-    const size_t tile = unit / np;
+    // word index within the destination: [tile][two pairs][1024 words of operand A per pair | 128 words of exponents]
+    const int np = p.out.np, tile_words = (int)(xt_run_bytes(np) / 4);
+    const size_t tile = idx / tile_words;
+    const int w = (int)(idx % tile_words), pair0 = w / (XT_GROUP / 4) * 2, r = w % (XT_GROUP / 4), here = min(2, np - pair0);
     const int e = (int)(tile / p.tiles_per_expert), t = (int)(tile % p.tiles_per_expert);
-    // source unit and row within it of tile row m; nullptr for rows past the end of the matrix
-    auto locate = [&](int m, int &rl) -> const uint8_t * {
+    // source unit of tile row m and pair, and the row within it; nullptr for rows past the end of the matrix
+    auto locate = [&](int m, int pair, int &rl) -> const uint8_t * {
         const MxDev &mat = (p.b.data && m >= 64) ? p.b : p.a;
         const int r = p.b.data ? t * 64 + (m & 63) : t * 128 + m;
         if (r >= p.rows_per_expert) return nullptr;
@@ -89,58 +100,86 @@ __global__ void mxt_pack_kernel(PackArgs p, size_t total_words) {
         return mat.data + mx_unit_off(row >> 4, pair, np);
     };
     uint32_t v = 0;
-    if (w < 1024) {
-        const int q = w >> 9, rem = w & 511, m = (rem >> 5) * 8 + ((rem >> 2) & 7), j = rem & 3;
-        int rl = 0;
-        const uint8_t *u = locate(m, rl);
+    int rl = 0;
+    if (r < here * 1024) {
+        const int q = (r & 1023) >> 9, rem = r & 511, m = (rem >> 5) * 8 + ((rem >> 2) & 7), j = rem & 3;
+        const uint8_t *u = locate(m, pair0 + (r >> 10), rl);
         if (u) v = *reinterpret_cast<const uint32_t *>(u + mx_word_off(rl, j) + q * 4);
     } else {
-        for (int k = 0; k < 2; k++) {                 // rows m0, m0 + 1: two exponent bytes each
-            int rl = 0;
-            const uint8_t *u = locate((w - 1024) * 2 + k, rl);
-            if (u) v |= (uint32_t)*reinterpret_cast<const unsigned short *>(u + MX_UNIT_EXPS + rl * 2) << (16 * k);
+        const int s = r - here * 1024, m = (s & 3) * 32 + (s >> 2);
+        for (int k = 0; k < 4; k++) {
+            uint32_t ex = 0x7Fu;                      // rows and blocks past the end
+            const uint8_t *u = (k >> 1) < here ? locate(m, pair0 + (k >> 1), rl) : nullptr;
+            if (u) {
+                ex = u[MX_UNIT_EXPS + rl * 2 + (k & 1)];
+                if (ex < (uint32_t)XT_EXP_MIN) ex = 0x7Fu;      // all-zero blocks only (launch_mx_exp_scan): any finite scale gives the same sums
+            }
+            v |= ex << (8 * k);
         }
     }
-    reinterpret_cast<uint32_t *>(p.out.data + unit * MXT_UNIT)[w] = v;
+    reinterpret_cast<uint32_t *>(p.out.data)[idx] = v;
+}
+
+// Block exponents of a tensor in GGUF form against the range of the scaled products: *bad != 0 when a block with a value other than zero
+// lies below it, or any block above it.
+__global__ void mx_exp_scan_kernel(const uint8_t *__restrict__ raw, size_t blocks, uint32_t *bad) {
+    bool b = false;
+    for (size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x; i < blocks; i += (size_t)gridDim.x * blockDim.x) {
+        const uint8_t *p = raw + i * 17;
+        if (p[0] > XT_EXP_MAX) b = true;
+        else if (p[0] < XT_EXP_MIN)
+            for (int k = 1; k <= 16; k++) b |= (p[k] & 0x77) != 0;
+    }
+    if (b) atomicOr(bad, 1u);
 }
 
 // ---------------------------------------------------------------- tensor-core plumbing
-// shared-memory matrix descriptor: K-major, no swizzle; core matrix = 8 rows x 16 bytes, 128 bytes
-// apart along M/N, `lbo` bytes apart along K
 // block-scaled instruction descriptor: A = B = e2m1 (format 1), both K-major, N / 8 at bit 17,
-// ue8m0 scales (bit 23), M / 16 at bit 24, scale-factor ids 0, K = 64
+// ue8m0 scales (bit 23), M / 16 at bit 24, K = 64; the rows' scale-factor id (bits 29-30) is 0 or 2: bytes 0, 1 or 2, 3 of their words
 constexpr uint32_t XT_IDESC = (1u << 7) | (1u << 10) | ((uint32_t)(XT_N >> 3) << 17) | (1u << 23) | ((128u >> 4) << 24);
 
-__device__ __forceinline__ void xt_mma(uint32_t tmem_d, uint64_t desc_a, uint64_t desc_b, uint32_t tmem_sfa, uint32_t tmem_sfb) {
+// The issuing warp's instructions carry its elected lane's predicate instead of standing in a one-lane branch: the loop around them stays
+// uniform and keeps descriptors and addresses in uniform registers, where these instructions want them.
+__device__ __forceinline__ void xt_mma(uint32_t issue, uint32_t tmem_d, uint64_t desc_a, uint64_t desc_b, uint32_t idesc, uint32_t tmem_sfa, uint32_t tmem_sfb) {
     asm volatile(
-        "{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %4, 0;\n\t"
-        "tcgen05.mma.cta_group::1.kind::mxf4.block_scale.block32 [%0], %1, %2, %3, [%5], [%6], p;\n\t}"
-        ::"r"(tmem_d), "l"(desc_a), "l"(desc_b), "r"(XT_IDESC), "r"(0u), "r"(tmem_sfa), "r"(tmem_sfb)
+        "{\n\t.reg .pred p, e;\n\tsetp.ne.b32 p, %4, 0;\n\tsetp.ne.b32 e, %7, 0;\n\t"
+        "@e tcgen05.mma.cta_group::1.kind::mxf4.block_scale.block32 [%0], %1, %2, %3, [%5], [%6], p;\n\t}"
+        ::"r"(tmem_d), "l"(desc_a), "l"(desc_b), "r"(idesc), "r"(0u), "r"(tmem_sfa), "r"(tmem_sfb), "r"(issue)
         : "memory");
 }
-__device__ __forceinline__ void xt_commit(uint64_t *bar) {
-    asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(smem_u32(bar)) : "memory");
+// 512 bytes of block scales -> four columns of tensor memory, the same 32 lanes for each of its quarters; in order with the products of the issuing thread
+__device__ __forceinline__ void xt_cp_scales(uint32_t issue, uint32_t tmem, uint64_t desc) {
+    asm volatile("{\n\t.reg .pred e;\n\tsetp.ne.b32 e, %2, 0;\n\t@e tcgen05.cp.cta_group::1.32x128b.warpx4 [%0], %1;\n\t}" ::"r"(tmem), "l"(desc), "r"(issue) : "memory");
+}
+__device__ __forceinline__ void xt_commit(uint32_t issue, uint64_t *bar) {
+    asm volatile("{\n\t.reg .pred e;\n\tsetp.ne.b32 e, %1, 0;\n\t@e tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];\n\t}" ::"r"(smem_u32(bar)), "r"(issue) : "memory");
 }
 __device__ __forceinline__ void xt_fence_before() { asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory"); }
 __device__ __forceinline__ void xt_fence_after() { asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory"); }
-// The 96 accumulator columns of a region (four block pairs) of this thread's row, asynchronously:
-// the registers are valid only after xt_wait_ld96 on the same array
-__device__ __forceinline__ void xt_ld96(uint32_t taddr, uint32_t *v) {
-    asm volatile("tcgen05.ld.sync.aligned.32x32b.x64.b32 {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15,%16,%17,%18,%19,%20,%21,%22,%23,%24,%25,%26,%27,%28,%29,%30,%31,%32,%33,%34,%35,%36,%37,%38,%39,%40,%41,%42,%43,%44,%45,%46,%47,%48,%49,%50,%51,%52,%53,%54,%55,%56,%57,%58,%59,%60,%61,%62,%63}, [%64];"
-                 : "=r"(v[0]), "=r"(v[1]), "=r"(v[2]), "=r"(v[3]), "=r"(v[4]), "=r"(v[5]), "=r"(v[6]), "=r"(v[7]), "=r"(v[8]), "=r"(v[9]), "=r"(v[10]), "=r"(v[11]), "=r"(v[12]), "=r"(v[13]), "=r"(v[14]), "=r"(v[15]), "=r"(v[16]), "=r"(v[17]), "=r"(v[18]), "=r"(v[19]), "=r"(v[20]), "=r"(v[21]), "=r"(v[22]), "=r"(v[23]), "=r"(v[24]), "=r"(v[25]), "=r"(v[26]), "=r"(v[27]), "=r"(v[28]), "=r"(v[29]), "=r"(v[30]), "=r"(v[31]), "=r"(v[32]), "=r"(v[33]), "=r"(v[34]), "=r"(v[35]), "=r"(v[36]), "=r"(v[37]), "=r"(v[38]), "=r"(v[39]), "=r"(v[40]), "=r"(v[41]), "=r"(v[42]), "=r"(v[43]), "=r"(v[44]), "=r"(v[45]), "=r"(v[46]), "=r"(v[47]), "=r"(v[48]), "=r"(v[49]), "=r"(v[50]), "=r"(v[51]), "=r"(v[52]), "=r"(v[53]), "=r"(v[54]), "=r"(v[55]), "=r"(v[56]), "=r"(v[57]), "=r"(v[58]), "=r"(v[59]), "=r"(v[60]), "=r"(v[61]), "=r"(v[62]), "=r"(v[63])
-                 : "r"(taddr) : "memory");
-    asm volatile("tcgen05.ld.sync.aligned.32x32b.x32.b32 {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15,%16,%17,%18,%19,%20,%21,%22,%23,%24,%25,%26,%27,%28,%29,%30,%31}, [%32];"
-                 : "=r"(v[64]), "=r"(v[65]), "=r"(v[66]), "=r"(v[67]), "=r"(v[68]), "=r"(v[69]), "=r"(v[70]), "=r"(v[71]), "=r"(v[72]), "=r"(v[73]), "=r"(v[74]), "=r"(v[75]), "=r"(v[76]), "=r"(v[77]), "=r"(v[78]), "=r"(v[79]), "=r"(v[80]), "=r"(v[81]), "=r"(v[82]), "=r"(v[83]), "=r"(v[84]), "=r"(v[85]), "=r"(v[86]), "=r"(v[87]), "=r"(v[88]), "=r"(v[89]), "=r"(v[90]), "=r"(v[91]), "=r"(v[92]), "=r"(v[93]), "=r"(v[94]), "=r"(v[95])
-                 : "r"(taddr + 64) : "memory");
+// Half the accumulator columns of a region (two chains of four block pairs: runs of 12 columns, 24 apart) of this thread's row, as pairs.
+// Loads, wait and packing are one statement, so nothing can use a register before the wait.
+__device__ __forceinline__ void xt_ld48(uint32_t taddr, f32x2 (&v)[24]) {
+    asm volatile("{\n\t.reg .b32 r<12>;\n\t.reg .b32 s<12>;\n\t.reg .b32 t<12>;\n\t.reg .b32 u<12>;\n\t"
+                 "tcgen05.ld.sync.aligned.32x32b.x8.b32 {r0,r1,r2,r3,r4,r5,r6,r7}, [%24];\n\t"
+                 "tcgen05.ld.sync.aligned.32x32b.x4.b32 {r8,r9,r10,r11}, [%25];\n\t"
+                 "tcgen05.ld.sync.aligned.32x32b.x8.b32 {s0,s1,s2,s3,s4,s5,s6,s7}, [%26];\n\t"
+                 "tcgen05.ld.sync.aligned.32x32b.x4.b32 {s8,s9,s10,s11}, [%27];\n\t"
+                 "tcgen05.ld.sync.aligned.32x32b.x8.b32 {t0,t1,t2,t3,t4,t5,t6,t7}, [%28];\n\t"
+                 "tcgen05.ld.sync.aligned.32x32b.x4.b32 {t8,t9,t10,t11}, [%29];\n\t"
+                 "tcgen05.ld.sync.aligned.32x32b.x8.b32 {u0,u1,u2,u3,u4,u5,u6,u7}, [%30];\n\t"
+                 "tcgen05.ld.sync.aligned.32x32b.x4.b32 {u8,u9,u10,u11}, [%31];\n\t"
+                 "tcgen05.wait::ld.sync.aligned;\n\t"
+                 "mov.b64 %0, {r0,r1};\n\tmov.b64 %1, {r2,r3};\n\tmov.b64 %2, {r4,r5};\n\tmov.b64 %3, {r6,r7};\n\tmov.b64 %4, {r8,r9};\n\tmov.b64 %5, {r10,r11};\n\t"
+                 "mov.b64 %6, {s0,s1};\n\tmov.b64 %7, {s2,s3};\n\tmov.b64 %8, {s4,s5};\n\tmov.b64 %9, {s6,s7};\n\tmov.b64 %10, {s8,s9};\n\tmov.b64 %11, {s10,s11};\n\t"
+                 "mov.b64 %12, {t0,t1};\n\tmov.b64 %13, {t2,t3};\n\tmov.b64 %14, {t4,t5};\n\tmov.b64 %15, {t6,t7};\n\tmov.b64 %16, {t8,t9};\n\tmov.b64 %17, {t10,t11};\n\t"
+                 "mov.b64 %18, {u0,u1};\n\tmov.b64 %19, {u2,u3};\n\tmov.b64 %20, {u4,u5};\n\tmov.b64 %21, {u6,u7};\n\tmov.b64 %22, {u8,u9};\n\tmov.b64 %23, {u10,u11};\n\t"
+                 "}"
+                 : "=l"(v[0]),"=l"(v[1]),"=l"(v[2]),"=l"(v[3]),"=l"(v[4]),"=l"(v[5]),"=l"(v[6]),"=l"(v[7]),"=l"(v[8]),"=l"(v[9]),"=l"(v[10]),"=l"(v[11]),"=l"(v[12]),"=l"(v[13]),"=l"(v[14]),"=l"(v[15]),"=l"(v[16]),"=l"(v[17]),"=l"(v[18]),"=l"(v[19]),"=l"(v[20]),"=l"(v[21]),"=l"(v[22]),"=l"(v[23])
+                 : "r"(taddr + 0), "r"(taddr + 8), "r"(taddr + 24), "r"(taddr + 32), "r"(taddr + 48), "r"(taddr + 56), "r"(taddr + 72), "r"(taddr + 80)
+                 : "memory");
 }
-// Wait for the loads in flight; the registers pass through the statement so that no use of them can
-// be scheduled before it.
-__device__ __forceinline__ void xt_wait_ld96(uint32_t *v) {
-    asm volatile("tcgen05.wait::ld.sync.aligned;"
-                 : "+r"(v[0]), "+r"(v[1]), "+r"(v[2]), "+r"(v[3]), "+r"(v[4]), "+r"(v[5]), "+r"(v[6]), "+r"(v[7]), "+r"(v[8]), "+r"(v[9]), "+r"(v[10]), "+r"(v[11]), "+r"(v[12]), "+r"(v[13]), "+r"(v[14]), "+r"(v[15]), "+r"(v[16]), "+r"(v[17]), "+r"(v[18]), "+r"(v[19]), "+r"(v[20]), "+r"(v[21]), "+r"(v[22]), "+r"(v[23]), "+r"(v[24]), "+r"(v[25]), "+r"(v[26]), "+r"(v[27]), "+r"(v[28]), "+r"(v[29]), "+r"(v[30]), "+r"(v[31]), "+r"(v[32]), "+r"(v[33]), "+r"(v[34]), "+r"(v[35]), "+r"(v[36]), "+r"(v[37]), "+r"(v[38]), "+r"(v[39]), "+r"(v[40]), "+r"(v[41]), "+r"(v[42]), "+r"(v[43]), "+r"(v[44]), "+r"(v[45]), "+r"(v[46]), "+r"(v[47]), "+r"(v[48]), "+r"(v[49]), "+r"(v[50]), "+r"(v[51]), "+r"(v[52]), "+r"(v[53]), "+r"(v[54]), "+r"(v[55]), "+r"(v[56]), "+r"(v[57]), "+r"(v[58]), "+r"(v[59]), "+r"(v[60]), "+r"(v[61]), "+r"(v[62]), "+r"(v[63]), "+r"(v[64]), "+r"(v[65]), "+r"(v[66]), "+r"(v[67]), "+r"(v[68]), "+r"(v[69]), "+r"(v[70]), "+r"(v[71]), "+r"(v[72]), "+r"(v[73]), "+r"(v[74]), "+r"(v[75]), "+r"(v[76]), "+r"(v[77]), "+r"(v[78]), "+r"(v[79]), "+r"(v[80]), "+r"(v[81]), "+r"(v[82]), "+r"(v[83]), "+r"(v[84]), "+r"(v[85]), "+r"(v[86]), "+r"(v[87]), "+r"(v[88]), "+r"(v[89]), "+r"(v[90]), "+r"(v[91]), "+r"(v[92]), "+r"(v[93]), "+r"(v[94]), "+r"(v[95])
-                 :: "memory");
-}
-__device__ __forceinline__ void xt_bar_epi() { asm volatile("bar.sync 1, 128;" ::: "memory"); }
+__device__ __forceinline__ void xt_bar_epi() { asm volatile("bar.sync 1, 256;" ::: "memory"); }       // both halves of the epilogue warps
+__device__ __forceinline__ void xt_bar_half() { asm volatile("bar.sync 2, 128;" ::: "memory"); }      // the half that finishes the rows
 
 // Waits of the pipeline loops.  The loops are executed by one warp per scheduler, so their code
 // has to stay small enough for the instruction cache next to the scheduler: the common case (phase
@@ -178,11 +217,11 @@ struct XtIssueWait {
     }
 };
 
-// Operand image of an activation that some other kernel quantised (stage-level entry points).
-__global__ void xt_bimg_kernel(const int8_t *__restrict__ xq, int nb, uint8_t *bimg) {
+// Digits of an activation that some other kernel quantised (stage-level entry points).
+__global__ void xt_digits_kernel(const int8_t *__restrict__ xq, int nb, uint8_t *dig) {
     const int b = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5), lane = threadIdx.x & 31;
     if (b >= nb) return;
-    xt_emit_block((int)xq[b * 32 + lane], lane, b, bimg);
+    xt_emit_digits((int)xq[b * 32 + lane], lane, b, dig);
 }
 
 // ---------------------------------------------------------------- the two expert kernels
@@ -194,16 +233,15 @@ struct XtArgs {
     const float *wts;           // down: nullable, see launch_down_t
     const float *est;           // nullable: router estimate; slot s belongs to its s-th largest entry
     int ne, topk, d;
-    const uint8_t *bimg;        // operand image of the activation: gate/up [np][768]; down [slot][np][768]
+    const uint8_t *bdig;        // digits of the activation (brrr_mxt.cuh): gate/up [blocks][48]; down [slot][blocks][48]
     const float *xs;            // its block scales:                gate/up [blocks];   down [slot][blocks]
-    int8_t *hq;                 // gate/up outputs: Q8 of h per slot, its scales, its operand image
+    int8_t *hq;                 // gate/up outputs: Q8 of h per slot, its scales, its digits
     float *hs;
-    uint8_t *himg;
+    uint8_t *hdig;
     float *x;                   // down: residual stream, updated in place
     float *part;                // down: [topk][tiles * 128] row sums before bias
     uint32_t *counter;          // down: [tiles] arrival counters, zero between launches
     DevState *state;
-    int stages;
     // expert parallelism (ep_on): w holds the experts [ep.e_lo, ep.e_lo + ep.e_cnt) only; CTAs of a slot
     // whose expert lives on another rank do nothing; down stores its row sums, each tagged with the step
     // number in one 64-bit word, into every rank's buffer ep.pairs ([layer][slot][d])
@@ -213,52 +251,37 @@ struct XtArgs {
 
 struct XtShared {
     unsigned char *ring, *bimg;
-    float *xsc, *tbl;
-    uint64_t *full, *empty, *dfull, *dempty, *bfull;
+    f32x2 *xsc;                 // block scales of the activation, each twice: the factor of two chains
+    uint64_t *full, *empty, *dfull, *dempty;
 };
 
-// One block pair of one row: the 8 exact lane dots from the three digit planes, then the two
-// blocks' fused multiply-adds of the four chains, in block order.  Two chains share an instruction
-// (fma.rn.f32x2: two independent round-to-nearest fused multiply-adds).
-struct XtAcc { f32x2 a01, a23; };       // chains (0, 1) and (2, 3), packed f32x2
-__device__ __forceinline__ void xt_pair(const uint32_t *v, float s0, float s1, XtAcc &acc) {
-    const f32x2 k49 = tl_pack2(0x42440000u, 0x42440000u), k7 = tl_pack2(0x40E00000u, 0x40E00000u);
-    f32x2 tq[4];
-#pragma unroll
-    for (int i = 0; i < 4; i++)
-        tq[i] = tl_fma2(tl_pack2(v[2 * i], v[2 * i + 1]), k49, tl_fma2(tl_pack2(v[8 + 2 * i], v[9 + 2 * i]), k7, tl_pack2(v[16 + 2 * i], v[17 + 2 * i])));
-    const f32x2 p0 = tl_pack2(__float_as_uint(s0), __float_as_uint(s0)), p1 = tl_pack2(__float_as_uint(s1), __float_as_uint(s1));
-    acc.a01 = tl_fma2(tq[0], p0, acc.a01); acc.a23 = tl_fma2(tq[1], p0, acc.a23);
-    acc.a01 = tl_fma2(tq[2], p1, acc.a01); acc.a23 = tl_fma2(tq[3], p1, acc.a23);
-}
-__device__ __forceinline__ float xt_row_sum(const XtAcc &acc) {       // (a0 + a1) + (a2 + a3)
-    float a0, a1, a2, a3;
-    tl_unpack2(acc.a01, a0, a1);
-    tl_unpack2(acc.a23, a2, a3);
-    return __fadd_rn(__fadd_rn(a0, a1), __fadd_rn(a2, a3));
+// One block pair of one row: two chains' scaled lane dots of its two blocks from the three digit planes, then their fused multiply-adds,
+// in block order.  Both chains share an instruction (two independent round-to-nearest operations).
+__device__ __forceinline__ void xt_pair(const f32x2 *v, f32x2 xs0, f32x2 xs1, f32x2 &acc) {
+    acc = tl_fma2(tl_add2(tl_add2(v[0], v[2]), v[4]), xs0, acc);
+    acc = tl_fma2(tl_add2(tl_add2(v[1], v[3]), v[5]), xs1, acc);
 }
 
 template <bool DOWN, bool EP>
-__global__ void __launch_bounds__(XT_THREADS) xt_expert_kernel(XtArgs a) {
+__global__ void __launch_bounds__(XT_THREADS, 2) xt_expert_kernel(XtArgs a) {
     extern __shared__ __align__(128) unsigned char smraw[];
-    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+    // the warp index as the compiler can see it: the same in every lane, so the roles' loops keep their values in uniform registers
+    const int tid = threadIdx.x, warp = __shfl_sync(0xffffffffu, tid >> 5, 0), lane = tid & 31;
     const int np = a.w.np, nb = np * 2;
     const int t = blockIdx.x, ei = blockIdx.y;
     const int nchunks = (np + XT_CH - 1) / XT_CH;
-    const size_t stage_bytes = (size_t)XT_CH * MXT_UNIT;
     XtShared sh;
     sh.ring = smraw;
-    sh.bimg = smraw + stage_bytes * a.stages;
-    sh.xsc = reinterpret_cast<float *>(sh.bimg + (size_t)np * XT_B_PAIR);
-    sh.tbl = sh.xsc + nb;
-    sh.full = reinterpret_cast<uint64_t *>(sh.tbl + 256);
-    sh.empty = sh.full + a.stages;
-    sh.dfull = sh.empty + a.stages;
+    sh.bimg = smraw + XT_STAGE * XT_STAGES;
+    sh.xsc = reinterpret_cast<f32x2 *>(sh.bimg + (size_t)np * XT_B_PAIR);
+    sh.full = reinterpret_cast<uint64_t *>(sh.xsc + nchunks * 2 * XT_CH);      // (whole rounds: the last one reads past the blocks)
+    sh.empty = sh.full + XT_STAGES;
+    sh.dfull = sh.empty + XT_STAGES;
     sh.dempty = sh.dfull + XT_REGIONS;
-    sh.bfull = sh.dempty + XT_REGIONS;
     __shared__ uint32_t tmem_base_sh;
     __shared__ int sel[8];
     __shared__ float lg[256];
+    __shared__ float half_s[128];
     __shared__ float gu_s[2][64];
     __shared__ int last_sh;
     uint32_t *err = a.state ? &a.state->err : nullptr;
@@ -268,50 +291,50 @@ __global__ void __launch_bounds__(XT_THREADS) xt_expert_kernel(XtArgs a) {
     BRRR_GT_START(a.state, DOWN ? 237 : 236);
 
     // ---- set-up that needs nothing from the kernels before
-    mx_fill_scale_table(sh.tbl, tid, XT_THREADS);
     if (tid == 0) {
-        for (int s = 0; s < a.stages; s++) { mbar_init(&sh.full[s], 1); mbar_init(&sh.empty[s], 4); }
-        for (int r = 0; r < XT_REGIONS; r++) { mbar_init(&sh.dfull[r], 1); mbar_init(&sh.dempty[r], 4); }
-        mbar_init(sh.bfull, 1);
+        for (int s = 0; s < XT_STAGES; s++) { mbar_init(&sh.full[s], 1); mbar_init(&sh.empty[s], 1); }
+        for (int r = 0; r < XT_REGIONS; r++) { mbar_init(&sh.dfull[r], 1); mbar_init(&sh.dempty[r], 8); }
         mbar_fence_init();
     }
     if (warp == 0) {
         asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(&tmem_base_sh)), "r"(XT_TMEM_COLS) : "memory");
         asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
     }
+    for (int i = tid; i < np * (XT_B_PAIR / 16); i += XT_THREADS) reinterpret_cast<uint4 *>(sh.bimg)[i] = make_uint4(0, 0, 0, 0);
+    for (int i = nb + tid; i < nchunks * 2 * XT_CH; i += XT_THREADS) sh.xsc[i] = 0ull;
     xt_fence_before();
     __syncthreads();
     xt_fence_after();
-    const uint32_t tmem_base = tmem_base_sh;
+    const uint32_t tmem_base = __shfl_sync(0xffffffffu, tmem_base_sh, 0);
     if (warp < 4) {
-        // unit scale factors (ue8m0 0x7F) in the 64 columns behind the accumulator regions, every lane
-        const uint32_t one = 0x7F7F7F7Fu, addr = tmem_base + ((uint32_t)(warp * 32) << 16) + XT_SF_COL;
-        for (int c = 0; c < 64; c += 8)
-            asm volatile("tcgen05.st.sync.aligned.32x32b.x8.b32 [%0], {%1,%1,%1,%1,%1,%1,%1,%1};" ::"r"(addr + c), "r"(one) : "memory");
+        // the columns' scales: lane n = column (plane (n % 12) / 4, block of the pair (n / 2) & 1), byte k = block k of the pair
+        const uint32_t sc = lane < XT_N ? (134u - 3u * (uint32_t)((lane % 12) >> 2)) << (8 * ((lane >> 1) & 1)) : 0u;
+        asm volatile("tcgen05.st.sync.aligned.32x32b.x4.b32 [%0], {%1,%2,%2,%2};" ::"r"(tmem_base + ((uint32_t)(warp * 32) << 16) + XT_SFB_COL), "r"(sc), "r"(0u) : "memory");
         asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
     }
     xt_fence_before();
-    __syncthreads();                 // scale factors in place before the issuing thread can reach its first MMA
+    __syncthreads();                 // scales in place before the issuing thread can reach its first MMA, the image zeroed before the digits come
     xt_fence_after();
     // ---- routing of this slot (the ei-th largest entry of the estimate, or the exact routing), the
     // weight stream, the activation image (one bulk copy) and its block scales
     int e = 0;
     bool local = true;
-    const unsigned char *src = nullptr;
+    const size_t tile_bytes = xt_run_bytes(np), expert_bytes = tile_bytes * a.w.tiles_per_expert;
+    const unsigned char *src = a.w.data + t * tile_bytes;
     const uint32_t ep_epoch = EP ? *a.ep.epoch : 0u;          // the step in flight (written by the step's first kernel)
     auto route_and_start = [&]() {
-        if (a.est && a.ne <= 32) e = warp_spec_expert(a.est, a.ne, a.topk, a.state, ei, lane);      // every warp by itself: no barrier, a tenth of the time
+        if (a.est && a.ne <= 32) e = warp_spec_expert(a.est, a.ne, a.topk, a.state, ei, lane);      // every warp by itself: no barrier
         else if (a.est) {
             block_spec_select(a.est, a.ne, a.topk, a.state, lg, sel, tid, XT_THREADS);
             __syncthreads();
             e = sel[ei];
         } else e = a.top[ei];
         local = !EP || (e >= a.ep.e_lo && e < a.ep.e_lo + a.ep.e_cnt);
-        src = a.w.data + ((size_t)(EP ? e - a.ep.e_lo : e) * a.w.tiles_per_expert + t) * np * MXT_UNIT;
-        if (local && warp == 4 && lane < min(a.stages, nchunks)) {          // one lane per copy: the first stages of the weight stream
-            const int cnt = min(XT_CH, np - lane * XT_CH);
-            mbar_expect_tx(&sh.full[lane], (uint32_t)cnt * MXT_UNIT);
-            bulk_g2s(sh.ring + stage_bytes * lane, src + (size_t)lane * stage_bytes, (uint32_t)cnt * MXT_UNIT, &sh.full[lane]);
+        src += (size_t)(EP ? e - a.ep.e_lo : e) * expert_bytes;
+        if (local && warp == XT_PRODUCER && lane < min(XT_STAGES, nchunks)) {          // one lane per copy: the first stages of the weight stream
+            const uint32_t bytes = xt_run_bytes(min(XT_CH, np - lane * XT_CH));
+            mbar_expect_tx(&sh.full[lane], bytes);
+            bulk_g2s(sh.ring + XT_STAGE * lane, src + (size_t)lane * XT_STAGE, bytes, &sh.full[lane]);
         }
     };
     // The down projection knows its expert before gate/up has finished (the routing is two kernels
@@ -324,118 +347,106 @@ __global__ void __launch_bounds__(XT_THREADS) xt_expert_kernel(XtArgs a) {
     BRRR_STAMP(a.state, SB + 2);
     BRRR_GT_GO(a.state, SB + 30);
     pdl_trigger();
-    // (gate/up learns whether its slot is local only below: it copies the image in any case)
-    const bool img_copy = early ? local : true;
-    if (img_copy && warp == 4 && lane == 31) {
-        const uint8_t *img = a.bimg + (DOWN ? (size_t)ei * np * XT_B_PAIR : 0);
-        mbar_expect_tx(sh.bfull, (uint32_t)np * XT_B_PAIR);
-        bulk_g2s(sh.bimg, img, (uint32_t)np * XT_B_PAIR, sh.bfull);
-    }
+    // the activation's block scales and digits: every load before the first store (each is a round trip to L2)
     float xs_mine = 0.0f;
-    if (tid < nb) xs_mine = (DOWN ? a.xs + (size_t)ei * nb : a.xs)[tid];      // nb <= 128: the epilogue warps hold all of it
+    if (tid < nb) xs_mine = (DOWN ? a.xs + (size_t)ei * nb : a.xs)[tid];      // nb <= 128
+    const uint4 *dig = reinterpret_cast<const uint4 *>(a.bdig + (DOWN ? (size_t)ei * nb * XT_DIG_BLOCK : 0));
+    uint4 dw[2];
+#pragma unroll
+    for (int k = 0; k < 2; k++) dw[k] = tid + k * XT_THREADS < nb * 3 ? dig[tid + k * XT_THREADS] : make_uint4(0, 0, 0, 0);      // nb * 3 <= 384
     if (!early) route_and_start();
-    if (tid < nb) sh.xsc[tid] = xs_mine;
-    if (warp < 4) xt_bar_epi();                                  // block scales visible to the epilogue warps
+    if (tid < nb) sh.xsc[tid] = tl_pack2(__float_as_uint(xs_mine), __float_as_uint(xs_mine));
+#pragma unroll
+    for (int k = 0; k < 2; k++) if (tid + k * XT_THREADS < nb * 3) xt_spread_digits(dw[k], tid + k * XT_THREADS, sh.bimg);
+    fence_proxy_async();                                         // these stores -> the tensor core's reads
+    __syncthreads();
     BRRR_STAMP(a.state, SB + 3);
 
     // Loop structure shared by the three roles: round r = ring stage r % stages = 4 block pairs =
     // accumulator region r % 2.  All indices advance incrementally.
     if (EP && !local) {
-        // the slot's expert lives on another rank: nothing to compute here (a copy in flight must land first)
-        if (img_copy && warp == 4 && lane == 31) xt_wait(sh.bfull, 0u, err, true);
-    } else if (warp == 4) {
-        // ---- producer: refill a stage once the four epilogue warps have left it
+        // the slot's expert lives on another rank: nothing to compute here
+    } else if (warp == XT_PRODUCER) {
+        // ---- producer: refill a stage once its products are complete
         if (lane == 0) {
             int s = 0;
             uint32_t par = 0;                        // parity of the release being waited for
-            for (int c = a.stages; c < nchunks; c++) {
-                const int cnt = min(XT_CH, np - c * XT_CH);
+            for (int c = XT_STAGES; c < nchunks; c++) {
+                const uint32_t bytes = xt_run_bytes(min(XT_CH, np - c * XT_CH));
                 xt_wait(&sh.empty[s], par, err, true);
-                mbar_expect_tx(&sh.full[s], (uint32_t)cnt * MXT_UNIT);
-                bulk_g2s(sh.ring + stage_bytes * s, src + (size_t)c * stage_bytes, (uint32_t)cnt * MXT_UNIT, &sh.full[s]);
-                if (++s == a.stages) { s = 0; par ^= 1u; }
+                mbar_expect_tx(&sh.full[s], bytes);
+                bulk_g2s(sh.ring + XT_STAGE * s, src + (size_t)c * XT_STAGE, bytes, &sh.full[s]);
+                if (++s == XT_STAGES) { s = 0; par ^= 1u; }
             }
         }
-    } else if (warp == 5) {
+    } else if (warp == XT_ISSUER) {
         // ---- MMA issue: one instruction per block pair, four per round into one accumulator region (the whole warp walks the loop, an
         // elected lane issues: in a one-lane branch every product costs 100 cycles of operand moves, 35 here)
         {
             XtIssueWait wait{err, err && *reinterpret_cast<volatile uint32_t *>(err) != 0u};
-            const uint32_t sfa = tmem_base + XT_SF_COL, sfb = tmem_base + XT_SF_COL + 32;
-            const uint64_t dhi = ((uint64_t)((128u >> 4) & 0x3FFF) << 32) | ((uint64_t)1 << 46);     // descriptor bits common to A and B
+            const uint32_t sfb = tmem_base + XT_SFB_COL;
+            const uint64_t dhi = ((uint64_t)((128u >> 4) & 0x3FFF) << 32) | ((uint64_t)1 << 46);     // descriptor bits common to A, B and the scales
             const uint64_t alo = dhi | ((uint64_t)((2048u >> 4) & 0x3FFF) << 16), blo = dhi | ((uint64_t)(((uint32_t)XT_B_PAIR / 2 >> 4) & 0x3FFF) << 16);
-            uint32_t baddr = smem_u32(sh.bimg) >> 4;              // descriptor start-address fields (16-byte units)
-            const uint32_t r0 = smem_u32(sh.ring) >> 4, stage16 = (uint32_t)(stage_bytes >> 4);
-            wait(sh.bfull, 0u);
+            const uint32_t b0 = smem_u32(sh.bimg) >> 4, r0 = smem_u32(sh.ring) >> 4;       // descriptor start-address fields (16-byte units)
+            const uint32_t issue = elect_one() ? 1u : 0u;
             int s = 0, reg = 0, left = np;
-            uint32_t fpar = 0, epar = 1;             // full-stage parity; region-free parity (first pass: free)
+            uint32_t fpar = 0, epar = 1, baddr = b0;             // full-stage parity; region-free parity (first pass: free)
+            // One body for every round and product: the instructions a CTA meets for the first time come from L2 or beyond and cost more
+            // than the running indices (a body per stage: 1300 cycles for each of the first four rounds).
 #pragma unroll 1
             for (int r = 0; r < nchunks; r++) {
                 wait(&sh.full[s], fpar);
                 wait(&sh.dempty[reg], epar);
                 xt_fence_after();
-                const uint32_t aaddr = r0 + s * stage16, d0 = tmem_base + reg * XT_REGION_COLS;
-                const int cnt = left < XT_CH ? left : XT_CH;
-                if (elect_one()) {
-#pragma unroll
-                    for (int k = 0; k < XT_CH; k++)
-                        if (k < cnt) xt_mma(d0 + k * XT_N, alo | (aaddr + k * (MXT_UNIT / 16)), blo | (baddr + k * (XT_B_PAIR / 16)), sfa, sfb);
-                    xt_commit(&sh.dfull[reg]);
+                const uint32_t sfa = tmem_base + XT_SFA_COL + reg * XT_CH * 2;
+                uint32_t d0 = tmem_base + reg * XT_REGION_COLS, aaddr = r0 + s * (XT_STAGE / 16), baddr1 = baddr;
+                const int cnt = min(left, XT_CH);
+#pragma unroll 1
+                for (int k = 0; k < cnt; k += 2) {
+                    const uint32_t two = cnt - k > 1 ? issue : 0u;
+                    xt_cp_scales(issue, sfa + k * 2, dhi | (aaddr + (cnt - k > 1 ? 2 : 1) * (MXT_PAIR / 16)));
+                    xt_mma(issue, d0, alo | aaddr, blo | baddr1, XT_IDESC, sfa + k * 2, sfb);
+                    xt_mma(two, d0 + XT_N, alo | (aaddr + MXT_PAIR / 16), blo | (baddr1 + XT_B_PAIR / 16), XT_IDESC | (2u << 29), sfa + k * 2, sfb);
+                    d0 += 2 * XT_N; aaddr += XT_GROUP / 16; baddr1 += 2 * XT_B_PAIR / 16;
                 }
+                xt_commit(r + XT_STAGES < nchunks ? issue : 0u, &sh.empty[s]);      // nobody waits for the last ones
+                xt_commit(issue, &sh.dfull[reg]);
                 __syncwarp();
                 baddr += XT_CH * XT_B_PAIR / 16;
                 left -= XT_CH;
-                if (++s == a.stages) { s = 0; fpar ^= 1u; }
+                if (++s == XT_STAGES) { s = 0; fpar ^= 1u; }
                 if (++reg == XT_REGIONS) { reg = 0; epar ^= 1u; }
             }
         }
     } else {
-        // ---- epilogue: thread m owns tile row m
-        const int m = tid;
-        const uint32_t lane_addr = tmem_base + ((uint32_t)(warp * 32) << 16);
-        XtAcc acc{0ull, 0ull};
+        // ---- epilogue: thread m of half h owns chains 2 h, 2 h + 1 of tile row m
+        const int m = tid & 127, h = warp >> 2;
+        const uint32_t lane_addr = tmem_base + ((uint32_t)((warp & 3) * 32) << 16) + h * (XT_N / 2);
+        f32x2 acc = 0ull;
         const float bias_pre = DOWN ? 0.0f : ((m >> 6) ? a.bias_b : a.bias_a)[(size_t)e * a.d + t * 64 + (m & 63)];   // in flight during the stream
-        uint32_t dv[XT_REGION_COLS] = {};
-        int s = 0, reg = 0, left = np;
-        uint32_t spar = 0, dpar = 0;
-        const float *xsp = sh.xsc;
-        long long tw_full = 0, tw_sc = 0, tw_d = 0, tw_ld = 0, tw_math = 0;
-        (void)tw_full; (void)tw_sc; (void)tw_d; (void)tw_ld; (void)tw_math;
+        int reg = 0, left = np;
+        uint32_t dpar = 0, xaddr = smem_u32(sh.xsc);
+        long long tw_d = 0, tw_ld = 0, tw_math = 0;
+        (void)tw_d; (void)tw_ld; (void)tw_math;
 #pragma unroll 1
         for (int r = 0; r < nchunks; r++) {
-            const int cnt = left < XT_CH ? left : XT_CH;
             XT_T0();
-            xt_wait(&sh.full[s], spar, err);                    // the stage's exponent bytes are visible
-            XT_ACC(tw_full);
-            const unsigned char *ex = sh.ring + stage_bytes * s + MXT_UNIT_EXPS + m * 2;
-            uint32_t e2[XT_CH];
+            f32x2 xs[2 * XT_CH], dv[XT_REGION_COLS / 4];
 #pragma unroll
-            for (int k = 0; k < XT_CH; k++) e2[k] = k < cnt ? *reinterpret_cast<const unsigned short *>(ex + k * MXT_UNIT) : 0u;
-            const float4 xa = *reinterpret_cast<const float4 *>(xsp), xb = *reinterpret_cast<const float4 *>(xsp + 4);
-            float sc[2 * XT_CH];                                // block scales: 2^(e-128) * xs
-            sc[0] = __fmul_rn(sh.tbl[e2[0] & 0xFFu], xa.x); sc[1] = __fmul_rn(sh.tbl[e2[0] >> 8], xa.y);
-            sc[2] = __fmul_rn(sh.tbl[e2[1] & 0xFFu], xa.z); sc[3] = __fmul_rn(sh.tbl[e2[1] >> 8], xa.w);
-            sc[4] = __fmul_rn(sh.tbl[e2[2] & 0xFFu], xb.x); sc[5] = __fmul_rn(sh.tbl[e2[2] >> 8], xb.y);
-            sc[6] = __fmul_rn(sh.tbl[e2[3] & 0xFFu], xb.z); sc[7] = __fmul_rn(sh.tbl[e2[3] >> 8], xb.w);
-            XT_ACC(tw_sc);
+            for (int k = 0; k < 2 * XT_CH; k += 2) lds_pairs(xaddr + k * 8, xs[k], xs[k + 1]);
             xt_wait(&sh.dfull[reg], dpar, err);
             XT_ACC(tw_d);
             xt_fence_after();
-            xt_ld96(lane_addr + reg * XT_REGION_COLS, dv);
-            xt_wait_ld96(dv);
+            xt_ld48(lane_addr + reg * XT_REGION_COLS, dv);
             XT_ACC(tw_ld);
             xt_fence_before();
             __syncwarp();
-            if (lane == 0) {
-                mbar_arrive(&sh.dempty[reg]);
-                mbar_arrive(&sh.empty[s]);                      // the stage's MMAs are complete and its exponents read
-            }
+            if (lane == 0) mbar_arrive(&sh.dempty[reg]);
 #pragma unroll
             for (int k = 0; k < XT_CH; k++)
-                if (k < cnt) xt_pair(dv + XT_N * k, sc[2 * k], sc[2 * k + 1], acc);
-            xsp += 2 * XT_CH;
+                if (k < left) xt_pair(dv + XT_N / 4 * k, xs[2 * k], xs[2 * k + 1], acc);
+            xaddr += 2 * XT_CH * 8;
             left -= XT_CH;
-            if (++s == a.stages) { s = 0; spar ^= 1u; }
             if (++reg == XT_REGIONS) { reg = 0; dpar ^= 1u; }
             XT_ACC(tw_math);
             if (r < 12) BRRR_STAMP(a.state, SB + 4 + r);
@@ -444,24 +455,33 @@ __global__ void __launch_bounds__(XT_THREADS) xt_expert_kernel(XtArgs a) {
 #ifdef BRRR_TEST_HOOKS
         if (a.state && tid == 0 && blockIdx.x == BRRR_STAMP_BX && blockIdx.y == 0) {
             long long *o = a.state->stamps + (DOWN ? 205 : 200);
-            o[0] = tw_full; o[1] = tw_sc; o[2] = tw_d; o[3] = tw_ld; o[4] = tw_math;
+            o[0] = tw_d; o[1] = tw_ld; o[2] = tw_math;
         }
 #endif
-        const float v = xt_row_sum(acc);
-        if (!DOWN) {
+        // row sum (a0 + a1) + (a2 + a3)
+        float c0, c1;
+        tl_unpack2(acc, c0, c1);
+        float v = __fadd_rn(c0, c1);
+        if (h) half_s[m] = v;
+        xt_bar_epi();
+        if (h) {
+            // done
+        } else if (!DOWN) {
+            v = __fadd_rn(v, half_s[m]);
             gu_s[m >> 6][m & 63] = __fadd_rn(v, bias_pre);
-            xt_bar_epi();
+            xt_bar_half();
             if (warp < 2) {
-                // SwiGLU, Q8 of this 32-block of h, and its share of the operand image down reads
+                // SwiGLU, Q8 of this 32-block of h, and the digits down reads
                 const float h = swiglu_oai(gu_s[0][warp * 32 + lane], gu_s[1][warp * 32 + lane]);
                 const float amax = fmaxf(warp_max(fabsf(h)), 1e-12f);
                 const float sc = __fdiv_rn(amax, 127.0f);
                 const int qv = brrr_q8_round_inv(h, sc, brrr_q8_inv(amax)), b = t * 2 + warp;
                 if (lane == 0) a.hs[ei * nb + b] = sc;
                 a.hq[(size_t)ei * a.d + b * 32 + lane] = (int8_t)qv;
-                xt_emit_block(qv, lane, b, a.himg + (size_t)ei * np * XT_B_PAIR);
+                xt_emit_digits(qv, lane, b, a.hdig + (size_t)ei * nb * XT_DIG_BLOCK);
             }
         } else {
+            v = __fadd_rn(v, half_s[m]);
             const int r = t * 128 + m, dpad = a.w.tiles_per_expert * 128;
             if (EP) {
                 // the row sum, tagged with the step number, to every rank: one plain 64-bit store over
@@ -474,9 +494,9 @@ __global__ void __launch_bounds__(XT_THREADS) xt_expert_kernel(XtArgs a) {
             } else a.part[(size_t)ei * dpad + r] = v;
             if (a.wts) {                     // exact routing known: fold here; else a fold kernel follows
                 __threadfence();
-                xt_bar_epi();
+                xt_bar_half();
                 if (m == 0) last_sh = atomicAdd(&a.counter[t], 1u) == (uint32_t)(a.topk - 1);
-                xt_bar_epi();
+                xt_bar_half();
             } else if (m == 0) last_sh = 0;
             if (a.wts && last_sh) {
                 // the last of the top-k CTAs of these 128 rows folds them in slot order
@@ -729,14 +749,14 @@ __global__ void __launch_bounds__(FN_THREADS) xt_fold_norm_kernel(FoldNormArgs a
     BRRR_GT_END(a.f.state, 240);
 }
 
-size_t xt_smem_bytes(int np, int stages) {
-    return (size_t)stages * XT_CH * MXT_UNIT + (size_t)np * XT_B_PAIR + (size_t)np * 2 * 4 + 256 * 4 + (size_t)(2 * stages + 2 * XT_REGIONS + 1) * 8;
+size_t xt_smem_bytes(int np) {
+    return (size_t)XT_STAGES * XT_STAGE + (size_t)np * XT_B_PAIR + (size_t)(np + XT_CH - 1) / XT_CH * XT_CH * 2 * 8 + (size_t)(2 * XT_STAGES + 2 * XT_REGIONS) * 8;
 }
 
 }  // namespace
 
 // ---------------------------------------------------------------- launchers
-size_t mxt_bytes(int experts, int tiles_per_expert, int np) { return (size_t)experts * tiles_per_expert * np * MXT_UNIT; }
+size_t mxt_bytes(int experts, int tiles_per_expert, int np) { return (size_t)experts * tiles_per_expert * xt_run_bytes(np); }
 
 void launch_mxt_pack(MxDev a, MxDev b, int experts, int rows_per_expert, MxtDev out, cudaStream_t st) {
     PackArgs p{};
@@ -746,55 +766,49 @@ void launch_mxt_pack(MxDev a, MxDev b, int experts, int rows_per_expert, MxtDev 
     mxt_pack_kernel<<<(unsigned)((words + 255) / 256), 256, 0, st>>>(p, words);
 }
 
-void launch_xt_bimg(const int8_t *xq, int nb, uint8_t *bimg, cudaStream_t st) {
-    if (nb > 0) xt_bimg_kernel<<<(nb + 3) / 4, 128, 0, st>>>(xq, nb, bimg);
+void launch_xt_digits(const int8_t *xq, int nb, uint8_t *dig, cudaStream_t st) {
+    if (nb > 0) xt_digits_kernel<<<(nb + 3) / 4, 128, 0, st>>>(xq, nb, dig);
+}
+
+void launch_mx_exp_scan(const uint8_t *raw, size_t blocks, uint32_t *bad, cudaStream_t st) {
+    if (blocks) mx_exp_scan_kernel<<<148 * 8, 256, 0, st>>>(raw, blocks, bad);
 }
 
 cudaError_t launch_gate_up_t(MxtDev gu, const float *gate_b, const float *up_b, const int32_t *top, const float *est, int ne, int topk,
-                             int d, const uint8_t *ximg, const float *xs, int8_t *hq, float *hs, uint8_t *himg, DevState *state,
+                             int d, const uint8_t *xdig, const float *xs, int8_t *hq, float *hs, uint8_t *hdig, DevState *state,
                              bool pdl, cudaStream_t st, const EpCtx *ep, int layer) {
     XtArgs a{};
     if (ep) { a.ep_on = 1; a.ep = *ep; a.layer = layer; }
     a.w = gu; a.bias_a = gate_b; a.bias_b = up_b; a.top = top; a.est = est; a.ne = ne; a.topk = topk; a.d = d;
-    a.bimg = ximg; a.xs = xs; a.hq = hq; a.hs = hs; a.himg = himg; a.state = state;
-    const int nchunks = (gu.np + XT_CH - 1) / XT_CH;
-#ifndef XT_GU_STAGES
-#define XT_GU_STAGES 4
-#endif
-    a.stages = nchunks < XT_GU_STAGES ? nchunks : XT_GU_STAGES;            // two CTAs per SM at the 20b shape
+    a.bdig = xdig; a.xs = xs; a.hq = hq; a.hs = hs; a.hdig = hdig; a.state = state;
     static unsigned long long configured = 0, configured_ep = 0;      // one bit per device
     {
         cudaError_t e = smem_optin(xt_expert_kernel<false, false>, 200 * 1024, configured);
         if (e == cudaSuccess) e = smem_optin(xt_expert_kernel<false, true>, 200 * 1024, configured_ep);
         if (e != cudaSuccess) return e;
     }
-    if (ep) return launch_k(xt_expert_kernel<false, true>, dim3(gu.tiles_per_expert, topk), dim3(XT_THREADS), xt_smem_bytes(gu.np, a.stages), st, pdl, a);
-    return launch_k(xt_expert_kernel<false, false>, dim3(gu.tiles_per_expert, topk), dim3(XT_THREADS), xt_smem_bytes(gu.np, a.stages), st, pdl, a);
+    if (ep) return launch_k(xt_expert_kernel<false, true>, dim3(gu.tiles_per_expert, topk), dim3(XT_THREADS), xt_smem_bytes(gu.np), st, pdl, a);
+    return launch_k(xt_expert_kernel<false, false>, dim3(gu.tiles_per_expert, topk), dim3(XT_THREADS), xt_smem_bytes(gu.np), st, pdl, a);
 }
 
 cudaError_t launch_down_t(MxtDev down, const float *down_b, const int32_t *top, const float *wts, const float *est, int ne, int topk,
-                          int d, const uint8_t *himg, const float *hs, float *x, float *part, uint32_t *counter, DevState *state,
+                          int d, const uint8_t *hdig, const float *hs, float *x, float *part, uint32_t *counter, DevState *state,
                           bool pdl, cudaStream_t st, const EpCtx *ep, int layer) {
     XtArgs a{};
     if (ep) { a.ep_on = 1; a.ep = *ep; a.layer = layer; }
     a.w = down; a.bias_a = down_b; a.top = top; a.wts = wts; a.est = est; a.ne = ne; a.topk = topk; a.d = d;
-    a.bimg = himg; a.xs = hs; a.x = x; a.part = part; a.counter = counter; a.state = state;
-    const int nchunks = (down.np + XT_CH - 1) / XT_CH;
+    a.bdig = hdig; a.xs = hs; a.x = x; a.part = part; a.counter = counter; a.state = state;
     // the same footprint as a gate/up CTA: a down CTA fits beside a running gate/up CTA, sets up and
     // starts its weight stream there, before gate/up has finished (measured: 745 tok/s against 728
     // with a 9-stage ring that needs an SM of its own)
-#ifndef XT_DOWN_STAGES
-#define XT_DOWN_STAGES 4
-#endif
-    a.stages = nchunks < XT_DOWN_STAGES ? nchunks : XT_DOWN_STAGES;
     static unsigned long long configured = 0, configured_ep = 0;      // one bit per device
     {
         cudaError_t e = smem_optin(xt_expert_kernel<true, false>, 210 * 1024, configured);
         if (e == cudaSuccess) e = smem_optin(xt_expert_kernel<true, true>, 210 * 1024, configured_ep);
         if (e != cudaSuccess) return e;
     }
-    if (ep) return launch_k(xt_expert_kernel<true, true>, dim3(down.tiles_per_expert, topk), dim3(XT_THREADS), xt_smem_bytes(down.np, a.stages), st, pdl, a);
-    return launch_k(xt_expert_kernel<true, false>, dim3(down.tiles_per_expert, topk), dim3(XT_THREADS), xt_smem_bytes(down.np, a.stages), st, pdl, a);
+    if (ep) return launch_k(xt_expert_kernel<true, true>, dim3(down.tiles_per_expert, topk), dim3(XT_THREADS), xt_smem_bytes(down.np), st, pdl, a);
+    return launch_k(xt_expert_kernel<true, false>, dim3(down.tiles_per_expert, topk), dim3(XT_THREADS), xt_smem_bytes(down.np), st, pdl, a);
 }
 
 cudaError_t launch_down_fold(const int32_t *top, const float *wts, const float *est, int ne, int topk, int d, const float *part,

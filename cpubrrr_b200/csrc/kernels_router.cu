@@ -465,7 +465,7 @@ struct HintArgs {
     int8_t *xq_out;          // nullable: Q8 of the normalised vector, each CTA writes a share
     float *xs_out;
     DevState *state;
-    uint8_t *bimg_out;       // nullable: digit-plane operand image of the same vector (brrr_mxt.cuh)
+    uint8_t *dig_out;       // nullable: digits of the same vector (brrr_mxt.cuh)
 };
 
 constexpr int HINT_THREADS = 128;
@@ -528,15 +528,15 @@ __global__ void __launch_bounds__(HINT_THREADS) router_hint_kernel(HintArgs a) {
             const int qv = brrr_q8_round_inv(v, sc, brrr_q8_inv(amax));
             if (lane == 0) a.xs_out[blk] = sc;
             a.xq_out[blk * 32 + lane] = (int8_t)qv;
-            if (a.bimg_out) xt_emit_block(qv, lane, blk, a.bimg_out);
+            if (a.dig_out) xt_emit_digits(qv, lane, blk, a.dig_out);
         }
     }
     BRRR_GT_END(a.state, 225);
 }
 
 cudaError_t launch_router_hint(const float *x_in, const float *norm_w, float eps, int d, const float *Wt, const float *b, int ne, int topk,
-                               float *est, int8_t *xq_out, float *xs_out, DevState *state, bool pdl, cudaStream_t st, uint8_t *bimg_out) {
-    HintArgs a{x_in, norm_w, eps, d, Wt, b, ne, topk, est, xq_out, xs_out, state, bimg_out};
+                               float *est, int8_t *xq_out, float *xs_out, DevState *state, bool pdl, cudaStream_t st, uint8_t *dig_out) {
+    HintArgs a{x_in, norm_w, eps, d, Wt, b, ne, topk, est, xq_out, xs_out, state, dig_out};
     size_t smem = (size_t)(d + ne + 4) * sizeof(float);
     return launch_k(router_hint_kernel, dim3(ne), dim3(HINT_THREADS), smem, st, pdl, a);
 }

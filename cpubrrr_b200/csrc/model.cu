@@ -8,6 +8,7 @@
 #include "../../include/brrr.h"
 #include "brrr_kernels.h"
 #include "brrr_synth.h"
+#include "brrr_mxt.cuh"
 #include "brrr_tile.cuh"
 
 #include <cmath>
@@ -143,7 +144,8 @@ struct brrr_model {
     bool use_mxt = false;
     float *dpart = nullptr;      // down: [topk][tiles * 128] row sums
     uint32_t *dcount = nullptr;  // down: arrival counters per row tile
-    uint8_t *ximg = nullptr, *himg = nullptr;   // operand images of the token's and of h's Q8 activation
+    uint8_t *xdig = nullptr, *hdig = nullptr;   // digits of the token's and of h's Q8 activation (brrr_mxt.cuh)
+    uint32_t *exp_bad = nullptr;                // while loading: set when a block exponent lies outside the range of the scaled products
     int8_t *nq = nullptr;        // Q8 of the normalised residual that the fold leaves for the next q/k/v projection
     float *ns = nullptr;
     bool fused_fold = true;      // speculative tensor-core step: fold + next norm/quant in one kernel that waits for the router by flag
@@ -273,6 +275,16 @@ int load_mx(brrr_model *m, const Source &s, uint32_t layer, int kind, int rows, 
     TRY(fetch(m, s, layer, kind, 39, (size_t)rows * blocks * 32, scratch, (size_t)row0 * blocks * 32, (size_t)(rows_total ? rows_total : rows) * blocks * 32));
     launch_mx_pack((const uint8_t *)scratch, *x, m->stream);
     CU(cudaGetLastError());
+    if (!m->exp_bad) return BRRR_OK;
+    launch_mx_exp_scan((const uint8_t *)scratch, (size_t)rows * blocks, m->exp_bad, m->stream);
+    // expert-parallel ranks have to run the same kind of step, so each looks at the other ranks' rows too
+    for (int r = 0; r < rows_total; r += rows) {
+        if (r == row0) continue;
+        const int n = std::min(rows, rows_total - r);
+        TRY(fetch(m, s, layer, kind, 39, (size_t)n * blocks * 32, scratch, (size_t)r * blocks * 32, (size_t)rows_total * blocks * 32));
+        launch_mx_exp_scan((const uint8_t *)scratch, (size_t)n * blocks, m->exp_bad, m->stream);
+    }
+    CU(cudaGetLastError());
     return BRRR_OK;
 }
 
@@ -376,17 +388,17 @@ int enqueue_step(brrr_model *m, bool want, float *trace_dev, int *nlaunch, unsig
             CU(cudaEventRecord(m->ev_join, m->side));
             n++;
             CUL(launch_router_hint(m->x, ly.ffn_norm, c.rms_eps, d, ly.ginp, ly.ginp_b, c.n_expert, topk, m->est, m->xq, m->xs, m->st, pdl, s,
-                                   m->use_mxt ? m->ximg : nullptr));
+                                   m->use_mxt ? m->xdig : nullptr));
             n++;
             const EpCtx *epc = m->ep ? &m->epc : nullptr;      // expert parallelism: local slots only, row sums exchanged by down, awaited by the fold
-            if (m->use_mxt) CUL(launch_gate_up_t(ly.gu_t, ly.gate_b, ly.up_b, nullptr, m->est, c.n_expert, topk, d, m->ximg, m->xs,
-                                                 m->hq, m->hs, m->himg, m->st, pdl, s, epc, il));
+            if (m->use_mxt) CUL(launch_gate_up_t(ly.gu_t, ly.gate_b, ly.up_b, nullptr, m->est, c.n_expert, topk, d, m->xdig, m->xs,
+                                                 m->hq, m->hs, m->hdig, m->st, pdl, s, epc, il));
             else CUL(launch_gate_up(ly.gate, ly.up, ly.gate_b, ly.up_b, nullptr, topk, d, nullptr, nullptr, c.rms_eps, m->xq, m->xs,
                                     m->hq, m->hs, nullptr, m->st, pdl, s, m->est, c.n_expert));
             if (m->use_mxt) {
                 // down for the estimated experts as well; only the fold waits for the exact routing
                 n++;
-                CUL(launch_down_t(ly.down_t, ly.down_b, nullptr, nullptr, m->est, c.n_expert, topk, d, m->himg, m->hs, m->x,
+                CUL(launch_down_t(ly.down_t, ly.down_b, nullptr, nullptr, m->est, c.n_expert, topk, d, m->hdig, m->hs, m->x,
                                   m->dpart, m->dcount, m->st, pdl, s, epc, il));
             }
             if (fused) {
@@ -413,10 +425,10 @@ int enqueue_step(brrr_model *m, bool want, float *trace_dev, int *nlaunch, unsig
             // activation and routing the last step left behind
             if (on(ST_ROUTER)) CUL(launch_ffn_in(m->x, ly.ffn_norm, c.rms_eps, d, ly.ginp, ly.ginp_b, c.n_expert, topk, m->rlogits, m->top, m->wts,
                                                  &m->st->router_done, m->st, pdl, s));
-            if (on(ST_GATE_UP)) CUL(launch_gate_up_t(ly.gu_t, ly.gate_b, ly.up_b, m->top, nullptr, 0, topk, d, m->ximg, m->xs, m->hq, m->hs, m->himg,
+            if (on(ST_GATE_UP)) CUL(launch_gate_up_t(ly.gu_t, ly.gate_b, ly.up_b, m->top, nullptr, 0, topk, d, m->xdig, m->xs, m->hq, m->hs, m->hdig,
                                                      m->st, pdl, s));
             const bool ff = m->use_spec && m->fused_fold;     // the fused step: down leaves partial sums, a fold kernel finishes
-            if (on(ST_DOWN)) CUL(launch_down_t(ly.down_t, ly.down_b, m->top, ff ? nullptr : m->wts, nullptr, 0, topk, d, m->himg, m->hs, m->x, m->dpart,
+            if (on(ST_DOWN)) CUL(launch_down_t(ly.down_t, ly.down_b, m->top, ff ? nullptr : m->wts, nullptr, 0, topk, d, m->hdig, m->hs, m->x, m->dpart,
                                                m->dcount, m->st, pdl, s));
             if (ff && on(ST_FOLD))
                 CUL(launch_fold_norm(m->top, m->wts, nullptr, 0, topk, d, m->dpart, ly.down_b, m->x,
@@ -530,6 +542,10 @@ int build_model(brrr_model *m, const Source &src) {
         if (const char *e = getenv("BRRR_NO_ATTN_ROWS")) m->no_attn_rows = e[0] && e[0] != '0';
         if (const char *e = getenv("BRRR_TILE_ROWS")) { const int v = atoi(e); if (v >= 2 && v <= BRRR_TILE_MAX) m->tile_rows = v; }
     }
+    if (m->use_mxt) {
+        TRY(m->alloc(&m->exp_bad, 1));
+        CU(cudaMemsetAsync(m->exp_bad, 0, 4, m->stream));
+    }
     for (int il = 0; il < c.n_layer; il++) {
         Layer &ly = m->L[il];
         TRY(load_f32(m, src, il, BRRR_T_ATTN_NORM, d, &ly.attn_norm));
@@ -579,6 +595,16 @@ int build_model(brrr_model *m, const Source &src) {
         CU(cudaMemsetAsync(ly.kc, 0, (size_t)BRRR_MAXSEQ * nkv * hd * 4, m->stream));   // layout [kv head][position][64]
         CU(cudaMemsetAsync(ly.vc, 0, (size_t)BRRR_MAXSEQ * nkv * hd * 4, m->stream));
     }
+    if (m->use_mxt) {
+        uint32_t bad = 0;
+        CU(cudaMemcpyAsync(&bad, m->exp_bad, 4, cudaMemcpyDeviceToHost, m->stream));
+        CU(cudaStreamSynchronize(m->stream));
+        m->release(&m->exp_bad);
+        if (bad) {                       // the scaled products would not be exact: the integer units run the experts (same bits)
+            m->use_mxt = false;
+            for (Layer &ly : m->L) { m->release(&ly.gu_t.data); m->release(&ly.down_t.data); }
+        }
+    }
     TRY(m->alloc(&m->tok_embd, (size_t)c.n_vocab * d));
     TRY(fetch(m, src, BRRR_L_GLOBAL, BRRR_T_TOK_EMBD, 30, (size_t)c.n_vocab * d, m->tok_embd));
     TRY(load_f32(m, src, BRRR_L_GLOBAL, BRRR_T_OUT_NORM, d, &m->out_norm));
@@ -600,10 +626,8 @@ int build_model(brrr_model *m, const Source &src) {
     TRY(m->alloc(&m->dpart, (size_t)topk * ((d + 127) / 128) * 128));
     TRY(m->alloc(&m->dcount, (size_t)(d + 127) / 128));
     CU(cudaMemsetAsync(m->dcount, 0, (size_t)((d + 127) / 128) * 4, m->stream));
-    TRY(m->alloc(&m->ximg, (size_t)(nb / 2 + 1) * 768));
-    TRY(m->alloc(&m->himg, (size_t)topk * (nb / 2 + 1) * 768));
-    CU(cudaMemsetAsync(m->ximg, 0, (size_t)(nb / 2 + 1) * 768, m->stream));      // producers only write the non-zero words
-    CU(cudaMemsetAsync(m->himg, 0, (size_t)topk * (nb / 2 + 1) * 768, m->stream));
+    TRY(m->alloc(&m->xdig, (size_t)nb * XT_DIG_BLOCK));
+    TRY(m->alloc(&m->hdig, (size_t)topk * nb * XT_DIG_BLOCK));
     CU(cudaMemsetAsync(m->st, 0, sizeof(DevState), m->stream));
     CU(cudaMemsetAsync(m->x, 0, d * 4, m->stream));
     CU(cudaMallocHost(&m->h_in, 16));
@@ -1335,9 +1359,9 @@ extern "C" int brrr_moe_ffn_step_tc(brrr_model *m, int il, const float *d_xn, fl
     cudaStream_t s = m->stream;
     CUL(launch_ffn_in(d_xn, nullptr, c.rms_eps, d, ly.ginp, ly.ginp_b, c.n_expert, topk, m->rlogits, m->top, m->wts, &m->st->router_done, m->st, false, s));
     launch_quant_q8(d_xn, d, m->xq, m->xs, s);
-    launch_xt_bimg(m->xq, d / 32, m->ximg, s);
-    CUL(launch_gate_up_t(ly.gu_t, ly.gate_b, ly.up_b, m->top, nullptr, 0, topk, d, m->ximg, m->xs, m->hq, m->hs, m->himg, m->st, false, s));
-    CUL(launch_down_t(ly.down_t, ly.down_b, m->top, m->wts, nullptr, 0, topk, d, m->himg, m->hs, d_x, m->dpart, m->dcount, m->st, false, s));
+    launch_xt_digits(m->xq, d / 32, m->xdig, s);
+    CUL(launch_gate_up_t(ly.gu_t, ly.gate_b, ly.up_b, m->top, nullptr, 0, topk, d, m->xdig, m->xs, m->hq, m->hs, m->hdig, m->st, false, s));
+    CUL(launch_down_t(ly.down_t, ly.down_b, m->top, m->wts, nullptr, 0, topk, d, m->hdig, m->hs, d_x, m->dpart, m->dcount, m->st, false, s));
     CU(cudaGetLastError());
     if (d_top) CU(cudaMemcpyAsync(d_top, m->top, topk * sizeof(int32_t), cudaMemcpyDeviceToDevice, s));
     if (d_wts) CU(cudaMemcpyAsync(d_wts, m->wts, topk * sizeof(float), cudaMemcpyDeviceToDevice, s));

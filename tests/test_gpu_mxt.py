@@ -106,3 +106,36 @@ def test_decode_same_with_and_without_tensor_experts(brrr, orc, monkeypatch):
     om = orc.Model.synth(ocfg_of(orc, cfg), 4)
     assert greedy(om.run, prompt, 64) == got
     assert np.array_equal(bits(om.logits()), bits(lg))
+
+
+@pytest.mark.parametrize("edge,tensor_experts", [
+    ([49, 190, 120, 60], True),          # the ends of the range whose scaled products are exact
+    ([(0, 0), (48, 0), 49], True),       # zero blocks below it
+    ([48], False),                       # values other than zero below it, any block above it: the integer units
+    ([191], False),
+    ([(255, 0)], False),
+])
+def test_block_exponents_choose_the_expert_kernels(brrr, orc, tmp_path, edge, tensor_experts):
+    """Gate blocks with the given exponents (pairs: exponent of a block of zeros) among the synthetic ones: whether the model's
+    experts run on the tensor cores, and the oracle's tokens and logits either way."""
+    import os
+    import refdata
+    cfg, d, blob = refdata.case_data_dir(str(tmp_path), "gptoss_d128", 12)
+    rows = [r.split() for r in open(os.path.join(d, "manifest.txt"))]
+    name, _, off, nel = next(r for r in rows if r[0] == "blk.1.ffn_gate_exps.weight")
+    raw = np.memmap(blob, np.uint8, "r+", int(rows[0][1]) + int(off), (int(nel) // 32, 17))
+    for i, b in enumerate(range(3, len(raw), 7)):
+        ex = edge[i % len(edge)]
+        if isinstance(ex, tuple):
+            ex = ex[0]
+            raw[b, 1:] = np.arange(16) % 2 * 0x80 + np.arange(16) % 3 % 2 * 8      # +0 and -0
+        raw[b, 0] = ex
+    raw.flush()
+    eng, om = brrr.Engine.open(d, blob), orc.Model.open(d, blob)
+    assert eng.uses_tensor_experts == tensor_experts
+    prompt = S.synth_prompt(12, 7, 500)
+    assert greedy(eng.run, prompt, 24) == greedy(om.run, prompt, 24)
+    assert np.array_equal(bits(eng.logits()), bits(om.logits()))
+    # the same prompt as token rows
+    assert eng.run_tile([int(t) for t in prompt], 0, True) == greedy(om.run, prompt, 1)[0]
+    eng.close()
