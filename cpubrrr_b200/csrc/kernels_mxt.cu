@@ -334,7 +334,7 @@ __global__ void __launch_bounds__(XT_THREADS, 2) xt_expert_kernel(XtArgs a) {
         if (local && warp == XT_PRODUCER && lane < min(XT_STAGES, nchunks)) {          // one lane per copy: the first stages of the weight stream
             const uint32_t bytes = xt_run_bytes(min(XT_CH, np - lane * XT_CH));
             mbar_expect_tx(&sh.full[lane], bytes);
-            bulk_g2s(sh.ring + XT_STAGE * lane, src + (size_t)lane * XT_STAGE, bytes, &sh.full[lane]);
+            bulk_g2s_once(sh.ring + XT_STAGE * lane, src + (size_t)lane * XT_STAGE, bytes, &sh.full[lane]);
         }
     };
     // The down projection knows its expert before gate/up has finished (the routing is two kernels
@@ -375,7 +375,7 @@ __global__ void __launch_bounds__(XT_THREADS, 2) xt_expert_kernel(XtArgs a) {
                 const uint32_t bytes = xt_run_bytes(min(XT_CH, np - c * XT_CH));
                 xt_wait(&sh.empty[s], par, err, true);
                 mbar_expect_tx(&sh.full[s], bytes);
-                bulk_g2s(sh.ring + XT_STAGE * s, src + (size_t)c * XT_STAGE, bytes, &sh.full[s]);
+                bulk_g2s_once(sh.ring + XT_STAGE * s, src + (size_t)c * XT_STAGE, bytes, &sh.full[s]);
                 if (++s == XT_STAGES) { s = 0; par ^= 1u; }
             }
         }

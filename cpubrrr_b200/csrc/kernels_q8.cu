@@ -158,7 +158,7 @@ __global__ void __launch_bounds__(Q8_THREADS) q8_stream_kernel(Q8Args a) {
         int cnt = min(a.ch, np - k * a.ch);
         int slot = c % a.stages;
         mbar_expect_tx(&bars[slot], (uint32_t)cnt * Q8_UNIT);
-        bulk_g2s(ring + stage_bytes * slot, a.m.data + q8_unit_off(u, k * a.ch, np), (uint32_t)cnt * Q8_UNIT, &bars[slot]);
+        bulk_g2s_once(ring + stage_bytes * slot, a.m.data + q8_unit_off(u, k * a.ch, np), (uint32_t)cnt * Q8_UNIT, &bars[slot]);
     };
 
     const int sb = (NORM || EPI == Q8_EPI_BIAS) ? 32 : 64;      // timeline slots of this kernel flavour (q/k/v, o-proj)
@@ -354,12 +354,13 @@ __global__ void __launch_bounds__(Q8_THREADS) q8_reg_kernel(Q8Args a) {
     const uint8_t *unit0 = a.m.data + q8_unit_off(u, 0, NP);
     const int2 *wp = reinterpret_cast<const int2 *>(unit0 + rl * 64 + c8 * 8);
     const float *sp = reinterpret_cast<const float *>(unit0 + Q8_UNIT_SCALES + rl * 8 + p * 4);
+    const uint64_t once = l2_once();
     int2 w[NP];
     float s[NP];
 #pragma unroll
     for (int i = 0; i < NP; i++) {
-        w[i] = __ldg(wp + (size_t)i * (Q8_UNIT / 8));
-        s[i] = __ldg(sp + (size_t)i * (Q8_UNIT / 4));
+        w[i] = ldg_once(wp + (size_t)i * (Q8_UNIT / 8), once);
+        s[i] = ldg_once(sp + (size_t)i * (Q8_UNIT / 4), once);
     }
     float bias_pre = 0.0f, resid_pre = 0.0f;
     if (c8 == 0 && row < a.m.rows) {
@@ -470,7 +471,7 @@ __global__ void __launch_bounds__(QH_THREADS) q8_head_ring_kernel(QHeadArgs a) {
         const int u = u0 + c / cpr, k = c % cpr, slot = c % a.stages;
         const uint32_t bytes = (uint32_t)min(a.ch, np - k * a.ch) * Q8_UNIT;
         mbar_expect_tx(&full[slot], bytes);
-        bulk_g2s(ring + stage_bytes * slot, a.m.data + q8_unit_off(u, k * a.ch, np), bytes, &full[slot]);
+        bulk_g2s_once(ring + stage_bytes * slot, a.m.data + q8_unit_off(u, k * a.ch, np), bytes, &full[slot]);
     };
     // the weights do not depend on the step: the first ring goes out before the dependency wait
     const bool producer = warp == 4;
