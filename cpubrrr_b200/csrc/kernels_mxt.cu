@@ -138,8 +138,7 @@ __global__ void mx_exp_scan_kernel(const uint8_t *__restrict__ raw, size_t block
 // ue8m0 scales (bit 23), M / 16 at bit 24, K = 64; the rows' scale-factor id (bits 29-30) is 0 or 2: bytes 0, 1 or 2, 3 of their words
 constexpr uint32_t XT_IDESC = (1u << 7) | (1u << 10) | ((uint32_t)(XT_N >> 3) << 17) | (1u << 23) | ((128u >> 4) << 24);
 
-// The issuing warp's instructions carry its elected lane's predicate instead of standing in a one-lane branch: the loop around them stays
-// uniform and keeps descriptors and addresses in uniform registers, where these instructions want them.
+// (predicates: tl_commit_if)
 __device__ __forceinline__ void xt_mma(uint32_t issue, uint32_t tmem_d, uint64_t desc_a, uint64_t desc_b, uint32_t idesc, uint32_t tmem_sfa, uint32_t tmem_sfb) {
     asm volatile(
         "{\n\t.reg .pred p, e;\n\tsetp.ne.b32 p, %4, 0;\n\tsetp.ne.b32 e, %7, 0;\n\t"
@@ -150,9 +149,6 @@ __device__ __forceinline__ void xt_mma(uint32_t issue, uint32_t tmem_d, uint64_t
 // 512 bytes of block scales -> four columns of tensor memory, the same 32 lanes for each of its quarters; in order with the products of the issuing thread
 __device__ __forceinline__ void xt_cp_scales(uint32_t issue, uint32_t tmem, uint64_t desc) {
     asm volatile("{\n\t.reg .pred e;\n\tsetp.ne.b32 e, %2, 0;\n\t@e tcgen05.cp.cta_group::1.32x128b.warpx4 [%0], %1;\n\t}" ::"r"(tmem), "l"(desc), "r"(issue) : "memory");
-}
-__device__ __forceinline__ void xt_commit(uint32_t issue, uint64_t *bar) {
-    asm volatile("{\n\t.reg .pred e;\n\tsetp.ne.b32 e, %1, 0;\n\t@e tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];\n\t}" ::"r"(smem_u32(bar)), "r"(issue) : "memory");
 }
 __device__ __forceinline__ void xt_fence_before() { asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory"); }
 __device__ __forceinline__ void xt_fence_after() { asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory"); }
@@ -409,8 +405,8 @@ __global__ void __launch_bounds__(XT_THREADS, 2) xt_expert_kernel(XtArgs a) {
                     xt_mma(two, d0 + XT_N, alo | (aaddr + MXT_PAIR / 16), blo | (baddr1 + XT_B_PAIR / 16), XT_IDESC | (2u << 29), sfa + k * 2, sfb);
                     d0 += 2 * XT_N; aaddr += XT_GROUP / 16; baddr1 += 2 * XT_B_PAIR / 16;
                 }
-                xt_commit(r + XT_STAGES < nchunks ? issue : 0u, &sh.empty[s]);      // nobody waits for the last ones
-                xt_commit(issue, &sh.dfull[reg]);
+                tl_commit_if(r + XT_STAGES < nchunks ? issue : 0u, &sh.empty[s]);      // nobody waits for the last ones
+                tl_commit_if(issue, &sh.dfull[reg]);
                 __syncwarp();
                 baddr += XT_CH * XT_B_PAIR / 16;
                 left -= XT_CH;
