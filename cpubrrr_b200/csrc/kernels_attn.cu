@@ -11,21 +11,29 @@
 // The cache is laid out [kv head][position][64] so the window of one head is one contiguous
 // range; K, then V run through one ring of tiles of 64 positions (32 for token rows) by bulk asynchronous copies, the first of them
 // issued before the kernel waits on its predecessor (the cached positions are older than this
-// token).  Long contexts are bound by the copies' latency and the chains over the keys: with two 128-position tiles in flight per tensor
-// and no reading ahead in the sums a key cost 23 ns, now 15.  The current position's k and v never come from the cache: every head recomputes them.
+// token).  The current position's k and v never come from the cache: every head recomputes them.
+//
+// Nobody waits for a whole CTA inside the loops over the tiles: a warp leaves a tile through the tile's barrier and a warp of its own refills the
+// ring.  A key's 16 chains belong to four neighbouring threads, four chains each in a 16-byte word.  The serial sums read sixteen keys ahead across
+// tile borders.  20b shape, one token, full layer, from the dependency wait to the end: 4.1 us at 130 keys, 8.5 at 600, 20.5 at 1900 (before:
+// 4.6, 11.5, 31.0).  Bound by the two serial sums, 8 to 10 cycles a key where the dependent multiply-add alone is 4.7, and by score passes of 8
+// cycles a key; the copies come at 25 of the 67 bytes a cycle that one CTA can draw from L2.
 #include "brrr_kernels.h"
 #include "brrr_block.cuh"
 #include "brrr_tma.cuh"
 #include "brrr_tile.cuh"
 
+#include <type_traits>
+
 namespace brrr {
 
 constexpr int HD = 64;
-constexpr int AT_THREADS = 256;
-constexpr int AT_ISSUER = 224;                     // refills the ring: a thread of the last warp, which carries no serial sum (an issue takes 220 cycles)
+constexpr int AT_WORKERS = 256;
 constexpr int AT_TILE_ONE = 64;                    // positions per tile: one token per launch (one CTA per SM streams its head's window)
 constexpr int AT_TILE_ROWS = 32;                   // token rows: many (head, row) CTAs share an SM, so each holds less
 __host__ __device__ constexpr int at_slots(int tile) { return tile == AT_TILE_ONE ? 8 : 4; }      // tiles in flight
+__host__ __device__ constexpr int at_issuers(int tile) { return tile == AT_TILE_ONE ? 4 : 1; }    // warps that refill the ring, a tile each in turn (a bulk copy takes its thread 240 cycles)
+__host__ __device__ constexpr int at_threads(int tile) { return AT_WORKERS + 32 * at_issuers(tile); }
 
 struct AttnArgs {
     const float *qkv;
@@ -60,16 +68,18 @@ __device__ __forceinline__ void attn_quant(float o, int lane, int b, int8_t *aq,
 
 
 template <int AT_TILE>
-__global__ void __launch_bounds__(AT_THREADS) attn_decode_kernel(AttnArgs a) {
+__global__ void __launch_bounds__(at_threads(AT_TILE)) attn_decode_kernel(AttnArgs a) {
     constexpr size_t AT_TILE_BYTES = (size_t)AT_TILE * HD * sizeof(float);
     constexpr int SLOTS = at_slots(AT_TILE);
     extern __shared__ __align__(128) unsigned char smraw[];
     float *tiles = reinterpret_cast<float *>(smraw);                                    // [SLOTS][AT_TILE][64]
     float *sc = reinterpret_cast<float *>(smraw + AT_TILE_BYTES * SLOTS);                // [MAXSEQ]
-    __shared__ __align__(8) uint64_t full[SLOTS];
-    __shared__ float q[HD], kcur[HD], vcur[HD];
-    __shared__ float red[AT_THREADS / 32];
+    __shared__ __align__(8) uint64_t full[SLOTS], left_k[SLOTS], left_v[SLOTS];         // a tile has landed; its K, V readers have left it
+    __shared__ __align__(16) float q[HD];
+    __shared__ float kcur[HD], vcur[HD];
+    __shared__ float red[AT_WORKERS / 32];
     __shared__ float den_sh;
+    constexpr int PASS = AT_WORKERS / 4 / AT_TILE;      // K tiles that the workers read side by side
     const int h = blockIdx.x, tid = threadIdx.x;
     const int group = a.nh / a.nkv, kvh = h / group;
     uint32_t *err = a.err_state ? &a.err_state->err : nullptr;
@@ -104,7 +114,7 @@ __global__ void __launch_bounds__(AT_THREADS) attn_decode_kernel(AttnArgs a) {
     BRRR_STAMP(a.err_state, 160);
     BRRR_GT_START(a.err_state, 233);
     if (tid == 0) {
-        for (int s = 0; s < SLOTS; s++) mbar_init(&full[s], 1);
+        for (int s = 0; s < SLOTS; s++) { mbar_init(&full[s], 1); mbar_init(&left_k[s], AT_WORKERS / 32 / PASS); mbar_init(&left_v[s], 2); }
         mbar_fence_init();
     }
     __syncwarp();
@@ -141,48 +151,92 @@ __global__ void __launch_bounds__(AT_THREADS) attn_decode_kernel(AttnArgs a) {
         if (tid < 64) a.kc[o] = kcur[tid]; else a.vc[o] = vcur[tid - 64];
     }
 
-    // ---- scores: 16 threads per key
-    {
-        const int g = tid >> 4, c = tid & 15;
-        const float q0 = q[c], q1 = q[16 + c], q2 = q[32 + c], q3 = q[48 + c];
-        for (int t = 0; t < ntiles; t++) {
-            const int slot = t % SLOTS, cnt = min(AT_TILE, ncached - t * AT_TILE);
-            waiter.wait(&full[slot], (uint32_t)(t / SLOTS) & 1u);
-            const float *kt = tiles + (size_t)slot * AT_TILE * HD;
-            // the tile's keys of this group side by side, so that their shuffles overlap (a key at a time: 265 cycles per sixteen keys); past the
-            // last key the sums are of no account
-            float s[AT_TILE / 16];
-#pragma unroll
-            for (int i = 0; i < AT_TILE / 16; i++) {
-                const float *kp = kt + (i * 16 + g) * HD;
-                s[i] = __fmaf_rn(kp[c], q0, 0.0f);
-                s[i] = __fmaf_rn(kp[16 + c], q1, s[i]);
-                s[i] = __fmaf_rn(kp[32 + c], q2, s[i]);
-                s[i] = __fmaf_rn(kp[48 + c], q3, s[i]);
-            }
-#pragma unroll
-            for (int o = 0; o < 4; o++) {
-                const int x = o == 0 ? 4 : o == 1 ? 8 : o == 2 ? 1 : 2;
-#pragma unroll
-                for (int i = 0; i < AT_TILE / 16; i++) s[i] = __fadd_rn(s[i], __shfl_xor_sync(0xffffffffu, s[i], x));
-            }
-            if (c == 0) {
-#pragma unroll
-                for (int i = 0; i < AT_TILE / 16; i++)
-                    if (i * 16 + g < cnt) sc[t * AT_TILE + i * 16 + g] = __fmul_rn(s[i], 0.125f);
-            }
-            if (t + SLOTS < 2 * ntiles) {
-                __syncthreads();
-                if (tid == AT_ISSUER) { fence_proxy_async(); issue(t + SLOTS); }
+    auto bar_workers = [&]() { asm volatile("bar.sync 1, %0;" ::"n"(AT_WORKERS) : "memory"); };
+    if (tid >= AT_WORKERS) {
+        // ---- ring: tile u + SLOTS takes the slot of tile u once its readers have left it
+        if ((tid & 31) == 0) {
+            for (int u = (tid - AT_WORKERS) >> 5; u + SLOTS < 2 * ntiles; u += at_issuers(AT_TILE)) {
+                const int slot = u % SLOTS;
+                // V tiles' uses of a slot are counted from its first one
+                if (u < ntiles) waiter.wait(&left_k[slot], (uint32_t)(u / SLOTS) & 1u);
+                else waiter.wait(&left_v[slot], (uint32_t)((u - ntiles) / SLOTS) & 1u);
+                fence_proxy_async();
+                issue(u + SLOTS);
             }
         }
+        return;
+    }
+    const int lane = tid & 31, warp = tid >> 5;
+    // ---- scores: four threads per key, thread j of them the chains 4 j .. 4 j + 3
+    {
+        const int j = tid & 3, key = (tid >> 2) % AT_TILE, odd = key & 1;
+        float4 qv[4];
+#pragma unroll
+        for (int i = 0; i < 4; i++) qv[i] = *reinterpret_cast<const float4 *>(q + 16 * i + 4 * j);
+        // U passes side by side, so that their loads and shuffles overlap
+        auto pass = [&](auto U_, int t) {
+            constexpr int U = decltype(U_)::value;
+            float s[U][4];
+            float4 f[U][4];
+            int slot[U];
+#pragma unroll
+            for (int u = 0; u < U; u++) {
+                slot[u] = (t + u * PASS) % SLOTS;
+                waiter.wait(&full[slot[u]], (uint32_t)((t + u * PASS) / SLOTS) & 1u);
+            }
+#pragma unroll
+            for (int u = 0; u < U; u++) {
+                const float *kp = tiles + ((size_t)slot[u] * AT_TILE + key) * HD + 4 * j;
+                // two neighbouring keys' words share banks: the odd key reads its quarters in the order 1, 0, 3, 2
+#pragma unroll
+                for (int i = 0; i < 4; i++) f[u][i] = *reinterpret_cast<const float4 *>(kp + 16 * (i ^ odd));
+            }
+#pragma unroll
+            for (int u = 0; u < U; u++) {
+#pragma unroll
+                for (int e = 0; e < 4; e++) s[u][e] = 0.0f;
+#pragma unroll
+                for (int i = 0; i < 4; i++) {
+                    const float4 k = odd ? f[u][i ^ 1] : f[u][i];
+                    s[u][0] = __fmaf_rn(k.x, qv[i].x, s[u][0]); s[u][1] = __fmaf_rn(k.y, qv[i].y, s[u][1]);
+                    s[u][2] = __fmaf_rn(k.z, qv[i].z, s[u][2]); s[u][3] = __fmaf_rn(k.w, qv[i].w, s[u][3]);
+                }
+            }
+            __syncwarp();
+#pragma unroll
+            for (int u = 0; u < U; u++) mbar_arrive_if(lane == 0 ? 1u : 0u, &left_k[slot[u]]);
+            // chains c and c ^ 4, then c ^ 8, then c ^ 1, then c ^ 2.  The first two partners sit in other threads: an even thread keeps
+            // chains 0 and 1 of its four and gives away 2 and 3, the odd one the other way round, and so on; every sum has two operands
+            const bool b0 = j & 1, b1 = j & 2;
+            float u0[U], u1[U], w[U];
+#pragma unroll
+            for (int u = 0; u < U; u++) {
+                u0[u] = __fadd_rn(b0 ? s[u][2] : s[u][0], __shfl_xor_sync(0xffffffffu, b0 ? s[u][0] : s[u][2], 1));
+                u1[u] = __fadd_rn(b0 ? s[u][3] : s[u][1], __shfl_xor_sync(0xffffffffu, b0 ? s[u][1] : s[u][3], 1));
+            }
+#pragma unroll
+            for (int u = 0; u < U; u++) w[u] = __fadd_rn(b1 ? u1[u] : u0[u], __shfl_xor_sync(0xffffffffu, b1 ? u0[u] : u1[u], 2));      // chains of residue 2 b0 + b1
+#pragma unroll
+            for (int u = 0; u < U; u++) w[u] = __fadd_rn(w[u], __shfl_xor_sync(0xffffffffu, w[u], 2));
+#pragma unroll
+            for (int u = 0; u < U; u++) {
+                w[u] = __fadd_rn(w[u], __shfl_xor_sync(0xffffffffu, w[u], 1));
+                const int at = (t + u * PASS) * AT_TILE + key;
+                if (j == 0 && at < ncached) sc[at] = __fmul_rn(w[u], 0.125f);
+            }
+        };
+        int t = tid / (4 * AT_TILE);
+#pragma unroll 1
+        for (; t + PASS < ntiles; t += 2 * PASS) pass(std::integral_constant<int, 2>{}, t);
+        if (t < ntiles) pass(std::integral_constant<int, 1>{}, t);
         // the current position, from this CTA's own rotated k
-        if (g == 0) {
+        if (tid < 16) {
+            const int c = tid;
             float s = 0.0f;
-            s = __fmaf_rn(kcur[c], q0, s);
-            s = __fmaf_rn(kcur[16 + c], q1, s);
-            s = __fmaf_rn(kcur[32 + c], q2, s);
-            s = __fmaf_rn(kcur[48 + c], q3, s);
+            s = __fmaf_rn(kcur[c], q[c], s);
+            s = __fmaf_rn(kcur[16 + c], q[16 + c], s);
+            s = __fmaf_rn(kcur[32 + c], q[32 + c], s);
+            s = __fmaf_rn(kcur[48 + c], q[48 + c], s);
             s = __fadd_rn(s, __shfl_xor_sync(0xffffu, s, 4));
             s = __fadd_rn(s, __shfl_xor_sync(0xffffu, s, 8));
             s = __fadd_rn(s, __shfl_xor_sync(0xffffu, s, 1));
@@ -190,86 +244,110 @@ __global__ void __launch_bounds__(AT_THREADS) attn_decode_kernel(AttnArgs a) {
             if (c == 0) sc[ncached] = __fmul_rn(s, 0.125f);
         }
     }
-    __syncthreads();
+    bar_workers();
 
     BRRR_STAMP(a.err_state, 163);
     // ---- max (order-free), then exponentials in place
     float mx = sink;
-    for (int t = tid; t < n; t += AT_THREADS) mx = fmaxf(mx, sc[t]);
+    for (int t = tid; t < n; t += AT_WORKERS) mx = fmaxf(mx, sc[t]);
     mx = warp_max(mx);
-    if ((tid & 31) == 0) red[tid >> 5] = mx;
-    __syncthreads();
+    if (lane == 0) red[warp] = mx;
+    bar_workers();
     mx = red[0];
 #pragma unroll
-    for (int w = 1; w < AT_THREADS / 32; w++) mx = fmaxf(mx, red[w]);
-    for (int t = tid; t < ((n + 3) & ~3); t += AT_THREADS) sc[t] = t < n ? brrr_expf_dev(__fsub_rn(sc[t], mx)) : 0.0f;      // +0 past the end changes no sum
-    __syncthreads();
+    for (int w = 1; w < AT_WORKERS / 32; w++) mx = fmaxf(mx, red[w]);
+    for (int t = tid; t < ((n + 3) & ~3); t += AT_WORKERS) sc[t] = t < n ? brrr_expf_dev(__fsub_rn(sc[t], mx)) : 0.0f;      // +0 past the end changes no sum
+    bar_workers();
 
     BRRR_STAMP(a.err_state, 164);
     // ---- serial sums: thread u < 64 owns output dim u, thread 64 the denominator
     float acc = 0.0f;
-    float den = tid == 64 ? brrr_expf_dev(__fsub_rn(sink, mx)) : 0.0f;      // tile by tile: its warp takes part in the ring's barriers
-    auto add_den = [&](int t0, int t1) {                                   // probabilities t0 .. t1 - 1, t0 a multiple of 4, the last four padded with +0
-        float4 p = *reinterpret_cast<const float4 *>(sc + t0);
-#pragma unroll 4
-        for (int t = t0 + 4; t < t1 + 4; t += 4) {
-            const float4 c = p;
-            p = *reinterpret_cast<const float4 *>(sc + (t < t1 ? t : t0));
-            den = __fadd_rn(den, c.x); den = __fadd_rn(den, c.y); den = __fadd_rn(den, c.z); den = __fadd_rn(den, c.w);
-        }
-    };
-    for (int t = 0; t < ntiles; t++) {
-        const int u = ntiles + t, slot = u % SLOTS, cnt = min(AT_TILE, ncached - t * AT_TILE);
-        if (tid < 64) {
-            waiter.wait(&full[slot], (uint32_t)(u / SLOTS) & 1u);
-            // sixteen keys at a time, the next sixteen's values on the way (two sets of registers: reloading one set in place exposed every load's
-            // latency, 19 cycles per key instead of 7); then the rest
-            const float *vt = tiles + (size_t)slot * AT_TILE * HD + tid, *pt = sc + t * AT_TILE;
-            float v0[16], v1[16];
-            float4 p0[4], p1[4];
-            auto load = [&](float (&v)[16], float4 (&p)[4], int k) {
-                const float *w = vt + (k & (AT_TILE - 1)) * HD, *o = pt + (k & (AT_TILE - 1));
+    if (warp < 2) {
+        // sixteen keys at a time, the next sixteen's values on the way, across tile borders (two sets of registers: reloading one set in place
+        // exposed every load's latency; so did branches between a load and its use)
+        constexpr int BLOCKS = AT_TILE / 16;
+        const int nfull = ncached / AT_TILE;
+        float v0[16], v1[16];
+        float4 p0[4], p1[4];
+        // (statements of their own, in program order: the compiler moves plain loads down to their uses)
+        auto load = [&](float (&v)[16], float4 (&p)[4], const float *w, const float *o) {
+            const uint32_t wa = smem_u32(w), oa = smem_u32(o);
 #pragma unroll
-                for (int i = 0; i < 16; i++) v[i] = w[i * HD];
+            for (int i = 0; i < 4; i++) asm volatile("ld.shared.v4.f32 {%0, %1, %2, %3}, [%4];" : "=f"(p[i].x), "=f"(p[i].y), "=f"(p[i].z), "=f"(p[i].w) : "r"(oa + 16 * i));
 #pragma unroll
-                for (int i = 0; i < 4; i++) p[i] = *reinterpret_cast<const float4 *>(o + 4 * i);
-            };
-            auto add = [&](const float (&v)[16], const float4 (&p)[4], int left) {
+            for (int i = 0; i < 16; i++) asm volatile("ld.shared.f32 %0, [%1];" : "=f"(v[i]) : "r"(wa + i * HD * 4));
+        };
+        auto add = [&](const float (&v)[16], const float4 (&p)[4], int left) {
 #pragma unroll
-                for (int i = 0; i < 4; i++) {
-                    if (4 * i < left) acc = __fmaf_rn(v[4 * i], p[i].x, acc);
-                    if (4 * i + 1 < left) acc = __fmaf_rn(v[4 * i + 1], p[i].y, acc);
-                    if (4 * i + 2 < left) acc = __fmaf_rn(v[4 * i + 2], p[i].z, acc);
-                    if (4 * i + 3 < left) acc = __fmaf_rn(v[4 * i + 3], p[i].w, acc);
-                }
-            };
-            load(v0, p0, 0);
-            int k = 0;
+            for (int i = 0; i < 4; i++) {
+                if (4 * i < left) acc = __fmaf_rn(v[4 * i], p[i].x, acc);
+                if (4 * i + 1 < left) acc = __fmaf_rn(v[4 * i + 1], p[i].y, acc);
+                if (4 * i + 2 < left) acc = __fmaf_rn(v[4 * i + 2], p[i].z, acc);
+                if (4 * i + 3 < left) acc = __fmaf_rn(v[4 * i + 3], p[i].w, acc);
+            }
+        };
+        int slot = ntiles % SLOTS;
+        uint32_t par = (uint32_t)(ntiles / SLOTS) & 1u;
+        const float *vt = tiles + (size_t)slot * AT_TILE * HD + tid, *pt = sc;
+        if (ntiles) { waiter.wait(&full[slot], par); load(v0, p0, vt, pt); }
 #pragma unroll 1
-            for (; k + 32 <= cnt; k += 32) {
-                load(v1, p1, k + 16);
+        for (int t = 0; t < nfull; t++) {
+            const int here = slot;
+            const float *vn = vt, *pn = pt;                    // the next tile; behind the last one: read again, not used
+            if (t + 1 < ntiles) {
+                if (++slot == SLOTS) { slot = 0; par ^= 1u; }
+                waiter.wait(&full[slot], par);
+                vn = tiles + (size_t)slot * AT_TILE * HD + tid; pn = pt + AT_TILE;
+            }
+#pragma unroll
+            for (int b = 0; b < BLOCKS; b += 2) {
+                load(v1, p1, vt + (b + 1) * 16 * HD, pt + (b + 1) * 16);
                 add(v0, p0, 16);
-                load(v0, p0, k + 32);
+                if (b + 2 < BLOCKS) load(v0, p0, vt + (b + 2) * 16 * HD, pt + (b + 2) * 16);
+                else load(v0, p0, vn, pn);
                 add(v1, p1, 16);
             }
-            if (k < cnt) {
-                load(v1, p1, k + 16);
-                add(v0, p0, cnt - k);
-                add(v1, p1, cnt - k - 16);
-            }
+            __syncwarp();
+            mbar_arrive_if(lane == 0 ? 1u : 0u, &left_v[here]);      // the tile's values are used: its slot may take another
+            vt = vn; pt = pn;
         }
-        if (tid == 64) add_den(t * AT_TILE, t + 1 < ntiles ? (t + 1) * AT_TILE : n);
-        if (u + SLOTS < 2 * ntiles) {
-            __syncthreads();
-            if (tid == AT_ISSUER) { fence_proxy_async(); issue(u + SLOTS); }
+        for (int k = nfull * AT_TILE; k < ncached; k += 32) {        // the last tile's keys
+            load(v1, p1, vt + 16 * HD, pt + 16);
+            add(v0, p0, ncached - k);
+            add(v1, p1, ncached - k - 16);
+            if (k + 32 < ncached) { vt += 32 * HD; pt += 32; load(v0, p0, vt, pt); }
         }
-    }
-    if (tid == 64) {
-        if (ntiles == 0) add_den(0, n);
+        acc = __fmaf_rn(vcur[tid], sc[ncached], acc);          // t = pos: this token's own v
+    } else if (tid == 64) {
+        float den = brrr_expf_dev(__fsub_rn(sink, mx));
+        // sixteen probabilities at a time, the next sixteen on the way; the last four padded with +0
+        const int quads = (n + 3) >> 2;
+        const uint32_t pa = smem_u32(sc);
+        float4 p0[4], p1[4];
+        auto load = [&](float4 (&p)[4], int k) {              // (past the end: the first quad again, not used)
+#pragma unroll
+            for (int i = 0; i < 4; i++) asm volatile("ld.shared.v4.f32 {%0, %1, %2, %3}, [%4];" : "=f"(p[i].x), "=f"(p[i].y), "=f"(p[i].z), "=f"(p[i].w) : "r"(pa + (k + i < quads ? k + i : 0) * 16));
+        };
+        auto add = [&](const float4 (&p)[4], int left) {
+#pragma unroll
+            for (int i = 0; i < 4; i++)
+                if (i < left) { den = __fadd_rn(den, p[i].x); den = __fadd_rn(den, p[i].y); den = __fadd_rn(den, p[i].z); den = __fadd_rn(den, p[i].w); }
+        };
+        load(p0, 0);
+        int k = 0;
+#pragma unroll 1
+        for (; k + 8 <= quads; k += 8) {
+            load(p1, k + 4);
+            add(p0, 4);
+            load(p0, k + 8);
+            add(p1, 4);
+        }
+        load(p1, k + 4);
+        add(p0, quads - k);
+        add(p1, quads - k - 4);
         den_sh = den;
     }
-    if (tid < 64) acc = __fmaf_rn(vcur[tid], sc[ncached], acc);          // t = pos: this token's own v
-    __syncthreads();
+    bar_workers();
     if (tid < 64) {
         float inv = __fdiv_rn(1.0f, den_sh);
         float o = __fmul_rn(acc, inv);
@@ -504,11 +582,11 @@ cudaError_t launch_attn_decode(const float *qkv, float *kc, float *vc, const flo
     if (row_pos) {
         cudaError_t e = smem_optin(attn_decode_kernel<AT_TILE_ROWS>, (int)attn_smem(AT_TILE_ROWS), configured_rows);
         if (e != cudaSuccess) return e;
-        return launch_k(attn_decode_kernel<AT_TILE_ROWS>, dim3(nh, rows), dim3(AT_THREADS), attn_smem(AT_TILE_ROWS), st, pdl, a);
+        return launch_k(attn_decode_kernel<AT_TILE_ROWS>, dim3(nh, rows), dim3(at_threads(AT_TILE_ROWS)), attn_smem(AT_TILE_ROWS), st, pdl, a);
     }
     cudaError_t e = smem_optin(attn_decode_kernel<AT_TILE_ONE>, (int)attn_smem(AT_TILE_ONE), configured);
     if (e != cudaSuccess) return e;
-    return launch_k(attn_decode_kernel<AT_TILE_ONE>, dim3(nh, 1), dim3(AT_THREADS), attn_smem(AT_TILE_ONE), st, pdl, a);
+    return launch_k(attn_decode_kernel<AT_TILE_ONE>, dim3(nh, 1), dim3(at_threads(AT_TILE_ONE)), attn_smem(AT_TILE_ONE), st, pdl, a);
 }
 
 // Attention for token rows of ONE sequence with ascending positions (a prompt tile): rows share the K / V tiles.

@@ -59,6 +59,27 @@ def test_batch_rows_equal_each_sequence_alone(brrr):
     eng.close()
 
 
+def test_batch_attention_at_tile_borders(brrr):
+    """Rows whose caches end at, before and behind the borders of the rows' 32-position tiles and around the ring's depth of four."""
+    cfg = brrr.make_cfg(128, 2, 4, 2, 8, 4, 512, sliding_window=64)
+    eng = brrr.Engine.synth(cfg, 23)
+    eng.set_tile_prefill(False)
+    lens = [2, 16, 17, 32, 33, 34, 64, 65, 66, 97, 128, 129, 130, 161, 193]
+    prompts = [[int(t) for t in S.synth_prompt(80 + i, n, 500)] for i, n in enumerate(lens)]
+    want = [serial_run(eng, p, 2, want_logits_at=1) for p in prompts]
+    eng.batch_open(len(prompts))
+    for s, p in enumerate(prompts):
+        eng.batch_prefill(s, p[:-1])
+    seqs = list(range(len(prompts)))
+    first = eng.batch_step([p[-1] for p in prompts], [n - 1 for n in lens], seqs)
+    assert [int(t) for t in first] == [w[0][0] for w in want]
+    second, lg = eng.batch_step([int(t) for t in first], lens, seqs, logits=True)
+    assert [int(t) for t in second] == [w[0][1] for w in want]
+    for s in seqs:
+        assert np.array_equal(bits(lg[s]), bits(want[s][1])), f"logits of sequence {s}"
+    eng.close()
+
+
 def test_batch_ragged_and_mixed_rows(brrr):
     """Sequences leave the batch at different times; one pass mixes the prompt rows of a late sequence
     (ascending positions of one sequence) with single decode rows of the others; 64 rows in one pass."""

@@ -247,6 +247,12 @@ def test_attention_decode(L, orc, brrr, dev, pos, start):
     assert np.array_equal(daq.cpu().numpy(), aq) and np.array_equal(bits(das.cpu().numpy()), bits(asb))
 
 
+@pytest.mark.parametrize("pos", [1, 15, 16, 17, 63, 64, 65, 127, 128, 191, 192, 193, 511, 512, 513, 575, 576, 577, 641])
+def test_attention_decode_at_tile_borders(L, orc, brrr, dev, pos):
+    """Whole and partial 64-position tiles around the ring's depth of eight, one and two score passes at a time, sums of 16 and of fewer keys."""
+    test_attention_decode(L, orc, brrr, dev, pos, 0)
+
+
 @pytest.mark.parametrize("kind,type_,n", [("BQ", 0, 4096), ("ATTN_NORM", 0, 2880), ("SINKS", 0, 64), ("WQ", 30, 64 * 2880), ("GATE", 39, 32 * 2880)])
 def test_synth_device_equals_numpy(L, dev, kind, type_, n):
     import torch
