@@ -39,6 +39,36 @@ __device__ __forceinline__ float brrr_expf_dev(float x) {
     return __fmul_rn(__fmul_rn(y, s1), s2);
 }
 
+// brrr_expf_dev of N values, step by step side by side, the special cases as selections (as branches they keep calls from overlapping: 260 cycles each
+// in a loop of 32).
+template <int N>
+__device__ __forceinline__ void brrr_expf_n(float *x) {
+    float kf[N], r[N], p[N], y[N];
+#pragma unroll
+    for (int i = 0; i < N; i++) kf[i] = rintf(__fmul_rn(x[i], 1.44269504088896341f));
+#pragma unroll
+    for (int i = 0; i < N; i++) r[i] = __fmaf_rn(kf[i], -0.693145751953125f, x[i]);
+#pragma unroll
+    for (int i = 0; i < N; i++) r[i] = __fmaf_rn(kf[i], -1.42860682030941723212e-6f, r[i]);
+    constexpr float c[5] = {1.3981999507e-3f, 8.3334519073e-3f, 4.1665795894e-2f, 1.6666665459e-1f, 5.0000001201e-1f};
+#pragma unroll
+    for (int i = 0; i < N; i++) p[i] = 1.9875691500e-4f;
+#pragma unroll
+    for (int k = 0; k < 5; k++)
+#pragma unroll
+        for (int i = 0; i < N; i++) p[i] = __fmaf_rn(p[i], r[i], c[k]);
+#pragma unroll
+    for (int i = 0; i < N; i++) y[i] = __fadd_rn(__fmaf_rn(p[i], __fmul_rn(r[i], r[i]), r[i]), 1.0f);
+#pragma unroll
+    for (int i = 0; i < N; i++) {
+        const int k = (int)kf[i], k1 = k >> 1, k2 = k - k1;
+        y[i] = __fmul_rn(__fmul_rn(y[i], __int_as_float((k1 + 127) << 23)), __int_as_float((k2 + 127) << 23));
+        y[i] = x[i] > 88.72283935546875f ? __int_as_float(0x7f800000) : y[i];
+        y[i] = x[i] < -104.0f ? 0.0f : y[i];
+        x[i] = x[i] != x[i] ? x[i] + x[i] : y[i];
+    }
+}
+
 // 2^(e-128) for an e8m0 byte (the doubled e2m1 table), exact including e = 0, 1 (subnormal).
 __device__ __forceinline__ float brrr_e8m0_scale(uint32_t e) {
     return __int_as_float(e >= 2u ? (e - 1u) << 23 : 0x00200000u << e);

@@ -21,6 +21,7 @@
 #include "brrr_kernels.h"
 #include "brrr_block.cuh"
 #include "brrr_tma.cuh"
+#include "brrr_tc.cuh"
 #include "brrr_tile.cuh"
 
 #include <type_traits>
@@ -367,16 +368,19 @@ __global__ void __launch_bounds__(at_threads(AT_TILE)) attn_decode_kernel(AttnAr
 // where kv_append_rows_kernel wrote the same bits):
 //   score(t)  one thread: the 16 four-term chains, then the pairwise combine of the shuffle butterfly (xor 4, 8, 1, 2)
 //   pass 1    scores of every key -> workspace, the pair's maximum;  pass 2  p = exp(s - mx) into shared memory,
-//             then, tile by tile in ascending key order, the serial denominator (one thread per pair) and the serial
-//             p.V sums (one thread per (dim, 8 pairs)).  Keys outside a pair's range carry p = +0: x + 0 = x exactly
+//             (half of the warps) and, a tile behind and in ascending key order, the serial p.V sums (the other half: a thread for 8 dims of 2
+//             pairs) and by the threads of the first dims the serial denominators.  Keys outside a pair's range carry p = +0: x + 0 = x exactly
 //             (no accumulator is ever -0: the sums start at +0 and round to nearest), so they need no branch.
-// 32 pairs x 4096 keys of scores do not fit shared memory: they wait in a workspace (written and read by the same thread, 128 bytes per key and
-// warp; mostly L2).  Formed twice instead, a 512-row tile at positions 1024 .. 1535 took 895 us, now 742.
+// 32 pairs x 4096 keys of scores do not fit shared memory: they wait in a workspace (128 bytes per key; mostly L2).
+// What bounds it is shared memory: a key's row reaches a warp as 16 broadcast words of 16 bytes, 3 to 4 cycles each, for 80 arithmetic instructions
+// (40 packed ones), and a key of the p.V sums costs every thread 40 bytes for 16 multiply-adds.  Two CTAs per SM fill each other's barriers.  512 rows of
+// the 20b shape: window layer 79 to 87 us, full layer 122 / 285 / 449 us at positions 0 / 512 / 1024 (before, with tiles of 128 keys, one CTA per SM,
+// scalar scores and every warp in the same phase: 140 to 146, 221 / 483 / 742).  Two pairs per thread and one CTA per SM took 85 to 95, 124 / 298 / 471.
 constexpr int AR_THREADS = 256;
-constexpr int AR_TILE = 128;
 constexpr int AR_PAIRS = 32;
+constexpr int AR_TILE = 64;
 constexpr size_t AR_TILE_BYTES = (size_t)AR_TILE * HD * sizeof(float);
-constexpr size_t AR_SMEM = 4 * AR_TILE_BYTES + (size_t)AR_TILE * AR_PAIRS * 4 + (size_t)AR_PAIRS * HD * 4;
+constexpr size_t AR_SMEM = 4 * AR_TILE_BYTES + 2 * (size_t)AR_TILE * AR_PAIRS * 4 + (size_t)AR_PAIRS * HD * 4;
 
 struct AttnRowsArgs {
     const float *qkv;        // [rows][ldq]: q | k | v of every row, bias added, not rotated
@@ -393,180 +397,235 @@ struct AttnRowsArgs {
     DevState *err_state;
 };
 
-// one score: q in registers, the key's 64 floats at kp (shared memory, the same address in every lane)
-__device__ __forceinline__ float ar_score(const float (&q)[HD], const float *kp) {
-    float a[16];
+// one score: q in registers, the key's 64 floats at kp (shared memory, the same address in every lane); two chains per instruction
+__device__ __forceinline__ float ar_score(const f32x2 (&q)[HD / 2], const float *kp) {
+    // butterfly xor 4, 8, 1, 2 of the 16-thread group, as one thread: chains i and 4 + i, 8 + i and 12 + i, then both, then across i
+    f32x2 a[2], lo[2];
+    const uint32_t ka = smem_u32(kp);
 #pragma unroll
     for (int c4 = 0; c4 < 4; c4++) {
-        const float4 k0 = *reinterpret_cast<const float4 *>(kp + 4 * c4), k1 = *reinterpret_cast<const float4 *>(kp + 16 + 4 * c4);
-        const float4 k2 = *reinterpret_cast<const float4 *>(kp + 32 + 4 * c4), k3 = *reinterpret_cast<const float4 *>(kp + 48 + 4 * c4);
-        const float kk0[4] = {k0.x, k0.y, k0.z, k0.w}, kk1[4] = {k1.x, k1.y, k1.z, k1.w}, kk2[4] = {k2.x, k2.y, k2.z, k2.w}, kk3[4] = {k3.x, k3.y, k3.z, k3.w};
+        f32x2 k[4][2];
 #pragma unroll
-        for (int i = 0; i < 4; i++) {
-            const int c = 4 * c4 + i;
-            float v = __fmaf_rn(kk0[i], q[c], 0.0f);
-            v = __fmaf_rn(kk1[i], q[16 + c], v);
-            v = __fmaf_rn(kk2[i], q[32 + c], v);
-            a[c] = __fmaf_rn(kk3[i], q[48 + c], v);
+        for (int m = 0; m < 4; m++) lds_pairs(ka + (16 * m + 4 * c4) * 4, k[m][0], k[m][1]);
+#pragma unroll
+        for (int i = 0; i < 2; i++) {
+            f32x2 v = tl_fma2(k[0][i], q[2 * c4 + i], 0ull);
+#pragma unroll
+            for (int m = 1; m < 4; m++) v = tl_fma2(k[m][i], q[8 * m + 2 * c4 + i], v);
+            if (c4 & 1) v = tl_add2(a[i], v);
+            if (c4 == 1) lo[i] = v;
+            else if (c4 == 3) lo[i] = tl_add2(lo[i], v);
+            else a[i] = v;
         }
     }
-    // butterfly xor 4, 8, 1, 2 of the 16-thread group, as one thread
-    const float b0 = __fadd_rn(a[0], a[4]), b1 = __fadd_rn(a[1], a[5]), b2 = __fadd_rn(a[2], a[6]), b3 = __fadd_rn(a[3], a[7]);
-    const float b8 = __fadd_rn(a[8], a[12]), b9 = __fadd_rn(a[9], a[13]), b10 = __fadd_rn(a[10], a[14]), b11 = __fadd_rn(a[11], a[15]);
-    const float c0 = __fadd_rn(b0, b8), c1 = __fadd_rn(b1, b9), c2 = __fadd_rn(b2, b10), c3 = __fadd_rn(b3, b11);
-    return __fmul_rn(__fadd_rn(__fadd_rn(c0, c1), __fadd_rn(c2, c3)), 0.125f);
+    float c[4];
+    tl_unpack2(lo[0], c[0], c[1]);
+    tl_unpack2(lo[1], c[2], c[3]);
+    return __fmul_rn(__fadd_rn(__fadd_rn(c[0], c[1]), __fadd_rn(c[2], c[3])), 0.125f);
 }
 
-__global__ void __launch_bounds__(AR_THREADS) attn_rows_kernel(AttnRowsArgs a) {
+__global__ void __launch_bounds__(AR_THREADS, 2) attn_rows_kernel(AttnRowsArgs a) {
+    constexpr int HALF = AR_THREADS / 2;                           // pass 2: threads of the sums, and of the probabilities
     extern __shared__ __align__(128) unsigned char smraw[];
     float *ktile = reinterpret_cast<float *>(smraw);                                    // [2][128][64]
     float *vtile = reinterpret_cast<float *>(smraw + 2 * AR_TILE_BYTES);                // [2][128][64]
-    float *psm = reinterpret_cast<float *>(smraw + 4 * AR_TILE_BYTES);                  // [128 keys][32 pairs]
-    float *qsm = psm + AR_TILE * AR_PAIRS;                                              // [32 pairs][64]
+    float *psm = reinterpret_cast<float *>(smraw + 4 * AR_TILE_BYTES);                  // [2][128 keys][pairs]
+    float *qsm = psm + 2 * AR_TILE * AR_PAIRS;                                             // [pairs][64]: q, then the outputs
     __shared__ __align__(8) uint64_t kbar[2], vbar[2];
     __shared__ float red[AR_THREADS / 32][AR_PAIRS];
     __shared__ float mx_sm[AR_PAIRS], den_sm[AR_PAIRS];
     __shared__ int pos_sm[AR_PAIRS];
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-    const int group = a.nh / a.nkv, rb = AR_PAIRS / group;        // rows per CTA
-    const int kvh = blockIdx.x, r0 = blockIdx.y * rb;
+    const int group = a.nh / a.nkv, lg = 31 - __clz(group), rb = AR_PAIRS >> lg;      // heads per KV head: a power of two; rows per CTA
+    const int kvh = blockIdx.x, r0 = (gridDim.y - 1 - blockIdx.y) * rb;      // the last rows, whose ranges are the longest, first
     const int nrows = min(rb, a.rows - r0);
     uint32_t *err = a.err_state ? &a.err_state->err : nullptr;
     Waiter waiter(err);
     if (tid == 0) {
-        mbar_init(&kbar[0], 1); mbar_init(&kbar[1], 1); mbar_init(&vbar[0], 1); mbar_init(&vbar[1], 1);
+        for (int i = 0; i < 2; i++) { mbar_init(&kbar[i], 1); mbar_init(&vbar[i], 1); }
         mbar_fence_init();
     }
     pdl_wait();          // q/k/v projection and the cache append of every row are done
     pdl_trigger();
     waiter.poison_if_failed();
     // ---- the pairs: pair = row-in-block * group + head-in-group
-    const int pr = lane;                                           // this thread's pair in the score phases
-    const int pr_row = pr / group, pr_h = kvh * group + pr % group;
-    const bool pr_live = pr_row < nrows;
-    if (tid < AR_PAIRS) pos_sm[tid] = (tid / group) < nrows ? a.row_pos[r0 + tid / group] : -1;
-    // RoPE of q (NeoX halves), 1024 rotations over 256 threads
-    for (int idx = tid; idx < AR_PAIRS * 32; idx += AR_THREADS) {
-        const int p2 = idx >> 5, i = idx & 31, rr = p2 / group;
-        if (rr < nrows) {
-            const int pos = a.row_pos[r0 + rr];
-            const float *src = a.qkv + (size_t)(r0 + rr) * a.ldq + (size_t)(kvh * group + p2 % group) * HD;
-            const float c = a.rope[((size_t)pos * 32 + i) * 2], sn = a.rope[((size_t)pos * 32 + i) * 2 + 1];
-            const float x0 = src[i], x1 = src[32 + i];
-            qsm[p2 * HD + i] = __fsub_rn(__fmul_rn(x0, c), __fmul_rn(x1, sn));
-            qsm[p2 * HD + 32 + i] = __fadd_rn(__fmul_rn(x1, c), __fmul_rn(x0, sn));
-        } else { qsm[p2 * HD + i] = 0.0f; qsm[p2 * HD + 32 + i] = 0.0f; }
+    if (tid < AR_PAIRS) pos_sm[tid] = (tid >> lg) < nrows ? a.row_pos[r0 + (tid >> lg)] : -1;
+    // RoPE of q (NeoX halves): a warp = a pair; every load before the first store (a store in between would order the loads behind it)
+    {
+        constexpr int N = AR_PAIRS / (AR_THREADS / 32);
+        float x0[N], x1[N], rc[N], rs[N];
+#pragma unroll
+        for (int k = 0; k < N; k++) {
+            const int p2 = warp + k * (AR_THREADS / 32), rr = p2 >> lg;
+            x0[k] = x1[k] = rc[k] = rs[k] = 0.0f;
+            if (rr < nrows) {
+                const float *src = a.qkv + (size_t)(r0 + rr) * a.ldq + (size_t)(kvh * group + (p2 & (group - 1))) * HD, *rot = a.rope + ((size_t)a.row_pos[r0 + rr] * 32 + lane) * 2;
+                x0[k] = src[lane]; x1[k] = src[32 + lane]; rc[k] = rot[0]; rs[k] = rot[1];
+            }
+        }
+#pragma unroll
+        for (int k = 0; k < N; k++) {
+            float *o = qsm + (warp + k * (AR_THREADS / 32)) * HD + lane;
+            o[0] = __fsub_rn(__fmul_rn(x0[k], rc[k]), __fmul_rn(x1[k], rs[k]));
+            o[32] = __fadd_rn(__fmul_rn(x1[k], rc[k]), __fmul_rn(x0[k], rs[k]));
+        }
     }
     __syncthreads();
-    float q[HD];
-#pragma unroll
-    for (int i = 0; i < HD; i++) q[i] = qsm[pr * HD + i];
-    const int my_pos = pos_sm[pr];
-    const int my_start = a.window > 0 ? max(my_pos - (a.window - 1), 0) : 0;
     // key range of the block: from the first row's window start to the last row's position
     const int pos_first = pos_sm[0], pos_last = pos_sm[(nrows - 1) * group];
     const int t_lo = a.window > 0 ? max(pos_first - (a.window - 1), 0) : 0;
     const int nkeys = pos_last - t_lo + 1, ntiles = (nkeys + AR_TILE - 1) / AR_TILE;
     const size_t seq_off = (size_t)a.row_seq[r0] * a.seq_stride;
-    const float *kbase = a.kc + seq_off + ((size_t)kvh * BRRR_MAXSEQ + t_lo) * HD;
-    const float *vbase = a.vc + seq_off + ((size_t)kvh * BRRR_MAXSEQ + t_lo) * HD;
-    int k_issued = 0, v_issued = 0, k_used = 0, v_used = 0;       // tiles issued / consumed so far (buffer = count & 1, parity = count >> 1 & 1)
-    auto issue_k = [&](int t) {       // thread 0
-        const int buf = k_issued & 1, cnt = min(AR_TILE, nkeys - t * AR_TILE);
-        mbar_expect_tx(&kbar[buf], (uint32_t)cnt * HD * 4);
-        bulk_g2s(ktile + (size_t)buf * AR_TILE * HD, kbase + (size_t)t * AR_TILE * HD, (uint32_t)cnt * HD * 4, &kbar[buf]);
-    };
-    auto issue_v = [&](int t) {
-        const int buf = v_issued & 1, cnt = min(AR_TILE, nkeys - t * AR_TILE);
-        mbar_expect_tx(&vbar[buf], (uint32_t)cnt * HD * 4);
-        bulk_g2s(vtile + (size_t)buf * AR_TILE * HD, vbase + (size_t)t * AR_TILE * HD, (uint32_t)cnt * HD * 4, &vbar[buf]);
+    // one thread: tile t of K or V into its buffer (t & 1)
+    auto issue = [&](const float *cache, float *buf, uint64_t *bar, int t) {
+        const uint32_t bytes = (uint32_t)min(AR_TILE, nkeys - t * AR_TILE) * HD * 4;
+        mbar_expect_tx(&bar[t & 1], bytes);
+        bulk_g2s(buf + (size_t)(t & 1) * AR_TILE * HD, cache + seq_off + ((size_t)kvh * BRRR_MAXSEQ + t_lo + (size_t)t * AR_TILE) * HD, bytes, &bar[t & 1]);
     };
 
-    float *my_scores = a.scores + ((size_t)blockIdx.y * a.nkv + kvh) * BRRR_MAXSEQ * AR_PAIRS + lane;
-    // ---- pass 1: the maximum of every pair's scores
+    const int my_pos = pos_sm[lane];                               // this thread's pair in the score phases; -1: no such row, and no key
+    const int my_start = a.window > 0 ? max(my_pos - (a.window - 1), 0) : 0;
     float mx = -3.4028234663852886e38f;
-    if (tid == 0) issue_k(0);
-    k_issued++;
-    for (int t = 0; t < ntiles; t++) {
-        if (t + 1 < ntiles) { if (tid == 0) issue_k(t + 1); k_issued++; }        // the other buffer: free since the barrier that ended tile t - 1
-        const int buf = k_used & 1;
-        waiter.wait(&kbar[buf], (uint32_t)(k_used >> 1) & 1u);
-        k_used++;
-        const float *kt = ktile + (size_t)buf * AR_TILE * HD;
-        const int cnt = min(AR_TILE, nkeys - t * AR_TILE), tb = t_lo + t * AR_TILE;
-        for (int kk = warp; kk < cnt; kk += AR_THREADS / 32) {
-            const float sc = ar_score(q, kt + kk * HD);
-            const int key = tb + kk;
-            my_scores[(size_t)(t * AR_TILE + kk) * AR_PAIRS] = sc;
-            if (pr_live && key >= my_start && key <= my_pos) mx = fmaxf(mx, sc);
+    float *my_scores = a.scores + ((size_t)blockIdx.y * a.nkv + kvh) * BRRR_MAXSEQ * AR_PAIRS + lane;
+    {
+        // ---- pass 1: the maximum of every pair's scores
+        f32x2 q[HD / 2];
+#pragma unroll
+        for (int i = 0; i < HD / 2; i += 2) lds_pairs(smem_u32(qsm + lane * HD + 2 * i), q[i], q[i + 1]);
+        if (tid == 0) { issue(a.kc, ktile, kbar, 0); issue(a.vc, vtile, vbar, 0); }
+        for (int t = 0; t < ntiles; t++) {
+            if (tid == 0 && t + 1 < ntiles) issue(a.kc, ktile, kbar, t + 1);      // the other buffer: free since the barrier that ended tile t - 1
+            waiter.wait(&kbar[t & 1], (uint32_t)(t >> 1) & 1u);
+            const float *kt = ktile + (size_t)(t & 1) * AR_TILE * HD;
+            const int cnt = min(AR_TILE, nkeys - t * AR_TILE), tb = t_lo + t * AR_TILE;
+            for (int kk = warp; kk < cnt; kk += AR_THREADS / 32) {
+                const float sc = ar_score(q, kt + kk * HD);
+                const int key = tb + kk;
+                my_scores[(size_t)(t * AR_TILE + kk) * AR_PAIRS] = sc;
+                if (key >= my_start && key <= my_pos) mx = fmaxf(mx, sc);
+            }
+            __syncthreads();              // everyone is done with this buffer
+            if (tid == 0) fence_proxy_async();
         }
-        __syncthreads();              // everyone is done with this buffer
-        if (tid == 0) fence_proxy_async();
     }
     red[warp][lane] = mx;
     __syncthreads();
     if (tid < AR_PAIRS) {
-        float m = a.sinks[kvh * group + tid % group];
+        const float sink = a.sinks[kvh * group + (tid & (group - 1))];
+        float m = sink;
 #pragma unroll
         for (int w = 0; w < AR_THREADS / 32; w++) m = fmaxf(m, red[w][tid]);
         mx_sm[tid] = m;
-        den_sm[tid] = brrr_expf_dev(__fsub_rn(a.sinks[kvh * group + tid % group], m));      // the sink's term opens the denominator
+        den_sm[tid] = brrr_expf_dev(__fsub_rn(sink, m));           // the sink's term opens the denominator
     }
     __syncthreads();
-    mx = mx_sm[pr];
+    mx = mx_sm[lane];
 
-    // ---- pass 2: probabilities tile by tile; denominator and p.V sums in ascending key order
-    const int u = tid & 63, grp = tid >> 6;                        // this thread in the p.V phase: dim u of pairs grp * 8 .. + 7
-    float acc[8];
+    // ---- pass 2: half of the warps make the probabilities of a tile while the other half forms the sums of the tile before, in ascending key order
+    if (tid >= HALF) {
+        constexpr int KEYS = AR_TILE / (HALF / 32);                // of a thread per tile: w, w + 4, ...
+        const int w = warp - HALF / 32;
+        float sv[KEYS], next[KEYS];                                // scores of this tile and of the next, on their way meanwhile
+        auto fetch = [&](float (&o)[KEYS], int t) {
+            const int cnt = min(AR_TILE, nkeys - t * AR_TILE);
+            const float *src = my_scores + (size_t)(t * AR_TILE + w) * AR_PAIRS;
 #pragma unroll
-    for (int j = 0; j < 8; j++) acc[j] = 0.0f;
-    float den = tid < AR_PAIRS ? den_sm[tid] : 0.0f;
-    if (tid == 0) issue_v(0);
-    v_issued++;
-    for (int t = 0; t < ntiles; t++) {
-        if (t + 1 < ntiles) { if (tid == 0) issue_v(t + 1); v_issued++; }
-        const int vb = v_used & 1;
-        const int cnt = min(AR_TILE, nkeys - t * AR_TILE), tb = t_lo + t * AR_TILE;
-        float sv[AR_TILE / 8];                // this thread's keys warp, warp + 8, ... of the tile
+            for (int i = 0; i < KEYS; i++) o[i] = w + HALF / 32 * i < cnt ? src[HALF / 32 * i * AR_PAIRS] : 0.0f;
+        };
+        fetch(sv, 0);
+#pragma unroll 1
+        for (int t = 0; t <= ntiles; t++) {
+            if (t < ntiles) {
+                if (t + 1 < ntiles) fetch(next, t + 1);
+                const int cnt = min(AR_TILE, nkeys - t * AR_TILE), tb = t_lo + t * AR_TILE;
+                float *pb = psm + (size_t)(t & 1) * AR_TILE * AR_PAIRS + lane;
+                // eight exponentials side by side (one after the other they take 190 cycles each)
+                constexpr int SIDE = 8;
 #pragma unroll
-        for (int i = 0; i < AR_TILE / 8; i++) sv[i] = warp + 8 * i < cnt ? my_scores[(size_t)(t * AR_TILE + warp + 8 * i) * AR_PAIRS] : 0.0f;
+                for (int i0 = 0; i0 < KEYS; i0 += SIDE) {
+                    float e[SIDE];
 #pragma unroll
-        for (int i = 0; i < AR_TILE / 8; i++) {
-            const int kk = warp + 8 * i, key = tb + kk;
-            const bool valid = kk < cnt && pr_live && key >= my_start && key <= my_pos;
-            if (kk < cnt) psm[kk * AR_PAIRS + pr] = valid ? brrr_expf_dev(__fsub_rn(sv[i], mx)) : 0.0f;
+                    for (int i = 0; i < SIDE; i++) e[i] = __fsub_rn(sv[i0 + i], mx);
+                    brrr_expf_n<SIDE>(e);
+#pragma unroll
+                    for (int i = 0; i < SIDE; i++) {
+                        const int kk = w + HALF / 32 * (i0 + i), key = tb + kk;
+                        if (kk < cnt) pb[kk * AR_PAIRS] = key >= my_start && key <= my_pos ? e[i] : 0.0f;
+                    }
+                }
+#pragma unroll
+                for (int i = 0; i < KEYS; i++) sv[i] = next[i];
+            }
+            __syncthreads();           // probabilities of tile t are there, the sums of tile t - 1 done
         }
+        __syncthreads();               // outputs in shared memory
+    } else {
+        const int dq = tid & 7, pg = tid >> 3;                     // dims 4 dq .. + 3 and 32 + 4 dq .. + 3 of pairs 2 pg and 2 pg + 1
+        float acc[2][8];
+#pragma unroll
+        for (int j = 0; j < 2; j++)
+#pragma unroll
+            for (int i = 0; i < 8; i++) acc[j][i] = 0.0f;
+        float den = den_sm[2 * pg + (dq & 1)];                     // of one of the pairs (the threads past the first two repeat them)
         __syncthreads();
-        if (tid < AR_PAIRS) {
-#pragma unroll 8
-            for (int kk = 0; kk < cnt; kk++) den = __fadd_rn(den, psm[kk * AR_PAIRS + tid]);
-        }
-        waiter.wait(&vbar[vb], (uint32_t)(v_used >> 1) & 1u);
-        v_used++;
-        const float *vt = vtile + (size_t)vb * AR_TILE * HD + u;
-        const float *pt = psm + grp * 8;
+        for (int t = 0; t < ntiles; t++) {
+            const int cnt = min(AR_TILE, nkeys - t * AR_TILE);
+            if (tid == 0 && t + 1 < ntiles) { fence_proxy_async(); issue(a.vc, vtile, vbar, t + 1); }      // its buffer: the sums of tile t - 1 are done
+            waiter.wait(&vbar[t & 1], (uint32_t)(t >> 1) & 1u);
+            const float *vt = vtile + (size_t)(t & 1) * AR_TILE * HD + 4 * dq, *pt = psm + (size_t)(t & 1) * AR_TILE * AR_PAIRS + 2 * pg;
 #pragma unroll 4
-        for (int kk = 0; kk < cnt; kk++) {
-            const float v = vt[kk * HD];
-            const float4 p0 = *reinterpret_cast<const float4 *>(pt + kk * AR_PAIRS), p1 = *reinterpret_cast<const float4 *>(pt + kk * AR_PAIRS + 4);
-            acc[0] = __fmaf_rn(v, p0.x, acc[0]); acc[1] = __fmaf_rn(v, p0.y, acc[1]); acc[2] = __fmaf_rn(v, p0.z, acc[2]); acc[3] = __fmaf_rn(v, p0.w, acc[3]);
-            acc[4] = __fmaf_rn(v, p1.x, acc[4]); acc[5] = __fmaf_rn(v, p1.y, acc[5]); acc[6] = __fmaf_rn(v, p1.z, acc[6]); acc[7] = __fmaf_rn(v, p1.w, acc[7]);
-        }
-        __syncthreads();              // the tile's buffers and the probabilities are free
-        if (tid == 0) fence_proxy_async();
-    }
-    if (tid < AR_PAIRS) den_sm[tid] = den;
-    __syncthreads();
-    // ---- outputs: o = acc / den, and the Q8 image of every pair's two 32-blocks (a warp = one 32-block of a pair)
+            for (int kk = 0; kk < cnt; kk++) {
+                const float4 v = *reinterpret_cast<const float4 *>(vt + kk * HD), v2 = *reinterpret_cast<const float4 *>(vt + kk * HD + 32);
+                const float2 w = *reinterpret_cast<const float2 *>(pt + kk * AR_PAIRS);
+                const float p[2] = {w.x, w.y};
 #pragma unroll
-    for (int j = 0; j < 8; j++) {
-        const int p2 = grp * 8 + j, rr = p2 / group, h = kvh * group + p2 % group;
-        if (rr < nrows) {             // uniform over the warp
-            const float inv = __fdiv_rn(1.0f, den_sm[p2]);
-            const float o = __fmul_rn(acc[j], inv);
+                for (int j = 0; j < 2; j++) {
+                    acc[j][0] = __fmaf_rn(v.x, p[j], acc[j][0]); acc[j][1] = __fmaf_rn(v.y, p[j], acc[j][1]);
+                    acc[j][2] = __fmaf_rn(v.z, p[j], acc[j][2]); acc[j][3] = __fmaf_rn(v.w, p[j], acc[j][3]);
+                    acc[j][4] = __fmaf_rn(v2.x, p[j], acc[j][4]); acc[j][5] = __fmaf_rn(v2.y, p[j], acc[j][5]);
+                    acc[j][6] = __fmaf_rn(v2.z, p[j], acc[j][6]); acc[j][7] = __fmaf_rn(v2.w, p[j], acc[j][7]);
+                }
+                den = __fadd_rn(den, (dq & 1) ? w.y : w.x);
+            }
+            __syncthreads();
+        }
+        // ---- outputs: o = acc / den through shared memory, then the Q8 image of every pair's two 32-blocks (a warp = one 32-block of a pair)
+        const float inv1 = __fdiv_rn(1.0f, den);                   // lane dq of a group of eight holds pair dq & 1
+#pragma unroll
+        for (int j = 0; j < 2; j++) {
+            const float inv = __shfl_sync(0xffffffffu, inv1, (lane & 24) + j);
+            float *o = qsm + (2 * pg + j) * HD + 4 * dq;
+            *reinterpret_cast<float4 *>(o) = make_float4(__fmul_rn(acc[j][0], inv), __fmul_rn(acc[j][1], inv), __fmul_rn(acc[j][2], inv), __fmul_rn(acc[j][3], inv));
+            *reinterpret_cast<float4 *>(o + 32) = make_float4(__fmul_rn(acc[j][4], inv), __fmul_rn(acc[j][5], inv), __fmul_rn(acc[j][6], inv), __fmul_rn(acc[j][7], inv));
+        }
+        __syncthreads();               // outputs in shared memory
+    }
+    // (four at a time, side by side)
+    constexpr int SIDE = 4, BLOCKS = 2 * AR_PAIRS / (AR_THREADS / 32);
+#pragma unroll 1
+    for (int k0 = warp * BLOCKS; k0 < (warp + 1) * BLOCKS; k0 += SIDE) {
+        float o[SIDE], amax[SIDE];
+#pragma unroll
+        for (int k = 0; k < SIDE; k++) { o[k] = qsm[(k0 + k) * 32 + lane]; amax[k] = fabsf(o[k]); }
+#pragma unroll
+        for (int x = 16; x > 0; x >>= 1)
+#pragma unroll
+            for (int k = 0; k < SIDE; k++) amax[k] = fmaxf(amax[k], __shfl_xor_sync(0xffffffffu, amax[k], x));
+#pragma unroll
+        for (int k = 0; k < SIDE; k++) amax[k] = fmaxf(amax[k], 1e-12f);
+        float sc[SIDE];
+#pragma unroll
+        for (int k = 0; k < SIDE; k++) sc[k] = __fdiv_rn(amax[k], 127.0f);
+#pragma unroll
+        for (int k = 0; k < SIDE; k++) {
+            const int p2 = (k0 + k) >> 1, rr = p2 >> lg, b = (kvh * group + (p2 & (group - 1))) * 2 + ((k0 + k) & 1);
+            if (rr >= nrows) break;             // uniform over the warp; the rows ascend
+            const int qv = brrr_q8_round_inv(o[k], sc[k], brrr_q8_inv(amax[k]));
             const size_t row = (size_t)(r0 + rr);
-            a.ao[row * a.nh * HD + h * HD + u] = o;
-            attn_quant(o, lane, h * 2 + (u >> 5), a.aq ? a.aq + row * a.nh * HD : nullptr, a.as + row * a.nh * 2, a.img ? a.img + row * a.nh * ti_pair(TI_HALF) : nullptr);
+            a.ao[row * a.nh * HD + b * 32 + lane] = o[k];
+            if (lane == 0) a.as[row * a.nh * 2 + b] = sc[k];
+            if (a.aq) a.aq[row * a.nh * HD + b * 32 + lane] = (int8_t)qv;
+            if (a.img) ti_emit_block<TI_HALF>(qv, lane, b, a.img + row * a.nh * ti_pair(TI_HALF));
         }
     }
 }
