@@ -50,9 +50,10 @@ __device__ __forceinline__ void kt_box(uint32_t dst, const CUtensorMap *map, int
                  "r"(smem_u32(bar))
                  : "memory");
 }
-__device__ __forceinline__ void kt_mma(uint32_t d, uint32_t a, uint64_t b, uint32_t idesc, uint32_t accumulate) {
-    asm volatile("{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %4, 0;\n\t"
-                 "tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], %2, %3, {%5, %5, %5, %5}, p;\n\t}" ::"r"(d), "r"(a), "l"(b), "r"(idesc), "r"(accumulate), "r"(0u)
+// (issue: the elected lane's predicate, see tl_commit_if)
+__device__ __forceinline__ void kt_mma(uint32_t issue, uint32_t d, uint32_t a, uint64_t b, uint32_t idesc, uint32_t accumulate) {
+    asm volatile("{\n\t.reg .pred p, e;\n\tsetp.ne.b32 p, %4, 0;\n\tsetp.ne.b32 e, %6, 0;\n\t"
+                 "@e tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], %2, %3, {%5, %5, %5, %5}, p;\n\t}" ::"r"(d), "r"(a), "l"(b), "r"(idesc), "r"(accumulate), "r"(0u), "r"(issue)
                  : "memory");
 }
 __device__ __forceinline__ void kt_st16(uint32_t t, const uint32_t (&v)[16]) {
@@ -123,7 +124,7 @@ __global__ void __launch_bounds__(KT_THREADS, 1) kqt_kernel(const __grid_constan
     __shared__ __align__(16) float ysr[8][KT_NT];    // activation scales, eight superblocks deep
     __shared__ short chunk_e[KT_MAXCHUNK], chunk_n[KT_MAXCHUNK];
     __shared__ uint32_t tmem_sh;
-    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, nsb = a.nsb;
+    const int tid = threadIdx.x, warp = __shfl_sync(0xffffffffu, tid >> 5, 0), lane = tid & 31, nsb = a.nsb;
     if (tid == 0) {
         for (int i = 0; i < KT_RAW_DEPTH; i++) { mbar_init(&rfull[i], 1); mbar_init(&rempty[i], 8); }
         for (int i = 0; i < KT_B_DEPTH; i++) mbar_init(&bfull[i], 1);
@@ -145,7 +146,7 @@ __global__ void __launch_bounds__(KT_THREADS, 1) kqt_kernel(const __grid_constan
     __syncthreads();
     tl_fence_after();
     pdl_trigger();
-    const uint32_t tmem = tmem_sh;
+    const uint32_t tmem = __shfl_sync(0xffffffffu, tmem_sh, 0);
     const int ntask = nchunk * a.tiles;
     TlWaiter wait{a.state ? &a.state->err : nullptr, a.state && *reinterpret_cast<volatile uint32_t *>(&a.state->err) != 0u};
     auto task = [&](int t) {
@@ -215,6 +216,7 @@ __global__ void __launch_bounds__(KT_THREADS, 1) kqt_kernel(const __grid_constan
         }
     } else if (warp == 16) {
         // ---------------- products (the whole warp walks the loop, an elected lane issues)
+        const uint32_t issue = elect_one() ? 1u : 0u;
         int n = 0, ca = 0;
         for (int t = blockIdx.x; t < ntask; t += gridDim.x) {
             const KtTask k = task(t);
@@ -234,13 +236,11 @@ __global__ void __launch_bounds__(KT_THREADS, 1) kqt_kernel(const __grid_constan
                     for (int g = 0; g < 2; g++) {
                         wait(&afull[g][ab], (ca >> 1) & 1);
                         tl_fence_after();
-                        if (elect_one()) {
 #pragma unroll
-                            for (int s = 0; s < 8; s++) kt_mma(d + g * 32, tmem + KT_COL_A + (g * 2 + ab) * 64 + s * 8, db + (g * 8 + s) * 2 * cap, idesc, s > 0);
-                            if (g == 1) kt_mma(d + 64, tmem + KT_COL_MIN + ab * 8, db + 32 * cap, idesc, 0);
-                            tl_commit(g == 0 ? &half0[n & 3] : &done[n & 3]);
-                            if (g == 1) mbar_arrive(&done[n & 3]);      // orders drow and ysr, seen through afull and bfull, before the readers
-                        }
+                        for (int s = 0; s < 8; s++) kt_mma(issue, d + g * 32, tmem + KT_COL_A + (g * 2 + ab) * 64 + s * 8, db + (g * 8 + s) * 2 * cap, idesc, s > 0);
+                        if (g == 1) kt_mma(issue, d + 64, tmem + KT_COL_MIN + ab * 8, db + 32 * cap, idesc, 0);
+                        tl_commit_if(issue, g == 0 ? &half0[n & 3] : &done[n & 3]);
+                        if (g == 1) mbar_arrive_if(issue, &done[n & 3]);      // orders drow and ysr, seen through afull and bfull, before the readers
                         __syncwarp();
                     }
                     ca++;
@@ -250,15 +250,13 @@ __global__ void __launch_bounds__(KT_THREADS, 1) kqt_kernel(const __grid_constan
 #pragma unroll
                         for (int dig = 0; dig < 2; dig++) wait(&afull[g][(ca + dig) & 1], ((ca + dig) >> 1) & 1);
                         tl_fence_after();
-                        if (elect_one()) {
 #pragma unroll
-                            for (int dig = 0; dig < 2; dig++)
+                        for (int dig = 0; dig < 2; dig++)
 #pragma unroll
-                                for (int s = 0; s < 8; s++)
-                                    kt_mma(d + dig * 32, tmem + KT_COL_A + (g * 2 + ((ca + dig) & 1)) * 64 + s * 8, db + (g * 8 + s) * 2 * cap, idesc, g > 0 || s > 0);
-                            tl_commit(g == 0 ? &half0[n & 3] : &done[n & 3]);
-                            if (g == 1) mbar_arrive(&done[n & 3]);
-                        }
+                            for (int s = 0; s < 8; s++)
+                                kt_mma(issue, d + dig * 32, tmem + KT_COL_A + (g * 2 + ((ca + dig) & 1)) * 64 + s * 8, db + (g * 8 + s) * 2 * cap, idesc, g > 0 || s > 0);
+                        tl_commit_if(issue, g == 0 ? &half0[n & 3] : &done[n & 3]);
+                        if (g == 1) mbar_arrive_if(issue, &done[n & 3]);
                         __syncwarp();
                     }
                     ca += 2;
