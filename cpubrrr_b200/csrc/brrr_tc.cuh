@@ -58,6 +58,41 @@ __device__ __forceinline__ void tl_ld8x2(uint32_t ta, uint32_t tb, f32x2 (&v)[4]
                  : "r"(ta), "r"(tb)
                  : "memory");
 }
+// four chains (`step` columns apart) x two blocks (8 apart): the first two or four columns of each, v[2 chain + block]
+__device__ __forceinline__ void tl_ld_blocks(uint32_t ta, uint32_t step, f32x2 (&v)[8][1]) {
+    asm volatile("{\n\t.reg .b32 r0_<2>;\n\t.reg .b32 r1_<2>;\n\t.reg .b32 r2_<2>;\n\t.reg .b32 r3_<2>;\n\t.reg .b32 r4_<2>;\n\t.reg .b32 r5_<2>;\n\t.reg .b32 r6_<2>;\n\t.reg .b32 r7_<2>;\n\t"
+                 "tcgen05.ld.sync.aligned.32x32b.x2.b32 {r0_0,r0_1}, [%8];\n\t"
+                 "tcgen05.ld.sync.aligned.32x32b.x2.b32 {r1_0,r1_1}, [%9];\n\t"
+                 "tcgen05.ld.sync.aligned.32x32b.x2.b32 {r2_0,r2_1}, [%10];\n\t"
+                 "tcgen05.ld.sync.aligned.32x32b.x2.b32 {r3_0,r3_1}, [%11];\n\t"
+                 "tcgen05.ld.sync.aligned.32x32b.x2.b32 {r4_0,r4_1}, [%12];\n\t"
+                 "tcgen05.ld.sync.aligned.32x32b.x2.b32 {r5_0,r5_1}, [%13];\n\t"
+                 "tcgen05.ld.sync.aligned.32x32b.x2.b32 {r6_0,r6_1}, [%14];\n\t"
+                 "tcgen05.ld.sync.aligned.32x32b.x2.b32 {r7_0,r7_1}, [%15];\n\t"
+                 "tcgen05.wait::ld.sync.aligned;\n\t"
+                 "mov.b64 %0, {r0_0,r0_1};\n\tmov.b64 %1, {r1_0,r1_1};\n\tmov.b64 %2, {r2_0,r2_1};\n\tmov.b64 %3, {r3_0,r3_1};\n\tmov.b64 %4, {r4_0,r4_1};\n\tmov.b64 %5, {r5_0,r5_1};\n\tmov.b64 %6, {r6_0,r6_1};\n\tmov.b64 %7, {r7_0,r7_1};\n\t"
+                 "}"
+                 : "=l"(v[0][0]), "=l"(v[1][0]), "=l"(v[2][0]), "=l"(v[3][0]), "=l"(v[4][0]), "=l"(v[5][0]), "=l"(v[6][0]), "=l"(v[7][0])
+                 : "r"(ta + 0 * step + 0), "r"(ta + 0 * step + 8), "r"(ta + 1 * step + 0), "r"(ta + 1 * step + 8), "r"(ta + 2 * step + 0), "r"(ta + 2 * step + 8), "r"(ta + 3 * step + 0), "r"(ta + 3 * step + 8)
+                 : "memory");
+}
+__device__ __forceinline__ void tl_ld_blocks(uint32_t ta, uint32_t step, f32x2 (&v)[8][2]) {
+    asm volatile("{\n\t.reg .b32 r0_<4>;\n\t.reg .b32 r1_<4>;\n\t.reg .b32 r2_<4>;\n\t.reg .b32 r3_<4>;\n\t.reg .b32 r4_<4>;\n\t.reg .b32 r5_<4>;\n\t.reg .b32 r6_<4>;\n\t.reg .b32 r7_<4>;\n\t"
+                 "tcgen05.ld.sync.aligned.32x32b.x4.b32 {r0_0,r0_1,r0_2,r0_3}, [%16];\n\t"
+                 "tcgen05.ld.sync.aligned.32x32b.x4.b32 {r1_0,r1_1,r1_2,r1_3}, [%17];\n\t"
+                 "tcgen05.ld.sync.aligned.32x32b.x4.b32 {r2_0,r2_1,r2_2,r2_3}, [%18];\n\t"
+                 "tcgen05.ld.sync.aligned.32x32b.x4.b32 {r3_0,r3_1,r3_2,r3_3}, [%19];\n\t"
+                 "tcgen05.ld.sync.aligned.32x32b.x4.b32 {r4_0,r4_1,r4_2,r4_3}, [%20];\n\t"
+                 "tcgen05.ld.sync.aligned.32x32b.x4.b32 {r5_0,r5_1,r5_2,r5_3}, [%21];\n\t"
+                 "tcgen05.ld.sync.aligned.32x32b.x4.b32 {r6_0,r6_1,r6_2,r6_3}, [%22];\n\t"
+                 "tcgen05.ld.sync.aligned.32x32b.x4.b32 {r7_0,r7_1,r7_2,r7_3}, [%23];\n\t"
+                 "tcgen05.wait::ld.sync.aligned;\n\t"
+                 "mov.b64 %0, {r0_0,r0_1};\n\tmov.b64 %1, {r0_2,r0_3};\n\tmov.b64 %2, {r1_0,r1_1};\n\tmov.b64 %3, {r1_2,r1_3};\n\tmov.b64 %4, {r2_0,r2_1};\n\tmov.b64 %5, {r2_2,r2_3};\n\tmov.b64 %6, {r3_0,r3_1};\n\tmov.b64 %7, {r3_2,r3_3};\n\tmov.b64 %8, {r4_0,r4_1};\n\tmov.b64 %9, {r4_2,r4_3};\n\tmov.b64 %10, {r5_0,r5_1};\n\tmov.b64 %11, {r5_2,r5_3};\n\tmov.b64 %12, {r6_0,r6_1};\n\tmov.b64 %13, {r6_2,r6_3};\n\tmov.b64 %14, {r7_0,r7_1};\n\tmov.b64 %15, {r7_2,r7_3};\n\t"
+                 "}"
+                 : "=l"(v[0][0]), "=l"(v[0][1]), "=l"(v[1][0]), "=l"(v[1][1]), "=l"(v[2][0]), "=l"(v[2][1]), "=l"(v[3][0]), "=l"(v[3][1]), "=l"(v[4][0]), "=l"(v[4][1]), "=l"(v[5][0]), "=l"(v[5][1]), "=l"(v[6][0]), "=l"(v[6][1]), "=l"(v[7][0]), "=l"(v[7][1])
+                 : "r"(ta + 0 * step + 0), "r"(ta + 0 * step + 8), "r"(ta + 1 * step + 0), "r"(ta + 1 * step + 8), "r"(ta + 2 * step + 0), "r"(ta + 2 * step + 8), "r"(ta + 3 * step + 0), "r"(ta + 3 * step + 8)
+                 : "memory");
+}
 __device__ __forceinline__ f32x2 tl_pack2(uint32_t lo, uint32_t hi) {
     f32x2 r;
     asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "r"(lo), "r"(hi));

@@ -31,6 +31,7 @@
 // operands have landed; empty[slot] the products have read them; dfull[buf] the pair's products are complete; dempty[buf]
 // every live worker warp has read them; scbar the rows' scales of all pairs have landed.
 #include <cuda.h>
+#include <type_traits>
 #include "brrr_kernels.h"
 #include "brrr_block.cuh"
 #include "brrr_tma.cuh"
@@ -103,7 +104,7 @@ size_t tl_smem(int np) {
            (size_t)np * 2 * NT * 4 + (KIND == TK_GLU ? NT * 128 * 4 : 0);
 }
 
-template <int KIND, int NT>
+template <int KIND, int NT, bool FEW = false>
 __global__ void __launch_bounds__(NT * 16 + 128, KIND == TK_Q8 || NT == 32 ? 1 : NT == 16 ? 2 : 3) tile_kernel(const __grid_constant__ TileArgs a) {
     constexpr int WORKERS = NT * 16, THREADS = WORKERS + 128;
     constexpr int TL_DEPTH = tl_depth<KIND, NT>(), SLOT = tl_slot_bytes<KIND, NT>(), A_BYTES = tl_a_bytes<KIND>(), B_OFF = A_BYTES, SC = tl_sc_bytes<KIND>();
@@ -381,11 +382,56 @@ __global__ void __launch_bounds__(NT * 16 + 128, KIND == TK_Q8 || NT == 32 ? 1 :
             }
             xs_addr += 2 * NT * 4;
         };
+        // A CTA of eight tokens often has one or two (a short prompt or a small batch meets most experts with a row each): then only their
+        // columns are read and their chains carried.
+        auto few_step = [&](auto pairs, int buf) {
+            constexpr int TP = decltype(pairs)::value;
+            uint32_t e2;
+            asm volatile("ld.shared.u16 %0, [%1];" : "=r"(e2) : "r"(sc_addr));
+            const uint32_t w0 = __float_as_uint(tbl[e2 & 0xFFu]), w1 = __float_as_uint(tbl[e2 >> 8]);
+            sc_addr += SC;
+            f32x2 s2[2][TP], v[8][TP];
+#pragma unroll
+            for (int q = 0; q < 2; q++) {
+                if (TP == 2) lds_pairs(xs_addr + q * NT * 4, s2[q][0], s2[q][TP - 1]);
+                else {
+                    const uint2 x = lds64(xs_addr + q * NT * 4);
+                    s2[q][0] = tl_pack2(x.x, x.y);
+                }
+#pragma unroll
+                for (int i = 0; i < TP; i++) s2[q][i] = tl_mul2(q ? tl_pack2(w1, w1) : tl_pack2(w0, w0), s2[q][i]);
+            }
+            xs_addr += 2 * NT * 4;
+            wait(&dfull[buf], par);
+            tl_fence_after();
+            tl_ld_blocks(lane_addr + buf * BUF_COLS, 2 * NT, v);
+            tl_fence_before();
+            __syncwarp();
+            if (lane == 0) mbar_arrive(&dempty[buf]);
+#pragma unroll
+            for (int q = 0; q < 2; q++)
+#pragma unroll
+                for (int j = 0; j < 4; j++)
+#pragma unroll
+                    for (int i = 0; i < TP; i++) acc[j][i] = tl_fma2(v[2 * j + q][i], s2[q][i], acc[j][i]);
+        };
+        auto few = [&](auto pairs) {
 #pragma unroll 1
-        for (int p = 0; p < np; p += 2) {
-            pair_step(0);
-            if (p + 1 < np) pair_step(1);
-            par ^= 1u;
+            for (int p = 0; p < np; p += 2) {
+                few_step(pairs, 0);
+                if (p + 1 < np) few_step(pairs, 1);
+                par ^= 1u;
+            }
+        };
+        if (FEW && n_ent <= 2) few(std::integral_constant<int, 1>{});
+        else if (FEW && n_ent <= 4) few(std::integral_constant<int, 2>{});
+        else {
+#pragma unroll 1
+            for (int p = 0; p < np; p += 2) {
+                pair_step(0);
+                if (p + 1 < np) pair_step(1);
+                par ^= 1u;
+            }
         }
         // ---------------- outputs
         const int row_local = KIND == TK_GLU ? tile * 64 + (m & 63) : tile * TL_ROWS + m - shift;
@@ -545,6 +591,15 @@ cudaError_t tl_launch(TileArgs a, int tiles, int entries, int experts, bool pdl,
     if (nt == 16) {
         if ((ce = smem_optin(tile_kernel<KIND, 16>, 220 * 1024, configured[1])) != cudaSuccess) return ce;
         return launch_k(tile_kernel<KIND, 16>, grid, dim3(16 * 16 + 128), tl_smem<KIND, 16>(a.np), st, pdl, a);
+    }
+    // up to three entries per expert on average: the variant that carries one or two pairs of tokens where that is all a CTA has (a kernel of its own:
+    // the general loop loses 7 % beside the others).  gate | up and down of the 20b shape, us, without and with: 3 rows 36 + 29, 30 + 24; 9 rows
+    // 73 + 50, 67 + 44; 16 rows 84 + 50, 76 + 49; 24 rows 93 + 57, 87 + 55; 30 rows 93 + 57, 94 + 59
+    constexpr bool MX = KIND != TK_Q8;
+    static unsigned long long configured_few = 0;
+    if (MX && a.cnt && avg <= 3) {
+        if ((ce = smem_optin(tile_kernel<KIND, 8, MX>, 220 * 1024, configured_few)) != cudaSuccess) return ce;
+        return launch_k(tile_kernel<KIND, 8, MX>, grid, dim3(256), tl_smem<KIND, 8>(a.np), st, pdl, a);
     }
     if ((ce = smem_optin(tile_kernel<KIND, 8>, 220 * 1024, configured[2])) != cudaSuccess) return ce;
     return launch_k(tile_kernel<KIND, 8>, grid, dim3(256), tl_smem<KIND, 8>(a.np), st, pdl, a);

@@ -104,3 +104,9 @@ def test_moe_ffn_tile_equals_token_by_token(brrr, dev, ntok):
     assert np.array_equal(bits(got_x.cpu().numpy()), bits(want_x.cpu().numpy()))
     assert len(np.unique(want_top.cpu().numpy())) > min(4, ntok)          # the tokens do not all share one expert set
     eng.close()
+
+
+@pytest.mark.parametrize("ntok", [2, 3, 8, 9, 23, 24, 25])
+def test_moe_ffn_tile_with_few_entries_per_expert(brrr, dev, ntok):
+    """Experts with one to a handful of entries: one pair, two pairs and whole groups of tokens, on either side of the line between the kernels."""
+    test_moe_ffn_tile_equals_token_by_token(brrr, dev, ntok)
