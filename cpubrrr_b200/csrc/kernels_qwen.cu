@@ -45,45 +45,51 @@ __global__ void __launch_bounds__(256) qw_embed_kernel(const uint8_t *__restrict
 }
 
 // ---------------------------------------------------------------- expert selection
-// sel[r] = expert of rank r of est[0 .. ne) (the larger first, the lower index among equals).  Block-wide over QG_THREADS (four threads count
-// the rank of an expert, a quarter of the others each); ends synchronised.  All in one warp - eight rounds of a maximum - it took 2.2 us.
-struct alignas(16) QSelect { uint32_t key[4 * 68]; };        // a quarter of the experts every per * 4 + 4 words: the four read different banks
-__device__ __forceinline__ void qw_select(const float *est, int ne, int topk, const DevState *state, QSelect &w, int *sel, int tid) {
+// The expert of rank r of est[0 .. ne) in lane r < topk (the larger first, the lower index among equals), by one warp without shared memory or
+// barriers: each warp that needs the experts picks them itself.  A lane holds PER consecutive experts; a turn is a maximum over the lane's
+// keys and one reduction over the warp, the index travels beside the next turn.  Ranking by four threads an expert, block-wide with three
+// barriers, gate/up had its experts 2400 cycles after its dependency wait and its copies out at 3700; 64 + 128 tokens of the 30b-a3b shape:
+// 209.2 ms before, 206.5 with the warps picking and the copies spread over them.
+template <int PER>
+__device__ __forceinline__ int qw_pick_from(const float *est, int ne, int topk, int lane) {
+    uint32_t key[PER];
+#pragma unroll
+    for (int i = 0; i < PER; i++) {
+        const int e = lane * PER + i;
+        key[i] = e < ne ? max(float_orderable(__ldcg(est + e)), 1u) : 0u;       // 0: absent or taken
+    }
+    int mine = 0;
+#pragma unroll 1
+    for (int r = 0; r < topk; r++) {
+        uint32_t m = key[0];
+#pragma unroll
+        for (int i = 1; i < PER; i++) m = max(m, key[i]);
+        const uint32_t best = __reduce_max_sync(0xffffffffu, m);
+        const int from = __ffs(__ballot_sync(0xffffffffu, m == best)) - 1;
+        int at = PER - 1;
+#pragma unroll
+        for (int i = PER - 2; i >= 0; i--) if (key[i] == best) at = i;
+        const int e = __shfl_sync(0xffffffffu, lane * PER + at, from);
+        if (lane == r) mine = e;
+#pragma unroll
+        for (int i = 0; i < PER; i++) if (lane == from && i == at) key[i] = 0u;
+    }
+    return mine;
+}
+__device__ __forceinline__ int qw_pick(const float *est, int ne, int topk, const DevState *state, int lane) {
+    const int e = ne <= 128 ? qw_pick_from<4>(est, ne, topk, lane) : qw_pick_from<8>(est, ne, topk, lane);      // ne <= 256
 #ifdef BRRR_TEST_HOOKS
-    const bool spoil = state && (state->test_hooks & 1u) && state->pos % 3 == 0;
+    if (state && (state->test_hooks & 1u) && state->pos % 3 == 0 && lane == topk - 1) return (e + 1) % ne;
 #else
-    constexpr bool spoil = false;
     (void)state;
 #endif
-    const int per = (ne + 15) / 16, stride = per * 4 + 4;        // groups of four experts per quarter
-    if (tid < 4 * per * 4) w.key[tid / (per * 4) * 4 + tid] = tid < ne ? max(float_orderable(__ldcg(est + tid)), 1u) : 0u;
-    if (tid >= 256 && tid < 264) sel[tid - 256] = 0;
-    __syncthreads();
-#pragma unroll 1
-    for (int e0 = 0; e0 < ne; e0 += QG_THREADS / 4) {
-        const int e = e0 + (tid >> 2), ec = min(e, ne - 1);
-        const int at = ec / (per * 4) * 4 + ec, quarter = tid & 3;
-        const uint32_t key = w.key[at];
-        const uint4 *others = reinterpret_cast<const uint4 *>(w.key + quarter * stride);
-        int r = 0;
-#pragma unroll 4
-        for (int o = 0; o < per; o++) {          // among equals the lower index comes first; those of its own group: below
-            const uint4 u = others[o];
-            const uint32_t t = quarter * per + o < (ec >> 2) ? key - 1 : key;
-            r += (u.x > t) + (u.y > t) + (u.z > t) + (u.w > t);
-        }
-        if (quarter < (ec & 3)) r += w.key[at - (ec & 3) + quarter] == key;
-        r += __shfl_xor_sync(0xffffffffu, r, 1);
-        r += __shfl_xor_sync(0xffffffffu, r, 2);
-        if (!(tid & 3) && e < ne && tid < QG_THREADS && r < topk) sel[r] = (spoil && r == topk - 1) ? (e + 1) % ne : e;
-    }
-    __syncthreads();
+    return e;
 }
 
 // The exact routing a step's combine uses, by one warp: slot_of[k] = slot (rank of the estimate) of the expert of rank k, wts[k] its weight.
 // est: the words of the step's seq-th publication by the router, awaited with a bound (the router does not depend on any kernel that waits
-// here, and the waiting kernels leave it room on an SM); sel: the estimate's experts.  Else top and weights as they are.
-__device__ __forceinline__ void qw_routing(bool est, const int *sel, const int32_t *top, const float *weights, int topk, uint32_t seq, DevState *state, int *slot_of, float *wts,
+// here, and the waiting kernels leave it room on an SM); picked: the estimate's expert of slot `lane`.  Else top and weights as they are.
+__device__ __forceinline__ void qw_routing(bool est, int picked, const int32_t *top, const float *weights, int topk, uint32_t seq, DevState *state, int *slot_of, float *wts,
                                            int lane) {
     uint32_t payload = 0u;
     if (lane < 16 && (lane & 7) < topk) {
@@ -106,11 +112,12 @@ __device__ __forceinline__ void qw_routing(bool est, const int *sel, const int32
         } else payload = lane < 8 ? (uint32_t)__ldcg(top + lane) : __float_as_uint(__ldcg(weights + (lane - 8)));
     }
     if (lane >= 8 && lane < 8 + topk) wts[lane - 8] = __uint_as_float(payload);
+    int found = -1;
+    for (int s = 0; s < topk; s++) if (__shfl_sync(0xffffffffu, picked, s) == (int)payload) found = s;
     if (lane < topk) {
         int slot = lane;
         if (est) {
-            slot = -1;
-            for (int s = 0; s < topk; s++) if (sel[s] == (int)payload) slot = s;
+            slot = found;
             if (slot < 0) { slot = 0; atomicMin(&state->spec_fail_step, state->n_out); }      // the estimate missed this expert
         }
         slot_of[lane] = slot;
@@ -611,40 +618,42 @@ template <int G, int U> struct KPair { static constexpr int gate = G, up = U; };
 template <int PASSES>
 __global__ void __launch_bounds__(QG_THREADS, 2) qw_gate_up_kernel(const __grid_constant__ QGateUpArgs a) {
     extern __shared__ __align__(16) unsigned char qsm[];
-    __shared__ QSelect ws;
-    __shared__ int sel[8];
     __shared__ __align__(8) uint64_t bar[16];
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, nsb = a.gate.cols / 256;
     const int i0 = blockIdx.x * a.per_cta, n = min(a.per_cta, a.topk * a.ff - i0), groups = (n + QG_WARPS - 1) / QG_WARPS;
     unsigned char *rg = qsm, *ru = qsm + (size_t)a.per_cta * a.stride_g;
     float *terms = reinterpret_cast<float *>(ru + (size_t)a.per_cta * a.stride_u);      // [row][gate, up][nsb]
     Waiter waiter(a.state ? &a.state->err : nullptr);
-    if (tid < 4 * groups && !(tid & 3)) {
-        mbar_init(&bar[tid >> 2], 1);
+    // copy = (group, matrix, first or second run: a group of sixteen pairs touches two slots at most), at most four per warp: a copy
+    // costs the warp that issues it about 100 cycles, so they are spread over the warps
+    const int copy = warp + QG_WARPS * lane, grp = copy >> 2;
+    if (copy < 4 * groups && !(copy & 3)) {
+        mbar_init(&bar[grp], 1);
         mbar_fence_init();
     }
-    // thread = (group, matrix, first or second run: a group of sixteen pairs touches two slots at most)
-    int run = 0, slot = 0, grp = tid >> 2;
+    int run = 0, slot = 0;
     uint32_t bytes = 0, expert_bytes = 0;
     const uint8_t *src = nullptr;
     unsigned char *dst = nullptr;
-    if (tid < 4 * groups) {
-        const int up = (tid >> 1) & 1, r0 = grp * QG_WARPS, cnt = min(QG_WARPS, n - r0), stride = up ? a.stride_u : a.stride_g;
+    if (copy < 4 * groups) {
+        const int up = (copy >> 1) & 1, r0 = grp * QG_WARPS, cnt = min(QG_WARPS, n - r0), stride = up ? a.stride_u : a.stride_g;
         int it = i0 + r0, r = r0;
         slot = it / a.ff;
         run = min(cnt, (slot + 1) * a.ff - it);
-        if (tid & 1) { r += run; it += run; run = cnt - run; slot++; }
+        if (copy & 1) { r += run; it += run; run = cnt - run; slot++; }
         dst = (up ? ru : rg) + (size_t)r * stride;
         src = (up ? a.up.p : a.gate.p) + (size_t)(it - slot * a.ff) * stride;
         bytes = (uint32_t)run * stride;
         expert_bytes = (uint32_t)a.ff * stride;
-        if ((tid & 3) == 0) mbar_expect_tx(&bar[grp], (uint32_t)cnt * (uint32_t)(a.stride_g + a.stride_u));
+        if ((copy & 3) == 0) mbar_expect_tx(&bar[grp], (uint32_t)cnt * (uint32_t)(a.stride_g + a.stride_u));
     }
     pdl_wait_cta();
-    if (a.est) qw_select(a.est, a.ne, a.topk, a.state, ws, sel, tid);
-    else { if (tid < a.topk) sel[tid] = a.top[tid]; __syncthreads(); }
-    if (tid < 4 * groups && run > 0) bulk_g2s(dst, src + (size_t)sel[slot] * expert_bytes, bytes, &bar[grp]);
-    pdl_trigger();           // only now: the down projection fetches its rows at once, and these come first
+    if (__any_sync(0xffffffffu, run > 0)) {
+        const int e = a.est ? qw_pick(a.est, a.ne, a.topk, a.state, lane) : a.top[min(lane, a.topk - 1)];
+        const int mine = __shfl_sync(0xffffffffu, e, slot);
+        if (run > 0) bulk_g2s(dst, src + (size_t)mine * expert_bytes, bytes, &bar[grp]);
+        if (warp == 0) pdl_trigger();           // only now (warp 0 always has a copy): the down projection fetches its rows at once, and these come first
+    }
     waiter.poison_if_failed();
     // the activation from global memory (L1 after the first warp)
     const uint32_t rg0 = smem_u32(rg), ru0 = smem_u32(ru);
@@ -709,8 +718,7 @@ __device__ __forceinline__ void qw_down_rows(const QDownArgs &a, uint32_t rows, 
 
 __global__ void __launch_bounds__(QD_THREADS, 2) qw_down_kernel(const __grid_constant__ QDownArgs a) {
     extern __shared__ __align__(16) unsigned char qsm[];
-    __shared__ QSelect ws;
-    __shared__ int sel[8], slot_of[8];
+    __shared__ int slot_of[8];
     __shared__ float wts[8];
     __shared__ __align__(8) uint64_t bar;
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
@@ -722,8 +730,8 @@ __global__ void __launch_bounds__(QD_THREADS, 2) qw_down_kernel(const __grid_con
     float *terms = reinterpret_cast<float *>(b16 + nun * 16);          // [row][slot][nsb]
     float *dots = terms + (size_t)a.per_cta * nun;                     // [slot][row]
     Waiter waiter(a.state ? &a.state->err : nullptr);
-    if (a.est) qw_select(a.est, a.ne, a.topk, a.state, ws, sel, tid);
-    else { if (tid < a.topk) sel[tid] = a.top[tid]; __syncthreads(); }
+    int picked = 0;              // warp 0 (the copies) and the last (the routing): the expert of slot `lane`
+    if (warp == 0 || warp == QG_WARPS) picked = a.est ? qw_pick(a.est, a.ne, a.topk, a.state, lane) : a.top[min(lane, a.topk - 1)];
     if (warp == 0) {
         if (lane == 0) {
             mbar_init(&bar, 1);
@@ -731,12 +739,12 @@ __global__ void __launch_bounds__(QD_THREADS, 2) qw_down_kernel(const __grid_con
             mbar_expect_tx(&bar, (uint32_t)a.topk * n * rb);
         }
         __syncwarp();
-        if (lane < a.topk) bulk_g2s(rows + (size_t)lane * a.per_cta * rb, a.down.p + ((size_t)sel[lane] * a.d + r0) * rb, (uint32_t)n * rb, &bar);
+        if (lane < a.topk) bulk_g2s(rows + (size_t)lane * a.per_cta * rb, a.down.p + ((size_t)picked * a.d + r0) * rb, (uint32_t)n * rb, &bar);
     }
     float xr = tid < n ? a.x[r0 + tid] : 0.0f;                         // written several kernels back
     pdl_wait_cta();      // h is complete
     pdl_trigger();
-    if (warp == QG_WARPS) qw_routing(a.est != nullptr, sel, a.top, a.wts, a.topk, a.seq, a.state, slot_of, wts, lane);
+    if (warp == QG_WARPS) qw_routing(a.est != nullptr, picked, a.top, a.wts, a.topk, a.seq, a.state, slot_of, wts, lane);
     else {
         for (int sb = warp; sb < nun; sb += QG_WARPS) {
             float v[8];

@@ -89,6 +89,20 @@ def test_qwen_rows_wider_than_eight_superblocks(brrr, orc, shape):
     eng.close(); om.close()
 
 
+@pytest.mark.parametrize("ne,topk", [(1, 1), (8, 8), (33, 5), (128, 8), (129, 8), (256, 8)])
+def test_qwen_picks_of_the_estimate(brrr, orc, ne, topk):
+    """Expert counts at the edges of the selection (four experts a lane up to 128, eight above): the estimate's picks are the router's, so
+    no step is run again, and the tokens are the oracle's.  With ff = 256 and eight slots a CTA's rows meet several slots."""
+    cfg = brrr.make_qwen_cfg(256, 2, 2, 1, ne, topk, 256, 512)
+    eng = brrr.QwenEngine.synth(cfg, 43)
+    om = orc.QwenModel.synth(ocfg_of(orc, cfg), 43)
+    prompt = S.synth_prompt(43, 5, cfg.n_vocab)
+    want = greedy(om.run, prompt, 24)
+    assert greedy(eng.run, prompt, 24) == want
+    assert eng.spec_redos() == 0
+    eng.close()
+
+
 def test_qwen_layer_trace_bit_exact(brrr, orc):
     cfg = brrr.make_qwen_cfg(512, 4, 4, 2, 16, 4, 256, 772)
     eng = brrr.QwenEngine.synth(cfg, 5)
