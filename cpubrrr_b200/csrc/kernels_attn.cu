@@ -427,9 +427,9 @@ __device__ __forceinline__ float ar_score(const f32x2 (&q)[HD / 2], const float 
 __global__ void __launch_bounds__(AR_THREADS, 2) attn_rows_kernel(AttnRowsArgs a) {
     constexpr int HALF = AR_THREADS / 2;                           // pass 2: threads of the sums, and of the probabilities
     extern __shared__ __align__(128) unsigned char smraw[];
-    float *ktile = reinterpret_cast<float *>(smraw);                                    // [2][128][64]
-    float *vtile = reinterpret_cast<float *>(smraw + 2 * AR_TILE_BYTES);                // [2][128][64]
-    float *psm = reinterpret_cast<float *>(smraw + 4 * AR_TILE_BYTES);                  // [2][128 keys][pairs]
+    float *ktile = reinterpret_cast<float *>(smraw);                                    // [2][AR_TILE][64]
+    float *vtile = reinterpret_cast<float *>(smraw + 2 * AR_TILE_BYTES);                // [2][AR_TILE][64]
+    float *psm = reinterpret_cast<float *>(smraw + 4 * AR_TILE_BYTES);                  // [2][AR_TILE keys][pairs]
     float *qsm = psm + 2 * AR_TILE * AR_PAIRS;                                             // [pairs][64]: q, then the outputs
     __shared__ __align__(8) uint64_t kbar[2], vbar[2];
     __shared__ float red[AR_THREADS / 32][AR_PAIRS];
