@@ -5,8 +5,8 @@
 --hooks also builds libbrrr_hooks.so: the same sources with -DBRRR_TEST_HOOKS, which compiles in what
 only tests and timeline measurements use (a way to spoil the routing estimate, a way to silence the
 router's publication, a bound on a model's device memory, in-kernel clock stamps, and the entry points
-that read the stamps, the memory taken and the room rule of the qwen3moe step).  The default
-library contains none of it.
+that read the stamps, the memory taken, the form of the expert matrices and the room rule of the
+qwen3moe step).  The default library contains none of it.
 
 The library is built in-tree so that it travels with the source tree.  nvcc cross-compiles
 without a GPU.  -fmad=false: kernels fuse multiply-adds only where written explicitly, which

@@ -138,11 +138,12 @@ struct EpCtx {
 // ---- single-token expert matvecs on the tensor cores in native fp4 (kernels_mxt.cu)
 // Tile units: [expert][tile of 128 rows][two block pairs][4096 B operand image per pair | 128 x 4 e8m0 bytes].
 constexpr int MXT_PAIR = 4096, MXT_SCALES = 512;
-// block exponents whose products with any activation scale are exact (kernels_mxt.cu)
-constexpr int XT_EXP_MIN = 49, XT_EXP_MAX = 190;
+// block exponents whose products with any activation scale, 1e-12 / 127 to FLT_MAX / 127, are exact (kernels_mxt.cu)
+constexpr int XT_EXP_MIN = 49, XT_EXP_MAX = 134;
 struct MxtDev {
     uint8_t *data;
     int tiles_per_expert, np;
+    bool wide;               // a block exponent lies outside that range: scales in the epilogue
 };
 size_t mxt_bytes(int experts, int tiles_per_expert, int np);
 // b.data == nullptr: tiles of 128 rows of a (rows past the end are zero); else rows 0-63 of a tile

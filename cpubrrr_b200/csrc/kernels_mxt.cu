@@ -17,8 +17,11 @@
 //     64, 8 or 1 times its plane's partial sum, times 2^(e_b-128);
 //   * every sum is an integer of at most 14 bits times 2^(e_b-128), exact in the f32 accumulator, and so are the two additions that
 //     join the planes.  The product of that sum with xs[b] is the exact t_j 2^(e_b-128) xs[b] of the chain's definition whenever
-//     2^(e_b-128) xs[b] neither underflows nor overflows: xs >= 1e-12 / 127, so exponents XT_EXP_MIN .. XT_EXP_MAX qualify
-//     (launch_mx_exp_scan; a model with others keeps the integer-unit kernels).
+//     2^(e_b-128) xs[b] neither underflows nor overflows: 1e-12 / 127 <= xs <= FLT_MAX / 127, so exponents XT_EXP_MIN .. XT_EXP_MAX qualify.
+// Matrices with other exponents (launch_mx_exp_scan; MxtDev.wide) run the same kernels in their WIDE form: every product is formed with one constant
+// row scale, column t then holds 64, 8 or 1 times its plane's partial sum, and the epilogue multiplies with the chain's own fl(2^(e_b-128) xs[b])
+// from the exponent bytes, as the definition states it.  A step of two layers of the 20b shape, position 140: 86 us scaled, 98 us with every matrix
+// wide, 116 us on the integer units.
 // The eight epilogue warps read the accumulator columns of their rows from tensor memory
 // (tcgen05.ld) and run the float chains, a thread for two chains of a row.
 //
@@ -80,7 +83,7 @@ struct PackArgs {
     MxDev a, b;              // b.data == nullptr: one matrix, 128 rows per tile; else rows 0-63 from a, 64-127 from b
     int rows_per_expert;     // logical rows of one expert in a (and b)
     int tiles_per_expert;
-    MxtDev out;
+    MxtDev out;              // out.wide: exponent bytes as they are
 };
 
 __global__ void mxt_pack_kernel(PackArgs p, size_t total_words) {
@@ -113,7 +116,7 @@ __global__ void mxt_pack_kernel(PackArgs p, size_t total_words) {
             const uint8_t *u = (k >> 1) < here ? locate(m, pair0 + (k >> 1), rl) : nullptr;
             if (u) {
                 ex = u[MX_UNIT_EXPS + rl * 2 + (k & 1)];
-                if (ex < (uint32_t)XT_EXP_MIN) ex = 0x7Fu;      // all-zero blocks only (launch_mx_exp_scan): any finite scale gives the same sums
+                if (!p.out.wide && ex < (uint32_t)XT_EXP_MIN) ex = 0x7Fu;      // all-zero blocks only (launch_mx_exp_scan): any finite scale gives the same sums
             }
             v |= ex << (8 * k);
         }
@@ -254,12 +257,20 @@ struct XtShared {
 
 // One block pair of one row: two chains' scaled lane dots of its two blocks from the three digit planes, then their fused multiply-adds,
 // in block order.  Both chains share an instruction (two independent round-to-nearest operations).
-__device__ __forceinline__ void xt_pair(const f32x2 *v, f32x2 xs0, f32x2 xs1, f32x2 &acc) {
+// ex (wide matrices): the row's exponent bytes of the two blocks in the low half; else the products carry them.
+template <bool WIDE>
+__device__ __forceinline__ void xt_pair(const f32x2 *v, f32x2 xs0, f32x2 xs1, uint32_t ex, f32x2 &acc) {
+    if (WIDE) {
+        const uint32_t s0 = __float_as_uint(brrr_e8m0_scale(ex & 0xFFu)), s1 = __float_as_uint(brrr_e8m0_scale((ex >> 8) & 0xFFu));
+        xs0 = tl_mul2(tl_pack2(s0, s0), xs0);
+        xs1 = tl_mul2(tl_pack2(s1, s1), xs1);
+    }
     acc = tl_fma2(tl_add2(tl_add2(v[0], v[2]), v[4]), xs0, acc);
     acc = tl_fma2(tl_add2(tl_add2(v[1], v[3]), v[5]), xs1, acc);
 }
 
-template <bool DOWN, bool EP>
+// WIDE: block exponents outside the range of the scaled products (top of this file)
+template <bool DOWN, bool EP, bool WIDE>
 __global__ void __launch_bounds__(XT_THREADS, 2) xt_expert_kernel(XtArgs a) {
     extern __shared__ __align__(128) unsigned char smraw[];
     // the warp index as the compiler can see it: the same in every lane, so the roles' loops keep their values in uniform registers
@@ -306,7 +317,11 @@ __global__ void __launch_bounds__(XT_THREADS, 2) xt_expert_kernel(XtArgs a) {
     if (warp < 4) {
         // the columns' scales: lane n = column (plane (n % 12) / 4, block of the pair (n / 2) & 1), byte k = block k of the pair
         const uint32_t sc = lane < XT_N ? (134u - 3u * (uint32_t)((lane % 12) >> 2)) << (8 * ((lane >> 1) & 1)) : 0u;
-        asm volatile("tcgen05.st.sync.aligned.32x32b.x4.b32 [%0], {%1,%2,%2,%2};" ::"r"(tmem_base + ((uint32_t)(warp * 32) << 16) + XT_SFB_COL), "r"(sc), "r"(0u) : "memory");
+        const uint32_t lanes = tmem_base + ((uint32_t)(warp * 32) << 16);
+        asm volatile("tcgen05.st.sync.aligned.32x32b.x4.b32 [%0], {%1,%2,%2,%2};" ::"r"(lanes + XT_SFB_COL), "r"(sc), "r"(0u) : "memory");
+        if (WIDE)      // 2 for every row and block: twice an e2m1 value is the doubled one
+            for (int k = 0; k < XT_REGIONS * XT_CH * 2; k += 4)
+                asm volatile("tcgen05.st.sync.aligned.32x32b.x4.b32 [%0], {%1,%1,%1,%1};" ::"r"(lanes + XT_SFA_COL + k), "r"(0x80808080u) : "memory");
         asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
     }
     xt_fence_before();
@@ -405,7 +420,7 @@ __global__ void __launch_bounds__(XT_THREADS, 2) xt_expert_kernel(XtArgs a) {
 #pragma unroll 1
                 for (int k = 0; k < cnt; k += 2) {
                     const uint32_t two = cnt - k > 1 ? issue : 0u;
-                    xt_cp_scales(issue, sfa + k * 2, dhi | (aaddr + (cnt - k > 1 ? 2 : 1) * (MXT_PAIR / 16)));
+                    if (!WIDE) xt_cp_scales(issue, sfa + k * 2, dhi | (aaddr + (cnt - k > 1 ? 2 : 1) * (MXT_PAIR / 16)));
                     xt_mma(issue, d0, alo | aaddr, blo | baddr1, XT_IDESC, sfa + k * 2, sfb);
                     xt_mma(two, d0 + XT_N, alo | (aaddr + MXT_PAIR / 16), blo | (baddr1 + XT_B_PAIR / 16), XT_IDESC | (2u << 29), sfa + k * 2, sfb);
                     d0 += 2 * XT_N; aaddr += XT_GROUP / 16; baddr1 += 2 * XT_B_PAIR / 16;
@@ -434,6 +449,12 @@ __global__ void __launch_bounds__(XT_THREADS, 2) xt_expert_kernel(XtArgs a) {
             f32x2 xs[2 * XT_CH], dv[XT_REGION_COLS / 4];
 #pragma unroll
             for (int k = 0; k < 2 * XT_CH; k += 2) lds_pairs(xaddr + k * 8, xs[k], xs[k + 1]);
+            uint32_t ex[XT_CH / 2] = {};
+            if (WIDE) {              // this row's word of each group's exponents (the word may be read before the round is through: weights do not change)
+#pragma unroll
+                for (int k = 0; k < XT_CH / 2; k++)
+                    if (2 * k < left) ex[k] = __ldg(reinterpret_cast<const uint32_t *>(src + (size_t)(r * (XT_CH / 2) + k) * XT_GROUP + min(2, left - 2 * k) * MXT_PAIR + (m & 31) * 16 + (m >> 5) * 4));
+            }
             xt_wait(&sh.dfull[reg], dpar, err);
             XT_ACC(tw_d);
             xt_fence_after();
@@ -444,7 +465,7 @@ __global__ void __launch_bounds__(XT_THREADS, 2) xt_expert_kernel(XtArgs a) {
             if (lane == 0) mbar_arrive(&sh.dempty[reg]);
 #pragma unroll
             for (int k = 0; k < XT_CH; k++)
-                if (k < left) xt_pair(dv + XT_N / 4 * k, xs[2 * k], xs[2 * k + 1], acc);
+                if (k < left) xt_pair<WIDE>(dv + XT_N / 4 * k, xs[2 * k], xs[2 * k + 1], ex[k / 2] >> (16 * (k & 1)), acc);
             xaddr += 2 * XT_CH * 8;
             left -= XT_CH;
             if (++reg == XT_REGIONS) { reg = 0; dpar ^= 1u; }
@@ -774,6 +795,21 @@ void launch_mx_exp_scan(const uint8_t *raw, size_t blocks, uint32_t *bad, cudaSt
     if (blocks) mx_exp_scan_kernel<<<148 * 8, 256, 0, st>>>(raw, blocks, bad);
 }
 
+// A down CTA has the footprint of a gate/up CTA: it fits beside a running one, sets up and starts its weight stream there, before gate/up has
+// finished (measured: 745 tok/s against 728 with a 9-stage ring that needs an SM of its own).
+template <bool DOWN, bool EP, bool WIDE>
+static cudaError_t xt_launch_form(const XtArgs &a, dim3 grid, bool pdl, cudaStream_t st) {
+    static unsigned long long configured = 0;      // one bit per device
+    const cudaError_t e = smem_optin(xt_expert_kernel<DOWN, EP, WIDE>, 200 * 1024, configured);
+    if (e != cudaSuccess) return e;
+    return launch_k(xt_expert_kernel<DOWN, EP, WIDE>, grid, dim3(XT_THREADS), xt_smem_bytes(a.w.np), st, pdl, a);
+}
+template <bool DOWN>
+static cudaError_t xt_launch(const XtArgs &a, dim3 grid, bool pdl, cudaStream_t st) {
+    if (a.w.wide) return a.ep_on ? xt_launch_form<DOWN, true, true>(a, grid, pdl, st) : xt_launch_form<DOWN, false, true>(a, grid, pdl, st);
+    return a.ep_on ? xt_launch_form<DOWN, true, false>(a, grid, pdl, st) : xt_launch_form<DOWN, false, false>(a, grid, pdl, st);
+}
+
 cudaError_t launch_gate_up_t(MxtDev gu, const float *gate_b, const float *up_b, const int32_t *top, const float *est, int ne, int topk,
                              int d, const uint8_t *xdig, const float *xs, int8_t *hq, float *hs, uint8_t *hdig, DevState *state,
                              bool pdl, cudaStream_t st, const EpCtx *ep, int layer) {
@@ -781,14 +817,7 @@ cudaError_t launch_gate_up_t(MxtDev gu, const float *gate_b, const float *up_b, 
     if (ep) { a.ep_on = 1; a.ep = *ep; a.layer = layer; }
     a.w = gu; a.bias_a = gate_b; a.bias_b = up_b; a.top = top; a.est = est; a.ne = ne; a.topk = topk; a.d = d;
     a.bdig = xdig; a.xs = xs; a.hq = hq; a.hs = hs; a.hdig = hdig; a.state = state;
-    static unsigned long long configured = 0, configured_ep = 0;      // one bit per device
-    {
-        cudaError_t e = smem_optin(xt_expert_kernel<false, false>, 200 * 1024, configured);
-        if (e == cudaSuccess) e = smem_optin(xt_expert_kernel<false, true>, 200 * 1024, configured_ep);
-        if (e != cudaSuccess) return e;
-    }
-    if (ep) return launch_k(xt_expert_kernel<false, true>, dim3(gu.tiles_per_expert, topk), dim3(XT_THREADS), xt_smem_bytes(gu.np), st, pdl, a);
-    return launch_k(xt_expert_kernel<false, false>, dim3(gu.tiles_per_expert, topk), dim3(XT_THREADS), xt_smem_bytes(gu.np), st, pdl, a);
+    return xt_launch<false>(a, dim3(gu.tiles_per_expert, topk), pdl, st);
 }
 
 cudaError_t launch_down_t(MxtDev down, const float *down_b, const int32_t *top, const float *wts, const float *est, int ne, int topk,
@@ -798,17 +827,7 @@ cudaError_t launch_down_t(MxtDev down, const float *down_b, const int32_t *top, 
     if (ep) { a.ep_on = 1; a.ep = *ep; a.layer = layer; }
     a.w = down; a.bias_a = down_b; a.top = top; a.wts = wts; a.est = est; a.ne = ne; a.topk = topk; a.d = d;
     a.bdig = hdig; a.xs = hs; a.x = x; a.part = part; a.counter = counter; a.state = state;
-    // the same footprint as a gate/up CTA: a down CTA fits beside a running gate/up CTA, sets up and
-    // starts its weight stream there, before gate/up has finished (measured: 745 tok/s against 728
-    // with a 9-stage ring that needs an SM of its own)
-    static unsigned long long configured = 0, configured_ep = 0;      // one bit per device
-    {
-        cudaError_t e = smem_optin(xt_expert_kernel<true, false>, 210 * 1024, configured);
-        if (e == cudaSuccess) e = smem_optin(xt_expert_kernel<true, true>, 210 * 1024, configured_ep);
-        if (e != cudaSuccess) return e;
-    }
-    if (ep) return launch_k(xt_expert_kernel<true, true>, dim3(down.tiles_per_expert, topk), dim3(XT_THREADS), xt_smem_bytes(down.np), st, pdl, a);
-    return launch_k(xt_expert_kernel<true, false>, dim3(down.tiles_per_expert, topk), dim3(XT_THREADS), xt_smem_bytes(down.np), st, pdl, a);
+    return xt_launch<true>(a, dim3(down.tiles_per_expert, topk), pdl, st);
 }
 
 cudaError_t launch_down_fold(const int32_t *top, const float *wts, const float *est, int ne, int topk, int d, const float *part,

@@ -145,7 +145,7 @@ struct brrr_model {
     float *dpart = nullptr;      // down: [topk][tiles * 128] row sums
     uint32_t *dcount = nullptr;  // down: arrival counters per row tile
     uint8_t *xdig = nullptr, *hdig = nullptr;   // digits of the token's and of h's Q8 activation (brrr_mxt.cuh)
-    uint32_t *exp_bad = nullptr;                // while loading: set when a block exponent lies outside the range of the scaled products
+    uint32_t *exp_bad = nullptr;                // while loading, per layer gate|up and down: set when a block exponent lies outside the range of the scaled products
     int8_t *nq = nullptr;        // Q8 of the normalised residual that the fold leaves for the next q/k/v projection
     float *ns = nullptr;
     bool fused_fold = true;      // speculative tensor-core step: fold + next norm/quant in one kernel that waits for the router by flag
@@ -269,20 +269,21 @@ int load_q8_part(brrr_model *m, const Source &s, uint32_t layer, int kind, int r
 }
 
 // rows [row0, row0 + rows) of an MXFP4 tensor of rows_total rows (an expert-parallel rank loads its experts only)
-int load_mx(brrr_model *m, const Source &s, uint32_t layer, int kind, int rows, int blocks, MxDev *x, void *scratch, int row0 = 0, int rows_total = 0) {
+// bad (nullable): word that launch_mx_exp_scan sets
+int load_mx(brrr_model *m, const Source &s, uint32_t layer, int kind, int rows, int blocks, MxDev *x, void *scratch, uint32_t *bad, int row0 = 0, int rows_total = 0) {
     x->rows = rows; x->blocks = blocks;
     TRY(m->alloc(&x->data, mx_bytes(rows, blocks)));
     TRY(fetch(m, s, layer, kind, 39, (size_t)rows * blocks * 32, scratch, (size_t)row0 * blocks * 32, (size_t)(rows_total ? rows_total : rows) * blocks * 32));
     launch_mx_pack((const uint8_t *)scratch, *x, m->stream);
     CU(cudaGetLastError());
-    if (!m->exp_bad) return BRRR_OK;
-    launch_mx_exp_scan((const uint8_t *)scratch, (size_t)rows * blocks, m->exp_bad, m->stream);
+    if (!bad) return BRRR_OK;
+    launch_mx_exp_scan((const uint8_t *)scratch, (size_t)rows * blocks, bad, m->stream);
     // expert-parallel ranks have to run the same kind of step, so each looks at the other ranks' rows too
     for (int r = 0; r < rows_total; r += rows) {
         if (r == row0) continue;
         const int n = std::min(rows, rows_total - r);
         TRY(fetch(m, s, layer, kind, 39, (size_t)n * blocks * 32, scratch, (size_t)r * blocks * 32, (size_t)rows_total * blocks * 32));
-        launch_mx_exp_scan((const uint8_t *)scratch, (size_t)n * blocks, m->exp_bad, m->stream);
+        launch_mx_exp_scan((const uint8_t *)scratch, (size_t)n * blocks, bad, m->stream);
     }
     CU(cudaGetLastError());
     return BRRR_OK;
@@ -543,8 +544,8 @@ int build_model(brrr_model *m, const Source &src) {
         if (const char *e = getenv("BRRR_TILE_ROWS")) { const int v = atoi(e); if (v >= 2 && v <= BRRR_TILE_MAX) m->tile_rows = v; }
     }
     if (m->use_mxt) {
-        TRY(m->alloc(&m->exp_bad, 1));
-        CU(cudaMemsetAsync(m->exp_bad, 0, 4, m->stream));
+        TRY(m->alloc(&m->exp_bad, 2 * (size_t)c.n_layer));
+        CU(cudaMemsetAsync(m->exp_bad, 0, 8 * (size_t)c.n_layer, m->stream));
     }
     for (int il = 0; il < c.n_layer; il++) {
         Layer &ly = m->L[il];
@@ -575,10 +576,14 @@ int build_model(brrr_model *m, const Source &src) {
         CU(cudaGetLastError());
         TRY(load_f32(m, src, il, BRRR_T_ROUTER_B, ne, &ly.ginp_b));
         const int e_lo = m->ep ? m->epc.e_lo : 0, e_cnt = m->ep ? m->epc.e_cnt : ne;
-        TRY(load_mx(m, src, il, BRRR_T_GATE, e_cnt * d, nb, &ly.gate, scratch, e_lo * d, ne * d));
-        TRY(load_mx(m, src, il, BRRR_T_UP, e_cnt * d, nb, &ly.up, scratch, e_lo * d, ne * d));
-        TRY(load_mx(m, src, il, BRRR_T_DOWN, e_cnt * d, nb, &ly.down, scratch, e_lo * d, ne * d));
+        uint32_t *bad = m->exp_bad ? m->exp_bad + 2 * il : nullptr, wide[2] = {0, 0};
+        TRY(load_mx(m, src, il, BRRR_T_GATE, e_cnt * d, nb, &ly.gate, scratch, bad, e_lo * d, ne * d));
+        TRY(load_mx(m, src, il, BRRR_T_UP, e_cnt * d, nb, &ly.up, scratch, bad, e_lo * d, ne * d));
+        TRY(load_mx(m, src, il, BRRR_T_DOWN, e_cnt * d, nb, &ly.down, scratch, bad ? bad + 1 : nullptr, e_lo * d, ne * d));
         if (m->use_mxt) {
+            CU(cudaMemcpyAsync(wide, bad, 8, cudaMemcpyDeviceToHost, m->stream));
+            CU(cudaStreamSynchronize(m->stream));
+            ly.gu_t.wide = wide[0]; ly.down_t.wide = wide[1];
             ly.gu_t.tiles_per_expert = d / 64; ly.gu_t.np = nb / 2;
             ly.down_t.tiles_per_expert = (d + 127) / 128; ly.down_t.np = nb / 2;
             TRY(m->alloc(&ly.gu_t.data, mxt_bytes(e_cnt, ly.gu_t.tiles_per_expert, nb / 2)));       // this rank's experts
@@ -595,16 +600,7 @@ int build_model(brrr_model *m, const Source &src) {
         CU(cudaMemsetAsync(ly.kc, 0, (size_t)BRRR_MAXSEQ * nkv * hd * 4, m->stream));   // layout [kv head][position][64]
         CU(cudaMemsetAsync(ly.vc, 0, (size_t)BRRR_MAXSEQ * nkv * hd * 4, m->stream));
     }
-    if (m->use_mxt) {
-        uint32_t bad = 0;
-        CU(cudaMemcpyAsync(&bad, m->exp_bad, 4, cudaMemcpyDeviceToHost, m->stream));
-        CU(cudaStreamSynchronize(m->stream));
-        m->release(&m->exp_bad);
-        if (bad) {                       // the scaled products would not be exact: the integer units run the experts (same bits)
-            m->use_mxt = false;
-            for (Layer &ly : m->L) { m->release(&ly.gu_t.data); m->release(&ly.down_t.data); }
-        }
-    }
+    m->release(&m->exp_bad);
     TRY(m->alloc(&m->tok_embd, (size_t)c.n_vocab * d));
     TRY(fetch(m, src, BRRR_L_GLOBAL, BRRR_T_TOK_EMBD, 30, (size_t)c.n_vocab * d, m->tok_embd));
     TRY(load_f32(m, src, BRRR_L_GLOBAL, BRRR_T_OUT_NORM, d, &m->out_norm));
@@ -1477,6 +1473,9 @@ extern "C" int brrr_stage_time(brrr_model *m, int stage, uint32_t pos, int reps,
 #ifdef BRRR_TEST_HOOKS
 // Test-hook builds only (not part of the public interface): device bytes the model holds (what BRRR_TEST_MEM_BYTES bounds).
 extern "C" uint64_t brrr_debug_taken(const brrr_model *m) { return m ? m->taken : 0; }
+
+// which expert matrices of layer il run in the wide form (bit 0: gate | up, bit 1: down)
+extern "C" int brrr_debug_wide(const brrr_model *m, int il) { return (m->L[il].gu_t.wide ? 1 : 0) | (m->L[il].down_t.wide ? 2 : 0); }
 
 // the in-kernel clock stamps of the last step.
 extern "C" int brrr_debug_stamps(brrr_model *m, long long *out256) {

@@ -416,8 +416,8 @@ int brrr_moe_ffn_step(brrr_model *m, int il, const float *d_xn, float *d_x, int3
  * the tensor cores in their native 4-bit format (tcgen05.mma kind::mxf4.block_scale on the raw e2m1
  * codes, the Q8 activation split into three exact digit planes), results bit-identical to
  * brrr_moe_ffn_step.  BRRR_ERR_STATE when the model holds no tile-unit copy of the experts
- * (expert-parallel models, shapes with n_embd % 64 != 0, BRRR_NOMXT=1, not enough memory, or a block exponent
- * outside 49 .. 190 in a block that is not zero: the decode step then runs on the integer units).
+ * (expert-parallel models, shapes with n_embd % 64 != 0, BRRR_NOMXT=1, not enough memory: the decode step
+ * then runs on the integer units).
  * Replaces src/bin/engine_gpt2.rs:847-923. */
 int brrr_moe_ffn_step_tc(brrr_model *m, int il, const float *d_xn, float *d_x, int32_t *d_top, float *d_wts);
 /* 1 when the decode step of this model runs its expert matvecs on the tensor cores. */

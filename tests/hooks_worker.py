@@ -3,7 +3,7 @@
 default build, which contains no hook.  No GPU fault is provoked: a missed speculation is a
 flagged step, a silent router is a bounded wait that runs out and is reported.
 
-    python tests/hooks_worker.py sabotage | mute | memory | qwen_sabotage | qwen_mute | qwen_memory
+    python tests/hooks_worker.py sabotage | mute | memory | exponents | qwen_sabotage | qwen_mute | qwen_memory
 """
 import os
 import sys
@@ -162,10 +162,33 @@ def memory(cfg, prompt):
     free()
 
 
+def exponents():
+    """The form each layer's expert matrices run in (brrr_debug_wide: bit 0 = gate | up, bit 1 = down)."""
+    import ctypes as C
+    import tempfile
+    import cpubrrr_b200 as B
+    import refdata
+    from test_gpu_mxt import EXPONENTS
+    wide_of = B.lib().brrr_debug_wide
+    wide_of.restype, wide_of.argtypes = C.c_int, [C.c_void_p, C.c_int]
+    for exps, wide in EXPONENTS:
+        for kind, bit in (("gate", 1), ("up", 1), ("down", 2)):
+            with tempfile.TemporaryDirectory() as tmp:
+                _, d, blob = refdata.case_data_dir(tmp, "gptoss_d128", 12)
+                refdata.set_exponents(d, blob, f"blk.1.ffn_{kind}_exps.weight", exps)
+                eng = B.Engine.open(d, blob)
+                assert (wide_of(eng._h, 0), wide_of(eng._h, 1)) == (0, bit if wide else 0), (exps, kind)
+                eng.close()
+
+
 def main(mode):
     assert os.environ.get("BRRR_LIBRARY", "").endswith("libbrrr_hooks.so")
     if mode.startswith("qwen"):
         qwen(mode)
+        print("hooks_worker ok:", mode)
+        return
+    if mode == "exponents":
+        exponents()
         print("hooks_worker ok:", mode)
         return
     import cpubrrr_b200 as B

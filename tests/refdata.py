@@ -137,3 +137,18 @@ def retype_qwen(data_dir, blob, cfg, seed, ktypes):
     assert int(head.split()[1]) + off == os.path.getsize(blob)
     with open(path, "w") as w:
         w.write("\n".join(out) + "\n")
+
+
+def set_exponents(data_dir, blob, tensor, exponents):
+    """Every seventh block of an MXFP4 tensor of a made data directory gets the next of the given exponents (a pair: exponent of a block of zeros)."""
+    import numpy as np
+    rows = [r.split() for r in open(os.path.join(data_dir, "manifest.txt"))]
+    _, _, off, nel = next(r for r in rows if r[0] == tensor)
+    raw = np.memmap(blob, np.uint8, "r+", int(rows[0][1]) + int(off), (int(nel) // 32, 17))
+    for i, b in enumerate(range(3, len(raw), 7)):
+        ex = exponents[i % len(exponents)]
+        if isinstance(ex, tuple):
+            ex = ex[0]
+            raw[b, 1:] = np.arange(16) % 2 * 0x80 + np.arange(16) % 3 % 2 * 8      # +0 and -0
+        raw[b, 0] = ex
+    raw.flush()

@@ -9,20 +9,20 @@ import pytest
 
 from conftest import bits, to_dev
 from cpubrrr_b200 import synth as S
-from test_gpu_model import greedy, ocfg_of
+from test_gpu_model import _run_with_hooks, greedy, ocfg_of
 
 pytestmark = pytest.mark.gpu
 
 
-def _ffn_oracle(orc, om, ocfg, xn):
+def _ffn_oracle(orc, om, ocfg, xn, il=0):
     Lo = orc.lib()
     vp = lambda a: a.ctypes.data_as(C.c_void_p)
     d, k = ocfg.d, ocfg.topk
     y = np.zeros(d, np.float32)
     top = np.zeros(k, np.int32); wts = np.zeros(k, np.float32)
-    Lo.orc_moe_ffn_step(C.byref(ocfg), vp(xn), Lo.orc_layer_f32(om.h, 0, S.T["ROUTER_W"]), Lo.orc_layer_f32(om.h, 0, S.T["ROUTER_B"]),
-                        Lo.orc_layer_mx(om.h, 0, 0), Lo.orc_layer_mx(om.h, 0, 1), Lo.orc_layer_mx(om.h, 0, 2),
-                        Lo.orc_layer_f32(om.h, 0, S.T["GATE_B"]), Lo.orc_layer_f32(om.h, 0, S.T["UP_B"]), Lo.orc_layer_f32(om.h, 0, S.T["DOWN_B"]),
+    Lo.orc_moe_ffn_step(C.byref(ocfg), vp(xn), Lo.orc_layer_f32(om.h, il, S.T["ROUTER_W"]), Lo.orc_layer_f32(om.h, il, S.T["ROUTER_B"]),
+                        Lo.orc_layer_mx(om.h, il, 0), Lo.orc_layer_mx(om.h, il, 1), Lo.orc_layer_mx(om.h, il, 2),
+                        Lo.orc_layer_f32(om.h, il, S.T["GATE_B"]), Lo.orc_layer_f32(om.h, il, S.T["UP_B"]), Lo.orc_layer_f32(om.h, il, S.T["DOWN_B"]),
                         vp(y), vp(top), vp(wts))
     return y, top, wts
 
@@ -108,34 +108,47 @@ def test_decode_same_with_and_without_tensor_experts(brrr, orc, monkeypatch):
     assert np.array_equal(bits(om.logits()), bits(lg))
 
 
-@pytest.mark.parametrize("edge,tensor_experts", [
-    ([49, 190, 120, 60], True),          # the ends of the range whose scaled products are exact
-    ([(0, 0), (48, 0), 49], True),       # zero blocks below it
-    ([48], False),                       # values other than zero below it, any block above it: the integer units
-    ([191], False),
-    ([(255, 0)], False),
-])
-def test_block_exponents_choose_the_expert_kernels(brrr, orc, tmp_path, edge, tensor_experts):
-    """Gate blocks with the given exponents (pairs: exponent of a block of zeros) among the synthetic ones: whether the model's
-    experts run on the tensor cores, and the oracle's tokens and logits either way."""
-    import os
+EXPONENTS = [
+    ([49, 134, 120, 60], False),         # the ends of the range whose scaled products are exact
+    ([(0, 0), (48, 0), 49], False),      # zero blocks below it
+    ([48], True),                        # values other than zero below it, any block above it: scales in the epilogue
+    ([135], True),
+    ([0, 1, 2, 190], True),
+    ([(255, 0)], True),
+]
+
+
+@pytest.mark.parametrize("kind", ["gate", "up", "down"])
+@pytest.mark.parametrize("exponents,wide", EXPONENTS)
+def test_block_exponents_of_any_size(brrr, orc, dev, tmp_path, exponents, wide, kind):
+    """Blocks with the given exponents (pairs: exponent of a block of zeros) among the synthetic ones of one layer's matrix: the experts stay on the
+    tensor cores and the oracle's tokens and logits come out, and the stage call answers, with activations from the smallest scale to huge ones."""
+    import torch
     import refdata
     cfg, d, blob = refdata.case_data_dir(str(tmp_path), "gptoss_d128", 12)
-    rows = [r.split() for r in open(os.path.join(d, "manifest.txt"))]
-    name, _, off, nel = next(r for r in rows if r[0] == "blk.1.ffn_gate_exps.weight")
-    raw = np.memmap(blob, np.uint8, "r+", int(rows[0][1]) + int(off), (int(nel) // 32, 17))
-    for i, b in enumerate(range(3, len(raw), 7)):
-        ex = edge[i % len(edge)]
-        if isinstance(ex, tuple):
-            ex = ex[0]
-            raw[b, 1:] = np.arange(16) % 2 * 0x80 + np.arange(16) % 3 % 2 * 8      # +0 and -0
-        raw[b, 0] = ex
-    raw.flush()
+    refdata.set_exponents(d, blob, f"blk.1.ffn_{kind}_exps.weight", exponents)
     eng, om = brrr.Engine.open(d, blob), orc.Model.open(d, blob)
-    assert eng.uses_tensor_experts == tensor_experts
+    assert eng.uses_tensor_experts
     prompt = S.synth_prompt(12, 7, 500)
     assert greedy(eng.run, prompt, 24) == greedy(om.run, prompt, 24)
     assert np.array_equal(bits(eng.logits()), bits(om.logits()))
     # the same prompt as token rows
     assert eng.run_tile([int(t) for t in prompt], 0, True) == greedy(om.run, prompt, 1)[0]
+    P = lambda t: C.c_void_p(t.data_ptr())
+    for scale in (1e-30, 1.0, 2.0 ** 66):
+        xn = S.synth_input(7, cfg.n_embd) * np.float32(scale)
+        dxn, y = to_dev(xn, dev), [torch.zeros(cfg.n_embd, dtype=torch.float32, device=dev) for _ in range(2)]
+        eng.moe_ffn_step_tc(1, P(dxn), P(y[0]), None, None)
+        eng.moe_ffn_step(1, P(dxn), P(y[1]), None, None)
+        tc, iu = (bits(t.cpu().numpy()) for t in y)
+        assert np.array_equal(tc, iu)
+        largest = max(e[0] if isinstance(e, tuple) else e for e in exponents)
+        if scale > 1 and largest >= 190:         # the block's scale, 2^62 x 2^66 and more, overflows: sums that are no numbers (inf - inf, 0 x inf)
+            continue
+        assert np.array_equal(tc, bits(_ffn_oracle(orc, om, ocfg_of(orc, cfg), xn, 1)[0]))
     eng.close()
+
+
+def test_block_exponents_choose_the_form(brrr):
+    """Which form the matrices of a layer run in: by the layer's own blocks, gate | up and down each by themselves."""
+    _run_with_hooks(brrr, "exponents")
