@@ -278,13 +278,6 @@ int load_mx(brrr_model *m, const Source &s, uint32_t layer, int kind, int rows, 
     CU(cudaGetLastError());
     if (!bad) return BRRR_OK;
     launch_mx_exp_scan((const uint8_t *)scratch, (size_t)rows * blocks, bad, m->stream);
-    // expert-parallel ranks have to run the same kind of step, so each looks at the other ranks' rows too
-    for (int r = 0; r < rows_total; r += rows) {
-        if (r == row0) continue;
-        const int n = std::min(rows, rows_total - r);
-        TRY(fetch(m, s, layer, kind, 39, (size_t)n * blocks * 32, scratch, (size_t)r * blocks * 32, (size_t)rows_total * blocks * 32));
-        launch_mx_exp_scan((const uint8_t *)scratch, (size_t)n * blocks, bad, m->stream);
-    }
     CU(cudaGetLastError());
     return BRRR_OK;
 }

@@ -1,6 +1,6 @@
 """Worker of the expert-parallel tests (launched by torch.distributed.run, one process per GPU):
-opens this rank's shard of a seeded synthetic model, decodes greedily and writes what it produced
-to <out>/rank<r>.json.  Usage: ep_worker.py <out-dir> <cfg-json> <seed> <n-steps> [stall]
+opens this rank's shard of a seeded synthetic model (or of a data directory with a model.gguf), decodes greedily and writes
+what it produced to <out>/rank<r>.json.  Usage: ep_worker.py <out-dir> <cfg-json | data-dir> <seed> <n-steps> [stall]
 
 With "stall" the last rank stops issuing steps after the prompt (it stays alive and keeps its memory
 mapped); the other ranks issue one more step, whose bounded wait for the stalled rank's row sums
@@ -27,9 +27,14 @@ def main():
     torch.cuda.set_device(local)
     dev = torch.device("cuda", local)
     dist.init_process_group("nccl", device_id=dev)
-    cfg = B.make_cfg(**json.loads(cfg_json))
-    eng = ep.open_synth_ep(cfg, seed, rank, world, device=local, dist=dist, torch_device=dev)
-    prompt = S.synth_prompt(seed, 9, cfg.n_vocab)
+    if os.path.isdir(cfg_json):
+        eng = ep.open_ep(cfg_json, os.path.join(cfg_json, "model.gguf"), rank, world, device=local, dist=dist, torch_device=dev)
+        n_vocab = int(dict(r.split() for r in open(os.path.join(cfg_json, "config.txt")))["n_vocab"])
+    else:
+        cfg = B.make_cfg(**json.loads(cfg_json))
+        eng = ep.open_synth_ep(cfg, seed, rank, world, device=local, dist=dist, torch_device=dev)
+        n_vocab = cfg.n_vocab
+    prompt = S.synth_prompt(seed, 9, n_vocab)
     first = eng.prefill(prompt)                                  # host-driven steps
     if stall:
         import time

@@ -139,13 +139,15 @@ def retype_qwen(data_dir, blob, cfg, seed, ktypes):
         w.write("\n".join(out) + "\n")
 
 
-def set_exponents(data_dir, blob, tensor, exponents):
-    """Every seventh block of an MXFP4 tensor of a made data directory gets the next of the given exponents (a pair: exponent of a block of zeros)."""
+def set_exponents(data_dir, blob, tensor, exponents, rows=None, cols=None):
+    """Every seventh block of an MXFP4 tensor of a made data directory (or of its rows lo .. hi - 1, each cols wide) gets the next of the given
+    exponents (a pair: exponent of a block of zeros)."""
     import numpy as np
-    rows = [r.split() for r in open(os.path.join(data_dir, "manifest.txt"))]
-    _, _, off, nel = next(r for r in rows if r[0] == tensor)
-    raw = np.memmap(blob, np.uint8, "r+", int(rows[0][1]) + int(off), (int(nel) // 32, 17))
-    for i, b in enumerate(range(3, len(raw), 7)):
+    lines = [r.split() for r in open(os.path.join(data_dir, "manifest.txt"))]
+    _, _, off, nel = next(r for r in lines if r[0] == tensor)
+    raw = np.memmap(blob, np.uint8, "r+", int(lines[0][1]) + int(off), (int(nel) // 32, 17))
+    lo, hi = (r * cols // 32 for r in rows) if rows else (0, len(raw))
+    for i, b in enumerate(range(lo + 3, hi, 7)):
         ex = exponents[i % len(exponents)]
         if isinstance(ex, tuple):
             ex = ex[0]

@@ -55,8 +55,8 @@ def _ocfg(orc, c):
                         topk=c.n_expert_used, nvocab=c.n_vocab, swa=c.sliding_window, rope_base=c.rope_freq_base, rms_eps=c.rms_eps)
 
 
-def _oracle_run(orc, cfg, seed, nsteps):
-    om = orc.Model.synth(_ocfg(orc, cfg), seed)
+def _oracle_run(orc, cfg, seed, nsteps, om=None):
+    om = om or orc.Model.synth(_ocfg(orc, cfg), seed)
     prompt = S.synth_prompt(seed, 9, cfg.n_vocab)
     tok = 0
     for i, t in enumerate(prompt):
@@ -94,10 +94,14 @@ def test_ep_multi_rank_equals_oracle(brrr, orc, tmp_path, world):
     cfg = brrr.make_cfg(**shape)
     seed, nsteps = 53, 48
     first, want, om = _oracle_run(orc, cfg, seed, nsteps)
+    _ranks_equal(tmp_path, world, json.dumps(shape), seed, nsteps, first, want, om)
+
+
+def _ranks_equal(tmp_path, world, model, seed, nsteps, first, want, om):
     port = 29600 + os.getpid() % 2000
     env = dict(os.environ, NCCL_NVLS_ENABLE="0")
     r = subprocess.run([sys.executable, "-m", "torch.distributed.run", "--nnodes=1", f"--nproc-per-node={world}", "--master-addr", "127.0.0.1",
-                        "--master-port", str(port), os.path.join(HERE, "ep_worker.py"), str(tmp_path), json.dumps(shape), str(seed), str(nsteps)],
+                        "--master-port", str(port), os.path.join(HERE, "ep_worker.py"), str(tmp_path), model, str(seed), str(nsteps)],
                        capture_output=True, timeout=600, env=env)
     assert r.returncode == 0, r.stderr.decode()[-3000:]
     for rank in range(world):
@@ -105,6 +109,67 @@ def test_ep_multi_rank_equals_oracle(brrr, orc, tmp_path, world):
         assert res["first"] == first and res["tokens"] == want, f"rank {rank}"
         assert res["hidden_bits"] == [int(b) for b in bits(om.hidden())], f"rank {rank}"
         assert res["logit_bits"] == [int(b) for b in bits(om.logits())[:64]], f"rank {rank}"
+
+
+def _wide_model(tmp_path, expert):
+    """A data directory whose layer 1 has blocks outside the scaled products' range, in one expert's gate and down."""
+    import refdata
+    cfg, d, blob = refdata.case_data_dir(str(tmp_path), "gptoss_d128", 12)
+    for kind in ("gate", "down"):
+        refdata.set_exponents(d, blob, f"blk.1.ffn_{kind}_exps.weight", [2, 190, 40], rows=(expert * cfg.n_embd, (expert + 1) * cfg.n_embd), cols=cfg.n_embd)
+    return cfg, d, blob
+
+
+@pytest.mark.gpu
+def test_ep_block_exponents_of_any_size(brrr, orc, tmp_path):
+    """The expert-parallel forms of the kernels on a layer with such blocks (one rank)."""
+    from cpubrrr_b200 import ep
+    cfg, d, blob = _wide_model(tmp_path, 5)
+    first, want, om = _oracle_run(orc, cfg, 12, 40, orc.Model.open(d, blob))
+    eng = ep.open_ep(d, blob, 0, 1)
+    assert eng.uses_tensor_experts
+    prompt = S.synth_prompt(12, 9, cfg.n_vocab)
+    assert eng.prefill(prompt) == first
+    assert [int(t) for t in eng.decode(first, len(prompt), 40)] == want
+    assert np.array_equal(bits(eng.hidden()), bits(om.hidden())) and np.array_equal(bits(eng.logits()), bits(om.logits()))
+    eng.close()
+
+
+@pytest.mark.gpu
+def test_ep_ranks_with_different_block_exponents(brrr, orc, tmp_path):
+    """Two ranks, one of which holds the expert with such blocks: each decides the form of its own matrices."""
+    import torch
+    if torch.cuda.device_count() < 2:
+        pytest.skip("needs 2 GPUs")
+    cfg, d, blob = _wide_model(tmp_path, 5)
+    first, want, om = _oracle_run(orc, cfg, 12, 40, orc.Model.open(d, blob))
+    _ranks_equal(tmp_path, 2, d, 12, 40, first, want, om)
+
+
+@pytest.mark.gpu
+def test_ep_rank_reads_its_own_experts_only(brrr, tmp_path):
+    """An expert tensor whose second half lies past the end of the file: the rank of the first half opens, the other one cannot."""
+    import ctypes as C
+    import refdata
+    cfg, d, blob = refdata.case_data_dir(str(tmp_path), "gptoss_d128", 12)
+    path, L = os.path.join(d, "manifest.txt"), brrr.lib()
+    head, *rows = open(path).read().strip().split("\n")
+    start, size = int(head.split()[1]), os.path.getsize(blob)
+    for i, row in enumerate(rows):
+        name, ty, off, nel = row.split()
+        if "exps.weight" not in name:
+            continue
+        with open(blob, "r+b") as f:                 # its first half again, as the end of the file
+            f.truncate(size)
+            f.seek(start + int(off))
+            half = f.read(int(nel) // 64 * 17)
+            f.seek(size)
+            f.write(half)
+        open(path, "w").write("\n".join([head, *rows[:i], f"{name} {ty} {size - start} {nel}", *rows[i + 1:]]) + "\n")
+        h = C.c_void_p()
+        assert L.brrr_model_open_ep(d.encode(), blob.encode(), 0, 1, 2, C.byref(h)) == 2, name      # BRRR_ERR_IO
+        assert L.brrr_model_open_ep(d.encode(), blob.encode(), 0, 0, 2, C.byref(h)) == 0, name
+        L.brrr_model_close(h)
 
 
 @pytest.mark.gpu
