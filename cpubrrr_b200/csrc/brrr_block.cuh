@@ -161,58 +161,49 @@ __device__ __forceinline__ void block_norm_quant_staged(const float *norm_w, con
     }
 }
 
-// The k largest of est[0..ne) by (value, lower index first): sel[r] gets the expert of rank r.
-// Every thread ranks the experts it owns against all others in shared memory (no shuffles, one
-// global round trip).  Used identically by every kernel that needs the speculative expert set
-// (the set comes from an order-free router estimate; correctness never depends on it).
-// Builds with BRRR_TEST_HOOKS only: when the state's test_hooks word has bit 0 set, the last pick is
-// replaced on every third position (the tests use it to force a missed speculation).
-// Block-wide; ends with sel[] written but not yet synchronised.  lg: ne floats of scratch.
-__device__ __forceinline__ void block_spec_select(const float *est, int ne, int topk, const DevState *state,
-                                                  float *lg, int *sel, int tid, int nthreads) {
-#ifdef BRRR_TEST_HOOKS
-    const bool sabotage = state && (state->test_hooks & 1u);
-    const uint32_t pos = sabotage ? state->pos : 0u;
-#else
-    constexpr bool sabotage = false;
-    constexpr uint32_t pos = 0u;
-    (void)state;
-#endif
-    for (int e = tid; e < ne; e += nthreads) lg[e] = __ldcg(est + e);
-    __syncthreads();
-    for (int e = tid; e < ne; e += nthreads) {
-        const float v = lg[e];
-        int rank = 0;
-        for (int o = 0; o < ne; o++) {
-            const float u = lg[o];
-            rank += (u > v || (u == v && o < e)) ? 1 : 0;
-        }
-        if (rank < topk) sel[rank] = (sabotage && rank == topk - 1 && pos % 3 == 0) ? (e + 1) % ne : e;
+// The largest entries of est[0 .. ne), ne <= 256: lane r < turns gets the expert of rank r (the larger first, the lower index among equals), by one
+// warp without shared memory or barriers: each warp that needs the experts picks them itself.  All 32 lanes call it; every entry is a valid
+// index whatever the values are (a NaN counts as larger than +inf or smaller than -inf, by its sign).  A lane holds PER consecutive experts as
+// order-preserving keys; a turn is a maximum over the lane's keys and one reduction over the warp, the index travels beside the next turn.
+// Used by every kernel that needs the speculative expert set (the set comes from an order-free router estimate; correctness never depends on
+// it).  Ranking every expert against every other, block-wide with barriers, took 2300 cycles at 32 experts; at 128 the qwen3moe gate/up had its experts
+// 2400 cycles after its dependency wait (64 + 128 tokens of the 30b-a3b shape: 209.2 ms, 206.5 with the warps picking and the copies spread over them).
+template <int PER>
+__device__ __forceinline__ int spec_pick_n(const float *est, int ne, int turns, int lane) {
+    uint32_t key[PER];
+#pragma unroll
+    for (int i = 0; i < PER; i++) {
+        const int e = lane * PER + i;
+        key[i] = e < ne ? max(float_orderable(__fadd_rn(__ldcg(est + e), 0.0f)), 1u) : 0u;       // +0 for -0; 0: absent or taken
     }
+    int mine = 0;
+#pragma unroll 1
+    for (int r = 0; r < turns; r++) {
+        uint32_t m = key[0];
+#pragma unroll
+        for (int i = 1; i < PER; i++) m = max(m, key[i]);
+        const uint32_t best = __reduce_max_sync(0xffffffffu, m);
+        const int from = __ffs(__ballot_sync(0xffffffffu, m == best)) - 1;
+        int at = PER - 1;
+#pragma unroll
+        for (int i = PER - 2; i >= 0; i--) if (key[i] == best) at = i;
+        const int e = PER == 1 ? from : __shfl_sync(0xffffffffu, lane * PER + at, from);
+        if (lane == r) mine = e;
+#pragma unroll
+        for (int i = 0; i < PER; i++) if (lane == from && i == at) key[i] = 0u;
+    }
+    return mine;
 }
-
-// The same selection for ne <= 32 inside one warp, without shared memory or block-wide barriers:
-// returns the expert of rank `want` (what block_spec_select would leave in sel[want]).  All 32
-// lanes must call it.
-__device__ __forceinline__ int warp_spec_expert(const float *est, int ne, int topk, const DevState *state, int want, int lane) {
+// turns <= topk ranks.  Builds with BRRR_TEST_HOOKS only: when the state's test_hooks word has bit 0 set, the last of the topk picks is replaced on every
+// third position (the tests use it to force a missed speculation).
+__device__ __forceinline__ int spec_pick(const float *est, int ne, int topk, int turns, const DevState *state, int lane) {
+    const int e = ne <= 32 ? spec_pick_n<1>(est, ne, turns, lane) : ne <= 128 ? spec_pick_n<4>(est, ne, turns, lane) : spec_pick_n<8>(est, ne, turns, lane);
 #ifdef BRRR_TEST_HOOKS
-    const bool sabotage = state && (state->test_hooks & 1u);
-    const uint32_t pos = sabotage ? state->pos : 0u;
+    if (state && (state->test_hooks & 1u) && state->pos % 3 == 0 && lane == topk - 1) return (e + 1) % ne;
 #else
-    constexpr bool sabotage = false;
-    constexpr uint32_t pos = 0u;
-    (void)state;
+    (void)topk; (void)state;
 #endif
-    // order-preserving keys (+0 for -0), the largest taken out `want` times: three instructions a turn, where ranking every lane against
-    // every other took 2300 cycles
-    uint32_t key = lane < ne ? float_orderable(__fadd_rn(__ldcg(est + lane), 0.0f)) : 0u;
-    int e = 0;
-    for (int r = 0; r <= want; r++) {
-        const uint32_t m = __reduce_max_sync(0xffffffffu, key);
-        e = __ffs(__ballot_sync(0xffffffffu, key == m)) - 1;
-        if (lane == e) key = 0u;
-    }
-    return (sabotage && want == topk - 1 && pos % 3 == 0) ? (e + 1) % ne : e;
+    return e;
 }
 
 // gpt-oss clamped SwiGLU: xg = min(g, 7), yu = clamp(u, -7, 7), (xg / (1 + exp(-1.702 xg))) (yu + 1)

@@ -146,10 +146,8 @@ __global__ void __launch_bounds__(256) gate_up_kernel(GateUpArgs a) {
     BRRR_GT_GO(a.state, 126);
     pdl_trigger();
     waiter.poison_if_failed();
-    __shared__ int sel[8];
-    __shared__ float lg[256];
     // all global reads of this phase are issued together: the activation words go to registers
-    // first, the expert set is ranked, then the activation is staged
+    // first, the expert is picked, then the activation is staged
     uint32_t xlo[2], xhi[2];
     if (!a.x_f32) {
 #pragma unroll
@@ -161,12 +159,8 @@ __global__ void __launch_bounds__(256) gate_up_kernel(GateUpArgs a) {
             }
         }
     }
-    if (a.est) {
-        block_spec_select(a.est, a.ne, a.topk, a.state, lg, sel, tid, 256);
-        __syncthreads();
-    }
+    const int e = a.est ? __shfl_sync(0xffffffffu, spec_pick(a.est, a.ne, a.topk, ei + 1, a.state, lane), ei) : a.top[ei];      // every warp by itself
     BRRR_STAMP(a.state, 102);
-    const int e = a.est ? sel[ei] : a.top[ei];
     const int el = e - a.e_lo;                       // index among the experts held here
     if (el < 0 || el >= a.e_cnt) return;             // this slot's expert lives on another rank
     const int nchunks = (np + a.ch - 1) / a.ch;
@@ -318,13 +312,9 @@ __global__ void __launch_bounds__(512) down_combine_kernel(DownArgs a) {
     // which slot of hq/hs holds this rank's expert (identity without speculation)
     int slot = ei;
     if (a.est) {
-        __shared__ int sel[8];
-        __shared__ float lg[256];
-        block_spec_select(a.est, a.ne, a.topk, a.state, lg, sel, tid, nthreads);
-        __syncthreads();
+        const int picked = spec_pick(a.est, a.ne, a.topk, a.topk, a.state, tid & 31), want = a.top[ei];      // (a warp works for one slot)
         slot = -1;
-        const int want = a.top[ei];
-        for (int s = 0; s < a.topk; s++) if (sel[s] == want) slot = s;
+        for (int s = 0; s < a.topk; s++) if (__shfl_sync(0xffffffffu, picked, s) == want) slot = s;
         if (slot < 0) {                       // the estimate missed this expert: flag the step, keep going
             slot = 0;
             if (t64 == 0 && blockIdx.x == 0 && a.state) atomicMin(&a.state->spec_fail_step, a.state->n_out);

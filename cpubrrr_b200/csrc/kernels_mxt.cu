@@ -287,11 +287,9 @@ __global__ void __launch_bounds__(XT_THREADS, 2) xt_expert_kernel(XtArgs a) {
     sh.dfull = sh.empty + XT_STAGES;
     sh.dempty = sh.dfull + XT_REGIONS;
     __shared__ uint32_t tmem_base_sh;
-    __shared__ int sel[8];
-    __shared__ float lg[256];
     __shared__ float half_s[128];
     __shared__ float gu_s[2][64];
-    __shared__ int last_sh;
+    __shared__ int last_sh, expert_sh;
     uint32_t *err = a.state ? &a.state->err : nullptr;
     constexpr int SB = DOWN ? 128 : 96;          // clock stamps of timeline builds
     (void)SB;
@@ -329,25 +327,21 @@ __global__ void __launch_bounds__(XT_THREADS, 2) xt_expert_kernel(XtArgs a) {
     xt_fence_after();
     // ---- routing of this slot (the ei-th largest entry of the estimate, or the exact routing), the
     // weight stream, the activation image (one bulk copy) and its block scales
-    int e = 0;
-    bool local = true;
     const size_t tile_bytes = xt_run_bytes(np), expert_bytes = tile_bytes * a.w.tiles_per_expert;
-    const unsigned char *src = a.w.data + t * tile_bytes;
+    auto is_local = [&](int e) { return !EP || (e >= a.ep.e_lo && e < a.ep.e_lo + a.ep.e_cnt); };
+    auto tile_of = [&](int e) { return a.w.data + t * tile_bytes + (size_t)(EP ? e - a.ep.e_lo : e) * expert_bytes; };
     const uint32_t ep_epoch = EP ? *a.ep.epoch : 0u;          // the step in flight (written by the step's first kernel)
+    // by the producer warp alone; the others read the expert behind the barrier in front of the rounds.  20b shape,
+    // 73 + 128 tokens: 126.9 ms with every warp picking for itself, 125.9 so; 120b shape (128 experts): 652 tok/s, 707 so, 687 with a block-wide ranking.
     auto route_and_start = [&]() {
-        if (a.est && a.ne <= 32) e = warp_spec_expert(a.est, a.ne, a.topk, a.state, ei, lane);      // every warp by itself: no barrier
-        else if (a.est) {
-            block_spec_select(a.est, a.ne, a.topk, a.state, lg, sel, tid, XT_THREADS);
-            __syncthreads();
-            e = sel[ei];
-        } else e = a.top[ei];
-        local = !EP || (e >= a.ep.e_lo && e < a.ep.e_lo + a.ep.e_cnt);
-        src += (size_t)(EP ? e - a.ep.e_lo : e) * expert_bytes;
-        if (local && warp == XT_PRODUCER && lane < min(XT_STAGES, nchunks)) {          // one lane per copy: the first stages of the weight stream
+        if (warp != XT_PRODUCER) return;
+        const int e = a.est ? __shfl_sync(0xffffffffu, spec_pick(a.est, a.ne, a.topk, ei + 1, a.state, lane), ei) : a.top[ei];
+        if (is_local(e) && lane < min(XT_STAGES, nchunks)) {          // one lane per copy: the first stages of the weight stream
             const uint32_t bytes = xt_run_bytes(min(XT_CH, np - lane * XT_CH));
             mbar_expect_tx(&sh.full[lane], bytes);
-            bulk_g2s_once(sh.ring + XT_STAGE * lane, src + (size_t)lane * XT_STAGE, bytes, &sh.full[lane]);
+            bulk_g2s_once(sh.ring + XT_STAGE * lane, tile_of(e) + (size_t)lane * XT_STAGE, bytes, &sh.full[lane]);
         }
+        if (lane == 0) expert_sh = e;
     };
     // The down projection knows its expert before gate/up has finished (the routing is two kernels
     // old), and its CTAs have the footprint of a gate/up CTA: they become resident beside running
@@ -372,6 +366,9 @@ __global__ void __launch_bounds__(XT_THREADS, 2) xt_expert_kernel(XtArgs a) {
     for (int k = 0; k < 2; k++) if (tid + k * XT_THREADS < nb * 3) xt_spread_digits(dw[k], tid + k * XT_THREADS, sh.bimg);
     fence_proxy_async();                                         // these stores -> the tensor core's reads
     __syncthreads();
+    const int e = expert_sh;
+    const bool local = is_local(e);
+    const unsigned char *src = tile_of(e);
     BRRR_STAMP(a.state, SB + 3);
 
     // Loop structure shared by the three roles: round r = ring stage r % stages = 4 block pairs =
@@ -553,24 +550,21 @@ struct FoldArgs {
 };
 
 __global__ void __launch_bounds__(128) xt_fold_kernel(FoldArgs a) {
-    __shared__ int sel[8];
-    __shared__ float lg[256];
     __shared__ int slot_of[8];
     const int tid = threadIdx.x;
     BRRR_GT_START(a.state, 238);
     pdl_wait();
     BRRR_GT_GO(a.state, 239);
     pdl_trigger();
-    if (a.est) {
-        block_spec_select(a.est, a.ne, a.topk, a.state, lg, sel, tid, 128);
-        __syncthreads();
+    int found = -1;                          // slot of the exact routing's tid-th expert in the estimate
+    if (a.est && tid < 32) {
+        const int picked = spec_pick(a.est, a.ne, a.topk, a.topk, a.state, tid), want = a.top[min(tid, a.topk - 1)];
+        for (int s = 0; s < a.topk; s++) if (__shfl_sync(0xffffffffu, picked, s) == want) found = s;
     }
     if (tid < a.topk) {
         int slot = tid;
         if (a.est) {
-            slot = -1;
-            const int want = a.top[tid];
-            for (int s = 0; s < a.topk; s++) if (sel[s] == want) slot = s;
+            slot = found;
             if (slot < 0) {                  // the estimate missed this expert: flag the step, keep going
                 slot = 0;
                 if (blockIdx.x == 0 && a.state) atomicMin(&a.state->spec_fail_step, a.state->n_out);
@@ -620,7 +614,6 @@ template <int MAXS, bool EP>       // slots held in registers: top-k <= MAXS; EP
 __global__ void __launch_bounds__(FN_THREADS) xt_fold_norm_kernel(FoldNormArgs a) {
     extern __shared__ __align__(16) float fsm[];          // d floats of the residual
     __shared__ int sel[8];
-    __shared__ float lg[256];
     __shared__ int slot_of[8];
     __shared__ float wts_sh[8];
     __shared__ float inv_sh;
@@ -636,7 +629,10 @@ __global__ void __launch_bounds__(FN_THREADS) xt_fold_norm_kernel(FoldNormArgs a
     const float4 zero4 = make_float4(0.f, 0.f, 0.f, 0.f);
     float4 xr = live ? reinterpret_cast<const float4 *>(a.f.x)[tid] : zero4, pb[MAXS], ps[MAXS];
     if (a.f.est) {
-        block_spec_select(a.f.est, a.f.ne, topk, a.f.state, lg, sel, tid, FN_THREADS);
+        if (tid < 32) {
+            const int picked = spec_pick(a.f.est, a.f.ne, topk, topk, a.f.state, tid);
+            if (tid < topk) sel[tid] = picked;
+        }
         __syncthreads();
 #pragma unroll
         for (int s = 0; s < MAXS; s++) pb[s] = (live && s < topk) ? reinterpret_cast<const float4 *>(a.f.down_b + (size_t)sel[s] * d)[tid] : zero4;

@@ -45,47 +45,6 @@ __global__ void __launch_bounds__(256) qw_embed_kernel(const uint8_t *__restrict
 }
 
 // ---------------------------------------------------------------- expert selection
-// The expert of rank r of est[0 .. ne) in lane r < topk (the larger first, the lower index among equals), by one warp without shared memory or
-// barriers: each warp that needs the experts picks them itself.  A lane holds PER consecutive experts; a turn is a maximum over the lane's
-// keys and one reduction over the warp, the index travels beside the next turn.  Ranking by four threads an expert, block-wide with three
-// barriers, gate/up had its experts 2400 cycles after its dependency wait and its copies out at 3700; 64 + 128 tokens of the 30b-a3b shape:
-// 209.2 ms before, 206.5 with the warps picking and the copies spread over them.
-template <int PER>
-__device__ __forceinline__ int qw_pick_from(const float *est, int ne, int topk, int lane) {
-    uint32_t key[PER];
-#pragma unroll
-    for (int i = 0; i < PER; i++) {
-        const int e = lane * PER + i;
-        key[i] = e < ne ? max(float_orderable(__ldcg(est + e)), 1u) : 0u;       // 0: absent or taken
-    }
-    int mine = 0;
-#pragma unroll 1
-    for (int r = 0; r < topk; r++) {
-        uint32_t m = key[0];
-#pragma unroll
-        for (int i = 1; i < PER; i++) m = max(m, key[i]);
-        const uint32_t best = __reduce_max_sync(0xffffffffu, m);
-        const int from = __ffs(__ballot_sync(0xffffffffu, m == best)) - 1;
-        int at = PER - 1;
-#pragma unroll
-        for (int i = PER - 2; i >= 0; i--) if (key[i] == best) at = i;
-        const int e = __shfl_sync(0xffffffffu, lane * PER + at, from);
-        if (lane == r) mine = e;
-#pragma unroll
-        for (int i = 0; i < PER; i++) if (lane == from && i == at) key[i] = 0u;
-    }
-    return mine;
-}
-__device__ __forceinline__ int qw_pick(const float *est, int ne, int topk, const DevState *state, int lane) {
-    const int e = ne <= 128 ? qw_pick_from<4>(est, ne, topk, lane) : qw_pick_from<8>(est, ne, topk, lane);      // ne <= 256
-#ifdef BRRR_TEST_HOOKS
-    if (state && (state->test_hooks & 1u) && state->pos % 3 == 0 && lane == topk - 1) return (e + 1) % ne;
-#else
-    (void)state;
-#endif
-    return e;
-}
-
 // The exact routing a step's combine uses, by one warp: slot_of[k] = slot (rank of the estimate) of the expert of rank k, wts[k] its weight.
 // est: the words of the step's seq-th publication by the router, awaited with a bound (the router does not depend on any kernel that waits
 // here, and the waiting kernels leave it room on an SM); picked: the estimate's expert of slot `lane`.  Else top and weights as they are.
@@ -649,7 +608,7 @@ __global__ void __launch_bounds__(QG_THREADS, 2) qw_gate_up_kernel(const __grid_
     }
     pdl_wait_cta();
     if (__any_sync(0xffffffffu, run > 0)) {
-        const int e = a.est ? qw_pick(a.est, a.ne, a.topk, a.state, lane) : a.top[min(lane, a.topk - 1)];
+        const int e = a.est ? spec_pick(a.est, a.ne, a.topk, a.topk, a.state, lane) : a.top[min(lane, a.topk - 1)];
         const int mine = __shfl_sync(0xffffffffu, e, slot);
         if (run > 0) bulk_g2s(dst, src + (size_t)mine * expert_bytes, bytes, &bar[grp]);
         if (warp == 0) pdl_trigger();           // only now (warp 0 always has a copy): the down projection fetches its rows at once, and these come first
@@ -731,7 +690,7 @@ __global__ void __launch_bounds__(QD_THREADS, 2) qw_down_kernel(const __grid_con
     float *dots = terms + (size_t)a.per_cta * nun;                     // [slot][row]
     Waiter waiter(a.state ? &a.state->err : nullptr);
     int picked = 0;              // warp 0 (the copies) and the last (the routing): the expert of slot `lane`
-    if (warp == 0 || warp == QG_WARPS) picked = a.est ? qw_pick(a.est, a.ne, a.topk, a.state, lane) : a.top[min(lane, a.topk - 1)];
+    if (warp == 0 || warp == QG_WARPS) picked = a.est ? spec_pick(a.est, a.ne, a.topk, a.topk, a.state, lane) : a.top[min(lane, a.topk - 1)];
     if (warp == 0) {
         if (lane == 0) {
             mbar_init(&bar, 1);

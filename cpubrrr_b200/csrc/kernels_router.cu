@@ -451,7 +451,7 @@ cudaError_t launch_router_rows(const float *xn, int d, const float *Wt, const fl
 // ---------------------------------------------------------------- routing hint (speculation)
 // A fast, order-free estimate of the router: one CTA per expert forms its logit with a parallel
 // reduction (a few ulps away from the serial chain); consumers pick the k largest themselves
-// (warp_spec_select).  The estimate only decides WHICH experts' gate/up weights start streaming while ffn_in_kernel walks
+// (spec_pick).  The estimate only decides WHICH experts' gate/up weights start streaming while ffn_in_kernel walks
 // the exact serial chains next to it; the exact top-k, its order and its weights still come from
 // ffn_in_kernel, and down_combine_kernel refuses (spec_fail_step) any step whose exact expert set
 // is not covered by the estimate, so results never depend on this kernel.

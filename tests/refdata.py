@@ -154,3 +154,23 @@ def set_exponents(data_dir, blob, tensor, exponents, rows=None, cols=None):
             raw[b, 1:] = np.arange(16) % 2 * 0x80 + np.arange(16) % 3 % 2 * 8      # +0 and -0
         raw[b, 0] = ex
     raw.flush()
+
+
+def plain_data_dir(out_dir, cfg, seed, edit=lambda name, raw: raw):
+    """The parts of a gpt-oss data directory that loading a model needs, for any shape: tensors of the synthetic model, each through
+    edit(name, bytes).  Returns (data_dir, blob_path)."""
+    blob, rows = os.path.join(out_dir, "model.bin"), ["data_start 0"]
+    with open(blob, "wb") as f:
+        for name, ty, dims, raw in S.model_tensors(cfg, seed):
+            nel = 1
+            for n in dims:
+                nel *= n
+            rows.append(f"{name} {ty} {f.tell()} {nel}")
+            f.write(edit(name, raw))
+            f.write(b"\0" * (-f.tell() % 32))
+    with open(os.path.join(out_dir, "manifest.txt"), "w") as w:
+        w.write("\n".join(rows) + "\n")
+    with open(os.path.join(out_dir, "config.txt"), "w") as w:
+        for k in ("n_embd", "n_layer", "n_head", "n_head_kv", "head_dim", "n_expert", "n_expert_used", "n_ff_exp", "n_vocab", "sliding_window", "rope_freq_base", "rms_eps"):
+            w.write(f"{k} {getattr(cfg, k)}\n")
+    return out_dir, blob

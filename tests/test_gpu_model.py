@@ -295,6 +295,39 @@ def test_speculation_can_be_disabled(brrr, orc, monkeypatch):
     eng.close()
 
 
+@pytest.mark.parametrize("ne,topk", [(8, 4), (40, 4), (200, 8)])
+def test_router_estimate_that_is_no_number(brrr, tmp_path, monkeypatch, ne, topk):
+    """A layer whose normalised residual is NaN: every entry of the router and of its estimate is one, and the picks still are experts.  The kernels that
+    speculate (tensor cores, integer units) and the plain step give the same bits, and a sound model runs after them as before."""
+    import refdata
+    cfg = brrr.make_cfg(128, 2, 4, 2, ne, topk, 512)
+    d, blob = refdata.plain_data_dir(str(tmp_path), cfg, 6, lambda name, raw: raw if name != "blk.0.ffn_norm.weight" else np.full(128, np.nan, np.float32).tobytes())
+    prompt = S.synth_prompt(6, 5, 500)
+
+    def run(var=None):
+        if var:
+            monkeypatch.setenv(var, "1")
+        eng = brrr.Engine.open(d, blob)
+        if var:
+            monkeypatch.delenv(var)
+        toks = greedy(eng.run, prompt, 12)
+        eng.prefill(prompt)
+        toks += [int(t) for t in eng.decode(toks[0], len(prompt), 12)]
+        out = toks, bits(eng.logits())
+        assert max(toks) < cfg.n_vocab and eng.wait_fallbacks() == 0
+        eng.close()
+        return out
+
+    sound = brrr.Engine.synth(cfg, 6)
+    want = greedy(sound.run, prompt, 12)
+    first = run()
+    for var in ("BRRR_NOMXT", "BRRR_NOSPEC"):
+        got = run(var)
+        assert got[0] == first[0] and np.array_equal(got[1], first[1]), var
+    assert greedy(sound.run, prompt, 12) == want
+    sound.close()
+
+
 def test_prompt_tiles_match_serial(brrr):
     """run_tile walks tiles of tokens through the layers together (MoE block on the tensor-core tile
     kernels); the reference guarantees its batched prefill is bit-identical to the token-serial
