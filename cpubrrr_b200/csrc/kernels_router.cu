@@ -98,7 +98,7 @@ template <int PER>
 __device__ __forceinline__ void warp_topk_n(const RouterArgs &a, const float *lg, int lane, uint32_t seq) {
     uint32_t key[PER];
 #pragma unroll
-    for (int i = 0; i < PER; i++) key[i] = lane * PER + i < a.ne ? max(float_orderable(lg[lane * PER + i]), 1u) : 0u;
+    for (int i = 0; i < PER; i++) key[i] = lane * PER + i < a.ne ? max(float_orderable(__fadd_rn(lg[lane * PER + i], 0.0f)), 1u) : 0u;      // (-0 and +0 are equals)
     float mine = 0.0f;                           // lane r: logit and expert of rank r
     int mine_e = 0;
 #pragma unroll 1

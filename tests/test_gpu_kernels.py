@@ -197,6 +197,23 @@ def test_router_topk(L, orc, dev, ne, d, topk, bias):
     assert np.array_equal(bits(dwt.cpu().numpy()), bits(wts))
 
 
+@pytest.mark.parametrize("ne,topk", [(8, 4), (40, 3), (200, 8)])
+def test_router_topk_signed_zeros(L, orc, dev, ne, topk):
+    """Logits -0 and +0 are equals: the lower index first."""
+    import torch
+    d = 64
+    w, xn, b = np.zeros((ne, d), np.float32), np.full(d, -1.0, np.float32), np.full(ne, -0.0, np.float32)
+    b[1::3] = 0.0
+    b[::5] = -1.0
+    dl, dwt = (torch.empty(n, dtype=torch.float32, device=dev) for n in (ne, topk))
+    dt = torch.empty(topk, dtype=torch.int32, device=dev)
+    dw, db, dxn = to_dev(w, dev), to_dev(b, dev), to_dev(xn, dev)
+    ok(L.brrr_router_topk(P(dw), P(db), P(dxn), ne, d, topk, P(dl), P(dt), P(dwt), None))
+    logits, top, wts = orc.router_topk(w, b, xn, topk)
+    assert np.signbit(logits[2]) and not np.signbit(logits[1])
+    assert np.array_equal(bits(dl.cpu().numpy()), bits(logits)) and np.array_equal(dt.cpu().numpy(), top) and np.array_equal(bits(dwt.cpu().numpy()), bits(wts))
+
+
 def test_swiglu_quant(L, orc, dev):
     import torch
     topk, d = 4, 2880
