@@ -14,33 +14,9 @@
 #endif
 
 // ---------------------------------------------------------------- scalar helpers
-__device__ __forceinline__ float brrr_expf_dev(float x) {
-    // Cephes-style expf as a fixed operation sequence (range reduction by ln2 hi/lo, degree-5
-    // polynomial, every multiply-add fused, two-step power-of-two scaling).
-    if (x != x) return x + x;
-    if (x > 88.72283935546875f) return __int_as_float(0x7f800000);
-    if (x < -104.0f) return 0.0f;
-    float kf = rintf(__fmul_rn(x, 1.44269504088896341f));
-    float r = __fmaf_rn(kf, -0.693145751953125f, x);
-    r = __fmaf_rn(kf, -1.42860682030941723212e-6f, r);
-    float p = 1.9875691500e-4f;
-    p = __fmaf_rn(p, r, 1.3981999507e-3f);
-    p = __fmaf_rn(p, r, 8.3334519073e-3f);
-    p = __fmaf_rn(p, r, 4.1665795894e-2f);
-    p = __fmaf_rn(p, r, 1.6666665459e-1f);
-    p = __fmaf_rn(p, r, 5.0000001201e-1f);
-    float r2 = __fmul_rn(r, r);
-    float y = __fmaf_rn(p, r2, r);
-    y = __fadd_rn(y, 1.0f);
-    int k = (int)kf;
-    int k1 = k >> 1, k2 = k - k1;
-    float s1 = __int_as_float((k1 + 127) << 23);
-    float s2 = __int_as_float((k2 + 127) << 23);
-    return __fmul_rn(__fmul_rn(y, s1), s2);
-}
-
-// brrr_expf_dev of N values, step by step side by side, the special cases as selections (as branches they keep calls from overlapping: 260 cycles each
-// in a loop of 32).
+// exp(x) of N values, step by step side by side: Cephes-style expf as a fixed operation sequence (range reduction by ln2 hi/lo, degree-5
+// polynomial, every multiply-add fused, two-step power-of-two scaling).  The special cases are selections: as branches they keep calls from
+// overlapping (260 cycles each in a loop of 32).
 template <int N>
 __device__ __forceinline__ void brrr_expf_n(float *x) {
     float kf[N], r[N], p[N], y[N];
@@ -62,11 +38,15 @@ __device__ __forceinline__ void brrr_expf_n(float *x) {
 #pragma unroll
     for (int i = 0; i < N; i++) {
         const int k = (int)kf[i], k1 = k >> 1, k2 = k - k1;
-        y[i] = __fmul_rn(__fmul_rn(y[i], __int_as_float((k1 + 127) << 23)), __int_as_float((k2 + 127) << 23));
+        y[i] = __fmul_rn(__fmul_rn(y[i], __uint_as_float((uint32_t)(k1 + 127) << 23)), __uint_as_float((uint32_t)(k2 + 127) << 23));
         y[i] = x[i] > 88.72283935546875f ? __int_as_float(0x7f800000) : y[i];
         y[i] = x[i] < -104.0f ? 0.0f : y[i];
         x[i] = x[i] != x[i] ? x[i] + x[i] : y[i];
     }
+}
+__device__ __forceinline__ float brrr_expf_dev(float x) {
+    brrr_expf_n<1>(&x);
+    return x;
 }
 
 // 2^(e-128) for an e8m0 byte (the doubled e2m1 table), exact including e = 0, 1 (subnormal).

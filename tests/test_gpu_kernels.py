@@ -30,9 +30,18 @@ def L(brrr):
 def test_expf_bits(L, orc, dev):
     import torch
     x = np.concatenate([np.linspace(-104.5, 89.0, 20001), np.linspace(-3, 3, 10001), [0.0, -0.0, 88.72283, -87.4, -103.0]]).astype(np.float32)
+    # the borders of the special cases with their neighbours, infinities, and every power of the scaling down to the subnormal results
+    edge = np.float32([88.72283935546875, -104.0, -87.33654, -87.33655, -103.97208, -103.2789])
+    x = np.concatenate([x, edge, np.nextafter(edge, np.float32(np.inf)), np.nextafter(edge, np.float32(-np.inf)), np.float32([np.inf, -np.inf, 3e38, -3e38, 1e-45]),
+                        (np.arange(-151, 129) * np.log(2.0)).astype(np.float32), ((np.arange(-151, 129) + 0.5) * np.log(2.0)).astype(np.float32)])
+    want = orc.expf(x)
+    assert ((want > 0) & (want < np.finfo(np.float32).tiny)).sum() > 100
     dx = to_dev(x, dev); dy = torch.empty_like(dx)
     ok(L.brrr_expf(P(dx), x.size, P(dy), None))
-    assert np.array_equal(bits(dy.cpu().numpy()), bits(orc.expf(x)))
+    assert np.array_equal(bits(dy.cpu().numpy()), bits(want))
+    nan = to_dev(np.float32([np.nan, -np.nan, 0.0]), dev)
+    ok(L.brrr_expf(P(nan), 3, P(nan), None))
+    assert np.isnan(nan.cpu().numpy()).tolist() == [True, True, False]
 
 
 @pytest.mark.parametrize("n", [32, 2880, 4096])
