@@ -70,8 +70,8 @@ def test_moe_ffn_step_tensor_cores_bit_exact(brrr, orc, dev, shape):
 
 
 def test_worst_case_magnitudes_stay_exact(brrr, orc, dev):
-    """Activation bytes at +-127 in every position (digits 3, -3, -1 / -3, 3, 1) against all weight codes:
-    the largest partial sums the digit planes can produce."""
+    """Activation bytes at +-127 in every position (the largest lane sums; digits 2, 0, -1 and -2, 0, 1), and at -36 and 92 in all but one of a
+    block's (digits 0, -4, -4 and 2, -4, -4: the largest sums of a digit plane), against all weight codes."""
     import torch
     cfg = brrr.make_cfg(n_embd=256, n_layer=1, n_head=4, n_head_kv=2, n_expert=4, n_expert_used=4, n_vocab=256)
     eng = brrr.Engine.synth(cfg, 9)
@@ -79,9 +79,12 @@ def test_worst_case_magnitudes_stay_exact(brrr, orc, dev):
     om = orc.Model.synth(ocfg, 9)
     rng = np.random.default_rng(3)
     P = lambda t: C.c_void_p(t.data_ptr())
-    for trial in range(4):
+    for trial in range(6):
         sign = rng.integers(0, 2, 256) * 2 - 1
         xn = (sign * (1.0 + 0.001 * (trial == 3) * rng.random(256))).astype(np.float32)     # every |x| equal: every byte +-127
+        if trial >= 4:
+            xn = np.full(256, (-36, 92)[trial - 4], np.float32)
+            xn[rng.integers(0, 32, 8) + 32 * np.arange(8)] = 127.0
         want_y, want_top, _ = _ffn_oracle(orc, om, ocfg, xn)
         dy = torch.zeros(256, dtype=torch.float32, device=dev)
         eng.moe_ffn_step_tc(0, P(to_dev(xn, dev)), P(dy), None, None)
@@ -152,3 +155,50 @@ def test_block_exponents_of_any_size(brrr, orc, dev, tmp_path, exponents, wide, 
 def test_block_exponents_choose_the_form(brrr):
     """Which form the matrices of a layer run in: by the layer's own blocks, gate | up and down each by themselves."""
     _run_with_hooks(brrr, "exponents")
+
+
+# gate and up exponent, down exponent, whether the matrices run in the wide form, activation scale (gate of the order of one, or h below
+# the quantiser's smallest block maximum of 1e-12)
+WHOLE = [
+    (49, 49, False, 2.0 ** 70),
+    (134, 134, False, 2.0 ** -14),
+    (123, 49, False, 2.0 ** -43),        # activation and h both at the smallest block scale, 1e-12 / 127
+    (49, 134, False, 2.0 ** 70),
+    (48, 48, True, 2.0 ** 71),
+    (135, 135, True, 2.0 ** -15),
+    (1, 0, True, 2.0 ** 118),            # block scales that are subnormal numbers
+    (190, 190, True, 2.0 ** -43),
+]
+
+
+@pytest.mark.parametrize("gate_up,down,wide,scale", WHOLE)
+def test_matrices_of_one_block_exponent(brrr, orc, dev, tmp_path, gate_up, down, wide, scale):
+    """Every block of a matrix at one end of a form's range, no bias, a residual of zero: nothing absorbs or clamps a product that is not exact.  Five
+    block pairs (a whole group of scales and half of one), a ragged tile of down."""
+    import torch
+    import refdata
+    cfg = brrr.make_cfg(320, 1, 4, 2, 8, 4, 256)
+
+    def edit(name, raw):
+        if name.endswith("_exps.bias"):
+            return bytes(len(raw))
+        if not name.endswith("_exps.weight"):
+            return raw
+        blocks = np.frombuffer(raw, np.uint8).reshape(-1, 17).copy()
+        blocks[:, 0] = down if "down" in name else gate_up
+        return blocks.tobytes()
+
+    d, blob = refdata.plain_data_dir(str(tmp_path), cfg, 21, edit)
+    eng, om = brrr.Engine.open(d, blob), orc.Model.open(d, blob)
+    assert eng.uses_tensor_experts
+    P = lambda t: C.c_void_p(t.data_ptr())
+    for seed in range(3):
+        xn = S.synth_input(40 + seed, cfg.n_embd) * np.float32(scale)
+        want = _ffn_oracle(orc, om, ocfg_of(orc, cfg), xn)[0]
+        assert np.isfinite(want).all() and np.count_nonzero(want) > 300 and len(np.unique(np.abs(want))) > 300      # (subnormal sums coincide at times)
+        dxn, y = to_dev(xn, dev), [torch.zeros(cfg.n_embd, dtype=torch.float32, device=dev) for _ in range(2)]
+        eng.moe_ffn_step_tc(0, P(dxn), P(y[0]), None, None)
+        eng.moe_ffn_step(0, P(dxn), P(y[1]), None, None)
+        for got in y:
+            assert np.array_equal(bits(got.cpu().numpy()), bits(want))
+    eng.close()
