@@ -17,10 +17,7 @@ __device__ __forceinline__ uint64_t tl_smem_desc(const void *p, uint32_t lbo, ui
     d |= (uint64_t)1 << 46;                      // descriptor version of this architecture
     return d;
 }
-__device__ __forceinline__ void tl_commit(uint64_t *bar) {
-    asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(smem_u32(bar)) : "memory");
-}
-// The same under a predicate: an issuing warp whose instructions carry its elected lane's predicate, instead of standing in a one-lane branch,
+// The barrier's phase completes with the products that the lanes with issue != 0 have issued so far.  A predicate: an issuing warp whose instructions carry its elected lane's predicate, instead of standing in a one-lane branch,
 // keeps a uniform loop and its descriptors and addresses in uniform registers, where these instructions want them.
 __device__ __forceinline__ void tl_commit_if(uint32_t issue, uint64_t *bar) {
     asm volatile("{\n\t.reg .pred e;\n\tsetp.ne.b32 e, %1, 0;\n\t@e tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];\n\t}" ::"r"(smem_u32(bar)), "r"(issue) : "memory");

@@ -71,11 +71,9 @@ constexpr int XT_PRODUCER = 8, XT_ISSUER = 9;
 #ifdef BRRR_TEST_HOOKS
 #define XT_T0() long long xt_t0_ = clock64()
 #define XT_ACC(v) do { long long xt_t1_ = clock64(); (v) += xt_t1_ - xt_t0_; xt_t0_ = xt_t1_; } while (0)
-#define XT_STAMP(state, i) do { if ((state) && blockIdx.x == BRRR_STAMP_BX && blockIdx.y == 0) (state)->stamps[i] = clock64(); } while (0)
 #else
 #define XT_T0() do { } while (0)
 #define XT_ACC(v) do { } while (0)
-#define XT_STAMP(state, i) do { } while (0)
 #endif
 
 // ---------------------------------------------------------------- pack: 16-row units -> tile units
