@@ -35,9 +35,9 @@
 // Operand B: the digits of an activation (brrr_mxt.cuh) are written once by the kernel that quantises it (the routing-estimate kernel
 // for the token, the gate/up epilogue for h); every CTA spreads them over a zeroed image in its shared memory.
 //
-// Pipeline per CTA, in rounds of four block pairs: warp 8 issues the bulk copies into a ring of stages, an elected lane of warp 9
-// the scale copies and the MMAs into one of two accumulator regions (96 columns), warps 0-3 and 4-7 read half a region each at once and carry two chains each.
-// Every wait is bounded.
+// Pipeline per CTA, in rounds of four block pairs: warp 8 issues the bulk copies into a ring of stages, an elected lane of warp 9 the scale copies
+// and the MMAs of the even rounds into one accumulator region (96 columns), one of warp 10 those of the odd rounds into the other, warps 0-3 and 4-7
+// read half a region each at once and carry two chains each.  Every wait is bounded.
 //
 // What bounds it: hand-overs and first instructions more than anything.  20b shape, position 100, gate/up from its dependency wait to its end 11.3 us
 // (14.3 with the planes joined by multiply-adds and the scales multiplied in by the epilogue) for 35 MB, down 6.9 us (8.2) for 18 MB: 1.7 us until
@@ -789,8 +789,7 @@ void launch_mx_exp_scan(const uint8_t *raw, size_t blocks, uint32_t *bad, cudaSt
     if (blocks) mx_exp_scan_kernel<<<148 * 8, 256, 0, st>>>(raw, blocks, bad);
 }
 
-// A down CTA has the footprint of a gate/up CTA: it fits beside a running one, sets up and starts its weight stream there, before gate/up has
-// finished (measured: 745 tok/s against 728 with a 9-stage ring that needs an SM of its own).
+// A down CTA has the footprint of a gate/up CTA: it fits beside a running one, sets up and starts its weight stream there, before gate/up has finished.
 template <bool DOWN, bool EP, bool WIDE>
 static cudaError_t xt_launch_form(const XtArgs &a, dim3 grid, bool pdl, cudaStream_t st) {
     static unsigned long long configured = 0;      // one bit per device
