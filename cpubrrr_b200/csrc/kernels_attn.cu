@@ -374,7 +374,7 @@ __global__ void __launch_bounds__(at_threads(AT_TILE)) attn_decode_kernel(AttnAr
 // 32 pairs x 4096 keys of scores do not fit shared memory: they wait in a workspace (128 bytes per key; mostly L2).
 // What bounds it is shared memory: a key's row reaches a warp as 16 broadcast words of 16 bytes, 3 to 4 cycles each, for 80 arithmetic instructions
 // (40 packed ones), and a key of the p.V sums costs every thread 40 bytes for 16 multiply-adds.  Two CTAs per SM fill each other's barriers.  512 rows of
-// the 20b shape: window layer 79 to 87 us, full layer 122 / 285 / 449 us at positions 0 / 512 / 1024 (before, with tiles of 128 keys, one CTA per SM,
+// the 20b shape: window layer 78 to 87 us, full layer 122 / 280 / 442 us at positions 0 / 512 / 1024 (before, with tiles of 128 keys, one CTA per SM,
 // scalar scores and every warp in the same phase: 140 to 146, 221 / 483 / 742).  Two pairs per thread and one CTA per SM took 85 to 95, 124 / 298 / 471.
 constexpr int AR_THREADS = 256;
 constexpr int AR_PAIRS = 32;

@@ -40,8 +40,9 @@
 // read half a region each at once and carry two chains each.  Every wait is bounded.
 //
 // What bounds it: hand-overs and first instructions more than anything.  20b shape, position 100, gate/up from its dependency wait to its end 11.3 us
-// (14.3 with the planes joined by multiply-adds and the scales multiplied in by the epilogue) for 35 MB, down 6.9 us (8.2) for 18 MB: 1.7 us until
-// the experts are picked, 2 us until the first round is through, then 600-700 cycles a round (975), 220 of them arithmetic.
+// (14.3 with the planes joined by multiply-adds and the scales multiplied in by the epilogue) for 35 MB, down 7.3 us (8.2) for 18 MB: 1.4 us until
+// the experts are picked and the digits spread, 2.1 us until the first round is through, then 500-700 cycles a round (975), 220 of them arithmetic, but
+// 1900 for the fifth, the first one whose copies were not under way from the beginning (down, whose copies start before h is there: 870).
 // What did not help: announcing down's tiles to L2 from gate/up's last rounds (no change), the issuing loop unrolled by ring stage (1300 cycles
 // for each of the first four rounds: instructions met for the first time), running indices in a one-lane branch (1091 against 1050 us a step).
 #include "brrr_kernels.h"

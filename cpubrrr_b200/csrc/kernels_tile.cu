@@ -21,9 +21,11 @@
 // What bounds it: the workers' instruction stream.  The chains - per row, token and block four fused multiply-adds that nothing may
 // reorder - take about 2.8 cycles per packed instruction (three 64-bit operands from the register file), 490 cycles per pair of
 // 128 rows x 32 tokens and scheduler; with reads, scales and barriers a pair takes 900.  Beside it run the products (four of 50 to
-// 60 cycles) and the copies.  Measured on 512 rows of the 20b shape (ncu, one launch): gate | up 671 us and down 313 us (before,
-// with int8 operands decoded by the workers and one conversion per dot: 2 x 835 and 835), q/k/v 160 and o-proj 142 us (integer
-// units: 520 and 480).
+// 60 cycles) and the copies.  Measured on 512 rows of the 20b shape (ncu, one launch): gate | up 595 us (671 with the products issued in a
+// one-lane branch) and down 309 us (before, with int8 operands decoded by the workers and one conversion per dot: 2 x 835 and 835),
+// q/k/v 161 and o-proj 142 us (integer units: 520 and 480).  At 8 tokens per CTA (64 rows, gate | up 138 us, three CTAs per SM) it is the workers too:
+// of 900 to 1140 cycles a pair (with clock stamps) they multiply for 370 to 470, prepare scales for 100 to 160, read tensor memory for 110 and wait
+// for products for 170 to 190, while the issuing warps wait for them to leave a buffer for three quarters of the time.
 //
 // Roles of a CTA (128 matrix rows x up to NT tokens).  Worker warps: NT / 8 groups of four.  Then two producer
 // warps (asynchronous copies of the pairs' operands into a ring) and two issuing warps (four products per pair, even
@@ -129,7 +131,7 @@ __global__ void __launch_bounds__(NT * 16 + 128, KIND == TK_Q8 || NT == 32 ? 1 :
     __shared__ uint32_t tmem_base_sh;
     __shared__ int task_sh[3];               // expert, first entry, entries
     __shared__ int ent[NT];
-    // gate | up: a warp index the compiler knows to be uniform (591 us per 512-row tile of the 20b shape against 636; the other kinds lose 3 to 8 % with it)
+    // gate | up: a warp index the compiler knows to be uniform (7 % of a 512-row tile of the 20b shape; the other kinds lose 3 to 8 % with it)
     const int tid = threadIdx.x, warp = KIND == TK_GLU ? __shfl_sync(0xffffffffu, tid >> 5, 0) : tid >> 5, lane = tid & 31;
     // ---- what needs nothing from the kernels before
     if (KIND != TK_Q8) mx_fill_scale_table(tbl, tid, THREADS);
